@@ -139,40 +139,215 @@ cudaError_t launch_tall_t_mul(const float* X, long long ldx, long long strideX, 
   return cudaGetLastError();
 }
 
+// ------------------------------------------------------------------------------------------ 128 x 128 triangular leaves
+// Both leaf kernels work on one (up to) 128 x 128 block per CTA of 1024 threads, the block and its inverse in shared memory
+// as 4 x 4 sub-blocks of 32.  A refresh of an eigenbasis factors 16 leaves per 2048-wide factor and round, one after the
+// other, so the latency of one CTA is all that counts; it is set by the length of the dependent chain, not by the 0.7 MFLOP.
+//   factor R^T R = G, panel of 32 rows by panel: the 32 x 32 diagonal block in one warp (lane = column, the column in
+//     registers, pivots and multipliers by shuffle), the rows of the panel to its right by substitution (thread = column,
+//     column in registers), the trailing blocks by a rank-32 update (4 x up to 3 elements per thread).  Every element
+//     receives the same products in the same order as in an element-wise right-looking factorisation; that form needed two
+//     barriers per pivot, 256 of them, and a leaf took 108 us (two SOAP steps on 8 x 1024^2, 32 leaves: 9.82 -> 8.19 ms).
+//   invert R: the four diagonal blocks (one warp each, lane = column in registers), then the blocks above the diagonal by
+//     distance d = 1, 2, 3:  X_IJ = -X_II (sum_{K = I+1 .. J} R_IK X_KJ), J = I + d, four rows per warp.
+// A non-positive or non-finite pivot is replaced by 1 and counted in info[b] (the result for that matrix is then
+// meaningless, the others are unaffected).
 namespace {
 
-// One CTA inverts one upper-triangular block by back substitution; thread j produces column j of the inverse:
-//   x_jj = 1 / t_jj,   x_ij = -(sum_{k = i+1 .. j} t_ik x_kj) / t_ii   for i = j-1 .. 0.
-// Both the block and its inverse sit in shared memory (2 x 128 x 129 floats).  The work is O(blk^3 / 6) FMAs spread
-// over 128 threads; at 64 blocks per call this takes tens of microseconds, against a library triangular solve per
-// leaf that walks the batch one matrix at a time.
-__global__ void __launch_bounds__(kTriBlock) tri_inv_blocks_kernel(const float* __restrict__ Q, long long ld, long long strideQ,
-                                                                 int n, float* __restrict__ X) {
-  extern __shared__ float tri_smem[];
-  float (*t)[kTriBlock + 1] = reinterpret_cast<float (*)[kTriBlock + 1]>(tri_smem);
-  float (*x)[kTriBlock + 1] = reinterpret_cast<float (*)[kTriBlock + 1]>(tri_smem + kTriBlock * (kTriBlock + 1));
-  const int blk = blockIdx.x, b = blockIdx.y, nblk = gridDim.x;
-  const int r0 = blk * kTriBlock, size = min(kTriBlock, n - r0);
-  const float* q = Q + (long long)b * strideQ + (long long)r0 * ld + r0;
-  const int j = threadIdx.x;
-  for (int i = 0; i < kTriBlock; ++i) {  // row i of the block, coalesced over j
-    float v = (i == j) ? 1.f : 0.f;
-    if (i < size && j < size && j >= i) v = q[(long long)i * ld + j];
-    t[i][j] = v;
-    x[i][j] = 0.f;
+constexpr int kLeafThreads = 1024;
+constexpr int kLeafLd = kTriBlock + 4;  // rows start on 16-byte boundaries: four values of a row per (broadcast) load
+constexpr int kLeafBytes = 2 * kTriBlock * kLeafLd * (int)sizeof(float);
+constexpr int kSub = 32, kSubs = kTriBlock / kSub;
+
+// Loads the upper part of a block of `size` rows; a short block is completed by an identity.  x <- 0.
+__device__ __forceinline__ void load_upper(const float* __restrict__ g, long long ld, int size, float* t, float* x) {
+  float v[kTriBlock * kTriBlock / kLeafThreads];
+#pragma unroll
+  for (int e = 0; e < kTriBlock * kTriBlock / kLeafThreads; ++e) {
+    const int idx = threadIdx.x + e * kLeafThreads, i = idx >> 7, j = idx & (kTriBlock - 1);
+    v[e] = (i == j) ? 1.f : 0.f;
+    if (i < size && j < size && j >= i) v[e] = g[(long long)i * ld + j];
   }
-  __syncthreads();
-  {
-    x[j][j] = 1.0f / t[j][j];
-    for (int i = j - 1; i >= 0; --i) {
-      float s = 0.f;
-      for (int k = i + 1; k <= j; ++k) s = fmaf(t[i][k], x[k][j], s);
-      x[i][j] = -s / t[i][i];
+#pragma unroll
+  for (int e = 0; e < kTriBlock * kTriBlock / kLeafThreads; ++e) {
+    const int idx = threadIdx.x + e * kLeafThreads, i = idx >> 7, j = idx & (kTriBlock - 1);
+    t[i * kLeafLd + j] = v[e];
+    x[i * kLeafLd + j] = 0.f;
+  }
+}
+
+// x <- t^-1 for the upper-triangular block t; the part of x below the diagonal blocks is scratch.
+__device__ __forceinline__ void invert_upper(const float* t, float* x) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < kSubs) {  // right-looking back substitution: row i of this lane's column is final when step i starts
+    const float* d = t + warp * kSub * (kLeafLd + 1);
+    float* xd = x + warp * kSub * (kLeafLd + 1);
+    float acc[kSub];
+#pragma unroll
+    for (int i = 0; i < kSub; ++i) acc[i] = 0.f;
+#pragma unroll
+    for (int i = kSub - 1; i >= 0; --i) {
+      const float piv = d[i * kLeafLd + i];
+      const float xi = i == lane ? 1.0f / piv : (i < lane ? -acc[i] / piv : 0.f);
+      xd[i * kLeafLd + lane] = xi;
+#pragma unroll
+      for (int k = 0; k < i; ++k) acc[k] = fmaf(d[k * kLeafLd + i], xi, acc[k]);
     }
   }
   __syncthreads();
-  float* out = X + ((long long)b * nblk + blk) * kTriBlock * kTriBlock;
-  for (int i = 0; i < kTriBlock; ++i) out[i * kTriBlock + j] = x[i][j];
+  const int I = warp >> 3, r0 = (warp & 7) * 4;  // four rows of the I-th block at the current distance
+#pragma unroll 1
+  for (int dist = 1; dist < kSubs; ++dist) {
+    const int J = I + dist;
+    const bool on = J < kSubs;
+    if (on) {  // S = sum_K R_IK X_KJ, parked in the mirror position below the diagonal
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int k = kSub * (I + 1); k < kSub * (J + 1); k += 4) {
+        float xv[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) xv[e] = x[(k + e) * kLeafLd + kSub * J + lane];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float4 a = *(const float4*)(t + (kSub * I + r0 + r) * kLeafLd + k);
+          s[r] = fmaf(a.x, xv[0], s[r]); s[r] = fmaf(a.y, xv[1], s[r]); s[r] = fmaf(a.z, xv[2], s[r]); s[r] = fmaf(a.w, xv[3], s[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) x[(kSub * J + r0 + r) * kLeafLd + kSub * I + lane] = s[r];
+    }
+    __syncthreads();
+    if (on) {
+      float s[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int k = r0; k < kSub; k += 4) {  // X_II is upper triangular: columns left of the row are zero
+        float sv[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) sv[e] = x[(kSub * J + k + e) * kLeafLd + kSub * I + lane];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float4 a = *(const float4*)(x + (kSub * I + r0 + r) * kLeafLd + kSub * I + k);
+          s[r] = fmaf(a.x, sv[0], s[r]); s[r] = fmaf(a.y, sv[1], s[r]); s[r] = fmaf(a.z, sv[2], s[r]); s[r] = fmaf(a.w, sv[3], s[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 4; ++r) x[(kSub * I + r0 + r) * kLeafLd + kSub * J + lane] = -s[r];
+    }
+    __syncthreads();
+  }
+}
+
+__global__ void __launch_bounds__(kLeafThreads) tri_inv_blocks_kernel(const float* __restrict__ Q, long long ld, long long strideQ,
+                                                                     int n, float* __restrict__ X) {
+  extern __shared__ __align__(16) float leaf_smem[];
+  float *t = leaf_smem, *x = leaf_smem + kTriBlock * kLeafLd;
+  const int blk = blockIdx.x, b = blockIdx.y, r0 = blk * kTriBlock;
+  load_upper(Q + (long long)b * strideQ + (long long)r0 * ld + r0, ld, min(kTriBlock, n - r0), t, x);
+  __syncthreads();
+  invert_upper(t, x);
+  float* out = X + ((long long)b * gridDim.x + blk) * kTriBlock * kTriBlock;
+  for (int idx = threadIdx.x; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
+    const int i = idx >> 7, j = idx & (kTriBlock - 1);
+    out[idx] = j >= i ? x[i * kLeafLd + j] : 0.f;
+  }
+}
+
+__global__ void __launch_bounds__(kLeafThreads) chol_inv_leaf_kernel(const float* __restrict__ G, long long ldg, long long strideG,
+                                                                     float* __restrict__ R, long long ldr, long long strideR,
+                                                                     float* __restrict__ X, long long strideX, int size,
+                                                                     int* __restrict__ info) {
+  extern __shared__ __align__(16) float leaf_smem[];
+  float *t = leaf_smem, *x = leaf_smem + kTriBlock * kLeafLd;
+  __shared__ float inv_piv[kSub];
+  __shared__ int failed;
+  const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) failed = 0;
+  load_upper(G + (long long)b * strideG, ldg, size, t, x);
+  __syncthreads();
+
+  for (int base = 0; base < size; base += kSub) {
+    float* d = t + base * (kLeafLd + 1);
+    if (warp == 0) {
+      float a[kSub];
+      bool bad = false;
+#pragma unroll
+      for (int i = 0; i < kSub; ++i) a[i] = d[i * kLeafLd + lane];
+#pragma unroll
+      for (int k = 0; k < kSub; ++k) {
+        const float piv = __shfl_sync(0xffffffffu, a[k], k);
+        const bool ok = piv > 0.f && piv < 3.0e38f;
+        const float inv = ok ? rsqrtf(piv) : 1.f;
+        bad = bad || !ok;
+        if (lane == k) {
+          a[k] = ok ? piv * inv : 1.f;  // sqrt of the pivot
+          inv_piv[k] = inv;
+        } else {
+          a[k] *= inv;
+        }
+#pragma unroll
+        for (int i = k + 1; i < kSub; ++i) a[i] = fmaf(-__shfl_sync(0xffffffffu, a[k], i), a[k], a[i]);
+      }
+#pragma unroll
+      for (int i = 0; i < kSub; ++i)
+        if (i <= lane) d[i * kLeafLd + lane] = a[i];
+      if (lane == 0 && bad) failed = 1;
+    }
+    __syncthreads();
+    const int rest = kTriBlock - base - kSub;  // columns right of the panel
+    if (tid < rest) {
+      float* col = d + kSub + tid;
+      float a[kSub];
+#pragma unroll
+      for (int i = 0; i < kSub; ++i) a[i] = col[i * kLeafLd];
+#pragma unroll
+      for (int k = 0; k < kSub; ++k) {
+        a[k] *= inv_piv[k];
+#pragma unroll
+        for (int i = k + 1; i < kSub; ++i) a[i] = fmaf(-d[k * kLeafLd + i], a[k], a[i]);
+        col[k * kLeafLd] = a[k];
+      }
+    }
+    __syncthreads();
+    if (warp * 4 < rest) {  // rows i0 .. i0+3 of the trailing block, columns from the 32-block of i0 on
+      const int i0 = warp * 4, first = i0 & ~(kSub - 1);
+      const float* panel = d + kSub;  // panel[k * ld + i] = r_ki of trailing row / column i
+      float* trail = t + (base + kSub) * (kLeafLd + 1);
+      for (int j = first + lane; j < rest; j += kSub) {
+        float acc[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) acc[r] = trail[(i0 + r) * kLeafLd + j];
+#pragma unroll 8
+        for (int k = 0; k < kSub; ++k) {
+          const float4 m = *(const float4*)(panel + k * kLeafLd + i0);
+          const float rkj = panel[k * kLeafLd + j];
+          acc[0] = fmaf(-m.x, rkj, acc[0]); acc[1] = fmaf(-m.y, rkj, acc[1]);
+          acc[2] = fmaf(-m.z, rkj, acc[2]); acc[3] = fmaf(-m.w, rkj, acc[3]);
+        }
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+          if (j >= i0 + r) trail[(i0 + r) * kLeafLd + j] = acc[r];
+      }
+    }
+    __syncthreads();
+  }
+
+  invert_upper(t, x);
+
+  float* r = R + (long long)b * strideR;
+  float* out = X + (long long)b * strideX;
+  for (int idx = tid; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
+    const int i = idx >> 7, j = idx & (kTriBlock - 1);
+    if (i < size && j < size) r[(long long)i * ldr + j] = j >= i ? t[i * kLeafLd + j] : 0.f;
+    out[idx] = j >= i ? x[i * kLeafLd + j] : 0.f;
+  }
+  if (tid == 0 && failed && info != nullptr) atomicAdd(info + b, 1);
+}
+
+cudaError_t configure_leaf_kernels() {
+  static bool configured = false;
+  if (configured) return cudaSuccess;
+  cudaError_t e = cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeafBytes);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(chol_inv_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeafBytes);
+  configured = e == cudaSuccess;
+  return e;
 }
 
 }  // namespace
@@ -180,132 +355,20 @@ __global__ void __launch_bounds__(kTriBlock) tri_inv_blocks_kernel(const float* 
 cudaError_t launch_tri_inv_blocks(const float* Q, long long ld, long long strideQ, int batch, int n, float* X,
                                   cudaStream_t stream) {
   if (batch == 0 || n == 0) return cudaSuccess;
-  constexpr int kBytes = 2 * kTriBlock * (kTriBlock + 1) * (int)sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  cudaError_t e = configure_leaf_kernels();
+  if (e != cudaSuccess) return e;
   dim3 grid((n + kTriBlock - 1) / kTriBlock, batch);
-  tri_inv_blocks_kernel<<<grid, kTriBlock, kBytes, stream>>>(Q, ld, strideQ, n, X);
+  tri_inv_blocks_kernel<<<grid, kLeafThreads, kLeafBytes, stream>>>(Q, ld, strideQ, n, X);
   return cudaGetLastError();
 }
-
-
-// ------------------------------------------------------------------------------------------ Cholesky leaf
-// One CTA of 1024 threads factors one (up to) 128 x 128 symmetric positive definite block G = R^T R (R upper triangular)
-// and inverts R, both in shared memory.
-//   factor (right-looking, every trailing element has its own thread slot):
-//     for k = 0 .. n-1:  r_kk = sqrt(g_kk);  r_kj = g_kj / r_kk (j > k);  g_ij -= r_ki r_kj (k < i <= j)
-//   invert: the four 32 x 32 diagonal blocks by back substitution (one warp each, lane = column), then the blocks
-//     above the diagonal by distance d = 1, 2, 3:  X_IJ = -X_II (sum_{K = I+1 .. J} R_IK X_KJ), J = I + d,
-//     as 32 x 32 block products with one output element per thread.
-// A non-positive or non-finite pivot is replaced by 1 and counted in info[b] (the result for that matrix is then
-// meaningless, the others are unaffected).  The refresh of an eigenbasis factors 16 leaves per 2048-wide factor and
-// round, one after the other, so the latency of this kernel is what counts: a thread-per-column version took 270 us
-// (dependent shared-memory loads), the batched library factorisation plus a separate inversion 230 us.
-namespace {
-
-constexpr int kLeafThreads = 1024;
-constexpr int kLeafLd = kTriBlock + 1;
-
-__global__ void __launch_bounds__(kLeafThreads) chol_inv_leaf_kernel(const float* __restrict__ G, long long ldg, long long strideG,
-                                                                     float* __restrict__ R, long long ldr, long long strideR,
-                                                                     float* __restrict__ X, long long strideX, int size,
-                                                                     int* __restrict__ info) {
-  extern __shared__ float leaf_smem[];
-  float(*t)[kLeafLd] = (float(*)[kLeafLd])leaf_smem;
-  float(*x)[kLeafLd] = (float(*)[kLeafLd])(leaf_smem + kTriBlock * kLeafLd);
-  __shared__ int failed;
-  const int b = blockIdx.x, tid = threadIdx.x, ty = tid >> 5, tx = tid & 31;
-  const float* g = G + (long long)b * strideG;
-  if (tid == 0) failed = 0;
-  for (int idx = tid; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {  // upper part; a short block is completed by an identity
-    const int i = idx >> 7, j = idx & (kTriBlock - 1);
-    float v = (i == j) ? 1.f : 0.f;
-    if (i < size && j < size && j >= i) v = g[(long long)i * ldg + j];
-    t[i][j] = v;
-    x[i][j] = 0.f;
-  }
-  __syncthreads();
-
-  for (int k = 0; k < size; ++k) {
-    const float d = t[k][k];  // written for the last time in the previous step's trailing update
-    const bool ok = d > 0.f && d < 3.0e38f;
-    const float inv_piv = ok ? rsqrtf(d) : 1.f;
-    if (tid > k && tid < size) t[k][tid] *= inv_piv;
-    __syncthreads();
-    if (tid == 0) {
-      t[k][k] = ok ? d * inv_piv : 1.f;  // sqrt(d); nobody reads the diagonal entry during the trailing update
-      if (!ok) failed = 1;
-    }
-    for (int i = k + 1 + ty; i < size; i += 32) {
-      const float rki = t[k][i];
-      for (int j = i + tx; j < size; j += 32) t[i][j] = fmaf(-rki, t[k][j], t[i][j]);
-    }
-    __syncthreads();
-  }
-
-  if (tid < kTriBlock) {  // diagonal 32 x 32 blocks: warp = block, lane = column
-    const int base = tid & ~31, jl = tid & 31, col = base + jl;
-    x[col][col] = 1.0f / t[col][col];
-    for (int i = jl - 1; i >= 0; --i) {
-      float sum = 0.f;
-      for (int k = i + 1; k <= jl; ++k) sum = fmaf(t[base + i][base + k], x[base + k][col], sum);
-      x[base + i][col] = -sum / t[base + i][base + i];
-    }
-  }
-  __syncthreads();
-  for (int dist = 1; dist < kTriBlock / 32; ++dist) {
-    // S_I = sum_K R_IK X_KJ, parked in the (otherwise unused) mirror position below the diagonal
-    for (int I = 0; I + dist < kTriBlock / 32; ++I) {
-      const int J = I + dist;
-      float s0 = 0.f, s1 = 0.f;
-      const float* rrow = &t[32 * I + ty][0];
-      for (int k = 32 * (I + 1); k < 32 * (J + 1); k += 2) {
-        s0 = fmaf(rrow[k], x[k][32 * J + tx], s0);
-        s1 = fmaf(rrow[k + 1], x[k + 1][32 * J + tx], s1);
-      }
-      x[32 * J + ty][32 * I + tx] = s0 + s1;
-    }
-    __syncthreads();
-    for (int I = 0; I + dist < kTriBlock / 32; ++I) {
-      const int J = I + dist;
-      float s0 = 0.f, s1 = 0.f;
-      for (int k = ty; k < 32; k += 2) {  // X_II is upper triangular: columns below the row index are zero
-        s0 = fmaf(x[32 * I + ty][32 * I + k], x[32 * J + k][32 * I + tx], s0);
-        if (k + 1 < 32) s1 = fmaf(x[32 * I + ty][32 * I + k + 1], x[32 * J + k + 1][32 * I + tx], s1);
-      }
-      x[32 * I + ty][32 * J + tx] = -(s0 + s1);
-    }
-    __syncthreads();
-  }
-
-  float* r = R + (long long)b * strideR;
-  float* out = X + (long long)b * strideX;
-  for (int idx = tid; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
-    const int i = idx >> 7, j = idx & (kTriBlock - 1);
-    if (i < size && j < size) r[(long long)i * ldr + j] = j >= i ? t[i][j] : 0.f;
-    out[idx] = j >= i ? x[i][j] : 0.f;
-  }
-  if (tid == 0 && failed && info != nullptr) atomicAdd(info + b, 1);
-}
-
-}  // namespace
 
 cudaError_t launch_chol_inv_leaf(const float* G, long long ldg, long long strideG, float* R, long long ldr, long long strideR,
                                  float* X, long long strideX, int batch, int size, int* info, cudaStream_t stream) {
   if (batch == 0 || size == 0) return cudaSuccess;
   if (size > kTriBlock) return cudaErrorInvalidValue;
-  constexpr int kBytes = 2 * kTriBlock * (kTriBlock + 1) * (int)sizeof(float);
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(chol_inv_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  chol_inv_leaf_kernel<<<batch, kLeafThreads, kBytes, stream>>>(G, ldg, strideG, R, ldr, strideR, X, strideX, size, info);
+  cudaError_t e = configure_leaf_kernels();
+  if (e != cudaSuccess) return e;
+  chol_inv_leaf_kernel<<<batch, kLeafThreads, kLeafBytes, stream>>>(G, ldg, strideG, R, ldr, strideR, X, strideX, size, info);
   return cudaGetLastError();
 }
 

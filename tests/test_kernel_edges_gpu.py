@@ -1,0 +1,39 @@
+"""Edges of tiles, chunks and leaves of the sm_100a kernels: remainders, smallest and largest sizes of a range, several sizes in
+one launch.  Oracles are fp64 restatements or the package's PyTorch definitions."""
+
+import pytest
+import torch
+
+from heavyball_b200 import ops
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# ---------------------------------------------------------------------------------------- triangular leaves
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 64, 95, 127, 128])
+def test_cholesky_leaf_at_sub_block_edges(n):
+    """Factor and inverse of one leaf at sizes around its 32-wide sub-blocks, for condition numbers up to 1e4: a backward
+    stable factorisation reproduces the matrix to n eps and the inverse to n eps times the condition number of the factor."""
+    ext = ops.load()
+    gen = torch.Generator(DEV).manual_seed(n)
+    q = torch.linalg.qr(torch.randn(3, n, n, device=DEV, generator=gen, dtype=torch.float64))[0]
+    lam = torch.logspace(0, -4 if n > 1 else 0, n, device=DEV, dtype=torch.float64)
+    g = ((q * lam) @ q.mT).float()
+    g = (g + g.mT) / 2
+    r, info = torch.zeros_like(g), torch.zeros(3, dtype=torch.int32, device=DEV)
+    inv = torch.full((3, 1, 128, 128), float("nan"), device=DEV)
+    ext.chol_inv_leaf(g, r, inv, 0, n, info)
+    assert info.sum().item() == 0
+    assert torch.equal(r, r.triu())
+    eps = 2.0**-23
+    assert (r.double().mT @ r.double() - g.double()).abs().max().item() < 8 * n * eps
+    x = inv[:, 0, :n, :n].double()
+    assert (x @ r.double() - torch.eye(n, device=DEV, dtype=torch.float64)).abs().max().item() < 8 * n * eps * 1e2
+    assert torch.equal(ext.tri_inv_blocks(r)[:, 0, :n, :n], inv[:, 0, :n, :n])
+    bad = g.clone()
+    bad[1, n // 2, n // 2] = -1.0
+    ext.chol_inv_leaf(bad, r, inv, 0, n, info)
+    assert info.tolist() == [0, 1, 0]
