@@ -868,7 +868,7 @@ def _run_precond(opt, prog: _Program, states, group, grads, params, on_gpu: bool
         b1 = utils.beta_debias(utils.get_beta1(group), step - 1)
         b2 = utils.beta_debias(utils.get_beta2(group), step - 1)
         stat_w = 1 - utils.beta_debias(group["shampoo_beta"], step)
-        vec = []  # members without any eigenbasis: plain Adam / LaProp on the update
+        vec, live = [], []  # members without any eigenbasis: plain Adam / LaProp on the update; buckets with one
         for shape, idx, U, O in buckets:
             members = [states[i] for i in idx]
             if all(q is None for q in members[0][keys["Q"]]):
@@ -876,9 +876,12 @@ def _run_precond(opt, prog: _Program, states, group, grads, params, on_gpu: bool
                 continue
             U3, O3 = (U, O) if U.ndim == 3 else (U.unsqueeze(1), O.unsqueeze(1))
             bucket = _stage_bucket(prog, group, shape, len(idx), lambda: matrix_stage.SoapBucket(keys, _SOAP_INNER[stage.fn_name]))
-            with _stage("soap.refresh" if group["is_preconditioning"] else "soap.project"):
-                bucket.run(members, U3, O3, group, b1=b1, b2=b2, eps=group["eps"], stat_w=stat_w,
-                           refresh=bool(group["is_preconditioning"]))  # fmt: skip
+            with _stage("soap.project"):
+                bucket.run(members, U3, O3, group, b1=b1, b2=b2, eps=group["eps"], stat_w=stat_w)
+            live.append(bucket)
+        if live and group["is_preconditioning"]:
+            with _stage("soap.refresh"):
+                matrix_stage.refresh(live)
         if vec:
             m = [states[i][keys["exp_avg"]] for i in vec]
             v = [states[i][keys["exp_avg_sq"]] for i in vec]

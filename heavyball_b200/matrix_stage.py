@@ -226,10 +226,10 @@ class SoapBucket:
         if ptrs != self.q_ptrs:
             self.q_ptrs, self.q_ops = ptrs, None
 
-    def run(self, members: List[dict], U: Tensor, out: Tensor, group, *, b1, b2, eps, stat_w, refresh: bool):
+    def run(self, members: List[dict], U: Tensor, out: Tensor, group, *, b1, b2, eps, stat_w):
         """``U``: ``(B, R, C)`` fp32 updates of the bucket (read only); ``out``: same shape, receives the
         preconditioned update.  ``b1`` / ``b2``: debiased moment coefficients; ``stat_w``: weight of this step's outer
-        products in the statistics; ``refresh``: advance the eigenbases after the statistics."""
+        products in the statistics."""
         self._adopt(members)
         Ql, Qr = self.Q
         B, R, C = U.shape
@@ -266,9 +266,13 @@ class SoapBucket:
             be.gemm(u_same, u_same, mode=ops.EPI_LERP, w=stat_w, out=self.GG[0])
         if len(self.GG) > 1 and self.GG[1] is not None:
             be.gemm(u_trans, u_trans, mode=ops.EPI_LERP, w=stat_w, out=self.GG[1])
-        if refresh:  # in place on the adopted state; its orthogonalisation replays its own graphs
-            utils.get_orthogonal_matrix_QR(self.GG, self.Q, self.m)
-            self.q_ops = None
+
+def refresh(buckets: Sequence["SoapBucket"]):
+    """Advances the eigenbases of all buckets of a step together, in place on the adopted state; the orthogonalisation
+    replays its own graphs."""
+    utils.refresh_eigenbases([(b.GG, b.Q, b.m) for b in buckets])
+    for b in buckets:
+        b.q_ops = None
 
 
 # ---------------------------------------------------------------------------------------- PSGD (Kron)

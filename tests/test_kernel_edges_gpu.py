@@ -4,7 +4,7 @@ one launch.  Oracles are fp64 restatements or the package's PyTorch definitions.
 import pytest
 import torch
 
-from heavyball_b200 import ops
+from heavyball_b200 import ops, utils
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -37,3 +37,28 @@ def test_cholesky_leaf_at_sub_block_edges(n):
     bad[1, n // 2, n // 2] = -1.0
     ext.chol_inv_leaf(bad, r, inv, 0, n, info)
     assert info.tolist() == [0, 1, 0]
+
+
+def test_eigenbases_of_several_buckets_refresh_together():
+    """One joint refresh of three buckets (shared sizes, one factor missing) against the bucket-by-bucket definition."""
+    gen = torch.Generator(DEV).manual_seed(5)
+
+    def factor(b, n):
+        q = torch.linalg.qr(torch.randn(b, n, n, device=DEV, generator=gen))[0]
+        noise = torch.randn(b, n, n, device=DEV, generator=gen) * 0.02 / n**0.5
+        return (q * torch.logspace(1, 0, n, device=DEV)) @ q.mT + noise + noise.mT, q
+
+    items = []
+    for b, (r, c) in ((2, (256, 256)), (3, (256, 384)), (1, (384, None))):
+        gl, ql = factor(b, r)
+        gr, qr = factor(b, c) if c else (None, None)
+        items.append(([gl, gr], [ql, qr], torch.randn(b, r, c or 64, device=DEV, generator=gen)))
+    clone = lambda xs: [None if x is None else x.clone() for x in xs]  # noqa: E731
+    want = [(clone(g), clone(q), m.clone()) for g, q, m in items]
+    for g, q, m in want:
+        utils.get_orthogonal_matrix_QR(g, q, m)
+    utils.refresh_eigenbases(items)
+    for (_, q, m), (_, q0, m0) in zip(items, want):
+        for x, y in zip([*q, m], [*q0, m0]):
+            if x is not None:
+                torch.testing.assert_close(x, y, rtol=0, atol=2e-4)
