@@ -10,6 +10,26 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
+# ---------------------------------------------------------------------------------------- fused chain
+
+
+def test_ecc_codec_over_all_exponents():
+    """State values over the whole exponent range (both sides of the codec's exponent threshold, zeros and subnormals): a step
+    with zero gradient and momentum coefficient 1 - eps decodes, scales and encodes each value once."""
+    exps = torch.arange(-148, 120, device=DEV, dtype=torch.float64)
+    value = torch.cat([torch.zeros(4, device=DEV, dtype=torch.float64), (2.0**exps) * 1.37, -(2.0**exps) * 1.91]).float()
+    prim = value.to(torch.bfloat16)
+    res = torch.randint(-127, 128, value.shape, device=DEV, dtype=torch.int8)
+    out = torch.empty_like(value)
+    ops.fused_chain(g=[torch.zeros_like(value)], u=[out], s0=[prim], s0e=[res], algo=ops.EXP_AVG, n_state=1, b1=1.0,
+                    out_mode=ops.OUT_UPDATE, dt_g=ops.F32, dt_u=ops.F32, dt_s=ops.BF16E8, dt_p=ops.NONE)  # fmt: skip
+    # half a unit in the last place of a bf16 value, times residual / 127
+    e = torch.clamp(torch.frexp(prim.double())[1] - 1, min=-126).double()
+    want = prim.double() + (res.double() / 127) * 2.0 ** (e - 8)
+    big = want.abs() > 1e-30
+    torch.testing.assert_close(out[big].double(), want[big], rtol=1e-6, atol=0)
+
+
 # ---------------------------------------------------------------------------------------- triangular leaves
 
 
