@@ -671,7 +671,7 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
         if side is not main:
             side.wait_event(ready)
             used.append(side)
-        chunk = max(1, _NS_WORKSPACE_BYTES // (R * Cc * 8))  # four bf16 work copies per matrix
+        chunk = max(1, _NS_WORKSPACE_BYTES // (R * Cc * 8))  # bf16 work copies per matrix: two of it, two of its Gram matrix
         with torch.cuda.stream(side), _stage(f"ns/{R}x{Cc}"):
             norms = sq.index_select(0, sel_idx)
             for c0 in range(0, len(idx), chunk):

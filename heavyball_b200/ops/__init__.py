@@ -228,10 +228,9 @@ def newton_schulz_batched(mats: Sequence[torch.Tensor], coeffs, out: Optional[to
     R, C = mats[0].shape
     dev = mats[0].device
     m, n = (R, C) if R <= C else (C, R)
-    ldx, ldxt, lds = _round_up(n, 8), _round_up(m, 8), _round_up(m, 8)
+    ldx, lds = _round_up(n, 8), _round_up(m, 8)
     bf = dict(dtype=torch.bfloat16, device=dev)
     X = [torch.empty(B, m, ldx, **bf) for _ in range(2)]
-    XT = [torch.empty(B, n, ldxt, **bf) for _ in range(2)]
     S = torch.empty(B, m, lds, **bf)
     Y = torch.empty(B, m, lds, **bf)
     if out is None:
@@ -244,14 +243,12 @@ def newton_schulz_batched(mats: Sequence[torch.Tensor], coeffs, out: Optional[to
         launch_counter.count += 1
     else:
         norms = sumsq.contiguous()
-    if R <= C:
-        ext.ns_prepare(srcs, dtype_code(mats[0]), R, C, norms, eps, X[0], ldx, XT[0], ldxt, seed)
-    else:  # work on the transpose so that the Gram matrix is the small one
-        ext.ns_prepare(srcs, dtype_code(mats[0]), R, C, norms, eps, XT[0], ldxt, X[0], ldx, seed)
+    # a tall matrix is worked on transposed so that the Gram matrix is the small one
+    ext.ns_prepare(srcs, dtype_code(mats[0]), R, C, norms, eps, X[0], ldx, R > C, seed)
     status = _status(dev)
     launch_counter.count += 1 + 3 * len(coeffs)
     # one call issues the three launches of every step (Gram, polynomial, apply; the last apply writes `out`)
-    ext.ns_chain(X, XT, S, Y, out, m, n, ldx, ldxt, lds, R, C, [[float(v) for v in abc] for abc in coeffs], float(out_scale),
+    ext.ns_chain(X, S, Y, out, m, n, ldx, lds, R, C, [[float(v) for v in abc] for abc in coeffs], float(out_scale),
                  status)  # fmt: skip
     return out
 

@@ -218,19 +218,20 @@ at::Tensor segmented_reduce(const std::vector<at::Tensor>& xs, const std::vector
   return out;
 }
 
-// Normalise + stochastically round a batch of same-shape matrices into the two bf16 work layouts.
+// Normalise + stochastically round a batch of same-shape matrices into the bf16 iterate: [batch, R, ld] as they are, or
+// [batch, C, ld] transposed.
 void ns_prepare(const std::vector<at::Tensor>& srcs, int src_dt, int64_t R, int64_t C, const at::Tensor& sumsq_t, double eps,
-                at::Tensor same, int64_t ld_same, at::Tensor trans, int64_t ld_trans, uint64_t seed) {
-  c10::cuda::CUDAGuard guard(same.device());
+                at::Tensor dst, int64_t ld, bool trans, uint64_t seed) {
+  c10::cuda::CUDAGuard guard(dst.device());
   std::vector<const void*> ptrs(srcs.size());
   for (size_t i = 0; i < srcs.size(); ++i) ptrs[i] = srcs[i].data_ptr();
-  at::Tensor dev = at::empty({(int64_t)(ptrs.size() * sizeof(void*))}, same.options().dtype(at::kByte));
+  at::Tensor dev = at::empty({(int64_t)(ptrs.size() * sizeof(void*))}, dst.options().dtype(at::kByte));
   auto stream = at::cuda::getCurrentCUDAStream();
   check(cudaMemcpyAsync(dev.data_ptr(), ptrs.data(), ptrs.size() * sizeof(void*), cudaMemcpyHostToDevice, stream),
         "pointer upload");
   check(hb::launch_ns_prepare((const void* const*)dev.data_ptr(), src_dt, (int)R, (int)C, (int)srcs.size(),
-                              sumsq_t.data_ptr<float>(), (float)eps, same.data_ptr(), ld_same, R * ld_same,
-                              trans.data_ptr(), ld_trans, C * ld_trans, seed, stream), "ns_prepare launch");
+                              sumsq_t.data_ptr<float>(), (float)eps, dst.data_ptr(), ld, (trans ? C : R) * ld, trans ? 1 : 0,
+                              seed, stream), "ns_prepare launch");
 }
 
 // D = A * B^T (bf16, K-major operands, batched) with the fused epilogues described in ns_gemm.h.
@@ -254,30 +255,40 @@ void ns_gemm(const at::Tensor& A, int64_t lda, int64_t strideA, const at::Tensor
 }
 
 // The whole Newton-Schulz iteration of one shape bucket in one call: per step Gram, polynomial and apply launches (the
-// last apply writes fp32 into `out`, in the caller's orientation).  x / xt: the two ping-pong pairs of the iterate
-// [batch, m, ldx] and its transpose [batch, n, ldxt] (bf16), pair 0 prepared by ns_prepare; s, y: [batch, m, lds] (bf16).
-void ns_chain(const std::vector<at::Tensor>& x, const std::vector<at::Tensor>& xt, const at::Tensor& s, const at::Tensor& y,
-              at::Tensor& out, int64_t m, int64_t n, int64_t ldx, int64_t ldxt, int64_t lds, int64_t R, int64_t C,
-              const std::vector<std::vector<double>>& coeffs, double out_scale, const at::Tensor& status) {
-  TORCH_CHECK(x.size() == 2 && xt.size() == 2, "ns_chain: two ping-pong buffers per orientation");
-  const int64_t batch = s.size(0);
+// last apply writes fp32 into `out`, in the caller's orientation).  x: the two ping-pong buffers of the iterate
+// [batch, m, ldx] (bf16), the first prepared by ns_prepare; s, y: [batch, m, lds] (bf16).
+void ns_chain(const std::vector<at::Tensor>& x, const at::Tensor& s, const at::Tensor& y, at::Tensor& out, int64_t m, int64_t n,
+              int64_t ldx, int64_t lds, int64_t R, int64_t C, const std::vector<std::vector<double>>& coeffs, double out_scale,
+              const at::Tensor& status) {
+  TORCH_CHECK(x.size() == 2, "ns_chain: two ping-pong buffers");
+  c10::cuda::CUDAGuard guard(s.device());
+  auto stream = at::cuda::getCurrentCUDAStream();
   int cur = 0;
-  const OptT none;
   for (size_t step = 0; step < coeffs.size(); ++step) {
     TORCH_CHECK(coeffs[step].size() == 3, "ns_chain: (a, b, c) per step");
-    const bool last = step + 1 == coeffs.size();
-    ns_gemm(x[cur], ldx, m * ldx, x[cur], ldx, m * ldx, m, m, n, batch, 0 /* gram */, true, s, lds, m * lds, s, lds, m * lds,
-            none, 0, 0, false, 1.0, none, 0, 0, 0.0, 0.0, 0.0, status);
-    ns_gemm(s, lds, m * lds, s, lds, m * lds, m, m, m, batch, 1 /* poly */, true, y, lds, m * lds, y, lds, m * lds, none, 0, 0,
-            false, 1.0, s, lds, m * lds, coeffs[step][0], coeffs[step][1], coeffs[step][2], status);
-    if (!last) {
-      ns_gemm(y, lds, m * lds, xt[cur], ldxt, n * ldxt, m, n, m, batch, 2 /* apply */, false, x[1 - cur], ldx, m * ldx,
-              xt[1 - cur], ldxt, n * ldxt, none, 0, 0, false, 1.0, none, 0, 0, 0.0, 0.0, 0.0, status);
-      cur = 1 - cur;
+    auto* X = (__nv_bfloat16*)x[cur].data_ptr();
+    auto* S = (__nv_bfloat16*)s.data_ptr();
+    auto* Y = (__nv_bfloat16*)y.data_ptr();
+    hb::GemmParams G{};  // S = X X^T
+    G.batch = (int)s.size(0); G.status = status.data_ptr<int>(); G.f_scale = 1.f;
+    G.M = G.N = (int)m;
+    hb::GemmParams A = G, Q = G;
+    G.mode = hb::kModeGram; G.K = (int)n; G.symmetric = 1;
+    G.C = G.CT = S; G.ldc = G.ldct = lds; G.strideC = G.strideCT = m * lds;
+    check(hb::launch_ns_gemm(X, ldx, m * ldx, X, ldx, m * ldx, G, stream), "ns_chain gram launch");
+    Q.mode = hb::kModePoly; Q.K = (int)m; Q.symmetric = 1;  // Y = c S S + b S + a I
+    Q.C = Q.CT = Y; Q.ldc = Q.ldct = lds; Q.strideC = Q.strideCT = m * lds;
+    Q.S = S; Q.lds = lds; Q.strideS = m * lds;
+    Q.ca = (float)coeffs[step][0]; Q.cb = (float)coeffs[step][1]; Q.cc = (float)coeffs[step][2];
+    check(hb::launch_ns_gemm(S, lds, m * lds, S, lds, m * lds, Q, stream), "ns_chain poly launch");
+    A.mode = hb::kModeApply; A.N = (int)n; A.K = (int)m; A.b_mn = 1;  // X' = Y X
+    if (step + 1 < coeffs.size()) {
+      A.C = (__nv_bfloat16*)x[1 - cur].data_ptr(); A.ldc = ldx; A.strideC = m * ldx;
     } else {
-      ns_gemm(y, lds, m * lds, xt[cur], ldxt, n * ldxt, m, n, m, batch, 2 /* apply */, false, none, 0, 0, none, 0, 0, out, C,
-              R * C, R > C, out_scale, none, 0, 0, 0.0, 0.0, 0.0, status);
+      A.F = out.data_ptr<float>(); A.ldf = C; A.strideF = R * C; A.f_transposed = R > C ? 1 : 0; A.f_scale = (float)out_scale;
     }
+    check(hb::launch_ns_gemm(Y, lds, m * lds, X, ldx, m * ldx, A, stream), "ns_chain apply launch");
+    cur = 1 - cur;
   }
 }
 

@@ -4,10 +4,12 @@
 // is executed as three batched bf16 GEMMs with fp32 accumulation in tensor memory:
 //     gram : S  = X  X^T                       (symmetric: upper-triangular tiles only, mirrored)
 //     poly : Y  = c S S + b S + a I            (symmetric; S is both operands and an epilogue input)
-//     apply: X' = Y X                          (also writes X'^T, the K-major operand of the next step)
-// All three are "TN" products D[M,N] = A[M,K] * B[N,K]^T with both operands K-major, so a single
-// kernel serves them; only the epilogue differs.  Keeping X^T alongside X is what makes the third
-// product K-major as well.
+//     apply: X' = Y X
+// Gram and polynomial are "TN" products D[M,N] = A[M,K] * B[N,K]^T with both operands K-major; the apply product takes
+// X as it lies in memory ([K, N], N contiguous) through an MN-major B descriptor, so the iterate exists once and no
+// transposed copy of it is ever written (half of the bytes of every apply epilogue and of the prologue; GPT-2-small's
+// 48 matrices: 2634 -> 2513 us, a Llama-3-8B layer: 19.97 -> 18.71 ms).
+// One kernel serves all three; only the B box, its descriptor and the epilogue differ.
 //
 // Kernel structure (one 128x128 output tile per CTA, 192 threads, two CTAs resident per SM so one
 // CTA's epilogue overlaps the other's main loop):
@@ -44,6 +46,12 @@ constexpr uint32_t kTmemCols = 128;
 
 // bf16 x bf16 -> fp32, both operands K-major, M = 128, N = 128.
 constexpr uint32_t kInstrDesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+
+// B given as [K, N] with N contiguous (MN-major): boxes of 64 columns x 64 rows of K, one 128-byte swizzle atom wide.
+// Consecutive groups of 64 columns are one box apart, groups of 8 rows of K 1 KiB; 16 rows of K are 2 KiB.
+constexpr int kMnBoxBytes = 64 * BK * 2;
+constexpr uint32_t kMnStep = (16 * 128) >> 4;
+constexpr uint32_t kInstrBMn = 1u << 16;
 
 // ------------------------------------------------------------------------------------------ kernel
 __global__ void __launch_bounds__(kGemmThreads, 2)
@@ -108,7 +116,12 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
           // diagonal tiles of a symmetric product multiply a row block with itself: one load feeds both operands
           mbar_expect_tx(&full_bar[s], same_ab ? kTileBytes : kStageBytes);
           tma_load_3d(a_dst, &map_a, &full_bar[s], kb * BK, tm * BM, batch);
-          if (!same_ab) tma_load_3d(a_dst + kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN, batch);
+          if (P.b_mn) {  // [K, N] operand: two boxes of 64 columns x 64 rows of K
+            tma_load_3d(a_dst + kTileBytes, &map_b, &full_bar[s], tn * BN, kb * BK, batch);
+            tma_load_3d(a_dst + kTileBytes + kMnBoxBytes, &map_b, &full_bar[s], tn * BN + 64, kb * BK, batch);
+          } else if (!same_ab) {
+            tma_load_3d(a_dst + kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN, batch);
+          }
         } else {
           mbar_expect_tx(&full_bar[s], kStageBytes);  // S[tm-block, tn-block] for the polynomial epilogue, as two 64-column halves
           tma_load_3d(a_dst, &map_a, &full_bar[s], tn * BN, tm * BM, batch);
@@ -126,11 +139,13 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
         const uint32_t a_addr = smem_u32(tiles + s * kStageBytes);
-        const uint64_t a_desc = make_smem_desc(a_addr), b_desc = same_ab ? a_desc : make_smem_desc(a_addr + kTileBytes);
+        const uint64_t a_desc = make_smem_desc(a_addr);
+        const uint64_t b_desc = same_ab ? a_desc : (P.b_mn ? make_smem_desc_mn(a_addr + kTileBytes, kMnBoxBytes) : make_smem_desc(a_addr + kTileBytes));
+        const uint32_t b_step = P.b_mn ? kMnStep : 2u, idesc = kInstrDesc | (P.b_mn ? kInstrBMn : 0u);
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) {
           // advancing 16 bf16 (32 B) along K inside the swizzle atom = +2 in 16-byte address units
-          tc_mma_bf16(tmem_base, a_desc + 2 * k, b_desc + 2 * k, kInstrDesc, (kb | k) ? 1u : 0u);
+          tc_mma_bf16(tmem_base, a_desc + 2 * k, b_desc + b_step * k, idesc, (kb | k) ? 1u : 0u);
         }
         tc_commit(&empty_bar[s]);
       }
@@ -326,8 +341,14 @@ ns_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         tma_load_3d(dst, &map_a, &full_bar[s], kb * BK, tm * BM2, batch);
         tma_load_3d(dst + kTileBytes, &map_a, &full_bar[s], kb * BK, tm * BM2 + 128, batch);
         if (!same_ab) {
-          tma_load_3d(dst + 2 * kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN2, batch);
-          tma_load_3d(dst + 3 * kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN2 + 128, batch);
+          if (P.b_mn) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              tma_load_3d(dst + 2 * kTileBytes + j * kMnBoxBytes, &map_b, &full_bar[s], tn * BN2 + j * 64, kb * BK, batch);
+          } else {
+            tma_load_3d(dst + 2 * kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN2, batch);
+            tma_load_3d(dst + 3 * kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN2 + 128, batch);
+          }
         }
         issued = kb + 1;
       }
@@ -343,12 +364,13 @@ ns_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
         const uint32_t base = smem_u32(tiles + s * kStageBytes2);
         const uint64_t a_top = make_smem_desc(base), a_bot = make_smem_desc(base + kTileBytes);
         // 256 operand rows = 32 eight-row groups, 1 KiB apart: the two 128-row boxes are contiguous
-        const uint64_t b_desc = same_ab ? a_top : make_smem_desc(base + 2 * kTileBytes);
+        const uint64_t b_desc = same_ab ? a_top : (P.b_mn ? make_smem_desc_mn(base + 2 * kTileBytes, kMnBoxBytes) : make_smem_desc(base + 2 * kTileBytes));
+        const uint32_t b_step = P.b_mn ? kMnStep : 2u, idesc = kInstrDesc256 | (P.b_mn ? kInstrBMn : 0u);
 #pragma unroll
         for (int k = 0; k < BK / 16; ++k) {
           const uint32_t acc = (kb | k) ? 1u : 0u;
-          tc_mma_bf16(tmem_base, a_top + 2 * k, b_desc + 2 * k, kInstrDesc256, acc);
-          tc_mma_bf16(tmem_base + 256u, a_bot + 2 * k, b_desc + 2 * k, kInstrDesc256, acc);
+          tc_mma_bf16(tmem_base, a_top + 2 * k, b_desc + b_step * k, idesc, acc);
+          tc_mma_bf16(tmem_base + 256u, a_bot + 2 * k, b_desc + b_step * k, idesc, acc);
         }
         tc_commit(&empty_bar[s]);
       }
@@ -480,16 +502,15 @@ ns_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 }
 
 // ------------------------------------------------------------------------------------------ prologue
-// X = SR_bf16(G / max(||G||_F, eps)) written twice: in the source orientation and transposed (one of the
-// two is the K-major operand X, the other X^T).  `sumsq[b]` holds ||G_b||_F^2.
+// X = SR_bf16(G / max(||G||_F, eps)), written in the source orientation (`trans` == 0) or transposed, whichever makes the
+// Gram matrix the small one.  `sumsq[b]` holds ||G_b||_F^2.
 // One block handles a 64 x 64 tile: 256 threads as 16 column-groups (4 columns each) x 16 rows, four row
-// passes.  Loads are 16 B (fp32) / 8 B (bf16), both outputs are written with 8-byte stores; the
-// transpose goes through shared memory.  Grid: (ceil(C/64), ceil(R/64), batch).
+// passes.  Loads are 16 B (fp32) / 8 B (bf16), stores 8 bytes; the transpose goes through shared memory.
+// Grid: (ceil(C/64), ceil(R/64), batch).
 __global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __restrict__ srcs, int src_dt, int R, int C,
                                                         const float* __restrict__ sumsq, float eps,
-                                                        __nv_bfloat16* __restrict__ same, int64_t ld_same,
-                                                        int64_t stride_same, __nv_bfloat16* __restrict__ trans,
-                                                        int64_t ld_trans, int64_t stride_trans, uint64_t seed) {
+                                                        __nv_bfloat16* __restrict__ dst, int64_t ld, int64_t stride, int trans,
+                                                        uint64_t seed) {
   __shared__ uint16_t tile[64][66];
   const int b = blockIdx.z;
   const void* src = srcs[b];
@@ -498,30 +519,35 @@ __global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __re
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
   const int c0 = blockIdx.x * 64 + tx * 4;
   const bool vec = (C & 3) == 0 && (((uintptr_t)src) & 15) == 0;
-  uint16_t* same_b = (uint16_t*)same + (int64_t)b * stride_same;
-  uint16_t* trans_b = (uint16_t*)trans + (int64_t)b * stride_trans;
+  uint16_t* dst_b = (uint16_t*)dst + (int64_t)b * stride;
+  float x[4][4];
 #pragma unroll
-  for (int pass = 0; pass < 4; ++pass) {
-    const int rl = ty + 16 * pass, r = blockIdx.y * 64 + rl;
-    float x[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int pass = 0; pass < 4; ++pass) {  // every load of the tile is in flight before the first value is used
+    const int r = blockIdx.y * 64 + ty + 16 * pass;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) x[pass][k] = 0.f;
     if (r < R && c0 < C) {
       const int64_t idx = (int64_t)r * C + c0;
       if (vec) {
         if (src_dt == kF32) {
           const float4 t = *(const float4*)((const float*)src + idx);
-          x[0] = t.x; x[1] = t.y; x[2] = t.z; x[3] = t.w;
+          x[pass][0] = t.x; x[pass][1] = t.y; x[pass][2] = t.z; x[pass][3] = t.w;
         } else {
           const uint2 t = *(const uint2*)((const uint16_t*)src + idx);
-          x[0] = bf16_bits_to_float(t.x & 0xFFFF); x[1] = bf16_bits_to_float(t.x >> 16);
-          x[2] = bf16_bits_to_float(t.y & 0xFFFF); x[3] = bf16_bits_to_float(t.y >> 16);
+          x[pass][0] = bf16_bits_to_float(t.x & 0xFFFF); x[pass][1] = bf16_bits_to_float(t.x >> 16);
+          x[pass][2] = bf16_bits_to_float(t.y & 0xFFFF); x[pass][3] = bf16_bits_to_float(t.y >> 16);
         }
       } else {
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           if (c0 + k < C)
-            x[k] = src_dt == kF32 ? ((const float*)src)[idx + k] : bf16_bits_to_float(((const uint16_t*)src)[idx + k]);
+            x[pass][k] = src_dt == kF32 ? ((const float*)src)[idx + k] : bf16_bits_to_float(((const uint16_t*)src)[idx + k]);
       }
     }
+  }
+#pragma unroll
+  for (int pass = 0; pass < 4; ++pass) {
+    const int rl = ty + 16 * pass, r = blockIdx.y * 64 + rl;
     uint16_t h[4] = {0, 0, 0, 0};
     if (r < R && c0 < C) {
       const int64_t idx = (int64_t)r * C + c0;
@@ -529,15 +555,20 @@ __global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __re
       const uint32_t rr[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
 #pragma unroll
       for (int k = 0; k < 4; ++k)
-        if (c0 + k < C) h[k] = sr_bf16_bits(x[k] * inv, rr[k]);
-      uint2 o;
-      o.x = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
-      o.y = (uint32_t)h[2] | ((uint32_t)h[3] << 16);
-      *(uint2*)(same_b + (int64_t)r * ld_same + c0) = o;  // columns past C land in the row padding (ld is a multiple of 8)
+        if (c0 + k < C) h[k] = sr_bf16_bits(x[pass][k] * inv, rr[k]);
+      if (!trans) {
+        uint2 o;
+        o.x = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
+        o.y = (uint32_t)h[2] | ((uint32_t)h[3] << 16);
+        *(uint2*)(dst_b + (int64_t)r * ld + c0) = o;  // columns past C land in the row padding (ld is a multiple of 8)
+      }
     }
+    if (trans) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) tile[rl][tx * 4 + k] = h[k];
+      for (int k = 0; k < 4; ++k) tile[rl][tx * 4 + k] = h[k];
+    }
   }
+  if (!trans) return;
   __syncthreads();
   // transposed output: this thread owns source rows r0..r0+3 (consecutive in the output row) of four source columns
   const int r0 = blockIdx.y * 64 + tx * 4;
@@ -548,54 +579,56 @@ __global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __re
       uint2 o;
       o.x = (uint32_t)tile[tx * 4 + 0][cl] | ((uint32_t)tile[tx * 4 + 1][cl] << 16);
       o.y = (uint32_t)tile[tx * 4 + 2][cl] | ((uint32_t)tile[tx * 4 + 3][cl] << 16);
-      *(uint2*)(trans_b + (int64_t)c * ld_trans + r0) = o;
+      *(uint2*)(dst_b + (int64_t)c * ld + r0) = o;
     }
   }
 }
 
 // ------------------------------------------------------------------------------------------ host side
-// bf16 tensor [batch, rows, cols] with leading dimension `ld` elements; box = 64 cols x 128 rows.
-static bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch);
+// bf16 tensor [batch, rows, cols] with leading dimension `ld` elements; box = 64 cols x `box_rows` rows.
+static bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch, int box_rows);
 
 // A step launches the same ~60 products over the same workspace addresses (the caching allocator hands the buffers
 // back), and every launch needs up to four descriptors: they are kept by their defining values instead of being
 // encoded again (about 0.6 us each on the host, which is what limits a step once the matrices are split over ranks).
-static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch) {
+static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch,
+                     int box_rows = BM) {
   struct Key {
-    const void* base; int64_t ld, stride; int rows, cols, batch;
+    const void* base; int64_t ld, stride; int rows, cols, batch, box_rows;
     bool operator==(const Key& o) const {
-      return base == o.base && ld == o.ld && stride == o.stride && rows == o.rows && cols == o.cols && batch == o.batch;
+      return base == o.base && ld == o.ld && stride == o.stride && rows == o.rows && cols == o.cols && batch == o.batch && box_rows == o.box_rows;
     }
   };
   struct Hash {
     size_t operator()(const Key& k) const {
       size_t h = std::hash<const void*>()(k.base);
-      for (int64_t v : {k.ld, k.stride, (int64_t)k.rows, (int64_t)k.cols, (int64_t)k.batch})
+      for (int64_t v : {k.ld, k.stride, (int64_t)k.rows, (int64_t)k.cols, (int64_t)k.batch, (int64_t)k.box_rows})
         h ^= std::hash<int64_t>()(v) + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
       return h;
     }
   };
   static std::unordered_map<Key, CUtensorMap, Hash> cache;
   static std::mutex guard;
-  const Key key{base, ld, batch_stride, rows, cols, batch};
+  const Key key{base, ld, batch_stride, rows, cols, batch, box_rows};
   std::lock_guard<std::mutex> lock(guard);
   auto it = cache.find(key);
   if (it != cache.end()) {
     *map = it->second;
     return true;
   }
-  if (!encode_map(map, base, rows, cols, ld, batch_stride, batch)) return false;
+  if (!encode_map(map, base, rows, cols, ld, batch_stride, batch, box_rows)) return false;
   if (cache.size() >= 4096) cache.clear();
   cache.emplace(key, *map);
   return true;
 }
 
-static bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch) {
+static bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch,
+                       int box_rows) {
   EncodeTiledFn fn = tensor_map_encoder();
   if (fn == nullptr) return false;
   cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
   cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)batch_stride * 2};
-  cuuint32_t box[3] = {BK, BM, 1};
+  cuuint32_t box[3] = {BK, (cuuint32_t)box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -615,9 +648,9 @@ cudaError_t launch_ns_gemm(const void* A, int64_t lda, int64_t strideA, const vo
     configured = true;
   }
   GemmParams Q = P;
-  Q.same_operand = (A == B && lda == ldb && strideA == strideB && P.M == P.N) ? 1 : 0;
+  Q.same_operand = (!P.b_mn && A == B && lda == ldb && strideA == strideB && P.M == P.N) ? 1 : 0;
   CUtensorMap ma, mb, mc, mct;
-  if (!make_map(&ma, A, P.M, P.K, lda, strideA, P.batch) || !make_map(&mb, B, P.N, P.K, ldb, strideB, P.batch))
+  if (!make_map(&ma, A, P.M, P.K, lda, strideA, P.batch) || !(P.b_mn ? make_map(&mb, B, P.K, P.N, ldb, strideB, P.batch, BK) : make_map(&mb, B, P.N, P.K, ldb, strideB, P.batch)))
     return cudaErrorInvalidValue;
   mc = ma;
   mct = ma;  // placeholders when an output is absent (never dereferenced by the kernel then)
@@ -650,11 +683,9 @@ cudaError_t launch_ns_gemm(const void* A, int64_t lda, int64_t strideA, const vo
 }
 
 cudaError_t launch_ns_prepare(const void* const* srcs, int src_dt, int R, int C, int batch, const float* sumsq, float eps,
-                              void* same, int64_t ld_same, int64_t stride_same, void* trans, int64_t ld_trans,
-                              int64_t stride_trans, uint64_t seed, cudaStream_t stream) {
+                              void* dst, int64_t ld, int64_t stride, int trans, uint64_t seed, cudaStream_t stream) {
   dim3 grid((C + 63) / 64, (R + 63) / 64, batch), block(256);
-  ns_prepare_kernel<<<grid, block, 0, stream>>>(srcs, src_dt, R, C, sumsq, eps, (__nv_bfloat16*)same, ld_same,
-                                                stride_same, (__nv_bfloat16*)trans, ld_trans, stride_trans, seed);
+  ns_prepare_kernel<<<grid, block, 0, stream>>>(srcs, src_dt, R, C, sumsq, eps, (__nv_bfloat16*)dst, ld, stride, trans, seed);
   return cudaGetLastError();
 }
 

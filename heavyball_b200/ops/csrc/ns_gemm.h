@@ -8,11 +8,13 @@ namespace hb {
 
 enum GemmMode : int { kModeGram = 0, kModePoly = 1, kModeApply = 2 };
 
-// D[M, N] = A[M, K] * B[N, K]^T per batch entry; all leading dimensions and strides in elements.
+// D[M, N] = A[M, K] * B[N, K]^T (b_mn: B is [K, N], N contiguous) per batch entry; all leading dimensions and strides
+// in elements.
 struct GemmParams {
   int M, N, K, batch;
   int mode;
   int symmetric;            // compute tiles with tile_n >= tile_m only and mirror them through CT
+  int b_mn;                 // B is stored [K, N]: its tiles are read through MN-major descriptors
   int same_operand;         // A and B are the same matrix (set by the launcher): diagonal tiles load it once
   __nv_bfloat16* C;         // bf16 output [M, N] (may be null)
   int64_t ldc, strideC;
@@ -35,7 +37,6 @@ void set_ns_gemm_tile_override(int tile);
 cudaError_t launch_ns_gemm(const void* A, int64_t lda, int64_t strideA, const void* B, int64_t ldb, int64_t strideB,
                            const GemmParams& P, cudaStream_t stream);
 cudaError_t launch_ns_prepare(const void* const* srcs, int src_dt, int R, int C, int batch, const float* sumsq, float eps,
-                              void* same, int64_t ld_same, int64_t stride_same, void* trans, int64_t ld_trans,
-                              int64_t stride_trans, uint64_t seed, cudaStream_t stream);
+                              void* dst, int64_t ld, int64_t stride, int trans, uint64_t seed, cudaStream_t stream);
 
 }  // namespace hb

@@ -101,6 +101,17 @@ __device__ inline uint64_t make_smem_desc(uint32_t smem_addr) {
   d |= (uint64_t)2 << 61;                       // SWIZZLE_128B
   return d;
 }
+// MN-major operand tile, 128-byte swizzle: the rows of K are 128 B (64 elements of M / N) long, 8 rows of K form a 1 KiB
+// group (stride byte offset), the next 64 elements of M / N follow `lead_bytes` further (leading byte offset).
+__device__ inline uint64_t make_smem_desc_mn(uint32_t smem_addr, uint32_t lead_bytes) {
+  uint64_t d = 0;
+  d |= (uint64_t)((smem_addr & 0x3FFFF) >> 4);
+  d |= (uint64_t)(lead_bytes >> 4) << 16;
+  d |= (uint64_t)(1024 >> 4) << 32;
+  d |= (uint64_t)1 << 46;
+  d |= (uint64_t)2 << 61;
+  return d;
+}
 __device__ inline void tma_store_3d(const CUtensorMap* map, const void* src, int c0, int c1, int c2) {
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];"
                ::"l"(map), "r"(smem_u32(src)), "r"(c0), "r"(c1), "r"(c2)
