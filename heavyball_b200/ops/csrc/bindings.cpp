@@ -40,12 +40,12 @@ struct Table {
   const int* prefix;
   int total_chunks;
   int n;
+  int chunk;
 };
 
 // Builds the per-tensor table and uploads it with one async copy on the current stream.
-Table upload(std::vector<hb::TensorMeta>& metas, const at::Device& dev) {
+Table upload(std::vector<hb::TensorMeta>& metas, const at::Device& dev, int chunk = hb::chain_chunk_elems()) {
   const int n = (int)metas.size();
-  const int chunk = hb::chain_chunk_elems();
   std::vector<int> prefix(n + 1, 0);
   for (int i = 0; i < n; ++i) prefix[i + 1] = prefix[i] + (int)((metas[i].numel + chunk - 1) / chunk);
   const size_t meta_bytes = sizeof(hb::TensorMeta) * n, prefix_bytes = sizeof(int) * (n + 1);
@@ -60,6 +60,7 @@ Table upload(std::vector<hb::TensorMeta>& metas, const at::Device& dev) {
   t.prefix = reinterpret_cast<const int*>((uint8_t*)t.device_blob.data_ptr() + meta_bytes);
   t.total_chunks = prefix[n];
   t.n = n;
+  t.chunk = chunk;
   return t;
 }
 
@@ -137,11 +138,9 @@ void fused_chain(const TList& p, const TList& pe, const TList& g, const TList& u
     m.vec_ok = ok ? 1 : 0;
     m.pad = 0;
   }
-  Table t = upload(metas, ref.device());
   hb::ChainParams P{};
   auto geti = [&](const char* k) { return cfg.contains(k) ? cfg[k].cast<int>() : 0; };
   auto getf = [&](const char* k) { return cfg.contains(k) ? cfg[k].cast<float>() : 0.f; };
-  P.n_tensors = t.n;
   P.algo = geti("algo"); P.out_mode = geti("out_mode"); P.n_state = geti("n_state");
   P.dt_p = geti("dt_p"); P.dt_g = geti("dt_g"); P.dt_u = geti("dt_u"); P.dt_s = geti("dt_s");
   P.u_is_input = geti("u_is_input"); P.mars = geti("mars"); P.cautious_wd = geti("cautious_wd");
@@ -169,8 +168,14 @@ void fused_chain(const TList& p, const TList& pe, const TList& g, const TList& u
   }
   P.g_mc_delta = cfg.contains("g_mc_delta") ? cfg["g_mc_delta"].cast<int64_t>() : 0;
   P.p_mc_delta = cfg.contains("p_mc_delta") ? cfg["p_mc_delta"].cast<int64_t>() : 0;
-  check(hb::launch_fused_chain(t.metas, t.prefix, t.total_chunks, P, geti("count_caution") != 0,
-                               at::cuda::getCurrentCUDAStream()), "fused_chain launch");
+  const bool count = geti("count_caution") != 0;
+  int64_t elems = 0;
+  for (const hb::TensorMeta& m : metas) elems += m.numel;
+  Table t = upload(metas, ref.device(), hb::chain_chunk_elems_for(P, count, elems));
+  P.n_tensors = t.n;
+  P.chunk = t.chunk;
+  check(hb::launch_fused_chain(t.metas, t.prefix, t.total_chunks, P, count, at::cuda::getCurrentCUDAStream()),
+        "fused_chain launch");
 }
 
 // out[i] = sum(x_i^2) in fp32.

@@ -18,6 +18,21 @@ __host__ __device__ inline bool is_ecc(int d) { return d >= kBF16E8 && d <= kF16
 __host__ __device__ inline bool is_bf16_like(int d) { return d == kBF16 || d == kBF16E8 || d == kBF16E16; }
 __host__ __device__ inline bool ecc_wide(int d) { return d == kBF16E16 || d == kF16E16; }
 
+// Index of the range that holds position `b`: the last entry of the ascending table `first` (n entries, first[0] == 0) that is
+// <= b.  A warp tests 32 entries at a time (one load for up to 32 ranges, two up to 1024) where a binary search is a chain of
+// five to ten dependent loads, paid by every block before its first data load.  Executed by whole warps.
+__device__ inline int find_range(const int* __restrict__ first, int n, int b) {
+  int lo = 0, len = n;
+  while (len > 1) {
+    const int step = (len + 31) >> 5, at = lo + (int)(threadIdx.x & 31) * step;
+    const unsigned below = __ballot_sync(0xFFFFFFFFu, at < lo + len && first[at] <= b);  // lane 0 always counts
+    const int k = 31 - __clz(below);
+    len = min(step, len - k * step);
+    lo += k * step;
+  }
+  return lo;
+}
+
 // ---------------------------------------------------------------------------------------------
 // Philox-4x32-10.  Streams are addressed by (seed, tensor index, element index / 4, draw id), never
 // by launch geometry, so results do not depend on grid shape or on which rank runs the update.

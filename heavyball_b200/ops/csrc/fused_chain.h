@@ -77,6 +77,7 @@ struct ChainParams {
   float b1, b2, b3, alpha;  // already debiased / scheduled on the host
   float mars_a;
   uint64_t seed;
+  int chunk;  // elements per block the prefix table was built with (0: chain_chunk_elems())
   // Peer-memory data parallelism (n_src / n_dst = 0 turns it off).  Gradient = g_scale * sum over sources
   // of the same element in every source's gradient slab; parameters (and their ECC residuals) are
   // written to every destination.  Deltas are byte offsets from this rank's address to the peer's.
@@ -93,6 +94,8 @@ struct ChainParams {
 };
 
 int chain_chunk_elems();
+// elements per block that a fused-chain launch over `total_elems` elements wants its prefix table built with
+int chain_chunk_elems_for(const ChainParams& P, bool count_caution, int64_t total_elems);
 cudaError_t launch_fused_chain(const TensorMeta* metas, const int* chunk_prefix, int total_chunks, const ChainParams& P,
                                bool count_caution, cudaStream_t stream);
 cudaError_t launch_sumsq(const TensorMeta* metas, const int* chunk_prefix, int total_chunks, int n_tensors, int dt,

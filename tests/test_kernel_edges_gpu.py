@@ -4,13 +4,41 @@ one launch.  Oracles are fp64 restatements or the package's PyTorch definitions.
 import pytest
 import torch
 
-from heavyball_b200 import ops, utils
+import heavyball_b200 as hb
+from heavyball_b200 import lowering, ops, utils
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
 
 
 # ---------------------------------------------------------------------------------------- fused chain
+
+
+@pytest.mark.parametrize("kw", [{}, {"ecc": "bf16+8", "mars": True, "caution": True}, {"ecc": "bf16+8"}, {"caution": True}], ids=str)
+@pytest.mark.parametrize("sizes", [(1,), (2047, 2048, 2049), (8191, 8193, 3, 16384), tuple(range(1, 41)), (10_000_000, 5)], ids=len)
+def test_fused_chain_at_chunk_edges(sizes, kw):
+    """Sizes around both chunk sizes, more tensors than a warp tests at once, and a launch large enough for the large chunk.
+    fp32: a handful of roundings per step (1e-6 of the value); error-corrected state keeps 16 + 8 bits (2^-15 of the value)
+    and moves a weight by lr = 1e-2 per step."""
+    results = []
+    for lowered in (True, False):
+        torch.manual_seed(0)
+        gen = torch.Generator(DEV).manual_seed(1)
+        params = [torch.nn.Parameter(torch.randn(n, device=DEV, generator=gen)) for n in sizes]
+        opt = hb.AdamW(params, lr=1e-2, weight_decay=0.1, **kw)
+        old, lowering.enabled = lowering.enabled, lowered
+        try:
+            for _ in range(3):
+                for p in params:
+                    p.grad = torch.randn(p.shape, device=DEV, generator=gen)
+                opt.step()
+        finally:
+            lowering.enabled = old
+        results.append([p.detach() for p in params])
+    for a, b in zip(*results):
+        # a value next to zero may round to the other side of caution's sign test when its state is stored in fewer bits
+        close = torch.isclose(a, b, rtol=1e-5, atol=2e-6 if not kw.get("ecc") else 2e-4)
+        assert close.float().mean().item() > (0.999 if kw.get("caution") and a.numel() > 1000 else 1 - 1e-9), (a - b).abs().max()
 
 
 def test_ecc_codec_over_all_exponents():
