@@ -649,39 +649,28 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
     scale_mode = "scale"
     final = list(scratch)
     buckets = [(shape, idx, U) for shape, idx, U, _ in layout if len(shape) >= 2]
-    # shape buckets are independent chains of small launches: run them on side streams so they share the GPU
-    main = torch.cuda.current_stream(dev)
-    streams = prog.workspace.get("streams")
-    if streams is None:
-        streams = prog.workspace["streams"] = [torch.cuda.Stream(device=dev) for _ in range(4)]
-    ready = torch.cuda.Event()
-    ready.record(main)
-    used = []
-    for k, (shape, idx, U) in enumerate(buckets):
+    pending = []  # (bytes of work copies, group); groups go through the iteration together, as many as the workspace holds
+    for shape, idx, U in buckets:
         R, Cc = shape[0], U[0].numel() // shape[0]
         U3 = U.view(len(idx), R, Cc)
         if not ops.ns_supported(R, Cc):
             for b in range(len(idx)):
                 utils.inplace_orthogonal_(U3[b], out=U3[b], scale_mode=scale_mode)
             continue
-        sel_idx = prog.workspace.get(("idx", R, Cc, tuple(idx)))
-        if sel_idx is None:
-            sel_idx = prog.workspace[("idx", R, Cc, tuple(idx))] = torch.tensor(idx, dtype=torch.long, device=dev)
-        side = streams[k % len(streams)] if len(buckets) > 1 else main
-        if side is not main:
-            side.wait_event(ready)
-            used.append(side)
-        chunk = max(1, _NS_WORKSPACE_BYTES // (R * Cc * 8))  # bf16 work copies per matrix: two of it, two of its Gram matrix
-        with torch.cuda.stream(side), _stage(f"ns/{R}x{Cc}"):
-            norms = sq.index_select(0, sel_idx)
-            for c0 in range(0, len(idx), chunk):
-                c1 = min(len(idx), c0 + chunk)
-                ops.newton_schulz_batched(
-                    list(U3[c0:c1].unbind(0)), utils.NS5_COEFFS, out=U3[c0:c1], out_scale=max(1, R / Cc) ** 0.5,
-                    seed=_seed(opt, group, 2 + len(final) + R + c0), sumsq=norms[c0:c1],
-                )
-    for side in used:
-        main.wait_stream(side)
+        per_matrix = R * Cc * 8  # bytes of bf16 work copies: two of the matrix, two of its Gram matrix (at most as large)
+        chunk = max(1, _NS_WORKSPACE_BYTES // per_matrix)
+        for c0 in range(0, len(idx), chunk):
+            part = idx[c0 : c0 + chunk]
+            pending.append((per_matrix * len(part), (U3[c0 : c0 + len(part)].unbind(0), part, U3[c0 : c0 + len(part)],
+                                                     max(1, R / Cc) ** 0.5, _seed(opt, group, 2 + len(final) + R + c0))))  # fmt: skip
+    with _stage("newton_schulz"):
+        while pending:
+            room, wave = _NS_WORKSPACE_BYTES, []
+            while pending and (not wave or pending[0][0] <= room):
+                size, entry = pending.pop(0)
+                room -= size
+                wave.append(entry)
+            ops.newton_schulz_groups(wave, sq, utils.NS5_COEFFS)
     with _stage("update"):
         _orthogonal_update(opt, group, caution, params_v, grads_v, final, pe, base, epilogue, peer_in, peer_out)
     return True

@@ -190,10 +190,6 @@ def absmax(xs: Sequence[torch.Tensor]) -> torch.Tensor:
 # ---------------------------------------------------------------------------------------- Newton–Schulz
 
 
-def _round_up(x, m):
-    return (x + m - 1) // m * m
-
-
 _status_cache = {}
 
 
@@ -223,34 +219,31 @@ def newton_schulz_batched(mats: Sequence[torch.Tensor], coeffs, out: Optional[to
     """Orthogonalises a list of same-shape ``(R, C)`` fp32 / bf16 matrices; returns fp32 ``(B, R, C)``
     holding ``out_scale * polar_factor``.  ``coeffs`` is a sequence of ``(a, b, c)`` per step.  ``sumsq``
     (fp32, one squared Frobenius norm per matrix) skips the reduction pass when the caller already has it."""
-    ext = load()
-    B = len(mats)
     R, C = mats[0].shape
-    dev = mats[0].device
-    m, n = (R, C) if R <= C else (C, R)
-    ldx, lds = _round_up(n, 8), _round_up(m, 8)
-    bf = dict(dtype=torch.bfloat16, device=dev)
-    X = [torch.empty(B, m, ldx, **bf) for _ in range(2)]
-    S = torch.empty(B, m, lds, **bf)
-    Y = torch.empty(B, m, lds, **bf)
     if out is None:
-        out = torch.empty(B, R, C, dtype=torch.float32, device=dev)
+        out = torch.empty(len(mats), R, C, dtype=torch.float32, device=mats[0].device)
     if seed is None:
         seed = int(torch.randint(0, 2**62, (1,)).item())
     srcs = [t.contiguous() for t in mats]
     if sumsq is None:
-        norms = ext.sumsq(srcs, dtype_code(mats[0]))
+        norms = load().sumsq(srcs, dtype_code(mats[0]))
         launch_counter.count += 1
     else:
         norms = sumsq.contiguous()
-    # a tall matrix is worked on transposed so that the Gram matrix is the small one
-    ext.ns_prepare(srcs, dtype_code(mats[0]), R, C, norms, eps, X[0], ldx, R > C, seed)
-    status = _status(dev)
-    launch_counter.count += 1 + 3 * len(coeffs)
-    # one call issues the three launches of every step (Gram, polynomial, apply; the last apply writes `out`)
-    ext.ns_chain(X, S, Y, out, m, n, ldx, lds, R, C, [[float(v) for v in abc] for abc in coeffs], float(out_scale),
-                 status)  # fmt: skip
+    newton_schulz_groups([(srcs, range(len(srcs)), out, out_scale, seed)], norms, coeffs, eps)
     return out
+
+
+def newton_schulz_groups(groups, sumsq: torch.Tensor, coeffs, eps: float = 1e-7) -> None:
+    """Orthogonalises several shape buckets in one chain of launches (each covers all buckets).  ``groups``: per bucket
+    ``(matrices, positions of their squared norms in sumsq, out, out_scale, seed)`` with contiguous ``(R, C)`` matrices of
+    one shape and, over all buckets, one dtype; ``out``: contiguous fp32 ``(B, R, C)`` (the matrices themselves may live
+    there)."""
+    mats, at, outs, scales, seeds = zip(*groups)
+    launch_counter.count += load().ns_orthogonalize(
+        [list(m) for m in mats], dtype_code(mats[0][0]), sumsq, [list(i) for i in at], list(outs), [float(s) for s in scales],
+        list(seeds), [[float(v) for v in abc] for abc in coeffs], eps, _status(sumsq.device),
+    )  # fmt: skip
 
 
 def newton_schulz(G: torch.Tensor, coeffs, out_scale: float = 1.0) -> Optional[torch.Tensor]:

@@ -4,6 +4,7 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <algorithm>
 #include <optional>
 #include <vector>
 
@@ -223,22 +224,6 @@ at::Tensor segmented_reduce(const std::vector<at::Tensor>& xs, const std::vector
   return out;
 }
 
-// Normalise + stochastically round a batch of same-shape matrices into the bf16 iterate: [batch, R, ld] as they are, or
-// [batch, C, ld] transposed.
-void ns_prepare(const std::vector<at::Tensor>& srcs, int src_dt, int64_t R, int64_t C, const at::Tensor& sumsq_t, double eps,
-                at::Tensor dst, int64_t ld, bool trans, uint64_t seed) {
-  c10::cuda::CUDAGuard guard(dst.device());
-  std::vector<const void*> ptrs(srcs.size());
-  for (size_t i = 0; i < srcs.size(); ++i) ptrs[i] = srcs[i].data_ptr();
-  at::Tensor dev = at::empty({(int64_t)(ptrs.size() * sizeof(void*))}, dst.options().dtype(at::kByte));
-  auto stream = at::cuda::getCurrentCUDAStream();
-  check(cudaMemcpyAsync(dev.data_ptr(), ptrs.data(), ptrs.size() * sizeof(void*), cudaMemcpyHostToDevice, stream),
-        "pointer upload");
-  check(hb::launch_ns_prepare((const void* const*)dev.data_ptr(), src_dt, (int)R, (int)C, (int)srcs.size(),
-                              sumsq_t.data_ptr<float>(), (float)eps, dst.data_ptr(), ld, (trans ? C : R) * ld, trans ? 1 : 0,
-                              seed, stream), "ns_prepare launch");
-}
-
 // D = A * B^T (bf16, K-major operands, batched) with the fused epilogues described in ns_gemm.h.
 void ns_gemm(const at::Tensor& A, int64_t lda, int64_t strideA, const at::Tensor& B, int64_t ldb, int64_t strideB,
              int64_t M, int64_t N, int64_t K, int64_t batch, int mode, bool symmetric, const OptT& C, int64_t ldc,
@@ -255,46 +240,109 @@ void ns_gemm(const at::Tensor& A, int64_t lda, int64_t strideA, const at::Tensor
   P.S = S.has_value() ? (const __nv_bfloat16*)S->data_ptr() : nullptr; P.lds = lds; P.strideS = strideS;
   P.ca = (float)ca; P.cb = (float)cb; P.cc = (float)cc;
   P.status = status.data_ptr<int>();
-  check(hb::launch_ns_gemm(A.data_ptr(), lda, strideA, B.data_ptr(), ldb, strideB, P, at::cuda::getCurrentCUDAStream()),
-        "ns_gemm launch");
+  const hb::NsProduct X{A.data_ptr(), lda, strideA, B.data_ptr(), ldb, strideB, P};
+  check(hb::launch_ns_products(&X, 1, nullptr, at::cuda::getCurrentCUDAStream()), "ns_gemm launch");
 }
 
-// The whole Newton-Schulz iteration of one shape bucket in one call: per step Gram, polynomial and apply launches (the
-// last apply writes fp32 into `out`, in the caller's orientation).  x: the two ping-pong buffers of the iterate
-// [batch, m, ldx] (bf16), the first prepared by ns_prepare; s, y: [batch, m, lds] (bf16).
-void ns_chain(const std::vector<at::Tensor>& x, const at::Tensor& s, const at::Tensor& y, at::Tensor& out, int64_t m, int64_t n,
-              int64_t ldx, int64_t lds, int64_t R, int64_t C, const std::vector<std::vector<double>>& coeffs, double out_scale,
-              const at::Tensor& status) {
-  TORCH_CHECK(x.size() == 2, "ns_chain: two ping-pong buffers");
-  c10::cuda::CUDAGuard guard(s.device());
+// The whole Newton-Schulz iteration of several shape buckets: one launch normalises and rounds every matrix, then each step is
+// a Gram, a polynomial and an apply product of all buckets together (the last apply writes fp32 into `outs`, in the caller's
+// orientation).  mats[g]: the matrices of bucket g, contiguous, one shape and dtype per bucket (one dtype for all);
+// sumsq / sumsq_at[g][j]: fp32 squared Frobenius norms and where matrix j of bucket g has its own; seeds[g]: rounding noise.
+// Returns the number of kernel launches.
+int64_t ns_orthogonalize(const std::vector<std::vector<at::Tensor>>& mats, int src_dt, const at::Tensor& sumsq,
+                         const std::vector<std::vector<int64_t>>& sumsq_at, const std::vector<at::Tensor>& outs,
+                         const std::vector<double>& out_scales, const std::vector<uint64_t>& seeds,
+                         const std::vector<std::vector<double>>& coeffs, double eps, const at::Tensor& status) {
+  const size_t n = mats.size();
+  TORCH_CHECK(n > 0 && sumsq_at.size() == n && outs.size() == n && out_scales.size() == n && seeds.size() == n,
+              "ns_orthogonalize: one entry per bucket");
+  TORCH_CHECK(sumsq.is_cuda() && sumsq.scalar_type() == at::kFloat && sumsq.is_contiguous(), "ns_orthogonalize: fp32 norms");
+  const at::Device dev = sumsq.device();
+  c10::cuda::CUDAGuard guard(dev);
   auto stream = at::cuda::getCurrentCUDAStream();
-  int cur = 0;
-  for (size_t step = 0; step < coeffs.size(); ++step) {
-    TORCH_CHECK(coeffs[step].size() == 3, "ns_chain: (a, b, c) per step");
-    auto* X = (__nv_bfloat16*)x[cur].data_ptr();
-    auto* S = (__nv_bfloat16*)s.data_ptr();
-    auto* Y = (__nv_bfloat16*)y.data_ptr();
-    hb::GemmParams G{};  // S = X X^T
-    G.batch = (int)s.size(0); G.status = status.data_ptr<int>(); G.f_scale = 1.f;
-    G.M = G.N = (int)m;
-    hb::GemmParams A = G, Q = G;
-    G.mode = hb::kModeGram; G.K = (int)n; G.symmetric = 1;
-    G.C = G.CT = S; G.ldc = G.ldct = lds; G.strideC = G.strideCT = m * lds;
-    check(hb::launch_ns_gemm(X, ldx, m * ldx, X, ldx, m * ldx, G, stream), "ns_chain gram launch");
-    Q.mode = hb::kModePoly; Q.K = (int)m; Q.symmetric = 1;  // Y = c S S + b S + a I
-    Q.C = Q.CT = Y; Q.ldc = Q.ldct = lds; Q.strideC = Q.strideCT = m * lds;
-    Q.S = S; Q.lds = lds; Q.strideS = m * lds;
-    Q.ca = (float)coeffs[step][0]; Q.cb = (float)coeffs[step][1]; Q.cc = (float)coeffs[step][2];
-    check(hb::launch_ns_gemm(S, lds, m * lds, S, lds, m * lds, Q, stream), "ns_chain poly launch");
-    A.mode = hb::kModeApply; A.N = (int)n; A.K = (int)m; A.b_mn = 1;  // X' = Y X
-    if (step + 1 < coeffs.size()) {
-      A.C = (__nv_bfloat16*)x[1 - cur].data_ptr(); A.ldc = ldx; A.strideC = m * ldx;
-    } else {
-      A.F = out.data_ptr<float>(); A.ldf = C; A.strideF = R * C; A.f_transposed = R > C ? 1 : 0; A.f_scale = (float)out_scale;
-    }
-    check(hb::launch_ns_gemm(Y, lds, m * lds, X, ldx, m * ldx, A, stream), "ns_chain apply launch");
-    cur = 1 - cur;
+  struct Bucket { int64_t batch, R, C, m, n, ldx, lds; __nv_bfloat16 *x[2], *s, *y; };
+  std::vector<Bucket> buckets(n);
+  auto up8 = [](int64_t v) { return (v + 7) / 8 * 8; };
+  auto room = [](int64_t elems) { return (elems + 127) / 128 * 128; };  // buffers start on 256-byte boundaries
+  int64_t elems = 0;
+  size_t total_mats = 0;
+  for (size_t g = 0; g < n; ++g) {
+    Bucket& b = buckets[g];
+    TORCH_CHECK(!mats[g].empty() && mats[g][0].dim() == 2 && sumsq_at[g].size() == mats[g].size(), "ns_orthogonalize: empty bucket");
+    b.batch = (int64_t)mats[g].size(); b.R = mats[g][0].size(0); b.C = mats[g][0].size(1);
+    b.m = std::min(b.R, b.C); b.n = std::max(b.R, b.C); b.ldx = up8(b.n); b.lds = up8(b.m);
+    const at::Tensor& o = outs[g];
+    TORCH_CHECK(o.device() == dev && o.scalar_type() == at::kFloat && o.is_contiguous() && o.numel() == b.batch * b.R * b.C,
+                "ns_orthogonalize: out must be contiguous fp32 [batch, R, C]");
+    elems += 2 * room(b.batch * b.m * b.ldx) + 2 * room(b.batch * b.m * b.lds);
+    total_mats += mats[g].size();
   }
+  at::Tensor slab = at::empty({elems}, sumsq.options().dtype(at::kBFloat16));
+  auto* cursor = (__nv_bfloat16*)slab.data_ptr();
+  std::vector<hb::NsSource> src;
+  std::vector<int> first(1, 0);
+  src.reserve(total_mats);
+  for (size_t g = 0; g < n; ++g) {
+    Bucket& b = buckets[g];
+    for (auto** p : {&b.x[0], &b.x[1]}) { *p = cursor; cursor += room(b.batch * b.m * b.ldx); }
+    for (auto** p : {&b.s, &b.y}) { *p = cursor; cursor += room(b.batch * b.m * b.lds); }
+    for (int64_t j = 0; j < b.batch; ++j) {
+      const at::Tensor& t = mats[g][j];
+      TORCH_CHECK(t.device() == dev && t.is_contiguous() && t.scalar_type() == mats[0][0].scalar_type() && t.dim() == 2 &&
+                      t.size(0) == b.R && t.size(1) == b.C, "ns_orthogonalize: contiguous matrices of one shape per bucket");
+      TORCH_CHECK(sumsq_at[g][j] >= 0 && sumsq_at[g][j] < sumsq.numel(), "ns_orthogonalize: norm index out of range");
+      src.push_back({t.data_ptr(), sumsq.data_ptr<float>() + sumsq_at[g][j], b.x[0] + j * b.m * b.ldx, seeds[g], b.ldx, (int)b.R,
+                     (int)b.C, b.R > b.C ? 1 : 0, (int)j});
+      first.push_back(first.back() + (int)(((b.R + 63) / 64) * ((b.C + 63) / 64)));
+    }
+  }
+  const size_t src_bytes = src.size() * sizeof(hb::NsSource), first_bytes = first.size() * sizeof(int);
+  std::vector<uint8_t> host(src_bytes + first_bytes);
+  memcpy(host.data(), src.data(), src_bytes);
+  memcpy(host.data() + src_bytes, first.data(), first_bytes);
+  at::Tensor table = at::empty({(int64_t)host.size()}, sumsq.options().dtype(at::kByte));
+  check(cudaMemcpyAsync(table.data_ptr(), host.data(), host.size(), cudaMemcpyHostToDevice, stream), "matrix table upload");
+  check(hb::launch_ns_prepare((const hb::NsSource*)table.data_ptr(), (const int*)((uint8_t*)table.data_ptr() + src_bytes),
+                              (int)src.size(), first.back(), src_dt, (float)eps, stream), "ns_prepare launch");
+  int launches = 1;
+  std::vector<hb::NsProduct> stage(n);
+  int cur = 0;
+  for (size_t step = 0; step < coeffs.size(); ++step, cur = 1 - cur) {
+    TORCH_CHECK(coeffs[step].size() == 3, "ns_orthogonalize: (a, b, c) per step");
+    for (int mode : {(int)hb::kModeGram, (int)hb::kModePoly, (int)hb::kModeApply}) {
+      for (size_t g = 0; g < n; ++g) {
+        const Bucket& b = buckets[g];
+        hb::NsProduct& X = stage[g];
+        hb::GemmParams P{};
+        P.mode = mode; P.batch = (int)b.batch; P.status = status.data_ptr<int>(); P.M = (int)b.m; P.f_scale = 1.f;
+        if (mode == hb::kModeApply) {  // X' = Y X
+          X = {b.y, b.lds, b.m * b.lds, b.x[cur], b.ldx, b.m * b.ldx, {}};
+          P.N = (int)b.n; P.K = (int)b.m; P.b_mn = 1;
+          if (step + 1 < coeffs.size()) {
+            P.C = b.x[1 - cur]; P.ldc = b.ldx; P.strideC = b.m * b.ldx;
+          } else {
+            P.F = outs[g].data_ptr<float>(); P.ldf = b.C; P.strideF = b.R * b.C; P.f_transposed = b.R > b.C ? 1 : 0;
+            P.f_scale = (float)out_scales[g];
+          }
+        } else {  // S = X X^T,  Y = c S S + b S + a I
+          const bool poly = mode == hb::kModePoly;
+          if (poly)
+            X = {b.s, b.lds, b.m * b.lds, b.s, b.lds, b.m * b.lds, {}};
+          else
+            X = {b.x[cur], b.ldx, b.m * b.ldx, b.x[cur], b.ldx, b.m * b.ldx, {}};
+          P.N = (int)b.m; P.K = (int)(poly ? b.m : b.n); P.symmetric = 1;
+          P.C = P.CT = poly ? b.y : b.s; P.ldc = P.ldct = b.lds; P.strideC = P.strideCT = b.m * b.lds;
+          if (poly) {
+            P.S = b.s; P.lds = b.lds; P.strideS = b.m * b.lds;
+            P.ca = (float)coeffs[step][0]; P.cb = (float)coeffs[step][1]; P.cc = (float)coeffs[step][2];
+          }
+        }
+        X.P = P;
+      }
+      check(hb::launch_ns_products(stage.data(), (int)n, &launches, stream), "ns_orthogonalize launch");
+    }
+  }
+  return launches;
 }
 
 // Store `epoch` into slot[rank] of every peer's flag array (after a system-scope fence).
@@ -643,9 +691,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("fused_chain", &fused_chain);
   m.def("sumsq", &sumsq);
   m.def("segmented_reduce", &segmented_reduce);
-  m.def("ns_prepare", &ns_prepare);
   m.def("ns_gemm", &ns_gemm);
-  m.def("ns_chain", &ns_chain);
+  m.def("ns_orthogonalize", &ns_orthogonalize);
   m.def("set_ns_gemm_tile", &hb::set_ns_gemm_tile_override);
   m.def("set_tf32_gemm_tile", &hb::set_tf32_gemm_tile_override);
   m.def("chol_inv_leaf", &chol_inv_leaf);

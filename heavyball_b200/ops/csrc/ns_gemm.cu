@@ -8,8 +8,8 @@
 // Gram and polynomial are "TN" products D[M,N] = A[M,K] * B[N,K]^T with both operands K-major; the apply product takes
 // X as it lies in memory ([K, N], N contiguous) through an MN-major B descriptor, so the iterate exists once and no
 // transposed copy of it is ever written (half of the bytes of every apply epilogue and of the prologue; GPT-2-small's
-// 48 matrices: 2634 -> 2513 us, a Llama-3-8B layer: 19.97 -> 18.71 ms).
-// One kernel serves all three; only the B box, its descriptor and the epilogue differ.
+// 48 matrices: 2634 -> 2513 us, a Llama-3-8B layer: 19.97 -> 18.71 ms).  The three differ only in the B box, its descriptor
+// and the epilogue.  Two kernels share them: 128 x 128 tiles for small matrices, 256 x 256 tiles on CTA pairs for large ones.
 //
 // Kernel structure (one 128x128 output tile per CTA, 192 threads, two CTAs resident per SM so one
 // CTA's epilogue overlaps the other's main loop):
@@ -30,8 +30,10 @@
 #include "common.cuh"
 #include "ns_gemm.h"
 
+#include <algorithm>
 #include <mutex>
 #include <unordered_map>
+#include <vector>
 #include "tc_common.cuh"
 
 namespace hb {
@@ -53,10 +55,40 @@ constexpr int kMnBoxBytes = 64 * BK * 2;
 constexpr uint32_t kMnStep = (16 * 128) >> 4;
 constexpr uint32_t kInstrBMn = 1u << 16;
 
+// ------------------------------------------------------------------------------------------ grouped launches
+// One launch covers the same stage of every shape bucket of a step (up to kMaxGroups products of different sizes): the tiles
+// of all of them share the machine, and a step is 15 launches instead of 15 per bucket (five small odd matrices in four shapes:
+// 654 -> 276 us; GPT-2-small's 48 matrices in four shapes: 2513 -> 1920 us together with the pair kernel below).
+constexpr int kMaxGroups = 8;
+struct GemmGroup {
+  CUtensorMap a, b, c, ct, s;  // s: the polynomial's epilogue operand (pair kernel); absent operands repeat `a`
+  GemmParams P;
+  int tiles_m, tiles_n, per_batch;
+  int f_bulk;                  // F leaves through bulk stores, described by `c` (pair kernel)
+};
+struct GemmGroups {
+  int n, total;
+  int first[kMaxGroups];       // index of each group's first tile within the launch
+  int* status;
+  GemmGroup g[kMaxGroups];
+};
+
+struct TileAt : PairTile {
+  int group;
+};
+__device__ __forceinline__ TileAt tile_at(const GemmGroups& L, int idx) {
+  TileAt t;
+  t.group = 0;
+#pragma unroll
+  for (int i = 1; i < kMaxGroups; ++i)
+    if (i < L.n && idx >= L.first[i]) t.group = i;
+  const GemmGroup& G = L.g[t.group];
+  static_cast<PairTile&>(t) = pair_tile(idx - L.first[t.group], G.tiles_m, G.tiles_n, G.per_batch, G.P.symmetric);
+  return t;
+}
+
 // ------------------------------------------------------------------------------------------ kernel
-__global__ void __launch_bounds__(kGemmThreads, 2)
-ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_ct, const GemmParams P) {
+__global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_constant__ GemmGroups L) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kStages];
   __shared__ __align__(8) uint64_t empty_bar[kStages];
@@ -64,24 +96,13 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
-  // a previous CTA of this stream already gave up on a wait: do not pile more work on a broken pipeline
-  if (P.status != nullptr && *(volatile const int*)P.status != 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
 
-  // ---- tile coordinates
-  const int tiles_m = (P.M + BM - 1) / BM, tiles_n = (P.N + BN - 1) / BN;
-  int tm, tn;
-  if (P.symmetric) {
-    int idx = blockIdx.x;
-    tm = 0;
-    while (idx >= tiles_m - tm) { idx -= tiles_m - tm; ++tm; }
-    tn = tm + idx;
-  } else {
-    tm = blockIdx.x / tiles_n;
-    tn = blockIdx.x % tiles_n;
-  }
-  const int batch = blockIdx.y;
+  const TileAt tile = tile_at(L, blockIdx.x);
+  const GemmGroup& G = L.g[tile.group];
+  const GemmParams P = G.P;  // by value: through the reference every use would be a load (nothing survives the asm fences)
+  const int tm = tile.tm, tn = tile.tn, batch = tile.batch;
   const int num_kb = (P.K + BK - 1) / BK;
   const bool poly = P.mode == kModePoly;
   const bool same_ab = P.same_operand && tm == tn;  // A and B tiles coincide
@@ -99,13 +120,18 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) { tmem_alloc(&tmem_base_slot, kTmemCols); tmem_relinquish(); }
+  griddep_wait();
+  // a kernel of this stream already gave up on a wait: do not pile more work on a broken pipeline
+  const bool skip = __syncthreads_or(threadIdx.x == 0 && L.status != nullptr && *(volatile const int*)L.status != 0);
+  griddep_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
 
   int issued = 0;  // producer: ring fills whose loads were issued
-  if (warp == 0) {
+  if (skip) {
+  } else if (warp == 0) {
     if (lane == 0) {
       const int total = num_kb + (poly ? 1 : 0);
       for (int kb = 0; kb < total; ++kb) {
@@ -115,17 +141,17 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (kb < num_kb) {
           // diagonal tiles of a symmetric product multiply a row block with itself: one load feeds both operands
           mbar_expect_tx(&full_bar[s], same_ab ? kTileBytes : kStageBytes);
-          tma_load_3d(a_dst, &map_a, &full_bar[s], kb * BK, tm * BM, batch);
+          tma_load_3d(a_dst, &G.a, &full_bar[s], kb * BK, tm * BM, batch);
           if (P.b_mn) {  // [K, N] operand: two boxes of 64 columns x 64 rows of K
-            tma_load_3d(a_dst + kTileBytes, &map_b, &full_bar[s], tn * BN, kb * BK, batch);
-            tma_load_3d(a_dst + kTileBytes + kMnBoxBytes, &map_b, &full_bar[s], tn * BN + 64, kb * BK, batch);
+            tma_load_3d(a_dst + kTileBytes, &G.b, &full_bar[s], tn * BN, kb * BK, batch);
+            tma_load_3d(a_dst + kTileBytes + kMnBoxBytes, &G.b, &full_bar[s], tn * BN + 64, kb * BK, batch);
           } else if (!same_ab) {
-            tma_load_3d(a_dst + kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN, batch);
+            tma_load_3d(a_dst + kTileBytes, &G.b, &full_bar[s], kb * BK, tn * BN, batch);
           }
         } else {
           mbar_expect_tx(&full_bar[s], kStageBytes);  // S[tm-block, tn-block] for the polynomial epilogue, as two 64-column halves
-          tma_load_3d(a_dst, &map_a, &full_bar[s], tn * BN, tm * BM, batch);
-          tma_load_3d(a_dst + kTileBytes, &map_a, &full_bar[s], tn * BN + BK, tm * BM, batch);
+          tma_load_3d(a_dst, &G.a, &full_bar[s], tn * BN, tm * BM, batch);
+          tma_load_3d(a_dst + kTileBytes, &G.a, &full_bar[s], tn * BN + BK, tm * BM, batch);
         }
         issued = kb + 1;
       }
@@ -245,9 +271,9 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
           if (want_c && tn * BN + hh * BK < P.N)
-            tma_store_3d(&map_c, c_stage + hh * kTileBytes, tn * BN + hh * BK, tm * BM, batch);
+            tma_store_3d(&G.c, c_stage + hh * kTileBytes, tn * BN + hh * BK, tm * BM, batch);
           if (want_ct && tm * BM + hh * BK < P.M)
-            tma_store_3d(&map_ct, ct_stage + hh * kTileBytes, tm * BM + hh * BK, tn * BN, batch);
+            tma_store_3d(&G.ct, ct_stage + hh * kTileBytes, tm * BM + hh * BK, tn * BN, batch);
         }
         asm volatile("cp.async.bulk.commit_group;" ::: "memory");
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
@@ -264,241 +290,264 @@ ns_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   }
   __syncthreads();
-  if (threadIdx.x == 0 && abort_flag && P.status != nullptr) atomicExch(P.status, 1);
+  if (threadIdx.x == 0 && abort_flag && L.status != nullptr) atomicExch(L.status, 1);
   if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTmemCols); }
 }
 
-// ------------------------------------------------------------------------------------------ large-tile kernel
-// Same product, roles and barrier protocol with a 256x256 output tile per CTA (one CTA per SM).  A 128x128 tile reads
-// 32 KiB of operands per 2.1 MFLOP k-block: at the tensor-core rate that is more than the L2 can deliver to 148 SMs, and
-// large matrices (the 4096 x 14336 weights of an 8B model) stall at about 0.6 PFLOP/s.  A 256x256 tile reads 64 KiB per
-// 8.4 MFLOP, half the bytes per flop, without any multicast: the CTA simply keeps four 128x128 accumulators - all 512
-// columns of tensor memory - as two 128x256 instructions per 16 of K that share one B tile.  The price is that nothing is
-// left to overlap the epilogue with, so this variant is chosen only when K is long enough to hide it.
-//   ring stage : A rows 0..127 | A rows 128..255 | B rows 0..127 | B rows 128..255   (4 x 16 KiB, 3 stages = 192 KiB)
-//   epilogue   : per 128-row half: [S half, poly only] | C staging | C^T staging      (3 x 64 KiB, the idle ring)
-constexpr int BM2 = 256, BN2 = 256;
-constexpr int kStageBytes2 = 4 * kTileBytes;                    // 64 KiB
-constexpr int kSmemBytes2 = kStages * kStageBytes2 + 1024;
-constexpr uint32_t kTmemCols2 = 512;
-constexpr uint32_t kInstrDesc256 = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-
-__global__ void __launch_bounds__(kGemmThreads, 1)
-ns_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ CUtensorMap map_c, const __grid_constant__ CUtensorMap map_ct, const GemmParams P) {
+// ------------------------------------------------------------------------------------------ pair kernel
+// Same products with a 256x256 output tile per PAIR of CTAs (cta_group::2, a cluster of two on neighbouring SMs), one
+// persistent pair per two SMs.  Each CTA stages 128 rows of A and half of B (32 KiB per 64 of K, 5 stages) and holds 128 rows
+// of the accumulator, 256 of the 512 columns of tensor memory, so two accumulators fit and the epilogue of one tile runs
+// under the main loop of the next.
+//   warp 0      : TMA producer of its CTA; completion of both CTAs' loads is counted on the even CTA's barrier
+//   warp 1      : of the even CTA: issues 256x256x16 instructions for the pair; commits release a ring slot in both CTAs
+//   warps 2..9  : epilogue of 32 rows x 128 columns each, 64 columns at a time and independent of the other warps: tensor
+//                 memory -> registers -> swizzled staging (for the polynomial the S block lands there first, by TMA, and
+//                 every thread overwrites what it read) -> bulk tensor store; the transposed copy is made by ldmatrix.trans /
+//                 stmatrix from that staging.  A 768-long K leaves 6100 cycles per tile to hide this in.
+constexpr int kPairStages = 5;
+constexpr int kPairStageBytes = 2 * kTileBytes;                       // this CTA's 128 rows of A | its half of B
+constexpr int kWarpStage = 32 * 64 * 2;                               // 32 rows x 64 columns of bf16
+constexpr int kPairEpiWarps = 8;
+constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;
+constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + kPairEpiWarps * 2 * kWarpStage + 1024;  // C and C^T of a warp
+constexpr uint32_t kInstrDescPair = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPairTile >> 3) << 17) | ((uint32_t)(kPairTile >> 4) << 24);
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_gemm_pair_kernel(const __grid_constant__ GemmGroups L) {
   extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kStages];
-  __shared__ __align__(8) uint64_t empty_bar[kStages];
-  __shared__ __align__(8) uint64_t accum_bar;
-  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ __align__(8) uint64_t full_bar[kPairStages];   // used in the even CTA: both CTAs' loads of a stage have landed
+  __shared__ __align__(8) uint64_t empty_bar[kPairStages];  // in each CTA: the products that read the stage have finished
+  __shared__ __align__(8) uint64_t acc_full[2];             // in each CTA: accumulator finished
+  __shared__ __align__(8) uint64_t acc_empty[2];            // in the even CTA: all sixteen epilogue warps have read it
+  __shared__ __align__(8) uint64_t s_bar[kPairEpiWarps];
   __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_flag;
+  __shared__ int abort_flag, skip_flag;
 
-  if (P.status != nullptr && *(volatile const int*)P.status != 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-
-  const int tiles_m = (P.M + BM2 - 1) / BM2, tiles_n = (P.N + BN2 - 1) / BN2;
-  int tm, tn;
-  if (P.symmetric) {
-    int idx = blockIdx.x;
-    tm = 0;
-    while (idx >= tiles_m - tm) { idx -= tiles_m - tm; ++tm; }
-    tn = tm + idx;
-  } else {
-    tm = blockIdx.x / tiles_n;
-    tn = blockIdx.x % tiles_n;
-  }
-  const int batch = blockIdx.y;
-  const int num_kb = (P.K + BK - 1) / BK;
-  const bool poly = P.mode == kModePoly;
-  const bool same_ab = P.same_operand && tm == tn;
-  uint8_t* s_tile = tiles;                          // epilogue regions: the ring is idle by then
-  uint8_t* c_stage = tiles + kStageBytes2;
-  uint8_t* ct_stage = tiles + 2 * kStageBytes2;
+  const uint32_t rank = cluster_rank();
+  uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int total = L.total, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    mbar_init(&accum_bar, 1);
-    mbar_init(&s_bar, 1);
+    for (int s = 0; s < kPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * kPairEpiWarps); }
+    for (int w = 0; w < kPairEpiWarps; ++w) mbar_init(&s_bar[w], 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) { tmem_alloc(&tmem_base_slot, kTmemCols2); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc_pair(&tmem_base_slot, 512); tmem_relinquish_pair(); }
+  griddep_wait();
+  // a kernel of this stream already gave up on a wait: do not pile more work on a broken pipeline (the even CTA decides)
+  if (threadIdx.x == 0) skip_flag = L.status != nullptr && *(volatile const int*)L.status != 0;
   tc_fence_before();
   __syncthreads();
+  cluster_sync();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
+  const bool skip = cluster_load(cluster_addr(&skip_flag, 0)) != 0;
 
-  int issued = 0;
-  if (warp == 0) {
+  if (skip) {
+  } else if (warp == 0) {
     if (lane == 0) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const int s = kb % kStages, round = kb / kStages;
-        if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag)) break;
-        uint8_t* dst = tiles + s * kStageBytes2;
-        mbar_expect_tx(&full_bar[s], same_ab ? 2 * kTileBytes : kStageBytes2);
-        tma_load_3d(dst, &map_a, &full_bar[s], kb * BK, tm * BM2, batch);
-        tma_load_3d(dst + kTileBytes, &map_a, &full_bar[s], kb * BK, tm * BM2 + 128, batch);
-        if (!same_ab) {
+      int n = 0;  // ring fills so far
+      bool ok = true;
+      for (int idx = pair; idx < total && ok; idx += pairs) {
+        const TileAt t = tile_at(L, idx);
+        const GemmGroup& G = L.g[t.group];
+        const GemmParams P = G.P;  // by value: through the reference every use would be a load (nothing survives the asm fences)
+        const bool same_ab = P.same_operand && t.tm == t.tn;
+        const int num_kb = (P.K + BK - 1) / BK;
+        const int a_row = t.tm * kPairTile + (int)rank * 128, b_row = t.tn * kPairTile + (int)rank * 128;
+        for (int kb = 0; kb < num_kb; ++kb, ++n) {
+          const int s = n % kPairStages, round = n / kPairStages;
+          ok = mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag);
+          if (!ok) break;
+          uint8_t* dst = ring + s * kPairStageBytes;
+          const uint32_t bar = cluster_addr(&full_bar[s], 0);
+          if (rank == 0) mbar_expect_tx(&full_bar[s], same_ab ? 2 * kTileBytes : 2 * kPairStageBytes);
+          tma_load_3d_pair(dst, &G.a, bar, kb * BK, a_row, t.batch);
           if (P.b_mn) {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              tma_load_3d(dst + 2 * kTileBytes + j * kMnBoxBytes, &map_b, &full_bar[s], tn * BN2 + j * 64, kb * BK, batch);
-          } else {
-            tma_load_3d(dst + 2 * kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN2, batch);
-            tma_load_3d(dst + 3 * kTileBytes, &map_b, &full_bar[s], kb * BK, tn * BN2 + 128, batch);
+            tma_load_3d_pair(dst + kTileBytes, &G.b, bar, b_row, kb * BK, t.batch);
+            tma_load_3d_pair(dst + kTileBytes + kMnBoxBytes, &G.b, bar, b_row + 64, kb * BK, t.batch);
+          } else if (!same_ab) {
+            tma_load_3d_pair(dst + kTileBytes, &G.b, bar, kb * BK, b_row, t.batch);
           }
         }
-        issued = kb + 1;
       }
+      griddep_launch();  // this CTA's last loads are on their way: the next kernel of the chain may take over SMs that drain
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && rank == 0) {
+      int n = 0, it = 0;
       bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int s = kb % kStages, round = kb / kStages;
-        ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
+      for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
+        const TileAt t = tile_at(L, idx);
+        const GemmGroup& G = L.g[t.group];
+        const GemmParams P = G.P;  // by value: through the reference every use would be a load (nothing survives the asm fences)
+        const bool same_ab = P.same_operand && t.tm == t.tn;
+        const int num_kb = (P.K + BK - 1) / BK;
+        const int acc = it & 1;
+        ok = mbar_wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1, &abort_flag);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t base = smem_u32(tiles + s * kStageBytes2);
-        const uint64_t a_top = make_smem_desc(base), a_bot = make_smem_desc(base + kTileBytes);
-        // 256 operand rows = 32 eight-row groups, 1 KiB apart: the two 128-row boxes are contiguous
-        const uint64_t b_desc = same_ab ? a_top : (P.b_mn ? make_smem_desc_mn(base + 2 * kTileBytes, kMnBoxBytes) : make_smem_desc(base + 2 * kTileBytes));
-        const uint32_t b_step = P.b_mn ? kMnStep : 2u, idesc = kInstrDesc256 | (P.b_mn ? kInstrBMn : 0u);
+        const uint32_t d = tmem_base + (uint32_t)acc * 256u;
+        const uint32_t b_step = P.b_mn ? kMnStep : 2u, idesc = kInstrDescPair | (P.b_mn ? kInstrBMn : 0u);
+        for (int kb = 0; kb < num_kb; ++kb, ++n) {
+          const int s = n % kPairStages, round = n / kPairStages;
+          ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t base = smem_u32(ring + s * kPairStageBytes);
+          const uint64_t a_desc = make_smem_desc(base);
+          const uint64_t b_desc = same_ab ? a_desc : (P.b_mn ? make_smem_desc_mn(base + kTileBytes, kMnBoxBytes) : make_smem_desc(base + kTileBytes));
 #pragma unroll
-        for (int k = 0; k < BK / 16; ++k) {
-          const uint32_t acc = (kb | k) ? 1u : 0u;
-          tc_mma_bf16(tmem_base, a_top + 2 * k, b_desc + b_step * k, idesc, acc);
-          tc_mma_bf16(tmem_base + 256u, a_bot + 2 * k, b_desc + b_step * k, idesc, acc);
+          for (int k = 0; k < BK / 16; ++k) tc_mma_bf16_pair(d, a_desc + 2 * k, b_desc + b_step * k, idesc, (kb | k) ? 1u : 0u);
+          tc_commit_pair(&empty_bar[s]);
         }
-        tc_commit(&empty_bar[s]);
+        if (ok) tc_commit_pair(&acc_full[acc]);
       }
-      if (ok) tc_commit(&accum_bar);
     }
   } else {
-    const int quarter = warp & 3;
-    const int r = quarter * 32 + lane;
-    bool have = (num_kb == 0) || mbar_wait(&accum_bar, 0, &abort_flag);
-    tc_fence_after();
-    const bool mirror = P.symmetric ? (tn != tm) : true;
-    const bool want_c = P.C != nullptr, want_ct = P.CT != nullptr && mirror;
-    const int64_t b64 = batch;
-#pragma unroll 1
-    for (int hm = 0; hm < 2; ++hm) {
-      const int row0 = tm * BM2 + hm * 128;   // first global row of this half
-      const int row = row0 + r;
-      const bool live = row0 < P.M;            // the second half of a ragged last tile may be empty
-      if (have && poly && live) {
-        if (warp == 2 && lane == 0) {
-          mbar_expect_tx(&s_bar, kStageBytes2);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) tma_load_3d(s_tile + j * kTileBytes, &map_a, &s_bar, tn * BN2 + j * BK, row0, batch);
-        }
-        have = mbar_wait(&s_bar, hm & 1, &abort_flag);
+    const int quarter = warp & 3, half = (warp - 2) >> 2;  // tensor-memory lanes this warp may read; its half of the columns
+    uint8_t* const stage = ring + kPairStages * kPairStageBytes + (warp - 2) * 2 * kWarpStage;
+    uint64_t* const sb = &s_bar[warp - 2];
+    const uint32_t tmem_warp = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
+    int it = 0;
+    bool ok = true;
+    for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
+      const TileAt t = tile_at(L, idx);
+      const GemmGroup& G = L.g[t.group];
+      const GemmParams P = G.P;  // by value: through the reference every use would be a load (nothing survives the asm fences)
+      const bool poly = P.mode == kModePoly, f_bulk = G.f_bulk != 0;
+      const int acc = it & 1, row0 = t.tm * kPairTile + (int)rank * 128 + quarter * 32, row = row0 + lane;
+      const int first = t.tn * kPairTile + half * 128;
+      const bool mirror = P.symmetric ? (t.tn != t.tm) : true;
+      const bool want_c = P.C != nullptr, want_ct = P.CT != nullptr && mirror;
+      const bool two = P.CT == nullptr && !poly;  // without a transposed copy its buffer is a second one for C
+      if (poly && lane == 0) {  // the first S block arrives while the tile is still being multiplied
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+        mbar_expect_tx(sb, kWarpStage);
+        tma_load_3d(stage, &G.s, sb, first, row0, t.batch);
       }
-      if (have && live) {
+      __syncwarp();
+      ok = mbar_wait(&acc_full[acc], (it >> 1) & 1, &abort_flag);
+      if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
+      tc_fence_after();
 #pragma unroll 1
-        for (int cb = 0; cb < BN2 / 32; ++cb) {
-          uint32_t acc[32];
-          if (num_kb > 0) {
-            tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(hm * 256 + cb * 32), acc);
-            tmem_ld_wait();
-          } else {
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc[j] = 0u;
+      for (int q = 0; q < 2; ++q) {
+        const int col0 = first + q * 64;
+        uint8_t* c_st = stage + (two ? q * kWarpStage : 0);
+        uint8_t* ct_st = stage + kWarpStage;
+        uint32_t acc_r[2][32];
+        tmem_ld32(tmem_warp + (uint32_t)(acc * 256 + q * 64), acc_r[0]);
+        tmem_ld32(tmem_warp + (uint32_t)(acc * 256 + q * 64 + 32), acc_r[1]);
+        tmem_ld_wait();
+        if (q == 1) {  // last read of this accumulator
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) cluster_arrive(cluster_addr(&acc_empty[acc], 0));
+        }
+        if (poly) {
+          ok = mbar_wait(sb, q, &abort_flag);  // two blocks per tile: the phase is the block
+          if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
+        } else if (!f_bulk) {  // the store that read this buffer last
+          if (lane == 0) {
+            if (two) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+            else asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           }
-          const int box = cb >> 1, q0 = (cb & 1) * 4;
-          const int col0 = tn * BN2 + cb * 32;
-          float v[32];
+          __syncwarp();
+        }
 #pragma unroll
-          for (int j = 0; j < 32; ++j) v[j] = __uint_as_float(acc[j]);
-          if (poly) {
+        for (int h = 0; h < 2; ++h) {
+          uint32_t packed[16];  // rounded once, so that the tile, its mirrored copy and F agree bit for bit
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint4 sv = *(const uint4*)(s_tile + box * kTileBytes + swz(r, q0 + q));
+          for (int c = 0; c < 4; ++c) {
+            float v[8];
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = __uint_as_float(acc_r[h][c * 8 + e]);
+            uint4* slot = (uint4*)(c_st + swz(lane, h * 4 + c));
+            if (poly) {
+              const uint4 sv = *slot;
               const uint32_t w[4] = {sv.x, sv.y, sv.z, sv.w};
 #pragma unroll
               for (int e = 0; e < 8; ++e) {
-                const int j = q * 8 + e;
                 const float sval = bf16_bits_to_float((uint16_t)((w[e >> 1] >> ((e & 1) * 16)) & 0xFFFF));
-                v[j] = P.cc * v[j] + P.cb * sval + ((col0 + j == row) ? P.ca : 0.f);
+                v[e] = P.cc * v[e] + P.cb * sval + ((col0 + h * 32 + c * 8 + e == row) ? P.ca : 0.f);
               }
             }
-          }
-          uint16_t h[32];
 #pragma unroll
-          for (int j = 0; j < 32; ++j) h[j] = rne_bf16_bits(v[j]);
-          if (want_c) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              uint4 o;
-              o.x = (uint32_t)h[q * 8 + 0] | ((uint32_t)h[q * 8 + 1] << 16);
-              o.y = (uint32_t)h[q * 8 + 2] | ((uint32_t)h[q * 8 + 3] << 16);
-              o.z = (uint32_t)h[q * 8 + 4] | ((uint32_t)h[q * 8 + 5] << 16);
-              o.w = (uint32_t)h[q * 8 + 6] | ((uint32_t)h[q * 8 + 7] << 16);
-              *(uint4*)(c_stage + box * kTileBytes + swz(r, q0 + q)) = o;
+            for (int e = 0; e < 4; ++e) {
+              const __nv_bfloat162 two_values = __floats2bfloat162_rn(v[2 * e], v[2 * e + 1]);
+              packed[c * 4 + e] = *reinterpret_cast<const uint32_t*>(&two_values);
             }
+            if (want_c || want_ct) *slot = make_uint4(packed[c * 4], packed[c * 4 + 1], packed[c * 4 + 2], packed[c * 4 + 3]);
           }
-          if (want_ct) {  // transposed half tile: rows = the 256 columns (two 128-row groups), columns = r (two 64-wide boxes)
-            uint8_t* dst = ct_stage + ((cb >> 2) * 2 + (r >> 6)) * kTileBytes + (r & 7) * 2;
-            const int qr = (r & 63) >> 3, ct_row0 = (cb & 3) * 32;
+          if (P.F != nullptr) {
+            const int fc = col0 + h * 32;
+            if (f_bulk) {  // 32 x 32 fp32 block, one staging buffer per half
+              if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+              __syncwarp();
+              uint8_t* f_st = stage + h * kWarpStage;
 #pragma unroll
-            for (int j = 0; j < 32; ++j) *(uint16_t*)(dst + swz(ct_row0 + j, qr)) = h[j];
-          }
-          if (P.F != nullptr && row < P.M) {
-            float* f = P.F + b64 * P.strideF;
-            if (P.f_transposed) {
+              for (int c = 0; c < 8; ++c)
+                *(float4*)(f_st + swz(lane, c)) =
+                    make_float4(bf16_bits_to_float((uint16_t)(packed[c * 2] & 0xFFFF)) * P.f_scale, bf16_bits_to_float((uint16_t)(packed[c * 2] >> 16)) * P.f_scale,
+                                bf16_bits_to_float((uint16_t)(packed[c * 2 + 1] & 0xFFFF)) * P.f_scale, bf16_bits_to_float((uint16_t)(packed[c * 2 + 1] >> 16)) * P.f_scale);
+              asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+              __syncwarp();
+              if (lane == 0) {
+                if (fc < P.N && row0 < P.M) tma_store_3d(&G.c, f_st, fc, row0, t.batch);
+                asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+              }
+            } else if (row < P.M) {
+              float* f = P.F + (int64_t)t.batch * P.strideF;
 #pragma unroll
-              for (int j = 0; j < 32; ++j)
-                if (col0 + j < P.N) f[(int64_t)(col0 + j) * P.ldf + row] = bf16_bits_to_float(h[j]) * P.f_scale;
-            } else {
-              float* frow = f + (int64_t)row * P.ldf + col0;
-              if (col0 + 32 <= P.N && (P.ldf & 3) == 0 && (((uintptr_t)f) & 15) == 0) {
-#pragma unroll
-                for (int q = 0; q < 8; ++q)
-                  *(float4*)(frow + q * 4) =
-                      make_float4(bf16_bits_to_float(h[q * 4]) * P.f_scale, bf16_bits_to_float(h[q * 4 + 1]) * P.f_scale,
-                                  bf16_bits_to_float(h[q * 4 + 2]) * P.f_scale, bf16_bits_to_float(h[q * 4 + 3]) * P.f_scale);
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if (col0 + j < P.N) frow[j] = bf16_bits_to_float(h[j]) * P.f_scale;
+              for (int j = 0; j < 32; ++j) {
+                const float y = bf16_bits_to_float((uint16_t)((packed[j >> 1] >> ((j & 1) * 16)) & 0xFFFF)) * P.f_scale;
+                if (fc + j < P.N) f[P.f_transposed ? (int64_t)(fc + j) * P.ldf + row : (int64_t)row * P.ldf + fc + j] = y;
               }
             }
           }
         }
-      }
-      if (want_c || want_ct || poly) {
-        // staged tile -> global, and nobody may refill the staging (or the S region) before the copies have read it
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("bar.sync 1, 128;" ::: "memory");
-        if (have && live && warp == 2 && lane == 0 && (want_c || want_ct)) {
+        if (want_c || want_ct) {
+          __syncwarp();
+          if (want_ct) {  // 8 columns at a time: four 8x8 blocks of the staged tile, transposed on the way to the registers
 #pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            if (want_c && tn * BN2 + j * BK < P.N) tma_store_3d(&map_c, c_stage + j * kTileBytes, tn * BN2 + j * BK, row0, batch);
-            const int ct_r = tn * BN2 + (j >> 1) * 128, ct_c = row0 + (j & 1) * BK;
-            if (want_ct && ct_r < P.N && ct_c < P.M) tma_store_3d(&map_ct, ct_stage + j * kTileBytes, ct_c, ct_r, batch);
+            for (int c = 0; c < 8; ++c) {
+              uint32_t blk[4];
+              ldmatrix_x4_trans(smem_u32(c_st + swz(lane, c)), blk);
+              const int ct_row = c * 8 + (lane & 7), chunk = lane >> 3;
+              stmatrix_x4(smem_u32(ct_st + ct_row * 64 + ((chunk ^ ((ct_row >> 1) & 3)) << 4)), blk);
+            }
           }
-          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          __syncwarp();
+          if (lane == 0) {
+            if (col0 < P.N && row0 < P.M) {
+              if (want_c) tma_store_3d(&G.c, c_st, col0, row0, t.batch);
+              if (want_ct) tma_store_3d(&G.ct, ct_st, row0, col0, t.batch);
+            }
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+          }
+        }
+        if (poly && q == 0 && lane == 0) {
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+          mbar_expect_tx(sb, kWarpStage);
+          tma_load_3d(c_st, &G.s, sb, col0 + 64, row0, t.batch);
         }
-        asm volatile("bar.sync 1, 128;" ::: "memory");
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
     tc_fence_before();
   }
 
-  if (warp == 0 && lane == 0 && abort_flag) {
-    for (int kb = max(0, issued - kStages); kb < issued; ++kb) {
-      const int s = kb % kStages, round = kb / kStages;
-      for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
-        if (mbar_try_wait(&full_bar[s], round & 1)) break;
-    }
-  }
+  // after an expired wait: loads, products and S blocks in flight land within microseconds; give them a millisecond before
+  // the shared memory of the pair goes away
   __syncthreads();
-  if (threadIdx.x == 0 && abort_flag && P.status != nullptr) atomicExch(P.status, 1);
-  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTmemCols2); }
+  if (abort_flag) __nanosleep(1000000);
+  __syncthreads();
+  cluster_sync();
+  if (threadIdx.x == 0 && abort_flag && L.status != nullptr) atomicExch(L.status, 1);
+  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
 }
 
 // ------------------------------------------------------------------------------------------ prologue
@@ -506,24 +555,26 @@ ns_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
 // Gram matrix the small one.  `sumsq[b]` holds ||G_b||_F^2.
 // One block handles a 64 x 64 tile: 256 threads as 16 column-groups (4 columns each) x 16 rows, four row
 // passes.  Loads are 16 B (fp32) / 8 B (bf16), stores 8 bytes; the transpose goes through shared memory.
-// Grid: (ceil(C/64), ceil(R/64), batch).
-__global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __restrict__ srcs, int src_dt, int R, int C,
-                                                        const float* __restrict__ sumsq, float eps,
-                                                        __nv_bfloat16* __restrict__ dst, int64_t ld, int64_t stride, int trans,
-                                                        uint64_t seed) {
+// All matrices of a step share the launch: block b belongs to the matrix whose tile range holds it.
+__global__ void __launch_bounds__(256) ns_prepare_kernel(const NsSource* __restrict__ mats, const int* __restrict__ first, int n_mats,
+                                                        int src_dt, float eps) {
   __shared__ uint16_t tile[64][66];
-  const int b = blockIdx.z;
-  const void* src = srcs[b];
-  const float inv = 1.0f / fmaxf(sqrtf(sumsq[b]), eps);
-  const Philox rng(seed);
+  const int at = find_range(first, n_mats, blockIdx.x);
+  const NsSource S = mats[at];
+  const int R = S.rows, C = S.cols, b = S.index, trans = S.trans, tiles_c = (C + 63) >> 6;
+  const int local = blockIdx.x - first[at], by = local / tiles_c, bx = local - by * tiles_c;
+  const void* src = S.src;
+  const int64_t ld = S.ld;
+  const float inv = 1.0f / fmaxf(sqrtf(*S.sumsq), eps);
+  const Philox rng(S.seed);
   const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int c0 = blockIdx.x * 64 + tx * 4;
+  const int c0 = bx * 64 + tx * 4;
   const bool vec = (C & 3) == 0 && (((uintptr_t)src) & 15) == 0;
-  uint16_t* dst_b = (uint16_t*)dst + (int64_t)b * stride;
+  uint16_t* dst_b = (uint16_t*)S.dst;
   float x[4][4];
 #pragma unroll
   for (int pass = 0; pass < 4; ++pass) {  // every load of the tile is in flight before the first value is used
-    const int r = blockIdx.y * 64 + ty + 16 * pass;
+    const int r = by * 64 + ty + 16 * pass;
 #pragma unroll
     for (int k = 0; k < 4; ++k) x[pass][k] = 0.f;
     if (r < R && c0 < C) {
@@ -545,14 +596,16 @@ __global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __re
       }
     }
   }
+  uint4 rnd = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
   for (int pass = 0; pass < 4; ++pass) {
-    const int rl = ty + 16 * pass, r = blockIdx.y * 64 + rl;
+    const int rl = ty + 16 * pass, r = by * 64 + rl;
     uint16_t h[4] = {0, 0, 0, 0};
     if (r < R && c0 < C) {
       const int64_t idx = (int64_t)r * C + c0;
-      const uint4 rnd = rng((uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)b, 7u);
-      const uint32_t rr[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
+      // rounding to bf16 takes 16 random bits: a draw serves two row passes (low halves, then high halves)
+      if ((pass & 1) == 0) rnd = rng((uint32_t)idx, (uint32_t)(idx >> 32), (uint32_t)b, 7u);
+      const uint32_t rr[4] = {rnd.x >> (pass & 1) * 16, rnd.y >> (pass & 1) * 16, rnd.z >> (pass & 1) * 16, rnd.w >> (pass & 1) * 16};
 #pragma unroll
       for (int k = 0; k < 4; ++k)
         if (c0 + k < C) h[k] = sr_bf16_bits(x[pass][k] * inv, rr[k]);
@@ -571,10 +624,10 @@ __global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __re
   if (!trans) return;
   __syncthreads();
   // transposed output: this thread owns source rows r0..r0+3 (consecutive in the output row) of four source columns
-  const int r0 = blockIdx.y * 64 + tx * 4;
+  const int r0 = by * 64 + tx * 4;
 #pragma unroll
   for (int pass = 0; pass < 4; ++pass) {
-    const int cl = ty + 16 * pass, c = blockIdx.x * 64 + cl;
+    const int cl = ty + 16 * pass, c = bx * 64 + cl;
     if (c < C && r0 < R) {
       uint2 o;
       o.x = (uint32_t)tile[tx * 4 + 0][cl] | ((uint32_t)tile[tx * 4 + 1][cl] << 16);
@@ -585,107 +638,144 @@ __global__ void __launch_bounds__(256) ns_prepare_kernel(const void* const* __re
 }
 
 // ------------------------------------------------------------------------------------------ host side
-// bf16 tensor [batch, rows, cols] with leading dimension `ld` elements; box = 64 cols x `box_rows` rows.
-static bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch, int box_rows);
+// Tensor [batch, rows, cols] with leading dimension `ld` elements (bf16, or fp32 when `f32`); box = box_cols x box_rows,
+// swizzled over the width of a box row (128 or 64 bytes).
+static bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch,
+                       int box_cols, int box_rows, bool f32) {
+  EncodeTiledFn fn = tensor_map_encoder();
+  if (fn == nullptr) return false;
+  const int elem = f32 ? 4 : 2;
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * elem, (cuuint64_t)batch_stride * elem};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, (cuuint32_t)box_rows, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims,
+            strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            box_cols * elem == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
 
 // A step launches the same ~60 products over the same workspace addresses (the caching allocator hands the buffers
-// back), and every launch needs up to four descriptors: they are kept by their defining values instead of being
+// back), and every launch needs up to five descriptors: they are kept by their defining values instead of being
 // encoded again (about 0.6 us each on the host, which is what limits a step once the matrices are split over ranks).
 static bool make_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch,
-                     int box_rows = BM) {
+                     int box_cols = BK, int box_rows = BM, bool f32 = false) {
   struct Key {
-    const void* base; int64_t ld, stride; int rows, cols, batch, box_rows;
+    const void* base; int64_t ld, stride; int rows, cols, batch, box;
     bool operator==(const Key& o) const {
-      return base == o.base && ld == o.ld && stride == o.stride && rows == o.rows && cols == o.cols && batch == o.batch && box_rows == o.box_rows;
+      return base == o.base && ld == o.ld && stride == o.stride && rows == o.rows && cols == o.cols && batch == o.batch && box == o.box;
     }
   };
   struct Hash {
     size_t operator()(const Key& k) const {
       size_t h = std::hash<const void*>()(k.base);
-      for (int64_t v : {k.ld, k.stride, (int64_t)k.rows, (int64_t)k.cols, (int64_t)k.batch, (int64_t)k.box_rows})
+      for (int64_t v : {k.ld, k.stride, (int64_t)k.rows, (int64_t)k.cols, (int64_t)k.batch, (int64_t)k.box})
         h ^= std::hash<int64_t>()(v) + 0x9e3779b97f4a7c15ull + (h << 6) + (h >> 2);
       return h;
     }
   };
   static std::unordered_map<Key, CUtensorMap, Hash> cache;
   static std::mutex guard;
-  const Key key{base, ld, batch_stride, rows, cols, batch, box_rows};
+  const Key key{base, ld, batch_stride, rows, cols, batch, (box_cols << 16) | (box_rows << 1) | (f32 ? 1 : 0)};
   std::lock_guard<std::mutex> lock(guard);
   auto it = cache.find(key);
   if (it != cache.end()) {
     *map = it->second;
     return true;
   }
-  if (!encode_map(map, base, rows, cols, ld, batch_stride, batch, box_rows)) return false;
+  if (!encode_map(map, base, rows, cols, ld, batch_stride, batch, box_cols, box_rows, f32)) return false;
   if (cache.size() >= 4096) cache.clear();
   cache.emplace(key, *map);
   return true;
-}
-
-static bool encode_map(CUtensorMap* map, const void* base, int rows, int cols, int64_t ld, int64_t batch_stride, int batch,
-                       int box_rows) {
-  EncodeTiledFn fn = tensor_map_encoder();
-  if (fn == nullptr) return false;
-  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
-  cuuint64_t strides[2] = {(cuuint64_t)ld * 2, (cuuint64_t)batch_stride * 2};
-  cuuint32_t box[3] = {BK, (cuuint32_t)box_rows, 1};
-  cuuint32_t estr[3] = {1, 1, 1};
-  return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 static int g_tile_override = 0;
 int ns_gemm_tile_override() { return g_tile_override; }
 void set_ns_gemm_tile_override(int tile) { g_tile_override = tile; }
 
-cudaError_t launch_ns_gemm(const void* A, int64_t lda, int64_t strideA, const void* B, int64_t ldb, int64_t strideB,
-                           const GemmParams& P, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(ns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
-  GemmParams Q = P;
-  Q.same_operand = (!P.b_mn && A == B && lda == ldb && strideA == strideB && P.M == P.N) ? 1 : 0;
-  CUtensorMap ma, mb, mc, mct;
-  if (!make_map(&ma, A, P.M, P.K, lda, strideA, P.batch) || !(P.b_mn ? make_map(&mb, B, P.K, P.N, ldb, strideB, P.batch, BK) : make_map(&mb, B, P.N, P.K, ldb, strideB, P.batch)))
-    return cudaErrorInvalidValue;
-  mc = ma;
-  mct = ma;  // placeholders when an output is absent (never dereferenced by the kernel then)
-  if (P.C != nullptr && !make_map(&mc, P.C, P.M, P.N, P.ldc, P.strideC, P.batch)) return cudaErrorInvalidValue;
-  if (P.CT != nullptr && !make_map(&mct, P.CT, P.N, P.M, P.ldct, P.strideCT, P.batch)) return cudaErrorInvalidValue;
-  {
-    // large problems: 256x256 tiles (half the operand bytes per flop); they need a long K to hide their epilogue and
-    // enough tiles to fill the machine
-    const int t2m = (P.M + BM2 - 1) / BM2, t2n = (P.N + BN2 - 1) / BN2;
-    const long long big_tiles = (long long)(P.symmetric ? t2m * (t2m + 1) / 2 : t2m * t2n) * P.batch;
-    const bool want_big = ns_gemm_tile_override() == 256 ||
-                          (ns_gemm_tile_override() == 0 && P.K >= 1024 && P.M >= 1024 && P.N >= 1024 && big_tiles >= 96);
-    if (want_big) {
-      static bool configured2 = false;
-      if (!configured2) {
-        cudaError_t e = cudaFuncSetAttribute(ns_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes2);
-        if (e != cudaSuccess) return e;
-        configured2 = true;
-      }
-      dim3 grid2((unsigned)(P.symmetric ? t2m * (t2m + 1) / 2 : t2m * t2n), P.batch);
-      ns_gemm256_kernel<<<grid2, kGemmThreads, kSmemBytes2, stream>>>(ma, mb, mc, mct, Q);
-      return cudaGetLastError();
-    }
-  }
-  const int tiles_m = (P.M + BM - 1) / BM, tiles_n = (P.N + BN - 1) / BN;
-  const int tiles = P.symmetric ? tiles_m * (tiles_m + 1) / 2 : tiles_m * tiles_n;
-  dim3 grid(tiles, P.batch);
-  ns_gemm_kernel<<<grid, kGemmThreads, kSmemBytes, stream>>>(ma, mb, mc, mct, Q);
-  return cudaGetLastError();
+// Which tile a product takes on its own merits: the pair's 256 x 256 tile halves the operand bytes per flop but needs rows,
+// columns and a main loop long enough to fill it.  All 15 products of GPT-2-small's step (768 x 768 .. 3072 at 12 each):
+// 98 us per launch on pairs, 128 us on 128 x 128 tiles; of a Llama-3-8B layer: 0.81 against 1.04 ms.
+static bool pair_sized(const GemmParams& P) { return P.M >= 512 && P.N >= 512 && P.K >= 512; }
+static int pair_tiles(const GemmParams& P) {
+  const int tm = (P.M + kPairTile - 1) / kPairTile, tn = (P.N + kPairTile - 1) / kPairTile;
+  return (P.symmetric ? tm * (tm + 1) / 2 : tm * tn) * P.batch;
 }
 
-cudaError_t launch_ns_prepare(const void* const* srcs, int src_dt, int R, int C, int batch, const float* sumsq, float eps,
-                              void* dst, int64_t ld, int64_t stride, int trans, uint64_t seed, cudaStream_t stream) {
-  dim3 grid((C + 63) / 64, (R + 63) / 64, batch), block(256);
-  ns_prepare_kernel<<<grid, block, 0, stream>>>(srcs, src_dt, R, C, sumsq, eps, (__nv_bfloat16*)dst, ld, stride, trans, seed);
+// One launch of the pair kernel (`pair`) or of the 128 x 128 kernel over up to kMaxGroups products.
+static cudaError_t launch_group(const NsProduct* const* products, int n, bool pair, cudaStream_t stream) {
+  static int max_pairs = 0;
+  if (max_pairs == 0) {
+    cudaError_t e = cudaFuncSetAttribute(ns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(ns_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+    if (e != cudaSuccess) return e;
+    int found = 0;
+    if ((e = max_resident_pairs(ns_gemm_pair_kernel, kPairThreads, kPairSmemBytes, &found)) != cudaSuccess) return e;
+    max_pairs = found;
+  }
+  GemmGroups L;
+  L.n = n;
+  L.total = 0;
+  L.status = products[0]->P.status;
+  for (int i = 0; i < n; ++i) {
+    const NsProduct& X = *products[i];
+    GemmGroup& G = L.g[i];
+    GemmParams& P = G.P;
+    P = X.P;
+    P.same_operand = (!P.b_mn && X.A == X.B && X.lda == X.ldb && X.strideA == X.strideB && P.M == P.N) ? 1 : 0;
+    const int tile = pair ? kPairTile : BM;
+    G.tiles_m = (P.M + tile - 1) / tile;
+    G.tiles_n = (P.N + tile - 1) / tile;
+    G.per_batch = P.symmetric ? G.tiles_m * (G.tiles_m + 1) / 2 : G.tiles_m * G.tiles_n;
+    L.first[i] = L.total;
+    L.total += G.per_batch * P.batch;
+    // fp32 results leave through bulk stores when rows start on 16-byte boundaries and no bf16 copy needs the staging
+    G.f_bulk = pair && P.F != nullptr && !P.f_transposed && P.C == nullptr && P.CT == nullptr && (P.ldf & 3) == 0 &&
+               (P.strideF & 3) == 0 && (((uintptr_t)P.F) & 15) == 0;
+    bool ok = make_map(&G.a, X.A, P.M, P.K, X.lda, X.strideA, P.batch);
+    ok = ok && (P.b_mn ? make_map(&G.b, X.B, P.K, P.N, X.ldb, X.strideB, P.batch, BK, BK)
+                       : make_map(&G.b, X.B, P.N, P.K, X.ldb, X.strideB, P.batch));
+    G.c = G.ct = G.s = G.a;  // placeholders where an operand is absent (never dereferenced by the kernels then)
+    if (P.C != nullptr) ok = ok && make_map(&G.c, P.C, P.M, P.N, P.ldc, P.strideC, P.batch, 64, pair ? 32 : BM);
+    if (G.f_bulk) ok = ok && make_map(&G.c, P.F, P.M, P.N, P.ldf, P.strideF, P.batch, 32, 32, true);
+    if (P.CT != nullptr) ok = ok && make_map(&G.ct, P.CT, P.N, P.M, P.ldct, P.strideCT, P.batch, pair ? 32 : 64, pair ? 64 : BM);
+    if (pair && P.mode == kModePoly) ok = ok && make_map(&G.s, P.S, P.M, P.N, P.lds, P.strideS, P.batch, 64, 32);
+    if (!ok) return cudaErrorInvalidValue;
+  }
+  if (L.total == 0) return cudaSuccess;
+  if (pair) {
+    const int pairs = L.total < max_pairs ? L.total : max_pairs;
+    return launch_chained(ns_gemm_pair_kernel, dim3(2 * pairs), kPairThreads, kPairSmemBytes, stream, L);
+  }
+  return launch_chained(ns_gemm_kernel, dim3(L.total), kGemmThreads, kSmemBytes, stream, L);
+}
+
+cudaError_t launch_ns_products(const NsProduct* products, int n, int* launches, cudaStream_t stream) {
+  // tiles of a pair go to products that suit them, provided there are enough of them to occupy a good part of the machine
+  int big_tiles = 0;
+  for (int i = 0; i < n; ++i)
+    if (pair_sized(products[i].P)) big_tiles += pair_tiles(products[i].P);
+  const int force = ns_gemm_tile_override();
+  std::vector<const NsProduct*> side[2];
+  for (int i = 0; i < n; ++i)
+    side[force == 256 || (force == 0 && big_tiles >= 24 && pair_sized(products[i].P)) ? 1 : 0].push_back(&products[i]);
+  for (int pair = 1; pair >= 0; --pair) {
+    auto& list = side[pair];
+    // tiles are dealt out in order: the ones with the longest main loop first
+    std::stable_sort(list.begin(), list.end(), [](const NsProduct* a, const NsProduct* b) { return a->P.K > b->P.K; });
+    for (size_t i = 0; i < list.size(); i += kMaxGroups) {
+      const cudaError_t e = launch_group(list.data() + i, (int)std::min<size_t>(kMaxGroups, list.size() - i), pair != 0, stream);
+      if (e != cudaSuccess) return e;
+      if (launches != nullptr) ++*launches;
+    }
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_ns_prepare(const NsSource* mats, const int* first, int n_mats, int total_tiles, int src_dt, float eps,
+                              cudaStream_t stream) {
+  if (total_tiles == 0) return cudaSuccess;
+  ns_prepare_kernel<<<total_tiles, 256, 0, stream>>>(mats, first, n_mats, src_dt, eps);
   return cudaGetLastError();
 }
 

@@ -34,9 +34,28 @@ struct GemmParams {
 int ns_gemm_tile_override();
 void set_ns_gemm_tile_override(int tile);
 
-cudaError_t launch_ns_gemm(const void* A, int64_t lda, int64_t strideA, const void* B, int64_t ldb, int64_t strideB,
-                           const GemmParams& P, cudaStream_t stream);
-cudaError_t launch_ns_prepare(const void* const* srcs, int src_dt, int R, int C, int batch, const float* sumsq, float eps,
-                              void* dst, int64_t ld, int64_t stride, int trans, uint64_t seed, cudaStream_t stream);
+struct NsProduct {
+  const void* A;
+  int64_t lda, strideA;
+  const void* B;
+  int64_t ldb, strideB;
+  GemmParams P;
+};
+// Independent products, in as few launches as their tile sizes allow; `launches` (may be null) is advanced by their number.
+cudaError_t launch_ns_products(const NsProduct* products, int n, int* launches, cudaStream_t stream);
+
+// One matrix to be normalised and rounded into the bf16 iterate (as it is, or transposed).
+struct NsSource {
+  const void* src;
+  const float* sumsq;  // squared Frobenius norm
+  void* dst;
+  uint64_t seed;
+  int64_t ld;
+  int rows, cols, trans;
+  int index;           // position within its bucket (part of the rounding noise's address)
+};
+// `first`: n_mats + 1 prefix sums of the matrices' 64 x 64 tile counts; both tables in device memory.
+cudaError_t launch_ns_prepare(const NsSource* mats, const int* first, int n_mats, int total_tiles, int src_dt, float eps,
+                              cudaStream_t stream);
 
 }  // namespace hb

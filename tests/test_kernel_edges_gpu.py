@@ -58,6 +58,51 @@ def test_ecc_codec_over_all_exponents():
     torch.testing.assert_close(out[big].double(), want[big], rtol=1e-6, atol=0)
 
 
+# ---------------------------------------------------------------------------------------- Newton-Schulz products
+
+
+def _poly_oracle(x, a, b, c):
+    """One polynomial step in fp64 with the kernel's bf16 roundings of S and of the polynomial."""
+    s = (x @ x.mT).to(torch.bfloat16).double()
+    y = (c * (s @ s) + b * s + a * torch.eye(x.shape[-2], dtype=torch.float64, device=x.device)).to(torch.bfloat16).double()
+    return (y @ x).to(torch.bfloat16).double()
+
+
+@pytest.mark.parametrize("tile", [0, 128, 256])
+@pytest.mark.parametrize("shapes", [((64, 64),), ((129, 257), (257, 129)), ((255, 520),), ((512, 512), (520, 768), (768, 513)),
+                                    ((1030, 512), (77, 200), (300, 300)), tuple((96 + 8 * i, 160) for i in range(11))], ids=str)  # fmt: skip
+def test_grouped_newton_schulz_step(tile, shapes):
+    """Several shapes (up to eleven: more than one launch holds) in one chain, both orientations, ragged tiles.  The iterate is
+    read back from a step with polynomial 1 (an identity), then one step with all three coefficients is compared with fp64
+    products of the same bf16 operands: what remains is the order of fp32 sums, which may move a value by one bf16 rounding
+    (2^-8) in S, in the polynomial and in the result."""
+    ext = ops.load()
+    ext.set_ns_gemm_tile(tile)
+    try:
+        gen = torch.Generator(DEV).manual_seed(3)
+        mats = [[torch.randn(s, device=DEV, generator=gen) for _ in range(2)] for s in shapes]
+        norms = torch.stack([m.square().sum() for pair in mats for m in pair])
+        at = [range(2 * k, 2 * k + 2) for k in range(len(shapes))]
+
+        def go(coeffs):
+            outs = [torch.full((2, *s), float("nan"), device=DEV) for s in shapes]
+            ops.newton_schulz_groups([(m, i, o, 1.0, 7 + k) for k, (m, i, o) in enumerate(zip(mats, at, outs))], norms, coeffs)
+            ops.check_status()
+            return outs
+
+        start, got = go([(1.0, 0.0, 0.0)]), go([(3.0, -4.0, 2.0)])
+    finally:
+        ext.set_ns_gemm_tile(0)
+    for m, x, y in zip(mats, start, got):
+        want_x = torch.stack(m) / torch.stack(m).norm(dim=(-2, -1), keepdim=True)
+        assert (x - want_x).abs().max() <= want_x.abs().max() * 2**-7  # stochastic rounding to bf16
+        flip = (lambda t: t.mT) if x.shape[-2] > x.shape[-1] else (lambda t: t)
+        want = flip(_poly_oracle(flip(x.double()), 3.0, -4.0, 2.0))
+        err = (y.double() - want).abs().max() / want.abs().max()
+        assert err < 3 * 2**-8, err
+        assert (y.double() - want).norm() / want.norm() < 2**-9
+
+
 # ---------------------------------------------------------------------------------------- triangular leaves
 
 
