@@ -106,6 +106,41 @@ __device__ inline int ecc_residual(float x, uint16_t prim, bool bf16, float smax
   return __float2int_rd(e + unit_rand);
 }
 
+// The same for four bf16 values with 8-bit residuals, the usual kind.  One test of the exponents serves the four (false: the
+// caller takes the element-wise path), and conversions between integers and floats go through the low mantissa bits of 2^23
+// instead of the conversion unit, which delivers 4 lanes a cycle: byte -> float as 2^23 + byte, floor -> byte by adding
+// 1.5 * 2^23 rounded down.  Same bits as the element-wise codec.
+__device__ inline bool ecc8_decode4(uint32_t lo, uint32_t hi, uint32_t res, float (&v)[4]) {
+  const uint32_t b[4] = {lo << 16, lo & 0xFFFF0000u, hi << 16, hi & 0xFFFF0000u};
+  const uint32_t e[4] = {b[0] & 0x7F800000u, b[1] & 0x7F800000u, b[2] & 0x7F800000u, b[3] & 0x7F800000u};
+  if (min(min(e[0], e[1]), min(e[2], e[3])) < kEccFastExp) return false;
+  const uint32_t biased = res ^ 0x80808080u;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float c = __uint_as_float(__byte_perm(biased, 0x4B000000u, 0x7650u + k)) - 8388736.0f;  // 2^23 + 128
+    v[k] = fmaf(c * (1.0f / 127.0f), __uint_as_float(e[k] - (8u << 23)), __uint_as_float(b[k]));
+  }
+  return true;
+}
+
+__device__ inline bool ecc8_encode4(const float (&x)[4], const uint32_t (&rnd)[4], uint32_t& lo, uint32_t& hi, uint32_t& res) {
+  const __nv_bfloat162 p0 = __floats2bfloat162_rn(x[0], x[1]), p1 = __floats2bfloat162_rn(x[2], x[3]);
+  lo = *reinterpret_cast<const uint32_t*>(&p0);
+  hi = *reinterpret_cast<const uint32_t*>(&p1);
+  const uint32_t b[4] = {lo << 16, lo & 0xFFFF0000u, hi << 16, hi & 0xFFFF0000u};
+  const uint32_t e[4] = {b[0] & 0x7F800000u, b[1] & 0x7F800000u, b[2] & 0x7F800000u, b[3] & 0x7F800000u};
+  if (min(min(e[0], e[1]), min(e[2], e[3])) < kEccFastExp) return false;
+  uint32_t r[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float d = (x[k] - __uint_as_float(b[k])) * __uint_as_float((262u << 23) - e[k]);
+    const float y = fminf(fmaxf(d, -1.0f), 1.0f) * 127.0f + u32_to_unit(rnd[k]);
+    r[k] = __float_as_uint(__fadd_rd(y, 12582912.0f));  // 1.5 * 2^23 + floor(y): the low byte is the residual
+  }
+  res = __byte_perm(__byte_perm(r[0], r[1], 0x0040), __byte_perm(r[2], r[3], 0x0040), 0x5410);
+  return true;
+}
+
 // ---------------------------------------------------------------------------------------------
 // 4-wide generic load / store.  `p` is the primary buffer, `c` the ECC residual buffer (or null).
 // ---------------------------------------------------------------------------------------------
@@ -241,6 +276,82 @@ __device__ inline void store4(void* p, void* c, int dt, int64_t i, int n_valid, 
         if (k < n_valid) cp[k] = (int8_t)corr[k];
     }
   }
+}
+
+// ---------------------------------------------------------------------------------------------
+// The load in two halves, for storage kinds known at compile time: the words of four elements, and their values.  Decoding an
+// error-corrected value branches on its exponent, and loads behind a branch that waits for a load wait with it: a kernel that
+// decoded each array as it arrived paid one memory round trip per array instead of one for all.
+// ---------------------------------------------------------------------------------------------
+struct Raw4 {
+  uint32_t w[4];
+};
+
+template <int DT>
+__device__ inline Raw4 load_raw(const void* p, const void* c, int64_t i, int n_valid, bool vec_ok) {
+  Raw4 r{{0u, 0u, 0u, 0u}};
+  if (DT == kNone || p == nullptr) return r;
+  const bool fast = vec_ok && n_valid == 4;
+  if (DT == kF32) {
+    const uint32_t* f = (const uint32_t*)p + i;
+    if (fast) {
+      const uint4 t = *(const uint4*)f;
+      r.w[0] = t.x; r.w[1] = t.y; r.w[2] = t.z; r.w[3] = t.w;
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (k < n_valid) r.w[k] = f[k];
+    }
+    return r;
+  }
+  const uint16_t* h = (const uint16_t*)p + i;
+  const uint8_t* e = (const uint8_t*)c + i;
+  if (fast) {
+    const uint2 t = *(const uint2*)h;
+    r.w[0] = t.x; r.w[1] = t.y;
+    if (DT == kBF16E8) r.w[2] = *(const uint32_t*)e;
+  } else {
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k < n_valid) {
+        r.w[k >> 1] |= (uint32_t)h[k] << (16 * (k & 1));
+        if (DT == kBF16E8) r.w[2] |= (uint32_t)e[k] << (8 * k);
+      }
+  }
+  return r;
+}
+
+template <int DT>
+__device__ inline F4 decode_raw(const Raw4& r) {
+  static_assert(DT == kF32 || DT == kBF16 || DT == kBF16E8 || DT == kNone, "storage kinds of the specialised kernels");
+  F4 out;
+  if (DT == kBF16E8) {
+    if (ecc8_decode4(r.w[0], r.w[1], r.w[2], out.v)) return out;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      out.v[k] = ecc_decode((uint16_t)(r.w[k >> 1] >> (16 * (k & 1))), (int)(int8_t)(r.w[2] >> (8 * k)), true, 1.0f / 127.0f);
+    return out;
+  }
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    out.v[k] = DT == kF32 ? __uint_as_float(r.w[k]) : __uint_as_float((k & 1) ? (r.w[k >> 1] & 0xFFFF0000u) : (r.w[k >> 1] << 16));
+  return out;
+}
+
+// store4 for a storage kind known at compile time.
+template <int DT>
+__device__ inline void store_values(void* p, void* c, int64_t i, int n_valid, bool vec_ok, const F4& x, uint4 rnd) {
+  if (DT == kBF16E8 && p != nullptr && c != nullptr && vec_ok && n_valid == 4) {
+    const uint32_t rr[4] = {rnd.x, rnd.y, rnd.z, rnd.w};
+    uint2 prim;
+    uint32_t res;
+    if (ecc8_encode4(x.v, rr, prim.x, prim.y, res)) {
+      *(uint2*)((uint16_t*)p + i) = prim;
+      *(uint32_t*)((int8_t*)c + i) = res;
+      return;
+    }
+  }
+  store4(p, c, DT, i, n_valid, vec_ok, x, rnd);
 }
 
 // ---------------------------------------------------------------------------------------------

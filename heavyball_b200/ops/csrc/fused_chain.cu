@@ -334,12 +334,12 @@ __global__ void __launch_bounds__(kThreads, 4) fused_chain_kernel(const TensorMe
 }
 
 // ---------------------------------------------------------------------------------------------
-// Specialised instances for the launches without peers, clips, update transforms, post-state, schedule-free output and
+// Specialised instances for the launches without peers, gradient clips, sign updates, post-state, schedule-free output and
 // third state, which are the bulk of every step: storage kinds, destination and source of the update are compile-time
-// constants, and kBatch vectors per thread are loaded before anything is computed or stored (stores may alias later loads,
+// constants, and a kind's batch of vectors per thread is loaded before anything is computed or stored (stores may alias later loads,
 // so the compiler cannot move those up by itself: a vector at a time is a memory round trip each).  Against the general kernel:
 // AdamW on the 39.5 M fp32 parameters of GPT-2-small's embeddings 242 -> 170 us (6.5 TB/s), cautious AdamW with error-corrected
-// state on 8 x 2048^2 965 -> 562 us.
+// state on 8 x 2048^2 965 -> 562 us, and 357 us with the loads separated from the codec.
 // ---------------------------------------------------------------------------------------------
 // One rule with at most two states on one element: advances the states and returns the new direction.
 template <int A>
@@ -380,15 +380,19 @@ __device__ __forceinline__ F4 apply_rule(const ChainParams& P, const F4& u, F4& 
   return out;
 }
 
-constexpr int kBatch = 2;
-
 template <int DTP, int DTG, int DTU, int DTS, int OUT, int UIN, bool COUNT>
 struct ChainKind {
   static constexpr int dt_p = DTP, dt_g = DTG, dt_u = DTU, dt_s = DTS, out_mode = OUT;
   static constexpr bool u_in = UIN != 0, count = COUNT, state = DTS != kNone;
   static constexpr bool reads_g = !u_in || count, reads_p = OUT == kOutParam;
-  // two vectors in flight through a rule need about 80 registers: three blocks per SM instead of four with spills
-  static constexpr int min_blocks = state ? 3 : 4;
+  // Vectors per thread loaded together, and blocks per SM.  Two vectors through a rule need about 80 registers: three blocks.
+  // The codec and its random bits are 190 instructions per element and want warps rather than vectors in flight: with
+  // error-corrected state one vector is as many as fit (momentum of a Llama-3-8B layer 1.76 -> 1.32 ms at one vector and four
+  // blocks; the three arrays of cautious Adam with MARS 295 us at two vectors and two blocks, 307 at one and four, 285 at one
+  // and three).
+  static constexpr bool ecc = DTS == kBF16E8;
+  static constexpr int batch = ecc ? 1 : 2;
+  static constexpr int min_blocks = state && !(ecc && !count) ? 3 : 4;
   static bool takes(const ChainParams& P, bool counting) {
     return counting == COUNT && P.out_mode == OUT && P.u_is_input == UIN && (!reads_p || P.dt_p == DTP) &&
            (!reads_g || P.dt_g == DTG) && ((OUT == kOutParam && !u_in) || P.dt_u == DTU) && P.dt_s == DTS;
@@ -417,24 +421,25 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
       cscale *= n / fmaxf(n - (float)(*M.masked), 1.0f);
     }
   }
+  constexpr int kBatch = K::batch;
   int masked_local = 0;
   float sumsq_local = 0.f, nonzero_local = 0.f;
 
 #pragma unroll 1
   for (int64_t i0 = base + threadIdx.x * 4; i0 < min(numel, base + P.chunk); i0 += kBatch * kThreads * 4) {
-    F4 s0[kBatch], s1[kBatch], old[kBatch], g[kBatch], u[kBatch], p[kBatch];
+    Raw4 s0[kBatch], s1[kBatch], old[kBatch], g[kBatch], u[kBatch], p[kBatch];
 #pragma unroll
     for (int v = 0; v < kBatch; ++v) {
       const int64_t i = i0 + v * (kThreads * 4);
       const int nv = (int)max((int64_t)0, min((int64_t)4, numel - i));
       if (K::state) {
-        s0[v] = load4(m0, m0e, K::dt_s, i, nv, vec_ok);
-        s1[v] = load4(m1, m1e, K::dt_s, i, nv, vec_ok);
-        if (P.mars) old[v] = load4(mm, mme, K::dt_s, i, nv, vec_ok);
+        s0[v] = load_raw<K::dt_s>(m0, m0e, i, nv, vec_ok);
+        s1[v] = load_raw<K::dt_s>(m1, m1e, i, nv, vec_ok);
+        if (P.mars) old[v] = load_raw<K::dt_s>(mm, mme, i, nv, vec_ok);
       }
-      if (K::reads_g) g[v] = load4(mg, nullptr, K::dt_g, i, nv, vec_ok);
-      if (K::u_in) u[v] = load4(mu, nullptr, K::dt_u, i, nv, vec_ok);
-      if (K::reads_p) p[v] = load4(mp, mpe, K::dt_p, i, nv, vec_ok);
+      if (K::reads_g) g[v] = load_raw<K::dt_g>(mg, nullptr, i, nv, vec_ok);
+      if (K::u_in) u[v] = load_raw<K::dt_u>(mu, nullptr, i, nv, vec_ok);
+      if (K::reads_p) p[v] = load_raw<K::dt_p>(mp, mpe, i, nv, vec_ok);
     }
 #pragma unroll
     for (int v = 0; v < kBatch; ++v) {
@@ -442,30 +447,40 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
       const int nv = (int)max((int64_t)0, min((int64_t)4, numel - i));
       if (nv == 0) break;
       const uint32_t ctr = (uint32_t)(i >> 2), ctr_hi = (uint32_t)(i >> 34);
-      F4 x = K::u_in ? u[v] : g[v];
+      F4 grad{}, x;
+      if (K::reads_g) grad = decode_raw<K::dt_g>(g[v]);
+      x = K::u_in ? decode_raw<K::u_in ? K::dt_u : (int)kNone>(u[v]) : grad;
+      if (K::u_in && P.u_op == kUopTrustRegion) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) x.v[k] = trust_region(x.v[k]);
+      }
       if (K::state && P.mars) {  // g <- lerp(g, g_prev, a); g_prev <- raw g
-        const F4 raw = x;
+        const F4 raw = x, before = decode_raw<K::dt_s>(old[v]);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          x.v[k] = x.v[k] * (1.0f - P.mars_a) + old[v].v[k] * P.mars_a;
-          g[v].v[k] = x.v[k];
+          x.v[k] = x.v[k] * (1.0f - P.mars_a) + before.v[k] * P.mars_a;
+          grad.v[k] = x.v[k];
         }
-        store4(mm, mme, K::dt_s, i, nv, vec_ok, raw, draw(K::dt_s, rng, ctr, ctr_hi ^ 0x40000000u, (uint32_t)t, 4u));
+        store_values<K::dt_s>(mm, mme, i, nv, vec_ok, raw, draw(K::dt_s, rng, ctr, ctr_hi ^ 0x40000000u, (uint32_t)t, 4u));
       }
-      F4 out = K::state ? apply_rule(P, x, s0[v], s1[v]) : x;
+      F4 out = x;
       if (K::state) {
-        if (P.n_state >= 1) store4(m0, m0e, K::dt_s, i, nv, vec_ok, s0[v], draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 0u));
-        if (P.n_state >= 2) store4(m1, m1e, K::dt_s, i, nv, vec_ok, s1[v], draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 1u));
+        F4 a{}, b{};
+        if (m0 != nullptr) a = decode_raw<K::dt_s>(s0[v]);
+        if (m1 != nullptr) b = decode_raw<K::dt_s>(s1[v]);
+        out = apply_rule(P, x, a, b);
+        if (P.n_state >= 1) store_values<K::dt_s>(m0, m0e, i, nv, vec_ok, a, draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 0u));
+        if (P.n_state >= 2) store_values<K::dt_s>(m1, m1e, i, nv, vec_ok, b, draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 1u));
       }
       if (K::count) {  // phase one of caution: mask, count, park the masked update
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-          const bool disagree = (__float_as_uint(g[v].v[k]) ^ __float_as_uint(out.v[k])) >> 31;
+          const bool disagree = (__float_as_uint(grad.v[k]) ^ __float_as_uint(out.v[k])) >> 31;
           if (k < nv && disagree) { out.v[k] = 0.f; ++masked_local; }
         }
       }
       if (!K::reads_p) {
-        store4(mu, nullptr, K::dt_u, i, nv, vec_ok, out, draw(K::dt_u, rng, ctr, ctr_hi, (uint32_t)t, 5u));
+        store_values<K::dt_u>(mu, nullptr, i, nv, vec_ok, out, draw(K::dt_u, rng, ctr, ctr_hi, (uint32_t)t, 5u));
         if (!K::count && P.accum_sumsq) {
 #pragma unroll
           for (int k = 0; k < 4; ++k)
@@ -477,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
         continue;
       }
       // parameter epilogue: p <- p (1 - d lr) - lr u
-      F4 np = p[v];
+      F4 np = decode_raw<K::reads_p ? K::dt_p : (int)kNone>(p[v]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float uu = out.v[k] * cscale;
@@ -485,7 +500,7 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
         if (P.cautious_wd && ((__float_as_uint(np.v[k]) ^ __float_as_uint(uu)) >> 31)) d = 0.f;
         np.v[k] = np.v[k] * (1.0f - d * P.lr) + uu * -P.lr;
       }
-      store4(mp, mpe, K::dt_p, i, nv, vec_ok, np, draw(K::dt_p, rng, ctr, ctr_hi, (uint32_t)t, 3u));
+      store_values<K::dt_p>(mp, mpe, i, nv, vec_ok, np, draw(K::dt_p, rng, ctr, ctr_hi, (uint32_t)t, 3u));
     }
   }
   finish_block<K::count>(P, M, sumsq_local, nonzero_local, masked_local);
@@ -597,7 +612,7 @@ using PlainLaunch = void (*)(const TensorMeta*, const int*, ChainParams);
 template <class... Ks>
 PlainLaunch find_kind(KindList<Ks...>, const ChainParams& P, bool count) {
   const bool plain = P.n_state <= 2 && P.algo != kAdemamix && P.n_src == 0 && P.n_dst == 0 && P.g_clip_mode == kClipNone &&
-                     P.u_op == kUopNone && P.post_state == kPostNone && P.out_mode != kOutScheduleFree &&
+                     (P.u_op == kUopNone || (P.u_op == kUopTrustRegion && P.u_is_input)) && P.post_state == kPostNone && P.out_mode != kOutScheduleFree &&
                      (!P.u_is_input || (P.algo == kIdentity && P.n_state == 0 && !P.mars)) && !(count && P.accum_sumsq);
   PlainLaunch hit = nullptr;
   if (plain) ((hit == nullptr && Ks::takes(P, count) ? (void)(hit = plain_chain_kernel<Ks>) : (void)0), ...);
