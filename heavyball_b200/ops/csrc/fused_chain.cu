@@ -391,7 +391,10 @@ struct ChainKind {
   // blocks; the three arrays of cautious Adam with MARS 295 us at two vectors and two blocks, 307 at one and four, 285 at one
   // and three).
   static constexpr bool ecc = DTS == kBF16E8;
-  static constexpr int batch = ecc ? 1 : 2;
+  // Otherwise a thread should have about 128 bytes on their way: two vectors of Adam's four arrays, four where a launch reads
+  // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 288 us with two vectors,
+  // 250 with four, of which the bytes take 204 at 6.65 TB/s).
+  static constexpr int batch = ecc ? 1 : (state && (reads_p || count) ? 2 : 4);
   static constexpr int min_blocks = state && !(ecc && !count) ? 3 : 4;
   static bool takes(const ChainParams& P, bool counting) {
     return counting == COUNT && P.out_mode == OUT && P.u_is_input == UIN && (!reads_p || P.dt_p == DTP) &&
@@ -407,7 +410,7 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
   const int b = (K::u_in && K::reads_p) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
   const int t = find_range(chunk_prefix, P.n_tensors, b);
   const TensorMeta& M = metas[t];
-  const int64_t numel = M.numel, base = (int64_t)(b - chunk_prefix[t]) * P.chunk;
+  const int64_t numel = M.numel, base = (int64_t)(b - chunk_prefix[t]) * P.chunk, end = min(numel, base + P.chunk);
   const bool vec_ok = M.vec_ok != 0;
   const Philox rng(P.seed);
   void *const mp = M.p, *const mpe = M.pe, *const mg = M.g, *const mu = M.u;
@@ -426,12 +429,12 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
   float sumsq_local = 0.f, nonzero_local = 0.f;
 
 #pragma unroll 1
-  for (int64_t i0 = base + threadIdx.x * 4; i0 < min(numel, base + P.chunk); i0 += kBatch * kThreads * 4) {
+  for (int64_t i0 = base + threadIdx.x * 4; i0 < end; i0 += kBatch * kThreads * 4) {
     Raw4 s0[kBatch], s1[kBatch], old[kBatch], g[kBatch], u[kBatch], p[kBatch];
 #pragma unroll
     for (int v = 0; v < kBatch; ++v) {
       const int64_t i = i0 + v * (kThreads * 4);
-      const int nv = (int)max((int64_t)0, min((int64_t)4, numel - i));
+      const int nv = (int)max((int64_t)0, min((int64_t)4, end - i));
       if (K::state) {
         s0[v] = load_raw<K::dt_s>(m0, m0e, i, nv, vec_ok);
         s1[v] = load_raw<K::dt_s>(m1, m1e, i, nv, vec_ok);
@@ -444,7 +447,7 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
 #pragma unroll
     for (int v = 0; v < kBatch; ++v) {
       const int64_t i = i0 + v * (kThreads * 4);
-      const int nv = (int)max((int64_t)0, min((int64_t)4, numel - i));
+      const int nv = (int)max((int64_t)0, min((int64_t)4, end - i));
       if (nv == 0) break;
       const uint32_t ctr = (uint32_t)(i >> 2), ctr_hi = (uint32_t)(i >> 34);
       F4 grad{}, x;
