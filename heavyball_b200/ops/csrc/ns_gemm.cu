@@ -34,6 +34,7 @@
 #include <mutex>
 #include <unordered_map>
 #include <vector>
+#include "pair_drain.h"
 #include "tc_common.cuh"
 
 namespace hb {
@@ -319,8 +320,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
   __shared__ __align__(8) uint64_t acc_full[2];             // in each CTA: accumulator finished
   __shared__ __align__(8) uint64_t acc_empty[2];            // in the even CTA: all sixteen epilogue warps have read it
   __shared__ __align__(8) uint64_t s_bar[kPairEpiWarps];
+  __shared__ __align__(8) uint64_t drain_bar;               // in each CTA, teardown only: all products have finished
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag, skip_flag;
+  __shared__ int fills, fill_bytes[kPairStages];            // ring fills this CTA issued, bytes of the last one of each stage
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();
@@ -331,7 +334,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
     for (int s = 0; s < kPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * kPairEpiWarps); }
     for (int w = 0; w < kPairEpiWarps; ++w) mbar_init(&s_bar[w], 1);
+    mbar_init(&drain_bar, 1);
     abort_flag = 0;
+    fills = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) { tmem_alloc_pair(&tmem_base_slot, 512); tmem_relinquish_pair(); }
@@ -363,6 +368,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
           if (!ok) break;
           uint8_t* dst = ring + s * kPairStageBytes;
           const uint32_t bar = cluster_addr(&full_bar[s], 0);
+          fill_bytes[s] = same_ab ? kTileBytes : kPairStageBytes;
           if (rank == 0) mbar_expect_tx(&full_bar[s], same_ab ? 2 * kTileBytes : 2 * kPairStageBytes);
           tma_load_3d_pair(dst, &G.a, bar, kb * BK, a_row, t.batch);
           if (P.b_mn) {
@@ -373,6 +379,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
           }
         }
       }
+      fills = n;
       griddep_launch();  // this CTA's last loads are on their way: the next kernel of the chain may take over SMs that drain
     }
   } else if (warp == 1) {
@@ -411,7 +418,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
     uint8_t* const stage = ring + kPairStages * kPairStageBytes + (warp - 2) * 2 * kWarpStage;
     uint64_t* const sb = &s_bar[warp - 2];
     const uint32_t tmem_warp = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
-    int it = 0;
+    int it = 0, s_block = -1;  // s_block: parity of the S load in flight, -1 without one
     bool ok = true;
     for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
       const TileAt t = tile_at(L, idx);
@@ -427,6 +434,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
         asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
         mbar_expect_tx(sb, kWarpStage);
         tma_load_3d(stage, &G.s, sb, first, row0, t.batch);
+        s_block = 0;
       }
       __syncwarp();
       ok = mbar_wait(&acc_full[acc], (it >> 1) & 1, &abort_flag);
@@ -449,6 +457,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
         if (poly) {
           ok = mbar_wait(sb, q, &abort_flag);  // two blocks per tile: the phase is the block
           if (!__all_sync(0xFFFFFFFFu, ok)) { ok = false; break; }
+          s_block = -1;
         } else if (!f_bulk) {  // the store that read this buffer last
           if (lane == 0) {
             if (two) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -533,19 +542,36 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           mbar_expect_tx(sb, kWarpStage);
           tma_load_3d(c_st, &G.s, sb, col0 + 64, row0, t.batch);
+          s_block = 1;
         }
       }
     }
-    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    if (lane == 0) {
+      if (s_block >= 0) mbar_drain(sb, s_block);
+      asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+    }
     tc_fence_before();
   }
 
-  // after an expired wait: loads, products and S blocks in flight land within microseconds; give them a millisecond before
-  // the shared memory of the pair goes away
+  // After an expired wait in either CTA, both wait (with a limit) for every product and every load that the pair issued before its
+  // shared and tensor memory go away; the blocks of S and the stores were waited for above.
   __syncthreads();
-  if (abort_flag) __nanosleep(1000000);
-  __syncthreads();
+  if (threadIdx.x == 0 && abort_flag) cluster_store(cluster_addr(&abort_flag, rank ^ 1), 1);
   cluster_sync();
+  if (abort_flag) {
+    if (rank == 0 && warp == 1 && lane == 0) tc_commit_pair(&drain_bar);  // the thread that issued the products
+    if (threadIdx.x == 0) mbar_drain(&drain_bar, 0);
+    if (rank == 0 && threadIdx.x == 0) {
+      const int even = fills, odd = cluster_load(cluster_addr(&fills, 1)), top = max(even, odd);
+      for (int n = pair_drain_first(even, odd, kPairStages); n < top; ++n) {
+        const int s = n % kPairStages, kind = pair_fill_kind(n, even, odd);
+        if (kind == kFillOddOnly) mbar_expect_tx(&full_bar[s], (uint32_t)cluster_load(cluster_addr(&fill_bytes[s], 1)));
+        if (kind == kFillEvenOnly) mbar_complete_tx(&full_bar[s], (uint32_t)fill_bytes[s]);
+        mbar_drain(&full_bar[s], (n / kPairStages) & 1);
+      }
+    }
+    cluster_sync();
+  }
   if (threadIdx.x == 0 && abort_flag && L.status != nullptr) atomicExch(L.status, 1);
   if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
 }

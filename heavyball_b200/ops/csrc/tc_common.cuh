@@ -40,6 +40,16 @@ __device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* a
   return false;
 }
 
+// Teardown after an expired wait: gives what is still in flight the same bounded time to finish.
+__device__ inline void mbar_drain(uint64_t* bar, uint32_t parity) {
+  for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
+    if (mbar_try_wait(bar, parity)) return;
+}
+// counts `bytes` off the barrier's current phase without a copy
+__device__ inline void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {
+  asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
 __device__ inline void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar, int c0, int c1, int c2) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
@@ -108,6 +118,9 @@ __device__ inline int cluster_load(uint32_t addr) {
   int v;
   asm volatile("ld.shared::cluster.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
   return v;
+}
+__device__ inline void cluster_store(uint32_t addr, int v) {
+  asm volatile("st.shared::cluster.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ inline void cluster_arrive(uint32_t bar_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar_addr) : "memory");

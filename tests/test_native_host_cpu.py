@@ -1,0 +1,90 @@
+"""Host-side pieces of the native sources, compiled with the system compiler and run here: protocol bookkeeping that a GPU run
+only reaches after a failure."""
+
+import os
+import shutil
+import subprocess
+
+import pytest
+
+from heavyball_b200 import ops
+
+_CSRC = os.path.join(os.path.dirname(os.path.abspath(ops.__file__)), "csrc")
+
+
+def _run(tmp_path, source):
+    compiler = shutil.which("g++") or shutil.which("c++")
+    if compiler is None:
+        pytest.skip("no C++ compiler")
+    (tmp_path / "t.cpp").write_text(source)
+    subprocess.run([compiler, "-std=c++17", "-O1", "-pthread", "-I", _CSRC, str(tmp_path / "t.cpp"), "-o", str(tmp_path / "t")], check=True)
+    done = subprocess.run([str(tmp_path / "t")], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0, done.stdout + done.stderr
+
+
+def test_pair_teardown_accounts_for_every_load_in_flight(tmp_path):
+    """Two producers fill a ring whose phases live on one barrier (one arrival announcing both CTAs' bytes, and the bytes as they
+    land) while a consumer frees stages in order.  Everything stops at a random point with loads still in flight; after the
+    bookkeeping of the teardown each phase that may hold a load completes exactly when its last load has landed, and no load in
+    flight belongs to a phase that is not waited for."""
+    _run(tmp_path, r"""
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+#include <vector>
+#include "pair_drain.h"
+struct Bar {  // an mbarrier with one expected arrival: phase ends when the arrival is there and no bytes are outstanding
+  int phase = 0, pending = 1; long tx = 0;
+  void settle() { if (pending == 0 && tx == 0) { ++phase; pending = 1; } }
+  void expect(long b) { if (pending == 0) { puts("second arrival in a phase"); exit(1); } tx += b; --pending; settle(); }
+  void count_off(long b) { tx -= b; settle(); }
+};
+struct Load { int fill; long bytes; };
+int main() {
+  std::mt19937 rng(1);
+  for (int trial = 0; trial < 20000; ++trial) {
+    const int stages = 1 + rng() % 6;
+    std::vector<Bar> full(stages);
+    std::vector<Load> flight;
+    std::vector<long> bytes(64);
+    for (auto& b : bytes) b = rng() % 2 ? 16384 : 32768;
+    int issued[2] = {0, 0}, consumed = 0;
+    const int steps = rng() % 120;
+    for (int i = 0; i < steps; ++i) {
+      const int what = rng() % 4;
+      if (what < 2) {
+        const int n = issued[what];
+        if (n < 64 && n < consumed + stages) {
+          if (what == 0) full[n % stages].expect(2 * bytes[n]);
+          flight.push_back({n, bytes[n]});
+          ++issued[what];
+        }
+      } else if (what == 2) {
+        if (!flight.empty()) {
+          const size_t k = rng() % flight.size();
+          full[flight[k].fill % stages].count_off(flight[k].bytes);
+          flight.erase(flight.begin() + k);
+        }
+      } else if (consumed < 64 && full[consumed % stages].phase > consumed / stages) {
+        ++consumed;
+      }
+    }
+    const int even = issued[0], odd = issued[1], top = even > odd ? even : odd, from = hb::pair_drain_first(even, odd, stages);
+    for (const Load& l : flight)
+      if (l.fill < from) { puts("a load in flight is not waited for"); return 1; }
+    for (int n = from; n < top; ++n) {
+      const int kind = hb::pair_fill_kind(n, even, odd);
+      if (kind == hb::kFillOddOnly) full[n % stages].expect(bytes[n]);
+      if (kind == hb::kFillEvenOnly) full[n % stages].count_off(bytes[n]);
+      while (full[n % stages].phase <= n / stages) {  // the wait: loads keep landing meanwhile, one at a time in random order
+        if (flight.empty()) { printf("stuck: fill %d of %d / %d\n", n, even, odd); return 1; }
+        const size_t k = rng() % flight.size();
+        full[flight[k].fill % stages].count_off(flight[k].bytes);
+        flight.erase(flight.begin() + k);
+      }
+    }
+    if (!flight.empty()) { puts("returned with a load in flight"); return 1; }
+  }
+  return 0;
+}
+""")
