@@ -35,6 +35,7 @@
 #include <unordered_map>
 #include <vector>
 #include "pair_drain.h"
+#include "per_device.h"
 #include "tc_common.cuh"
 
 namespace hb {
@@ -728,17 +729,24 @@ static int pair_tiles(const GemmParams& P) {
   return (P.symmetric ? tm * (tm + 1) / 2 : tm * tn) * P.batch;
 }
 
+// Pairs of CTAs that the current device holds at once, after allowing both kernels their shared memory there.
+static cudaError_t resident_pairs(int* out) {
+  static PerDevice<int> pairs;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return pairs.get(device, cudaSuccess, out, [](int& found) {
+    cudaError_t s = cudaFuncSetAttribute(ns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    if (s == cudaSuccess) s = cudaFuncSetAttribute(ns_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+    return s != cudaSuccess ? s : max_resident_pairs(ns_gemm_pair_kernel, kPairThreads, kPairSmemBytes, &found);
+  });
+}
+
 // One launch of the pair kernel (`pair`) or of the 128 x 128 kernel over up to kMaxGroups products.
 static cudaError_t launch_group(const NsProduct* const* products, int n, bool pair, cudaStream_t stream) {
-  static int max_pairs = 0;
-  if (max_pairs == 0) {
-    cudaError_t e = cudaFuncSetAttribute(ns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(ns_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
-    if (e != cudaSuccess) return e;
-    int found = 0;
-    if ((e = max_resident_pairs(ns_gemm_pair_kernel, kPairThreads, kPairSmemBytes, &found)) != cudaSuccess) return e;
-    max_pairs = found;
-  }
+  int max_pairs = 0;
+  const cudaError_t e = resident_pairs(&max_pairs);
+  if (e != cudaSuccess) return e;
   GemmGroups L;
   L.n = n;
   L.total = 0;

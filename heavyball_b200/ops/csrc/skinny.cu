@@ -11,6 +11,8 @@
 // plenty of row parallelism and stays a library GEMM (a version written here the same way was slower).
 #include "skinny.h"
 
+#include "per_device.h"
+
 #include <stdint.h>
 
 namespace hb {
@@ -342,12 +344,15 @@ __global__ void __launch_bounds__(kLeafThreads) chol_inv_leaf_kernel(const float
 }
 
 cudaError_t configure_leaf_kernels() {
-  static bool configured = false;
-  if (configured) return cudaSuccess;
-  cudaError_t e = cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeafBytes);
-  if (e == cudaSuccess) e = cudaFuncSetAttribute(chol_inv_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeafBytes);
-  configured = e == cudaSuccess;
-  return e;
+  static PerDevice<bool> configured;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  bool done = false;
+  return configured.get(device, cudaSuccess, &done, [](bool&) {
+    const cudaError_t s = cudaFuncSetAttribute(tri_inv_blocks_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeafBytes);
+    return s != cudaSuccess ? s : cudaFuncSetAttribute(chol_inv_leaf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeafBytes);
+  });
 }
 
 }  // namespace

@@ -24,6 +24,7 @@
 // Waits are bounded as in the bf16 kernels: on expiry the CTA flags `status`, drains, frees TMEM and returns.
 #include "tf32_gemm.h"
 
+#include "per_device.h"
 #include "tc_common.cuh"
 
 namespace hb {
@@ -587,14 +588,16 @@ void set_tf32_gemm_tile_override(int tile) { g_tf32_tile_override = (tile == 128
 
 cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int K, int batch, const Tf32Epilogue& E,
                              int* status, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(tf32_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(tf32_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes2);
-    if (e != cudaSuccess) return e;
-    configured = true;
-  }
+  static PerDevice<bool> configured;
+  int device = 0;
+  bool done = false;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess)
+    e = configured.get(device, cudaSuccess, &done, [](bool&) {
+      const cudaError_t s = cudaFuncSetAttribute(tf32_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
+      return s != cudaSuccess ? s : cudaFuncSetAttribute(tf32_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes2);
+    });
+  if (e != cudaSuccess) return e;
   if (M == 0 || N == 0 || batch == 0) return cudaSuccess;
   if ((E.mode == kEpiAdam || E.mode == kEpiLaProp) && (E.m == nullptr || E.v == nullptr)) return cudaErrorInvalidValue;
   if ((E.mode == kEpiLerp || E.mode == kEpiAdd) && E.C == nullptr) return cudaErrorInvalidValue;

@@ -6,8 +6,9 @@ import shutil
 import subprocess
 
 import pytest
+import torch
 
-from heavyball_b200 import ops
+from heavyball_b200 import ops, utils
 
 _CSRC = os.path.join(os.path.dirname(os.path.abspath(ops.__file__)), "csrc")
 
@@ -88,3 +89,49 @@ int main() {
   return 0;
 }
 """)
+
+
+def test_settings_are_made_once_for_every_device(tmp_path):
+    """The second device of a process gets its own, from several threads each is made once, and an error is not remembered."""
+    _run(tmp_path, r"""
+#include <atomic>
+#include <cstdio>
+#include <thread>
+#include <vector>
+#include "per_device.h"
+int main() {
+  hb::PerDevice<int> values;
+  std::atomic<int> made[3] = {};
+  std::atomic<bool> wrong{false};
+  auto ask = [&](int device, int status) {
+    int got = -1;
+    const int s = values.get(device, 0, &got, [&](int& v) { ++made[device]; v = 100 + device; return status; });
+    if (s != status && s != 0) wrong = true;
+    if (s == 0 && got != 100 + device) wrong = true;
+    return s;
+  };
+  if (ask(0, 7) != 7 || ask(0, 0) != 0) { puts("an error has to come back once and be forgotten"); return 1; }
+  std::vector<std::thread> threads;
+  for (int t = 0; t < 8; ++t)
+    threads.emplace_back([&, t] { for (int i = 0; i < 1000; ++i) ask((t + i) % 3, 0); });
+  for (auto& t : threads) t.join();
+  if (wrong || made[0] != 2 || made[1] != 1 || made[2] != 1) { puts("made more than once, or a wrong value"); return 1; }
+  return 0;
+}
+""")
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
+def test_tensor_core_and_leaf_kernels_run_on_a_second_device_of_the_process():
+    for dev in ("cuda:0", "cuda:1"):
+        mats = [torch.randn(96, 160, device=dev) for _ in range(2)]
+        out = ops.newton_schulz_batched(mats, utils.NS5_COEFFS)
+        assert 0.5 < torch.linalg.svdvals(out).mean().item() < 1.5
+        a = torch.randn(2, 256, 256, device=dev)
+        torch.testing.assert_close(ops.matmul3(a, a), a @ a, rtol=1e-3, atol=1e-3)
+        r, info = torch.empty_like(a), torch.zeros(2, dtype=torch.int32, device=dev)
+        inv = torch.empty(2, 1, 128, 128, device=dev)
+        ops.load().chol_inv_leaf(a @ a.mT + 256 * torch.eye(256, device=dev), r, inv, 0, 128, info)
+        assert info.sum().item() == 0
+        ops.check_status()
