@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_c
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kStages];
   __shared__ __align__(8) uint64_t empty_bar[kStages];
-  __shared__ __align__(8) uint64_t accum_bar;
+  __shared__ __align__(8) uint64_t accum_bar, drain_bar;  // drain_bar: teardown only
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
@@ -118,6 +118,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_c
   if (threadIdx.x == 0) {
     for (int s = 0; s < kStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     mbar_init(&accum_bar, 1);
+    mbar_init(&drain_bar, 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -283,16 +284,14 @@ __global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_c
     }
   }
 
-  // ---- teardown: the producer makes sure nothing it issued is still landing in shared memory
-  if (warp == 0 && lane == 0 && abort_flag) {
-    for (int kb = max(0, issued - kStages); kb < issued; ++kb) {
-      const int s = kb % kStages, round = kb / kStages;
-      for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
-        if (mbar_try_wait(&full_bar[s], round & 1)) break;
-    }
-  }
+  // ---- teardown: after an expired wait, nothing may still land in shared memory or be multiplied when they are given back
   __syncthreads();
-  if (threadIdx.x == 0 && abort_flag && L.status != nullptr) atomicExch(L.status, 1);
+  if (abort_flag) {
+    if (warp == 0 && lane == 0) ring_drain(full_bar, issued, kStages);
+    if (warp == 1 && lane == 0) products_drain(&drain_bar);
+    __syncthreads();
+    if (threadIdx.x == 0 && L.status != nullptr) atomicExch(L.status, 1);
+  }
   if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTmemCols); }
 }
 

@@ -45,6 +45,10 @@ __device__ inline void mbar_drain(uint64_t* bar, uint32_t parity) {
   for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
     if (mbar_try_wait(bar, parity)) return;
 }
+// ... for a ring of `stages` barriers after `issued` fills: all but the last `stages` have been read by a product already
+__device__ inline void ring_drain(uint64_t* full_bar, int issued, int stages) {
+  for (int n = issued > stages ? issued - stages : 0; n < issued; ++n) mbar_drain(&full_bar[n % stages], (n / stages) & 1);
+}
 // counts `bytes` off the barrier's current phase without a copy
 __device__ inline void mbar_complete_tx(uint64_t* bar, uint32_t bytes) {
   asm volatile("mbarrier.complete_tx.relaxed.cta.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
@@ -69,6 +73,11 @@ __device__ inline void tc_fence_after() { asm volatile("tcgen05.fence::after_thr
 __device__ inline void tc_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+// ... for the products this thread has issued; `bar` counts one arrival and is used for nothing else
+__device__ inline void products_drain(uint64_t* bar) {
+  tc_commit(bar);
+  mbar_drain(bar, 0);
 }
 __device__ inline void tc_mma_bf16(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
   asm volatile(

@@ -252,7 +252,7 @@ tf32_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kTStages];
   __shared__ __align__(8) uint64_t empty_bar[kTStages];
-  __shared__ __align__(8) uint64_t accum_bar;
+  __shared__ __align__(8) uint64_t accum_bar, drain_bar;  // drain_bar: teardown only
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
@@ -280,6 +280,7 @@ tf32_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
   if (threadIdx.x == 0) {
     for (int s = 0; s < kTStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     mbar_init(&accum_bar, 1);
+    mbar_init(&drain_bar, 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -357,15 +358,13 @@ tf32_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     }
   }
 
-  if (warp == 0 && lane == 0 && abort_flag) {  // let in-flight loads land before the CTA's shared memory goes away
-    for (int kb = max(0, issued - kTStages); kb < issued; ++kb) {
-      const int s = kb % kTStages, round = kb / kTStages;
-      for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
-        if (mbar_try_wait(&full_bar[s], round & 1)) break;
-    }
-  }
   __syncthreads();
-  if (threadIdx.x == 0 && abort_flag && status != nullptr) atomicExch(status, 1);
+  if (abort_flag) {  // after an expired wait: loads and products in flight end before shared and tensor memory go away
+    if (warp == 0 && lane == 0) ring_drain(full_bar, issued, kTStages);
+    if (warp == 1 && lane == 0) products_drain(&drain_bar);
+    __syncthreads();
+    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
+  }
   if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTTmemCols); }
 }
 
@@ -389,7 +388,7 @@ tf32_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kTStages];
   __shared__ __align__(8) uint64_t empty_bar[kTStages];
-  __shared__ __align__(8) uint64_t accum_bar;
+  __shared__ __align__(8) uint64_t accum_bar, drain_bar;  // drain_bar: teardown only
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
@@ -416,6 +415,7 @@ tf32_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   if (threadIdx.x == 0) {
     for (int s = 0; s < kTStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
     mbar_init(&accum_bar, 1);
+    mbar_init(&drain_bar, 1);
     abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -476,15 +476,13 @@ tf32_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tc_fence_before();
   }
 
-  if (warp == 0 && lane == 0 && abort_flag) {
-    for (int kb = max(0, issued - kTStages); kb < issued; ++kb) {
-      const int s = kb % kTStages, round = kb / kTStages;
-      for (uint32_t spin = 0; spin < kSpinLimit; ++spin)
-        if (mbar_try_wait(&full_bar[s], round & 1)) break;
-    }
-  }
   __syncthreads();
-  if (threadIdx.x == 0 && abort_flag && status != nullptr) atomicExch(status, 1);
+  if (abort_flag) {
+    if (warp == 0 && lane == 0) ring_drain(full_bar, issued, kTStages);
+    if (warp == 1 && lane == 0) products_drain(&drain_bar);
+    __syncthreads();
+    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
+  }
   if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTTmemCols2); }
 }
 
