@@ -29,6 +29,7 @@
 
 #include "common.cuh"
 #include "ns_gemm.h"
+#include "ns_tiles.h"
 
 #include <algorithm>
 #include <mutex>
@@ -719,15 +720,6 @@ static int g_tile_override = 0;
 int ns_gemm_tile_override() { return g_tile_override; }
 void set_ns_gemm_tile_override(int tile) { g_tile_override = tile; }
 
-// Which tile a product takes on its own merits: the pair's 256 x 256 tile halves the operand bytes per flop but needs rows,
-// columns and a main loop long enough to fill it.  All 15 products of GPT-2-small's step (768 x 768 .. 3072 at 12 each):
-// 98 us per launch on pairs, 128 us on 128 x 128 tiles; of a Llama-3-8B layer: 0.81 against 1.04 ms.
-static bool pair_sized(const GemmParams& P) { return P.M >= 512 && P.N >= 512 && P.K >= 512; }
-static int pair_tiles(const GemmParams& P) {
-  const int tm = (P.M + kPairTile - 1) / kPairTile, tn = (P.N + kPairTile - 1) / kPairTile;
-  return (P.symmetric ? tm * (tm + 1) / 2 : tm * tn) * P.batch;
-}
-
 // Pairs of CTAs that the current device holds at once, after allowing both kernels their shared memory there.
 static cudaError_t resident_pairs(int* out) {
   static PerDevice<int> pairs;
@@ -742,10 +734,7 @@ static cudaError_t resident_pairs(int* out) {
 }
 
 // One launch of the pair kernel (`pair`) or of the 128 x 128 kernel over up to kMaxGroups products.
-static cudaError_t launch_group(const NsProduct* const* products, int n, bool pair, cudaStream_t stream) {
-  int max_pairs = 0;
-  const cudaError_t e = resident_pairs(&max_pairs);
-  if (e != cudaSuccess) return e;
+static cudaError_t launch_group(const NsProduct* const* products, int n, bool pair, int max_pairs, cudaStream_t stream) {
   GemmGroups L;
   L.n = n;
   L.total = 0;
@@ -784,20 +773,23 @@ static cudaError_t launch_group(const NsProduct* const* products, int n, bool pa
 }
 
 cudaError_t launch_ns_products(const NsProduct* products, int n, int* launches, cudaStream_t stream) {
-  // tiles of a pair go to products that suit them, provided there are enough of them to occupy a good part of the machine
-  int big_tiles = 0;
+  int max_pairs = 0;
+  const cudaError_t found = resident_pairs(&max_pairs);
+  if (found != cudaSuccess) return found;
+  std::vector<NsExtent> extents;
+  extents.reserve(n);
   for (int i = 0; i < n; ++i)
-    if (pair_sized(products[i].P)) big_tiles += pair_tiles(products[i].P);
+    extents.push_back({products[i].P.M, products[i].P.N, products[i].P.K, products[i].P.batch, products[i].P.symmetric != 0});
   const int force = ns_gemm_tile_override();
+  const bool pairs = force == 0 && ns_take_pairs(extents.data(), n, max_pairs);
   std::vector<const NsProduct*> side[2];
-  for (int i = 0; i < n; ++i)
-    side[force == 256 || (force == 0 && big_tiles >= 24 && pair_sized(products[i].P)) ? 1 : 0].push_back(&products[i]);
+  for (int i = 0; i < n; ++i) side[force == 256 || (pairs && ns_pair_sized(extents[i])) ? 1 : 0].push_back(&products[i]);
   for (int pair = 1; pair >= 0; --pair) {
     auto& list = side[pair];
     // tiles are dealt out in order: the ones with the longest main loop first
     std::stable_sort(list.begin(), list.end(), [](const NsProduct* a, const NsProduct* b) { return a->P.K > b->P.K; });
     for (size_t i = 0; i < list.size(); i += kMaxGroups) {
-      const cudaError_t e = launch_group(list.data() + i, (int)std::min<size_t>(kMaxGroups, list.size() - i), pair != 0, stream);
+      const cudaError_t e = launch_group(list.data() + i, (int)std::min<size_t>(kMaxGroups, list.size() - i), pair != 0, max_pairs, stream);
       if (e != cudaSuccess) return e;
       if (launches != nullptr) ++*launches;
     }

@@ -30,7 +30,7 @@ struct GemmParams {
   int* status;              // set to 1 if a bounded wait expired
 };
 
-// Tile choice of launch_ns_gemm: 0 = by problem size (default), 128 / 256 = force that output tile (tests, tuning).
+// Tile choice of launch_ns_products: 0 = by problem size (ns_tiles.h, default), 128 / 256 = force that output tile (tests, tuning).
 int ns_gemm_tile_override();
 void set_ns_gemm_tile_override(int tile);
 

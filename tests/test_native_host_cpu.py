@@ -121,6 +121,41 @@ int main() {
 """)
 
 
+def test_newton_schulz_tile_choice(tmp_path):
+    """Sizes at which either tile was measured to be the faster one, on 74 pairs: one wave of small tiles and its end, waves that
+    pairs need more of, rows off the 128-byte lines, a main loop too short, products of several sizes."""
+    _run(tmp_path, r"""
+#include <cstdio>
+#include <vector>
+#include "ns_tiles.h"
+int bad = 0;
+void expect(bool pairs, std::vector<hb::NsExtent> p) {
+  if (hb::ns_take_pairs(p.data(), (int)p.size(), 74) != pairs) { printf("%d x %d x %d, %d: expected %d\n", p[0].M, p[0].N, p[0].K, p[0].batch, pairs); ++bad; }
+}
+int main() {
+  expect(false, {{512, 512, 512, 8, true}});      // 24 pair tiles, a third of the pairs
+  expect(false, {{1024, 1024, 1024, 8, true}});   // 288 small tiles: one wave; 80 pair tiles: two
+  expect(false, {{640, 640, 640, 10, false}});
+  expect(false, {{768, 3072, 768, 2, false}});    // 288 small tiles
+  expect(true, {{768, 2304, 768, 3, false}});     // 324
+  expect(true, {{1024, 1024, 1024, 8, false}});   // 512
+  expect(false, {{1024, 1024, 1024, 16, true}});  // two waves of small tiles, three of pairs
+  expect(true, {{1024, 1024, 1024, 24, true}});   // three and four
+  expect(false, {{640, 640, 640, 20, false}});
+  expect(true, {{900, 900, 1300, 6, true}});      // unaligned rows
+  expect(false, {{900, 900, 1300, 8, true}});     // ... but 80 pair tiles
+  expect(true, {{900, 900, 1300, 3, true}});      // 108 small tiles
+  expect(false, {{900, 900, 1300, 2, true}});     // 72
+  expect(true, {{600, 600, 1800, 32, true}});
+  expect(false, {{700, 700, 700, 8, false}});     // unaligned, but a short K
+  expect(false, {{768, 768, 511, 100, false}});   // main loop too short
+  expect(true, {{768, 768, 768, 48, true}, {77, 200, 77, 1, false}});
+  expect(true, {{768, 768, 768, 12, true}, {768, 768, 2304, 12, true}, {768, 768, 3072, 12, true}});
+  return bad;
+}
+""")
+
+
 @pytest.mark.gpu
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_tensor_core_and_leaf_kernels_run_on_a_second_device_of_the_process():
