@@ -17,7 +17,7 @@ import enum
 import itertools
 import math
 import sys
-from typing import List, Union
+from typing import List, Sequence, Union
 
 import torch
 from torch import Tensor
@@ -376,30 +376,73 @@ def _panel_qr_replayed(x: Tensor, fallback: Tensor = None):
     return static_out.clone()
 
 
-def _qr_basis(x: Tensor, fallback: Tensor = None) -> Tensor:
+def _cholqr_applies(x: Tensor) -> bool:
+    return (x.is_cuda and _settings().fast_qr and x.shape[-2] >= x.shape[-1] >= _CHOLQR_MIN
+            and not torch.cuda.is_current_stream_capturing())  # fmt: skip
+
+
+def _ladder_key(x: Tensor):
+    return x.device, tuple(x.shape)
+
+
+def _ladder_won(key, level: int):
+    qr_stats["cholesky_qr2" if level == 0 else f"cholesky_qr_shifted_{_CHOLQR_LADDER[level]}"] += 1
+    # start where it worked next time, and try one step cheaper every eighth success
+    wins = _cholqr_wins[key] = _cholqr_wins.get(key, 0) + 1
+    _cholqr_level[key] = max(0, level - 1) if wins % 8 == 0 else level
+
+
+def _panel_basis(x: Tensor, fallback: Tensor = None):
+    """The panel-wise route (``None``: not for this input, or a matrix failed and there was nothing to keep)."""
+    if not (x.is_cuda and _settings().fast_qr and x.shape[-2] >= x.shape[-1] >= 2 * _QR_PANEL):
+        return None
+    return _panel_qr_replayed(x.contiguous(), fallback) if _settings().graph_qr else _panel_cholesky_qr(x)
+
+
+def _qr_basis(x: Tensor, fallback: Tensor = None, lowest: int = 0) -> Tensor:
     """Q factor of ``x``.  ``fallback``: orthonormal matrix to keep where the fast factorisation fails (see
-    :func:`_panel_qr_replayed`); without it a failure costs a host synchronisation and Householder QR."""
+    :func:`_panel_qr_replayed`); without it a failure costs a host synchronisation and Householder QR.  ``lowest``: first
+    step of the ladder that is worth trying."""
     x32 = promote(x)
-    if (x32.is_cuda and _settings().fast_qr and x32.shape[-2] >= x32.shape[-1] >= _CHOLQR_MIN
-            and not torch.cuda.is_current_stream_capturing()):  # fmt: skip
+    if _cholqr_applies(x32):
         xc = x32.contiguous()
-        key = (xc.device, tuple(xc.shape))
-        start = _cholqr_level.get(key, 0)
-        for level in range(start, len(_CHOLQR_LADDER)):
+        key = _ladder_key(xc)
+        for level in range(max(lowest, _cholqr_level.get(key, 0)), len(_CHOLQR_LADDER)):
             q, bad = _cholesky_qr2_replayed(xc, _CHOLQR_LADDER[level])
             if int(bad.sum()) == 0:  # one host read per attempt; a failure climbs the ladder, then takes the panel-wise route
-                qr_stats["cholesky_qr2" if level == 0 else f"cholesky_qr_shifted_{_CHOLQR_LADDER[level]}"] += 1
-                # start where it worked next time, and try one step cheaper every eighth success
-                wins = _cholqr_wins[key] = _cholqr_wins.get(key, 0) + 1
-                _cholqr_level[key] = max(0, level - 1) if wins % 8 == 0 else level
+                _ladder_won(key, level)
                 return q.clone() if q.data_ptr() != x32.data_ptr() else q
         _cholqr_level[key] = len(_CHOLQR_LADDER) - 1
         qr_stats["cholesky_qr2_rejected"] += 1
-    if x32.is_cuda and _settings().fast_qr and x32.shape[-2] >= x32.shape[-1] >= 2 * _QR_PANEL:
-        q = _panel_qr_replayed(x32.contiguous(), fallback) if _settings().graph_qr else _panel_cholesky_qr(x32)
-        if q is not None:
-            return q
-    return torch.linalg.qr(x32).Q
+    q = _panel_basis(x32, fallback)
+    return q if q is not None else torch.linalg.qr(x32).Q
+
+
+def _qr_bases(x: Tensor, fallback: Tensor, sizes: Sequence[int]) -> Tensor:
+    """:func:`_qr_basis` of independent batches that follow one another in ``x`` (``sizes`` matrices each), as one chain of
+    launches where that changes nothing for any of them.  Every batch is accepted or refused by itself and keeps its own
+    place on the ladder: a refused one climbs alone, and while the batches stand on different steps each takes its own
+    route, so a factor that is hard to refresh costs the others neither their variant nor their result."""
+    x32 = promote(x).contiguous()
+    alone = lambda: torch.cat([_qr_basis(m, f) for m, f in zip(x32.split(sizes), fallback.split(sizes))])  # noqa: E731
+    if not _cholqr_applies(x32):
+        q = _panel_basis(x32, fallback)  # a failure in the joint run must not send the others to another factorisation
+        return q if q is not None else alone()
+    keys = [_ladder_key(m) for m in x32.split(sizes)]
+    levels = {_cholqr_level.get(key, 0) for key in keys}
+    if len(levels) > 1:
+        return alone()
+    (level,) = levels
+    q, bad = _cholesky_qr2_replayed(x32, _CHOLQR_LADDER[level])
+    refused = [bool(flags.any()) for flags in bad.cpu().split(sizes)]
+    q = q.clone() if q.data_ptr() != x32.data_ptr() else q
+    for key, no in zip(keys, refused):
+        if not no:
+            _ladder_won(key, level)
+    for out, m, f, no in zip(q.split(sizes), x32.split(sizes), fallback.split(sizes), refused):
+        if no:
+            out.copy_(_qr_basis(m, f, level + 1))
+    return q
 
 
 def _compilable_orthogonal_(x: Tensor, mode, out, scale_mode):

@@ -132,26 +132,77 @@ def test_cholesky_leaf_at_sub_block_edges(n):
     assert info.tolist() == [0, 1, 0]
 
 
-def test_eigenbases_of_several_buckets_refresh_together():
-    """One joint refresh of three buckets (shared sizes, one factor missing) against the bucket-by-bucket definition."""
+def _factor(gen, b, n):
+    """Statistics whose eigenbasis is known to a few percent, and that basis."""
+    q = torch.linalg.qr(torch.randn(b, n, n, device=DEV, generator=gen))[0]
+    noise = torch.randn(b, n, n, device=DEV, generator=gen) * 0.02 / n**0.5
+    return (q * torch.logspace(1, 0, n, device=DEV)) @ q.mT + noise + noise.mT, q
+
+
+def _copies(items):
+    clone = lambda xs: [None if x is None else x.clone() for x in xs]  # noqa: E731
+    return [(clone(g), clone(q), m.clone()) for g, q, m in items]
+
+
+def _ladder(monkeypatch):
+    """An empty ladder memory; returns the list that the calls of the factorisation are added to as (matrices, rounds)."""
+    from heavyball_b200.utils import orthogonal
+
+    calls, run = [], orthogonal._cholesky_qr2_replayed
+    monkeypatch.setattr(orthogonal, "_cholesky_qr2_replayed", lambda x, rounds=0: calls.append((x.shape[0], rounds)) or run(x, rounds))
+    monkeypatch.setattr(orthogonal, "_cholqr_level", {})
+    monkeypatch.setattr(orthogonal, "_cholqr_wins", {})
+    return calls
+
+
+@pytest.mark.parametrize("limit", [None, 256 * 256 * 5, 1])
+def test_eigenbases_of_several_buckets_refresh_together(limit, monkeypatch):
+    """One joint refresh of three buckets (shared sizes, one factor missing) against the bucket-by-bucket definition; ``limit``:
+    elements of a joint batch (the default, room for two of the three members of one size, room for none)."""
+    from heavyball_b200.utils import soap
+
     gen = torch.Generator(DEV).manual_seed(5)
-
-    def factor(b, n):
-        q = torch.linalg.qr(torch.randn(b, n, n, device=DEV, generator=gen))[0]
-        noise = torch.randn(b, n, n, device=DEV, generator=gen) * 0.02 / n**0.5
-        return (q * torch.logspace(1, 0, n, device=DEV)) @ q.mT + noise + noise.mT, q
-
     items = []
     for b, (r, c) in ((2, (256, 256)), (3, (256, 384)), (1, (384, None))):
-        gl, ql = factor(b, r)
-        gr, qr = factor(b, c) if c else (None, None)
+        gl, ql = _factor(gen, b, r)
+        gr, qr = _factor(gen, b, c) if c else (None, None)
         items.append(([gl, gr], [ql, qr], torch.randn(b, r, c or 64, device=DEV, generator=gen)))
-    clone = lambda xs: [None if x is None else x.clone() for x in xs]  # noqa: E731
-    want = [(clone(g), clone(q), m.clone()) for g, q, m in items]
+    want = _copies(items)
     for g, q, m in want:
         utils.get_orthogonal_matrix_QR(g, q, m)
+    if limit is not None:
+        monkeypatch.setattr(soap, "_JOINT_REFRESH_ELEMENTS", limit)
+    calls = _ladder(monkeypatch)
     utils.refresh_eigenbases(items)
+    assert sorted(n for n, _ in calls) == {None: [4, 7], 1: [1, 2, 2, 3, 3]}.get(limit, [1, 3, 3, 4])
     for (_, q, m), (_, q0, m0) in zip(items, want):
         for x, y in zip([*q, m], [*q0, m0]):
             if x is not None:
                 torch.testing.assert_close(x, y, rtol=0, atol=2e-4)
+
+
+@pytest.mark.parametrize("n", [128, 256, 384])
+def test_a_rank_deficient_factor_does_not_change_how_the_others_refresh(n, monkeypatch):
+    """Statistics with rows of zeros (a dead head) in one of three buckets.  The other two take the variants and get the bases that
+    they get without it; n = 128 lies below the whole-matrix factorisation and takes the panel-wise one."""
+    gen = torch.Generator(DEV).manual_seed(n)
+    items = []
+    for b in (2, 1, 3):
+        g, q = _factor(gen, b, n)
+        items.append(([g, None], [q, None], torch.randn(b, n, 64, device=DEV, generator=gen)))
+    items[1][0][0][:, n // 2 :] = 0
+    items[1][0][0][:, :, n // 2 :] = 0
+    want = _copies([items[0], items[2]])
+    for g, q, m in want:
+        utils.get_orthogonal_matrix_QR(g, q, m)
+    calls = _ladder(monkeypatch)
+    eye = torch.eye(n, device=DEV)
+    for again in range(3):  # eager, captured and replayed; the first refresh finds out, the later ones know
+        before, now = len(calls), _copies(items)
+        utils.refresh_eigenbases(now)
+        assert all(size == 1 for size, rounds in calls[before:] if rounds), calls  # only the deficient bucket climbs
+        for (_, q, m), (_, q0, m0) in zip([now[0], now[2]], want):
+            torch.testing.assert_close(q[0], q0[0], rtol=0, atol=2e-5)
+            torch.testing.assert_close(m, m0, rtol=0, atol=2e-4)
+            assert (q[0].mT @ q[0] - eye).abs().max().item() < 1e-4
+        assert all(torch.isfinite(q[0]).all() for _, q, _ in now)

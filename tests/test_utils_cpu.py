@@ -332,3 +332,48 @@ def test_smallest_eigenvalue_of_a_symmetric_psd_matrix(n, decades, dtype, rtol):
     want = float(torch.linalg.eigvalsh(a.double()).min())
     got = float(utils.min_singular_value(a, power_iter=20))
     assert abs(got - want) <= rtol * want + 1e-5
+
+
+def test_batches_refreshed_together_are_accepted_or_refused_one_by_one(monkeypatch):
+    """Three batches share a refresh and one of them holds a matrix that needs a shifted variant: only that batch climbs, the
+    others keep the plain variant's result and their place on the ladder, and afterwards each takes its own route until all
+    stand on one step again.  The factorisation is replaced by one that refuses matrices by their scale."""
+    from heavyball_b200.utils import orthogonal as O
+
+    calls = []
+
+    def factor(x, rounds=0):
+        calls.append((x.shape[0], rounds))
+        need = x.abs().amax(dim=(-2, -1)).log10().div(3).floor()  # 1e3: one shifted round, 1e6: three, 1e9: none suffices
+        return torch.linalg.qr(x).Q * (1 + rounds), (need > torch.tensor({0: 0, 1: 1, 3: 2}[rounds])).int()
+
+    monkeypatch.setattr(O, "_cholesky_qr2_replayed", factor)
+    monkeypatch.setattr(O, "_cholqr_applies", lambda x: True)
+    for name in ("_cholqr_level", "_cholqr_wins"):
+        monkeypatch.setattr(O, name, {})
+    monkeypatch.setattr(O, "qr_stats", dict.fromkeys(O.qr_stats, 0))
+    torch.manual_seed(0)
+    sizes = [2, 1, 3]
+    x = torch.randn(6, 8, 8)
+    q = torch.linalg.qr(x).Q
+    keep = torch.linalg.qr(torch.randn(6, 8, 8)).Q
+
+    assert torch.equal(O._qr_bases(x, keep, sizes), q) and calls == [(6, 0)]  # all easy: one chain
+    calls.clear()
+    x[2] *= 2e3  # the single matrix of the second batch
+    out = O._qr_bases(x, keep, sizes)
+    assert calls == [(6, 0), (1, 1)]
+    assert torch.equal(out[:2], q[:2]) and torch.equal(out[3:], q[3:])  # bit for bit what they are without it
+    torch.testing.assert_close(out[2], 2 * q[2])
+    level = lambda n: O._cholqr_level[(x.device, (n, 8, 8))]  # noqa: E731
+    assert (level(2), level(1), level(3)) == (0, 1, 0)
+    assert O.qr_stats == {"cholesky_qr2": 5, "cholesky_qr_shifted_1": 1, "cholesky_qr_shifted_3": 0, "cholesky_qr2_rejected": 0}
+    calls.clear()
+    out = O._qr_bases(x, keep, sizes)  # different steps: each alone, on its own
+    assert calls == [(2, 0), (1, 1), (3, 0)]
+    assert torch.equal(out[:2], q[:2]) and torch.equal(out[3:], q[3:])
+    calls.clear()
+    x[2] *= 1e9  # beyond the ladder: the fallback route, alone
+    out = O._qr_bases(x, keep, sizes)
+    assert calls == [(2, 0), (1, 1), (1, 3), (3, 0)] and O.qr_stats["cholesky_qr2_rejected"] == 1
+    torch.testing.assert_close(out, q)
