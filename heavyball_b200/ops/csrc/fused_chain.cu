@@ -6,17 +6,19 @@
 // 736-776 momentum, 3616-3627 MARS, 2373-2406 parameter update, 3652-3658 caution).  Arithmetic is
 // restated from heavyball_b200/utils/first_order.py, which is also the test oracle.
 //
-// Work decomposition: tensors are cut into CHUNK-element chunks; block b owns chunk b and finds its
-// tensor by binary search in a prefix table.  All tensor addresses come from a device-resident table,
-// so the launch count is independent of the number of tensors.
+// Work decomposition: tensors are cut into chunks (chain_chunks.h); block b owns chunk b, and its warps find the tensor in a
+// table of prefix sums, 32 entries at a time (find_range).  All tensor addresses come from a device-resident table, so the
+// launch count is independent of the number of tensors.
+//
+// Two kernels: the general one below takes every storage kind, rule and destination from run-time parameters; the specialised
+// instances after it (Kinds) cover the launches that most steps consist of.
+#include "chain_chunks.h"
 #include "common.cuh"
 #include "fused_chain.h"
 
 namespace hb {
 
 constexpr int kThreads = 256;
-constexpr int kChunk = 8192;      // elements per block
-constexpr int kSmallChunk = 2048;  // ... of launches too small to fill the machine with those
 
 // Random bits are only generated for storage kinds that consume them (bf16 rounding, ECC residuals).
 __device__ inline uint4 draw(int dt, const Philox& rng, uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) {
@@ -611,14 +613,19 @@ using Kinds = KindList<
 
 using PlainLaunch = void (*)(const TensorMeta*, const int*, ChainParams);
 
-// The first specialised instance that covers the launch; null when the general kernel has to run it.
+struct PlainKind {
+  PlainLaunch kernel = nullptr;
+  int vectors = 0;  // in flight per thread
+};
+
+// The first specialised instance that covers the launch; without a kernel when the general one has to run it.
 template <class... Ks>
-PlainLaunch find_kind(KindList<Ks...>, const ChainParams& P, bool count) {
+PlainKind find_kind(KindList<Ks...>, const ChainParams& P, bool count) {
   const bool plain = P.n_state <= 2 && P.algo != kAdemamix && P.n_src == 0 && P.n_dst == 0 && P.g_clip_mode == kClipNone &&
                      (P.u_op == kUopNone || (P.u_op == kUopTrustRegion && P.u_is_input)) && P.post_state == kPostNone && P.out_mode != kOutScheduleFree &&
                      (!P.u_is_input || (P.algo == kIdentity && P.n_state == 0 && !P.mars)) && !(count && P.accum_sumsq);
-  PlainLaunch hit = nullptr;
-  if (plain) ((hit == nullptr && Ks::takes(P, count) ? (void)(hit = plain_chain_kernel<Ks>) : (void)0), ...);
+  PlainKind hit;
+  if (plain) ((hit.kernel == nullptr && Ks::takes(P, count) ? (void)(hit = {plain_chain_kernel<Ks>, Ks::batch}) : (void)0), ...);
   return hit;
 }
 
@@ -627,9 +634,8 @@ PlainLaunch find_kind(KindList<Ks...>, const ChainParams& P, bool count) {
 int chain_chunk_elems() { return kChunk; }
 
 int chain_chunk_elems_for(const ChainParams& P, bool count_caution, int64_t total_elems) {
-  // below two blocks of the default size per resident slot the machine is not filled, and a block's dependent iterations
-  // are what the launch takes: cut the work finer
-  return total_elems <= (int64_t)kChunk * 148 * 4 * 2 && find_kind(Kinds{}, P, count_caution) != nullptr ? kSmallChunk : kChunk;
+  const PlainKind kind = find_kind(Kinds{}, P, count_caution);
+  return kind.kernel != nullptr ? chain_chunk(kind.vectors, total_elems) : kChunk;
 }
 
 cudaError_t launch_fused_chain(const TensorMeta* metas, const int* chunk_prefix, int total_chunks, const ChainParams& P0,
@@ -637,7 +643,7 @@ cudaError_t launch_fused_chain(const TensorMeta* metas, const int* chunk_prefix,
   if (total_chunks <= 0) return cudaSuccess;
   ChainParams P = P0;
   if (P.chunk == 0) P.chunk = kChunk;
-  if (const PlainLaunch kernel = find_kind(Kinds{}, P, count_caution))
+  if (const PlainLaunch kernel = find_kind(Kinds{}, P, count_caution).kernel)
     kernel<<<total_chunks, kThreads, 0, stream>>>(metas, chunk_prefix, P);
   else if (P.chunk != kChunk)
     return cudaErrorInvalidValue;  // the general kernel is compiled for one chunk size

@@ -15,9 +15,11 @@ DEV = "cuda"
 
 
 @pytest.mark.parametrize("kw", [{}, {"ecc": "bf16+8", "mars": True, "caution": True}, {"ecc": "bf16+8"}, {"caution": True}], ids=str)
-@pytest.mark.parametrize("sizes", [(1,), (2047, 2048, 2049), (8191, 8193, 3, 16384), tuple(range(1, 41)), (10_000_000, 5)], ids=len)
+@pytest.mark.parametrize("sizes", [(1,), (2047, 2048, 2049), (8191, 8193, 3, 16384), tuple(range(1, 41)), (10_000_000, 5),
+                                   (4095, 4096, 4097, 2_500_001, 7), (8191, 8192, 8193, 1, 10_000_000, 5)], ids=len)  # fmt: skip
 def test_fused_chain_at_chunk_edges(sizes, kw):
-    """Sizes around both chunk sizes, more tensors than a warp tests at once, and a launch large enough for the large chunk.
+    """Sizes around the three chunk sizes in launches of the size that takes each (2048 up to 0.9 M or 2.4 M elements, 8192 from
+    4.8 M or 9.7 M), more tensors than a warp tests at once, and a launch large enough for the large chunk.
     fp32: a handful of roundings per step (1e-6 of the value); error-corrected state keeps 16 + 8 bits (2^-15 of the value)
     and moves a weight by lr = 1e-2 per step."""
     results = []

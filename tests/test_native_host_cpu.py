@@ -156,6 +156,30 @@ int main() {
 """)
 
 
+def test_fused_chain_chunk_sizes(tmp_path):
+    """Sizes at which one chunk was measured to be clearly the fastest, for the three numbers of vectors in flight."""
+    _run(tmp_path, r"""
+#include <cstdio>
+#include <initializer_list>
+#include "chain_chunks.h"
+int bad = 0;
+void expect(int vectors, long long elems, int chunk) {
+  const int got = hb::chain_chunk(vectors, elems);
+  if (got != chunk) { printf("%d vectors, %lld elements: %d\n", vectors, elems, got); ++bad; }
+}
+int main() {
+  for (int vectors : {1, 2, 4}) { expect(vectors, 1, 2048); expect(vectors, 600000, 2048); expect(vectors, 14000000, 8192); }
+  expect(1, 1200000, 2048);
+  expect(2, 4800000, 4096);
+  expect(4, 1200000, 4096);
+  expect(4, 4800000, 4096);
+  expect(4, 7000000, 8192);
+  expect(4, 9600000, 8192);
+  return bad;
+}
+""")
+
+
 @pytest.mark.gpu
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_tensor_core_and_leaf_kernels_run_on_a_second_device_of_the_process():
