@@ -43,21 +43,67 @@ def test_fused_chain_at_chunk_edges(sizes, kw):
         assert close.float().mean().item() > (0.999 if kw.get("caution") and a.numel() > 1000 else 1 - 1e-9), (a - b).abs().max()
 
 
-def test_ecc_codec_over_all_exponents():
-    """State values over the whole exponent range (both sides of the codec's exponent threshold, zeros and subnormals): a step
-    with zero gradient and momentum coefficient 1 - eps decodes, scales and encodes each value once."""
-    exps = torch.arange(-148, 120, device=DEV, dtype=torch.float64)
-    value = torch.cat([torch.zeros(4, device=DEV, dtype=torch.float64), (2.0**exps) * 1.37, -(2.0**exps) * 1.91]).float()
-    prim = value.to(torch.bfloat16)
-    res = torch.randint(-127, 128, value.shape, device=DEV, dtype=torch.int8)
-    out = torch.empty_like(value)
-    ops.fused_chain(g=[torch.zeros_like(value)], u=[out], s0=[prim], s0e=[res], algo=ops.EXP_AVG, n_state=1, b1=1.0,
+def _ecc_step(g, prim, res, b1, shift):
+    """One momentum step (``s <- s b1 + g``) on error-corrected state; returns what it hands on and the stored pair.  ``shift``:
+    elements by which every buffer starts past a 16-byte boundary."""
+    place = lambda t: torch.cat([t[:1].expand(shift), t])[shift:] if shift else t.clone()  # noqa: E731
+    g, prim, res, out = place(g), place(prim), place(res), place(torch.zeros_like(g))
+    ops.fused_chain(g=[g], u=[out], s0=[prim], s0e=[res], algo=ops.HEAVYBALL, n_state=1, b1=b1, seed=11,
                     out_mode=ops.OUT_UPDATE, dt_g=ops.F32, dt_u=ops.F32, dt_s=ops.BF16E8, dt_p=ops.NONE)  # fmt: skip
-    # half a unit in the last place of a bf16 value, times residual / 127
-    e = torch.clamp(torch.frexp(prim.double())[1] - 1, min=-126).double()
-    want = prim.double() + (res.double() / 127) * 2.0 ** (e - 8)
-    big = want.abs() > 1e-30
-    torch.testing.assert_close(out[big].double(), want[big], rtol=1e-6, atol=0)
+    return out, prim, res
+
+
+def _ecc_value(prim, res):
+    """The pair's value in 64 bits, and its unit: half a unit in the last place of the primary, over 127."""
+    e = torch.where(prim == 0, -126, torch.clamp(torch.frexp(prim.double())[1] - 1, min=-126)).double()
+    unit = 2.0 ** (e - 8) / 127
+    return prim.double() + res.double() * unit, unit
+
+
+_FLUSH = 2.0**-126  # single-precision subnormals count as zero in these kernels
+
+
+@pytest.mark.parametrize("shift", [0, 1], ids=["four at a time", "one at a time"])
+def test_ecc_codec_decodes_every_primary(shift):
+    """All 65536 primaries (zeros, subnormals, infinities and NaN among them) under random residuals: the value handed on is the
+    pair's to fp32 rounding, and the pair that is stored for it again is within one residual unit of it."""
+    prim = torch.arange(-32768, 32768, device=DEV, dtype=torch.int32).to(torch.int16).view(torch.bfloat16)
+    prim = prim[torch.randperm(65536, generator=torch.Generator().manual_seed(1)).to(DEV)]
+    res = torch.randint(-127, 128, prim.shape, device=DEV, dtype=torch.int8, generator=torch.Generator(DEV).manual_seed(2))
+    out, new, left = _ecc_step(torch.zeros(65536, device=DEV), prim, res, 1.0, shift)
+    finite = torch.isfinite(prim)
+    want, unit = _ecc_value(prim, res)
+    assert ((out.double() - want).abs() <= want.abs() * 1e-6 + _FLUSH)[finite].all()
+    again, _ = _ecc_value(new, left)
+    held = finite & torch.isfinite(new)  # the largest value plus its residual rounds up to infinity
+    assert (finite & ~held).sum().item() <= 2
+    assert ((again - out.double()).abs() <= unit * 1.001 + 2 * _FLUSH)[held].all()
+    assert torch.equal(torch.isnan(out), torch.isnan(prim)) and torch.equal(torch.isnan(new), torch.isnan(prim))
+    assert torch.equal(out[torch.isinf(prim)], prim[torch.isinf(prim)].float()) and torch.equal(new[torch.isinf(prim)], prim[torch.isinf(prim)])
+
+
+def test_ecc_codec_encodes_the_same_bits_four_and_one_at_a_time():
+    """fp32 values of all exponents, ties of the bf16 rounding, the largest ones, infinities and NaN.  The primary is the value
+    rounded to nearest, the pair is within one residual unit of it, and the codec that handles four values at once stores the
+    same bits as the element-wise one (which buffers off a 16-byte boundary take)."""
+    gen = torch.Generator(DEV).manual_seed(3)
+    bits = torch.randint(-(2**31), 2**31, (1 << 17,), device=DEV, generator=gen)
+    ties = (torch.arange(0, 65536, 7, device=DEV) << 16 | 0x8000) - 2**31
+    edge = torch.tensor([0x7F7F0000, 0x7F7F7FFF, 0x7F7F8000, 0x7F800000, 0x7FC00000, 0x00800000, 0x007FFFFF, 1, 0, 0x0FFFFFFF, 0x10000000], device=DEV)
+    x = torch.cat([bits, ties, edge, edge - 2**31]).to(torch.int32).view(torch.float32)
+    zero, none = torch.zeros(x.shape, device=DEV, dtype=torch.bfloat16), torch.zeros(x.shape, device=DEV, dtype=torch.int8)
+    out, prim, res = _ecc_step(x, zero, none, 0.0, 0)
+    one_out, one_prim, one_res = _ecc_step(x, zero, none, 0.0, 1)
+    number = ~torch.isnan(x)
+    assert torch.equal(torch.isnan(prim), ~number) and torch.equal(torch.isnan(one_prim), ~number)
+    assert torch.equal(out[number], one_out[number])
+    assert torch.equal(prim.view(torch.int16)[number], one_prim.view(torch.int16)[number]) and torch.equal(res[number], one_res[number])
+    normal = number & (x.abs() >= _FLUSH)
+    assert torch.equal(prim[normal], x.to(torch.bfloat16)[normal])
+    value, unit = _ecc_value(prim, res)
+    held = torch.isfinite(prim) & number
+    assert ((value - x.double()).abs() <= unit * 1.001 + 2 * _FLUSH)[held].all()
+    assert res[held].to(torch.int32).abs().max().item() <= 127
 
 
 # ---------------------------------------------------------------------------------------- Newton-Schulz products
