@@ -1,9 +1,9 @@
 """Profiler ranges around the stages of a lowered optimizer step.
 
 Off by default (a no-op costing one attribute test per stage).  ``HB200_NVTX=1`` in the environment, or
-``tracing.enable()``, pushes an NVTX range per stage - ``momentum``, ``ns/<rows>x<cols>``, ``update``, ``soap.project``,
-``soap.refresh``, ``psgd.apply``, ``psgd.fit``, ``peer.begin``, ``peer.end`` - so a timeline shows where a step spends its
-time.  The ranges are also recorded by ``torch.profiler`` (as user annotations) when it is active.
+``tracing.enable()``, pushes an NVTX range per stage - ``momentum``, ``newton_schulz`` and ``soap.refresh`` (all shape buckets
+together), ``soap.project``, ``psgd.apply`` and ``psgd.fit`` (one per bucket), ``update``, ``peer.begin``, ``peer.end`` - so a
+timeline shows where a step spends its time.  The ranges are also recorded by ``torch.profiler`` (as user annotations) when it is active.
 """
 
 from __future__ import annotations

@@ -151,6 +151,26 @@ def test_grouped_newton_schulz_step(tile, shapes):
         assert (y.double() - want).norm() / want.norm() < 2**-9
 
 
+def test_stage_ranges_of_a_muon_step():
+    """The names that a profiler filter would look for: one range each, whatever the number of shape buckets."""
+    from heavyball_b200.utils import tracing
+
+    params = [torch.nn.Parameter(torch.randn(s, device=DEV)) for s in ((64, 128), (96, 64), (128, 128))]
+    opt = hb.Muon(params, lr=1e-2)
+    for step in range(2):  # the first step creates the state
+        for p in params:
+            p.grad = torch.randn_like(p)
+        if step:
+            tracing.enable(True, record=True)
+            tracing.seen.clear()
+        try:
+            opt.step()
+        finally:
+            tracing.enable(False)
+    assert tracing.seen == ["momentum", "newton_schulz", "update"]
+    tracing.seen.clear()
+
+
 # ---------------------------------------------------------------------------------------- triangular leaves
 
 
