@@ -3,6 +3,7 @@
     python benchmarks/profile_targets.py opt_step_gpt2   # 3 optimizer steps, GPT-2-small parameter shapes
     python benchmarks/profile_targets.py ns_small        # Newton-Schulz on 8 x (1024 x 4096) bf16-sized work
     python benchmarks/profile_targets.py adam_small      # fused AdamW over 64M fp32 parameters (768 MB state+params)
+    python benchmarks/profile_targets.py chain_small     # adam_small, then cautious AdamW + MARS, error-corrected state, 8 x 2048^2
     python benchmarks/profile_targets.py ce_small        # cross-entropy fwd+bwd kernel, 4096 x 50304 bf16 logits (412 MB)
     python benchmarks/profile_targets.py ln_small        # LayerNorm fwd + bwd kernels, 16384 x 768 fp32 (50 MB) x 4 tensors
     python benchmarks/profile_targets.py gelu_small      # GELU fwd, and bwd + bias gradient, 16384 x 3072 bf16 (100 MB per tensor)
@@ -13,6 +14,7 @@
     python benchmarks/profile_targets.py psgd_small      # one plain PSGDKron step on 8 x 1024^2 (cached P = Q^T Q operands)
     python benchmarks/profile_targets.py psgd_fit        # one PSGDKron step with a preconditioner fit, 8 x (1024 x 4096)
     python benchmarks/profile_targets.py soap_refresh    # one SOAP step with an eigenbasis refresh, 8 x (2048 x 2048)
+    python benchmarks/profile_targets.py launches NAME,. # device time by kernel of workloads of perf/cases.py (torch.profiler)
 
 Each case holds well under a few GB on the device and launches only a handful of kernels.
 """
@@ -78,6 +80,56 @@ def adam_small():
     opt.step()
     torch.cuda.synchronize()
     torch.cuda.profiler.stop()
+
+
+def chain_small():
+    adam_small()
+    params = [torch.nn.Parameter(torch.randn(2048, 2048, device="cuda")) for _ in range(8)]
+    opt = hb.AdamW(params, lr=1e-3, weight_decay=0.01, ecc="bf16+8", mars=True, caution=True, consume_grad=False)
+    for p in params:
+        p.grad = torch.randn_like(p)
+    for _ in range(3):
+        opt.step()
+    torch.cuda.synchronize()
+    torch.cuda.profiler.start()
+    opt.step()
+    torch.cuda.synchronize()
+    torch.cuda.profiler.stop()
+
+
+def launches():
+    """For each workload: the host's time to issue a pass, the time of a pass among others, and the device's time by kernel."""
+    import time
+
+    from torch.profiler import ProfilerActivity, profile
+
+    from perf import cases
+
+    by_name, passes = {c["name"]: c for c in cases.listed()}, 20
+    for name in sys.argv[2].split(","):
+        state = cases.prepare(by_name[name], 1)
+        for _ in range(12):
+            cases.run(state)
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        for _ in range(passes):
+            cases.run(state)
+        t1 = time.perf_counter()
+        torch.cuda.synchronize()
+        t2 = time.perf_counter()
+        with profile(activities=[ProfilerActivity.CUDA]) as prof:
+            cases.run(state)
+            torch.cuda.synchronize()
+        spans = sorted((e.time_range.start, e.time_range.end, e.name) for e in prof.events() if e.device_type == torch.autograd.DeviceType.CUDA)
+        busy, last, kernels = 0.0, float("-inf"), {}
+        for start, end, kernel in spans:
+            busy += max(0.0, end - max(start, last))
+            last = max(last, end)
+            n, us = kernels.get(kernel, (0, 0.0))
+            kernels[kernel] = n + 1, us + end - start
+        print(f"{name}: host {(t1 - t0) / passes * 1e6:.0f} us, pass {(t2 - t0) / passes * 1e6:.0f} us; {len(spans)} launches, device busy {busy:.0f} us")
+        for kernel, (n, us) in sorted(kernels.items(), key=lambda kv: -kv[1][1])[:12]:
+            print(f"  {us:9.1f} us {n:5d} x {us / n:7.2f} us  {kernel[:100]}")
 
 
 def _timed(fn, reps=5):
@@ -283,5 +335,5 @@ def soap_refresh():
 
 
 if __name__ == "__main__":
-    {"psgd_fit": psgd_fit, "soap_refresh": soap_refresh, "ns_big": ns_big, "soap_small": soap_small, "psgd_small": psgd_small, "qr_small": qr_small, "opt_step_gpt2": opt_step_gpt2, "ns_small": ns_small, "adam_small": adam_small, "ce_small": ce_small,
+    {"psgd_fit": psgd_fit, "soap_refresh": soap_refresh, "ns_big": ns_big, "soap_small": soap_small, "psgd_small": psgd_small, "qr_small": qr_small, "opt_step_gpt2": opt_step_gpt2, "ns_small": ns_small, "adam_small": adam_small, "chain_small": chain_small, "launches": launches, "ce_small": ce_small,
      "ln_small": ln_small, "tf32_small": tf32_small, "gelu_small": gelu_small}[sys.argv[1]]()

@@ -341,7 +341,9 @@ __global__ void __launch_bounds__(kThreads, 4) fused_chain_kernel(const TensorMe
 // constants, and a kind's batch of vectors per thread is loaded before anything is computed or stored (stores may alias later loads,
 // so the compiler cannot move those up by itself: a vector at a time is a memory round trip each).  Against the general kernel:
 // AdamW on the 39.5 M fp32 parameters of GPT-2-small's embeddings 242 -> 170 us (6.5 TB/s), cautious AdamW with error-corrected
-// state on 8 x 2048^2 965 -> 562 us, and 357 us with the loads separated from the codec.
+// state on 8 x 2048^2 965 -> 562 us, and 353 us with the loads separated from the codec.
+// Storage kinds outside the list below (fp16, 16-bit residuals, plain bf16 state, bf16 gradients into an update with fp32 state or
+// without state), peers, clips and the other launches named here run the general kernel at its speed.
 // ---------------------------------------------------------------------------------------------
 // One rule with at most two states on one element: advances the states and returns the new direction.
 template <int A>
@@ -389,13 +391,15 @@ struct ChainKind {
   static constexpr bool reads_g = !u_in || count, reads_p = OUT == kOutParam;
   // Vectors per thread loaded together, and blocks per SM.  Two vectors through a rule need about 80 registers: three blocks.
   // The codec and its random bits are 190 instructions per element and want warps rather than vectors in flight: with
-  // error-corrected state one vector is as many as fit (momentum of a Llama-3-8B layer 1.76 -> 1.32 ms at one vector and four
-  // blocks; the three arrays of cautious Adam with MARS 295 us at two vectors and two blocks, 307 at one and four, 285 at one
+  // error-corrected state one vector is as many as fit (momentum of a Llama-3-8B layer by itself 1.76 -> 1.32 ms at one vector
+  // and four blocks, 1.65 at three; the three arrays of cautious Adam with MARS 295 us at two vectors and two blocks, 307 at one and four, 285 at one
   // and three).
   static constexpr bool ecc = DTS == kBF16E8;
   // Otherwise a thread should have about 128 bytes on their way: two vectors of Adam's four arrays, four where a launch reads
   // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 288 us with two vectors,
-  // 250 with four, of which the bytes take 204 at 6.65 TB/s).
+  // 250 with four, of which the bytes take 207 at 6.54 TB/s).
+  // The momentum kinds spill at these counts (60 to 148 bytes per thread; the others at most 20): the times above are with
+  // the spills, and the counts that spill 12 bytes or nothing are the slower ones.
   static constexpr int batch = ecc ? 1 : (state && (reads_p || count) ? 2 : 4);
   static constexpr int min_blocks = state && !(ecc && !count) ? 3 : 4;
   static bool takes(const ChainParams& P, bool counting) {

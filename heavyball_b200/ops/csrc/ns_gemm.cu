@@ -9,7 +9,7 @@
 // X as it lies in memory ([K, N], N contiguous) through an MN-major B descriptor, so the iterate exists once and no
 // transposed copy of it is ever written (half of the bytes of every apply epilogue and of the prologue; GPT-2-small's
 // 48 matrices: 2634 -> 2513 us, a Llama-3-8B layer: 19.97 -> 18.71 ms).  The three differ only in the B box, its descriptor
-// and the epilogue.  Two kernels share them: 128 x 128 tiles for small matrices, 256 x 256 tiles on CTA pairs for large ones.
+// and the epilogue.  Two kernels share them: 128 x 128 tiles, and 256 x 256 tiles on CTA pairs for large launches (ns_tiles.h).
 //
 // Kernel structure (one 128x128 output tile per CTA, 192 threads, two CTAs resident per SM so one
 // CTA's epilogue overlaps the other's main loop):
