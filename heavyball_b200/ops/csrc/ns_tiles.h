@@ -5,9 +5,9 @@
 //   - The 128 x 128 tiles fit at once: up to 1.7 times as fast, at most 2 % slower.  Gram products, 128 / pairs:
 //     8 of 512 x 512 8.5 / 12.1 us, 16 of 640 x 1920 18.4 / 31.8, 8 of 1024 x 1024 14.2 / 22.9, 2 of 2048 x 2048 22.6 / 24.7.
 //   - They need more than one wave: pairs are as fast or faster, in the same number of waves or up to a third more (apply
-//     products, 32 of 900 x 1300: 152.7 / 91.7 us).  All 15 products of GPT-2-small's 48 matrices: 128 / 98 us per launch, of a Llama-3-8B layer
-//     1.04 / 0.81 ms.  With half as many waves again they are not: 16 of 1024 x 1024 in two waves of small tiles or three of
-//     pairs 25.7 / 30.4 us, 20 of 640 x 640 18.2 / 21.3.
+//     products, 32 of 900 x 1300: 152.7 / 91.7 us).  All 15 products of GPT-2-small's 48 matrices: 128 / 98 us per launch, of a
+//     Llama-3-8B layer 1.04 / 0.81 ms.  With half as many waves again they are not: 16 of 1024 x 1024 in two waves of small tiles
+//     or three of pairs 25.7 / 30.4 us, 20 of 640 x 640 18.2 / 21.3.
 //   - Rows along a long K that do not start on 128-byte lines: with two CTAs on an SM the small tile pays for its greater operand
 //     traffic (6 of 900 x 1300 24.6 / 19.3 us, 3 of 1500 x 1700 34.0 / 25.1), and in every wave.  At K below 800 it still wins
 //     (8 of 700 x 700 10.2 / 12.5).  Between 100 and 148 tiles it is faster by itself, but the apply product after it is then
