@@ -6,6 +6,7 @@
 
 #include <algorithm>
 #include <optional>
+#include <string>
 #include <vector>
 
 #include "colsum.h"
@@ -92,22 +93,22 @@ void fused_chain(const TList& p, const TList& pe, const TList& g, const TList& u
                           {&s2, "s2", ds, false}, {&s2e, "s2e", ds, true}, {&mars, "mars", ds, false}, {&marse, "marse", ds, true}};
     for (const Slot& sl : slots) {
       if (sl.list->empty()) continue;
-      TORCH_CHECK(sl.list->size() == n, "fused_chain: list '", sl.name, "' has ", sl.list->size(), " entries, expected ", n);
+      TORCH_CHECK(sl.list->size() == n, "fused_chain: list '", sl.name, "' has ", std::to_string(sl.list->size()), " entries, expected ", std::to_string(n));
       const int want = sl.residual ? residual_bytes(sl.dt) : primary_bytes(sl.dt);
       for (size_t i = 0; i < n; ++i) {
         const OptT& t = (*sl.list)[i];
-        TORCH_CHECK(t.has_value() && t->defined(), "fused_chain: '", sl.name, "'[", i, "] is missing");
-        TORCH_CHECK(t->is_cuda() && t->device() == ref.device() && t->is_contiguous(), "fused_chain: '", sl.name, "'[", i,
+        TORCH_CHECK(t.has_value() && t->defined(), "fused_chain: '", sl.name, "'[", std::to_string(i), "] is missing");
+        TORCH_CHECK(t->is_cuda() && t->device() == ref.device() && t->is_contiguous(), "fused_chain: '", sl.name, "'[", std::to_string(i),
                     "] must be a contiguous CUDA tensor on the launch device");
-        TORCH_CHECK(want != 0 && (int)t->element_size() == want, "fused_chain: '", sl.name, "'[", i, "] has ", t->element_size(),
-                    "-byte elements, its storage kind needs ", want);
+        TORCH_CHECK(want != 0 && (int)t->element_size() == want, "fused_chain: '", sl.name, "'[", std::to_string(i), "] has ", std::to_string(t->element_size()),
+                    "-byte elements, its storage kind needs ", std::to_string(want));
       }
     }
     for (const at::Tensor* aux : {scale.has_value() ? &*scale : nullptr, masked.has_value() ? &*masked : nullptr}) {
       if (aux == nullptr) continue;
       const size_t per = aux == (scale.has_value() ? &*scale : nullptr) ? (size_t)scale_stride : 1;
       TORCH_CHECK(aux->is_cuda() && aux->is_contiguous() && (size_t)aux->numel() >= n * per && aux->element_size() == 4,
-                  "fused_chain: per-tensor scalars need ", per, " 4-byte entries per tensor");
+                  "fused_chain: per-tensor scalars need ", std::to_string(per), " 4-byte entries per tensor");
     }
     if (gsq.has_value())
       TORCH_CHECK(gsq->is_cuda() && gsq->is_contiguous() && gsq->scalar_type() == at::kFloat &&
@@ -133,7 +134,7 @@ void fused_chain(const TList& p, const TList& pe, const TList& g, const TList& u
     const at::Tensor& any = !g.empty() && g[i].has_value() ? *g[i] : (!u.empty() && u[i].has_value() ? *u[i] : *p[i]);
     m.numel = any.numel();
     for (const TList* l : {&p, &pe, &g, &u, &s0, &s0e, &s1, &s1e, &s2, &s2e, &mars, &marse})
-      TORCH_CHECK(l->empty() || (*l)[i]->numel() == m.numel, "fused_chain: buffers of tensor ", i, " differ in element count");
+      TORCH_CHECK(l->empty() || (*l)[i]->numel() == m.numel, "fused_chain: buffers of tensor ", std::to_string(i), " differ in element count");
     bool ok = true;
     for (void* q : {m.p, m.pe, m.g, m.u, m.s0, m.s0e, m.s1, m.s1e, m.s2, m.s2e, m.mars, m.marse}) ok = ok && aligned16(q);
     m.vec_ok = ok ? 1 : 0;
@@ -409,7 +410,7 @@ at::Tensor tf32_gemm(const at::Tensor& a2, const at::Tensor& b2, int64_t K, int 
                   a2.dim() == 3 && b2.dim() == 3 && a2.is_contiguous() && b2.is_contiguous() && a2.size(0) == b2.size(0),
               "tf32_gemm: contiguous fp32 split operands [batch, rows, 2 kp]");
   const int64_t batch = a2.size(0), M = a2.size(1), N = b2.size(1), kp = hb::tf32_split_kp(K);
-  TORCH_CHECK(a2.size(2) == 2 * kp && b2.size(2) == 2 * kp, "tf32_gemm: operands were not split for K = ", K);
+  TORCH_CHECK(a2.size(2) == 2 * kp && b2.size(2) == 2 * kp, "tf32_gemm: operands were not split for K = ", std::to_string(K));
   c10::cuda::CUDAGuard guard(a2.device());
   hb::Tf32Epilogue E{};
   E.mode = mode; E.alpha = (float)alpha; E.w = (float)w; E.b1 = (float)b1; E.b2 = (float)b2c; E.eps = (float)eps;
