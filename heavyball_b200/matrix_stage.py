@@ -80,34 +80,42 @@ class TorchBackend:
             return _TorchOperand(acc.transpose(-1, -2))
         return None
 
-
-class _SplitOperand:
-    __slots__ = ("data", "K")
-
-    def __init__(self, data, K):
-        self.data, self.K = data, K
+    @staticmethod
+    def statistics(x: Tensor, left: Optional[Tensor], right: Optional[Tensor], w: float):
+        for outer, target in ((lambda: x @ x.mT, left), (lambda: x.mT @ x, right)):
+            if target is not None:
+                target.add_((outer() - target) * w)
 
 
 class TensorCoreBackend:
-    """Split-tf32 tcgen05 GEMM with fused epilogues (``ops.tf32_split`` / ``ops.tf32_gemm``)."""
+    """fp16-pair tcgen05 GEMM with fused epilogues (``ops.split16`` / ``ops.split16_gemm``)."""
 
     name = "tcgen05"
 
     @staticmethod
     def operands(x: Tensor, same: bool = True, trans: bool = False):
-        x = x if x.is_contiguous() else x.contiguous()
-        s, t = ops.tf32_split(x, same, trans)
-        return (_SplitOperand(s, x.shape[-1]) if same else None), (_SplitOperand(t, x.shape[-2]) if trans else None)
+        return ops.split16(x if x.is_contiguous() else x.contiguous(), same, trans)
 
     @staticmethod
     def gemm(a, b, *, mode=ops.EPI_STORE, alpha=1.0, w=0.0, b1=0.0, b2=0.0, eps=0.0, out=None, split_out=ops.SPLIT_NONE,
              m=None, v=None):  # fmt: skip
-        s = ops.tf32_gemm(a.data, b.data, a.K, mode=mode, alpha=alpha, w=w, b1=b1, b2c=b2, eps=eps, out=out,
-                          split_out=split_out, m=m, v=v)  # fmt: skip
+        if out is None:  # rows start on 16-byte boundaries
+            rows, cols = a.data.shape[1], b.data.shape[1]
+            out = torch.empty(a.data.shape[0], rows, -(-cols // 4) * 4, device=a.data.device)[..., :cols]
+        ops.split16_gemm(a, b, mode=mode, alpha=alpha, w=w, b1=b1, b2c=b2, eps=eps, out=out, m=m, v=v)
         if split_out == ops.SPLIT_NONE:
             return None
-        M, N = a.data.shape[1], b.data.shape[1]
-        return _SplitOperand(s, N if split_out == ops.SPLIT_ROWS else M)
+        by_rows = split_out == ops.SPLIT_ROWS
+        return ops.split16(out, by_rows, not by_rows)[0 if by_rows else 1]
+
+    @staticmethod
+    def statistics(x: Tensor, left: Optional[Tensor], right: Optional[Tensor], w: float):
+        """``left <- lerp(left, X X^T)``, ``right <- lerp(right, X^T X)``, on the split-tf32 product like all that eigenbases come from
+        (see ``utils.core``)."""
+        sides = ops.tf32_split(x, left is not None, right is not None)
+        for side, target, K in zip(sides, (left, right), (x.shape[2], x.shape[1])):
+            if target is not None:
+                ops.tf32_gemm(side, side, K, mode=ops.EPI_LERP, w=w, out=target)
 
 
 def backend_for(t: Tensor, dims: Sequence[int]):
@@ -243,9 +251,7 @@ class SoapBucket:
         mode = ops.EPI_ADAM if self.inner == "adam" else ops.EPI_LAPROP
         adam = dict(mode=mode, b1=b1, b2=b2, eps=eps, m=self.m, v=self.v)
         has_l, has_r = Ql is not None, Qr is not None
-        need_same = has_l or (has_r and not has_l)
-        need_trans = has_l or has_r
-        u_same, u_trans = be.operands(U, need_same, need_trans)
+        u_same, u_trans = be.operands(U, not has_l, has_l)
 
         if has_l and has_r:
             p1 = be.gemm(l_trans, u_trans, split_out=ops.SPLIT_ROWS)                      # Ql^T U
@@ -261,11 +267,10 @@ class SoapBucket:
         else:
             raise RuntimeError("bucket without eigenbases must take the element-wise path")
 
-        # statistics: GG_l <- lerp(GG_l, U U^T), GG_r <- lerp(GG_r, U^T U)
-        if self.GG[0] is not None:
-            be.gemm(u_same, u_same, mode=ops.EPI_LERP, w=stat_w, out=self.GG[0])
-        if len(self.GG) > 1 and self.GG[1] is not None:
-            be.gemm(u_trans, u_trans, mode=ops.EPI_LERP, w=stat_w, out=self.GG[1])
+        right = self.GG[1] if len(self.GG) > 1 else None
+        if self.GG[0] is not None or right is not None:
+            be.statistics(U, self.GG[0], right, stat_w)
+
 
 def refresh(buckets: Sequence["SoapBucket"]):
     """Advances the eigenbases of all buckets of a step together, in place on the adopted state; the orthogonalisation

@@ -17,6 +17,7 @@
 #include "ns_gemm.h"
 #include "peer_sync.h"
 #include "skinny.h"
+#include "split16_gemm.h"
 #include "tf32_gemm.h"
 
 namespace py = pybind11;
@@ -443,6 +444,82 @@ at::Tensor tf32_gemm(const at::Tensor& a2, const at::Tensor& b2, int64_t K, int 
   return s;
 }
 
+// Operands of the fp16-pair product of an fp32 [batch, R, C] tensor (see split16_gemm.h): (same, same_unit, trans, trans_unit); an
+// orientation that was not asked for comes back undefined.
+std::vector<at::Tensor> split16(const at::Tensor& x, bool want_same, bool want_trans) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 3 && x.stride(2) == 1 && x.size(0) >= 1 && x.size(1) >= 1 &&
+                  x.size(2) >= 1 && x.size(0) <= 65535, "split16: fp32 [batch, rows, cols] CUDA tensor with unit inner stride");
+  c10::cuda::CUDAGuard guard(x.device());
+  const int64_t batch = x.size(0), R = x.size(1), C = x.size(2);
+  std::vector<at::Tensor> out(4);
+  hb::Split16Operand op[2] = {};
+  for (int i = 0; i < 2; ++i) {
+    if (!(i == 0 ? want_same : want_trans)) continue;
+    const int64_t rows = i == 0 ? R : C, K = i == 0 ? C : R;
+    out[2 * i] = at::empty({batch, rows, 2 * hb::split16_kp(K)}, x.options().dtype(at::kHalf).memory_format(at::MemoryFormat::Contiguous));
+    out[2 * i + 1] = at::empty({batch, hb::split16_units(rows)}, x.options().memory_format(at::MemoryFormat::Contiguous));
+    op[i] = {out[2 * i].data_ptr(), out[2 * i + 1].data_ptr<float>()};
+  }
+  check(hb::launch_split16(x.data_ptr<float>(), x.stride(1), x.stride(0), (int)R, (int)C, (int)batch, op[0], op[1],
+                           at::cuda::getCurrentCUDAStream()), "split16");
+  return out;
+}
+
+// epilogue(A * B^T) over operands of split16; arguments as for tf32_gemm.  Both operands being one buffer makes the product symmetric.
+void split16_gemm(const at::Tensor& a, const at::Tensor& ua, const at::Tensor& b, const at::Tensor& ub, int64_t K, int mode, double alpha,
+                  double w, double b1, double b2c, double eps, const OptT& c, const OptT& m, const OptT& v, bool upper_upper,
+                  const at::Tensor& status) {
+  TORCH_CHECK(a.is_cuda() && b.is_cuda() && a.scalar_type() == at::kHalf && b.scalar_type() == at::kHalf && a.dim() == 3 && b.dim() == 3 &&
+                  a.is_contiguous() && b.is_contiguous() && a.size(0) == b.size(0) && K >= 1,
+              "split16_gemm: contiguous fp16 operands [batch, rows, 2 kp]");
+  const int64_t batch = a.size(0), M = a.size(1), N = b.size(1), kp = hb::split16_kp(K);
+  TORCH_CHECK(a.size(2) == 2 * kp && b.size(2) == 2 * kp, "split16_gemm: operands were not split for K = ", std::to_string(K));
+  for (const auto& [u, rows] : {std::pair<const at::Tensor&, int64_t>(ua, M), std::pair<const at::Tensor&, int64_t>(ub, N)})
+    TORCH_CHECK(u.is_cuda() && u.scalar_type() == at::kFloat && u.is_contiguous() && u.numel() == batch * hb::split16_units(rows) &&
+                    u.device() == a.device(), "split16_gemm: units of another operand");
+  c10::cuda::CUDAGuard guard(a.device());
+  hb::Tf32Epilogue E{};
+  E.mode = mode; E.alpha = (float)alpha; E.w = (float)w; E.b1 = (float)b1; E.b2 = (float)b2c; E.eps = (float)eps;
+  if (c.has_value() && c->defined()) {
+    TORCH_CHECK(c->is_cuda() && c->scalar_type() == at::kFloat && c->dim() == 3 && c->size(0) == batch && c->size(1) == M &&
+                    c->size(2) >= N && c->stride(2) == 1 && c->stride(1) >= N && c->device() == a.device(),
+                "split16_gemm: c must be fp32 [batch, M, >= N] with unit inner stride");
+    E.C = c->data_ptr<float>(); E.ldc = c->stride(1); E.strideC = c->stride(0);
+  }
+  if (mode == hb::kEpiAdam || mode == hb::kEpiLaProp) {
+    TORCH_CHECK(m.has_value() && v.has_value(), "split16_gemm: moment buffers required");
+    for (const at::Tensor* t : {&*m, &*v})
+      TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->numel() == batch * M * N &&
+                      t->device() == a.device(), "split16_gemm: moments must be contiguous fp32 [batch, M, N]");
+    E.m = m->data_ptr<float>(); E.v = v->data_ptr<float>();
+  }
+  TORCH_CHECK(E.C != nullptr, "split16_gemm: no output requested");
+  TORCH_CHECK(!upper_upper || (M == N && M == K && a.data_ptr() != b.data_ptr()), "split16_gemm: upper_upper needs two square matrices of one size");
+  E.tri = upper_upper ? 1 : 0;
+  E.symmetric = (a.data_ptr() == b.data_ptr() && M == N && (mode == hb::kEpiStore || mode == hb::kEpiLerp || mode == hb::kEpiAdd)) ? 1 : 0;
+  check(hb::launch_split16_gemm({a.data_ptr(), ua.data_ptr<float>()}, {b.data_ptr(), ub.data_ptr<float>()}, (int)M, (int)N, (int)K, (int)batch,
+                                E, status.data_ptr<int>(), at::cuda::getCurrentCUDAStream()), "split16 gemm");
+}
+
+// op(a) @ op(b) for batched fp32 matrices from fp16 pairs; arguments and result as for tf32x3_matmul.
+at::Tensor split16_matmul(const at::Tensor& a, const at::Tensor& b, bool ta, bool tb, double alpha, const at::Tensor& status,
+                          bool upper_upper) {
+  TORCH_CHECK(a.dim() == 3 && b.dim() == 3, "split16_matmul: fp32 [batch, rows, cols] CUDA tensors");
+  const int64_t batch = a.size(0), M = ta ? a.size(2) : a.size(1), K = ta ? a.size(1) : a.size(2), N = tb ? b.size(1) : b.size(2);
+  TORCH_CHECK(b.size(0) == batch && (tb ? b.size(2) : b.size(1)) == K, "split16_matmul: batches or inner dimensions differ");
+  const bool same_operand = a.data_ptr() == b.data_ptr() && a.sizes() == b.sizes() && a.strides() == b.strides() && ta != tb;  // X X^T or X^T X
+  TORCH_CHECK(!(upper_upper && same_operand), "split16_matmul: upper_upper needs two square matrices of one size");
+  const std::vector<at::Tensor> sa = split16(a, !ta, ta);
+  // B as the K-major [N, K] operand: b given as [K, N] must be transposed, b given as [N, K] is used as it is
+  const std::vector<at::Tensor> sb = same_operand ? sa : split16(b, tb, !tb);
+  const int ia = ta ? 2 : 0, ib = same_operand ? ia : (tb ? 0 : 2);
+  const int64_t ldc = (N + 3) / 4 * 4;
+  at::Tensor c = at::empty({batch, M, ldc}, a.options().memory_format(at::MemoryFormat::Contiguous));
+  const at::Tensor view = ldc == N ? c : c.narrow(2, 0, N);
+  split16_gemm(sa[ia], sa[ia + 1], sb[ib], sb[ib + 1], K, hb::kEpiStore, alpha, 0, 0, 0, 0, view, {}, {}, upper_upper, status);
+  return view;
+}
+
 // op(a) @ op(b) for batched fp32 matrices on the split-tf32 tensor-core path.  a: [batch, R, C]; ta = 0 uses a as
 // [M, K], ta = 1 as [K, M]; likewise b is [K, N] for tb = 0 and [N, K] for tb = 1.  Returns [batch, M, N].
 // upper_upper: op(a) and op(b) are both upper triangular (square, same size): only the non-zero K range of every tile
@@ -676,6 +753,10 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("tf32x3_matmul", &tf32x3_matmul);
   m.def("tf32_split", &tf32_split);
   m.def("tf32_gemm", &tf32_gemm);
+  m.def("split16", &split16);
+  m.def("split16_matmul", &split16_matmul);
+  m.def("split16_gemm", &split16_gemm);
+  m.def("set_split16_gemm_tile", &hb::set_split16_gemm_tile_override);
   m.def("colsum_bf16", &colsum_bf16);
   m.def("colsum_bf16_batch", &colsum_bf16_batch);
   m.def("gelu_fwd", &gelu_fwd);

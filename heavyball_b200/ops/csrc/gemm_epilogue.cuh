@@ -1,0 +1,386 @@
+// Epilogue and 128 x 128 kernel shared by the split-operand GEMMs (tf32_gemm.cu, split16_gemm.cu).
+//
+// 128 x 128 tiles, one per CTA, 192 threads, two CTAs per SM:
+//   warp 0     : TMA producer, cp.async.bulk.tensor 3-D loads (128-byte swizzle, 128 bytes of K per row) into a 3-stage ring
+//   warp 1     : tcgen05.mma.cta_group::1, 128 x 128 x 32 bytes of K per instruction, accumulator in 128 TMEM columns
+//   warps 2..5 : tcgen05.ld, then the epilogue.  Plain stores go through the (now idle) ring and four bulk tensor stores, the
+//                others through epilogue_direct.
+#pragma once
+#include "tc_common.cuh"
+#include "tf32_gemm.h"
+
+namespace hb {
+namespace {
+
+constexpr int TBM = 128, TBN = 128;
+constexpr int kTStages = 3;
+constexpr int kTTileBytes = TBM * 128;               // 16 KiB per operand tile
+constexpr int kTStageBytes = 2 * kTTileBytes;
+constexpr int kTSmemBytes = kTStages * kTStageBytes + 1024;
+constexpr int kTThreads = 192;
+constexpr uint32_t kTTmemCols = 128;
+
+__device__ __forceinline__ float tf32_hi(float x) {
+  uint32_t bits;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(bits) : "f"(x));
+  return __uint_as_float(bits);
+}
+
+__device__ __forceinline__ float lerp_w(float s, float x, float w) { return s * (1.0f - w) + x * w; }
+
+// Accumulators of 32 columns of one row, times the units of the row and of each column.  The smaller factor goes first: their product
+// alone may leave the range of fp32 where the result does not.
+__device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_factor, const float* col_unit) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float4 c = *(const float4*)(col_unit + q * 4);
+    const float f[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      acc[q * 4 + e] = __float_as_uint(__uint_as_float(acc[q * 4 + e]) * fminf(row_factor, f[e]) * fmaxf(row_factor, f[e]));
+  }
+}
+
+constexpr int kStageLd = 36;                         // floats per staged row: rows stay 16-byte aligned and float4
+                                                     // accesses of a quarter-warp fall into distinct banks
+constexpr int kStageWarpBytes = 32 * kStageLd * 4;   // one warp's 32 rows x 32 columns
+
+// Fused epilogue of one warp: its 32 accumulator rows of the 128x128 tile, 32 columns at a time.  A thread reads
+// its own row from tensor memory; global memory wants the other orientation (consecutive lanes on consecutive
+// columns), so the block is turned through the warp's `stage` in shared memory (the idle operand ring):
+//   pass 1 (lane = row):                   accumulators * alpha -> stage
+//   pass 2 (8 lanes per row, 4 rows/step): moments, lerp, C store, split-operand store - every global access is a full
+//                                          128-byte line per row; the final values go back to the stage when needed
+//   pass 3 (lane = row):                   outputs that run along the rows: transposed split operand, mirror tile
+// Values outside [M, N] are never stored; the zero padding of a split output (columns [K, kp) of the operand being
+// produced) is.
+// `tmem_warp`: tensor-memory address of the warp's first row and the tile's first column; `row0` / `col_base`: their
+// global indices; `n_cb`: 32-column blocks in the tile; `off_diagonal`: the tile is not on the diagonal (mirror stores).
+// `zero_acc`: the tile had no product (its accumulator was never written): the values are zeros.
+// `kScaled`: the operands were scaled by powers of two per row; `row_unit` / `col_unit` are what one unit of an accumulator row /
+// column stands for (arrays of this batch entry, padded to whole tiles).
+template <bool kScaled>
+__device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, float* stage, int row0, int col_base, int n_cb,
+                                                bool off_diagonal, bool zero_acc, int batch, int M, int N,
+                                                const Tf32Epilogue& E, const float* row_unit = nullptr, const float* col_unit = nullptr) {
+  const int64_t b64 = batch;
+  const bool state_vec = (N & 3) == 0;
+  const bool c_vec = (E.ldc & 3) == 0 && ((E.strideC & 3) == 0) && ((((uintptr_t)E.C) & 15) == 0);
+  const bool moments = E.mode == kEpiAdam || E.mode == kEpiLaProp;
+  const bool mirror = E.symmetric && off_diagonal && E.C != nullptr;
+  const bool along_rows = mirror || (E.S != nullptr && E.s_transposed);
+  const bool s_rows = E.S != nullptr && !E.s_transposed;
+  const int sub = lane >> 3, cg = (lane & 7) * 4;
+  const float w1 = 1.0f - E.b1, w2 = 1.0f - E.b2;
+  float* mine = stage + lane * kStageLd;
+  float row_factor = 1.0f;
+  if constexpr (kScaled) row_factor = row_unit[row0 + lane];
+#pragma unroll 1
+  for (int cb = 0; cb < n_cb; ++cb) {
+    const int col0 = col_base + cb * 32;
+    {
+      uint32_t acc[32];
+      if (!zero_acc) {
+        tmem_ld32(tmem_warp + (uint32_t)(cb * 32), acc);
+        tmem_ld_wait();
+      } else {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) acc[j] = 0u;
+      }
+      if constexpr (kScaled) unscale32(acc, row_factor, col_unit + col0);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        *(float4*)(mine + q * 4) =
+            make_float4(__uint_as_float(acc[q * 4]) * E.alpha, __uint_as_float(acc[q * 4 + 1]) * E.alpha,
+                        __uint_as_float(acc[q * 4 + 2]) * E.alpha, __uint_as_float(acc[q * 4 + 3]) * E.alpha);
+    }
+    __syncwarp();
+
+    const int col = col0 + cg;
+    // What the epilogue reads from global memory (moments, or the old value of C) is fetched four steps at a time
+    // before the first of them is used: a step-by-step load -> compute -> store chain pays one memory round trip per step
+    // (stores may alias the next step's loads, so the compiler cannot hoist them), which for the small products of a
+    // blocked solve was longer than the product itself.
+    const bool fast_state = moments && state_vec && col + 3 < N;
+    const bool fast_old = (E.mode == kEpiLerp || E.mode == kEpiAdd) && E.C != nullptr && c_vec && col + 3 < N;
+    float4 pa[4], pb[4];
+#pragma unroll 1
+    for (int half = 0; half < 2; ++half) {
+    if (fast_state || fast_old) {
+#pragma unroll
+      for (int i4 = 0; i4 < 4; ++i4) {
+        const int row = row0 + (half * 4 + i4) * 4 + sub;
+        pa[i4] = make_float4(0.f, 0.f, 0.f, 0.f);
+        pb[i4] = pa[i4];
+        if (row < M) {
+          if (fast_state) {
+            pa[i4] = *(const float4*)(E.m + (b64 * M + row) * (int64_t)N + col);
+            pb[i4] = *(const float4*)(E.v + (b64 * M + row) * (int64_t)N + col);
+          } else {
+            pa[i4] = *(const float4*)(E.C + b64 * E.strideC + (int64_t)row * E.ldc + col);
+          }
+        }
+      }
+    }
+#pragma unroll
+    for (int i4 = 0; i4 < 4; ++i4) {
+      const int it = half * 4 + i4;
+      const int lr = it * 4 + sub, row = row0 + lr;
+      float* sp = stage + lr * kStageLd + cg;
+      const float4 x4 = *(const float4*)sp;
+      float x[4] = {x4.x, x4.y, x4.z, x4.w};
+      if (row < M && col < N) {
+        if (moments) {
+          float* mp = E.m + (b64 * M + row) * (int64_t)N + col;
+          float* vp = E.v + (b64 * M + row) * (int64_t)N + col;
+          const bool fast = fast_state;
+          float m4[4], s4[4];
+          if (fast) {
+            const float4 a = pa[i4], c = pb[i4];
+            m4[0] = a.x; m4[1] = a.y; m4[2] = a.z; m4[3] = a.w;
+            s4[0] = c.x; s4[1] = c.y; s4[2] = c.z; s4[3] = c.w;
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              m4[e] = col + e < N ? mp[e] : 0.f;
+              s4[e] = col + e < N ? vp[e] : 0.f;
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            s4[e] = lerp_w(s4[e], x[e] * x[e], w2);
+            const float d = fmaxf(sqrtf(s4[e]), E.eps);
+            if (E.mode == kEpiAdam) {
+              m4[e] = lerp_w(m4[e], x[e], w1);
+              x[e] = m4[e] / d;
+            } else {
+              m4[e] = lerp_w(m4[e], x[e] / d, w1);
+              x[e] = m4[e];
+            }
+          }
+          if (fast) {
+            *(float4*)mp = make_float4(m4[0], m4[1], m4[2], m4[3]);
+            *(float4*)vp = make_float4(s4[0], s4[1], s4[2], s4[3]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (col + e < N) { mp[e] = m4[e]; vp[e] = s4[e]; }
+          }
+        }
+        if (E.C != nullptr) {
+          float* cp = E.C + b64 * E.strideC + (int64_t)row * E.ldc + col;
+          const bool fast = c_vec && col + 3 < N;
+          if (E.mode == kEpiLerp || E.mode == kEpiAdd) {
+            // lerp: o + (x - o) w;  add: o + x  (the same expression with the old value left out of the difference)
+            const float keep = E.mode == kEpiLerp ? 1.f : 0.f, w = E.mode == kEpiLerp ? E.w : 1.f;
+            if (fast) {
+              const float4 o = pa[i4];
+              x[0] = o.x + (x[0] - keep * o.x) * w; x[1] = o.y + (x[1] - keep * o.y) * w;
+              x[2] = o.z + (x[2] - keep * o.z) * w; x[3] = o.w + (x[3] - keep * o.w) * w;
+            } else {
+#pragma unroll
+              for (int e = 0; e < 4; ++e)
+                if (col + e < N) { const float o = cp[e]; x[e] = o + (x[e] - keep * o) * w; }
+            }
+          }
+          if (fast) {
+            *(float4*)cp = make_float4(x[0], x[1], x[2], x[3]);
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (col + e < N) cp[e] = x[e];
+          }
+        }
+      }
+      if (s_rows && row < M && col < E.kpS) {  // operand rows = output rows, K over the output columns (zero from N to kp)
+        float* srow = E.S + b64 * E.strideS + (int64_t)row * (2 * E.kpS) + col;
+        float hi[4], lo[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float y = col + e < N ? x[e] : 0.f;
+          hi[e] = tf32_hi(y);
+          lo[e] = tf32_hi(y - hi[e]);
+        }
+        *(float4*)srow = make_float4(hi[0], hi[1], hi[2], hi[3]);
+        *(float4*)(srow + E.kpS) = make_float4(lo[0], lo[1], lo[2], lo[3]);
+      }
+      if (along_rows) *(float4*)sp = make_float4(x[0], x[1], x[2], x[3]);
+    }
+    }
+
+    if (along_rows) {
+      __syncwarp();
+      const int row = row0 + lane;
+      float v[32];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 t = *(const float4*)(mine + q * 4);
+        v[q * 4] = t.x; v[q * 4 + 1] = t.y; v[q * 4 + 2] = t.z; v[q * 4 + 3] = t.w;
+      }
+      if (mirror && row < M) {  // consecutive lanes hold consecutive rows: one accumulator column is one contiguous line
+        float* ccol = E.C + b64 * E.strideC + row;
+#pragma unroll
+        for (int j = 0; j < 32; ++j)
+          if (col0 + j < N) ccol[(int64_t)(col0 + j) * E.ldc] = v[j];
+      }
+      if (E.S != nullptr && E.s_transposed && row < E.kpS) {
+        // operand rows = output columns, K over the output rows (zero from M up to kp)
+        float* sb = E.S + b64 * E.strideS + row;
+        const int64_t ld = 2 * E.kpS;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          if (col0 + j < N) {
+            const float y = row < M ? v[j] : 0.f;
+            const float hi = tf32_hi(y);
+            float* dst = sb + (int64_t)(col0 + j) * ld;
+            dst[0] = hi;
+            dst[E.kpS] = tf32_hi(y - hi);
+          }
+        }
+      }
+    }
+    __syncwarp();  // the stage is rewritten by the next block of columns
+  }
+}
+
+// `Kind`: operand type.  kBlock elements of K fill a 128-byte row; kDesc is the instruction descriptor for a 128 x 128 tile; the product
+// is three walks over K, of which walk kTermLoA takes the low parts of A and walk kTermLoB those of B; kCrossFirst: these two come
+// first, and the sum they leave is scaled by 2^-11 when the walk over the high parts begins.
+template <class Kind>
+__global__ void __launch_bounds__(kTThreads, 2)
+gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+               const __grid_constant__ CUtensorMap map_c, int M, int N, int kp, const Tf32Epilogue E, const float* row_units, int64_t stride_ru,
+               const float* col_units, int64_t stride_cu, int bulk_store, int* status) {
+  constexpr int TBK = Kind::kBlock;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[kTStages];
+  __shared__ __align__(8) uint64_t empty_bar[kTStages];
+  __shared__ __align__(8) uint64_t accum_bar, drain_bar;  // drain_bar: teardown only
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int abort_flag;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int tiles_n = (N + TBN - 1) / TBN;
+  int tm = blockIdx.x / tiles_n, tn = blockIdx.x % tiles_n;
+  if (E.symmetric) {  // blockIdx.x counts the tiles on or above the diagonal, row by row
+    int left = blockIdx.x;
+    tm = 0;
+    while (left >= tiles_n - tm) { left -= tiles_n - tm; ++tm; }
+    tn = tm + left;
+  }
+  const int batch = blockIdx.y;
+  int kb_lo = 0, kb_hi = kp / TBK;  // K blocks of one term of the split product that this tile walks
+  if (E.tri) {
+    kb_lo = min(kb_hi, tm * (TBM / TBK));
+    kb_hi = tn < tm ? kb_lo : min(kb_hi, (tn + 1) * (TBN / TBK));
+  }
+  const int seg_kb = kb_hi - kb_lo;
+  const int num_kb = 3 * seg_kb;    // three terms of the split product
+  const float alpha = E.alpha;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kTStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    mbar_init(&accum_bar, 1);
+    mbar_init(&drain_bar, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) { tmem_alloc(&tmem_base_slot, kTTmemCols); tmem_relinquish(); }
+  griddep_wait();
+  // a kernel of this stream already gave up on a wait: do not pile more work on a broken pipeline
+  const bool skip = __syncthreads_or(threadIdx.x == 0 && status != nullptr && *(volatile const int*)status != 0);
+  griddep_launch();
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+
+  int issued = 0;
+  if (skip) {
+  } else if (warp == 0) {
+    if (lane == 0) {
+      for (int kb = 0; kb < num_kb; ++kb) {
+        const int s = kb % kTStages, round = kb / kTStages;
+        if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag)) break;
+        uint8_t* dst = tiles + s * kTStageBytes;
+        const int seg = kb / seg_kb, k0 = (kb_lo + kb - seg * seg_kb) * TBK;
+        mbar_expect_tx(&full_bar[s], kTStageBytes);
+        tma_load_3d(dst, &map_a, &full_bar[s], k0 + (seg == Kind::kTermLoA ? kp : 0), tm * TBM, batch);
+        tma_load_3d(dst + kTTileBytes, &map_b, &full_bar[s], k0 + (seg == Kind::kTermLoB ? kp : 0), tn * TBN, batch);
+        issued = kb + 1;
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      bool ok = true;
+      for (int kb = 0; kb < num_kb && ok; ++kb) {
+        const int s = kb % kTStages, round = kb / kTStages;
+        ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t a_addr = smem_u32(tiles + s * kTStageBytes);
+        const uint64_t a_desc = make_smem_desc(a_addr), b_desc = make_smem_desc(a_addr + kTTileBytes);
+#pragma unroll
+        for (int k = 0; k < 4; ++k)  // 32 B along K inside the swizzle atom = +2 address units
+          if (Kind::kCrossFirst && k == 0 && kb == 2 * seg_kb)
+            tc_mma_f16_d11(tmem_base, a_desc, b_desc, Kind::kDesc);
+          else
+            Kind::mma(tmem_base, a_desc + 2 * k, b_desc + 2 * k, Kind::kDesc, (kb | k) ? 1u : 0u);
+        tc_commit(&empty_bar[s]);
+      }
+      if (ok) tc_commit(&accum_bar);
+    }
+  } else {
+    const int quarter = warp & 3, r = quarter * 32 + lane;
+    const bool have = (num_kb == 0) || mbar_wait(&accum_bar, 0, &abort_flag);
+    const float* row_unit = Kind::kScaled ? row_units + batch * stride_ru : nullptr;
+    const float* col_unit = Kind::kScaled ? col_units + batch * stride_cu : nullptr;
+    tc_fence_after();
+    if (have && bulk_store) {
+      // every load has landed and every MMA has retired: the ring is free and stages the output tile as four
+      // [128 rows x 32 fp32] boxes in the swizzled layout the bulk store expects
+#pragma unroll 1
+      for (int cb = 0; cb < TBN / 32; ++cb) {
+        uint32_t acc[32];
+        tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32), acc);
+        tmem_ld_wait();
+        if constexpr (Kind::kScaled) unscale32(acc, row_unit[tm * TBM + r], col_unit + tn * TBN + cb * 32);
+        uint8_t* box = tiles + cb * kTTileBytes;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          *(float4*)(box + swz(r, q)) =
+              make_float4(__uint_as_float(acc[q * 4]) * alpha, __uint_as_float(acc[q * 4 + 1]) * alpha,
+                          __uint_as_float(acc[q * 4 + 2]) * alpha, __uint_as_float(acc[q * 4 + 3]) * alpha);
+      }
+    } else if (have) {
+      epilogue_direct<Kind::kScaled>(tmem_base + ((uint32_t)(quarter * 32) << 16), lane, (float*)(tiles + quarter * kStageWarpBytes),
+                      tm * TBM + quarter * 32, tn * TBN, TBN / 32, tm != tn, num_kb == 0, batch, M, N, E,
+                      row_unit, col_unit);
+    }
+    tc_fence_before();
+    if (bulk_store) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (have && warp == 2 && lane == 0) {
+#pragma unroll
+        for (int cb = 0; cb < TBN / 32; ++cb)
+          if (tn * TBN + cb * 32 < N) tma_store_3d(&map_c, tiles + cb * kTTileBytes, tn * TBN + cb * 32, tm * TBM, batch);
+        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+      }
+    }
+  }
+
+  __syncthreads();
+  if (abort_flag) {  // after an expired wait: loads and products in flight end before shared and tensor memory go away
+    if (warp == 0 && lane == 0) ring_drain(full_bar, issued, kTStages);
+    if (warp == 1 && lane == 0) products_drain(&drain_bar);
+    __syncthreads();
+    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
+  }
+  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTTmemCols); }
+}
+
+}  // namespace
+}  // namespace hb

@@ -1,0 +1,485 @@
+// fp32-in / fp32-out batched GEMM at fp32-level accuracy on the fp16 tensor-core path of sm_100a.
+//
+// The 3-term split product of tf32_gemm.cu with fp16 in the place of tf32: both carry 11 significant bits, so hi + lo keep 22 bits
+// of a value either way, but fp16 operands are half as wide and their products run at twice the rate.  What fp16 lacks is range,
+// hence one power of two per operand row that takes the row's largest value to the top of it and comes off again in the epilogue
+// (exact both ways).  Values down to 2^-29 of their row's largest keep all 22 bits; below that the error is 2^-51 of the largest,
+// far under the rounding of any sum in which both take part.
+//
+// Three walks over K share one fp32 accumulator: hi lo^T and lo hi^T first, with lo stored times 2^11 (so that small values keep it,
+// too), then hi hi^T on top, whose first instruction takes 2^-11 off the accumulator (the scale-input-d operand of tcgen05.mma).  The
+// large sum is rounded once per 16 of K that way; with the high parts first, as tf32 walks them, the two small sums would be rounded
+// at its magnitude as well.  Error against 64 bits, relative 2-norm, K = 1024 / 2048 / 8192: 1.2e-6 / 2.5e-6 / 9.7e-6 (tf32: 1.1e-5 /
+// 2.1e-5 / 8.4e-5), the same with rows over thirty decades and with entries over eight decades along K.
+//
+// Measured on one B200, of measured peak (1.64 PFLOP/s / 3): 2 of 5504 x 2048 x 2048 224 us = 412 TFLOP/s, 0.75 (split tf32 409 us);
+// 4 of 2048^3 176 us = 390, 0.71 (277); 8 of 1024^3 64 us = 269, 0.49, one wave (98).
+#include "split16_gemm.h"
+
+#include <cuda_fp16.h>
+
+#include "gemm_epilogue.cuh"
+#include "pair_drain.h"
+#include "per_device.h"
+
+namespace hb {
+namespace {
+
+constexpr int HBK = 64;  // fp16 elements of K in a 128-byte row
+// fp16 x fp16 -> fp32, both operands K-major
+constexpr uint32_t half_desc(int m, int n) { return (1u << 4) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
+
+struct HalfKind {
+  static constexpr int kBlock = HBK;
+  static constexpr bool kScaled = true, kCrossFirst = true;
+  static constexpr int kTermLoA = 1, kTermLoB = 0;  // A: hi, lo, hi   B: lo, hi, hi
+  static constexpr uint32_t kDesc = half_desc(TBM, TBN);
+  __device__ static __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, uint32_t accumulate) {
+    tc_mma_bf16(d, a, b, desc, accumulate);  // kind::f16; the operand type is in the descriptor
+  }
+};
+
+// ------------------------------------------------------------------------------------------ pair kernel
+// 256 x 256 tiles on CTA pairs (cta_group::2), one persistent pair per two SMs; structure as in ns_gemm.cu: each CTA stages 128 rows of
+// A and half of B (32 KiB per 64 of K, 5 stages), two accumulators, eight epilogue warps of 32 rows x 128 columns under the next
+// tile's main loop.
+constexpr int kHPairStages = 5;
+constexpr int kHPairStageBytes = 2 * kTTileBytes;
+constexpr int kHPairEpiWarps = 8;
+constexpr int kHPairThreads = 64 + 32 * kHPairEpiWarps;
+constexpr uint32_t kHPairDesc = half_desc(kPairTile, kPairTile);
+constexpr int kHPairSmemBytes = kHPairStages * kHPairStageBytes + kHPairEpiWarps * kStageWarpBytes + 1024;
+
+struct HalfTile {
+  int kb_lo, seg;  // K blocks of one term that the tile walks: [kb_lo, kb_lo + seg)
+};
+__device__ __forceinline__ HalfTile half_tile(const PairTile& t, int kp, int tri) {
+  int lo = 0, hi = kp / HBK;
+  if (tri) {
+    lo = min(hi, t.tm * (kPairTile / HBK));
+    hi = t.tn < t.tm ? lo : min(hi, (t.tn + 1) * (kPairTile / HBK));
+  }
+  return {lo, hi - lo};
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHPairThreads, 1)
+split16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N, int kp, int tiles_m,
+                    int tiles_n, int per_batch, int total, const Tf32Epilogue E, const float* row_units, int64_t stride_ru,
+                    const float* col_units, int64_t stride_cu, int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[kHPairStages];   // used in the even CTA: both CTAs' loads of a stage have landed
+  __shared__ __align__(8) uint64_t empty_bar[kHPairStages];  // in each CTA: the products that read the stage have finished
+  __shared__ __align__(8) uint64_t acc_full[2];              // in each CTA: accumulator finished
+  __shared__ __align__(8) uint64_t acc_empty[2];             // in the even CTA: all sixteen epilogue warps have read it
+  __shared__ __align__(8) uint64_t drain_bar;                // in each CTA, teardown only: all products have finished
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int abort_flag, skip_flag;
+  __shared__ int fills;                                      // ring fills this CTA issued
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kHPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * kHPairEpiWarps); }
+    mbar_init(&drain_bar, 1);
+    abort_flag = 0;
+    fills = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) { tmem_alloc_pair(&tmem_base_slot, 512); tmem_relinquish_pair(); }
+  griddep_wait();
+  // a kernel of this stream already gave up on a wait: do not pile more work on a broken pipeline (the even CTA decides)
+  if (threadIdx.x == 0) skip_flag = status != nullptr && *(volatile const int*)status != 0;
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+  const bool skip = cluster_load(cluster_addr(&skip_flag, 0)) != 0;
+
+  if (skip) {
+  } else if (warp == 0) {
+    if (lane == 0) {
+      int n = 0;  // ring fills so far
+      bool ok = true;
+      for (int idx = pair; idx < total && ok; idx += pairs) {
+        const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
+        const HalfTile h = half_tile(t, kp, E.tri);
+        const int a_row = t.tm * kPairTile + (int)rank * 128, b_row = t.tn * kPairTile + (int)rank * 128;
+        for (int term = 0; term < 3 && ok; ++term) {
+          const int ka = (term == HalfKind::kTermLoA ? kp : 0), kb_off = (term == HalfKind::kTermLoB ? kp : 0);
+          for (int kb = 0; kb < h.seg; ++kb, ++n) {
+            const int s = n % kHPairStages, round = n / kHPairStages, k0 = (h.kb_lo + kb) * HBK;
+            ok = mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag);
+            if (!ok) break;
+            uint8_t* dst = ring + s * kHPairStageBytes;
+            const uint32_t bar = cluster_addr(&full_bar[s], 0);
+            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kHPairStageBytes);
+            tma_load_3d_pair(dst, &map_a, bar, ka + k0, a_row, t.batch);  // rows past the operand's end arrive as zeros and count
+            tma_load_3d_pair(dst + kTTileBytes, &map_b, bar, kb_off + k0, b_row, t.batch);
+          }
+        }
+      }
+      fills = n;
+      griddep_launch();  // this CTA's last loads are on their way: the next kernel may take over SMs that drain
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && rank == 0) {
+      int n = 0, it = 0;
+      bool ok = true;
+      for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
+        const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
+        const int seg = half_tile(t, kp, E.tri).seg, num_kb = 3 * seg, acc = it & 1;
+        ok = mbar_wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1, &abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + (uint32_t)acc * 256u;
+        for (int kb = 0; kb < num_kb; ++kb, ++n) {
+          const int s = n % kHPairStages, round = n / kHPairStages;
+          ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t base = smem_u32(ring + s * kHPairStageBytes);
+          const uint64_t a_desc = make_smem_desc(base), b_desc = make_smem_desc(base + kTTileBytes);
+#pragma unroll
+          for (int k = 0; k < HBK / 16; ++k)
+            if (k == 0 && kb == 2 * seg)
+              tc_mma_f16_d11_pair(d, a_desc, b_desc, kHPairDesc);
+            else
+              tc_mma_bf16_pair(d, a_desc + 2 * k, b_desc + 2 * k, kHPairDesc, (kb | k) ? 1u : 0u);
+          tc_commit_pair(&empty_bar[s]);
+        }
+        if (ok) tc_commit_pair(&acc_full[acc]);
+      }
+    }
+  } else {
+    const int quarter = warp & 3, half = (warp - 2) >> 2;  // tensor-memory lanes this warp may read; its half of the columns
+    float* const stage = (float*)(ring + kHPairStages * kHPairStageBytes + (warp - 2) * kStageWarpBytes);
+    const uint32_t tmem_warp = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
+    int it = 0;
+    for (int idx = pair; idx < total; idx += pairs, ++it) {
+      const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
+      const int acc = it & 1, row0 = t.tm * kPairTile + (int)rank * 128 + quarter * 32, col0 = t.tn * kPairTile + half * 128;
+      const bool ok = mbar_wait(&acc_full[acc], (it >> 1) & 1, &abort_flag);
+      if (!__all_sync(0xFFFFFFFFu, ok)) break;
+      tc_fence_after();
+      const int blocks = min(4, (N - col0 + 31) / 32);
+      if (row0 < M && blocks > 0)
+        epilogue_direct<true>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, t.tm != t.tn,
+                              half_tile(t, kp, E.tri).seg == 0, t.batch, M, N, E, row_units + t.batch * stride_ru,
+                              col_units + t.batch * stride_cu);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) cluster_arrive(cluster_addr(&acc_empty[acc], 0));
+    }
+    tc_fence_before();
+  }
+
+  // After an expired wait in either CTA, both wait (with a limit) for every product and every load that the pair issued before its
+  // shared and tensor memory go away.
+  __syncthreads();
+  if (threadIdx.x == 0 && abort_flag) cluster_store(cluster_addr(&abort_flag, rank ^ 1), 1);
+  cluster_sync();
+  if (abort_flag) {
+    if (rank == 0 && warp == 1 && lane == 0) tc_commit_pair(&drain_bar);  // the thread that issued the products
+    if (threadIdx.x == 0) mbar_drain(&drain_bar, 0);
+    if (rank == 0 && threadIdx.x == 0) {
+      const int even = fills, odd = cluster_load(cluster_addr(&fills, 1)), top = max(even, odd);
+      for (int n = pair_drain_first(even, odd, kHPairStages); n < top; ++n) {
+        const int s = n % kHPairStages, kind = pair_fill_kind(n, even, odd);
+        if (kind == kFillOddOnly) mbar_expect_tx(&full_bar[s], (uint32_t)kHPairStageBytes);
+        if (kind == kFillEvenOnly) mbar_complete_tx(&full_bar[s], (uint32_t)kHPairStageBytes);
+        mbar_drain(&full_bar[s], (n / kHPairStages) & 1);
+      }
+    }
+    cluster_sync();
+  }
+  if (threadIdx.x == 0 && abort_flag && status != nullptr) atomicExch(status, 1);
+  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
+}
+
+// ------------------------------------------------------------------------------------------ operand split
+// One launch, two kinds of block; a row's exponent has to be known before its first value can be stored, so both kinds first look for
+// the largest value and then convert:
+//   blocks [0, row_blocks) : eight source rows, one per warp -> `same`
+//   the others             : clusters of up to eight share a strip of 32 source columns, 256 rows at a time each, and exchange their
+//                            column maxima -> `trans`, turned through shared memory
+// What both saw first stays in registers (1024 columns of a row, 256 rows of a strip); only longer ones are read again, from L1 or L2.
+// Bound by memory: 4 of 2048^2 rows 24 us (5.6 TB/s; split tf32, twice the bytes out, 37), columns 38 us, both 50 (59); one block per
+// strip of 16 columns instead of a cluster 70 us for the columns.
+constexpr int kSplitThreads = 256;
+constexpr int kRowChunk = 1024;
+constexpr int kStrip = 32, kStripRows = 256, kMaxSplitCluster = 8;
+
+struct RowScale {
+  float mul, unit;  // 2^e, 2^-e
+};
+// `bits`: largest absolute value of the row, as its bits (NaN above infinity above everything finite)
+__device__ __forceinline__ RowScale row_scale(uint32_t bits) {
+  const int field = (int)(bits >> 23);
+  // zero and subnormal rows, and rows with an infinity or NaN (all of whose results are NaN: lo = inf - inf), stay as they are
+  const int e = (field == 0 || field == 255) ? 0 : min(126, 141 - field);
+  return {__uint_as_float((uint32_t)(127 + e) << 23), __uint_as_float((uint32_t)(127 - e) << 23)};
+}
+__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+__device__ __forceinline__ void split_pair(float x, uint16_t& hi, uint16_t& lo) {
+  const __half h = __float2half_rn(x);
+  hi = __half_as_ushort(h);
+  lo = __half_as_ushort(__float2half_rn((x - __half2float(h)) * 2048.0f));
+}
+__device__ __forceinline__ void split_store4(uint16_t* row, int64_t kp, const float (&x)[4]) {
+  uint16_t h[4], l[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) split_pair(x[e], h[e], l[e]);
+  *(uint2*)row = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+  *(uint2*)(row + kp) = make_uint2((uint32_t)l[0] | ((uint32_t)l[1] << 16), (uint32_t)l[2] | ((uint32_t)l[3] << 16));
+}
+__device__ __forceinline__ float4 load4(const float* p, int left, bool vec) {
+  if (vec && left >= 4) return *(const float4*)p;
+  return make_float4(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
+}
+
+__device__ __forceinline__ uint32_t abs_max4(float4 v) {
+  return max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
+}
+// position of row r of column c in the turned tile: four columns of a thread and four rows of a warp fall into distinct banks
+__device__ __forceinline__ int turned(int c, int r) { return c * kStripRows + (r ^ (c & ~3)); }
+
+__global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* __restrict__ src, int64_t ld_src, int64_t stride_src, int R, int C,
+                                                                 int row_blocks, int cluster, uint16_t* __restrict__ same,
+                                                                 float* __restrict__ same_unit, uint16_t* __restrict__ trans,
+                                                                 float* __restrict__ trans_unit) {
+  griddep_wait();
+  griddep_launch();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t batch = blockIdx.y;
+  const float* s = src + batch * stride_src;
+  const bool vec = (ld_src & 3) == 0 && (stride_src & 3) == 0 && (((uintptr_t)src) & 15) == 0;
+
+  if ((int)blockIdx.x < row_blocks) {  // whole clusters take this branch (row_blocks is a multiple of `cluster`)
+    const int r = blockIdx.x * (kSplitThreads / 32) + warp;
+    if (r >= R) return;
+    const int kp = (C + 63) / 64 * 64;
+    const float* row = s + (int64_t)r * ld_src;
+    float4 v[kRowChunk / 128];
+    uint32_t top = 0;
+    const auto fetch = [&](int base) {
+#pragma unroll
+      for (int i = 0; i < kRowChunk / 128; ++i) {
+        const int c = base + i * 128 + lane * 4;
+        v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (c < C) v[i] = load4(row + c, C - c, vec);
+      }
+    };
+    for (int base = 0; base < C; base += kRowChunk) {
+      fetch(base);
+#pragma unroll
+      for (int i = 0; i < kRowChunk / 128; ++i) top = max(top, abs_max4(v[i]));
+    }
+    const RowScale f = row_scale(__reduce_max_sync(0xFFFFFFFFu, top));
+    if (lane == 0) same_unit[batch * ((R + 255) / 256 * 256) + r] = f.unit;
+    uint16_t* dst = same + (batch * R + r) * 2 * kp;
+    for (int base = 0; base < C; base += kRowChunk) {
+      if (C > kRowChunk) fetch(base);
+#pragma unroll
+      for (int i = 0; i < kRowChunk / 128; ++i) {
+        const int c = base + i * 128 + lane * 4;
+        if (c < kp) {
+          const float x[4] = {v[i].x * f.mul, v[i].y * f.mul, v[i].z * f.mul, v[i].w * f.mul};
+          split_store4(dst + c, kp, x);
+        }
+      }
+    }
+    return;
+  }
+
+  __shared__ __align__(16) float tile[kStrip * kStripRows];
+  __shared__ uint32_t warp_tops[kSplitThreads / 32][kStrip];
+  __shared__ uint32_t tops[kStrip];  // of this block's rows; the blocks of the cluster read each other's
+  __shared__ float muls[kStrip];
+  const int at = blockIdx.x - row_blocks, rank = at % cluster, c0 = at / cluster * kStrip;
+  const int q = threadIdx.x & 7, line = threadIdx.x >> 3, c = c0 + q * 4, kp = (R + 63) / 64 * 64;
+  const int first = rank * kStripRows, step = cluster * kStripRows;
+  float4 v[kStripRows / 32];
+  const auto fetch = [&](int r0) {  // rows r0 + line + 32 i, four columns each
+#pragma unroll
+    for (int i = 0; i < kStripRows / 32; ++i) {
+      const int r = r0 + line + 32 * i;
+      v[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < R && c < C) v[i] = load4(s + (int64_t)r * ld_src + c, C - c, vec);
+    }
+  };
+  uint32_t top[4] = {0, 0, 0, 0};
+  for (int r0 = first; r0 < R; r0 += step) {
+    fetch(r0);
+#pragma unroll
+    for (int i = 0; i < kStripRows / 32; ++i) {
+      top[0] = max(top[0], abs_bits(v[i].x));
+      top[1] = max(top[1], abs_bits(v[i].y));
+      top[2] = max(top[2], abs_bits(v[i].z));
+      top[3] = max(top[3], abs_bits(v[i].w));
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    top[e] = max(top[e], __shfl_xor_sync(0xFFFFFFFFu, top[e], 8));
+    top[e] = max(top[e], __shfl_xor_sync(0xFFFFFFFFu, top[e], 16));
+    if (lane < 8) warp_tops[warp][lane * 4 + e] = top[e];
+  }
+  __syncthreads();
+  if (threadIdx.x < kStrip) {
+    uint32_t t = 0;
+#pragma unroll
+    for (int w = 0; w < kSplitThreads / 32; ++w) t = max(t, warp_tops[w][threadIdx.x]);
+    tops[threadIdx.x] = t;
+  }
+  if (cluster > 1) cluster_sync(); else __syncthreads();
+  if (threadIdx.x < kStrip) {
+    uint32_t t = tops[threadIdx.x];
+    for (int k = 1; k < cluster; ++k)
+      t = max(t, (uint32_t)cluster_load(cluster_addr(&tops[threadIdx.x], (rank + k) % cluster)));
+    const RowScale f = row_scale(t);
+    muls[threadIdx.x] = f.mul;
+    if (rank == 0 && c0 + (int)threadIdx.x < C) trans_unit[batch * ((C + 255) / 256 * 256) + c0 + threadIdx.x] = f.unit;
+  }
+  if (cluster > 1) cluster_sync(); else __syncthreads();  // no block leaves while its maxima may still be read
+  const int oc = threadIdx.x >> 4, k4 = (threadIdx.x & 15) * 4;  // output: rows c0 + oc (+ 16) of the operand, four of K at a time
+  for (int r0 = first; r0 < R; r0 += step) {
+    if (R > step) fetch(r0);
+#pragma unroll
+    for (int i = 0; i < kStripRows / 32; ++i) {
+      const int r = line + 32 * i;
+      tile[turned(q * 4 + 0, r)] = v[i].x * muls[q * 4 + 0];
+      tile[turned(q * 4 + 1, r)] = v[i].y * muls[q * 4 + 1];
+      tile[turned(q * 4 + 2, r)] = v[i].z * muls[q * 4 + 2];
+      tile[turned(q * 4 + 3, r)] = v[i].w * muls[q * 4 + 3];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int g = 0; g < kStrip; g += 16) {
+      if (c0 + oc + g >= C) continue;
+      uint16_t* dst = trans + (batch * C + c0 + oc + g) * 2 * kp + r0;
+#pragma unroll
+      for (int k = k4; k < kStripRows; k += 64) {
+        if (r0 + k < kp) {
+          const float4 t = *(const float4*)&tile[turned(oc + g, k)];
+          const float x[4] = {t.x, t.y, t.z, t.w};
+          split_store4(dst + k, kp, x);
+        }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// fp16 operand [batch, rows, cols]; box = 64 columns x 128 rows, 128-byte swizzle
+bool make_half_map(CUtensorMap* map, const void* base, int rows, int64_t cols, int batch) {
+  EncodeTiledFn fn = tensor_map_encoder();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+  cuuint64_t strides[2] = {(cuuint64_t)cols * 2, (cuuint64_t)cols * rows * 2};
+  cuuint32_t box[3] = {HBK, TBM, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// fp32 output for the 128 x 128 kernel's bulk stores; box = 32 columns x 128 rows
+bool make_store_map(CUtensorMap* map, float* base, int rows, int cols, int64_t ld, int64_t stride, int batch) {
+  EncodeTiledFn fn = tensor_map_encoder();
+  if (fn == nullptr) return false;
+  cuuint64_t dims[3] = {(cuuint64_t)cols, (cuuint64_t)rows, (cuuint64_t)batch};
+  cuuint64_t strides[2] = {(cuuint64_t)ld * 4, (cuuint64_t)stride * 4};
+  cuuint32_t box[3] = {32, TBM, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, base, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+            CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// Whether a product takes pairs, from the waves that 128 x 128 tiles (four in the place of a pair) and pairs need.  150 sizes measured,
+// 128 / pairs: what fits in one wave of small tiles is theirs (640 x 512 x 2048 37.5 / 47.3 us, 8 of 512 x 1024 x 4096 113 / 100 is the
+// exception), and so is a short K, whose three walks do not cover a pair's epilogue (16 of 1024 x 768 x 128 28.5 / 44.3 us, 6 of
+// 5504 x 1536 x 512 220 / 195 - from seven waves on K = 512 is long enough); a half more waves cost more than the tile
+// gains (8 of 1024 x 1024 x 2048 symmetric, one wave or two, 73 / 114 us).  Elsewhere pairs are up to 1.29 times as fast (4 of
+// 2048^3 217 / 202, 8 of 3000 x 1536 x 4096 865 / 737) and at worst 5 % slower.
+bool split16_take_pairs(int M, int N, int K, int64_t small_waves, int64_t big_waves) {
+  return M > 128 && N > 128 && small_waves >= 2 && 3 * big_waves <= 4 * small_waves && (K >= 768 || (K >= 512 && small_waves >= 7));
+}
+
+int g_split16_tile = 0;
+
+}  // namespace
+
+void set_split16_gemm_tile_override(int tile) { g_split16_tile = (tile == 128 || tile == 256) ? tile : 0; }
+
+cudaError_t launch_split16(const float* src, int64_t ld_src, int64_t stride_src, int R, int C, int batch, Split16Operand same,
+                           Split16Operand trans, cudaStream_t stream) {
+  if (R == 0 || C == 0 || batch == 0 || (same.data == nullptr && trans.data == nullptr)) return cudaSuccess;
+  const int strips = trans.data != nullptr ? (C + kStrip - 1) / kStrip : 0;
+  int cluster = 1;  // strips longer than one block's rows are shared
+  while (strips > 0 && cluster < kMaxSplitCluster && cluster * kStripRows < R) cluster *= 2;
+  int row_blocks = same.data != nullptr ? (R + kSplitThreads / 32 - 1) / (kSplitThreads / 32) : 0;
+  row_blocks = (row_blocks + cluster - 1) / cluster * cluster;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(row_blocks + strips * cluster, batch);
+  cfg.blockDim = dim3(kSplitThreads);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  return cudaLaunchKernelEx(&cfg, split16_kernel, src, ld_src, stride_src, R, C, row_blocks, cluster, (uint16_t*)same.data, same.unit,
+                            (uint16_t*)trans.data, trans.unit);
+}
+
+cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N, int K, int batch, const Tf32Epilogue& E, int* status,
+                                cudaStream_t stream) {
+  static PerDevice<int> pairs;
+  int device = 0, max_pairs = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess)
+    e = pairs.get(device, cudaSuccess, &max_pairs, [](int& found) {
+      cudaError_t s = cudaFuncSetAttribute(gemm128_kernel<HalfKind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
+      if (s == cudaSuccess) s = cudaFuncSetAttribute(split16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHPairSmemBytes);
+      return s != cudaSuccess ? s : max_resident_pairs(split16_pair_kernel, kHPairThreads, kHPairSmemBytes, &found);
+    });
+  if (e != cudaSuccess) return e;
+  if (M == 0 || N == 0 || batch == 0) return cudaSuccess;
+  const bool moments = E.mode == kEpiAdam || E.mode == kEpiLaProp;
+  if (K == 0 || E.S != nullptr || (moments && (E.m == nullptr || E.v == nullptr))) return cudaErrorInvalidValue;
+  if (!moments && E.C == nullptr) return cudaErrorInvalidValue;
+  if (E.tri && (M != N || M != K || E.symmetric)) return cudaErrorInvalidValue;
+  if (E.symmetric && (A.data != B.data || M != N || E.C == nullptr || moments)) return cudaErrorInvalidValue;
+  const int64_t kp = split16_kp(K), stride_ru = split16_units(M), stride_cu = split16_units(N);
+  CUtensorMap ma, mb;
+  if (!make_half_map(&ma, A.data, M, 2 * kp, batch) || !make_half_map(&mb, B.data, N, 2 * kp, batch)) return cudaErrorInvalidValue;
+  const auto tiles = [&](int tile) {
+    const int m = (M + tile - 1) / tile, n = (N + tile - 1) / tile;
+    return E.symmetric ? n * (n + 1) / 2 : m * n;
+  };
+  const int64_t small = (int64_t)tiles(TBM) * batch, big = (int64_t)tiles(kPairTile) * batch;
+  const int64_t small_waves = (small + 4 * max_pairs - 1) / (4 * max_pairs), big_waves = (big + max_pairs - 1) / max_pairs;
+  bool pair = split16_take_pairs(M, N, K, small_waves, big_waves);
+  if (g_split16_tile != 0) pair = g_split16_tile == 256;
+  if (pair) {
+    const int tm = (M + kPairTile - 1) / kPairTile, tn = (N + kPairTile - 1) / kPairTile;
+    const int grid = 2 * (int)(big < max_pairs ? big : max_pairs);
+    return launch_chained(split16_pair_kernel, dim3(grid), kHPairThreads, kHPairSmemBytes, stream, ma, mb, M, N, (int)kp, tm, tn,
+                          tiles(kPairTile), (int)big, E, A.unit, stride_ru, B.unit, stride_cu, status);
+  }
+  // bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing past it
+  const int bulk = (!E.symmetric && !E.tri && E.mode == kEpiStore && (N & 3) == 0 && (E.ldc & 3) == 0 && (E.strideC & 3) == 0 &&
+                    (((uintptr_t)E.C) & 15) == 0) ? 1 : 0;
+  CUtensorMap mc = ma;  // placeholder when the bulk-store path is not taken (never dereferenced then)
+  if (bulk && !make_store_map(&mc, E.C, M, N, E.ldc, E.strideC, batch)) return cudaErrorInvalidValue;
+  return launch_chained(gemm128_kernel<HalfKind>, dim3(tiles(TBM), batch), kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, A.unit,
+                        stride_ru, B.unit, stride_cu, bulk, status);
+}
+
+}  // namespace hb

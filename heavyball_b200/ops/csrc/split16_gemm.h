@@ -1,0 +1,33 @@
+// fp32 GEMM at near-fp32 accuracy from products of fp16 pairs, with the epilogues of tf32_gemm.h (see split16_gemm.cu).
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "tf32_gemm.h"
+
+namespace hb {
+
+// Operand: [rows, 2 * kp] fp16 with kp = K rounded up to 64; a row holds [hi | lo], hi = fp16(x 2^e), lo = fp16((x 2^e - hi) 2^11),
+// where the exponent e of the row takes its largest value to [2^14, 2^15); columns [K, kp) of both halves are zero.  `unit` holds 2^-e per
+// row, [batch, split16_units(rows)] (padded to whole tiles; the padding is read but never reaches a result).
+inline int64_t split16_kp(int64_t K) { return (K + 63) / 64 * 64; }
+inline int64_t split16_units(int64_t rows) { return (rows + 255) / 256 * 256; }
+
+struct Split16Operand {
+  void* data;    // fp16
+  float* unit;
+};
+
+// src: [batch, R, C] fp32 (row stride ld_src, batch stride stride_src).  Writes either or both operands (data null = not wanted):
+//   same : rows = src rows, K = C;   trans: rows = src columns, K = R
+cudaError_t launch_split16(const float* src, int64_t ld_src, int64_t stride_src, int R, int C, int batch, Split16Operand same,
+                           Split16Operand trans, cudaStream_t stream);
+
+// out[b] = epilogue(A[b] * B[b]^T); epilogue and flags as for launch_tf32_gemm, without split outputs (E.S null).
+cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N, int K, int batch, const Tf32Epilogue& E, int* status,
+                                cudaStream_t stream);
+
+// Tile choice: 0 = by problem size, 128 or 256 = forced (tests and measurements).
+void set_split16_gemm_tile_override(int tile);
+
+}  // namespace hb

@@ -24,349 +24,26 @@
 // Waits are bounded as in the bf16 kernels: on expiry the CTA flags `status`, drains, frees TMEM and returns.
 #include "tf32_gemm.h"
 
+#include "gemm_epilogue.cuh"
 #include "per_device.h"
-#include "tc_common.cuh"
 
 namespace hb {
 namespace {
 
-constexpr int TBM = 128, TBN = 128, TBK = 32;
-constexpr int kTStages = 3;
-constexpr int kTTileBytes = TBM * TBK * 4;           // 16 KiB per operand tile
-constexpr int kTStageBytes = 2 * kTTileBytes;
-constexpr int kTSmemBytes = kTStages * kTStageBytes + 1024;
-constexpr int kTThreads = 192;
-constexpr uint32_t kTTmemCols = 128;
+constexpr int TBK = 32;
 // tf32 x tf32 -> fp32, both operands K-major, M = 128, N = 128
 constexpr uint32_t kTf32InstrDesc =
     (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TBN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
 
-__device__ __forceinline__ float tf32_hi(float x) {
-  uint32_t bits;
-  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(bits) : "f"(x));
-  return __uint_as_float(bits);
-}
-
-__device__ __forceinline__ float lerp_w(float s, float x, float w) { return s * (1.0f - w) + x * w; }
-
-constexpr int kStageLd = 36;                         // floats per staged row: rows stay 16-byte aligned and float4
-                                                     // accesses of a quarter-warp fall into distinct banks
-constexpr int kStageWarpBytes = 32 * kStageLd * 4;   // one warp's 32 rows x 32 columns
-
-// Fused epilogue of one warp: its 32 accumulator rows of the 128x128 tile, 32 columns at a time.  A thread reads
-// its own row from tensor memory; global memory wants the other orientation (consecutive lanes on consecutive
-// columns), so the block is turned through the warp's `stage` in shared memory (the idle operand ring):
-//   pass 1 (lane = row):                   accumulators * alpha -> stage
-//   pass 2 (8 lanes per row, 4 rows/step): moments, lerp, C store, split-operand store - every global access is a full
-//                                          128-byte line per row; the final values go back to the stage when needed
-//   pass 3 (lane = row):                   outputs that run along the rows: transposed split operand, mirror tile
-// Values outside [M, N] are never stored; the zero padding of a split output (columns [K, kp) of the operand being
-// produced) is.
-// `tmem_warp`: tensor-memory address of the warp's first row and the tile's first column; `row0` / `col_base`: their
-// global indices; `n_cb`: 32-column blocks in the tile; `off_diagonal`: the tile is not on the diagonal (mirror stores).
-// `zero_acc`: the tile had no product (its accumulator was never written): the values are zeros.
-__device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, float* stage, int row0, int col_base, int n_cb,
-                                                bool off_diagonal, bool zero_acc, int batch, int M, int N,
-                                                const Tf32Epilogue& E) {
-  const int64_t b64 = batch;
-  const bool state_vec = (N & 3) == 0;
-  const bool c_vec = (E.ldc & 3) == 0 && ((E.strideC & 3) == 0) && ((((uintptr_t)E.C) & 15) == 0);
-  const bool moments = E.mode == kEpiAdam || E.mode == kEpiLaProp;
-  const bool mirror = E.symmetric && off_diagonal && E.C != nullptr;
-  const bool along_rows = mirror || (E.S != nullptr && E.s_transposed);
-  const bool s_rows = E.S != nullptr && !E.s_transposed;
-  const int sub = lane >> 3, cg = (lane & 7) * 4;
-  const float w1 = 1.0f - E.b1, w2 = 1.0f - E.b2;
-  float* mine = stage + lane * kStageLd;
-#pragma unroll 1
-  for (int cb = 0; cb < n_cb; ++cb) {
-    const int col0 = col_base + cb * 32;
-    {
-      uint32_t acc[32];
-      if (!zero_acc) {
-        tmem_ld32(tmem_warp + (uint32_t)(cb * 32), acc);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] = 0u;
-      }
-#pragma unroll
-      for (int q = 0; q < 8; ++q)
-        *(float4*)(mine + q * 4) =
-            make_float4(__uint_as_float(acc[q * 4]) * E.alpha, __uint_as_float(acc[q * 4 + 1]) * E.alpha,
-                        __uint_as_float(acc[q * 4 + 2]) * E.alpha, __uint_as_float(acc[q * 4 + 3]) * E.alpha);
-    }
-    __syncwarp();
-
-    const int col = col0 + cg;
-    // What the epilogue reads from global memory (moments, or the old value of C) is fetched four steps at a time
-    // before the first of them is used: a step-by-step load -> compute -> store chain pays one memory round trip per step
-    // (stores may alias the next step's loads, so the compiler cannot hoist them), which for the small products of a
-    // blocked solve was longer than the product itself.
-    const bool fast_state = moments && state_vec && col + 3 < N;
-    const bool fast_old = (E.mode == kEpiLerp || E.mode == kEpiAdd) && E.C != nullptr && c_vec && col + 3 < N;
-    float4 pa[4], pb[4];
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
-    if (fast_state || fast_old) {
-#pragma unroll
-      for (int i4 = 0; i4 < 4; ++i4) {
-        const int row = row0 + (half * 4 + i4) * 4 + sub;
-        pa[i4] = make_float4(0.f, 0.f, 0.f, 0.f);
-        pb[i4] = pa[i4];
-        if (row < M) {
-          if (fast_state) {
-            pa[i4] = *(const float4*)(E.m + (b64 * M + row) * (int64_t)N + col);
-            pb[i4] = *(const float4*)(E.v + (b64 * M + row) * (int64_t)N + col);
-          } else {
-            pa[i4] = *(const float4*)(E.C + b64 * E.strideC + (int64_t)row * E.ldc + col);
-          }
-        }
-      }
-    }
-#pragma unroll
-    for (int i4 = 0; i4 < 4; ++i4) {
-      const int it = half * 4 + i4;
-      const int lr = it * 4 + sub, row = row0 + lr;
-      float* sp = stage + lr * kStageLd + cg;
-      const float4 x4 = *(const float4*)sp;
-      float x[4] = {x4.x, x4.y, x4.z, x4.w};
-      if (row < M && col < N) {
-        if (moments) {
-          float* mp = E.m + (b64 * M + row) * (int64_t)N + col;
-          float* vp = E.v + (b64 * M + row) * (int64_t)N + col;
-          const bool fast = fast_state;
-          float m4[4], s4[4];
-          if (fast) {
-            const float4 a = pa[i4], c = pb[i4];
-            m4[0] = a.x; m4[1] = a.y; m4[2] = a.z; m4[3] = a.w;
-            s4[0] = c.x; s4[1] = c.y; s4[2] = c.z; s4[3] = c.w;
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              m4[e] = col + e < N ? mp[e] : 0.f;
-              s4[e] = col + e < N ? vp[e] : 0.f;
-            }
-          }
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            s4[e] = lerp_w(s4[e], x[e] * x[e], w2);
-            const float d = fmaxf(sqrtf(s4[e]), E.eps);
-            if (E.mode == kEpiAdam) {
-              m4[e] = lerp_w(m4[e], x[e], w1);
-              x[e] = m4[e] / d;
-            } else {
-              m4[e] = lerp_w(m4[e], x[e] / d, w1);
-              x[e] = m4[e];
-            }
-          }
-          if (fast) {
-            *(float4*)mp = make_float4(m4[0], m4[1], m4[2], m4[3]);
-            *(float4*)vp = make_float4(s4[0], s4[1], s4[2], s4[3]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (col + e < N) { mp[e] = m4[e]; vp[e] = s4[e]; }
-          }
-        }
-        if (E.C != nullptr) {
-          float* cp = E.C + b64 * E.strideC + (int64_t)row * E.ldc + col;
-          const bool fast = c_vec && col + 3 < N;
-          if (E.mode == kEpiLerp || E.mode == kEpiAdd) {
-            // lerp: o + (x - o) w;  add: o + x  (the same expression with the old value left out of the difference)
-            const float keep = E.mode == kEpiLerp ? 1.f : 0.f, w = E.mode == kEpiLerp ? E.w : 1.f;
-            if (fast) {
-              const float4 o = pa[i4];
-              x[0] = o.x + (x[0] - keep * o.x) * w; x[1] = o.y + (x[1] - keep * o.y) * w;
-              x[2] = o.z + (x[2] - keep * o.z) * w; x[3] = o.w + (x[3] - keep * o.w) * w;
-            } else {
-#pragma unroll
-              for (int e = 0; e < 4; ++e)
-                if (col + e < N) { const float o = cp[e]; x[e] = o + (x[e] - keep * o) * w; }
-            }
-          }
-          if (fast) {
-            *(float4*)cp = make_float4(x[0], x[1], x[2], x[3]);
-          } else {
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (col + e < N) cp[e] = x[e];
-          }
-        }
-      }
-      if (s_rows && row < M && col < E.kpS) {  // operand rows = output rows, K over the output columns (zero from N to kp)
-        float* srow = E.S + b64 * E.strideS + (int64_t)row * (2 * E.kpS) + col;
-        float hi[4], lo[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const float y = col + e < N ? x[e] : 0.f;
-          hi[e] = tf32_hi(y);
-          lo[e] = tf32_hi(y - hi[e]);
-        }
-        *(float4*)srow = make_float4(hi[0], hi[1], hi[2], hi[3]);
-        *(float4*)(srow + E.kpS) = make_float4(lo[0], lo[1], lo[2], lo[3]);
-      }
-      if (along_rows) *(float4*)sp = make_float4(x[0], x[1], x[2], x[3]);
-    }
-    }
-
-    if (along_rows) {
-      __syncwarp();
-      const int row = row0 + lane;
-      float v[32];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 t = *(const float4*)(mine + q * 4);
-        v[q * 4] = t.x; v[q * 4 + 1] = t.y; v[q * 4 + 2] = t.z; v[q * 4 + 3] = t.w;
-      }
-      if (mirror && row < M) {  // consecutive lanes hold consecutive rows: one accumulator column is one contiguous line
-        float* ccol = E.C + b64 * E.strideC + row;
-#pragma unroll
-        for (int j = 0; j < 32; ++j)
-          if (col0 + j < N) ccol[(int64_t)(col0 + j) * E.ldc] = v[j];
-      }
-      if (E.S != nullptr && E.s_transposed && row < E.kpS) {
-        // operand rows = output columns, K over the output rows (zero from M up to kp)
-        float* sb = E.S + b64 * E.strideS + row;
-        const int64_t ld = 2 * E.kpS;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          if (col0 + j < N) {
-            const float y = row < M ? v[j] : 0.f;
-            const float hi = tf32_hi(y);
-            float* dst = sb + (int64_t)(col0 + j) * ld;
-            dst[0] = hi;
-            dst[E.kpS] = tf32_hi(y - hi);
-          }
-        }
-      }
-    }
-    __syncwarp();  // the stage is rewritten by the next block of columns
+struct Tf32Kind {
+  static constexpr int kBlock = TBK;
+  static constexpr bool kScaled = false, kCrossFirst = false;
+  static constexpr int kTermLoA = 2, kTermLoB = 1;  // A: hi, hi, lo   B: hi, lo, hi
+  static constexpr uint32_t kDesc = kTf32InstrDesc;
+  __device__ static __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, uint32_t accumulate) {
+    tc_mma_tf32(d, a, b, desc, accumulate);
   }
-}
-
-__global__ void __launch_bounds__(kTThreads, 2)
-tf32_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                 const __grid_constant__ CUtensorMap map_c, int M, int N, int kp, const Tf32Epilogue E, int bulk_store,
-                 int* status) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kTStages];
-  __shared__ __align__(8) uint64_t empty_bar[kTStages];
-  __shared__ __align__(8) uint64_t accum_bar, drain_bar;  // drain_bar: teardown only
-  __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_flag;
-
-  if (status != nullptr && *(volatile const int*)status != 0) return;  // an earlier CTA gave up: do not pile on
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tiles_n = (N + TBN - 1) / TBN;
-  int tm = blockIdx.x / tiles_n, tn = blockIdx.x % tiles_n;
-  if (E.symmetric) {  // blockIdx.x counts the tiles on or above the diagonal, row by row
-    int left = blockIdx.x;
-    tm = 0;
-    while (left >= tiles_n - tm) { left -= tiles_n - tm; ++tm; }
-    tn = tm + left;
-  }
-  const int batch = blockIdx.y;
-  int kb_lo = 0, kb_hi = kp / TBK;  // K blocks of one term of the split product that this tile walks
-  if (E.tri) {
-    kb_lo = min(kb_hi, tm * (TBM / TBK));
-    kb_hi = tn < tm ? kb_lo : min(kb_hi, (tn + 1) * (TBN / TBK));
-  }
-  const int seg_kb = kb_hi - kb_lo;
-  const int num_kb = 3 * seg_kb;    // hi*hi, hi*lo, lo*hi
-  const float alpha = E.alpha;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kTStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    mbar_init(&accum_bar, 1);
-    mbar_init(&drain_bar, 1);
-    abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) { tmem_alloc(&tmem_base_slot, kTTmemCols); tmem_relinquish(); }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-
-  int issued = 0;
-  if (warp == 0) {
-    if (lane == 0) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const int s = kb % kTStages, round = kb / kTStages;
-        if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag)) break;
-        uint8_t* dst = tiles + s * kTStageBytes;
-        const int seg = kb / seg_kb, k0 = (kb_lo + kb - seg * seg_kb) * TBK;
-        mbar_expect_tx(&full_bar[s], kTStageBytes);
-        tma_load_3d(dst, &map_a, &full_bar[s], k0 + (seg == 2 ? kp : 0), tm * TBM, batch);               // hi, hi, lo
-        tma_load_3d(dst + kTTileBytes, &map_b, &full_bar[s], k0 + (seg == 1 ? kp : 0), tn * TBN, batch);  // hi, lo, hi
-        issued = kb + 1;
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int s = kb % kTStages, round = kb / kTStages;
-        ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t a_addr = smem_u32(tiles + s * kTStageBytes);
-        const uint64_t a_desc = make_smem_desc(a_addr), b_desc = make_smem_desc(a_addr + kTTileBytes);
-#pragma unroll
-        for (int k = 0; k < TBK / 8; ++k)  // 8 fp32 = 32 B along K inside the swizzle atom = +2 address units
-          tc_mma_tf32(tmem_base, a_desc + 2 * k, b_desc + 2 * k, kTf32InstrDesc, (kb | k) ? 1u : 0u);
-        tc_commit(&empty_bar[s]);
-      }
-      if (ok) tc_commit(&accum_bar);
-    }
-  } else {
-    const int quarter = warp & 3, r = quarter * 32 + lane;
-    const bool have = (num_kb == 0) || mbar_wait(&accum_bar, 0, &abort_flag);
-    tc_fence_after();
-    if (have && bulk_store) {
-      // every load has landed and every MMA has retired: the ring is free and stages the output tile as four
-      // [128 rows x 32 fp32] boxes in the swizzled layout the bulk store expects
-#pragma unroll 1
-      for (int cb = 0; cb < TBN / 32; ++cb) {
-        uint32_t acc[32];
-        tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32), acc);
-        tmem_ld_wait();
-        uint8_t* box = tiles + cb * kTTileBytes;
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          *(float4*)(box + swz(r, q)) =
-              make_float4(__uint_as_float(acc[q * 4]) * alpha, __uint_as_float(acc[q * 4 + 1]) * alpha,
-                          __uint_as_float(acc[q * 4 + 2]) * alpha, __uint_as_float(acc[q * 4 + 3]) * alpha);
-      }
-    } else if (have) {
-      epilogue_direct(tmem_base + ((uint32_t)(quarter * 32) << 16), lane, (float*)(tiles + quarter * kStageWarpBytes),
-                      tm * TBM + quarter * 32, tn * TBN, TBN / 32, tm != tn, num_kb == 0, batch, M, N, E);
-    }
-    tc_fence_before();
-    if (bulk_store) {
-      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (have && warp == 2 && lane == 0) {
-#pragma unroll
-        for (int cb = 0; cb < TBN / 32; ++cb)
-          if (tn * TBN + cb * 32 < N) tma_store_3d(&map_c, tiles + cb * kTTileBytes, tn * TBN + cb * 32, tm * TBM, batch);
-        asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-        asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
-      }
-    }
-  }
-
-  __syncthreads();
-  if (abort_flag) {  // after an expired wait: loads and products in flight end before shared and tensor memory go away
-    if (warp == 0 && lane == 0) ring_drain(full_bar, issued, kTStages);
-    if (warp == 1 && lane == 0) products_drain(&drain_bar);
-    __syncthreads();
-    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
-  }
-  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTTmemCols); }
-}
+};
 
 // ------------------------------------------------------------------------------------------ 256 x 256 tiles
 // A 128 x 128 tile asks the L2 for 32 KiB of operands per 256 tensor-core cycles (tf32 runs at half the bf16 rate on
@@ -470,7 +147,7 @@ tf32_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     tc_fence_after();
     const int row0 = tm * TBM2 + half * 128 + quarter * 32;
     if (have && row0 < M)
-      epilogue_direct(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 256), lane,
+      epilogue_direct<false>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 256), lane,
                       (float*)(tiles + (warp - 2) * kStageWarpBytes), row0, tn * TBN2, TBN2 / 32, tm != tn, num_kb == 0,
                       batch, M, N, E);
     tc_fence_before();
@@ -592,7 +269,7 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess)
     e = configured.get(device, cudaSuccess, &done, [](bool&) {
-      const cudaError_t s = cudaFuncSetAttribute(tf32_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
+      const cudaError_t s = cudaFuncSetAttribute(gemm128_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
       return s != cudaSuccess ? s : cudaFuncSetAttribute(tf32_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes2);
     });
   if (e != cudaSuccess) return e;
@@ -627,8 +304,7 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   if (bulk && !make_f32_map(&mc, E.C, M, N, E.ldc, E.strideC, batch)) return cudaErrorInvalidValue;
   const int tiles_m = (M + TBM - 1) / TBM, tiles_n = (N + TBN - 1) / TBN;
   dim3 grid(E.symmetric ? tiles_n * (tiles_n + 1) / 2 : tiles_m * tiles_n, batch);
-  tf32_gemm_kernel<<<grid, kTThreads, kTSmemBytes, stream>>>(ma, mb, mc, M, N, (int)kp, E, bulk, status);
-  return cudaGetLastError();
+  return launch_chained(gemm128_kernel<Tf32Kind>, grid, kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, nullptr, 0, nullptr, 0, bulk, status);
 }
 
 }  // namespace hb

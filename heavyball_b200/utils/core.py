@@ -454,20 +454,26 @@ def apply_flat_add(params: List[Tensor], update: Tensor, alpha):
 # ---------------------------------------------------------------------------------------- tensor-core products
 
 
-def _tc_matmul(a: Tensor, b: Tensor, ta: bool = False, tb: bool = False, upper_upper: bool = False):
-    """``op(a) @ op(b)`` on the split-tf32 tensor-core kernel when it applies (fp32 CUDA matrices on sm_100a with
-    every dimension >= 128 and ``utils.tensor_core_matmul`` on), else ``None``."""
+# Two tensor-core products of fp32 matrices exist: of fp16 pairs (the faster and more exact one) and split-tf32.  Everything that an
+# eigenbasis is made from - statistics, power iteration, orthogonalisation, the rotation of the moments that follows - asks for the
+# second (``pairs=False``): eigenvectors with nearly equal Rayleigh quotients trade places when the last bits of any of these change,
+# so moving them would move every trajectory (two refreshes of eleven 2048-wide bases: one to three such pairs).
+
+
+def _tc_matmul(a: Tensor, b: Tensor, ta: bool = False, tb: bool = False, upper_upper: bool = False, pairs: bool = True):
+    """``op(a) @ op(b)`` on a tensor-core kernel when it applies (fp32 CUDA matrices on sm_100a with every dimension >= 128 and
+    ``utils.tensor_core_matmul`` on), else ``None``."""
     if not (a.is_cuda and getattr(_settings(), "tensor_core_matmul", True)):
         return None
     from .. import ops
 
     if not ops.matmul_supported(a, b):
         return None
-    return ops.matmul3(a, b, ta, tb, upper_upper=upper_upper)
+    return (ops.matmul16 if pairs else ops.matmul3)(a, b, ta, tb, upper_upper=upper_upper)
 
 
-def _mm(a: Tensor, b: Tensor, ta: bool = False, tb: bool = False) -> Tensor:
-    out = _tc_matmul(a, b, ta, tb)
+def _mm(a: Tensor, b: Tensor, ta: bool = False, tb: bool = False, pairs: bool = True) -> Tensor:
+    out = _tc_matmul(a, b, ta, tb, pairs=pairs)
     return out if out is not None else (a.mT if ta else a) @ (b.mT if tb else b)
 
 
@@ -496,7 +502,7 @@ def _leaf_inverses(q: Tensor):
     return ops.load().tri_inv_blocks(q)
 
 
-def _tc_sub_product(c: Tensor, a: Tensor, b: Tensor, b_transposed: bool = False) -> bool:
+def _tc_sub_product(c: Tensor, a: Tensor, b: Tensor, b_transposed: bool = False, pairs: bool = True) -> bool:
     """``c -= a @ b`` (``b_transposed``: ``c -= a @ b^T``) in place on the view ``c`` with the subtraction in the
     product's epilogue and the operands split straight from their views; ``False`` when the tensor-core path does not
     apply (the caller then uses plain tensor arithmetic)."""
@@ -504,21 +510,24 @@ def _tc_sub_product(c: Tensor, a: Tensor, b: Tensor, b_transposed: bool = False)
         return False
     from .. import ops
 
-    K = a.shape[-1]
-    if not ops.available() or min(c.shape[-2], c.shape[-1], K) < 128:
+    if not ops.available() or min(c.shape[-2], c.shape[-1], a.shape[-1]) < 128:
         return False
     if any(t.stride(-1) != 1 or t.dtype != torch.float32 for t in (a, b, c)) or c.data_ptr() % 16 or c.stride(-2) % 4 or c.stride(0) % 4:
         return False
-    a_s, _ = ops.tf32_split(a, True, False)
+    split = ops.split16 if pairs else ops.tf32_split
+    a_s, _ = split(a, True, False)
     if b_transposed:
-        b_s = a_s if (b.data_ptr() == a.data_ptr() and b.shape == a.shape and b.stride() == a.stride()) else ops.tf32_split(b, True, False)[0]
+        b_s = a_s if (b.data_ptr() == a.data_ptr() and b.shape == a.shape and b.stride() == a.stride()) else split(b, True, False)[0]
     else:
-        b_s = ops.tf32_split(b, False, True)[1]
-    ops.tf32_gemm(a_s, b_s, K, mode=ops.EPI_ADD, alpha=-1.0, out=c)
+        b_s = split(b, False, True)[1]
+    if pairs:
+        ops.split16_gemm(a_s, b_s, mode=ops.EPI_ADD, alpha=-1.0, out=c)
+    else:
+        ops.tf32_gemm(a_s, b_s, a.shape[-1], mode=ops.EPI_ADD, alpha=-1.0, out=c)
     return True
 
 
-def _solve_right_upper_into(q: Tensor, b: Tensor, x: Tensor, inv: Tensor, first_block: int):
+def _solve_right_upper_into(q: Tensor, b: Tensor, x: Tensor, inv: Tensor, first_block: int, pairs: bool):
     """``x <- b q^-1`` for upper-triangular ``q`` through the leaf inverses ``inv``; ``b`` is consumed (its columns to the
     right receive the updates in place).  All three are views with unit inner stride; nothing is allocated besides the
     split operands, nothing is concatenated."""
@@ -527,13 +536,14 @@ def _solve_right_upper_into(q: Tensor, b: Tensor, x: Tensor, inv: Tensor, first_
         torch.bmm(b, inv[:, first_block, :d, :d], out=x)
         return
     h = max(_TRSM_LEAF, (d // 2) // _TRSM_LEAF * _TRSM_LEAF)
-    _solve_right_upper_into(q[..., :h, :h], b[..., :h], x[..., :h], inv, first_block)
-    if not _tc_sub_product(b[..., h:], x[..., :h], q[..., :h, h:]):
+    _solve_right_upper_into(q[..., :h, :h], b[..., :h], x[..., :h], inv, first_block, pairs)
+    if not _tc_sub_product(b[..., h:], x[..., :h], q[..., :h, h:], pairs=pairs):
         torch.baddbmm(b[..., h:], x[..., :h], q[..., :h, h:], alpha=-1.0, out=b[..., h:])
-    _solve_right_upper_into(q[..., h:, h:], b[..., h:], x[..., h:], inv, first_block + h // _TRSM_LEAF)
+    _solve_right_upper_into(q[..., h:, h:], b[..., h:], x[..., h:], inv, first_block + h // _TRSM_LEAF, pairs)
 
 
-def _solve_right_upper(q: Tensor, b: Tensor, inv: Optional[Tensor] = None, first_block: int = 0, consume_b: bool = False) -> Tensor:
+def _solve_right_upper(q: Tensor, b: Tensor, inv: Optional[Tensor] = None, first_block: int = 0, consume_b: bool = False,
+                       pairs: bool = True) -> Tensor:  # fmt: skip
     """``X`` with ``X q = b`` for upper-triangular ``q`` (batched).  Large CUDA problems are split recursively,
     ``X_1 = b_1 q_11^-1``, ``X_2 = (b_2 - X_1 q_12) q_22^-1``, so that everything is matrix products: the off-diagonal
     updates run on the tensor cores (subtraction in the epilogue, in place), and the 128-wide leaves multiply by block
@@ -548,15 +558,15 @@ def _solve_right_upper(q: Tensor, b: Tensor, inv: Optional[Tensor] = None, first
     if fast and inv is not None and q.ndim == 3 and b.ndim == 3 and b.dtype == torch.float32:
         work = b if (consume_b and b.stride(-1) == 1) else b.clone(memory_format=torch.contiguous_format)
         x = torch.empty(b.shape, device=b.device, dtype=b.dtype)
-        _solve_right_upper_into(q, work, x, inv, first_block)
+        _solve_right_upper_into(q, work, x, inv, first_block, pairs)
         return x
     if d <= _TRSM_LEAF or not fast:
         if inv is not None and fast:
             return b @ inv[:, first_block, :d, :d]
         return torch.linalg.solve_triangular(q, b, upper=True, left=False)
     h = max(_TRSM_LEAF, (d // 2) // _TRSM_LEAF * _TRSM_LEAF)
-    x1 = _solve_right_upper(q[..., :h, :h], b[..., :h], inv, first_block)
-    x2 = _solve_right_upper(q[..., h:, h:], b[..., h:] - _mm(x1, q[..., :h, h:]), inv, first_block + h // _TRSM_LEAF)
+    x1 = _solve_right_upper(q[..., :h, :h], b[..., :h], inv, first_block, pairs=pairs)
+    x2 = _solve_right_upper(q[..., h:, h:], b[..., h:] - _mm(x1, q[..., :h, h:], pairs=pairs), inv, first_block + h // _TRSM_LEAF, pairs=pairs)
     return torch.cat([x1, x2], dim=-1)
 
 

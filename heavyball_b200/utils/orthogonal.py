@@ -232,10 +232,10 @@ def _chol_upper_blocked(G: Tensor, R: Tensor, bad: Tensor, lo: int, hi: int, inv
     mid = lo + max(_CHOL_LEAF, (n // 2) // _CHOL_LEAF * _CHOL_LEAF)
     _chol_upper_blocked(G, R, bad, lo, mid, inv)
     # X^T R11 = G12^T  <=>  X = R11^-T G12 = R12
-    xt = _solve_right_upper(R[:, lo:mid, lo:mid], G[:, lo:mid, mid:hi].mT.contiguous(), inv, lo // _CHOL_LEAF, consume_b=True)
+    xt = _solve_right_upper(R[:, lo:mid, lo:mid], G[:, lo:mid, mid:hi].mT.contiguous(), inv, lo // _CHOL_LEAF, consume_b=True, pairs=False)
     R[:, lo:mid, mid:hi] = xt.mT
-    if not _tc_sub_product(G[:, mid:hi, mid:hi], xt, xt, b_transposed=True):  # Schur complement, upper tiles mirrored
-        G[:, mid:hi, mid:hi] -= _mm(xt, xt, False, True)
+    if not _tc_sub_product(G[:, mid:hi, mid:hi], xt, xt, b_transposed=True, pairs=False):  # Schur complement, upper tiles mirrored
+        G[:, mid:hi, mid:hi] -= _mm(xt, xt, False, True, pairs=False)
     _chol_upper_blocked(G, R, bad, mid, hi, inv)
 
 
@@ -273,17 +273,17 @@ def _cholesky_qr2(x: Tensor, shifted_rounds: int = 0):
     rounds = shifted_rounds + 2
     info = torch.zeros_like(bad)  # failed leaves do not decide: what counts is the orthogonality reached at the end
     for rnd in range(rounds):
-        gram = _mm(a, a, True, False)
+        gram = _mm(a, a, True, False, pairs=False)
         if rnd < shifted_rounds:
             # unit columns: the diagonal is 1 and lambda_max <= k
             gram.diagonal(dim1=-2, dim2=-1).add_(_CHOLQR_SHIFT * k)
         r = torch.zeros_like(gram)
         inv = _leaf_inverse_buffer(gram)
         _chol_upper_blocked(gram, r, info, 0, k, inv)
-        a = _solve_right_upper(r, a, inv, 0, consume_b=rnd > 0 or a.data_ptr() != x.data_ptr())
+        a = _solve_right_upper(r, a, inv, 0, consume_b=rnd > 0 or a.data_ptr() != x.data_ptr(), pairs=False)
         if rnd < shifted_rounds:  # columns shrank by different amounts: back to unit columns for the next round
             a = a / a.norm(dim=-2, keepdim=True).clamp_(min=tiny)
-    bad += (_mm(a, a, True, False) - eye).abs().amax(dim=(-2, -1)).gt(_CHOLQR_ACCEPT)
+    bad += (_mm(a, a, True, False, pairs=False) - eye).abs().amax(dim=(-2, -1)).gt(_CHOLQR_ACCEPT)
     bad += (~torch.isfinite(a)).flatten(1).any(dim=1)
     return a.reshape(*batch, n, k), bad
 

@@ -1,0 +1,114 @@
+"""fp16-pair operands and products on a B200 against 64-bit products: edges of tiles and K blocks, every epilogue, wide ranges."""
+
+import pytest
+import torch
+
+from heavyball_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(params=[0, 128, 256], ids=["tile-auto", "tile-128", "tile-256"])
+def tile(request):
+    ext = ops.load()
+    ext.set_split16_gemm_tile(request.param)
+    yield request.param
+    ext.set_split16_gemm_tile(0)
+
+
+def _rand(*shape, seed):
+    return torch.randn(*shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
+
+
+def _off(got, a, b, want=None):
+    """Largest error in units of its bound: 22 bits of either operand and the dropped product of low parts (4 units of 2^-22), and one
+    rounding of the accumulator per 16 of K in the last of three walks plus a few for the first two (2^-23 of |a| |b| each)."""
+    K = a.shape[-1]
+    bound = (a.abs() @ b.abs().mT) * (2.0**-20 + (K / 16 + 4) * 2.0**-23)
+    return float(((got.double() - (a @ b.mT if want is None else want)).abs() / bound.clamp_min(1e-300)).max())
+
+
+EDGES = [(1, 128, 128, 64), (2, 127, 129, 65), (1, 257, 255, 193), (3, 1, 256, 1), (1, 2048, 384, 1000), (2, 300, 1030, 3)]
+
+
+@pytest.mark.parametrize("B,M,N,K", EDGES)
+def test_products_and_both_orientations(B, M, N, K, tile):
+    a, b = _rand(B, M, K, seed=1), _rand(B, N, K, seed=2)
+    wide = torch.full((B, M, N + 5), -7.0, device="cuda")
+    out = wide[..., :N]
+    ops.split16_gemm(ops.split16(a)[0], ops.split16(b)[0], out=out)
+    assert _off(out, a.double(), b.double()) < 1 and bool((wide[..., N:] == -7.0).all())
+    at, bt = (torch.empty(B, K, t.shape[1] + 3, device="cuda")[..., : t.shape[1]].copy_(t.mT) for t in (a, b))  # views, odd row strides
+    again = torch.empty(B, M, N, device="cuda")
+    ops.split16_gemm(ops.split16(at, False, True)[1], ops.split16(bt, False, True)[1], out=again)
+    assert torch.equal(again, out)
+    ops.check_status()
+
+
+@pytest.mark.parametrize("R,C", [(5504, 33), (31, 2500), (256, 1024), (257, 1025), (2304, 64)])
+def test_operand_of_either_orientation_holds_the_values(R, C):
+    """Rows longer than a warp keeps, strips shared by one to eight blocks and by fewer blocks than rows need; padding is zero."""
+    x = _rand(2, R, C, seed=3) * torch.logspace(-6, 6, C, device="cuda") * torch.logspace(8, -8, R, device="cuda")[:, None]
+    for op, rows in zip(ops.split16(x, True, True), (x, x.mT)):
+        kp, n, K = op.data.shape[2] // 2, *rows.shape[1:]
+        hi, lo = op.data[..., :kp].double(), op.data[..., kp:].double() / 2048
+        got = (hi + lo) * op.unit[:, :n, None].double()
+        top = rows.double().abs().amax(-1, keepdim=True)
+        assert float(hi.abs().max()) <= 2**15 and float(hi.abs().amax(-1).min()) >= 2**14
+        assert bool(((got[..., :K] - rows.double()).abs() <= torch.maximum(rows.double().abs() * 2.0**-22, top * 2.0**-50)).all())
+        assert bool((op.data[..., K:kp] == 0).all()) and bool((op.data[..., kp + K :] == 0).all())
+
+
+@pytest.mark.parametrize("B,M,N,K", [(2, 200, 136, 160), (1, 520, 264, 70)])
+@pytest.mark.parametrize("mode", ["lerp", "add", "adam", "laprop"])
+def test_epilogues(mode, B, M, N, K, tile):
+    a, b, old = _rand(B, M, K, seed=4), _rand(B, N, K, seed=5), _rand(B, M, N, seed=6)
+    x, out = a.double() @ b.double().mT, old.clone()
+    pa, pb = ops.split16(a)[0], ops.split16(b)[0]
+    if mode in ("lerp", "add"):
+        kwargs = dict(mode=ops.EPI_LERP, w=0.25) if mode == "lerp" else dict(mode=ops.EPI_ADD, alpha=-1.0)
+        ops.split16_gemm(pa, pb, out=out, **kwargs)
+        want = old.double() * 0.75 + 0.25 * x if mode == "lerp" else old.double() - x
+        assert float((out.double() - want).abs().max()) < 1e-5 * float((a.abs() @ b.abs().mT).max())
+        return
+    m, v = _rand(B, M, N, seed=7) * 0.1, _rand(B, M, N, seed=8).abs()
+    m64, v64 = m.double(), v.double() * 0.95 + x * x * (1 - 0.95)
+    d = v64.sqrt().clamp(min=1e-8)
+    m64 = m64 * 0.9 + (x if mode == "adam" else x / d) * (1 - 0.9)
+    ops.split16_gemm(pa, pb, mode=ops.EPI_ADAM if mode == "adam" else ops.EPI_LAPROP, b1=0.9, b2c=0.95, eps=1e-8, m=m, v=v, out=out)
+    # 0.95 and 0.9 in fp32 (2^-24 each) and the approximate square root and quotient (2 ulp) dominate the product's error
+    for got, want in ((m, m64), (v, v64), (out, m64 / d if mode == "adam" else m64)):
+        assert float((got.double() - want).abs().max()) < 2e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("B,n,K", [(2, 129, 64), (1, 520, 200), (3, 256, 512)])
+def test_symmetric_and_triangular_products(B, n, K, tile):
+    x = _rand(B, n, K, seed=9)
+    op, out = ops.split16(x)[0], torch.empty(B, n, n, device="cuda")
+    ops.split16_gemm(op, op, out=out)
+    assert _off(out, x.double(), x.double()) < 1
+    r, s = _rand(B, n, n, seed=10).triu(), _rand(B, n, n, seed=11).triu()
+    got = ops.matmul16(r, s, upper_upper=True)
+    assert _off(got, r.double(), s.double().mT) < 1 and float(got.tril(-1).abs().max()) == 0
+    ops.check_status()
+
+
+def test_ranges_that_fp16_does_not_have(tile):
+    """Rows over sixty decades, rows of zeros, of subnormals and with an infinity or a NaN next to ordinary ones."""
+    a, b = _rand(1, 300, 96, seed=12), _rand(1, 140, 96, seed=13)
+    a, b = a * torch.logspace(-30, 30, 300, device="cuda")[:, None], b * torch.logspace(6, -6, 140, device="cuda")[:, None]
+    a[0, 7], a[0, 8], b[0, 3] = 0.0, 1e-41, 0.0
+    assert _off(ops.matmul16(a, b, False, True), torch.where(a.abs() < 2.0**-126, 0, a).double(), b.double()) < 1
+    a[0, 20, 5], a[0, 21, 6], b[0, 9, 1] = float("nan"), float("inf"), float("-inf")
+    got, general = ops.matmul16(a, b, False, True), ops.matmul3(a, b, False, True)
+    assert torch.equal(torch.isfinite(got), torch.isfinite(general)) and torch.equal(got.isnan(), general.isnan())
+
+
+def test_refused_operands():
+    a, b = ops.split16(_rand(1, 128, 64, seed=14))[0], ops.split16(_rand(1, 128, 128, seed=15))[0]
+    with pytest.raises(RuntimeError):
+        ops.split16_gemm(a, b, out=torch.empty(1, 128, 128, device="cuda"))  # contraction lengths differ
+    with pytest.raises(RuntimeError):
+        ops.split16_gemm(a, a, out=torch.empty(1, 128, 100, device="cuda"))
+    with pytest.raises(RuntimeError):
+        ops.split16(_rand(1, 64, 128, seed=16).mT)
