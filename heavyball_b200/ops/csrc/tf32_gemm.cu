@@ -69,7 +69,6 @@ tf32_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __shared__ uint32_t tmem_base_slot;
   __shared__ int abort_flag;
 
-  if (status != nullptr && *(volatile const int*)status != 0) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tiles_n = (N + TBN2 - 1) / TBN2;
@@ -97,13 +96,17 @@ tf32_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 1) { tmem_alloc(&tmem_base_slot, kTTmemCols2); tmem_relinquish(); }
+  griddep_wait();
+  const bool skip = __syncthreads_or(threadIdx.x == 0 && status != nullptr && *(volatile const int*)status != 0);
+  griddep_launch();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = tmem_base_slot;
 
   int issued = 0;
-  if (warp == 0) {
+  if (skip) {
+  } else if (warp == 0) {
     if (lane == 0) {
       for (int kb = 0; kb < num_kb; ++kb) {
         const int s = kb % kTStages, round = kb / kTStages;
@@ -171,6 +174,8 @@ __global__ void __launch_bounds__(256) tf32_split_kernel(const float* __restrict
                                                         int R, int C, float* __restrict__ dst_same,
                                                         float* __restrict__ dst_trans, int kpC, int kpR) {
   __shared__ float tile[64][65];  // [source row][source column]
+  griddep_wait();
+  griddep_launch();
   const float* s = src + (int64_t)blockIdx.z * stride_src;
   const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64;
   const int lane4 = (threadIdx.x & 15) * 4, line = threadIdx.x >> 4;
@@ -253,8 +258,7 @@ cudaError_t launch_tf32_split(const float* src, int64_t ld_src, int64_t stride_s
   if (R == 0 || C == 0 || batch == 0 || (dst_same == nullptr && dst_trans == nullptr)) return cudaSuccess;
   const int kpC = (int)tf32_split_kp(C), kpR = (int)tf32_split_kp(R);
   dim3 grid((kpC + 63) / 64, (kpR + 63) / 64, batch);
-  tf32_split_kernel<<<grid, 256, 0, stream>>>(src, ld_src, stride_src, R, C, dst_same, dst_trans, kpC, kpR);
-  return cudaGetLastError();
+  return launch_chained(tf32_split_kernel, grid, 256, 0, stream, src, ld_src, stride_src, R, C, dst_same, dst_trans, kpC, kpR);
 }
 
 static int g_tf32_tile_override = 0;  // 0 = by size, 128 / 256 = forced (tests and measurements)
@@ -293,12 +297,12 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   if (g_tf32_tile_override == 256) big = true;
   if (big) {
     dim3 grid(E.symmetric ? big_n * (big_n + 1) / 2 : big_m * big_n, batch);
-    tf32_gemm256_kernel<<<grid, kTThreads2, kTSmemBytes2, stream>>>(ma, mb, M, N, (int)kp, E, status);
-    return cudaGetLastError();
+    return launch_chained(tf32_gemm256_kernel, grid, kTThreads2, kTSmemBytes2, stream, ma, mb, M, N, (int)kp, E, status);
   }
 
-  // plain products leave through the bulk-store path; everything else is written by the epilogue threads themselves
-  const int bulk = (!E.symmetric && !E.tri && E.mode == kEpiStore && E.S == nullptr && E.C != nullptr && (E.ldc & 3) == 0 &&
+  // plain products leave through the bulk-store path (bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing
+  // past it); everything else is written by the epilogue threads themselves
+  const int bulk = (!E.symmetric && !E.tri && E.mode == kEpiStore && E.S == nullptr && E.C != nullptr && (N & 3) == 0 && (E.ldc & 3) == 0 &&
                     (E.strideC & 3) == 0 && (((uintptr_t)E.C) & 15) == 0) ? 1 : 0;
   mc = ma;  // placeholder when the bulk-store path is not taken (never dereferenced then)
   if (bulk && !make_f32_map(&mc, E.C, M, N, E.ldc, E.strideC, batch)) return cudaErrorInvalidValue;

@@ -104,6 +104,17 @@ def test_ranges_that_fp16_does_not_have(tile):
     assert torch.equal(torch.isfinite(got), torch.isfinite(general)) and torch.equal(got.isnan(), general.isnan())
 
 
+@pytest.mark.parametrize("N", [128, 129, 130, 131])
+def test_plain_stores_end_with_the_row(N):
+    """Rows of a view that end inside a 16-byte unit: nothing past them is written (bulk stores would fill the unit with zeros)."""
+    a, b = _rand(2, 200, 96, seed=17), _rand(2, N, 96, seed=18)
+    for product in (lambda out: ops.split16_gemm(ops.split16(a)[0], ops.split16(b)[0], out=out),
+                    lambda out: ops.tf32_gemm(ops.tf32_split(a)[0], ops.tf32_split(b)[0], 96, out=out)):  # fmt: skip
+        wide = torch.full((2, 200, 136), -7.0, device="cuda")
+        product(wide[..., :N])
+        assert bool((wide[..., N:] == -7.0).all()) and float((wide[..., :N] - a @ b.mT).abs().max()) < 0.1
+
+
 def test_refused_operands():
     a, b = ops.split16(_rand(1, 128, 64, seed=14))[0], ops.split16(_rand(1, 128, 128, seed=15))[0]
     with pytest.raises(RuntimeError):
