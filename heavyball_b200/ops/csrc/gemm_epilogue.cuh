@@ -357,6 +357,7 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   __shared__ int abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool leader = elect_one();  // issues the loads (warp 0) and the products (warp 1), and waits for them in the teardown
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int tiles_n = (N + TBN - 1) / TBN;
   int tm = blockIdx.x / tiles_n, tn = blockIdx.x % tiles_n;
@@ -396,7 +397,7 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   int issued = 0;
   if (skip) {
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (leader) {
       for (int kb = 0; kb < num_kb; ++kb) {
         const int s = kb % kTStages, round = kb / kTStages;
         if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag)) break;
@@ -409,7 +410,7 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (leader) {
       bool ok = true;
       for (int kb = 0; kb < num_kb && ok; ++kb) {
         const int s = kb % kTStages, round = kb / kTStages;
@@ -471,8 +472,8 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 
   __syncthreads();
   if (abort_flag) {  // after an expired wait: loads and products in flight end before shared and tensor memory go away
-    if (warp == 0 && lane == 0) ring_drain(full_bar, issued, kTStages);
-    if (warp == 1 && lane == 0) products_drain(&drain_bar);
+    if (warp == 0 && leader) ring_drain(full_bar, issued, kTStages);
+    if (warp == 1 && leader) products_drain(&drain_bar);
     __syncthreads();
     if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
   }

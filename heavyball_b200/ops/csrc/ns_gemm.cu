@@ -100,6 +100,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_c
   __shared__ int abort_flag;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool leader = elect_one();  // issues the loads (warp 0) and the products (warp 1), and waits for them in the teardown
   uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
 
   const TileAt tile = tile_at(L, blockIdx.x);
@@ -136,7 +137,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_c
   int issued = 0;  // producer: ring fills whose loads were issued
   if (skip) {
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (leader) {
       const int total = num_kb + (poly ? 1 : 0);
       for (int kb = 0; kb < total; ++kb) {
         const int s = kb % kStages, round = kb / kStages;
@@ -161,7 +162,7 @@ __global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_c
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (leader) {
       bool ok = true;
       for (int kb = 0; kb < num_kb && ok; ++kb) {
         const int s = kb % kStages, round = kb / kStages;
@@ -288,8 +289,8 @@ __global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_c
   // ---- teardown: after an expired wait, nothing may still land in shared memory or be multiplied when they are given back
   __syncthreads();
   if (abort_flag) {
-    if (warp == 0 && lane == 0) ring_drain(full_bar, issued, kStages);
-    if (warp == 1 && lane == 0) products_drain(&drain_bar);
+    if (warp == 0 && leader) ring_drain(full_bar, issued, kStages);
+    if (warp == 1 && leader) products_drain(&drain_bar);
     __syncthreads();
     if (threadIdx.x == 0 && L.status != nullptr) atomicExch(L.status, 1);
   }
@@ -327,6 +328,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
   __shared__ int fills, fill_bytes[kPairStages];            // ring fills this CTA issued, bytes of the last one of each stage
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool leader = elect_one();  // issues the loads (warp 0) and the products (warp 1), and waits for them in the teardown
   const uint32_t rank = cluster_rank();
   uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int total = L.total, pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -353,7 +355,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
 
   if (skip) {
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (leader) {
       int n = 0;  // ring fills so far
       bool ok = true;
       for (int idx = pair; idx < total && ok; idx += pairs) {
@@ -384,7 +386,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
       griddep_launch();  // this CTA's last loads are on their way: the next kernel of the chain may take over SMs that drain
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (leader && rank == 0) {
       int n = 0, it = 0;
       bool ok = true;
       for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
@@ -560,7 +562,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_
   if (threadIdx.x == 0 && abort_flag) cluster_store(cluster_addr(&abort_flag, rank ^ 1), 1);
   cluster_sync();
   if (abort_flag) {
-    if (rank == 0 && warp == 1 && lane == 0) tc_commit_pair(&drain_bar);  // the thread that issued the products
+    if (rank == 0 && warp == 1 && leader) tc_commit_pair(&drain_bar);  // the thread that issued the products
     if (threadIdx.x == 0) mbar_drain(&drain_bar, 0);
     if (rank == 0 && threadIdx.x == 0) {
       const int even = fills, odd = cluster_load(cluster_addr(&fills, 1)), top = max(even, odd);

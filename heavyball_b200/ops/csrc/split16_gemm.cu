@@ -77,6 +77,7 @@ split16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   __shared__ int fills;                                      // ring fills this CTA issued
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool leader = elect_one();  // issues the loads (warp 0) and the products (warp 1), and waits for them in the teardown
   const uint32_t rank = cluster_rank();
   uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
@@ -102,7 +103,7 @@ split16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
 
   if (skip) {
   } else if (warp == 0) {
-    if (lane == 0) {
+    if (leader) {
       int n = 0;  // ring fills so far
       bool ok = true;
       for (int idx = pair; idx < total && ok; idx += pairs) {
@@ -127,7 +128,7 @@ split16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
       griddep_launch();  // this CTA's last loads are on their way: the next kernel may take over SMs that drain
     }
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (leader && rank == 0) {
       int n = 0, it = 0;
       bool ok = true;
       for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
@@ -184,7 +185,7 @@ split16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_cons
   if (threadIdx.x == 0 && abort_flag) cluster_store(cluster_addr(&abort_flag, rank ^ 1), 1);
   cluster_sync();
   if (abort_flag) {
-    if (rank == 0 && warp == 1 && lane == 0) tc_commit_pair(&drain_bar);  // the thread that issued the products
+    if (rank == 0 && warp == 1 && leader) tc_commit_pair(&drain_bar);  // the thread that issued the products
     if (threadIdx.x == 0) mbar_drain(&drain_bar, 0);
     if (rank == 0 && threadIdx.x == 0) {
       const int even = fills, odd = cluster_load(cluster_addr(&fills, 1)), top = max(even, odd);
