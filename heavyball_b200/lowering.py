@@ -246,6 +246,20 @@ def _mark_initialized(tr: C.FunctionTransform, st: dict):
         C._mark(st, index)
 
 
+def _mark_all(prog, states: List[dict]):
+    """:func:`_mark_initialized` for every transform of the program; one set comparison for a state that carries all marks."""
+    marked = [prog.rule, prog.mars, prog.ortho, prog.post, *prog.stateless]
+    if prog.after is not None and prog.after[0] in ("msam", "hyperball"):
+        marked.append(prog.after[1])
+    marked = [tr for tr in marked if tr is not None]
+    every = frozenset(layer.index for tr in marked for layer in tr.layers if isinstance(layer, _MARKED_LAYERS))
+    for st in states:
+        done = st.get("is_initialized")
+        if not (isinstance(done, set) and every <= done):
+            for tr in marked:
+                _mark_initialized(tr, st)
+
+
 def _state_ready(tr: C.FunctionTransform, states: List[dict], ecc: bool) -> bool:
     keys = [k for layer in tr.layers if not isinstance(layer, C.AccumSlots) for k in layer.keys.values()]
     warm = [(layer.counter, len(layer.warmup_fns)) for layer in tr.layers if isinstance(layer, C.Warmup)]
@@ -481,18 +495,7 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
 
     if prog.palm is not None:
         prog.palm(None, group, None, None, None)
-    for st in states:
-        _mark_initialized(prog.rule, st)
-        if prog.mars is not None:
-            _mark_initialized(prog.mars, st)
-        if prog.ortho is not None:
-            _mark_initialized(prog.ortho, st)
-        if post is not None:
-            _mark_initialized(post, st)
-        for tr in prog.stateless:
-            _mark_initialized(tr, st)
-        if prog.after is not None and prog.after[0] in ("msam", "hyperball"):
-            _mark_initialized(prog.after[1], st)
+    _mark_all(prog, states)
 
     # ---- selection: everything (single process / replicated) or this rank's share (peer data parallelism)
     peer_in, peer_out = {}, {}
@@ -508,16 +511,15 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
         peer_in = {"g_delta": args["g_delta"], "g_scale": args["g_scale"], "g_mc_delta": args["g_mc_delta"]}
         peer_out = {"p_delta": args["p_delta"], "p_mc_delta": args["p_mc_delta"]}
     else:
-        sel = [(i, None) for i in range(len(params))]
-    pick = lambda xs: [_cut(xs[i], seg) for i, seg in sel] if len(xs) else []  # noqa: E731
+        sel = None
+    pick = lambda xs: xs if sel is None else [_cut(xs[i], seg) for i, seg in sel]  # noqa: E731
     params_v, grads_v = pick(params), pick(grads)
     if plan is not None:  # the kernels add cross-GPU offsets to these addresses: never launch on anything but slab views
         for (i, seg), pv, gv in zip(sel, params_v, grads_v):
             peer.validate(params[i], seg, pv, gv)
-    sub_states = [states[i] for i, _ in sel]
-    s0, s0e, s1, s1e, s2, s2e = (
-        [_cut(t, seg) for t, (_, seg) in zip(lst, sel)] for lst in _slots(prog.rule, sub_states, names, bool(ecc_mode))
-    )
+    sub_states = states if sel is None else [states[i] for i, _ in sel]
+    cut = lambda xs: xs if sel is None else [_cut(t, seg) for t, (_, seg) in zip(xs, sel)]  # noqa: E731
+    s0, s0e, s1, s1e, s2, s2e = (cut(lst) for lst in _slots(prog.rule, sub_states, names, bool(ecc_mode)))
     base = dict(
         dt_g=ops.dtype_code(grads[0]), dt_s=ops.dtype_code(states[0][key0], ecc_mode),
         dt_p=ops.dtype_code(params[0], pecc_mode), n_state=len(names), algo=algo,
@@ -535,11 +537,11 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
         mkey = prog.mars._val_names["mars_old_grad"]
         gamma, beta1 = utils.get_beta1(group), group["mars_gamma"]  # argument order of the transform
         mars_kw = dict(
-            mars=[_cut(st[mkey], seg) for st, (_, seg) in zip(sub_states, sel)],
-            marse=[_cut(st[mkey + "::ecc"], seg) for st, (_, seg) in zip(sub_states, sel)] if ecc_mode else [],
+            mars=cut([st[mkey] for st in sub_states]),
+            marse=cut([st[mkey + "::ecc"] for st in sub_states]) if ecc_mode else [],
             mars_a=-gamma * beta1 / (1 - beta1),
         )  # fmt: skip
-    pe = [_cut(st["param::ecc"], seg) for st, (_, seg) in zip(sub_states, sel)] if pecc_mode else []
+    pe = cut([st["param::ecc"] for st in sub_states]) if pecc_mode else []
     epilogue = dict(
         lr=group["lr"], wd=_weight_decay(rule_name, group), cautious_wd=int(bool(group.get("cautious_weight_decay", False)))
     )
@@ -559,7 +561,7 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
             group["_sf_step"] = step
         total = group["weight_sum"]
         ckp1 = C._sf_weight(group) / total if total != 0 else 0
-        z = [_cut(st[post._val_names["z"]], seg) for st, (_, seg) in zip(sub_states, sel)]
+        z = cut([st[post._val_names["z"]] for st in sub_states])
         base.update(b3=ckp1, alpha=utils.get_beta1(group))
         launch(p=params_v, g=grads_v, s0=s0, s1=s1, s2=z, out_mode=ops.OUT_SCHEDULE_FREE, seed=_seed(opt, group, 0),
                **base, **epilogue)  # fmt: skip

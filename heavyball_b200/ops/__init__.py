@@ -122,15 +122,21 @@ def load():
     return _ext
 
 
+_blackwell = {}  # device index -> compute capability 10.x (the hardware's: it holds for the life of the process)
+
+
 def available() -> bool:
     """True when kernels can run here: a CUDA device of compute capability 10.x is present.  The
     extension itself is loaded on first use and failure to load is an error, not a fallback."""
     if os.environ.get("HB200_DISABLE_OPS") == "1":
         return False
-    if not torch.cuda.is_available():
-        return False
-    major, _ = torch.cuda.get_device_capability()
-    return major == 10
+    if not torch.cuda.is_initialized():  # also in a forked child, which must not take its parent's answer
+        return torch.cuda.is_available() and torch.cuda.get_device_capability()[0] == 10
+    index = torch.cuda.current_device()
+    known = _blackwell.get(index)
+    if known is None:
+        known = _blackwell[index] = torch.cuda.get_device_capability(index)[0] == 10
+    return known
 
 
 class _LaunchCounter:

@@ -7,6 +7,8 @@
 #include <algorithm>
 #include <optional>
 #include <string>
+#include <string_view>
+#include <unordered_map>
 #include <vector>
 
 #include "colsum.h"
@@ -46,11 +48,47 @@ struct Table {
   int chunk;
 };
 
+std::vector<int> chunk_prefix(const std::vector<hb::TensorMeta>& metas, int chunk) {
+  std::vector<int> prefix(metas.size() + 1, 0);
+  for (size_t i = 0; i < metas.size(); ++i) prefix[i + 1] = prefix[i] + (int)((metas[i].numel + chunk - 1) / chunk);
+  return prefix;
+}
+
+// The settings of a fused-chain launch, collected in one walk over the dict (a lookup by name builds a string object each time, and
+// there are forty of them).
+struct ChainConfig {
+  enum Key { algo, out_mode, n_state, dt_p, dt_g, dt_u, dt_s, u_is_input, mars, cautious_wd, caution_apply, use_tensor_scale, accum_sumsq, u_op,
+             post_state, g_clip_mode, g_clip_at, g_clip_numel, lr, wd, eps, b1, b2, b3, alpha, mars_a, seed, g_delta, g_scale, p_delta, g_mc_delta,
+             p_mc_delta, count_caution, scale_stride, gsq_stride, kKeys };
+  py::handle values[kKeys];
+  explicit ChainConfig(const py::dict& cfg) {
+    static const std::unordered_map<std::string_view, int> index = {
+        {"algo", algo}, {"out_mode", out_mode}, {"n_state", n_state}, {"dt_p", dt_p}, {"dt_g", dt_g}, {"dt_u", dt_u}, {"dt_s", dt_s},
+        {"u_is_input", u_is_input}, {"mars", mars}, {"cautious_wd", cautious_wd}, {"caution_apply", caution_apply},
+        {"use_tensor_scale", use_tensor_scale}, {"accum_sumsq", accum_sumsq}, {"u_op", u_op}, {"post_state", post_state},
+        {"g_clip_mode", g_clip_mode}, {"g_clip_at", g_clip_at}, {"g_clip_numel", g_clip_numel}, {"lr", lr}, {"wd", wd}, {"eps", eps}, {"b1", b1},
+        {"b2", b2}, {"b3", b3}, {"alpha", alpha}, {"mars_a", mars_a}, {"seed", seed}, {"g_delta", g_delta}, {"g_scale", g_scale},
+        {"p_delta", p_delta}, {"g_mc_delta", g_mc_delta}, {"p_mc_delta", p_mc_delta}, {"count_caution", count_caution},
+        {"scale_stride", scale_stride}, {"gsq_stride", gsq_stride}};
+    for (const auto& item : cfg) {
+      Py_ssize_t len = 0;
+      const char* name = PyUnicode_AsUTF8AndSize(item.first.ptr(), &len);
+      if (name == nullptr) throw py::error_already_set();
+      const auto it = index.find(std::string_view(name, (size_t)len));
+      if (it != index.end()) values[it->second] = item.second;
+    }
+  }
+  bool has(Key k) const { return values[k].ptr() != nullptr; }
+  template <class T>
+  T get(Key k, T otherwise) const { return has(k) ? values[k].cast<T>() : otherwise; }
+  int i(Key k) const { return get<int>(k, 0); }
+  float f(Key k) const { return get<float>(k, 0.f); }
+};
+
 // Builds the per-tensor table and uploads it with one async copy on the current stream.
 Table upload(std::vector<hb::TensorMeta>& metas, const at::Device& dev, int chunk = hb::chain_chunk_elems()) {
   const int n = (int)metas.size();
-  std::vector<int> prefix(n + 1, 0);
-  for (int i = 0; i < n; ++i) prefix[i + 1] = prefix[i] + (int)((metas[i].numel + chunk - 1) / chunk);
+  const std::vector<int> prefix = chunk_prefix(metas, chunk);
   const size_t meta_bytes = sizeof(hb::TensorMeta) * n, prefix_bytes = sizeof(int) * (n + 1);
   std::vector<uint8_t> host(meta_bytes + prefix_bytes);
   memcpy(host.data(), metas.data(), meta_bytes);
@@ -74,21 +112,22 @@ Table upload(std::vector<hb::TensorMeta>& metas, const at::Device& dev, int chun
 // use_tensor_scale, count_caution (ints); lr, wd, eps, b1, b2, b3, alpha, mars_a (floats); seed.
 void fused_chain(const TList& p, const TList& pe, const TList& g, const TList& u, const TList& s0, const TList& s0e,
                  const TList& s1, const TList& s1e, const TList& s2, const TList& s2e, const TList& mars,
-                 const TList& marse, const OptT& scale, const OptT& masked, const OptT& gsq, const py::dict& cfg) {
+                 const TList& marse, const OptT& scale, const OptT& masked, const OptT& gsq, const py::dict& settings) {
   const size_t n = !g.empty() ? g.size() : (!u.empty() ? u.size() : p.size());
   if (n == 0) return;
   const at::Tensor& ref = !g.empty() ? *g[0] : (!u.empty() ? *u[0] : *p[0]);
   c10::cuda::CUDAGuard guard(ref.device());
-  const int scale_stride = cfg.contains("scale_stride") ? std::max(1, cfg["scale_stride"].cast<int>()) : 1;
-  const int gsq_stride = cfg.contains("gsq_stride") ? std::max(1, cfg["gsq_stride"].cast<int>()) : 1;
+  using Key = ChainConfig;
+  const ChainConfig cfg(settings);
+  const int scale_stride = std::max(1, cfg.i(Key::scale_stride));
+  const int gsq_stride = std::max(1, cfg.i(Key::gsq_stride));
   {  // the kernel trusts the table: every buffer must be a contiguous CUDA tensor of the element count and storage
      // kind its slot is declared with, on the device of the launch
     // storage kinds as in common.cuh: 0 fp32, 1 bf16, 2 fp16, 3 bf16+8, 4 bf16+16, 5 fp16+8, 6 fp16+16, 7 none
-    auto dt_of = [&](const char* k) { return cfg.contains(k) ? cfg[k].cast<int>() : 0; };
     auto primary_bytes = [](int dt) { return dt == 0 ? 4 : (dt == 7 ? 0 : 2); };
     auto residual_bytes = [](int dt) { return (dt == 3 || dt == 5) ? 1 : ((dt == 4 || dt == 6) ? 2 : 0); };
     struct Slot { const TList* list; const char* name; int dt; bool residual; };
-    const int dp = dt_of("dt_p"), dg = dt_of("dt_g"), du = dt_of("dt_u"), ds = dt_of("dt_s");
+    const int dp = cfg.i(Key::dt_p), dg = cfg.i(Key::dt_g), du = cfg.i(Key::dt_u), ds = cfg.i(Key::dt_s);
     const Slot slots[] = {{&p, "p", dp, false}, {&pe, "pe", dp, true}, {&g, "g", dg, false}, {&u, "u", du, false},
                           {&s0, "s0", ds, false}, {&s0e, "s0e", ds, true}, {&s1, "s1", ds, false}, {&s1e, "s1e", ds, true},
                           {&s2, "s2", ds, false}, {&s2e, "s2e", ds, true}, {&mars, "mars", ds, false}, {&marse, "marse", ds, true}};
@@ -115,11 +154,11 @@ void fused_chain(const TList& p, const TList& pe, const TList& g, const TList& u
       TORCH_CHECK(gsq->is_cuda() && gsq->is_contiguous() && gsq->scalar_type() == at::kFloat &&
                       (gsq->numel() == 1 || (size_t)gsq->numel() >= n * (size_t)gsq_stride),
                   "fused_chain: gsq needs one fp32 entry, or gsq_stride per tensor");
-    const int clip_mode = cfg.contains("g_clip_mode") ? cfg["g_clip_mode"].cast<int>() : 0;
+    const int clip_mode = cfg.i(Key::g_clip_mode);
     TORCH_CHECK(clip_mode != hb::kClipOrtho || (gsq.has_value() && gsq_stride == 3 && !p.empty()),
                 "fused_chain: the OrthoGrad projection needs the parameters and three dot products per tensor");
-    const int uop = cfg.contains("u_op") ? cfg["u_op"].cast<int>() : 0;
-    const int acc = cfg.contains("accum_sumsq") ? cfg["accum_sumsq"].cast<int>() : 0;
+    const int uop = cfg.i(Key::u_op);
+    const int acc = cfg.i(Key::accum_sumsq);
     TORCH_CHECK((uop != hb::kUopSignGraft && acc != 2) || (scale.has_value() && scale_stride == 2),
                 "fused_chain: sign grafting keeps two sums per tensor in `scale`");
   }
@@ -142,39 +181,45 @@ void fused_chain(const TList& p, const TList& pe, const TList& g, const TList& u
     m.pad = 0;
   }
   hb::ChainParams P{};
-  auto geti = [&](const char* k) { return cfg.contains(k) ? cfg[k].cast<int>() : 0; };
-  auto getf = [&](const char* k) { return cfg.contains(k) ? cfg[k].cast<float>() : 0.f; };
-  P.algo = geti("algo"); P.out_mode = geti("out_mode"); P.n_state = geti("n_state");
-  P.dt_p = geti("dt_p"); P.dt_g = geti("dt_g"); P.dt_u = geti("dt_u"); P.dt_s = geti("dt_s");
-  P.u_is_input = geti("u_is_input"); P.mars = geti("mars"); P.cautious_wd = geti("cautious_wd");
-  P.caution_apply = geti("caution_apply"); P.use_tensor_scale = geti("use_tensor_scale");
-  P.accum_sumsq = geti("accum_sumsq"); P.u_op = geti("u_op"); P.post_state = geti("post_state");
+  P.algo = cfg.i(Key::algo); P.out_mode = cfg.i(Key::out_mode); P.n_state = cfg.i(Key::n_state);
+  P.dt_p = cfg.i(Key::dt_p); P.dt_g = cfg.i(Key::dt_g); P.dt_u = cfg.i(Key::dt_u); P.dt_s = cfg.i(Key::dt_s);
+  P.u_is_input = cfg.i(Key::u_is_input); P.mars = cfg.i(Key::mars); P.cautious_wd = cfg.i(Key::cautious_wd);
+  P.caution_apply = cfg.i(Key::caution_apply); P.use_tensor_scale = cfg.i(Key::use_tensor_scale);
+  P.accum_sumsq = cfg.i(Key::accum_sumsq); P.u_op = cfg.i(Key::u_op); P.post_state = cfg.i(Key::post_state);
   TORCH_CHECK(P.post_state != hb::kPostMsam || (!s0.empty() && !s2.empty() && P.n_state == 3),
               "fused_chain: Momentum-SAM keeps its momentum in s0 and the unperturbed weights in s2");
   TORCH_CHECK(P.post_state != hb::kPostDecayIn || !p.empty(), "fused_chain: decay folded into the update reads the parameters");
-  P.g_clip_mode = geti("g_clip_mode"); P.g_clip_at = getf("g_clip_at"); P.g_clip_numel = getf("g_clip_numel");
-  P.lr = getf("lr"); P.wd = getf("wd"); P.eps = getf("eps");
-  P.b1 = getf("b1"); P.b2 = getf("b2"); P.b3 = getf("b3"); P.alpha = getf("alpha"); P.mars_a = getf("mars_a");
-  P.seed = cfg.contains("seed") ? cfg["seed"].cast<uint64_t>() : 0;
-  if (cfg.contains("g_delta")) {
-    auto d = cfg["g_delta"].cast<std::vector<int64_t>>();
+  P.g_clip_mode = cfg.i(Key::g_clip_mode); P.g_clip_at = cfg.f(Key::g_clip_at); P.g_clip_numel = cfg.f(Key::g_clip_numel);
+  P.lr = cfg.f(Key::lr); P.wd = cfg.f(Key::wd); P.eps = cfg.f(Key::eps);
+  P.b1 = cfg.f(Key::b1); P.b2 = cfg.f(Key::b2); P.b3 = cfg.f(Key::b3); P.alpha = cfg.f(Key::alpha); P.mars_a = cfg.f(Key::mars_a);
+  P.seed = cfg.get<uint64_t>(Key::seed, 0);
+  if (cfg.has(Key::g_delta)) {
+    auto d = cfg.get<std::vector<int64_t>>(Key::g_delta, {});
     TORCH_CHECK((int)d.size() <= hb::kMaxPeers, "too many gradient sources");
     P.n_src = (int)d.size();
     for (size_t i = 0; i < d.size(); ++i) P.g_delta[i] = d[i];
-    P.g_scale = getf("g_scale");
+    P.g_scale = cfg.f(Key::g_scale);
   }
-  if (cfg.contains("p_delta")) {
-    auto d = cfg["p_delta"].cast<std::vector<int64_t>>();
+  if (cfg.has(Key::p_delta)) {
+    auto d = cfg.get<std::vector<int64_t>>(Key::p_delta, {});
     TORCH_CHECK((int)d.size() <= hb::kMaxPeers, "too many parameter destinations");
     P.n_dst = (int)d.size();
     for (size_t i = 0; i < d.size(); ++i) P.p_delta[i] = d[i];
   }
-  P.g_mc_delta = cfg.contains("g_mc_delta") ? cfg["g_mc_delta"].cast<int64_t>() : 0;
-  P.p_mc_delta = cfg.contains("p_mc_delta") ? cfg["p_mc_delta"].cast<int64_t>() : 0;
-  const bool count = geti("count_caution") != 0;
+  P.g_mc_delta = cfg.get<int64_t>(Key::g_mc_delta, 0);
+  P.p_mc_delta = cfg.get<int64_t>(Key::p_mc_delta, 0);
+  const bool count = cfg.i(Key::count_caution) != 0;
   int64_t elems = 0;
   for (const hb::TensorMeta& m : metas) elems += m.numel;
-  Table t = upload(metas, ref.device(), hb::chain_chunk_elems_for(P, count, elems));
+  const int chunk = hb::chain_chunk_elems_for(P, count, elems);
+  if (hb::chain_takes_inline(P, count, (int)n, elems)) {
+    const std::vector<int> prefix = chunk_prefix(metas, chunk);
+    P.n_tensors = (int)n;
+    P.chunk = chunk;
+    check(hb::launch_fused_chain_inline(metas.data(), prefix.data(), prefix[n], P, count, at::cuda::getCurrentCUDAStream()), "fused_chain launch");
+    return;
+  }
+  Table t = upload(metas, ref.device(), chunk);
   P.n_tensors = t.n;
   P.chunk = t.chunk;
   check(hb::launch_fused_chain(t.metas, t.prefix, t.total_chunks, P, count, at::cuda::getCurrentCUDAStream()),

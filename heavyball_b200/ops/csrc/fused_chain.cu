@@ -7,14 +7,17 @@
 // restated from heavyball_b200/utils/first_order.py, which is also the test oracle.
 //
 // Work decomposition: tensors are cut into chunks (chain_chunks.h); block b owns chunk b, and its warps find the tensor in a
-// table of prefix sums, 32 entries at a time (find_range).  All tensor addresses come from a device-resident table, so the
-// launch count is independent of the number of tensors.
+// table of prefix sums, 32 entries at a time (find_range).  All tensor addresses come from a table (in device memory, or in the
+// launch's arguments where tensors and elements are few), so the launch count is independent of the number of tensors.
 //
 // Two kernels: the general one below takes every storage kind, rule and destination from run-time parameters; the specialised
 // instances after it (Kinds) cover the launches that most steps consist of.
 #include "chain_chunks.h"
 #include "common.cuh"
 #include "fused_chain.h"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace hb {
 
@@ -408,15 +411,19 @@ struct ChainKind {
   }
 };
 
-template <class K>
-__global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(const TensorMeta* __restrict__ metas,
-                                                                              const int* __restrict__ chunk_prefix,
-                                                                              ChainParams P) {
+template <class K, class Table>
+__global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(const __grid_constant__ Table T, ChainParams P) {
   // a launch that applies a parked update walks backwards: what the launch before it wrote last is still in the L2
   const int b = (K::u_in && K::reads_p) ? (int)(gridDim.x - 1 - blockIdx.x) : (int)blockIdx.x;
-  const int t = find_range(chunk_prefix, P.n_tensors, b);
-  const TensorMeta& M = metas[t];
-  const int64_t numel = M.numel, base = (int64_t)(b - chunk_prefix[t]) * P.chunk, end = min(numel, base + P.chunk);
+  int t = 0;
+  if constexpr (std::is_same<Table, DeviceTable>::value) {
+    t = find_range(T.prefix, P.n_tensors, b);
+  } else {
+    for (int i = 1; i < P.n_tensors; ++i)
+      if (T.prefix[i] <= b) t = i;
+  }
+  const TensorMeta& M = T.metas[t];
+  const int64_t numel = M.numel, base = (int64_t)(b - T.prefix[t]) * P.chunk, end = min(numel, base + P.chunk);
   const bool vec_ok = M.vec_ok != 0;
   const Philox rng(P.seed);
   void *const mp = M.p, *const mpe = M.pe, *const mg = M.g, *const mu = M.u;
@@ -615,10 +622,12 @@ using Kinds = KindList<
     ChainKind<kBF16, kNone, kF32, kNone, kOutParam, 1, false>,
     ChainKind<kBF16E8, kNone, kF32, kNone, kOutParam, 1, false>>;
 
-using PlainLaunch = void (*)(const TensorMeta*, const int*, ChainParams);
+using PlainLaunch = void (*)(DeviceTable, ChainParams);
+using InlineLaunch = void (*)(InlineTable, ChainParams);
 
 struct PlainKind {
   PlainLaunch kernel = nullptr;
+  InlineLaunch kernel_inline = nullptr;
   int vectors = 0;  // in flight per thread
 };
 
@@ -629,7 +638,7 @@ PlainKind find_kind(KindList<Ks...>, const ChainParams& P, bool count) {
                      (P.u_op == kUopNone || (P.u_op == kUopTrustRegion && P.u_is_input)) && P.post_state == kPostNone && P.out_mode != kOutScheduleFree &&
                      (!P.u_is_input || (P.algo == kIdentity && P.n_state == 0 && !P.mars)) && !(count && P.accum_sumsq);
   PlainKind hit;
-  if (plain) ((hit.kernel == nullptr && Ks::takes(P, count) ? (void)(hit = {plain_chain_kernel<Ks>, Ks::batch}) : (void)0), ...);
+  if (plain) ((hit.kernel == nullptr && Ks::takes(P, count) ? (void)(hit = {plain_chain_kernel<Ks, DeviceTable>, plain_chain_kernel<Ks, InlineTable>, Ks::batch}) : (void)0), ...);
   return hit;
 }
 
@@ -648,13 +657,29 @@ cudaError_t launch_fused_chain(const TensorMeta* metas, const int* chunk_prefix,
   ChainParams P = P0;
   if (P.chunk == 0) P.chunk = kChunk;
   if (const PlainLaunch kernel = find_kind(Kinds{}, P, count_caution).kernel)
-    kernel<<<total_chunks, kThreads, 0, stream>>>(metas, chunk_prefix, P);
+    kernel<<<total_chunks, kThreads, 0, stream>>>(DeviceTable{metas, chunk_prefix}, P);
   else if (P.chunk != kChunk)
     return cudaErrorInvalidValue;  // the general kernel is compiled for one chunk size
   else if (count_caution)
     fused_chain_kernel<true><<<total_chunks, kThreads, 0, stream>>>(metas, chunk_prefix, P);
   else
     fused_chain_kernel<false><<<total_chunks, kThreads, 0, stream>>>(metas, chunk_prefix, P);
+  return cudaGetLastError();
+}
+
+bool chain_takes_inline(const ChainParams& P, bool count_caution, int n_tensors, int64_t total_elems) {
+  return n_tensors <= kInlineTensors && total_elems <= (1 << 23) && find_kind(Kinds{}, P, count_caution).kernel != nullptr;
+}
+
+cudaError_t launch_fused_chain_inline(const TensorMeta* host_metas, const int* host_prefix, int total_chunks, const ChainParams& P,
+                                      bool count_caution, cudaStream_t stream) {
+  if (total_chunks <= 0) return cudaSuccess;
+  const InlineLaunch kernel = find_kind(Kinds{}, P, count_caution).kernel_inline;
+  if (kernel == nullptr || P.n_tensors > kInlineTensors || P.chunk == 0) return cudaErrorInvalidValue;
+  InlineTable T;
+  std::copy(host_prefix, host_prefix + P.n_tensors + 1, T.prefix);
+  std::copy(host_metas, host_metas + P.n_tensors, T.metas);
+  kernel<<<total_chunks, kThreads, 0, stream>>>(T, P);
   return cudaGetLastError();
 }
 

@@ -93,11 +93,31 @@ struct ChainParams {
   int64_t p_mc_delta;
 };
 
+// The table of a launch: in device memory, or inside the kernel's own arguments, which saves an upload (an allocation and a copy, 8 us
+// of the host's time).
+struct DeviceTable {
+  const TensorMeta* metas;
+  const int* prefix;
+};
+constexpr int kInlineTensors = 24;  // what fits 4 KB of arguments
+struct InlineTable {
+  int prefix[kInlineTensors + 1];
+  TensorMeta metas[kInlineTensors];
+};
+static_assert(sizeof(InlineTable) + sizeof(ChainParams) <= 4096, "kernel arguments");
+// Whether a launch takes its table in the arguments: few tensors, and few elements - up to 8 M the host's time is the longer one, beyond
+// it the kernel's is, which reads the table from global memory a little faster (cautious AdamW on 8 x 2048^2: 351 us, 356 with the
+// table in the arguments).
+bool chain_takes_inline(const ChainParams& P, bool count_caution, int n_tensors, int64_t total_elems);
+
 int chain_chunk_elems();
 // elements per block that a fused-chain launch over `total_elems` elements wants its prefix table built with
 int chain_chunk_elems_for(const ChainParams& P, bool count_caution, int64_t total_elems);
 cudaError_t launch_fused_chain(const TensorMeta* metas, const int* chunk_prefix, int total_chunks, const ChainParams& P,
                                bool count_caution, cudaStream_t stream);
+// ... with a table in host memory (see chain_takes_inline)
+cudaError_t launch_fused_chain_inline(const TensorMeta* host_metas, const int* host_prefix, int total_chunks, const ChainParams& P,
+                                      bool count_caution, cudaStream_t stream);
 cudaError_t launch_sumsq(const TensorMeta* metas, const int* chunk_prefix, int total_chunks, int n_tensors, int dt,
                          float* out, cudaStream_t stream);
 

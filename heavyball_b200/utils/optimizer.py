@@ -451,7 +451,9 @@ class StatefulOptimizer(torch.optim.Optimizer):
                     continue
                 self.views.register_plain(p)
                 if grad is not None:
-                    grad = (promote(grad) if should_promote else grad).detach()
+                    grad = promote(grad) if should_promote else grad
+                    if grad.requires_grad:
+                        grad = grad.detach()
                 yield p, grad
                 continue
             stored = Scratch.take(group, p, "grad", "vector", "hessian_vector")
@@ -555,7 +557,8 @@ class StatefulOptimizer(torch.optim.Optimizer):
         try:
             with torch.no_grad():
                 for group in self.param_groups:
-                    group.setdefault("param_count", sum(p.numel() for p in group["params"]))
+                    if "param_count" not in group:
+                        group["param_count"] = sum(p.numel() for p in group["params"])
                     group["is_preconditioning"] = self._is_preconditioning
                     self._step(group)
         finally:

@@ -14,6 +14,29 @@ DEV = "cuda"
 # ---------------------------------------------------------------------------------------- fused chain
 
 
+@pytest.mark.parametrize("extra", [(1,), (8_500_000,)], ids=["25 tensors", "more than 8 M elements"])
+@pytest.mark.parametrize("ecc", [None, "bf16+8"])
+def test_table_in_the_arguments_and_in_memory(ecc, extra):
+    """24 small tensors take their table in the launch's arguments; with one more tensor or with too many elements it is in memory:
+    the results of the 24 are the same bits either way (rounding noise is addressed by tensor and element)."""
+    sizes = [1, 2048, 2049, *range(3, 24)]
+
+    def run(sizes):
+        draw = lambda salt: [torch.randn(n, device=DEV, generator=torch.Generator(DEV).manual_seed(100 * salt + i)) for i, n in enumerate(sizes)]  # noqa: E731
+        p, g, dtype = draw(1), draw(2), torch.bfloat16 if ecc else torch.float32
+        m, v = [t.to(dtype) for t in draw(3)], [t.square().to(dtype) for t in draw(4)]
+        residuals = lambda: [torch.zeros(n, dtype=torch.int8, device=DEV) for n in sizes] if ecc else []  # noqa: E731
+        me, ve = residuals(), residuals()
+        for seed in (5, 6):
+            ops.fused_chain(p=p, g=g, s0=m, s0e=me, s1=v, s1e=ve, algo=ops.ADAM, n_state=2, out_mode=ops.OUT_PARAM, dt_p=ops.F32, dt_g=ops.F32,
+                            dt_s=ops.BF16E8 if ecc else ops.F32, lr=1e-2, wd=0.1, eps=1e-8, b1=0.9, b2=0.99, seed=seed)  # fmt: skip
+        return [t for lst in zip(*[x for x in (p, m, v, me, ve) if x]) for t in lst]
+
+    assert len(sizes) == 24
+    for few, more in zip(run(sizes), run([*sizes, *extra])):
+        assert torch.equal(few, more)
+
+
 @pytest.mark.parametrize("kw", [{}, {"ecc": "bf16+8", "mars": True, "caution": True}, {"ecc": "bf16+8"}, {"caution": True}], ids=str)
 @pytest.mark.parametrize("sizes", [(1,), (2047, 2048, 2049), (8191, 8193, 3, 16384), tuple(range(1, 41)), (10_000_000, 5),
                                    (4095, 4096, 4097, 2_500_001, 7), (8191, 8192, 8193, 1, 10_000_000, 5)], ids=len)  # fmt: skip
