@@ -633,6 +633,32 @@ at::Tensor tri_inv_blocks(const at::Tensor& q) {
   return x;
 }
 
+// Columns of the contiguous fp32 [batch, n, k] tensor x in the order of the permutations `order` (contiguous int64 [batch, k]), or put
+// back from it (inverse).
+at::Tensor permute_columns(const at::Tensor& x, const at::Tensor& order, bool inverse) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 3 && x.is_contiguous() && x.size(2) <= hb::kMaxPermuted && x.size(0) <= 65535,
+              "permute_columns: contiguous fp32 [batch, n, k] CUDA tensor, k <= 12288");
+  TORCH_CHECK(order.device() == x.device() && order.scalar_type() == at::kLong && order.is_contiguous() && order.dim() == 2 &&
+                  order.size(0) == x.size(0) && order.size(1) == x.size(2), "permute_columns: contiguous int64 [batch, k] order");
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor out = at::empty_like(x);
+  check(hb::launch_permute_columns(x.data_ptr<float>(), reinterpret_cast<const long long*>(order.data_ptr<int64_t>()), out.data_ptr<float>(),
+                                   (int)x.size(0), (int)x.size(1), (int)x.size(2), inverse ? 1 : 0, at::cuda::getCurrentCUDAStream()),
+        "permute_columns launch");
+  return out;
+}
+
+// bad[b] |= 1 where the fp32 [batch, k, k] matrix g[b] (unit inner stride) is further than `limit` from the identity, or not finite.
+void identity_defect(const at::Tensor& g, double limit, at::Tensor& bad) {
+  TORCH_CHECK(g.is_cuda() && g.scalar_type() == at::kFloat && g.dim() == 3 && g.size(1) == g.size(2) && g.stride(2) == 1 && g.size(0) <= 65535,
+              "identity_defect: fp32 [batch, k, k] CUDA tensor with unit inner stride");
+  TORCH_CHECK(bad.device() == g.device() && bad.scalar_type() == at::kInt && bad.is_contiguous() && bad.numel() == g.size(0),
+              "identity_defect: one int32 flag per matrix");
+  c10::cuda::CUDAGuard guard(g.device());
+  check(hb::launch_identity_defect(g.data_ptr<float>(), g.stride(1), g.stride(0), (int)g.size(0), (int)g.size(1), (float)limit, bad.data_ptr<int>(),
+                                   at::cuda::getCurrentCUDAStream()), "identity_defect launch");
+}
+
 // Factors the diagonal leaf [lo, lo + size) of the batched symmetric positive definite fp32 matrices g ([batch, n, n], unit
 // inner stride) as R^T R: writes R's block into r (same layout as g) and the block's inverse into inv[:, lo / 128]
 // (inv: contiguous [batch, ceil(n / 128), 128, 128]); info: int32 [batch], incremented per matrix with a bad pivot.
@@ -808,6 +834,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gelu_bwd", &gelu_bwd);
   m.def("tall_t_mul", &tall_t_mul);
   m.def("tri_inv_blocks", &tri_inv_blocks);
+  m.def("permute_columns", &permute_columns);
+  m.def("identity_defect", &identity_defect);
   m.def("layer_norm_fwd", &layer_norm_fwd);
   m.def("layer_norm_bwd", &layer_norm_bwd);
   m.def("layer_norm_supported", &hb::layer_norm_supported);

@@ -422,4 +422,55 @@ cudaError_t launch_triu_unpack(const void* line, void* dense, int elem_bytes, in
   return cudaGetLastError();
 }
 
+// ------------------------------------------------------------------------------------------ around the eigenbasis refresh
+// Passes over n x k matrices that only memory bounds: a block turns a few rows in shared memory, so that both sides are read and written
+// in whole lines.
+__global__ void __launch_bounds__(256) permute_columns_kernel(const float* __restrict__ x, const long long* __restrict__ order, float* __restrict__ out,
+                                                             int n, int k, int rows, int inverse) {
+  extern __shared__ float turned[];  // rows x k
+  const int r0 = blockIdx.x * rows, count = min(rows, n - r0);
+  const long long base = ((long long)blockIdx.y * n + r0) * k;
+  const long long* o = order + (long long)blockIdx.y * k;
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    const long long to = inverse ? o[j] : j;
+    if (to < 0 || to >= k) continue;
+#pragma unroll 8
+    for (int r = 0; r < count; ++r) turned[r * k + to] = x[base + (long long)r * k + j];
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < k; j += blockDim.x) {
+    const long long from = inverse ? j : o[j];
+    if (from < 0 || from >= k) continue;
+#pragma unroll 8
+    for (int r = 0; r < count; ++r) out[base + (long long)r * k + j] = turned[r * k + from];
+  }
+}
+
+cudaError_t launch_permute_columns(const float* x, const long long* order, float* out, int batch, int n, int k, int inverse, cudaStream_t stream) {
+  if (batch == 0 || n == 0 || k == 0) return cudaSuccess;
+  if (k > kMaxPermuted || batch > 65535) return cudaErrorInvalidValue;
+  const int rows = kMaxPermuted / k < 8 ? kMaxPermuted / k : 8;  // 48 KB of shared memory at most
+  permute_columns_kernel<<<dim3((n + rows - 1) / rows, batch), 256, (size_t)rows * k * sizeof(float), stream>>>(x, order, out, n, k, rows, inverse);
+  return cudaGetLastError();
+}
+
+__global__ void __launch_bounds__(256) identity_defect_kernel(const float* __restrict__ G, long long ld, long long strideG, int k, float limit,
+                                                             int* __restrict__ bad) {
+  const int r = blockIdx.x * 8 + (threadIdx.x >> 5);
+  bool off = false;
+  if (r < k) {
+    const float* row = G + blockIdx.y * strideG + r * ld;
+#pragma unroll 8
+    for (int c = threadIdx.x & 31; c < k; c += 32) off |= !(fabsf(row[c] - (c == r ? 1.0f : 0.0f)) <= limit);
+  }
+  if (__syncthreads_or(off) && threadIdx.x == 0) atomicOr(bad + blockIdx.y, 1);
+}
+
+cudaError_t launch_identity_defect(const float* G, long long ld, long long strideG, int batch, int k, float limit, int* bad, cudaStream_t stream) {
+  if (batch == 0 || k == 0) return cudaSuccess;
+  if (batch > 65535) return cudaErrorInvalidValue;
+  identity_defect_kernel<<<dim3((k + 7) / 8, batch), 256, 0, stream>>>(G, ld, strideG, k, limit, bad);
+  return cudaGetLastError();
+}
+
 }  // namespace hb

@@ -30,4 +30,12 @@ cudaError_t launch_chol_inv_leaf(const float* G, long long ldg, long long stride
 cudaError_t launch_triu_pack(const void* dense, void* line, int elem_bytes, int batch, int n, cudaStream_t stream);
 cudaError_t launch_triu_unpack(const void* line, void* dense, int elem_bytes, int batch, int n, cudaStream_t stream);
 
+// out[b][i][j] = x[b][i][order[b][j]] or, `inverse`, out[b][i][order[b][j]] = x[b][i][j]; x, out: [batch, n, k] fp32, order: [batch, k]
+// permutations (entries outside [0, k) are skipped), k <= kMaxPermuted.
+constexpr int kMaxPermuted = 12288;
+cudaError_t launch_permute_columns(const float* x, const long long* order, float* out, int batch, int n, int k, int inverse, cudaStream_t stream);
+
+// bad[b] |= not (largest |G[b] - I| <= limit), so a NaN counts; G: [batch, k, k] fp32, row stride ld, batch stride strideG.
+cudaError_t launch_identity_defect(const float* G, long long ld, long long strideG, int batch, int k, float limit, int* bad, cudaStream_t stream);
+
 }  // namespace hb

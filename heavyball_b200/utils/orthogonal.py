@@ -269,7 +269,6 @@ def _cholesky_qr2(x: Tensor, shifted_rounds: int = 0):
     tiny = torch.finfo(a.dtype).tiny
     a = a / a.norm(dim=-2, keepdim=True).clamp_(min=tiny)
     bad = torch.zeros(a.shape[0], dtype=torch.int32, device=a.device)
-    eye = torch.eye(k, device=a.device, dtype=a.dtype)
     rounds = shifted_rounds + 2
     info = torch.zeros_like(bad)  # failed leaves do not decide: what counts is the orthogonality reached at the end
     for rnd in range(rounds):
@@ -283,8 +282,13 @@ def _cholesky_qr2(x: Tensor, shifted_rounds: int = 0):
         a = _solve_right_upper(r, a, inv, 0, consume_b=rnd > 0 or a.data_ptr() != x.data_ptr(), pairs=False)
         if rnd < shifted_rounds:  # columns shrank by different amounts: back to unit columns for the next round
             a = a / a.norm(dim=-2, keepdim=True).clamp_(min=tiny)
-    bad += (_mm(a, a, True, False, pairs=False) - eye).abs().amax(dim=(-2, -1)).gt(_CHOLQR_ACCEPT)
-    bad += (~torch.isfinite(a)).flatten(1).any(dim=1)
+    gram = _mm(a, a, True, False, pairs=False)
+    ext = _skinny_kernels(gram)
+    if ext is not None:  # one pass; an entry of ``a`` that is not finite leaves one in the Gram matrix
+        ext.identity_defect(gram, _CHOLQR_ACCEPT, bad)
+    else:
+        bad += (gram - torch.eye(k, device=a.device, dtype=a.dtype)).abs().amax(dim=(-2, -1)).gt(_CHOLQR_ACCEPT)
+        bad += (~torch.isfinite(a)).flatten(1).any(dim=1)
     return a.reshape(*batch, n, k), bad
 
 
@@ -392,17 +396,23 @@ def _ladder_won(key, level: int):
     _cholqr_level[key] = max(0, level - 1) if wins % 8 == 0 else level
 
 
-def _panel_basis(x: Tensor, fallback: Tensor = None):
+def _kept(fallback):
+    """``fallback`` is a tensor, ``None``, or what makes the tensor: most refreshes never need it."""
+    return fallback() if callable(fallback) else fallback
+
+
+def _panel_basis(x: Tensor, fallback=None):
     """The panel-wise route (``None``: not for this input, or a matrix failed and there was nothing to keep)."""
     if not (x.is_cuda and _settings().fast_qr and x.shape[-2] >= x.shape[-1] >= 2 * _QR_PANEL):
         return None
-    return _panel_qr_replayed(x.contiguous(), fallback) if _settings().graph_qr else _panel_cholesky_qr(x)
+    return _panel_qr_replayed(x.contiguous(), _kept(fallback)) if _settings().graph_qr else _panel_cholesky_qr(x)
 
 
-def _qr_basis(x: Tensor, fallback: Tensor = None, lowest: int = 0) -> Tensor:
+def _qr_basis(x: Tensor, fallback=None, lowest: int = 0, own: bool = True) -> Tensor:
     """Q factor of ``x``.  ``fallback``: orthonormal matrix to keep where the fast factorisation fails (see
-    :func:`_panel_qr_replayed`); without it a failure costs a host synchronisation and Householder QR.  ``lowest``: first
-    step of the ladder that is worth trying."""
+    :func:`_panel_qr_replayed`, :func:`_kept`); without it a failure costs a host synchronisation and Householder QR.
+    ``lowest``: first step of the ladder that is worth trying.  ``own=False``: the caller reads the result before anything else
+    is factored, so it may be the buffer of a captured factorisation."""
     x32 = promote(x)
     if _cholqr_applies(x32):
         xc = x32.contiguous()
@@ -411,20 +421,20 @@ def _qr_basis(x: Tensor, fallback: Tensor = None, lowest: int = 0) -> Tensor:
             q, bad = _cholesky_qr2_replayed(xc, _CHOLQR_LADDER[level])
             if int(bad.sum()) == 0:  # one host read per attempt; a failure climbs the ladder, then takes the panel-wise route
                 _ladder_won(key, level)
-                return q.clone() if q.data_ptr() != x32.data_ptr() else q
+                return q.clone() if own and q.data_ptr() != x32.data_ptr() else q
         _cholqr_level[key] = len(_CHOLQR_LADDER) - 1
         qr_stats["cholesky_qr2_rejected"] += 1
     q = _panel_basis(x32, fallback)
     return q if q is not None else torch.linalg.qr(x32).Q
 
 
-def _qr_bases(x: Tensor, fallback: Tensor, sizes: Sequence[int]) -> Tensor:
-    """:func:`_qr_basis` of independent batches that follow one another in ``x`` (``sizes`` matrices each), as one chain of
+def _qr_bases(x: Tensor, fallback, sizes: Sequence[int]) -> Tensor:
+    """:func:`_qr_basis` (``own=False``) of independent batches that follow one another in ``x`` (``sizes`` matrices each), as one chain of
     launches where that changes nothing for any of them.  Every batch is accepted or refused by itself and keeps its own
     place on the ladder: a refused one climbs alone, and while the batches stand on different steps each takes its own
     route, so a factor that is hard to refresh costs the others neither their variant nor their result."""
     x32 = promote(x).contiguous()
-    alone = lambda: torch.cat([_qr_basis(m, f) for m, f in zip(x32.split(sizes), fallback.split(sizes))])  # noqa: E731
+    alone = lambda: torch.cat([_qr_basis(m, f) for m, f in zip(x32.split(sizes), _kept(fallback).split(sizes))])  # noqa: E731
     if not _cholqr_applies(x32):
         q = _panel_basis(x32, fallback)  # a failure in the joint run must not send the others to another factorisation
         return q if q is not None else alone()
@@ -435,10 +445,12 @@ def _qr_bases(x: Tensor, fallback: Tensor, sizes: Sequence[int]) -> Tensor:
     (level,) = levels
     q, bad = _cholesky_qr2_replayed(x32, _CHOLQR_LADDER[level])
     refused = [bool(flags.any()) for flags in bad.cpu().split(sizes)]
-    q = q.clone() if q.data_ptr() != x32.data_ptr() else q
     for key, no in zip(keys, refused):
         if not no:
             _ladder_won(key, level)
+    if not any(refused):
+        return q
+    q, fallback = q.clone(), _kept(fallback)
     for out, m, f, no in zip(q.split(sizes), x32.split(sizes), fallback.split(sizes), refused):
         if no:
             out.copy_(_qr_basis(m, f, level + 1))

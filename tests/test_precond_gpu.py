@@ -196,3 +196,34 @@ def test_skinny_gram_of_very_tall_matrices(n, r):
     want = a.double().T @ b.double()
     assert got.shape == (r, r)
     assert float((got.double() - want).abs().max()) < 1e-5 * float((a.double().abs().T @ b.double().abs()).max())
+
+
+@pytest.mark.parametrize("B,n,k", [(2, 1, 1), (3, 9, 257), (2, 260, 1024), (1, 5, 12288), (1, 3, 12289)])
+def test_columns_in_order_and_back(B, n, k):
+    """Moved as bits, NaN and infinities too; one column past what the kernel takes goes the general way."""
+    from heavyball_b200.utils.soap import _permute_columns
+
+    g = torch.Generator(device="cuda").manual_seed(k)
+    x = torch.randn(B, n, k, device="cuda", generator=g)
+    x[0, 0, 0], x[0, -1, -1] = float("nan"), float("-inf")
+    order = torch.stack([torch.randperm(k, device="cuda", generator=g) for _ in range(B)])
+    moved = _permute_columns(x, order)
+    assert torch.equal(moved.view(torch.int32), x.view(torch.int32).gather(-1, order.unsqueeze(-2).expand_as(x)))
+    assert torch.equal(_permute_columns(moved, order, inverse=True).view(torch.int32), x.view(torch.int32))
+
+
+@pytest.mark.parametrize("k", [1, 33, 256, 1000])
+def test_identity_defect_flags_what_the_definition_flags(k):
+    from heavyball_b200 import ops
+
+    base = torch.eye(k, device="cuda").expand(6, k, k)
+    padded = torch.full((6, k, k + 3), 9.0, device="cuda")
+    gram = padded[..., :k].copy_(base)
+    gram[1, -1, -1] += 2e-4
+    gram[2, k // 2, 0] += -2e-4
+    gram[3, 0, -1] = float("nan")
+    gram[4, -1, 0] = float("inf")
+    gram[5] += 0.5e-4
+    bad = torch.zeros(6, dtype=torch.int32, device="cuda")
+    ops.load().identity_defect(gram, 1e-4, bad)
+    assert bad.tolist() == [0, 1, 1, 1, 1, 0]
