@@ -1,4 +1,4 @@
-// Epilogue and 128 x 128 kernel shared by the split-operand GEMMs (tf32_gemm.cu, split16_gemm.cu).
+// Epilogue and kernels (128 x 128 tiles, and 256 x 256 on CTA pairs) shared by the split-operand GEMMs (tf32_gemm.cu, split16_gemm.cu).
 //
 // 128 x 128 tiles, one per CTA, 192 threads, two CTAs per SM (a ring of six stages and one CTA per SM is no faster, not even for launches
 // of a few tiles: a tile by itself takes 0.43 us per 128 bytes of K because its products and its loads share the shared memory):
@@ -7,6 +7,7 @@
 //   warps 2..5 : tcgen05.ld, then the epilogue.  Plain stores go through the (now idle) ring and four bulk tensor stores, the
 //                others through epilogue_direct.
 #pragma once
+#include "pair_drain.h"
 #include "tc_common.cuh"
 #include "tf32_gemm.h"
 
@@ -342,7 +343,8 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
 
 // `Kind`: operand type.  kBlock elements of K fill a 128-byte row; kDesc is the instruction descriptor for a 128 x 128 tile; the product
 // is three walks over K, of which walk kTermLoA takes the low parts of A and walk kTermLoB those of B; kCrossFirst: these two come
-// first, and the sum they leave is scaled by 2^-11 when the walk over the high parts begins.
+// first, and the sum they leave is scaled by 2^-11 when the walk over the high parts begins.  kPairDesc, mma_pair: the same for the pair
+// kernel.
 template <class Kind>
 __global__ void __launch_bounds__(kTThreads, 2)
 gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
@@ -478,6 +480,171 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
   }
   if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTTmemCols); }
+}
+
+// ------------------------------------------------------------------------------------------ pair kernel
+// 256 x 256 tiles on CTA pairs (cta_group::2), one persistent pair per two SMs; structure as in ns_gemm.cu: each CTA stages 128 rows of
+// A and half of B (32 KiB per 128 bytes of K, 5 stages), two accumulators, eight epilogue warps of 32 rows x 128 columns under the next
+// tile's main loop.
+// In the place of the one-CTA 256 x 256 tile that split tf32 used (64 KiB stages, one accumulator over all of tensor memory, its epilogue
+// exposed), same bits: 16 of 1024^3 166 -> 147 us, symmetric 169 -> 114, 2 of 5504 x 2048 x 2048 405 -> 342, 11 of 2048^3 718 -> 690.
+constexpr int kGPairStages = 5;
+constexpr int kGPairStageBytes = 2 * kTTileBytes;
+constexpr int kGPairEpiWarps = 8;
+constexpr int kGPairThreads = 64 + 32 * kGPairEpiWarps;
+constexpr int kGPairSmemBytes = kGPairStages * kGPairStageBytes + kGPairEpiWarps * kStageWarpBytes + 1024;
+
+struct WalkTile {
+  int kb_lo, seg;  // K blocks of one term that the tile walks: [kb_lo, kb_lo + seg)
+};
+__device__ __forceinline__ WalkTile walk_tile(const PairTile& t, int kp, int tri, int block) {
+  int lo = 0, hi = kp / block;
+  if (tri) {
+    lo = min(hi, t.tm * (kPairTile / block));
+    hi = t.tn < t.tm ? lo : min(hi, (t.tn + 1) * (kPairTile / block));
+  }
+  return {lo, hi - lo};
+}
+
+template <class Kind>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGPairThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N, int kp, int tiles_m,
+                    int tiles_n, int per_batch, int total, const Tf32Epilogue E, const float* row_units, int64_t stride_ru,
+                    const float* col_units, int64_t stride_cu, int* status) {
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t full_bar[kGPairStages];   // used in the even CTA: both CTAs' loads of a stage have landed
+  __shared__ __align__(8) uint64_t empty_bar[kGPairStages];  // in each CTA: the products that read the stage have finished
+  __shared__ __align__(8) uint64_t acc_full[2];              // in each CTA: accumulator finished
+  __shared__ __align__(8) uint64_t acc_empty[2];             // in the even CTA: all sixteen epilogue warps have read it
+  __shared__ __align__(8) uint64_t drain_bar;                // in each CTA, teardown only: all products have finished
+  __shared__ uint32_t tmem_base_slot;
+  __shared__ int abort_flag, skip_flag;
+  __shared__ int fills;                                      // ring fills this CTA issued
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const bool leader = elect_one();  // issues the loads (warp 0) and the products (warp 1), and waits for them in the teardown
+  const uint32_t rank = cluster_rank();
+  uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kGPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
+    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * kGPairEpiWarps); }
+    mbar_init(&drain_bar, 1);
+    abort_flag = 0;
+    fills = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) { tmem_alloc_pair(&tmem_base_slot, 512); tmem_relinquish_pair(); }
+  griddep_wait();
+  // a kernel of this stream already gave up on a wait: do not pile more work on a broken pipeline (the even CTA decides)
+  if (threadIdx.x == 0) skip_flag = status != nullptr && *(volatile const int*)status != 0;
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();
+  tc_fence_after();
+  const uint32_t tmem_base = tmem_base_slot;
+  const bool skip = cluster_load(cluster_addr(&skip_flag, 0)) != 0;
+
+  if (skip) {
+  } else if (warp == 0) {
+    if (leader) {
+      int n = 0;  // ring fills so far
+      bool ok = true;
+      for (int idx = pair; idx < total && ok; idx += pairs) {
+        const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
+        const WalkTile h = walk_tile(t, kp, E.tri, Kind::kBlock);
+        const int a_row = t.tm * kPairTile + (int)rank * 128, b_row = t.tn * kPairTile + (int)rank * 128;
+        for (int term = 0; term < 3 && ok; ++term) {
+          const int ka = (term == Kind::kTermLoA ? kp : 0), kb_off = (term == Kind::kTermLoB ? kp : 0);
+          for (int kb = 0; kb < h.seg; ++kb, ++n) {
+            const int s = n % kGPairStages, round = n / kGPairStages, k0 = (h.kb_lo + kb) * Kind::kBlock;
+            ok = mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag);
+            if (!ok) break;
+            uint8_t* dst = ring + s * kGPairStageBytes;
+            const uint32_t bar = cluster_addr(&full_bar[s], 0);
+            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kGPairStageBytes);
+            tma_load_3d_pair(dst, &map_a, bar, ka + k0, a_row, t.batch);  // rows past the operand's end arrive as zeros and count
+            tma_load_3d_pair(dst + kTTileBytes, &map_b, bar, kb_off + k0, b_row, t.batch);
+          }
+        }
+      }
+      fills = n;
+      griddep_launch();  // this CTA's last loads are on their way: the next kernel may take over SMs that drain
+    }
+  } else if (warp == 1) {
+    if (leader && rank == 0) {
+      int n = 0, it = 0;
+      bool ok = true;
+      for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
+        const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
+        const int seg = walk_tile(t, kp, E.tri, Kind::kBlock).seg, num_kb = 3 * seg, acc = it & 1;
+        ok = mbar_wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1, &abort_flag);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d = tmem_base + (uint32_t)acc * 256u;
+        for (int kb = 0; kb < num_kb; ++kb, ++n) {
+          const int s = n % kGPairStages, round = n / kGPairStages;
+          ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t base = smem_u32(ring + s * kGPairStageBytes);
+          const uint64_t a_desc = make_smem_desc(base), b_desc = make_smem_desc(base + kTTileBytes);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            if (Kind::kCrossFirst && k == 0 && kb == 2 * seg)
+              tc_mma_f16_d11_pair(d, a_desc, b_desc, Kind::kPairDesc);
+            else
+              Kind::mma_pair(d, a_desc + 2 * k, b_desc + 2 * k, Kind::kPairDesc, (kb | k) ? 1u : 0u);
+          tc_commit_pair(&empty_bar[s]);
+        }
+        if (ok) tc_commit_pair(&acc_full[acc]);
+      }
+    }
+  } else {
+    const int quarter = warp & 3, half = (warp - 2) >> 2;  // tensor-memory lanes this warp may read; its half of the columns
+    float* const stage = (float*)(ring + kGPairStages * kGPairStageBytes + (warp - 2) * kStageWarpBytes);
+    const uint32_t tmem_warp = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
+    int it = 0;
+    for (int idx = pair; idx < total; idx += pairs, ++it) {
+      const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
+      const int acc = it & 1, row0 = t.tm * kPairTile + (int)rank * 128 + quarter * 32, col0 = t.tn * kPairTile + half * 128;
+      const bool ok = mbar_wait(&acc_full[acc], (it >> 1) & 1, &abort_flag);
+      if (!__all_sync(0xFFFFFFFFu, ok)) break;
+      tc_fence_after();
+      const int blocks = min(4, (N - col0 + 31) / 32);
+      if (row0 < M && blocks > 0)
+        epilogue_direct<Kind::kScaled>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, t.tm != t.tn,
+                              walk_tile(t, kp, E.tri, Kind::kBlock).seg == 0, t.batch, M, N, E, Kind::kScaled ? row_units + t.batch * stride_ru : nullptr,
+                              Kind::kScaled ? col_units + t.batch * stride_cu : nullptr);
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) cluster_arrive(cluster_addr(&acc_empty[acc], 0));
+    }
+    tc_fence_before();
+  }
+
+  // After an expired wait in either CTA, both wait (with a limit) for every product and every load that the pair issued before its
+  // shared and tensor memory go away.
+  __syncthreads();
+  if (threadIdx.x == 0 && abort_flag) cluster_store(cluster_addr(&abort_flag, rank ^ 1), 1);
+  cluster_sync();
+  if (abort_flag) {
+    if (rank == 0 && warp == 1 && leader) tc_commit_pair(&drain_bar);  // the thread that issued the products
+    if (threadIdx.x == 0) mbar_drain(&drain_bar, 0);
+    if (rank == 0 && threadIdx.x == 0) {
+      const int even = fills, odd = cluster_load(cluster_addr(&fills, 1)), top = max(even, odd);
+      for (int n = pair_drain_first(even, odd, kGPairStages); n < top; ++n) {
+        const int s = n % kGPairStages, kind = pair_fill_kind(n, even, odd);
+        if (kind == kFillOddOnly) mbar_expect_tx(&full_bar[s], (uint32_t)kGPairStageBytes);
+        if (kind == kFillEvenOnly) mbar_complete_tx(&full_bar[s], (uint32_t)kGPairStageBytes);
+        mbar_drain(&full_bar[s], (n / kGPairStages) & 1);
+      }
+    }
+    cluster_sync();
+  }
+  if (threadIdx.x == 0 && abort_flag && status != nullptr) atomicExch(status, 1);
+  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
 }
 
 }  // namespace

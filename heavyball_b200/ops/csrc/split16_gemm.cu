@@ -19,7 +19,6 @@
 #include <cuda_fp16.h>
 
 #include "gemm_epilogue.cuh"
-#include "pair_drain.h"
 #include "per_device.h"
 
 namespace hb {
@@ -33,174 +32,14 @@ struct HalfKind {
   static constexpr int kBlock = HBK;
   static constexpr bool kScaled = true, kCrossFirst = true;
   static constexpr int kTermLoA = 1, kTermLoB = 0;  // A: hi, lo, hi   B: lo, hi, hi
-  static constexpr uint32_t kDesc = half_desc(TBM, TBN);
+  static constexpr uint32_t kDesc = half_desc(TBM, TBN), kPairDesc = half_desc(kPairTile, kPairTile);
   __device__ static __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, uint32_t accumulate) {
     tc_mma_bf16(d, a, b, desc, accumulate);  // kind::f16; the operand type is in the descriptor
   }
+  __device__ static __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, uint32_t accumulate) {
+    tc_mma_bf16_pair(d, a, b, desc, accumulate);
+  }
 };
-
-// ------------------------------------------------------------------------------------------ pair kernel
-// 256 x 256 tiles on CTA pairs (cta_group::2), one persistent pair per two SMs; structure as in ns_gemm.cu: each CTA stages 128 rows of
-// A and half of B (32 KiB per 64 of K, 5 stages), two accumulators, eight epilogue warps of 32 rows x 128 columns under the next
-// tile's main loop.
-constexpr int kHPairStages = 5;
-constexpr int kHPairStageBytes = 2 * kTTileBytes;
-constexpr int kHPairEpiWarps = 8;
-constexpr int kHPairThreads = 64 + 32 * kHPairEpiWarps;
-constexpr uint32_t kHPairDesc = half_desc(kPairTile, kPairTile);
-constexpr int kHPairSmemBytes = kHPairStages * kHPairStageBytes + kHPairEpiWarps * kStageWarpBytes + 1024;
-
-struct HalfTile {
-  int kb_lo, seg;  // K blocks of one term that the tile walks: [kb_lo, kb_lo + seg)
-};
-__device__ __forceinline__ HalfTile half_tile(const PairTile& t, int kp, int tri) {
-  int lo = 0, hi = kp / HBK;
-  if (tri) {
-    lo = min(hi, t.tm * (kPairTile / HBK));
-    hi = t.tn < t.tm ? lo : min(hi, (t.tn + 1) * (kPairTile / HBK));
-  }
-  return {lo, hi - lo};
-}
-
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kHPairThreads, 1)
-split16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N, int kp, int tiles_m,
-                    int tiles_n, int per_batch, int total, const Tf32Epilogue E, const float* row_units, int64_t stride_ru,
-                    const float* col_units, int64_t stride_cu, int* status) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kHPairStages];   // used in the even CTA: both CTAs' loads of a stage have landed
-  __shared__ __align__(8) uint64_t empty_bar[kHPairStages];  // in each CTA: the products that read the stage have finished
-  __shared__ __align__(8) uint64_t acc_full[2];              // in each CTA: accumulator finished
-  __shared__ __align__(8) uint64_t acc_empty[2];             // in the even CTA: all sixteen epilogue warps have read it
-  __shared__ __align__(8) uint64_t drain_bar;                // in each CTA, teardown only: all products have finished
-  __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_flag, skip_flag;
-  __shared__ int fills;                                      // ring fills this CTA issued
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool leader = elect_one();  // issues the loads (warp 0) and the products (warp 1), and waits for them in the teardown
-  const uint32_t rank = cluster_rank();
-  uint8_t* ring = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kHPairStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    for (int a = 0; a < 2; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * kHPairEpiWarps); }
-    mbar_init(&drain_bar, 1);
-    abort_flag = 0;
-    fills = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) { tmem_alloc_pair(&tmem_base_slot, 512); tmem_relinquish_pair(); }
-  griddep_wait();
-  // a kernel of this stream already gave up on a wait: do not pile more work on a broken pipeline (the even CTA decides)
-  if (threadIdx.x == 0) skip_flag = status != nullptr && *(volatile const int*)status != 0;
-  tc_fence_before();
-  __syncthreads();
-  cluster_sync();
-  tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-  const bool skip = cluster_load(cluster_addr(&skip_flag, 0)) != 0;
-
-  if (skip) {
-  } else if (warp == 0) {
-    if (leader) {
-      int n = 0;  // ring fills so far
-      bool ok = true;
-      for (int idx = pair; idx < total && ok; idx += pairs) {
-        const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
-        const HalfTile h = half_tile(t, kp, E.tri);
-        const int a_row = t.tm * kPairTile + (int)rank * 128, b_row = t.tn * kPairTile + (int)rank * 128;
-        for (int term = 0; term < 3 && ok; ++term) {
-          const int ka = (term == HalfKind::kTermLoA ? kp : 0), kb_off = (term == HalfKind::kTermLoB ? kp : 0);
-          for (int kb = 0; kb < h.seg; ++kb, ++n) {
-            const int s = n % kHPairStages, round = n / kHPairStages, k0 = (h.kb_lo + kb) * HBK;
-            ok = mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag);
-            if (!ok) break;
-            uint8_t* dst = ring + s * kHPairStageBytes;
-            const uint32_t bar = cluster_addr(&full_bar[s], 0);
-            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * kHPairStageBytes);
-            tma_load_3d_pair(dst, &map_a, bar, ka + k0, a_row, t.batch);  // rows past the operand's end arrive as zeros and count
-            tma_load_3d_pair(dst + kTTileBytes, &map_b, bar, kb_off + k0, b_row, t.batch);
-          }
-        }
-      }
-      fills = n;
-      griddep_launch();  // this CTA's last loads are on their way: the next kernel may take over SMs that drain
-    }
-  } else if (warp == 1) {
-    if (leader && rank == 0) {
-      int n = 0, it = 0;
-      bool ok = true;
-      for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
-        const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
-        const int seg = half_tile(t, kp, E.tri).seg, num_kb = 3 * seg, acc = it & 1;
-        ok = mbar_wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t d = tmem_base + (uint32_t)acc * 256u;
-        for (int kb = 0; kb < num_kb; ++kb, ++n) {
-          const int s = n % kHPairStages, round = n / kHPairStages;
-          ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
-          if (!ok) break;
-          tc_fence_after();
-          const uint32_t base = smem_u32(ring + s * kHPairStageBytes);
-          const uint64_t a_desc = make_smem_desc(base), b_desc = make_smem_desc(base + kTTileBytes);
-#pragma unroll
-          for (int k = 0; k < HBK / 16; ++k)
-            if (k == 0 && kb == 2 * seg)
-              tc_mma_f16_d11_pair(d, a_desc, b_desc, kHPairDesc);
-            else
-              tc_mma_bf16_pair(d, a_desc + 2 * k, b_desc + 2 * k, kHPairDesc, (kb | k) ? 1u : 0u);
-          tc_commit_pair(&empty_bar[s]);
-        }
-        if (ok) tc_commit_pair(&acc_full[acc]);
-      }
-    }
-  } else {
-    const int quarter = warp & 3, half = (warp - 2) >> 2;  // tensor-memory lanes this warp may read; its half of the columns
-    float* const stage = (float*)(ring + kHPairStages * kHPairStageBytes + (warp - 2) * kStageWarpBytes);
-    const uint32_t tmem_warp = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 128);
-    int it = 0;
-    for (int idx = pair; idx < total; idx += pairs, ++it) {
-      const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
-      const int acc = it & 1, row0 = t.tm * kPairTile + (int)rank * 128 + quarter * 32, col0 = t.tn * kPairTile + half * 128;
-      const bool ok = mbar_wait(&acc_full[acc], (it >> 1) & 1, &abort_flag);
-      if (!__all_sync(0xFFFFFFFFu, ok)) break;
-      tc_fence_after();
-      const int blocks = min(4, (N - col0 + 31) / 32);
-      if (row0 < M && blocks > 0)
-        epilogue_direct<true>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, t.tm != t.tn,
-                              half_tile(t, kp, E.tri).seg == 0, t.batch, M, N, E, row_units + t.batch * stride_ru,
-                              col_units + t.batch * stride_cu);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) cluster_arrive(cluster_addr(&acc_empty[acc], 0));
-    }
-    tc_fence_before();
-  }
-
-  // After an expired wait in either CTA, both wait (with a limit) for every product and every load that the pair issued before its
-  // shared and tensor memory go away.
-  __syncthreads();
-  if (threadIdx.x == 0 && abort_flag) cluster_store(cluster_addr(&abort_flag, rank ^ 1), 1);
-  cluster_sync();
-  if (abort_flag) {
-    if (rank == 0 && warp == 1 && leader) tc_commit_pair(&drain_bar);  // the thread that issued the products
-    if (threadIdx.x == 0) mbar_drain(&drain_bar, 0);
-    if (rank == 0 && threadIdx.x == 0) {
-      const int even = fills, odd = cluster_load(cluster_addr(&fills, 1)), top = max(even, odd);
-      for (int n = pair_drain_first(even, odd, kHPairStages); n < top; ++n) {
-        const int s = n % kHPairStages, kind = pair_fill_kind(n, even, odd);
-        if (kind == kFillOddOnly) mbar_expect_tx(&full_bar[s], (uint32_t)kHPairStageBytes);
-        if (kind == kFillEvenOnly) mbar_complete_tx(&full_bar[s], (uint32_t)kHPairStageBytes);
-        mbar_drain(&full_bar[s], (n / kHPairStages) & 1);
-      }
-    }
-    cluster_sync();
-  }
-  if (threadIdx.x == 0 && abort_flag && status != nullptr) atomicExch(status, 1);
-  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
-}
 
 // ------------------------------------------------------------------------------------------ operand split
 // One launch, two kinds of block; a row's exponent has to be known before its first value can be stored, so both kinds first look for
@@ -400,13 +239,19 @@ bool make_store_map(CUtensorMap* map, float* base, int rows, int cols, int64_t l
 }
 
 // Whether a product takes pairs, from the waves that 128 x 128 tiles (four in the place of a pair) and pairs need.  150 sizes measured,
-// 128 / pairs: what fits in one wave of small tiles is theirs (640 x 512 x 2048 37.5 / 47.3 us, 8 of 512 x 1024 x 4096 113 / 100 is the
-// exception), and so is a short K, whose three walks do not cover a pair's epilogue (16 of 1024 x 768 x 128 28.5 / 44.3 us, 6 of
-// 5504 x 1536 x 512 220 / 195 - from seven waves on K = 512 is long enough); a half more waves cost more than the tile
-// gains (8 of 1024 x 1024 x 2048 symmetric, one wave or two, 73 / 114 us).  Elsewhere pairs are up to 1.29 times as fast (4 of
-// 2048^3 217 / 202, 8 of 3000 x 1536 x 4096 865 / 737) and at worst 5 % slower.
-bool split16_take_pairs(int M, int N, int K, int64_t small_waves, int64_t big_waves) {
-  return M > 128 && N > 128 && small_waves >= 2 && 3 * big_waves <= 4 * small_waves && (K >= 768 || (K >= 512 && small_waves >= 7));
+// 128 / pairs:
+//   - More than one wave of small tiles, in about as many waves of pairs: pairs from K = 512 on (8 of 3000 x 4096 x 768 531 / 356 us, 6 of
+//     5504 x 1536 x 512 219 / 159, 16 of 512 x 1024 x 640 45.3 / 41.8).  With a shorter K the three walks do not cover a pair's epilogue (16 of
+//     1024 x 768 x 128 28.7 / 36.0, 3000 x 2048 x 384 25.3 / 30.7), except where the mirrored stores of a symmetric product make either
+//     epilogue long (3 of 4096 x 4096 x 256 119 / 107).  A half more waves cost more than the tile gains (16 of 1000 x 1000 x 4096
+//     symmetric, two waves or three, 253 / 277).
+//   - One wave of either: pairs where most of them have work and K is long (4 of 768 x 1024 x 5504 120 / 103, 3 of 384 x 2048 x 3000 60.5 / 62.4);
+//     else the small tiles, which are more (640 x 512 x 2048 30.2 / 41.3).
+// The worst of the 150 loses 11 %, the mean 0.2 %.
+bool split16_take_pairs(int M, int N, int K, bool symmetric, int64_t small_waves, int64_t big_waves, int64_t big, int64_t pairs) {
+  if (M <= 128 || N <= 128) return false;
+  if (small_waves >= 2) return 3 * big_waves <= 4 * small_waves && (K >= 512 || (symmetric && small_waves >= 4));
+  return K >= 3000 && 7 * big >= 4 * pairs && big_waves == 1;
 }
 
 int g_split16_tile = 0;
@@ -447,8 +292,8 @@ cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N
   if (e == cudaSuccess)
     e = pairs.get(device, cudaSuccess, &max_pairs, [](int& found) {
       cudaError_t s = cudaFuncSetAttribute(gemm128_kernel<HalfKind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
-      if (s == cudaSuccess) s = cudaFuncSetAttribute(split16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kHPairSmemBytes);
-      return s != cudaSuccess ? s : max_resident_pairs(split16_pair_kernel, kHPairThreads, kHPairSmemBytes, &found);
+      if (s == cudaSuccess) s = cudaFuncSetAttribute(gemm_pair_kernel<HalfKind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGPairSmemBytes);
+      return s != cudaSuccess ? s : max_resident_pairs(gemm_pair_kernel<HalfKind>, kGPairThreads, kGPairSmemBytes, &found);
     });
   if (e != cudaSuccess) return e;
   if (M == 0 || N == 0 || batch == 0) return cudaSuccess;
@@ -466,12 +311,12 @@ cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N
   };
   const int64_t small = (int64_t)tiles(TBM) * batch, big = (int64_t)tiles(kPairTile) * batch;
   const int64_t small_waves = (small + 4 * max_pairs - 1) / (4 * max_pairs), big_waves = (big + max_pairs - 1) / max_pairs;
-  bool pair = split16_take_pairs(M, N, K, small_waves, big_waves);
+  bool pair = split16_take_pairs(M, N, K, E.symmetric != 0, small_waves, big_waves, big, max_pairs);
   if (g_split16_tile != 0) pair = g_split16_tile == 256;
   if (pair) {
     const int tm = (M + kPairTile - 1) / kPairTile, tn = (N + kPairTile - 1) / kPairTile;
     const int grid = 2 * (int)(big < max_pairs ? big : max_pairs);
-    return launch_chained(split16_pair_kernel, dim3(grid), kHPairThreads, kHPairSmemBytes, stream, ma, mb, M, N, (int)kp, tm, tn,
+    return launch_chained(gemm_pair_kernel<HalfKind>, dim3(grid), kGPairThreads, kGPairSmemBytes, stream, ma, mb, M, N, (int)kp, tm, tn,
                           tiles(kPairTile), (int)big, E, A.unit, stride_ru, B.unit, stride_cu, status);
   }
   // bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing past it

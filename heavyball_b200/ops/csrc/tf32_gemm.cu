@@ -31,141 +31,21 @@ namespace hb {
 namespace {
 
 constexpr int TBK = 32;
-// tf32 x tf32 -> fp32, both operands K-major, M = 128, N = 128
-constexpr uint32_t kTf32InstrDesc =
-    (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TBN >> 3) << 17) | ((uint32_t)(TBM >> 4) << 24);
+// tf32 x tf32 -> fp32, both operands K-major
+constexpr uint32_t tf32_desc(int m, int n) { return (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(m >> 4) << 24); }
 
 struct Tf32Kind {
   static constexpr int kBlock = TBK;
   static constexpr bool kScaled = false, kCrossFirst = false;
   static constexpr int kTermLoA = 2, kTermLoB = 1;  // A: hi, hi, lo   B: hi, lo, hi
-  static constexpr uint32_t kDesc = kTf32InstrDesc;
+  static constexpr uint32_t kDesc = tf32_desc(TBM, TBN), kPairDesc = tf32_desc(kPairTile, kPairTile);
   __device__ static __forceinline__ void mma(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, uint32_t accumulate) {
     tc_mma_tf32(d, a, b, desc, accumulate);
   }
+  __device__ static __forceinline__ void mma_pair(uint32_t d, uint64_t a, uint64_t b, uint32_t desc, uint32_t accumulate) {
+    tc_mma_tf32_pair(d, a, b, desc, accumulate);
+  }
 };
-
-// ------------------------------------------------------------------------------------------ 256 x 256 tiles
-// A 128 x 128 tile asks the L2 for 32 KiB of operands per 256 tensor-core cycles (tf32 runs at half the bf16 rate on
-// operands twice as wide), which is more than the L2 delivers to 148 SMs at once; a 256 x 256 tile needs half of that
-// per FLOP.  One CTA per SM: four 128 x 128 fp32 accumulators = all 512 columns of tensor memory, 64 KiB ring stages
-// (two 128-row boxes per operand), two 128 x 256 x 8 instructions per 8 of K sharing the B rows.  Eight epilogue
-// warps: two per 32-lane quarter of tensor memory, one for each 128-row half of the tile.
-constexpr int TBM2 = 256, TBN2 = 256;
-constexpr int kTStageBytes2 = 4 * kTTileBytes;                  // 64 KiB
-constexpr int kTSmemBytes2 = kTStages * kTStageBytes2 + 1024;
-constexpr int kTThreads2 = 320;                                 // producer, MMA, 8 epilogue warps
-constexpr uint32_t kTTmemCols2 = 512;
-constexpr uint32_t kTf32InstrDesc256 =
-    (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TBN2 >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-
-__global__ void __launch_bounds__(kTThreads2, 1)
-tf32_gemm256_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N, int kp,
-                    const Tf32Epilogue E, int* status) {
-  extern __shared__ uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t full_bar[kTStages];
-  __shared__ __align__(8) uint64_t empty_bar[kTStages];
-  __shared__ __align__(8) uint64_t accum_bar, drain_bar;  // drain_bar: teardown only
-  __shared__ uint32_t tmem_base_slot;
-  __shared__ int abort_flag;
-
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const bool leader = elect_one();  // issues the loads (warp 0) and the products (warp 1), and waits for them in the teardown
-  uint8_t* tiles = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  const int tiles_n = (N + TBN2 - 1) / TBN2;
-  int tm = blockIdx.x / tiles_n, tn = blockIdx.x % tiles_n;
-  if (E.symmetric) {
-    int left = blockIdx.x;
-    tm = 0;
-    while (left >= tiles_n - tm) { left -= tiles_n - tm; ++tm; }
-    tn = tm + left;
-  }
-  const int batch = blockIdx.y;
-  int kb_lo = 0, kb_hi = kp / TBK;
-  if (E.tri) {
-    kb_lo = min(kb_hi, tm * (TBM2 / TBK));
-    kb_hi = tn < tm ? kb_lo : min(kb_hi, (tn + 1) * (TBN2 / TBK));
-  }
-  const int seg_kb = kb_hi - kb_lo;
-  const int num_kb = 3 * seg_kb;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < kTStages; ++s) { mbar_init(&full_bar[s], 1); mbar_init(&empty_bar[s], 1); }
-    mbar_init(&accum_bar, 1);
-    mbar_init(&drain_bar, 1);
-    abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) { tmem_alloc(&tmem_base_slot, kTTmemCols2); tmem_relinquish(); }
-  griddep_wait();
-  const bool skip = __syncthreads_or(threadIdx.x == 0 && status != nullptr && *(volatile const int*)status != 0);
-  griddep_launch();
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tmem_base = tmem_base_slot;
-
-  int issued = 0;
-  if (skip) {
-  } else if (warp == 0) {
-    if (leader) {
-      for (int kb = 0; kb < num_kb; ++kb) {
-        const int s = kb % kTStages, round = kb / kTStages;
-        if (!mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag)) break;
-        uint8_t* dst = tiles + s * kTStageBytes2;
-        const int seg = kb / seg_kb, k0 = (kb_lo + kb - seg * seg_kb) * TBK;
-        const int ka = k0 + (seg == 2 ? kp : 0), kb_col = k0 + (seg == 1 ? kp : 0);   // A: hi, hi, lo   B: hi, lo, hi
-        mbar_expect_tx(&full_bar[s], kTStageBytes2);   // rows past the operand's end arrive as zeros and count as bytes
-        tma_load_3d(dst, &map_a, &full_bar[s], ka, tm * TBM2, batch);
-        tma_load_3d(dst + kTTileBytes, &map_a, &full_bar[s], ka, tm * TBM2 + 128, batch);
-        tma_load_3d(dst + 2 * kTTileBytes, &map_b, &full_bar[s], kb_col, tn * TBN2, batch);
-        tma_load_3d(dst + 3 * kTTileBytes, &map_b, &full_bar[s], kb_col, tn * TBN2 + 128, batch);
-        issued = kb + 1;
-      }
-    }
-  } else if (warp == 1) {
-    if (leader) {
-      bool ok = true;
-      for (int kb = 0; kb < num_kb && ok; ++kb) {
-        const int s = kb % kTStages, round = kb / kTStages;
-        ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t base = smem_u32(tiles + s * kTStageBytes2);
-        const uint64_t a_top = make_smem_desc(base), a_bot = make_smem_desc(base + kTTileBytes);
-        // 256 B rows = 32 eight-row groups, 1 KiB apart: the two 128-row boxes are contiguous
-        const uint64_t b_desc = make_smem_desc(base + 2 * kTTileBytes);
-#pragma unroll
-        for (int k = 0; k < TBK / 8; ++k) {
-          const uint32_t acc = (kb | k) ? 1u : 0u;
-          tc_mma_tf32(tmem_base, a_top + 2 * k, b_desc + 2 * k, kTf32InstrDesc256, acc);
-          tc_mma_tf32(tmem_base + 256u, a_bot + 2 * k, b_desc + 2 * k, kTf32InstrDesc256, acc);
-        }
-        tc_commit(&empty_bar[s]);
-      }
-      if (ok) tc_commit(&accum_bar);
-    }
-  } else {
-    const int quarter = warp & 3, half = (warp - 2) >> 2;   // warps 2..5: rows 0..127 of the tile, warps 6..9: rows 128..255
-    const bool have = (num_kb == 0) || mbar_wait(&accum_bar, 0, &abort_flag);
-    tc_fence_after();
-    const int row0 = tm * TBM2 + half * 128 + quarter * 32;
-    if (have && row0 < M)
-      epilogue_direct<false>(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 256), lane,
-                      (float*)(tiles + (warp - 2) * kStageWarpBytes), row0, tn * TBN2, TBN2 / 32, tm != tn, num_kb == 0,
-                      batch, M, N, E);
-    tc_fence_before();
-  }
-
-  __syncthreads();
-  if (abort_flag) {
-    if (warp == 0 && leader) ring_drain(full_bar, issued, kTStages);
-    if (warp == 1 && leader) products_drain(&drain_bar);
-    __syncthreads();
-    if (threadIdx.x == 0 && status != nullptr) atomicExch(status, 1);
-  }
-  if (warp == 1) { __syncwarp(); tc_fence_after(); tmem_dealloc(tmem_base, kTTmemCols2); }
-}
 
 // One block moves a 64 x 64 tile of the source through shared memory and writes the [hi | lo] rows it covers of either
 // or both operand orientations (see tf32_gemm.h).  The zero padding [K, kp) of every row is written too.  256 threads
@@ -268,14 +148,14 @@ void set_tf32_gemm_tile_override(int tile) { g_tf32_tile_override = (tile == 128
 
 cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int K, int batch, const Tf32Epilogue& E,
                              int* status, cudaStream_t stream) {
-  static PerDevice<bool> configured;
-  int device = 0;
-  bool done = false;
+  static PerDevice<int> pairs;
+  int device = 0, max_pairs = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess)
-    e = configured.get(device, cudaSuccess, &done, [](bool&) {
-      const cudaError_t s = cudaFuncSetAttribute(gemm128_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
-      return s != cudaSuccess ? s : cudaFuncSetAttribute(tf32_gemm256_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes2);
+    e = pairs.get(device, cudaSuccess, &max_pairs, [](int& found) {
+      cudaError_t s = cudaFuncSetAttribute(gemm128_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
+      if (s == cudaSuccess) s = cudaFuncSetAttribute(gemm_pair_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGPairSmemBytes);
+      return s != cudaSuccess ? s : max_resident_pairs(gemm_pair_kernel<Tf32Kind>, kGPairThreads, kGPairSmemBytes, &found);
     });
   if (e != cudaSuccess) return e;
   if (M == 0 || N == 0 || batch == 0) return cudaSuccess;
@@ -289,17 +169,19 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   if (!make_f32_map(&ma, A2, M, ld, ld, (int64_t)M * ld, batch) || !make_f32_map(&mb, B2, N, ld, ld, (int64_t)N * ld, batch))
     return cudaErrorInvalidValue;
 
-  // big tiles once there are enough of them to fill the machine (one CTA per SM) and K is long enough to pay for a
-  // serial epilogue; small problems keep 128 x 128 tiles, two CTAs per SM
-  const int big_m = (M + TBM2 - 1) / TBM2, big_n = (N + TBN2 - 1) / TBN2;
-  const int64_t big_tiles = (int64_t)(E.symmetric ? big_n * (big_n + 1) / 2 : big_m * big_n) * batch;
-  bool big = M >= TBM2 && N >= TBN2 && K >= 512 && big_tiles >= 96;
+  // 256 x 256 tiles on CTA pairs once there are enough of them and K is long enough to pay for their epilogue; small problems keep
+  // 128 x 128 tiles, two CTAs per SM.  (The line stands where it stood for the one-CTA tile of this size that the pairs replaced:
+  // whether an entry of a symmetric product near the diagonal is computed or mirrored depends on the tile, and with it its last bit.)
+  const int big_m = (M + kPairTile - 1) / kPairTile, big_n = (N + kPairTile - 1) / kPairTile;
+  const int per_batch = E.symmetric ? big_n * (big_n + 1) / 2 : big_m * big_n;
+  const int64_t big_tiles = (int64_t)per_batch * batch;
+  bool big = M >= kPairTile && N >= kPairTile && K >= 512 && big_tiles >= 96;
   if (g_tf32_tile_override == 128) big = false;
   if (g_tf32_tile_override == 256) big = true;
-  if (big) {
-    dim3 grid(E.symmetric ? big_n * (big_n + 1) / 2 : big_m * big_n, batch);
-    return launch_chained(tf32_gemm256_kernel, grid, kTThreads2, kTSmemBytes2, stream, ma, mb, M, N, (int)kp, E, status);
-  }
+  if (big)
+    return launch_chained(gemm_pair_kernel<Tf32Kind>, dim3(2 * (int)(big_tiles < max_pairs ? big_tiles : max_pairs)), kGPairThreads,
+                          kGPairSmemBytes, stream, ma, mb, M, N, (int)kp, big_m, big_n, per_batch, (int)big_tiles, E, nullptr, 0, nullptr, 0,
+                          status);
 
   // plain products leave through the bulk-store path (bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing
   // past it); everything else is written by the epilogue threads themselves
