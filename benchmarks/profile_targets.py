@@ -8,6 +8,7 @@
     python benchmarks/profile_targets.py ln_small        # LayerNorm fwd + bwd kernels, 16384 x 768 fp32 (50 MB) x 4 tensors
     python benchmarks/profile_targets.py gelu_small      # GELU fwd, and bwd + bias gradient, 16384 x 3072 bf16 (100 MB per tensor)
     python benchmarks/profile_targets.py tf32_small      # split-tf32 GEMM, 4 x (2048 x 2048 x 2048)
+    python benchmarks/profile_targets.py split16_small   # the same product of fp16 pairs
     python benchmarks/profile_targets.py qr_small        # panel-wise Cholesky QR of 8 x (1024 x 1024), eager launches
     python benchmarks/profile_targets.py ns_big          # Newton-Schulz on 4 x (4096 x 4096): the 256 x 256-tile kernel
     python benchmarks/profile_targets.py soap_small      # one plain SOAP step on 8 x 1024^2 (tf32 GEMMs with fused epilogues)
@@ -207,24 +208,33 @@ def gelu_small():
     torch.cuda.profiler.stop()
 
 
-def tf32_small():
+def _product(name):
+    product = getattr(ops, name)
     a = torch.randn(4, 2048, 2048, device="cuda")
     b = torch.randn(4, 2048, 2048, device="cuda")
-    out = ops.matmul3(a, b)
-    us = _timed(lambda: ops.matmul3(a, b))
+    out = product(a, b)
+    us = _timed(lambda: product(a, b))
     us_ref = _timed(lambda: torch.matmul(a, b))
     flops = 2 * 4 * 2048**3
-    print(f"matmul3 4x2048^3: {us:.1f} us incl. both split passes = {flops / us / 1e6:.1f} useful TFLOP/s "
-          f"({3 * flops / us / 1e6:.1f} tf32 TFLOP/s issued); torch fp32 matmul {us_ref:.1f} us = {flops / us_ref / 1e6:.1f} TFLOP/s")
+    print(f"{name} 4x2048^3: {us:.1f} us incl. both split passes = {flops / us / 1e6:.1f} useful TFLOP/s "
+          f"({3 * flops / us / 1e6:.1f} TFLOP/s issued); torch fp32 matmul {us_ref:.1f} us = {flops / us_ref / 1e6:.1f} TFLOP/s")
     err = (out.double() - a.double() @ b.double()).abs().max().item()
     ref_err = (torch.matmul(a, b).double() - a.double() @ b.double()).abs().max().item()
     print(f"max abs error vs fp64: ours {err:.3e}, torch fp32 {ref_err:.3e}")
     torch.cuda.synchronize()
     torch.cuda.profiler.start()
-    ops.matmul3(a, b)
+    product(a, b)
     torch.cuda.synchronize()
     torch.cuda.profiler.stop()
     ops.check_status()
+
+
+def tf32_small():
+    _product("matmul3")
+
+
+def split16_small():
+    _product("matmul16")
 
 
 def qr_small():
@@ -336,4 +346,4 @@ def soap_refresh():
 
 if __name__ == "__main__":
     {"psgd_fit": psgd_fit, "soap_refresh": soap_refresh, "ns_big": ns_big, "soap_small": soap_small, "psgd_small": psgd_small, "qr_small": qr_small, "opt_step_gpt2": opt_step_gpt2, "ns_small": ns_small, "adam_small": adam_small, "chain_small": chain_small, "launches": launches, "ce_small": ce_small,
-     "ln_small": ln_small, "tf32_small": tf32_small, "gelu_small": gelu_small}[sys.argv[1]]()
+     "ln_small": ln_small, "tf32_small": tf32_small, "split16_small": split16_small, "gelu_small": gelu_small}[sys.argv[1]]()
