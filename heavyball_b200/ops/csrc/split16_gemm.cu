@@ -12,8 +12,8 @@
 // at its magnitude as well.  Error against 64 bits, relative 2-norm, K = 1024 / 2048 / 8192: 1.2e-6 / 2.5e-6 / 9.7e-6 (tf32: 1.1e-5 /
 // 2.1e-5 / 8.4e-5), the same with rows over thirty decades and with entries over eight decades along K.
 //
-// Measured on one B200, of measured peak (1.64 PFLOP/s / 3): 2 of 5504 x 2048 x 2048 224 us = 412 TFLOP/s, 0.75 (split tf32 409 us);
-// 4 of 2048^3 176 us = 390, 0.71 (277); 8 of 1024^3 64 us = 269, 0.49, one wave (98).
+// Measured on one B200, of measured peak (1.64 PFLOP/s / 3): 2 of 5504 x 2048 x 2048 205 us = 451 TFLOP/s, 0.82 (split tf32 340 us);
+// 4 of 2048^3 159 us = 431, 0.79 (265); 8 of 1024^3 50 us = 346, 0.63, one wave (76).
 #include "split16_gemm.h"
 
 #include <cuda_fp16.h>
