@@ -613,8 +613,11 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (!__all_sync(0xFFFFFFFFu, ok)) break;
       tc_fence_after();
       const int blocks = min(4, (N - col0 + 31) / 32);
-      if (row0 < M && blocks > 0)
-        epilogue_direct<Kind::kScaled>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, t.tm != t.tn,
+      // a tile on the diagonal: computed whole, or (symmetric == 2) as three of 128 x 128 whose middle one is mirrored
+      const bool thirds = E.symmetric == 2 && t.tm == t.tn;
+      const bool mirrored = thirds ? rank == 0 && half == 1 : t.tm != t.tn;
+      if (row0 < M && blocks > 0 && !(thirds && rank == 1 && half == 0))
+        epilogue_direct<Kind::kScaled>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, mirrored,
                               walk_tile(t, kp, E.tri, Kind::kBlock).seg == 0, t.batch, M, N, E, Kind::kScaled ? row_units + t.batch * stride_ru : nullptr,
                               Kind::kScaled ? col_units + t.batch * stride_cu : nullptr);
       tc_fence_before();

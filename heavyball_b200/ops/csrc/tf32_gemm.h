@@ -43,6 +43,7 @@ struct Tf32Epilogue {
                            // tiles below the diagonal are stored as zeros without a product
   int symmetric;           // A2 == B2 (so M == N and the product is symmetric): only tiles on or above the diagonal are
                            // computed and each is also stored transposed.  kEpiStore / kEpiLerp / kEpiAdd with C set and S null.
+                           // 2 (set by launch_tf32_gemm): 256 x 256 tiles on the diagonal are stored as 128 x 128 ones would be
 };
 
 // out[b] = epilogue(A[b] * B[b]^T) over split operands A2: [batch, M, 2 * kp(K)], B2: [batch, N, 2 * kp(K)].

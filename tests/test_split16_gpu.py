@@ -93,6 +93,23 @@ def test_symmetric_and_triangular_products(B, n, K, tile):
     ops.check_status()
 
 
+@pytest.mark.parametrize("B,n,K", [(1, 1500, 4100), (2, 1300, 4096), (1, 2048, 4128), (2, 1537, 1025), (6, 1280, 512)])
+@pytest.mark.parametrize("mode", ["store", "lerp"])
+def test_symmetric_split_tf32_has_the_bits_of_small_tiles(mode, B, n, K):
+    """Below 96 large tiles, pairs store their diagonal as 128 x 128 tiles do: ragged edges, one and two waves, every branch of the rule."""
+    x, old = _rand(B, n, K, seed=19), _rand(B, n, n, seed=20)
+    op, _ = ops.tf32_split(x, True, False)
+    kwargs = dict(mode=ops.EPI_LERP, w=0.25) if mode == "lerp" else {}
+    results = []
+    for forced in (0, 128):
+        ops.load().set_tf32_gemm_tile(forced)
+        results.append(old.clone())
+        ops.tf32_gemm(op, op, K, out=results[-1], **kwargs)
+    ops.load().set_tf32_gemm_tile(0)
+    ops.check_status()
+    assert torch.equal(*results)
+
+
 def test_ranges_that_fp16_does_not_have(tile):
     """Rows over sixty decades, rows of zeros, of subnormals and with an infinity or a NaN next to ordinary ones."""
     a, b = _rand(1, 300, 96, seed=12), _rand(1, 140, 96, seed=13)
