@@ -101,7 +101,7 @@ class TensorCoreBackend:
              m=None, v=None):  # fmt: skip
         if out is None:  # rows start on 16-byte boundaries
             rows, cols = a.data.shape[1], b.data.shape[1]
-            out = torch.empty(a.data.shape[0], rows, -(-cols // 4) * 4, device=a.data.device)[..., :cols]
+            out = torch.empty(a.data.shape[0], rows, -(-cols // 4) * 4, device=a.data.device, dtype=torch.float32)[..., :cols]
         ops.split16_gemm(a, b, mode=mode, alpha=alpha, w=w, b1=b1, b2c=b2, eps=eps, out=out, m=m, v=v)
         if split_out == ops.SPLIT_NONE:
             return None

@@ -227,3 +227,28 @@ def test_identity_defect_flags_what_the_definition_flags(k):
     bad = torch.zeros(6, dtype=torch.int32, device="cuda")
     ops.load().identity_defect(gram, 1e-4, bad)
     assert bad.tolist() == [0, 1, 1, 1, 1, 0]
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float64])
+@pytest.mark.parametrize("name", ["SOAP", "PSGDKron"])
+def test_a_step_does_not_depend_on_the_default_dtype(name, dtype):
+    """Scripts that build their models under another default dtype: intermediates of the matrix stages stay fp32."""
+
+    def run(default):
+        torch.manual_seed(0)
+        ws = [torch.nn.Parameter(torch.randn(200, 333, device="cuda") * 0.1) for _ in range(2)]
+        grads = [[torch.randn_like(w) * 1e-2 for w in ws] for _ in range(4)]
+        kwargs = dict(preconditioner_update_probability=1.0) if name == "PSGDKron" else dict(precondition_frequency=2)
+        opt = getattr(hb, name)(ws, lr=1e-2, **kwargs)
+        for i, gs in enumerate(grads):
+            for w, g in zip(ws, gs):
+                w.grad = g.clone()
+            torch.set_default_dtype(default if i == 3 else torch.float32)
+            try:
+                opt.step()
+            finally:
+                torch.set_default_dtype(torch.float32)
+        return ws
+
+    for got, want in zip(run(dtype), run(torch.float32)):
+        assert torch.isfinite(want).all() and float((got - want).abs().max()) < 1e-5 * float(want.abs().max())
