@@ -212,6 +212,17 @@ def test_columns_in_order_and_back(B, n, k):
     assert torch.equal(_permute_columns(moved, order, inverse=True).view(torch.int32), x.view(torch.int32))
 
 
+@pytest.mark.parametrize("B", [65535, 65536])
+def test_columns_of_more_matrices_than_a_grid_has(B):
+    """The kernel counts matrices in the grid's second dimension; one more goes the general way."""
+    from heavyball_b200.utils.soap import _permute_columns
+
+    g = torch.Generator(device="cuda").manual_seed(B)
+    x, order = torch.randn(B, 2, 3, device="cuda", generator=g), torch.rand(B, 3, device="cuda", generator=g).argsort(-1)
+    moved = _permute_columns(x, order)
+    assert torch.equal(moved, x.gather(-1, order.unsqueeze(-2).expand_as(x))) and torch.equal(_permute_columns(moved, order, inverse=True), x)
+
+
 @pytest.mark.parametrize("k", [1, 33, 256, 1000])
 def test_identity_defect_flags_what_the_definition_flags(k):
     from heavyball_b200 import ops
