@@ -25,6 +25,7 @@
 #include "tf32_gemm.h"
 
 #include "gemm_epilogue.cuh"
+#include "gemm_rules.h"
 #include "per_device.h"
 
 namespace hb {
@@ -142,19 +143,6 @@ cudaError_t launch_tf32_split(const float* src, int64_t ld_src, int64_t stride_s
   return launch_chained(tf32_split_kernel, grid, 256, 0, stream, src, ld_src, stride_src, R, C, dst_same, dst_trans, kpC, kpR);
 }
 
-// Symmetric products with fewer than 96 of the large tiles: whether pairs are the faster ones, from the numbers of 128 x 128 tiles and of
-// pairs' tiles.  65 sizes measured, 128 / pairs:
-//   - Small tiles that do not fit at once: pairs in two waves (3072 x 3072 x 2048 163 / 134 us, 4 of 1536 x 1536 x 1024 95 / 80).
-//   - They do, but two on an SM: pairs in one wave from K = 1024 on (2 of 2048 x 2048 x 5504 251 / 204, 2 of 1536 x 1536 x 1024 45.7 / 44.5), not
-//     in two (8 of 1024 x 1024 x 2048 112 / 143).
-//   - One on an SM: only a long K and enough tiles (2048 x 2048 x 5504 206 / 165, 2 of 1024 x 1024 x 4096 144 / 127, 1024 x 1024 x 5504
-//     142 / 158, 2048 x 2048 x 2048 62.5 / 69.3).
-static bool pairs_for_symmetric(int K, int64_t small, int64_t big, int64_t pairs) {
-  if (small > 4 * pairs) return big <= 2 * pairs;
-  if (big > pairs) return false;
-  return small > 2 * pairs ? K >= 1024 : K >= 4096 && big >= 20;
-}
-
 static int g_tf32_tile_override = 0;  // 0 = by size, 128 / 256 = forced (tests and measurements)
 int tf32_gemm_tile_override() { return g_tf32_tile_override; }
 void set_tf32_gemm_tile_override(int tile) { g_tf32_tile_override = (tile == 128 || tile == 256) ? tile : 0; }
@@ -182,26 +170,18 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   if (!make_f32_map(&ma, A2, M, ld, ld, (int64_t)M * ld, batch) || !make_f32_map(&mb, B2, N, ld, ld, (int64_t)N * ld, batch))
     return cudaErrorInvalidValue;
 
-  // 256 x 256 tiles on CTA pairs once there are enough of them and K is long enough to pay for their epilogue; small problems keep
-  // 128 x 128 tiles, two CTAs per SM.  (The line stands where it stood for the one-CTA tile of this size that the pairs replaced:
-  // whether an entry of a symmetric product near the diagonal is computed or mirrored depends on the tile, and with it its last bit.)
-  const int big_m = (M + kPairTile - 1) / kPairTile, big_n = (N + kPairTile - 1) / kPairTile;
-  const int per_batch = E.symmetric ? big_n * (big_n + 1) / 2 : big_m * big_n;
-  const int64_t big_tiles = (int64_t)per_batch * batch;
-  bool big = M >= kPairTile && N >= kPairTile && K >= 512 && big_tiles >= 96;
-  Tf32Epilogue E2 = E;
-  // Symmetric products below that line with a long K: pairs as well, with the diagonal stored as 128 x 128 tiles store it.
-  const int small_n = (N + TBN - 1) / TBN;
-  if (!big && E.symmetric && M >= kPairTile && pairs_for_symmetric(K, (int64_t)small_n * (small_n + 1) / 2 * batch, big_tiles, max_pairs)) {
-    big = true;
-    E2.symmetric = 2;
+  TileChoice tiles = tf32_tiles(M, N, K, batch, E.symmetric != 0, max_pairs);
+  if (g_tf32_tile_override == 128) tiles = kSmallTiles;
+  if (g_tf32_tile_override == 256 && tiles == kSmallTiles) tiles = kPairTiles;
+  if (tiles != kSmallTiles) {
+    const int big_m = (M + kPairTile - 1) / kPairTile, big_n = (N + kPairTile - 1) / kPairTile;
+    const int per_batch = (int)output_tiles(M, N, kPairTile, E.symmetric != 0);
+    const int64_t total = (int64_t)per_batch * batch;
+    Tf32Epilogue E2 = E;
+    if (tiles == kPairTilesSmallDiagonal) E2.symmetric = 2;
+    return launch_chained(gemm_pair_kernel<Tf32Kind>, dim3(2 * (int)(total < max_pairs ? total : max_pairs)), kGPairThreads, kGPairSmemBytes, stream,
+                          ma, mb, M, N, (int)kp, big_m, big_n, per_batch, (int)total, E2, nullptr, 0, nullptr, 0, status);
   }
-  if (g_tf32_tile_override == 128) big = false;
-  if (g_tf32_tile_override == 256) big = true;
-  if (big)
-    return launch_chained(gemm_pair_kernel<Tf32Kind>, dim3(2 * (int)(big_tiles < max_pairs ? big_tiles : max_pairs)), kGPairThreads,
-                          kGPairSmemBytes, stream, ma, mb, M, N, (int)kp, big_m, big_n, per_batch, (int)big_tiles, E2, nullptr, 0, nullptr, 0,
-                          status);
 
   // plain products leave through the bulk-store path (bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing
   // past it); everything else is written by the epilogue threads themselves

@@ -194,3 +194,24 @@ def test_tensor_core_and_leaf_kernels_run_on_a_second_device_of_the_process():
         ops.load().chol_inv_leaf(a @ a.mT + 256 * torch.eye(256, device=dev), r, inv, 0, 128, info)
         assert info.sum().item() == 0
         ops.check_status()
+
+
+def test_tile_of_symmetric_products(tmp_path):
+    """Sizes on both sides of every line of the rule, with the pairs of a B200: (batch, n, K, expected choice)."""
+    cases = [(4, 1536, 64, 0), (4, 2048, 192, 0), (4, 1536, 255, 0), (4, 1536, 256, 2), (3, 2048, 511, 2), (3, 2048, 512, 1), (2, 3072, 511, 0),
+             (8, 1024, 2048, 0), (2, 1536, 1023, 0), (2, 1536, 1024, 2), (1, 2048, 4095, 0), (1, 2048, 4096, 2), (1, 1024, 5504, 0),
+             (300, 255, 4096, 0), (300, 256, 512, 1)]  # fmt: skip
+    table = ", ".join("{%d, %d, %d, %d}" % c for c in cases)
+    _run(tmp_path, r"""
+#include <cstdio>
+#include "gemm_rules.h"
+int main() {
+  const int cases[][4] = {%s};
+  int wrong = 0;
+  for (const auto& c : cases) {
+    const int got = hb::tf32_tiles(c[1], c[1], c[2], c[0], true, 74);
+    if (got != c[3]) { printf("%%d of %%d, K %%d: %%d\n", c[0], c[1], c[2], got); wrong = 1; }
+  }
+  return wrong || hb::tf32_tiles(2048, 2048, 256, 4, false, 74) != hb::kSmallTiles;
+}
+""" % table)  # fmt: skip
