@@ -308,20 +308,30 @@ def tf32_gemm(a2: torch.Tensor, b2: torch.Tensor, K: int, *, mode: int = EPI_STO
 
 
 class Split16:
-    """Operand of :func:`split16_gemm`: ``data`` (fp16 ``[batch, rows, 2 kp(K)]``, rows of ``[hi | lo]``), ``unit`` (what one unit of
-    a row stands for, a power of two) and the contraction length ``K``."""
+    """Operand of :func:`split16_gemm`: ``data`` (fp16 ``[batch, rows, 2 kp(K)]``, rows of ``[hi | lo]``), ``scale`` (what one unit of
+    a row stands for, a power of two; in the mantissa, the number of the row's values that are too small for 22 bits), the contraction
+    length ``K`` and the tensor ``x`` that it was made from (``trans``: with its columns as rows).  Results that hang on such values are
+    computed from ``x``: it must not change while the operand is in use."""
 
-    __slots__ = ("data", "unit", "K")
+    __slots__ = ("data", "scale", "K", "x", "trans")
 
-    def __init__(self, data, unit, K):
-        self.data, self.unit, self.K = data, unit, K
+    def __init__(self, data, scale, K, x, trans):
+        self.data, self.scale, self.K, self.x, self.trans = data, scale, K, x, trans
+
+    @property
+    def unit(self):
+        return (self.scale.view(torch.int32) & 0x7F800000).view(torch.float32)
+
+    @property
+    def short(self):
+        return self.scale.view(torch.int32) & 0x7FFFFF
 
 
 def split16(x: torch.Tensor, same: bool = True, trans: bool = False):
     """:func:`tf32_split` for the fp16-pair product: operands with the rows / the columns of ``x`` as operand rows."""
     launch_counter.count += 1
     s, su, t, tu = load().split16(x, same, trans)
-    return (Split16(s, su, x.shape[2]) if same else None), (Split16(t, tu, x.shape[1]) if trans else None)
+    return (Split16(s, su, x.shape[2], x, False) if same else None), (Split16(t, tu, x.shape[1], x, True) if trans else None)
 
 
 def split16_gemm(a: Split16, b: Split16, *, mode: int = EPI_STORE, alpha: float = 1.0, w: float = 0.0, b1: float = 0.0, b2c: float = 0.0,
@@ -330,7 +340,8 @@ def split16_gemm(a: Split16, b: Split16, *, mode: int = EPI_STORE, alpha: float 
     """``epilogue(A @ B^T)`` over fp16-pair operands, at twice the tensor-core rate of :func:`tf32_gemm` and half its operand bytes;
     modes and outputs as there, without split outputs (a row's exponent is known when the row is)."""
     launch_counter.count += 1
-    load().split16_gemm(a.data, a.unit, b.data, b.unit, a.K, mode, alpha, w, b1, b2c, eps, out, m, v, upper_upper, _status(a.data.device))
+    load().split16_gemm(a.data, a.scale, a.x, a.trans, b.data, b.scale, b.x, b.trans, a.K, mode, alpha, w, b1, b2c, eps, out, m, v, upper_upper,
+                        _status(a.data.device))  # fmt: skip
 
 
 def matmul3(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: bool = False, alpha: float = 1.0,
@@ -344,9 +355,9 @@ def matmul3(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: bo
 
 def matmul16(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: bool = False, alpha: float = 1.0,
              upper_upper: bool = False) -> torch.Tensor:
-    """:func:`matmul3` from fp16 pairs (:func:`split16_gemm`): one and a half to twice as fast, with an eighth of its error.  Measured
-    against ``|op(a)| @ |op(b)|``; entries 2^-29 and more below the largest of their row of ``op(a)`` (column of ``op(b)``) keep fewer
-    than 22 bits, down to an absolute error of 2^-51 of that largest one."""
+    """:func:`matmul3` from fp16 pairs (:func:`split16_gemm`): one and a half to twice as fast, with an eighth of its error against
+    ``|op(a)| @ |op(b)|``.  Results that hang on entries 2^-29 and more below the largest of their row of ``op(a)`` (column of ``op(b)``),
+    which the pairs hold in fewer than 22 bits, are computed from the matrices in fp32."""
     return _matmul(load().split16_matmul, a, b, trans_a, trans_b, alpha, upper_upper)
 
 

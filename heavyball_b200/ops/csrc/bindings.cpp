@@ -4,6 +4,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/extension.h>
 
+#include <ATen/MemoryOverlap.h>
+
 #include <algorithm>
 #include <optional>
 #include <string>
@@ -489,6 +491,11 @@ at::Tensor tf32_gemm(const at::Tensor& a2, const at::Tensor& b2, int64_t K, int 
   return s;
 }
 
+// The matrix x behind an operand whose rows are the rows (trans: the columns) of x.
+hb::Split16Source source_of(const at::Tensor& x, bool trans) {
+  return {x.data_ptr<float>(), x.stride(0), trans ? x.stride(2) : x.stride(1), trans ? x.stride(1) : x.stride(2)};
+}
+
 // Operands of the fp16-pair product of an fp32 [batch, R, C] tensor (see split16_gemm.h): (same, same_unit, trans, trans_unit); an
 // orientation that was not asked for comes back undefined.
 std::vector<at::Tensor> split16(const at::Tensor& x, bool want_same, bool want_trans) {
@@ -503,7 +510,7 @@ std::vector<at::Tensor> split16(const at::Tensor& x, bool want_same, bool want_t
     const int64_t rows = i == 0 ? R : C, K = i == 0 ? C : R;
     out[2 * i] = at::empty({batch, rows, 2 * hb::split16_kp(K)}, x.options().dtype(at::kHalf).memory_format(at::MemoryFormat::Contiguous));
     out[2 * i + 1] = at::empty({batch, hb::split16_units(rows)}, x.options().memory_format(at::MemoryFormat::Contiguous));
-    op[i] = {out[2 * i].data_ptr(), out[2 * i + 1].data_ptr<float>()};
+    op[i] = {out[2 * i].data_ptr(), out[2 * i + 1].data_ptr<float>(), source_of(x, i == 1)};
   }
   check(hb::launch_split16(x.data_ptr<float>(), x.stride(1), x.stride(0), (int)R, (int)C, (int)batch, op[0], op[1],
                            at::cuda::getCurrentCUDAStream()), "split16");
@@ -511,17 +518,28 @@ std::vector<at::Tensor> split16(const at::Tensor& x, bool want_same, bool want_t
 }
 
 // epilogue(A * B^T) over operands of split16; arguments as for tf32_gemm.  Both operands being one buffer makes the product symmetric.
-void split16_gemm(const at::Tensor& a, const at::Tensor& ua, const at::Tensor& b, const at::Tensor& ub, int64_t K, int mode, double alpha,
-                  double w, double b1, double b2c, double eps, const OptT& c, const OptT& m, const OptT& v, bool upper_upper,
-                  const at::Tensor& status) {
+// xa, xb: the tensors the operands were made from, with their columns (ta, tb) or rows as operand rows; neither may be written here.
+void split16_gemm(const at::Tensor& a, const at::Tensor& ua, const at::Tensor& xa, bool ta, const at::Tensor& b, const at::Tensor& ub,
+                  const at::Tensor& xb, bool tb, int64_t K, int mode, double alpha, double w, double b1, double b2c, double eps, const OptT& c,
+                  const OptT& m, const OptT& v, bool upper_upper, const at::Tensor& status) {
   TORCH_CHECK(a.is_cuda() && b.is_cuda() && a.scalar_type() == at::kHalf && b.scalar_type() == at::kHalf && a.dim() == 3 && b.dim() == 3 &&
                   a.is_contiguous() && b.is_contiguous() && a.size(0) == b.size(0) && K >= 1,
               "split16_gemm: contiguous fp16 operands [batch, rows, 2 kp]");
   const int64_t batch = a.size(0), M = a.size(1), N = b.size(1), kp = hb::split16_kp(K);
   TORCH_CHECK(a.size(2) == 2 * kp && b.size(2) == 2 * kp, "split16_gemm: operands were not split for K = ", std::to_string(K));
-  for (const auto& [u, rows] : {std::pair<const at::Tensor&, int64_t>(ua, M), std::pair<const at::Tensor&, int64_t>(ub, N)})
-    TORCH_CHECK(u.is_cuda() && u.scalar_type() == at::kFloat && u.is_contiguous() && u.numel() == batch * hb::split16_units(rows) &&
-                    u.device() == a.device(), "split16_gemm: units of another operand");
+  struct Side { const at::Tensor &u, &x; bool trans; int64_t rows; };
+  for (const Side& s : {Side{ua, xa, ta, M}, Side{ub, xb, tb, N}}) {
+    TORCH_CHECK(s.u.is_cuda() && s.u.scalar_type() == at::kFloat && s.u.is_contiguous() && s.u.numel() == batch * hb::split16_units(s.rows) &&
+                    s.u.device() == a.device(), "split16_gemm: units of another operand");
+    TORCH_CHECK(s.x.device() == a.device() && s.x.scalar_type() == at::kFloat && s.x.dim() == 3 && s.x.size(0) == batch && s.x.stride(2) == 1 &&
+                    s.x.size(s.trans ? 2 : 1) == s.rows && s.x.size(s.trans ? 1 : 2) == K, "split16_gemm: the source of another operand");
+    for (const OptT* out : {&c, &m, &v})
+      if (out->has_value() && (*out)->defined()) {
+        const at::MemOverlapStatus overlap = at::get_overlap_status(**out, s.x);
+        TORCH_CHECK(overlap != at::MemOverlapStatus::Full && overlap != at::MemOverlapStatus::Partial,
+                    "split16_gemm: an output lies over the matrix that an operand was made from");
+      }
+  }
   c10::cuda::CUDAGuard guard(a.device());
   hb::Tf32Epilogue E{};
   E.mode = mode; E.alpha = (float)alpha; E.w = (float)w; E.b1 = (float)b1; E.b2 = (float)b2c; E.eps = (float)eps;
@@ -542,8 +560,8 @@ void split16_gemm(const at::Tensor& a, const at::Tensor& ua, const at::Tensor& b
   TORCH_CHECK(!upper_upper || (M == N && M == K && a.data_ptr() != b.data_ptr()), "split16_gemm: upper_upper needs two square matrices of one size");
   E.tri = upper_upper ? 1 : 0;
   E.symmetric = (a.data_ptr() == b.data_ptr() && M == N && (mode == hb::kEpiStore || mode == hb::kEpiLerp || mode == hb::kEpiAdd)) ? 1 : 0;
-  check(hb::launch_split16_gemm({a.data_ptr(), ua.data_ptr<float>()}, {b.data_ptr(), ub.data_ptr<float>()}, (int)M, (int)N, (int)K, (int)batch,
-                                E, status.data_ptr<int>(), at::cuda::getCurrentCUDAStream()), "split16 gemm");
+  check(hb::launch_split16_gemm({a.data_ptr(), ua.data_ptr<float>(), source_of(xa, ta)}, {b.data_ptr(), ub.data_ptr<float>(), source_of(xb, tb)},
+                                (int)M, (int)N, (int)K, (int)batch, E, status.data_ptr<int>(), at::cuda::getCurrentCUDAStream()), "split16 gemm");
 }
 
 // op(a) @ op(b) for batched fp32 matrices from fp16 pairs; arguments and result as for tf32x3_matmul.
@@ -561,7 +579,7 @@ at::Tensor split16_matmul(const at::Tensor& a, const at::Tensor& b, bool ta, boo
   const int64_t ldc = (N + 3) / 4 * 4;
   at::Tensor c = at::empty({batch, M, ldc}, a.options().memory_format(at::MemoryFormat::Contiguous));
   const at::Tensor view = ldc == N ? c : c.narrow(2, 0, N);
-  split16_gemm(sa[ia], sa[ia + 1], sb[ib], sb[ib + 1], K, hb::kEpiStore, alpha, 0, 0, 0, 0, view, {}, {}, upper_upper, status);
+  split16_gemm(sa[ia], sa[ia + 1], a, ta, sb[ib], sb[ib + 1], b, !tb, K, hb::kEpiStore, alpha, 0, 0, 0, 0, view, {}, {}, upper_upper, status);
   return view;
 }
 

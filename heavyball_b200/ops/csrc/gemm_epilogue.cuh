@@ -30,30 +30,146 @@ __device__ __forceinline__ float tf32_hi(float x) {
 
 __device__ __forceinline__ float lerp_w(float s, float x, float w) { return s * (1.0f - w) + x * w; }
 
-// Accumulators of 32 columns of one row, times the units of the row and of each column.  The smaller factor goes first: their product
-// alone may leave the range of fp32 where the result does not.
-__device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_factor, const float* col_unit) {
-#pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const float4 c = *(const float4*)(col_unit + q * 4);
-    const float f[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-      acc[q * 4 + e] = __float_as_uint(__uint_as_float(acc[q * 4 + e]) * fminf(row_factor, f[e]) * fmaxf(row_factor, f[e]));
-  }
-}
-
 constexpr int kStageLd = 36;                         // floats per staged row: rows stay 16-byte aligned and float4
                                                      // accesses of a quarter-warp fall into distinct banks
 constexpr int kStageWarpBytes = 32 * kStageLd * 4;   // one warp's 32 rows x 32 columns
 
+// What the epilogue knows of an operand of scaled fp16 pairs (split16_gemm.h): what one unit of each of its rows stands for with the number of
+// values that the row's pairs hold in fewer bits than split tf32 would, and the matrix that it was made from: element (row, k) of batch
+// entry b is src[b * src_batch + row * src_row + k * src_k].
+struct PairOperand {
+  const float* unit;
+  int64_t unit_batch;
+  const float* src;
+  int64_t src_batch, src_row, src_k;
+};
+struct PairOperands {
+  PairOperand a, b;
+  int K;
+};
+
+// 32 rows x 32 of K of an operand's matrix (zeros outside it), fetched in the order in which they lie in memory and put down as rows
+__device__ __forceinline__ void fetch_source(float (&v)[32], int lane, const PairOperand& op, int batch, int row0, int rows, int k0, int K) {
+  const float* p = op.src + batch * op.src_batch + row0 * op.src_row + k0 * op.src_k;
+  const bool along_k = op.src_k == 1;
+  const int64_t step = along_k ? op.src_row : op.src_k;
+  const int mine = along_k ? K - k0 : rows - row0, others = along_k ? rows - row0 : K - k0;
+#pragma unroll
+  for (int i = 0; i < 32; ++i) v[i] = (lane < mine && i < others) ? p[(along_k ? lane : lane * op.src_row) + i * step] : 0.0f;
+}
+__device__ __forceinline__ void stage_source(float* stage, const float (&v)[32], int lane, const PairOperand& op) {
+  if (op.src_k == 1) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) stage[i * kStageLd + lane] = v[i];
+  } else {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) stage[lane * kStageLd + i] = v[i];
+  }
+}
+
+__device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
+
+// A row's unit carries the number of its values below 2^-14 units in the mantissa.
+__device__ __forceinline__ float unit_of(float u) { return __uint_as_float(__float_as_uint(u) & 0x7F800000u); }
+__device__ __forceinline__ uint32_t short_values(float u, bool inside) { return inside ? __float_as_uint(u) & 0x7FFFFFu : 0u; }
+
+constexpr uint32_t kManyShort = 1u << 19;  // counts of short values from here on stand for "any number"
+
+// Entries of the product for blocks with values short of bits or with units whose product may leave the range of fp32, times alpha, into
+// `stage` (row = lane).  `tmem`: the block's accumulators.
+// A value below 2^-14 in units of its row is held with an error of up to 2^-36 of a unit instead of 22 bits of itself.  With the other
+// operand's values (2^15 at most) and the product of low parts that is left out, n of them bring an error of at most n 2^-20: where the
+// accumulator is 4 n or more, less than 2^-22 of the result.  Smaller accumulators of such rows and columns may consist of nothing else:
+// the block is computed from the matrices themselves, in fp32 arithmetic (subnormals kept), sums of 32 at a time, the next 32 of K on their
+// way meanwhile.  (One such value among ordinary ones, as in one of a hundred thousand rows of 1024 normally distributed values, does not
+// lead there: sums over ordinary values are around 2^25 and more.)
+// `tri`: entries below the diagonal are zeros whatever the values.
+__device__ __noinline__ void settle_slowly(uint32_t tmem, int lane, float* stage, const PairOperands& P, int batch, int row0, int col0, int M, int N,
+                                           int tri, float alpha) {
+  const float row = P.a.unit[batch * P.a.unit_batch + row0 + lane], col = P.b.unit[batch * P.b.unit_batch + col0 + lane];
+  float* const mine = stage + lane * kStageLd;
+  uint32_t acc[32];
+  tmem_ld32(tmem, acc);
+  tmem_ld_wait();
+  const uint32_t n_row = short_values(row, row0 + lane < M), n_col = short_values(col, col0 + lane < N);
+  const float by_row = 4.0f * (n_row >= kManyShort ? (float)P.K : (float)n_row), by_col = 4.0f * (n_col >= kManyShort ? (float)P.K : (float)n_col);
+  bool small = false;
+#pragma unroll
+  for (int j = 0; j < 32; ++j) {
+    const float least = by_row + __shfl_sync(0xFFFFFFFFu, by_col, j);
+    small |= row0 + lane < M && col0 + j < N && !(tri && row0 + lane > col0 + j) && fabsf(__uint_as_float(acc[j])) < least;
+  }
+  if (!__any_sync(0xFFFFFFFFu, small)) {  // units in two steps of half the exponent each: neither leaves the range unless the result does
+    const int e_row = (int)(__float_as_uint(unit_of(row)) >> 23) - 127, e_mine = (int)(__float_as_uint(unit_of(col)) >> 23) - 127;
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+      const int e = max(-252, min(252, e_row + __shfl_sync(0xFFFFFFFFu, e_mine, j))), half = e >> 1;  // (padding holds anything)
+      mine[j] = __uint_as_float(acc[j]) * pow2(half) * pow2(e - half) * alpha;
+    }
+    return;
+  }
+  float out[32], a[32], next_a[32], next_b[32];
+  for (int j = 0; j < 32; ++j) out[j] = 0.0f;
+  fetch_source(next_a, lane, P.a, batch, row0, M, 0, P.K);
+  fetch_source(next_b, lane, P.b, batch, col0, N, 0, P.K);
+#pragma unroll 1
+  for (int k0 = 0; k0 < P.K; k0 += 32) {
+    __syncwarp();
+    stage_source(stage, next_a, lane, P.a);
+    __syncwarp();
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const float4 t = *(const float4*)(stage + lane * kStageLd + q * 4);
+      a[q * 4] = t.x; a[q * 4 + 1] = t.y; a[q * 4 + 2] = t.z; a[q * 4 + 3] = t.w;
+    }
+    __syncwarp();
+    stage_source(stage, next_b, lane, P.b);
+    __syncwarp();
+    if (k0 + 32 < P.K) {
+      fetch_source(next_a, lane, P.a, batch, row0, M, k0 + 32, P.K);
+      fetch_source(next_b, lane, P.b, batch, col0, N, k0 + 32, P.K);
+    }
+#pragma unroll 4
+    for (int j = 0; j < 32; ++j) {
+      float sum = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const float4 t = *(const float4*)(stage + j * kStageLd + q * 4);
+        const float b[4] = {t.x, t.y, t.z, t.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum) : "f"(a[q * 4 + e]), "f"(b[e]));
+      }
+      float total = out[j];
+      asm("add.rn.f32 %0, %0, %1;" : "+f"(total) : "f"(sum));
+      out[j] = total;
+    }
+  }
+  __syncwarp();
+  for (int j = 0; j < 32; ++j) mine[j] = out[j] * alpha;
+}
+
+// Whether the units of this lane's row and column allow the usual way: no values short of bits, far from the ends of the range.
+__device__ __forceinline__ bool ordinary_unit(float u, bool inside) { return !inside || (short_values(u, true) == 0 && u > 0x1p-63f && u < 0x1p63f); }
+
+// Accumulators of an ordinary 32 x 32 block (lane = row, `row_unit`) -> entries of the product.
+__device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_unit, const float* col_units) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float4 c = *(const float4*)(col_units + q * 4);
+    const float f[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) acc[q * 4 + e] = __float_as_uint(__uint_as_float(acc[q * 4 + e]) * (row_unit * f[e]));
+  }
+}
+
 // The usual case of the epilogue below: a 32 x 32 block inside the output, C aligned, no split output.  With the mode known at compile
 // time, no bounds to check and all reads in flight before the first use a tile's epilogue is a third as long (8 of 128^3, whole
 // launch: added to C 15.8 -> 9.3 us, symmetric 13.1 -> 7.8, Adam 21.1 -> 12.6, stored in bulk 7.2).
-// `c`, `cm`, `m`, `v`: the block's first element in the output, in its mirror image (null: not stored) and in the moments.
+// `c`, `cm`, `m`, `v`: the block's first element in the output, in its mirror image (null: not stored) and in the moments.  `staged`: the
+// product's entries are in the stage already.
 template <bool kScaled, int kMode>
 __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* stage, const Tf32Epilogue& E, float* c, float* cm, float* m,
-                                               float* v, int64_t ld_state, float row_factor, const float* col_unit) {
+                                               float* v, int64_t ld_state, bool staged, float row_unit, const float* col_units) {
   constexpr bool kOld = kMode == kEpiLerp || kMode == kEpiAdd, kMoments = kMode == kEpiAdam || kMode == kEpiLaProp;
   const int sub = lane >> 3, cg = (lane & 7) * 4;
   float* const mine = stage + lane * kStageLd;
@@ -74,11 +190,11 @@ __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* s
       pb[i] = *(const float4*)(v + i * sstep);
     }
   }
-  {
+  if (!kScaled || !staged) {
     uint32_t acc[32];
     tmem_ld32(tmem, acc);
     tmem_ld_wait();
-    if constexpr (kScaled) unscale32(acc, row_factor, col_unit);
+    if constexpr (kScaled) unscale32(acc, row_unit, col_units);
 #pragma unroll
     for (int q = 0; q < 8; ++q)
       *(float4*)(mine + q * 4) =
@@ -140,43 +256,51 @@ __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* s
 // `tmem_warp`: tensor-memory address of the warp's first row and the tile's first column; `row0` / `col_base`: their
 // global indices; `n_cb`: 32-column blocks in the tile; `off_diagonal`: the tile is not on the diagonal (mirror stores).
 // `zero_acc`: the tile had no product (its accumulator was never written): the values are zeros.
-// `kScaled`: the operands were scaled by powers of two per row; `row_unit` / `col_unit` are what one unit of an accumulator row /
-// column stands for (arrays of this batch entry, padded to whole tiles).
+// `kScaled`: the operands are fp16 pairs, described by `P`; their products have no split outputs.
 template <bool kScaled>
 __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, float* stage, int row0, int col_base, int n_cb,
                                                 bool off_diagonal, bool zero_acc, int batch, int M, int N,
-                                                const Tf32Epilogue& E, const float* row_unit = nullptr, const float* col_unit = nullptr) {
+                                                const Tf32Epilogue& E, const PairOperands& P) {
   const int64_t b64 = batch;
   const bool state_vec = (N & 3) == 0;
   const bool c_vec = (E.ldc & 3) == 0 && ((E.strideC & 3) == 0) && ((((uintptr_t)E.C) & 15) == 0);
   const bool moments = E.mode == kEpiAdam || E.mode == kEpiLaProp;
   const bool mirror = E.symmetric && off_diagonal && E.C != nullptr;
-  const bool along_rows = mirror || (E.S != nullptr && E.s_transposed);
-  const bool s_rows = E.S != nullptr && !E.s_transposed;
+  const bool s_cols = !kScaled && E.S != nullptr && E.s_transposed, s_rows = !kScaled && E.S != nullptr && !E.s_transposed;
+  const bool along_rows = mirror || s_cols;
   const int sub = lane >> 3, cg = (lane & 7) * 4;
   const float w1 = 1.0f - E.b1, w2 = 1.0f - E.b2;
   float* mine = stage + lane * kStageLd;
-  float row_factor = 1.0f;
-  if constexpr (kScaled) row_factor = row_unit[row0 + lane];
+  const float* const col_units = kScaled ? P.b.unit + b64 * P.b.unit_batch + col_base : nullptr;
+  float row_unit = 1.0f, col_unit = 1.0f;
+  if constexpr (kScaled) {
+    row_unit = P.a.unit[b64 * P.a.unit_batch + row0 + lane];
+    col_unit = col_units[lane];
+  }
 #pragma unroll 1
   for (int cb = 0; cb < n_cb; ++cb) {
     const int col0 = col_base + cb * 32;
-    if (!zero_acc && E.S == nullptr && c_vec && E.C != nullptr && row0 + 32 <= M && col0 + 32 <= N && (!moments || state_vec)) {
+    bool staged = false;
+    if constexpr (kScaled) {
+      staged = !zero_acc && !__all_sync(0xFFFFFFFFu, ordinary_unit(row_unit, row0 + lane < M) && ordinary_unit(col_unit, col0 + lane < N));
+      if (staged) settle_slowly(tmem_warp + (uint32_t)(cb * 32), lane, stage, P, batch, row0, col0, M, N, E.tri, E.alpha);
+      if (cb + 1 < n_cb) col_unit = col_units[(cb + 1) * 32 + lane];
+    }
+    if (!zero_acc && !s_rows && !s_cols && c_vec && E.C != nullptr && row0 + 32 <= M && col0 + 32 <= N && (!moments || state_vec)) {
       const uint32_t t = tmem_warp + (uint32_t)(cb * 32);
       float* c = E.C + b64 * E.strideC + (int64_t)row0 * E.ldc + col0;
       float* cm = mirror ? E.C + b64 * E.strideC + (int64_t)col0 * E.ldc + row0 : nullptr;
       const int64_t st = (b64 * M + row0) * (int64_t)N + col0;
-      const float* cu = kScaled ? col_unit + col0 : nullptr;
       switch (E.mode) {
-        case kEpiStore: epilogue_block<kScaled, kEpiStore>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, row_factor, cu); break;
-        case kEpiLerp: epilogue_block<kScaled, kEpiLerp>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, row_factor, cu); break;
-        case kEpiAdd: epilogue_block<kScaled, kEpiAdd>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, row_factor, cu); break;
-        case kEpiAdam: epilogue_block<kScaled, kEpiAdam>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, row_factor, cu); break;
-        default: epilogue_block<kScaled, kEpiLaProp>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, row_factor, cu); break;
+        case kEpiStore: epilogue_block<kScaled, kEpiStore>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, row_unit, col_units + cb * 32); break;
+        case kEpiLerp: epilogue_block<kScaled, kEpiLerp>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, row_unit, col_units + cb * 32); break;
+        case kEpiAdd: epilogue_block<kScaled, kEpiAdd>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, row_unit, col_units + cb * 32); break;
+        case kEpiAdam: epilogue_block<kScaled, kEpiAdam>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, row_unit, col_units + cb * 32); break;
+        default: epilogue_block<kScaled, kEpiLaProp>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, row_unit, col_units + cb * 32); break;
       }
       continue;
     }
-    {
+    if (!kScaled || !staged) {
       uint32_t acc[32];
       if (!zero_acc) {
         tmem_ld32(tmem_warp + (uint32_t)(cb * 32), acc);
@@ -185,7 +309,8 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
 #pragma unroll
         for (int j = 0; j < 32; ++j) acc[j] = 0u;
       }
-      if constexpr (kScaled) unscale32(acc, row_factor, col_unit + col0);
+      if constexpr (kScaled)
+        if (!zero_acc) unscale32(acc, row_unit, col_units + cb * 32);
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *(float4*)(mine + q * 4) =
@@ -321,7 +446,7 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
         for (int j = 0; j < 32; ++j)
           if (col0 + j < N) ccol[(int64_t)(col0 + j) * E.ldc] = v[j];
       }
-      if (E.S != nullptr && E.s_transposed && row < E.kpS) {
+      if (s_cols && row < E.kpS) {
         // operand rows = output columns, K over the output rows (zero from M up to kp)
         float* sb = E.S + b64 * E.strideS + row;
         const int64_t ld = 2 * E.kpS;
@@ -348,8 +473,8 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
 template <class Kind>
 __global__ void __launch_bounds__(kTThreads, 2)
 gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_c, int M, int N, int kp, const Tf32Epilogue E, const float* row_units, int64_t stride_ru,
-               const float* col_units, int64_t stride_cu, int bulk_store, int* status) {
+               const __grid_constant__ CUtensorMap map_c, int M, int N, int kp, const Tf32Epilogue E, const __grid_constant__ PairOperands P,
+               int bulk_store, int* status) {
   constexpr int TBK = Kind::kBlock;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kTStages];
@@ -434,8 +559,6 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   } else {
     const int quarter = warp & 3, r = quarter * 32 + lane;
     const bool have = (num_kb == 0) || mbar_wait(&accum_bar, 0, &abort_flag);
-    const float* row_unit = Kind::kScaled ? row_units + batch * stride_ru : nullptr;
-    const float* col_unit = Kind::kScaled ? col_units + batch * stride_cu : nullptr;
     tc_fence_after();
     if (have && bulk_store) {
       // every load has landed and every MMA has retired: the ring is free and stages the output tile as four
@@ -443,9 +566,26 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
 #pragma unroll 1
       for (int cb = 0; cb < TBN / 32; ++cb) {
         uint32_t acc[32];
-        tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32), acc);
-        tmem_ld_wait();
-        if constexpr (Kind::kScaled) unscale32(acc, row_unit[tm * TBM + r], col_unit + tn * TBN + cb * 32);
+        const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32);
+        if constexpr (Kind::kScaled) {
+          const int row = tm * TBM + quarter * 32 + lane, col0 = tn * TBN + cb * 32;
+          const float* const col_units = P.b.unit + batch * P.b.unit_batch + col0;
+          const float row_unit = P.a.unit[batch * P.a.unit_batch + row];
+          if (__all_sync(0xFFFFFFFFu, ordinary_unit(row_unit, row < M) && ordinary_unit(col_units[lane], col0 + lane < N))) {
+            tmem_ld32(t, acc);
+            tmem_ld_wait();
+            unscale32(acc, row_unit, col_units);
+          } else {
+            float* const stage = (float*)(tiles + (TBN / 32) * kTTileBytes + quarter * kStageWarpBytes);  // behind the boxes
+            settle_slowly(t, lane, stage, P, batch, row - lane, col0, M, N, 0, 1.0f);
+#pragma unroll
+            for (int j = 0; j < 32; ++j) acc[j] = __float_as_uint(stage[lane * kStageLd + j]);
+            __syncwarp();
+          }
+        } else {
+          tmem_ld32(t, acc);
+          tmem_ld_wait();
+        }
         uint8_t* box = tiles + cb * kTTileBytes;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
@@ -455,8 +595,7 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     } else if (have) {
       epilogue_direct<Kind::kScaled>(tmem_base + ((uint32_t)(quarter * 32) << 16), lane, (float*)(tiles + quarter * kStageWarpBytes),
-                      tm * TBM + quarter * 32, tn * TBN, TBN / 32, tm != tn, num_kb == 0, batch, M, N, E,
-                      row_unit, col_unit);
+                      tm * TBM + quarter * 32, tn * TBN, TBN / 32, tm != tn, num_kb == 0, batch, M, N, E, P);
     }
     tc_fence_before();
     if (bulk_store) {
@@ -494,6 +633,10 @@ constexpr int kGPairEpiWarps = 8;
 constexpr int kGPairThreads = 64 + 32 * kGPairEpiWarps;
 constexpr int kGPairSmemBytes = kGPairStages * kGPairStageBytes + kGPairEpiWarps * kStageWarpBytes + 1024;
 
+// Epilogues of scaled operands may compute blocks from the matrices (16 ms for a tile's column of 2^17 of K), and everything in the pair waits for
+// them.
+constexpr uint32_t kLongSpinLimit = kSpinLimit << 5;
+
 struct WalkTile {
   int kb_lo, seg;  // K blocks of one term that the tile walks: [kb_lo, kb_lo + seg)
 };
@@ -509,8 +652,7 @@ __device__ __forceinline__ WalkTile walk_tile(const PairTile& t, int kp, int tri
 template <class Kind>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N, int kp, int tiles_m,
-                    int tiles_n, int per_batch, int total, const Tf32Epilogue E, const float* row_units, int64_t stride_ru,
-                    const float* col_units, int64_t stride_cu, int* status) {
+                    int tiles_n, int per_batch, int total, const Tf32Epilogue E, const __grid_constant__ PairOperands P, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kGPairStages];   // used in the even CTA: both CTAs' loads of a stage have landed
   __shared__ __align__(8) uint64_t empty_bar[kGPairStages];  // in each CTA: the products that read the stage have finished
@@ -559,7 +701,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
           const int ka = (term == Kind::kTermLoA ? kp : 0), kb_off = (term == Kind::kTermLoB ? kp : 0);
           for (int kb = 0; kb < h.seg; ++kb, ++n) {
             const int s = n % kGPairStages, round = n / kGPairStages, k0 = (h.kb_lo + kb) * Kind::kBlock;
-            ok = mbar_wait(&empty_bar[s], (round & 1) ^ 1, &abort_flag);
+            ok = mbar_wait<Kind::kScaled ? kLongSpinLimit : kSpinLimit>(&empty_bar[s], (round & 1) ^ 1, &abort_flag);
             if (!ok) break;
             uint8_t* dst = ring + s * kGPairStageBytes;
             const uint32_t bar = cluster_addr(&full_bar[s], 0);
@@ -579,13 +721,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       for (int idx = pair; idx < total && ok; idx += pairs, ++it) {
         const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
         const int seg = walk_tile(t, kp, E.tri, Kind::kBlock).seg, num_kb = 3 * seg, acc = it & 1;
-        ok = mbar_wait(&acc_empty[acc], ((it >> 1) & 1) ^ 1, &abort_flag);
+        ok = mbar_wait<Kind::kScaled ? kLongSpinLimit : kSpinLimit>(&acc_empty[acc], ((it >> 1) & 1) ^ 1, &abort_flag);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d = tmem_base + (uint32_t)acc * 256u;
         for (int kb = 0; kb < num_kb; ++kb, ++n) {
           const int s = n % kGPairStages, round = n / kGPairStages;
-          ok = mbar_wait(&full_bar[s], round & 1, &abort_flag);
+          ok = mbar_wait<Kind::kScaled ? kLongSpinLimit : kSpinLimit>(&full_bar[s], round & 1, &abort_flag);
           if (!ok) break;
           tc_fence_after();
           const uint32_t base = smem_u32(ring + s * kGPairStageBytes);
@@ -609,7 +751,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     for (int idx = pair; idx < total; idx += pairs, ++it) {
       const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
       const int acc = it & 1, row0 = t.tm * kPairTile + (int)rank * 128 + quarter * 32, col0 = t.tn * kPairTile + half * 128;
-      const bool ok = mbar_wait(&acc_full[acc], (it >> 1) & 1, &abort_flag);
+      const bool ok = mbar_wait<Kind::kScaled ? kLongSpinLimit : kSpinLimit>(&acc_full[acc], (it >> 1) & 1, &abort_flag);
       if (!__all_sync(0xFFFFFFFFu, ok)) break;
       tc_fence_after();
       const int blocks = min(4, (N - col0 + 31) / 32);
@@ -618,8 +760,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       const bool mirrored = thirds ? rank == 0 && half == 1 : t.tm != t.tn;
       if (row0 < M && blocks > 0 && !(thirds && rank == 1 && half == 0))
         epilogue_direct<Kind::kScaled>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, mirrored,
-                              walk_tile(t, kp, E.tri, Kind::kBlock).seg == 0, t.batch, M, N, E, Kind::kScaled ? row_units + t.batch * stride_ru : nullptr,
-                              Kind::kScaled ? col_units + t.batch * stride_cu : nullptr);
+                              walk_tile(t, kp, E.tri, Kind::kBlock).seg == 0, t.batch, M, N, E, P);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) cluster_arrive(cluster_addr(&acc_empty[acc], 0));

@@ -60,11 +60,19 @@ struct RowScale {
 // `bits`: largest absolute value of the row, as its bits (NaN above infinity above everything finite)
 __device__ __forceinline__ RowScale row_scale(uint32_t bits) {
   const int field = (int)(bits >> 23);
-  // zero and subnormal rows, and rows with an infinity or NaN (all of whose results are NaN: lo = inf - inf), stay as they are
-  const int e = (field == 0 || field == 255) ? 0 : min(126, 141 - field);
-  return {__uint_as_float((uint32_t)(127 + e) << 23), __uint_as_float((uint32_t)(127 - e) << 23)};
+  // rows with an infinity or NaN stay as they are: all of their results are NaN (lo = inf - inf)
+  const int e = field == 255 ? 0 : min(126, 141 - field);
+  return {pow2(e), pow2(-e)};
 }
 __device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
+// x, scaled: too small for 22 bits in a pair
+__device__ __forceinline__ bool is_short(float x, float y) { return x != 0.0f && fabsf(y) < 0x1p-14f; }
+// without flushing subnormals
+__device__ __forceinline__ float scaled(float x, float mul) {
+  float y;
+  asm("mul.rn.f32 %0, %1, %2;" : "=f"(y) : "f"(x), "f"(mul));
+  return y;
+}
 __device__ __forceinline__ void split_pair(float x, uint16_t& hi, uint16_t& lo) {
   const __half h = __float2half_rn(x);
   hi = __half_as_ushort(h);
@@ -105,7 +113,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
     const int kp = (C + 63) / 64 * 64;
     const float* row = s + (int64_t)r * ld_src;
     float4 v[kRowChunk / 128];
-    uint32_t top = 0;
+    uint32_t top = 0, n_short = 0;
     const auto fetch = [&](int base) {
 #pragma unroll
       for (int i = 0; i < kRowChunk / 128; ++i) {
@@ -120,7 +128,6 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
       for (int i = 0; i < kRowChunk / 128; ++i) top = max(top, abs_max4(v[i]));
     }
     const RowScale f = row_scale(__reduce_max_sync(0xFFFFFFFFu, top));
-    if (lane == 0) same_unit[batch * ((R + 255) / 256 * 256) + r] = f.unit;
     uint16_t* dst = same + (batch * R + r) * 2 * kp;
     for (int base = 0; base < C; base += kRowChunk) {
       if (C > kRowChunk) fetch(base);
@@ -128,17 +135,21 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
       for (int i = 0; i < kRowChunk / 128; ++i) {
         const int c = base + i * 128 + lane * 4;
         if (c < kp) {
-          const float x[4] = {v[i].x * f.mul, v[i].y * f.mul, v[i].z * f.mul, v[i].w * f.mul};
+          const float x[4] = {scaled(v[i].x, f.mul), scaled(v[i].y, f.mul), scaled(v[i].z, f.mul), scaled(v[i].w, f.mul)};
+          n_short += is_short(v[i].x, x[0]) + is_short(v[i].y, x[1]) + is_short(v[i].z, x[2]) + is_short(v[i].w, x[3]);
           split_store4(dst + c, kp, x);
         }
       }
     }
+    n_short = min(__reduce_add_sync(0xFFFFFFFFu, n_short), kManyShort);
+    if (lane == 0) same_unit[batch * ((R + 255) / 256 * 256) + r] = __uint_as_float(__float_as_uint(f.unit) | n_short);
     return;
   }
 
   __shared__ __align__(16) float tile[kStrip * kStripRows];
   __shared__ uint32_t warp_tops[kSplitThreads / 32][kStrip];
   __shared__ uint32_t tops[kStrip];  // of this block's rows; the blocks of the cluster read each other's
+  __shared__ uint32_t shorts[kStrip];
   __shared__ float muls[kStrip];
   const int at = blockIdx.x - row_blocks, rank = at % cluster, c0 = at / cluster * kStrip;
   const int q = threadIdx.x & 7, line = threadIdx.x >> 3, c = c0 + q * 4, kp = (R + 63) / 64 * 64;
@@ -175,6 +186,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
 #pragma unroll
     for (int w = 0; w < kSplitThreads / 32; ++w) t = max(t, warp_tops[w][threadIdx.x]);
     tops[threadIdx.x] = t;
+    shorts[threadIdx.x] = 0;
   }
   if (cluster > 1) cluster_sync(); else __syncthreads();
   if (threadIdx.x < kStrip) {
@@ -189,14 +201,20 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
   const int oc = threadIdx.x >> 4, k4 = (threadIdx.x & 15) * 4;  // output: rows c0 + oc (+ 16) of the operand, four of K at a time
   for (int r0 = first; r0 < R; r0 += step) {
     if (R > step) fetch(r0);
+    uint32_t n_short = 0;  // a byte per column: a thread has eight rows
 #pragma unroll
     for (int i = 0; i < kStripRows / 32; ++i) {
       const int r = line + 32 * i;
-      tile[turned(q * 4 + 0, r)] = v[i].x * muls[q * 4 + 0];
-      tile[turned(q * 4 + 1, r)] = v[i].y * muls[q * 4 + 1];
-      tile[turned(q * 4 + 2, r)] = v[i].z * muls[q * 4 + 2];
-      tile[turned(q * 4 + 3, r)] = v[i].w * muls[q * 4 + 3];
+      const float x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float y = scaled(x[e], muls[q * 4 + e]);
+        tile[turned(q * 4 + e, r)] = y;
+        n_short += (uint32_t)is_short(x[e], y) << (8 * e);
+      }
     }
+    if (n_short != 0)
+      for (int e = 0; e < 4; ++e) atomicAdd(&shorts[q * 4 + e], n_short >> (8 * e) & 255u);
     __syncthreads();
 #pragma unroll
     for (int g = 0; g < kStrip; g += 16) {
@@ -213,6 +231,9 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
     }
     __syncthreads();
   }
+  // (rank 0's unit is there: the cluster has met since)
+  if (threadIdx.x < kStrip && c0 + (int)threadIdx.x < C && shorts[threadIdx.x] != 0)
+    atomicAdd((uint32_t*)&trans_unit[batch * ((C + 255) / 256 * 256) + c0 + threadIdx.x], min(shorts[threadIdx.x], kManyShort));
 }
 
 // fp16 operand [batch, rows, cols]; box = 64 columns x 128 rows, 128-byte swizzle
@@ -298,11 +319,15 @@ cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N
   if (e != cudaSuccess) return e;
   if (M == 0 || N == 0 || batch == 0) return cudaSuccess;
   const bool moments = E.mode == kEpiAdam || E.mode == kEpiLaProp;
-  if (K == 0 || E.S != nullptr || (moments && (E.m == nullptr || E.v == nullptr))) return cudaErrorInvalidValue;
+  if (K == 0 || A.src.p == nullptr || B.src.p == nullptr || E.S != nullptr || (moments && (E.m == nullptr || E.v == nullptr))) return cudaErrorInvalidValue;
   if (!moments && E.C == nullptr) return cudaErrorInvalidValue;
   if (E.tri && (M != N || M != K || E.symmetric)) return cudaErrorInvalidValue;
   if (E.symmetric && (A.data != B.data || M != N || E.C == nullptr || moments)) return cudaErrorInvalidValue;
-  const int64_t kp = split16_kp(K), stride_ru = split16_units(M), stride_cu = split16_units(N);
+  const int64_t kp = split16_kp(K);
+  const auto pair_operand = [](const Split16Operand& o, int64_t rows) {
+    return PairOperand{o.unit, split16_units(rows), o.src.p, o.src.batch, o.src.row, o.src.k};
+  };
+  const PairOperands P{pair_operand(A, M), pair_operand(B, N), K};
   CUtensorMap ma, mb;
   if (!make_half_map(&ma, A.data, M, 2 * kp, batch) || !make_half_map(&mb, B.data, N, 2 * kp, batch)) return cudaErrorInvalidValue;
   const auto tiles = [&](int tile) {
@@ -317,15 +342,15 @@ cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N
     const int tm = (M + kPairTile - 1) / kPairTile, tn = (N + kPairTile - 1) / kPairTile;
     const int grid = 2 * (int)(big < max_pairs ? big : max_pairs);
     return launch_chained(gemm_pair_kernel<HalfKind>, dim3(grid), kGPairThreads, kGPairSmemBytes, stream, ma, mb, M, N, (int)kp, tm, tn,
-                          tiles(kPairTile), (int)big, E, A.unit, stride_ru, B.unit, stride_cu, status);
+                          tiles(kPairTile), (int)big, E, P, status);
   }
   // bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing past it
   const int bulk = (!E.symmetric && !E.tri && E.mode == kEpiStore && (N & 3) == 0 && (E.ldc & 3) == 0 && (E.strideC & 3) == 0 &&
                     (((uintptr_t)E.C) & 15) == 0) ? 1 : 0;
   CUtensorMap mc = ma;  // placeholder when the bulk-store path is not taken (never dereferenced then)
   if (bulk && !make_store_map(&mc, E.C, M, N, E.ldc, E.strideC, batch)) return cudaErrorInvalidValue;
-  return launch_chained(gemm128_kernel<HalfKind>, dim3(tiles(TBM), batch), kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, A.unit,
-                        stride_ru, B.unit, stride_cu, bulk, status);
+  return launch_chained(gemm128_kernel<HalfKind>, dim3(tiles(TBM), batch), kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, P, bulk,
+                        status);
 }
 
 }  // namespace hb

@@ -40,8 +40,9 @@ __device__ inline bool elect_one() {
   return p != 0;
 }
 // Returns false if the wait expired or another role already aborted.
+template <uint32_t kLimit = kSpinLimit>
 __device__ inline bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
-  for (uint32_t spin = 0; spin < kSpinLimit; ++spin) {
+  for (uint32_t spin = 0; spin < kLimit; ++spin) {
     if (mbar_try_wait(bar, parity)) return true;
     if (*abort_flag) return false;
   }

@@ -180,7 +180,7 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
     Tf32Epilogue E2 = E;
     if (tiles == kPairTilesSmallDiagonal) E2.symmetric = 2;
     return launch_chained(gemm_pair_kernel<Tf32Kind>, dim3(2 * (int)(total < max_pairs ? total : max_pairs)), kGPairThreads, kGPairSmemBytes, stream,
-                          ma, mb, M, N, (int)kp, big_m, big_n, per_batch, (int)total, E2, nullptr, 0, nullptr, 0, status);
+                          ma, mb, M, N, (int)kp, big_m, big_n, per_batch, (int)total, E2, PairOperands{}, status);
   }
 
   // plain products leave through the bulk-store path (bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing
@@ -191,7 +191,7 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   if (bulk && !make_f32_map(&mc, E.C, M, N, E.ldc, E.strideC, batch)) return cudaErrorInvalidValue;
   const int tiles_m = (M + TBM - 1) / TBM, tiles_n = (N + TBN - 1) / TBN;
   dim3 grid(E.symmetric ? tiles_n * (tiles_n + 1) / 2 : tiles_m * tiles_n, batch);
-  return launch_chained(gemm128_kernel<Tf32Kind>, grid, kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, nullptr, 0, nullptr, 0, bulk, status);
+  return launch_chained(gemm128_kernel<Tf32Kind>, grid, kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, PairOperands{}, bulk, status);
 }
 
 }  // namespace hb

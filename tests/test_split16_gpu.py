@@ -20,11 +20,12 @@ def _rand(*shape, seed):
     return torch.randn(*shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(seed))
 
 
-def _off(got, a, b, want=None):
+def _off(got, a, b, want=None, floor=0.0):
     """Largest error in units of its bound: 22 bits of either operand and the dropped product of low parts (4 units of 2^-22), and one
-    rounding of the accumulator per 16 of K in the last of three walks plus a few for the first two (2^-23 of |a| |b| each)."""
+    rounding of the accumulator per 16 of K in the last of three walks plus a few for the first two (2^-23 of |a| |b| each).  Blocks that
+    are computed in fp32 stay under it, too: sums of 32 products at a time round 32 + K / 32 times by 2^-24."""
     K = a.shape[-1]
-    bound = (a.abs() @ b.abs().mT) * (2.0**-20 + (K / 16 + 4) * 2.0**-23)
+    bound = (a.abs() @ b.abs().mT) * (2.0**-20 + (K / 16 + 4) * 2.0**-23) + floor
     return float(((got.double() - (a @ b.mT if want is None else want)).abs() / bound.clamp_min(1e-300)).max())
 
 
@@ -115,7 +116,8 @@ def test_ranges_that_fp16_does_not_have(tile):
     a, b = _rand(1, 300, 96, seed=12), _rand(1, 140, 96, seed=13)
     a, b = a * torch.logspace(-30, 30, 300, device="cuda")[:, None], b * torch.logspace(6, -6, 140, device="cuda")[:, None]
     a[0, 7], a[0, 8], b[0, 3] = 0.0, 1e-41, 0.0
-    assert _off(ops.matmul16(a, b, False, True), torch.where(a.abs() < 2.0**-126, 0, a).double(), b.double()) < 1
+    # (the epilogues' arithmetic flushes results below 2^-126)
+    assert _off(ops.matmul16(a, b, False, True), a.double(), b.double(), floor=2.0**-126) < 1
     a[0, 20, 5], a[0, 21, 6], b[0, 9, 1] = float("nan"), float("inf"), float("-inf")
     got, general = ops.matmul16(a, b, False, True), ops.matmul3(a, b, False, True)
     assert torch.equal(torch.isfinite(got), torch.isfinite(general)) and torch.equal(got.isnan(), general.isnan())
@@ -140,3 +142,107 @@ def test_refused_operands():
         ops.split16_gemm(a, a, out=torch.empty(1, 128, 100, device="cuda"))
     with pytest.raises(RuntimeError):
         ops.split16(_rand(1, 64, 128, seed=16).mT)
+
+
+@pytest.mark.parametrize("R,C", [(5504, 33), (31, 2500), (257, 1025), (1, 1)])
+def test_values_that_are_short_of_bits_are_counted(R, C):
+    x = _rand(2, R, C, seed=35)
+    x = torch.where(_rand(2, R, C, seed=36) > 1, x * 1e-12, x) * torch.logspace(-20, 20, R, device="cuda")[:, None]
+    x[0, 0], x[1, :, 0] = 0.0, 0.0
+    for op, rows in zip(ops.split16(x, True, True), (x, x.mT)):
+        n = rows.shape[1]
+        short = (rows != 0) & (rows.double().abs() < 2.0**-14 * op.unit[:, :n, None].double())
+        assert torch.equal(op.short[:, :n].long(), short.sum(-1))
+
+
+def _graded(B, rows, K, how, seed):
+    """Operands whose rows hold values that differ by more than a pair of fp16 numbers covers, opposite zeros of the other operand."""
+    a, b = _rand(B, rows, K, seed=seed), _rand(B, K, K, seed=seed + 1)
+    h = K // 3
+    if how == "identity":  # the result is the graded matrix itself
+        return a * torch.logspace(0, -30, K, device="cuda"), torch.eye(K, device="cuda").expand(B, K, K).contiguous()
+    a[..., h:] *= float(how)
+    b[:, :h, h:], b[:, h:, :h] = 0, 0
+    return a, b
+
+
+@pytest.mark.parametrize("how", ["identity", "1e-9", "1e-12", "1e-15", "1e-30"])
+@pytest.mark.parametrize("B,M,K", [(2, 200, 136), (1, 300, 517)])
+def test_small_values_opposite_zeros(B, M, K, how, tile):
+    """Entry by entry as exact as |a| |b| asks, whichever operand is graded, from rows, columns and views."""
+    a, b = _graded(B, M, K, how, 21)
+    want = a.double() @ b.double().mT
+    pa, pb = ops.split16(a)[0], ops.split16(b)[0]
+    out = torch.empty(B, M, K, device="cuda")
+    ops.split16_gemm(pa, pb, out=out)
+    assert _off(out, a.double(), b.double()) < 1
+    turned = torch.empty(B, K, M, device="cuda")
+    ops.split16_gemm(pb, pa, out=turned)
+    assert _off(turned, b.double(), a.double()) < 1
+    at, bt = (torch.empty(B, K, t.shape[1] + 3, device="cuda")[..., : t.shape[1]].copy_(t.mT) for t in (a, b))
+    ops.split16_gemm(ops.split16(at, False, True)[1], ops.split16(bt, False, True)[1], out=out)
+    assert _off(out, a.double(), b.double()) < 1
+    old = _rand(B, M, K, seed=23) * want.abs().float()
+    out = old.clone()
+    ops.split16_gemm(pa, pb, mode=ops.EPI_LERP, w=0.25, out=out)
+    want_lerp = old.double() * 0.75 + 0.25 * want  # in fp32: four roundings of values up to |old| + |x|
+    assert bool(((out.double() - want_lerp).abs() <= (old.double().abs() + a.double().abs() @ b.double().abs().mT) * 2.0**-15).all())
+    m, v = torch.zeros(B, M, K, device="cuda"), torch.zeros(B, M, K, device="cuda")
+    ops.split16_gemm(pa, pb, mode=ops.EPI_ADAM, b1=0.5, b2c=0.5, eps=1e-30, m=m, v=v, out=out)
+    assert _off(m, a.double(), b.double(), want * 0.5) < 1
+    ops.check_status()
+
+
+def test_small_values_in_symmetric_and_triangular_products(tile):
+    x = _rand(2, 390, 200, seed=24)
+    x[:, 130:, :100], x[:, :130, 100:] = 0, 0
+    x[:, 130:] *= torch.logspace(0, -16, 100, device="cuda").repeat(2)
+    x[:, 131, 100:] *= 1e12
+    op, out = ops.split16(x)[0], torch.empty(2, 390, 390, device="cuda")
+    ops.split16_gemm(op, op, out=out)
+    assert _off(out, x.double(), x.double()) < 1
+    r, s = _rand(2, 390, 390, seed=25).triu(), _rand(2, 390, 390, seed=26).triu()
+    r, s = r * torch.logspace(0, -15, 390, device="cuda"), s * torch.logspace(0, 15, 390, device="cuda")[:, None]
+    s[:, :, 200:] *= 1e-20
+    got = ops.matmul16(r, s, upper_upper=True)
+    assert _off(got, r.double(), s.double().mT) < 1 and float(got.tril(-1).abs().max()) == 0
+    ops.check_status()
+
+
+def test_values_below_the_normal_range_count(tile):
+    """Split tf32 multiplies subnormal values; rows of them, and rows whose only larger values meet zeros."""
+    a, b = torch.zeros(1, 130, 140, device="cuda"), _rand(1, 150, 140, seed=27) * 1e20
+    a[0, :65] = _rand(65, 140, seed=28) * 1e-41
+    a[0, 65:, :70], a[0, 65:, 70:] = 3e-40, 1e-30
+    b[0, :, 70:] = 0
+    assert _off(ops.matmul16(a, b, False, True), a.double(), b.double()) < 1
+
+
+def test_sources_are_read_only_where_a_result_hangs_on_them(tile):
+    a, b = _rand(2, 300, 256, seed=29), _rand(2, 260, 256, seed=30)
+    a[0, 7, 3], b[1, 100, 200] = 1e-12, -1e-30  # short of bits, but lost in sums over ordinary values
+    pa, pb, out = ops.split16(a)[0], ops.split16(b)[0], torch.empty(2, 300, 260, device="cuda")
+    assert int(pa.short[0, 7]) == 1 and int(pb.short[1, 100]) == 1
+    pa.x, pb.x = torch.full_like(a, float("nan")), torch.full_like(b, float("nan"))
+    ops.split16_gemm(pa, pb, out=out)
+    assert _off(out, a.double(), b.double()) < 1
+    with pytest.raises(RuntimeError):  # an output over a source
+        ops.split16_gemm(ops.split16(c := _rand(1, 256, 128, seed=33))[0], ops.split16(_rand(1, 128, 128, seed=34))[0], out=c)
+
+
+@pytest.mark.parametrize("decades", [0, 12, 25])
+def test_solves_with_graded_factors_lose_nothing_to_split_tf32(decades):
+    """The blocked solve of a preconditioner fit: residual per entry in units of ``|x| |q|``, next to the split-tf32 product's."""
+    from heavyball_b200.utils.core import _solve_right_upper
+
+    d, rows = 640, 300
+    scale = torch.logspace(0, -decades, d, device="cuda")
+    q = (_rand(2, d, d, seed=31).triu(1) * 0.02 + torch.eye(d, device="cuda") * 2) * scale[:, None]
+    q[:, :256, 384:] = 0
+    b = _rand(2, rows, d, seed=32) * scale.flip(0)
+
+    def residual(pairs):
+        x = _solve_right_upper(q, b, pairs=pairs).double()
+        return float(((x @ q.double() - b.double()).abs() / (x.abs() @ q.double().abs() + b.double().abs())).max())
+
+    assert residual(True) <= 2 * residual(False) + 2.0**-20
