@@ -48,23 +48,25 @@ struct PairOperands {
   int K;
 };
 
-// 32 rows x 32 of K of an operand's matrix (zeros outside it), fetched in the order in which they lie in memory and put down as rows
-__device__ __forceinline__ void fetch_source(float (&v)[32], int lane, const PairOperand& op, int batch, int row0, int rows, int k0, int K) {
-  const float* p = op.src + batch * op.src_batch + row0 * op.src_row + k0 * op.src_k;
+// 32 rows x 16 of K of an operand's matrix (zeros outside it), fetched in the order in which they lie in memory and put down as rows
+__device__ __forceinline__ void fetch_source(float (&v)[16], int lane, const PairOperand& op, int batch, int row0, int rows, int k0, int K) {
   const bool along_k = op.src_k == 1;
-  const int64_t step = along_k ? op.src_row : op.src_k;
-  const int mine = along_k ? K - k0 : rows - row0, others = along_k ? rows - row0 : K - k0;
+  const int r = along_k ? lane >> 4 : lane, k = along_k ? lane & 15 : 0;  // of v[0]; v[i] is two rows (along_k) or one k further each time
+  const int64_t step = along_k ? 2 * op.src_row : op.src_k;
+  const float* p = op.src + batch * op.src_batch + (row0 + r) * op.src_row + (k0 + k) * op.src_k;
+  if (row0 + 32 <= rows && k0 + 16 <= K) {
 #pragma unroll
-  for (int i = 0; i < 32; ++i) v[i] = (lane < mine && i < others) ? p[(along_k ? lane : lane * op.src_row) + i * step] : 0.0f;
-}
-__device__ __forceinline__ void stage_source(float* stage, const float (&v)[32], int lane, const PairOperand& op) {
-  if (op.src_k == 1) {
-#pragma unroll
-    for (int i = 0; i < 32; ++i) stage[i * kStageLd + lane] = v[i];
+    for (int i = 0; i < 16; ++i) v[i] = p[i * step];
   } else {
 #pragma unroll
-    for (int i = 0; i < 32; ++i) stage[lane * kStageLd + i] = v[i];
+    for (int i = 0; i < 16; ++i) v[i] = (row0 + r + (along_k ? 2 * i : 0) < rows && k0 + k + (along_k ? 0 : i) < K) ? p[i * step] : 0.0f;
   }
+}
+__device__ __forceinline__ void stage_source(float* stage, const float (&v)[16], int lane, const PairOperand& op) {
+  const bool along_k = op.src_k == 1;
+  float* p = stage + (along_k ? (lane >> 4) * kStageLd + (lane & 15) : lane * kStageLd);
+#pragma unroll
+  for (int i = 0; i < 16; ++i) p[i * (along_k ? 2 * kStageLd : 1)] = v[i];
 }
 
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
@@ -80,7 +82,7 @@ constexpr uint32_t kManyShort = 1u << 19;  // counts of short values from here o
 // A value below 2^-14 in units of its row is held with an error of up to 2^-36 of a unit instead of 22 bits of itself.  With the other
 // operand's values (2^15 at most) and the product of low parts that is left out, n of them bring an error of at most n 2^-20: where the
 // accumulator is 4 n or more, less than 2^-22 of the result.  Smaller accumulators of such rows and columns may consist of nothing else:
-// the block is computed from the matrices themselves, in fp32 arithmetic (subnormals kept), sums of 32 at a time, the next 32 of K on their
+// the block is computed from the matrices themselves, in fp32 arithmetic (subnormals kept), sums of 16 at a time, the next 16 of K on their
 // way meanwhile.  (One such value among ordinary ones, as in one of a hundred thousand rows of 1024 normally distributed values, does not
 // lead there: sums over ordinary values are around 2^25 and more.)
 // `tri`: entries below the diagonal are zeros whatever the values.
@@ -108,58 +110,82 @@ __device__ __noinline__ void settle_slowly(uint32_t tmem, int lane, float* stage
     }
     return;
   }
-  float out[32], a[32], next_a[32], next_b[32];
-  for (int j = 0; j < 32; ++j) out[j] = 0.0f;
+  // a lane has rows y + 8 i and columns x + 4 j: twelve loads from the stage for 128 products, no two of a quarter warp in one bank
+  const int x = lane & 3, y = lane >> 2;
+  float out[4][8], next_a[16], next_b[16];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) out[i][j] = 0.0f;
   fetch_source(next_a, lane, P.a, batch, row0, M, 0, P.K);
   fetch_source(next_b, lane, P.b, batch, col0, N, 0, P.K);
 #pragma unroll 1
-  for (int k0 = 0; k0 < P.K; k0 += 32) {
+  for (int k0 = 0; k0 < P.K; k0 += 16) {
     __syncwarp();
-    stage_source(stage, next_a, lane, P.a);
+    stage_source(stage, next_a, lane, P.a);       // columns 0 .. 15 of the stage
+    stage_source(stage + 16, next_b, lane, P.b);  // columns 16 .. 31
     __syncwarp();
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const float4 t = *(const float4*)(stage + lane * kStageLd + q * 4);
-      a[q * 4] = t.x; a[q * 4 + 1] = t.y; a[q * 4 + 2] = t.z; a[q * 4 + 3] = t.w;
+    if (k0 + 16 < P.K) {
+      fetch_source(next_a, lane, P.a, batch, row0, M, k0 + 16, P.K);
+      fetch_source(next_b, lane, P.b, batch, col0, N, k0 + 16, P.K);
     }
-    __syncwarp();
-    stage_source(stage, next_b, lane, P.b);
-    __syncwarp();
-    if (k0 + 32 < P.K) {
-      fetch_source(next_a, lane, P.a, batch, row0, M, k0 + 32, P.K);
-      fetch_source(next_b, lane, P.b, batch, col0, N, k0 + 32, P.K);
-    }
-#pragma unroll 4
-    for (int j = 0; j < 32; ++j) {
-      float sum = 0.0f;
+    float sum[4][8];
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        const float4 t = *(const float4*)(stage + j * kStageLd + q * 4);
-        const float b[4] = {t.x, t.y, t.z, t.w};
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum) : "f"(a[q * 4 + e]), "f"(b[e]));
+      for (int j = 0; j < 8; ++j) sum[i][j] = 0.0f;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float a[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) *(float4*)a[i] = *(const float4*)(stage + (y + 8 * i) * kStageLd + q * 4);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float b[4];
+        *(float4*)b = *(const float4*)(stage + (x + 4 * j) * kStageLd + 16 + q * 4);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum[i][j]) : "f"(a[i][e]), "f"(b[e]));
       }
-      float total = out[j];
-      asm("add.rn.f32 %0, %0, %1;" : "+f"(total) : "f"(sum));
-      out[j] = total;
     }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int j = 0; j < 8; ++j) asm("add.rn.f32 %0, %0, %1;" : "+f"(out[i][j]) : "f"(sum[i][j]));
   }
   __syncwarp();
-  for (int j = 0; j < 32; ++j) mine[j] = out[j] * alpha;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) stage[(y + 8 * i) * kStageLd + x + 4 * j] = out[i][j] * alpha;
+  __syncwarp();
 }
 
-// Whether the units of this lane's row and column allow the usual way: no values short of bits, far from the ends of the range.
+// Units of a warp's 32 rows (lane = row) and four blocks of 32 columns (lane = column), fetched while the products are under way; `slow`: the blocks
+// that are not ordinary - some value short of bits, or a unit far from one.
+struct BlockUnits {
+  float row, col[4];
+  uint32_t slow;
+};
 __device__ __forceinline__ bool ordinary_unit(float u, bool inside) { return !inside || (short_values(u, true) == 0 && u > 0x1p-63f && u < 0x1p63f); }
+__device__ __forceinline__ BlockUnits fetch_units(const PairOperands& P, int lane, int batch, int row0, int col0, int M, int N) {
+  BlockUnits u;
+  u.row = P.a.unit[batch * P.a.unit_batch + row0 + lane];
+#pragma unroll
+  for (int cb = 0; cb < 4; ++cb) u.col[cb] = P.b.unit[batch * P.b.unit_batch + col0 + cb * 32 + lane];
+  u.slow = 0;
+#pragma unroll
+  for (int cb = 0; cb < 4; ++cb)
+    if (!__all_sync(0xFFFFFFFFu, ordinary_unit(u.row, row0 + lane < M) && ordinary_unit(u.col[cb], col0 + cb * 32 + lane < N))) u.slow |= 1u << cb;
+  return u;
+}
+__device__ __forceinline__ float col_unit_of(const BlockUnits& u, int cb) { return cb < 2 ? (cb == 0 ? u.col[0] : u.col[1]) : (cb == 2 ? u.col[2] : u.col[3]); }
 
-// Accumulators of an ordinary 32 x 32 block (lane = row, `row_unit`) -> entries of the product.
-__device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_unit, const float* col_units) {
+// Accumulators of an ordinary 32 x 32 block (lane = row) -> entries of the product.
+__device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_unit, float col_unit) {
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const float4 c = *(const float4*)(col_units + q * 4);
-    const float f[4] = {c.x, c.y, c.z, c.w};
-#pragma unroll
-    for (int e = 0; e < 4; ++e) acc[q * 4 + e] = __float_as_uint(__uint_as_float(acc[q * 4 + e]) * (row_unit * f[e]));
-  }
+  for (int j = 0; j < 32; ++j) acc[j] = __float_as_uint(__uint_as_float(acc[j]) * (row_unit * __shfl_sync(0xFFFFFFFFu, col_unit, j)));
 }
 
 // The usual case of the epilogue below: a 32 x 32 block inside the output, C aligned, no split output.  With the mode known at compile
@@ -169,7 +195,7 @@ __device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_unit, c
 // product's entries are in the stage already.
 template <bool kScaled, int kMode>
 __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* stage, const Tf32Epilogue& E, float* c, float* cm, float* m,
-                                               float* v, int64_t ld_state, bool staged, float row_unit, const float* col_units) {
+                                               float* v, int64_t ld_state, bool staged, float row_unit, float col_unit) {
   constexpr bool kOld = kMode == kEpiLerp || kMode == kEpiAdd, kMoments = kMode == kEpiAdam || kMode == kEpiLaProp;
   const int sub = lane >> 3, cg = (lane & 7) * 4;
   float* const mine = stage + lane * kStageLd;
@@ -194,7 +220,7 @@ __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* s
     uint32_t acc[32];
     tmem_ld32(tmem, acc);
     tmem_ld_wait();
-    if constexpr (kScaled) unscale32(acc, row_unit, col_units);
+    if constexpr (kScaled) unscale32(acc, row_unit, col_unit);
 #pragma unroll
     for (int q = 0; q < 8; ++q)
       *(float4*)(mine + q * 4) =
@@ -256,11 +282,11 @@ __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* s
 // `tmem_warp`: tensor-memory address of the warp's first row and the tile's first column; `row0` / `col_base`: their
 // global indices; `n_cb`: 32-column blocks in the tile; `off_diagonal`: the tile is not on the diagonal (mirror stores).
 // `zero_acc`: the tile had no product (its accumulator was never written): the values are zeros.
-// `kScaled`: the operands are fp16 pairs, described by `P`; their products have no split outputs.
+// `kScaled`: the operands are fp16 pairs, described by `P` and by the units `U` of the warp's blocks; their products have no split outputs.
 template <bool kScaled>
 __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, float* stage, int row0, int col_base, int n_cb,
                                                 bool off_diagonal, bool zero_acc, int batch, int M, int N,
-                                                const Tf32Epilogue& E, const PairOperands& P) {
+                                                const Tf32Epilogue& E, const PairOperands& P, const BlockUnits& U) {
   const int64_t b64 = batch;
   const bool state_vec = (N & 3) == 0;
   const bool c_vec = (E.ldc & 3) == 0 && ((E.strideC & 3) == 0) && ((((uintptr_t)E.C) & 15) == 0);
@@ -271,20 +297,15 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
   const int sub = lane >> 3, cg = (lane & 7) * 4;
   const float w1 = 1.0f - E.b1, w2 = 1.0f - E.b2;
   float* mine = stage + lane * kStageLd;
-  const float* const col_units = kScaled ? P.b.unit + b64 * P.b.unit_batch + col_base : nullptr;
-  float row_unit = 1.0f, col_unit = 1.0f;
-  if constexpr (kScaled) {
-    row_unit = P.a.unit[b64 * P.a.unit_batch + row0 + lane];
-    col_unit = col_units[lane];
-  }
 #pragma unroll 1
   for (int cb = 0; cb < n_cb; ++cb) {
     const int col0 = col_base + cb * 32;
+    float col_unit = 1.0f;
     bool staged = false;
     if constexpr (kScaled) {
-      staged = !zero_acc && !__all_sync(0xFFFFFFFFu, ordinary_unit(row_unit, row0 + lane < M) && ordinary_unit(col_unit, col0 + lane < N));
+      col_unit = col_unit_of(U, cb);
+      staged = !zero_acc && (U.slow >> cb & 1);
       if (staged) settle_slowly(tmem_warp + (uint32_t)(cb * 32), lane, stage, P, batch, row0, col0, M, N, E.tri, E.alpha);
-      if (cb + 1 < n_cb) col_unit = col_units[(cb + 1) * 32 + lane];
     }
     if (!zero_acc && !s_rows && !s_cols && c_vec && E.C != nullptr && row0 + 32 <= M && col0 + 32 <= N && (!moments || state_vec)) {
       const uint32_t t = tmem_warp + (uint32_t)(cb * 32);
@@ -292,11 +313,11 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
       float* cm = mirror ? E.C + b64 * E.strideC + (int64_t)col0 * E.ldc + row0 : nullptr;
       const int64_t st = (b64 * M + row0) * (int64_t)N + col0;
       switch (E.mode) {
-        case kEpiStore: epilogue_block<kScaled, kEpiStore>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, row_unit, col_units + cb * 32); break;
-        case kEpiLerp: epilogue_block<kScaled, kEpiLerp>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, row_unit, col_units + cb * 32); break;
-        case kEpiAdd: epilogue_block<kScaled, kEpiAdd>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, row_unit, col_units + cb * 32); break;
-        case kEpiAdam: epilogue_block<kScaled, kEpiAdam>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, row_unit, col_units + cb * 32); break;
-        default: epilogue_block<kScaled, kEpiLaProp>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, row_unit, col_units + cb * 32); break;
+        case kEpiStore: epilogue_block<kScaled, kEpiStore>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, U.row, col_unit); break;
+        case kEpiLerp: epilogue_block<kScaled, kEpiLerp>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, U.row, col_unit); break;
+        case kEpiAdd: epilogue_block<kScaled, kEpiAdd>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, U.row, col_unit); break;
+        case kEpiAdam: epilogue_block<kScaled, kEpiAdam>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, U.row, col_unit); break;
+        default: epilogue_block<kScaled, kEpiLaProp>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, U.row, col_unit); break;
       }
       continue;
     }
@@ -310,7 +331,7 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
         for (int j = 0; j < 32; ++j) acc[j] = 0u;
       }
       if constexpr (kScaled)
-        if (!zero_acc) unscale32(acc, row_unit, col_units + cb * 32);
+        if (!zero_acc) unscale32(acc, U.row, col_unit);
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *(float4*)(mine + q * 4) =
@@ -558,6 +579,8 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     }
   } else {
     const int quarter = warp & 3, r = quarter * 32 + lane;
+    BlockUnits U{};
+    if constexpr (Kind::kScaled) U = fetch_units(P, lane, batch, tm * TBM + quarter * 32, tn * TBN, M, N);
     const bool have = (num_kb == 0) || mbar_wait(&accum_bar, 0, &abort_flag);
     tc_fence_after();
     if (have && bulk_store) {
@@ -568,19 +591,16 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         uint32_t acc[32];
         const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32);
         if constexpr (Kind::kScaled) {
-          const int row = tm * TBM + quarter * 32 + lane, col0 = tn * TBN + cb * 32;
-          const float* const col_units = P.b.unit + batch * P.b.unit_batch + col0;
-          const float row_unit = P.a.unit[batch * P.a.unit_batch + row];
-          if (__all_sync(0xFFFFFFFFu, ordinary_unit(row_unit, row < M) && ordinary_unit(col_units[lane], col0 + lane < N))) {
-            tmem_ld32(t, acc);
-            tmem_ld_wait();
-            unscale32(acc, row_unit, col_units);
-          } else {
+          if (U.slow >> cb & 1) {
             float* const stage = (float*)(tiles + (TBN / 32) * kTTileBytes + quarter * kStageWarpBytes);  // behind the boxes
-            settle_slowly(t, lane, stage, P, batch, row - lane, col0, M, N, 0, 1.0f);
+            settle_slowly(t, lane, stage, P, batch, tm * TBM + quarter * 32, tn * TBN + cb * 32, M, N, 0, 1.0f);
 #pragma unroll
             for (int j = 0; j < 32; ++j) acc[j] = __float_as_uint(stage[lane * kStageLd + j]);
             __syncwarp();
+          } else {
+            tmem_ld32(t, acc);
+            tmem_ld_wait();
+            unscale32(acc, U.row, col_unit_of(U, cb));
           }
         } else {
           tmem_ld32(t, acc);
@@ -595,7 +615,7 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
       }
     } else if (have) {
       epilogue_direct<Kind::kScaled>(tmem_base + ((uint32_t)(quarter * 32) << 16), lane, (float*)(tiles + quarter * kStageWarpBytes),
-                      tm * TBM + quarter * 32, tn * TBN, TBN / 32, tm != tn, num_kb == 0, batch, M, N, E, P);
+                      tm * TBM + quarter * 32, tn * TBN, TBN / 32, tm != tn, num_kb == 0, batch, M, N, E, P, U);
     }
     tc_fence_before();
     if (bulk_store) {
@@ -751,16 +771,19 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
     for (int idx = pair; idx < total; idx += pairs, ++it) {
       const PairTile t = pair_tile(idx, tiles_m, tiles_n, per_batch, E.symmetric);
       const int acc = it & 1, row0 = t.tm * kPairTile + (int)rank * 128 + quarter * 32, col0 = t.tn * kPairTile + half * 128;
+      const int blocks = min(4, (N - col0 + 31) / 32);
+      BlockUnits U{};
+      if constexpr (Kind::kScaled)
+        if (row0 < M && blocks > 0) U = fetch_units(P, lane, t.batch, row0, col0, M, N);
       const bool ok = mbar_wait<Kind::kScaled ? kLongSpinLimit : kSpinLimit>(&acc_full[acc], (it >> 1) & 1, &abort_flag);
       if (!__all_sync(0xFFFFFFFFu, ok)) break;
       tc_fence_after();
-      const int blocks = min(4, (N - col0 + 31) / 32);
       // a tile on the diagonal: computed whole, or (symmetric == 2) as three of 128 x 128 whose middle one is mirrored
       const bool thirds = E.symmetric == 2 && t.tm == t.tn;
       const bool mirrored = thirds ? rank == 0 && half == 1 : t.tm != t.tn;
       if (row0 < M && blocks > 0 && !(thirds && rank == 1 && half == 0))
         epilogue_direct<Kind::kScaled>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, mirrored,
-                              walk_tile(t, kp, E.tri, Kind::kBlock).seg == 0, t.batch, M, N, E, P);
+                              walk_tile(t, kp, E.tri, Kind::kBlock).seg == 0, t.batch, M, N, E, P, U);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) cluster_arrive(cluster_addr(&acc_empty[acc], 0));

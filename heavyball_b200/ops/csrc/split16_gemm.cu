@@ -54,19 +54,28 @@ constexpr int kSplitThreads = 256;
 constexpr int kRowChunk = 1024;
 constexpr int kStrip = 32, kStripRows = 256, kMaxSplitCluster = 8;
 
-struct RowScale {
-  float mul, unit;  // 2^e, 2^-e
+// Largest absolute value (not counting NaN) and smallest one other than zero, the latter as its bits without the sign, shifted left, less
+// one: zeros come out above everything.
+struct RowRange {
+  float top = 0.0f;
+  uint32_t low = 0xFFFFFFFFu;
+  __device__ __forceinline__ void add(float x) {
+    top = fmaxf(top, fabsf(x));
+    low = min(low, (__float_as_uint(x) << 1) - 1u);
+  }
 };
-// `bits`: largest absolute value of the row, as its bits (NaN above infinity above everything finite)
-__device__ __forceinline__ RowScale row_scale(uint32_t bits) {
-  const int field = (int)(bits >> 23);
-  // rows with an infinity or NaN stay as they are: all of their results are NaN (lo = inf - inf)
-  const int e = field == 255 ? 0 : min(126, 141 - field);
-  return {pow2(e), pow2(-e)};
+struct RowScale {
+  float mul, unit;       // 2^e, 2^-e
+  uint32_t short_below;  // 2^(-14 - e) in the form of RowRange::low: values under it are too small for 22 bits in a pair
+};
+__device__ __forceinline__ RowScale row_scale(uint32_t top_bits) {
+  const int field = (int)(top_bits >> 23);
+  // rows with an infinity stay as they are: all of their results are NaN (lo = inf - inf)
+  if (field == 255) return {1.0f, 1.0f, 0u};
+  const int e = min(126, 141 - field), f = 113 - e;  // f: exponent field of 2^(-14 - e); 0 and below: subnormal
+  return {pow2(e), pow2(-e), ((f > 0 ? (uint32_t)f << 23 : 1u << (22 + f)) << 1) - 1u};
 }
-__device__ __forceinline__ uint32_t abs_bits(float x) { return __float_as_uint(x) & 0x7FFFFFFFu; }
-// x, scaled: too small for 22 bits in a pair
-__device__ __forceinline__ bool is_short(float x, float y) { return x != 0.0f && fabsf(y) < 0x1p-14f; }
+__device__ __forceinline__ uint32_t is_short(float x, uint32_t short_below) { return (__float_as_uint(x) << 1) - 1u < short_below ? 1u : 0u; }
 // without flushing subnormals
 __device__ __forceinline__ float scaled(float x, float mul) {
   float y;
@@ -90,9 +99,6 @@ __device__ __forceinline__ float4 load4(const float* p, int left, bool vec) {
   return make_float4(left > 0 ? p[0] : 0.f, left > 1 ? p[1] : 0.f, left > 2 ? p[2] : 0.f, left > 3 ? p[3] : 0.f);
 }
 
-__device__ __forceinline__ uint32_t abs_max4(float4 v) {
-  return max(max(abs_bits(v.x), abs_bits(v.y)), max(abs_bits(v.z), abs_bits(v.w)));
-}
 // position of row r of column c in the turned tile: four columns of a thread and four rows of a warp fall into distinct banks
 __device__ __forceinline__ int turned(int c, int r) { return c * kStripRows + (r ^ (c & ~3)); }
 
@@ -113,7 +119,8 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
     const int kp = (C + 63) / 64 * 64;
     const float* row = s + (int64_t)r * ld_src;
     float4 v[kRowChunk / 128];
-    uint32_t top = 0, n_short = 0;
+    RowRange range;
+    uint32_t n_short = 0;
     const auto fetch = [&](int base) {
 #pragma unroll
       for (int i = 0; i < kRowChunk / 128; ++i) {
@@ -125,18 +132,27 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
     for (int base = 0; base < C; base += kRowChunk) {
       fetch(base);
 #pragma unroll
-      for (int i = 0; i < kRowChunk / 128; ++i) top = max(top, abs_max4(v[i]));
+      for (int i = 0; i < kRowChunk / 128; ++i) {
+        range.add(v[i].x);
+        range.add(v[i].y);
+        range.add(v[i].z);
+        range.add(v[i].w);
+      }
     }
-    const RowScale f = row_scale(__reduce_max_sync(0xFFFFFFFFu, top));
+    const RowScale f = row_scale(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(range.top)));
     uint16_t* dst = same + (batch * R + r) * 2 * kp;
     for (int base = 0; base < C; base += kRowChunk) {
       if (C > kRowChunk) fetch(base);
+      if (range.low < f.short_below) {
+#pragma unroll
+        for (int i = 0; i < kRowChunk / 128; ++i)
+          n_short += is_short(v[i].x, f.short_below) + is_short(v[i].y, f.short_below) + is_short(v[i].z, f.short_below) + is_short(v[i].w, f.short_below);
+      }
 #pragma unroll
       for (int i = 0; i < kRowChunk / 128; ++i) {
         const int c = base + i * 128 + lane * 4;
         if (c < kp) {
           const float x[4] = {scaled(v[i].x, f.mul), scaled(v[i].y, f.mul), scaled(v[i].z, f.mul), scaled(v[i].w, f.mul)};
-          n_short += is_short(v[i].x, x[0]) + is_short(v[i].y, x[1]) + is_short(v[i].z, x[2]) + is_short(v[i].w, x[3]);
           split_store4(dst + c, kp, x);
         }
       }
@@ -149,7 +165,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
   __shared__ __align__(16) float tile[kStrip * kStripRows];
   __shared__ uint32_t warp_tops[kSplitThreads / 32][kStrip];
   __shared__ uint32_t tops[kStrip];  // of this block's rows; the blocks of the cluster read each other's
-  __shared__ uint32_t shorts[kStrip];
+  __shared__ uint32_t short_below[kStrip], shorts[kStrip];
   __shared__ float muls[kStrip];
   const int at = blockIdx.x - row_blocks, rank = at % cluster, c0 = at / cluster * kStrip;
   const int q = threadIdx.x & 7, line = threadIdx.x >> 3, c = c0 + q * 4, kp = (R + 63) / 64 * 64;
@@ -163,22 +179,22 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
       if (r < R && c < C) v[i] = load4(s + (int64_t)r * ld_src + c, C - c, vec);
     }
   };
-  uint32_t top[4] = {0, 0, 0, 0};
+  RowRange range[4];
   for (int r0 = first; r0 < R; r0 += step) {
     fetch(r0);
 #pragma unroll
     for (int i = 0; i < kStripRows / 32; ++i) {
-      top[0] = max(top[0], abs_bits(v[i].x));
-      top[1] = max(top[1], abs_bits(v[i].y));
-      top[2] = max(top[2], abs_bits(v[i].z));
-      top[3] = max(top[3], abs_bits(v[i].w));
+      range[0].add(v[i].x);
+      range[1].add(v[i].y);
+      range[2].add(v[i].z);
+      range[3].add(v[i].w);
     }
   }
 #pragma unroll
   for (int e = 0; e < 4; ++e) {
-    top[e] = max(top[e], __shfl_xor_sync(0xFFFFFFFFu, top[e], 8));
-    top[e] = max(top[e], __shfl_xor_sync(0xFFFFFFFFu, top[e], 16));
-    if (lane < 8) warp_tops[warp][lane * 4 + e] = top[e];
+    float top = fmaxf(range[e].top, __shfl_xor_sync(0xFFFFFFFFu, range[e].top, 8));
+    top = fmaxf(top, __shfl_xor_sync(0xFFFFFFFFu, top, 16));
+    if (lane < 8) warp_tops[warp][lane * 4 + e] = __float_as_uint(top);
   }
   __syncthreads();
   if (threadIdx.x < kStrip) {
@@ -195,26 +211,31 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
       t = max(t, (uint32_t)cluster_load(cluster_addr(&tops[threadIdx.x], (rank + k) % cluster)));
     const RowScale f = row_scale(t);
     muls[threadIdx.x] = f.mul;
+    short_below[threadIdx.x] = f.short_below;
     if (rank == 0 && c0 + (int)threadIdx.x < C) trans_unit[batch * ((C + 255) / 256 * 256) + c0 + threadIdx.x] = f.unit;
   }
   if (cluster > 1) cluster_sync(); else __syncthreads();  // no block leaves while its maxima may still be read
   const int oc = threadIdx.x >> 4, k4 = (threadIdx.x & 15) * 4;  // output: rows c0 + oc (+ 16) of the operand, four of K at a time
   for (int r0 = first; r0 < R; r0 += step) {
     if (R > step) fetch(r0);
-    uint32_t n_short = 0;  // a byte per column: a thread has eight rows
 #pragma unroll
     for (int i = 0; i < kStripRows / 32; ++i) {
       const int r = line + 32 * i;
-      const float x[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+      tile[turned(q * 4 + 0, r)] = scaled(v[i].x, muls[q * 4 + 0]);
+      tile[turned(q * 4 + 1, r)] = scaled(v[i].y, muls[q * 4 + 1]);
+      tile[turned(q * 4 + 2, r)] = scaled(v[i].z, muls[q * 4 + 2]);
+      tile[turned(q * 4 + 3, r)] = scaled(v[i].w, muls[q * 4 + 3]);
+    }
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float y = scaled(x[e], muls[q * 4 + e]);
-        tile[turned(q * 4 + e, r)] = y;
-        n_short += (uint32_t)is_short(x[e], y) << (8 * e);
+    for (int e = 0; e < 4; ++e) {
+      const uint32_t below = short_below[q * 4 + e];
+      if (range[e].low < below) {  // this thread has some in column e
+        uint32_t n = 0;
+#pragma unroll
+        for (int i = 0; i < kStripRows / 32; ++i) n += is_short(e == 0 ? v[i].x : e == 1 ? v[i].y : e == 2 ? v[i].z : v[i].w, below);
+        atomicAdd(&shorts[q * 4 + e], n);
       }
     }
-    if (n_short != 0)
-      for (int e = 0; e < 4; ++e) atomicAdd(&shorts[q * 4 + e], n_short >> (8 * e) & 255u);
     __syncthreads();
 #pragma unroll
     for (int g = 0; g < kStrip; g += 16) {

@@ -9,7 +9,7 @@ namespace hb {
 
 // Operand: [rows, 2 * kp] fp16 with kp = K rounded up to 64; a row holds [hi | lo], hi = fp16(x 2^e), lo = fp16((x 2^e - hi) 2^11),
 // where the exponent e of the row takes its largest value to [2^14, 2^15), 126 at most (rows below 2^-112 stay under that; rows with an
-// infinity or a NaN have e = 0); columns [K, kp) of both halves are zero.  `unit` holds 2^-e per row and, in the mantissa, the number of the
+// infinity have e = 0); columns [K, kp) of both halves are zero.  `unit` holds 2^-e per row and, in the mantissa, the number of the
 // row's values below 2^-14 2^-e other than zero, which a pair holds in fewer than 22 bits (2^19 and more: any number);
 // [batch, split16_units(rows)] (padded to whole tiles; the padding is read but never reaches a result).
 inline int64_t split16_kp(int64_t K) { return (K + 63) / 64 * 64; }

@@ -23,7 +23,7 @@ def _rand(*shape, seed):
 def _off(got, a, b, want=None, floor=0.0):
     """Largest error in units of its bound: 22 bits of either operand and the dropped product of low parts (4 units of 2^-22), and one
     rounding of the accumulator per 16 of K in the last of three walks plus a few for the first two (2^-23 of |a| |b| each).  Blocks that
-    are computed in fp32 stay under it, too: sums of 32 products at a time round 32 + K / 32 times by 2^-24."""
+    are computed in fp32 stay under it, too: sums of 16 products at a time round 16 + K / 16 times by 2^-24."""
     K = a.shape[-1]
     bound = (a.abs() @ b.abs().mT) * (2.0**-20 + (K / 16 + 4) * 2.0**-23) + floor
     return float(((got.double() - (a @ b.mT if want is None else want)).abs() / bound.clamp_min(1e-300)).max())
