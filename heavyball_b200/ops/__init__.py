@@ -361,6 +361,13 @@ def matmul16(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: b
     return _matmul(load().split16_matmul, a, b, trans_a, trans_b, alpha, upper_upper)
 
 
+def split16_accumulate(c: torch.Tensor, a: torch.Tensor, b: torch.Tensor, trans_b: bool = False, alpha: float = 1.0):
+    """``c += alpha * a @ op(b)`` from fp16 pairs, in place on the fp32 view ``c``; all three ``[batch, rows, cols]`` with unit inner
+    stride, ``c`` apart from the others."""
+    load().split16_accumulate(c, a, b, trans_b, alpha, _status(a.device))
+    launch_counter.count += 3
+
+
 def _matmul(kernel, a, b, trans_a, trans_b, alpha, upper_upper):
     lead = a.shape[:-2]
     if b.shape[:-2] != lead:

@@ -491,6 +491,11 @@ at::Tensor tf32_gemm(const at::Tensor& a2, const at::Tensor& b2, int64_t K, int 
   return s;
 }
 
+void check_split16_source(const at::Tensor& x) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 3 && x.stride(2) == 1 && x.size(0) >= 1 && x.size(1) >= 1 &&
+                  x.size(2) >= 1 && x.size(0) <= 65535, "split16: fp32 [batch, rows, cols] CUDA tensor with unit inner stride");
+}
+
 // The matrix x behind an operand whose rows are the rows (trans: the columns) of x.
 hb::Split16Source source_of(const at::Tensor& x, bool trans) {
   return {x.data_ptr<float>(), x.stride(0), trans ? x.stride(2) : x.stride(1), trans ? x.stride(1) : x.stride(2)};
@@ -499,8 +504,7 @@ hb::Split16Source source_of(const at::Tensor& x, bool trans) {
 // Operands of the fp16-pair product of an fp32 [batch, R, C] tensor (see split16_gemm.h): (same, same_unit, trans, trans_unit); an
 // orientation that was not asked for comes back undefined.
 std::vector<at::Tensor> split16(const at::Tensor& x, bool want_same, bool want_trans) {
-  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 3 && x.stride(2) == 1 && x.size(0) >= 1 && x.size(1) >= 1 &&
-                  x.size(2) >= 1 && x.size(0) <= 65535, "split16: fp32 [batch, rows, cols] CUDA tensor with unit inner stride");
+  check_split16_source(x);
   c10::cuda::CUDAGuard guard(x.device());
   const int64_t batch = x.size(0), R = x.size(1), C = x.size(2);
   std::vector<at::Tensor> out(4);
@@ -515,6 +519,14 @@ std::vector<at::Tensor> split16(const at::Tensor& x, bool want_same, bool want_t
   check(hb::launch_split16(x.data_ptr<float>(), x.stride(1), x.stride(0), (int)R, (int)C, (int)batch, op[0], op[1],
                            at::cuda::getCurrentCUDAStream()), "split16");
   return out;
+}
+
+// Results may be computed from the matrices after others have been stored.  (Interleaved views of one buffer pass: whether they share
+// entries is the caller's business.)
+void check_split16_overlap(const at::Tensor& out, const at::Tensor& source) {
+  const at::MemOverlapStatus overlap = at::get_overlap_status(out, source);
+  TORCH_CHECK(overlap != at::MemOverlapStatus::Full && overlap != at::MemOverlapStatus::Partial,
+              "split16: an output lies over the matrix that an operand was made from");
 }
 
 // epilogue(A * B^T) over operands of split16; arguments as for tf32_gemm.  Both operands being one buffer makes the product symmetric.
@@ -534,11 +546,7 @@ void split16_gemm(const at::Tensor& a, const at::Tensor& ua, const at::Tensor& x
     TORCH_CHECK(s.x.device() == a.device() && s.x.scalar_type() == at::kFloat && s.x.dim() == 3 && s.x.size(0) == batch && s.x.stride(2) == 1 &&
                     s.x.size(s.trans ? 2 : 1) == s.rows && s.x.size(s.trans ? 1 : 2) == K, "split16_gemm: the source of another operand");
     for (const OptT* out : {&c, &m, &v})
-      if (out->has_value() && (*out)->defined()) {
-        const at::MemOverlapStatus overlap = at::get_overlap_status(**out, s.x);
-        TORCH_CHECK(overlap != at::MemOverlapStatus::Full && overlap != at::MemOverlapStatus::Partial,
-                    "split16_gemm: an output lies over the matrix that an operand was made from");
-      }
+      if (out->has_value() && (*out)->defined()) check_split16_overlap(**out, s.x);
   }
   c10::cuda::CUDAGuard guard(a.device());
   hb::Tf32Epilogue E{};
@@ -564,23 +572,61 @@ void split16_gemm(const at::Tensor& a, const at::Tensor& ua, const at::Tensor& x
                                 (int)M, (int)N, (int)K, (int)batch, E, status.data_ptr<int>(), at::cuda::getCurrentCUDAStream()), "split16 gemm");
 }
 
+// c <- alpha op(a) op(b), or c + alpha op(a) op(b) (kEpiAdd): both operand passes and the product.  The operands share one allocation: a
+// captured region cannot use blocks of the memory outside it, and what it pays for its own goes by their number.
+void split16_product(const at::Tensor& a, const at::Tensor& b, bool ta, bool tb, int mode, double alpha, const at::Tensor& c, bool upper_upper,
+                     const at::Tensor& status) {
+  const int64_t batch = a.size(0), M = ta ? a.size(2) : a.size(1), K = ta ? a.size(1) : a.size(2), N = tb ? b.size(1) : b.size(2);
+  TORCH_CHECK(b.device() == a.device() && b.size(0) == batch && (tb ? b.size(2) : b.size(1)) == K, "split16: batches or inner dimensions differ");
+  const bool one = a.data_ptr() == b.data_ptr() && a.sizes() == b.sizes() && a.strides() == b.strides() && ta != tb;  // X X^T or X^T X
+  TORCH_CHECK(!upper_upper || (M == N && M == K && !one), "split16: upper_upper needs two square matrices of one size");
+  c10::cuda::CUDAGuard guard(a.device());
+  const auto stream = at::cuda::getCurrentCUDAStream();
+  // rows of pairs are multiples of 256 bytes, units of 1 KiB
+  const int64_t kp = hb::split16_kp(K), a_bytes = batch * M * 4 * kp, b_bytes = one ? 0 : batch * N * 4 * kp;
+  const int64_t a_units = batch * hb::split16_units(M) * 4, b_units = one ? 0 : batch * hb::split16_units(N) * 4;
+  const at::Tensor memory = at::empty({a_bytes + b_bytes + a_units + b_units}, a.options().dtype(at::kByte).memory_format(at::MemoryFormat::Contiguous));
+  uint8_t* const p = memory.data_ptr<uint8_t>();
+  const hb::Split16Operand none{};
+  const hb::Split16Operand A{p, (float*)(p + a_bytes + b_bytes), source_of(a, ta)};
+  // B as the K-major [N, K] operand: b given as [K, N] must be transposed, b given as [N, K] is used as it is
+  const hb::Split16Operand B = one ? A : hb::Split16Operand{p + a_bytes, (float*)(p + a_bytes + b_bytes + a_units), source_of(b, !tb)};
+  check(hb::launch_split16(a.data_ptr<float>(), a.stride(1), a.stride(0), (int)a.size(1), (int)a.size(2), (int)batch, ta ? none : A, ta ? A : none, stream),
+        "split16 of the left operand");
+  if (!one)
+    check(hb::launch_split16(b.data_ptr<float>(), b.stride(1), b.stride(0), (int)b.size(1), (int)b.size(2), (int)batch, tb ? B : none, tb ? none : B, stream),
+          "split16 of the right operand");
+  hb::Tf32Epilogue E{};
+  E.mode = mode; E.alpha = (float)alpha;
+  E.C = c.data_ptr<float>(); E.ldc = c.stride(1); E.strideC = c.stride(0);
+  E.tri = upper_upper ? 1 : 0;
+  E.symmetric = one ? 1 : 0;
+  check(hb::launch_split16_gemm(A, B, (int)M, (int)N, (int)K, (int)batch, E, status.data_ptr<int>(), stream), "split16 gemm");
+}
+
 // op(a) @ op(b) for batched fp32 matrices from fp16 pairs; arguments and result as for tf32x3_matmul.
 at::Tensor split16_matmul(const at::Tensor& a, const at::Tensor& b, bool ta, bool tb, double alpha, const at::Tensor& status,
                           bool upper_upper) {
-  TORCH_CHECK(a.dim() == 3 && b.dim() == 3, "split16_matmul: fp32 [batch, rows, cols] CUDA tensors");
-  const int64_t batch = a.size(0), M = ta ? a.size(2) : a.size(1), K = ta ? a.size(1) : a.size(2), N = tb ? b.size(1) : b.size(2);
-  TORCH_CHECK(b.size(0) == batch && (tb ? b.size(2) : b.size(1)) == K, "split16_matmul: batches or inner dimensions differ");
-  const bool same_operand = a.data_ptr() == b.data_ptr() && a.sizes() == b.sizes() && a.strides() == b.strides() && ta != tb;  // X X^T or X^T X
-  TORCH_CHECK(!(upper_upper && same_operand), "split16_matmul: upper_upper needs two square matrices of one size");
-  const std::vector<at::Tensor> sa = split16(a, !ta, ta);
-  // B as the K-major [N, K] operand: b given as [K, N] must be transposed, b given as [N, K] is used as it is
-  const std::vector<at::Tensor> sb = same_operand ? sa : split16(b, tb, !tb);
-  const int ia = ta ? 2 : 0, ib = same_operand ? ia : (tb ? 0 : 2);
-  const int64_t ldc = (N + 3) / 4 * 4;
-  at::Tensor c = at::empty({batch, M, ldc}, a.options().memory_format(at::MemoryFormat::Contiguous));
+  check_split16_source(a);
+  check_split16_source(b);
+  const int64_t M = ta ? a.size(2) : a.size(1), N = tb ? b.size(1) : b.size(2), ldc = (N + 3) / 4 * 4;
+  c10::cuda::CUDAGuard guard(a.device());
+  const at::Tensor c = at::empty({a.size(0), M, ldc}, a.options().memory_format(at::MemoryFormat::Contiguous));
   const at::Tensor view = ldc == N ? c : c.narrow(2, 0, N);
-  split16_gemm(sa[ia], sa[ia + 1], a, ta, sb[ib], sb[ib + 1], b, !tb, K, hb::kEpiStore, alpha, 0, 0, 0, 0, view, {}, {}, upper_upper, status);
+  split16_product(a, b, ta, tb, hb::kEpiStore, alpha, view, upper_upper, status);
   return view;
+}
+
+// c <- c + alpha a op(b), in place on the view c (unit inner stride), which neither operand may overlap.
+void split16_accumulate(const at::Tensor& c, const at::Tensor& a, const at::Tensor& b, bool tb, double alpha, const at::Tensor& status) {
+  check_split16_source(a);
+  check_split16_source(b);
+  TORCH_CHECK(c.device() == a.device() && c.scalar_type() == at::kFloat && c.dim() == 3 && c.stride(2) == 1 && c.size(0) == a.size(0) &&
+                  c.size(1) == a.size(1) && c.size(2) == (tb ? b.size(1) : b.size(2)) && c.stride(1) >= c.size(2),
+              "split16_accumulate: c must be fp32 [batch, M, N] with unit inner stride");
+  check_split16_overlap(c, a);
+  check_split16_overlap(c, b);
+  split16_product(a, b, false, tb, hb::kEpiAdd, alpha, c, false, status);
 }
 
 // op(a) @ op(b) for batched fp32 matrices on the split-tf32 tensor-core path.  a: [batch, R, C]; ta = 0 uses a as
@@ -844,6 +890,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("tf32_gemm", &tf32_gemm);
   m.def("split16", &split16);
   m.def("split16_matmul", &split16_matmul);
+  m.def("split16_accumulate", &split16_accumulate);
   m.def("split16_gemm", &split16_gemm);
   m.def("set_split16_gemm_tile", &hb::set_split16_gemm_tile_override);
   m.def("colsum_bf16", &colsum_bf16);

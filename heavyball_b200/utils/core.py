@@ -514,16 +514,15 @@ def _tc_sub_product(c: Tensor, a: Tensor, b: Tensor, b_transposed: bool = False,
         return False
     if any(t.stride(-1) != 1 or t.dtype != torch.float32 for t in (a, b, c)) or c.data_ptr() % 16 or c.stride(-2) % 4 or c.stride(0) % 4:
         return False
-    split = ops.split16 if pairs else ops.tf32_split
-    a_s, _ = split(a, True, False)
-    if b_transposed:
-        b_s = a_s if (b.data_ptr() == a.data_ptr() and b.shape == a.shape and b.stride() == a.stride()) else split(b, True, False)[0]
-    else:
-        b_s = split(b, False, True)[1]
     if pairs:
-        ops.split16_gemm(a_s, b_s, mode=ops.EPI_ADD, alpha=-1.0, out=c)
+        ops.split16_accumulate(c, a, b, b_transposed, -1.0)
+        return True
+    a_s, _ = ops.tf32_split(a, True, False)
+    if b_transposed:
+        b_s = a_s if (b.data_ptr() == a.data_ptr() and b.shape == a.shape and b.stride() == a.stride()) else ops.tf32_split(b, True, False)[0]
     else:
-        ops.tf32_gemm(a_s, b_s, a.shape[-1], mode=ops.EPI_ADD, alpha=-1.0, out=c)
+        b_s = ops.tf32_split(b, False, True)[1]
+    ops.tf32_gemm(a_s, b_s, a.shape[-1], mode=ops.EPI_ADD, alpha=-1.0, out=c)
     return True
 
 

@@ -246,3 +246,32 @@ def test_solves_with_graded_factors_lose_nothing_to_split_tf32(decades):
         return float(((x @ q.double() - b.double()).abs() / (x.abs() @ q.double().abs() + b.double().abs())).max())
 
     assert residual(True) <= 2 * residual(False) + 2.0**-20
+
+
+@pytest.mark.parametrize("M,N,K,tb", [(200, 136, 160, False), (129, 300, 130, True), (390, 390, 128, "same")])
+def test_accumulation_into_a_view_with_one_allocation(M, N, K, tb, tile):
+    """``c -= a op(b)`` on views; the operands of a product share one block of memory (captured regions pay for each of their own)."""
+    wide = _rand(2, M, N + 12, seed=37)
+    a = _rand(2, M, K + 4, seed=38)[..., :K]
+    b = a if tb == "same" else (_rand(2, N, K + 8, seed=39)[..., 8:] if tb else _rand(2, K, N + 4, seed=39)[..., :N])
+    c = wide[..., 8 : 8 + N]
+    if tb == "same":  # a symmetric product goes onto a symmetric target: upper tiles, mirrored
+        c.copy_(c + c.mT.clone())
+    old = wide.clone()
+    ops.split16_accumulate(c, a, b, bool(tb), -1.0)
+    bt = b.double() if tb else b.double().mT
+    x = a.double() @ bt.mT
+    bound = a.double().abs() @ bt.abs().mT * (2.0**-20 + (K / 16 + 4) * 2.0**-23) + (old[..., 8 : 8 + N].double().abs() + x.abs()) * 2.0**-24
+    assert bool(((c.double() - (old[..., 8 : 8 + N].double() - x)).abs() <= bound).all())
+    assert torch.equal(wide[..., :8], old[..., :8]) and torch.equal(wide[..., 8 + N :], old[..., 8 + N :])
+    count = lambda: torch.cuda.memory_stats()["allocation.all.allocated"]  # noqa: E731
+    before = count()
+    ops.split16_accumulate(c, a, b, bool(tb), -1.0)
+    assert count() - before == 1
+    ac, bc = a.contiguous(), b.contiguous()
+    before = count()
+    ops.matmul16(ac, bc, False, bool(tb))
+    assert count() - before == 2
+    with pytest.raises(RuntimeError):
+        ops.split16_accumulate(ac, ac, bc, bool(tb))
+    ops.check_status()
