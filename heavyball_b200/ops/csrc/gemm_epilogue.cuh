@@ -48,26 +48,44 @@ struct PairOperands {
   int K;
 };
 
-// 32 rows x 16 of K of an operand's matrix (zeros outside it), fetched in the order in which they lie in memory and put down as rows
-__device__ __forceinline__ void fetch_source(float (&v)[16], int lane, const PairOperand& op, int batch, int row0, int rows, int k0, int K) {
-  const bool along_k = op.src_k == 1;
-  const int r = along_k ? lane >> 4 : lane, k = along_k ? lane & 15 : 0;  // of v[0]; v[i] is two rows (along_k) or one k further each time
-  const int64_t step = along_k ? 2 * op.src_row : op.src_k;
-  const float* p = op.src + batch * op.src_batch + (row0 + r) * op.src_row + (k0 + k) * op.src_k;
-  if (row0 + 32 <= rows && k0 + 16 <= K) {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = p[i * step];
-  } else {
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = (row0 + r + (along_k ? 2 * i : 0) < rows && k0 + k + (along_k ? 0 : i) < K) ? p[i * step] : 0.0f;
+// kRows (32 or 16) rows of an operand's matrix, 16 of K at a time (zeros outside it), fetched in the order in which they lie in memory and put
+// down as rows of the stage.
+template <int kRows>
+struct SourceWalk {
+  static constexpr int kValues = kRows / 2;  // a lane's
+  const float* p;         // of this lane's first value
+  int64_t step, advance;  // to its next value; to the next 16 of K
+  int rows, left;         // rows and values of K from here on, as seen from the first value
+  int at, at_step;        // where they go
+  bool along_k;           // a lane's values are two rows (or else one of K) apart
+  __device__ __forceinline__ SourceWalk(const PairOperand& op, int lane, int batch, int row0, int n_rows, int K) {
+    along_k = op.src_k == 1;
+    const int r = along_k ? lane >> 4 : lane & (kRows - 1), k = along_k ? lane & 15 : lane / kRows * kValues;
+    p = op.src + batch * op.src_batch + (row0 + r) * op.src_row + k * op.src_k;
+    step = along_k ? 2 * op.src_row : op.src_k;
+    advance = 16 * op.src_k;
+    rows = n_rows - row0 - r;
+    left = K - k;
+    at = r * kStageLd + k;
+    at_step = along_k ? 2 * kStageLd : 1;
   }
-}
-__device__ __forceinline__ void stage_source(float* stage, const float (&v)[16], int lane, const PairOperand& op) {
-  const bool along_k = op.src_k == 1;
-  float* p = stage + (along_k ? (lane >> 4) * kStageLd + (lane & 15) : lane * kStageLd);
+  __device__ __forceinline__ void fetch(float (&v)[kValues]) {
+    const int n = along_k ? (left > 0 ? (rows + 1) / 2 : 0) : (rows > 0 ? left : 0);  // values inside the matrix
+    if (__all_sync(0xFFFFFFFFu, n >= kValues)) {
 #pragma unroll
-  for (int i = 0; i < 16; ++i) p[i * (along_k ? 2 * kStageLd : 1)] = v[i];
-}
+      for (int i = 0; i < kValues; ++i) v[i] = p[i * step];
+    } else {
+#pragma unroll
+      for (int i = 0; i < kValues; ++i) v[i] = i < n ? p[i * step] : 0.0f;
+    }
+    p += advance;
+    left -= 16;
+  }
+  __device__ __forceinline__ void put(float* stage, const float (&v)[kValues]) const {
+#pragma unroll
+    for (int i = 0; i < kValues; ++i) stage[at + i * at_step] = v[i];
+  }
+};
 
 __device__ __forceinline__ float pow2(int e) { return __uint_as_float((uint32_t)(127 + e) << 23); }
 
@@ -77,19 +95,20 @@ __device__ __forceinline__ uint32_t short_values(float u, bool inside) { return 
 
 constexpr uint32_t kManyShort = 1u << 19;  // counts of short values from here on stand for "any number"
 
-// Entries of the product for blocks with values short of bits or with units whose product may leave the range of fp32, times alpha, into
-// `stage` (row = lane).  `tmem`: the block's accumulators.
+// Accumulators of a block (32 x 32, in tensor memory) with values short of bits or with units whose product may leave the range of fp32 <-
+// entries of the product.
 // A value below 2^-14 in units of its row is held with an error of up to 2^-36 of a unit instead of 22 bits of itself.  With the other
 // operand's values (2^15 at most) and the product of low parts that is left out, n of them bring an error of at most n 2^-20: where the
 // accumulator is 4 n or more, less than 2^-22 of the result.  Smaller accumulators of such rows and columns may consist of nothing else:
 // the block is computed from the matrices themselves, in fp32 arithmetic (subnormals kept), sums of 16 at a time, the next 16 of K on their
 // way meanwhile.  (One such value among ordinary ones, as in one of a hundred thousand rows of 1024 normally distributed values, does not
 // lead there: sums over ordinary values are around 2^25 and more.)
+// Measured, a warp by itself: 1.6 us per 16 of K.  A product half of which comes this way takes twenty times its tf32 time (4 of 2048^3 5.1 ms, 8
+// of 128^3 47 us instead of 14): rare by design, and bound by the latency of the loads.
 // `tri`: entries below the diagonal are zeros whatever the values.
 __device__ __noinline__ void settle_slowly(uint32_t tmem, int lane, float* stage, const PairOperands& P, int batch, int row0, int col0, int M, int N,
-                                           int tri, float alpha) {
+                                           int tri) {
   const float row = P.a.unit[batch * P.a.unit_batch + row0 + lane], col = P.b.unit[batch * P.b.unit_batch + col0 + lane];
-  float* const mine = stage + lane * kStageLd;
   uint32_t acc[32];
   tmem_ld32(tmem, acc);
   tmem_ld_wait();
@@ -106,64 +125,93 @@ __device__ __noinline__ void settle_slowly(uint32_t tmem, int lane, float* stage
 #pragma unroll
     for (int j = 0; j < 32; ++j) {
       const int e = max(-252, min(252, e_row + __shfl_sync(0xFFFFFFFFu, e_mine, j))), half = e >> 1;  // (padding holds anything)
-      mine[j] = __uint_as_float(acc[j]) * pow2(half) * pow2(e - half) * alpha;
+      acc[j] = __float_as_uint(__uint_as_float(acc[j]) * pow2(half) * pow2(e - half));
     }
+    tmem_st32(tmem, acc);
     return;
   }
-  // a lane has rows y + 8 i and columns x + 4 j: twelve loads from the stage for 128 products, no two of a quarter warp in one bank
+  // Half of the columns at a time: with all 32 the registers do not suffice, and what is spilled comes back from the L2 (shared memory leaves
+  // the L1 next to nothing).  A lane has rows y + 8 i and columns x + 4 j: eight loads from the stage for 64 products, no two of a quarter warp in
+  // one bank.
   const int x = lane & 3, y = lane >> 2;
-  float out[4][8], next_a[16], next_b[16];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) out[i][j] = 0.0f;
-  fetch_source(next_a, lane, P.a, batch, row0, M, 0, P.K);
-  fetch_source(next_b, lane, P.b, batch, col0, N, 0, P.K);
+  float kept[4][4];
 #pragma unroll 1
-  for (int k0 = 0; k0 < P.K; k0 += 16) {
-    __syncwarp();
-    stage_source(stage, next_a, lane, P.a);       // columns 0 .. 15 of the stage
-    stage_source(stage + 16, next_b, lane, P.b);  // columns 16 .. 31
-    __syncwarp();
-    if (k0 + 16 < P.K) {
-      fetch_source(next_a, lane, P.a, batch, row0, M, k0 + 16, P.K);
-      fetch_source(next_b, lane, P.b, batch, col0, N, k0 + 16, P.K);
-    }
-    float sum[4][8];
+  for (int half = 0; half < 2; ++half) {
+    float out[4][4], next_a[16], next_b[8];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) sum[i][j] = 0.0f;
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      float a[4][4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) *(float4*)a[i] = *(const float4*)(stage + (y + 8 * i) * kStageLd + q * 4);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float b[4];
-        *(float4*)b = *(const float4*)(stage + (x + 4 * j) * kStageLd + 16 + q * 4);
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-#pragma unroll
-          for (int i = 0; i < 4; ++i) asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum[i][j]) : "f"(a[i][e]), "f"(b[e]));
+      for (int j = 0; j < 4; ++j) out[i][j] = 0.0f;
+    SourceWalk<32> walk_a(P.a, lane, batch, row0, M, P.K);
+    SourceWalk<16> walk_b(P.b, lane, batch, col0 + 16 * half, N, P.K);
+    walk_a.fetch(next_a);
+    walk_b.fetch(next_b);
+#pragma unroll 1
+    for (int left = P.K; left > 0; left -= 16) {
+      __syncwarp();
+      walk_a.put(stage, next_a);       // columns 0 .. 15 of the stage
+      walk_b.put(stage + 16, next_b);  // columns 16 .. 31 of its first 16 rows
+      __syncwarp();
+      if (left > 16) {
+        walk_a.fetch(next_a);
+        walk_b.fetch(next_b);
       }
+      float sum[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) sum[i][j] = 0.0f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        float a[4][4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) *(float4*)a[i] = *(const float4*)(stage + (y + 8 * i) * kStageLd + q * 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          float b[4];
+          *(float4*)b = *(const float4*)(stage + (x + 4 * j) * kStageLd + 16 + q * 4);
+#pragma unroll
+          for (int e = 0; e < 4; ++e)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum[i][j]) : "f"(a[i][e]), "f"(b[e]));
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) asm("add.rn.f32 %0, %0, %1;" : "+f"(out[i][j]) : "f"(sum[i][j]));
+    }
+    __syncwarp();
+    if (half == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) kept[i][j] = out[i][j];
+      continue;
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 8; ++j) asm("add.rn.f32 %0, %0, %1;" : "+f"(out[i][j]) : "f"(sum[i][j]));
+      for (int j = 0; j < 4; ++j) {
+        stage[(y + 8 * i) * kStageLd + x + 4 * j] = kept[i][j];
+        stage[(y + 8 * i) * kStageLd + 16 + x + 4 * j] = out[i][j];
+      }
   }
   __syncwarp();
+  uint32_t settled[32];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) stage[(y + 8 * i) * kStageLd + x + 4 * j] = out[i][j] * alpha;
+  for (int q = 0; q < 8; ++q) {
+    const float4 t = *(const float4*)(stage + lane * kStageLd + q * 4);
+    settled[q * 4] = __float_as_uint(t.x); settled[q * 4 + 1] = __float_as_uint(t.y);
+    settled[q * 4 + 2] = __float_as_uint(t.z); settled[q * 4 + 3] = __float_as_uint(t.w);
+  }
   __syncwarp();
+  tmem_st32(tmem, settled);
 }
 
 // Units of a warp's 32 rows (lane = row) and four blocks of 32 columns (lane = column), fetched while the products are under way; `slow`: the blocks
-// that are not ordinary - some value short of bits, or a unit far from one.
+// that are not ordinary - some value short of bits, or a unit far from one - and are settled in tensor memory before the epilogue proper, which
+// thereby keeps its registers.
 struct BlockUnits {
   float row, col[4];
   uint32_t slow;
@@ -180,7 +228,18 @@ __device__ __forceinline__ BlockUnits fetch_units(const PairOperands& P, int lan
     if (!__all_sync(0xFFFFFFFFu, ordinary_unit(u.row, row0 + lane < M) && ordinary_unit(u.col[cb], col0 + cb * 32 + lane < N))) u.slow |= 1u << cb;
   return u;
 }
-__device__ __forceinline__ float col_unit_of(const BlockUnits& u, int cb) { return cb < 2 ? (cb == 0 ? u.col[0] : u.col[1]) : (cb == 2 ? u.col[2] : u.col[3]); }
+__device__ __forceinline__ void settle_blocks(const BlockUnits& u, uint32_t tmem, int lane, float* stage, const PairOperands& P, int batch, int row0,
+                                              int col0, int M, int N, int tri) {
+#pragma unroll 1
+  for (uint32_t left = u.slow; left != 0; left &= left - 1) {
+    const int cb = __ffs((int)left) - 1;
+    settle_slowly(tmem + (uint32_t)(cb * 32), lane, stage, P, batch, row0, col0 + cb * 32, M, N, tri);
+  }
+}
+__device__ __forceinline__ float row_unit_of(const BlockUnits& u, int cb) { return u.slow >> cb & 1 ? 1.0f : u.row; }
+__device__ __forceinline__ float col_unit_of(const BlockUnits& u, int cb) {
+  return u.slow >> cb & 1 ? 1.0f : cb < 2 ? (cb == 0 ? u.col[0] : u.col[1]) : (cb == 2 ? u.col[2] : u.col[3]);
+}
 
 // Accumulators of an ordinary 32 x 32 block (lane = row) -> entries of the product.
 __device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_unit, float col_unit) {
@@ -191,11 +250,10 @@ __device__ __forceinline__ void unscale32(uint32_t (&acc)[32], float row_unit, f
 // The usual case of the epilogue below: a 32 x 32 block inside the output, C aligned, no split output.  With the mode known at compile
 // time, no bounds to check and all reads in flight before the first use a tile's epilogue is a third as long (8 of 128^3, whole
 // launch: added to C 15.8 -> 9.3 us, symmetric 13.1 -> 7.8, Adam 21.1 -> 12.6, stored in bulk 7.2).
-// `c`, `cm`, `m`, `v`: the block's first element in the output, in its mirror image (null: not stored) and in the moments.  `staged`: the
-// product's entries are in the stage already.
+// `c`, `cm`, `m`, `v`: the block's first element in the output, in its mirror image (null: not stored) and in the moments.
 template <bool kScaled, int kMode>
 __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* stage, const Tf32Epilogue& E, float* c, float* cm, float* m,
-                                               float* v, int64_t ld_state, bool staged, float row_unit, float col_unit) {
+                                               float* v, int64_t ld_state, float row_unit, float col_unit) {
   constexpr bool kOld = kMode == kEpiLerp || kMode == kEpiAdd, kMoments = kMode == kEpiAdam || kMode == kEpiLaProp;
   const int sub = lane >> 3, cg = (lane & 7) * 4;
   float* const mine = stage + lane * kStageLd;
@@ -216,7 +274,7 @@ __device__ __forceinline__ void epilogue_block(uint32_t tmem, int lane, float* s
       pb[i] = *(const float4*)(v + i * sstep);
     }
   }
-  if (!kScaled || !staged) {
+  {
     uint32_t acc[32];
     tmem_ld32(tmem, acc);
     tmem_ld_wait();
@@ -300,12 +358,10 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
 #pragma unroll 1
   for (int cb = 0; cb < n_cb; ++cb) {
     const int col0 = col_base + cb * 32;
-    float col_unit = 1.0f;
-    bool staged = false;
+    float row_unit = 1.0f, col_unit = 1.0f;
     if constexpr (kScaled) {
+      row_unit = row_unit_of(U, cb);
       col_unit = col_unit_of(U, cb);
-      staged = !zero_acc && (U.slow >> cb & 1);
-      if (staged) settle_slowly(tmem_warp + (uint32_t)(cb * 32), lane, stage, P, batch, row0, col0, M, N, E.tri, E.alpha);
     }
     if (!zero_acc && !s_rows && !s_cols && c_vec && E.C != nullptr && row0 + 32 <= M && col0 + 32 <= N && (!moments || state_vec)) {
       const uint32_t t = tmem_warp + (uint32_t)(cb * 32);
@@ -313,15 +369,15 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
       float* cm = mirror ? E.C + b64 * E.strideC + (int64_t)col0 * E.ldc + row0 : nullptr;
       const int64_t st = (b64 * M + row0) * (int64_t)N + col0;
       switch (E.mode) {
-        case kEpiStore: epilogue_block<kScaled, kEpiStore>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, U.row, col_unit); break;
-        case kEpiLerp: epilogue_block<kScaled, kEpiLerp>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, U.row, col_unit); break;
-        case kEpiAdd: epilogue_block<kScaled, kEpiAdd>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, staged, U.row, col_unit); break;
-        case kEpiAdam: epilogue_block<kScaled, kEpiAdam>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, U.row, col_unit); break;
-        default: epilogue_block<kScaled, kEpiLaProp>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, staged, U.row, col_unit); break;
+        case kEpiStore: epilogue_block<kScaled, kEpiStore>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, row_unit, col_unit); break;
+        case kEpiLerp: epilogue_block<kScaled, kEpiLerp>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, row_unit, col_unit); break;
+        case kEpiAdd: epilogue_block<kScaled, kEpiAdd>(t, lane, stage, E, c, cm, nullptr, nullptr, 0, row_unit, col_unit); break;
+        case kEpiAdam: epilogue_block<kScaled, kEpiAdam>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, row_unit, col_unit); break;
+        default: epilogue_block<kScaled, kEpiLaProp>(t, lane, stage, E, c, nullptr, E.m + st, E.v + st, N, row_unit, col_unit); break;
       }
       continue;
     }
-    if (!kScaled || !staged) {
+    {
       uint32_t acc[32];
       if (!zero_acc) {
         tmem_ld32(tmem_warp + (uint32_t)(cb * 32), acc);
@@ -331,7 +387,7 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
         for (int j = 0; j < 32; ++j) acc[j] = 0u;
       }
       if constexpr (kScaled)
-        if (!zero_acc) unscale32(acc, U.row, col_unit);
+        if (!zero_acc) unscale32(acc, row_unit, col_unit);
 #pragma unroll
       for (int q = 0; q < 8; ++q)
         *(float4*)(mine + q * 4) =
@@ -583,29 +639,19 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if constexpr (Kind::kScaled) U = fetch_units(P, lane, batch, tm * TBM + quarter * 32, tn * TBN, M, N);
     const bool have = (num_kb == 0) || mbar_wait(&accum_bar, 0, &abort_flag);
     tc_fence_after();
+    if constexpr (Kind::kScaled)  // (its stage: behind what the epilogues use)
+      if (have && num_kb != 0 && U.slow != 0)
+        settle_blocks(U, tmem_base + ((uint32_t)(quarter * 32) << 16), lane, (float*)(tiles + (TBN / 32) * kTTileBytes + quarter * kStageWarpBytes), P,
+                      batch, tm * TBM + quarter * 32, tn * TBN, M, N, E.tri);
     if (have && bulk_store) {
       // every load has landed and every MMA has retired: the ring is free and stages the output tile as four
       // [128 rows x 32 fp32] boxes in the swizzled layout the bulk store expects
 #pragma unroll 1
       for (int cb = 0; cb < TBN / 32; ++cb) {
         uint32_t acc[32];
-        const uint32_t t = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32);
-        if constexpr (Kind::kScaled) {
-          if (U.slow >> cb & 1) {
-            float* const stage = (float*)(tiles + (TBN / 32) * kTTileBytes + quarter * kStageWarpBytes);  // behind the boxes
-            settle_slowly(t, lane, stage, P, batch, tm * TBM + quarter * 32, tn * TBN + cb * 32, M, N, 0, 1.0f);
-#pragma unroll
-            for (int j = 0; j < 32; ++j) acc[j] = __float_as_uint(stage[lane * kStageLd + j]);
-            __syncwarp();
-          } else {
-            tmem_ld32(t, acc);
-            tmem_ld_wait();
-            unscale32(acc, U.row, col_unit_of(U, cb));
-          }
-        } else {
-          tmem_ld32(t, acc);
-          tmem_ld_wait();
-        }
+        tmem_ld32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(cb * 32), acc);
+        tmem_ld_wait();
+        if constexpr (Kind::kScaled) unscale32(acc, row_unit_of(U, cb), col_unit_of(U, cb));
         uint8_t* box = tiles + cb * kTTileBytes;
 #pragma unroll
         for (int q = 0; q < 8; ++q)
@@ -781,6 +827,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       // a tile on the diagonal: computed whole, or (symmetric == 2) as three of 128 x 128 whose middle one is mirrored
       const bool thirds = E.symmetric == 2 && t.tm == t.tn;
       const bool mirrored = thirds ? rank == 0 && half == 1 : t.tm != t.tn;
+      if constexpr (Kind::kScaled)
+        if (U.slow != 0 && walk_tile(t, kp, E.tri, Kind::kBlock).seg != 0)
+          settle_blocks(U, tmem_warp + (uint32_t)(acc * 256), lane, stage, P, t.batch, row0, col0, M, N, E.tri);
       if (row0 < M && blocks > 0 && !(thirds && rank == 1 && half == 0))
         epilogue_direct<Kind::kScaled>(tmem_warp + (uint32_t)(acc * 256), lane, stage, row0, col0, blocks, mirrored,
                               walk_tile(t, kp, E.tri, Kind::kBlock).seg == 0, t.batch, M, N, E, P, U);
