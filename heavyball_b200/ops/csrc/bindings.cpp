@@ -915,6 +915,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("ns_orthogonalize", &ns_orthogonalize);
   m.def("set_ns_gemm_tile", &hb::set_ns_gemm_tile_override);
   m.def("set_tf32_gemm_tile", &hb::set_tf32_gemm_tile_override);
+  m.def("tf32_gemm_tiles", [](int M, int N, int K, int batch, bool symmetric) {
+    int choice = 0;
+    check(hb::tf32_gemm_tiles(M, N, K, batch, symmetric, &choice), "tf32 tile choice");
+    return choice;
+  });
   m.def("chol_inv_leaf", &chol_inv_leaf);
   m.def("triu_pack", &triu_pack);
   m.def("triu_unpack", &triu_unpack);

@@ -147,17 +147,30 @@ static int g_tf32_tile_override = 0;  // 0 = by size, 128 / 256 = forced (tests 
 int tf32_gemm_tile_override() { return g_tf32_tile_override; }
 void set_tf32_gemm_tile_override(int tile) { g_tf32_tile_override = (tile == 128 || tile == 256) ? tile : 0; }
 
+// Pairs of CTAs that can be resident at once on the current device; also sets the kernels' shared memory up there.
+static cudaError_t resident_pairs(int* out) {
+  static PerDevice<int> pairs;
+  int device = 0;
+  const cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  return pairs.get(device, cudaSuccess, out, [](int& found) {
+    cudaError_t s = cudaFuncSetAttribute(gemm128_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
+    if (s == cudaSuccess) s = cudaFuncSetAttribute(gemm_pair_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGPairSmemBytes);
+    return s != cudaSuccess ? s : max_resident_pairs(gemm_pair_kernel<Tf32Kind>, kGPairThreads, kGPairSmemBytes, &found);
+  });
+}
+
+cudaError_t tf32_gemm_tiles(int M, int N, int K, int batch, int symmetric, int* choice) {
+  int max_pairs = 0;
+  const cudaError_t e = resident_pairs(&max_pairs);
+  if (e == cudaSuccess) *choice = tf32_tiles(M, N, K, batch, symmetric != 0, max_pairs);
+  return e;
+}
+
 cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int K, int batch, const Tf32Epilogue& E,
                              int* status, cudaStream_t stream) {
-  static PerDevice<int> pairs;
-  int device = 0, max_pairs = 0;
-  cudaError_t e = cudaGetDevice(&device);
-  if (e == cudaSuccess)
-    e = pairs.get(device, cudaSuccess, &max_pairs, [](int& found) {
-      cudaError_t s = cudaFuncSetAttribute(gemm128_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTSmemBytes);
-      if (s == cudaSuccess) s = cudaFuncSetAttribute(gemm_pair_kernel<Tf32Kind>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGPairSmemBytes);
-      return s != cudaSuccess ? s : max_resident_pairs(gemm_pair_kernel<Tf32Kind>, kGPairThreads, kGPairSmemBytes, &found);
-    });
+  int max_pairs = 0;
+  const cudaError_t e = resident_pairs(&max_pairs);
   if (e != cudaSuccess) return e;
   if (M == 0 || N == 0 || batch == 0) return cudaSuccess;
   if ((E.mode == kEpiAdam || E.mode == kEpiLaProp) && (E.m == nullptr || E.v == nullptr)) return cudaErrorInvalidValue;

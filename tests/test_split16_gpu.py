@@ -111,6 +111,70 @@ def test_symmetric_split_tf32_has_the_bits_of_small_tiles(mode, B, n, K):
     assert torch.equal(*results)
 
 
+@pytest.mark.parametrize("B,n,K,tiles", [(2, 1300, 4096, 2), (2, 1537, 1025, 2), (4, 1536, 256, 2), (4, 1536, 255, 0), (7, 1280, 512, 1)])
+def test_updates_of_symmetric_views_by_either_tile_of_split_tf32(B, n, K, tiles):
+    """Schur complements: subtracted from a view, the tile that the sizes ask for against 128 x 128 tiles."""
+    ext, x, old = ops.load(), _rand(B, n, K, seed=40), _rand(B, n, n, seed=41)
+    assert ext.tf32_gemm_tiles(n, n, K, B, True) == tiles
+    old, op = old + old.mT, ops.tf32_split(x, True, False)[0]
+    results = []
+    for forced in (0, 128):
+        ext.set_tf32_gemm_tile(forced)
+        wide = torch.full((B, n + 4, n + 12), -7.0, device="cuda")
+        out = wide[:, 4:, 8 : 8 + n].copy_(old)
+        ops.tf32_gemm(op, op, K, mode=ops.EPI_ADD, alpha=-1.0, out=out)
+        results.append(out)
+        assert bool((wide[:, :4] == -7.0).all() and (wide[..., :8] == -7.0).all() and (wide[..., 8 + n :] == -7.0).all())
+    ext.set_tf32_gemm_tile(0)
+    ops.check_status()
+    # 22 bits of either operand and the dropped product, the accumulator rounded once per 8 of K in each of three walks (2^-23), and the sum with
+    # the target; kPairTiles (1) computes what small tiles mirror next to the diagonal, so last bits may differ there
+    x64 = x.double() @ x.double().mT
+    bound = (x.double().abs() @ x.double().abs().mT) * (2.0**-20 + 3 * K / 8 * 2.0**-23) + (old.double().abs() + x64.abs()) * 2.0**-23
+    assert bool(((results[0].double() - (old.double() - x64)).abs() <= bound).all())
+    assert torch.equal(*results) if tiles != 1 else bool(((results[0] - results[1]).abs() <= 2 * bound).all())
+
+
+@pytest.mark.parametrize("B,M,N,K", [(3, 1800, 2100, 130), (1, 5000, 3000, 64), (2, 2300, 2304, 200)])
+@pytest.mark.parametrize("mode", ["store", "add", "adam"])
+def test_pairs_of_ctas_with_several_tiles_each(mode, B, M, N, K):
+    """More 256 x 256 tiles than resident pairs: both accumulators, the ring across tiles, the epilogue under the next main loop."""
+    assert B * -(-M // 256) * -(-N // 256) > 148
+    a, b, out = _rand(B, M, K, seed=42), _rand(B, N, K, seed=43), _rand(B, M, N, seed=44)
+    a[0, 5] *= 1e-12  # one row in units of its own
+    pa, pb, old = ops.split16(a)[0], ops.split16(b)[0], out.clone()
+    m, v = torch.zeros_like(out), torch.zeros_like(out)
+    kwargs = {"store": {}, "add": dict(mode=ops.EPI_ADD, alpha=-1.0), "adam": dict(mode=ops.EPI_ADAM, b1=0.5, b2c=0.5, eps=1e-30, m=m, v=v)}[mode]
+    results = []
+    for forced in (256, 128):
+        ops.load().set_split16_gemm_tile(forced)
+        ops.split16_gemm(pa, pb, out=out, **kwargs)
+        results.append([t.clone() for t in (out, m, v)])
+        out.copy_(old), m.zero_(), v.zero_()
+    ops.load().set_split16_gemm_tile(0)
+    ops.check_status()
+    assert all(torch.equal(x, y) for x, y in zip(*results))  # one accumulator per entry and the same walk over K
+    if mode == "store":
+        assert _off(results[0][0], a.double(), b.double()) < 1
+
+
+@pytest.mark.parametrize("B,n,K", [(2, 520, 200), (7, 1300, 130)])
+@pytest.mark.parametrize("mode", ["lerp", "add"])
+def test_symmetric_updates_of_fp16_pairs(mode, B, n, K, tile):
+    """Onto a symmetric target that is a view, upper tiles mirrored; the second size gives a pair of CTAs more than one tile."""
+    x, old = _rand(B, n, K, seed=45), _rand(B, n, n, seed=46)
+    old, op = old + old.mT, ops.split16(x)[0]
+    out = torch.empty(B, n, n + 4, device="cuda")[..., :n].copy_(old)
+    kwargs = dict(mode=ops.EPI_LERP, w=0.25) if mode == "lerp" else dict(mode=ops.EPI_ADD, alpha=-1.0)
+    ops.split16_gemm(op, op, out=out, **kwargs)
+    ops.check_status()
+    x64 = x.double() @ x.double().mT
+    want = old.double() * 0.75 + 0.25 * x64 if mode == "lerp" else old.double() - x64
+    # the product's bound and three roundings in fp32 of values up to |old| + |x|
+    bound = (x.double().abs() @ x.double().abs().mT) * (2.0**-20 + (K / 16 + 4) * 2.0**-23) + (old.double().abs() + x64.abs()) * 2.0**-22
+    assert bool(((out.double() - want).abs() <= bound).all())
+
+
 def test_ranges_that_fp16_does_not_have(tile):
     """Rows over sixty decades, rows of zeros, of subnormals and with an infinity or a NaN next to ordinary ones."""
     a, b = _rand(1, 300, 96, seed=12), _rand(1, 140, 96, seed=13)
