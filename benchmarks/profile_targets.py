@@ -11,7 +11,7 @@
     python benchmarks/profile_targets.py split16_small   # the same product of fp16 pairs
     python benchmarks/profile_targets.py qr_small        # panel-wise Cholesky QR of 8 x (1024 x 1024), eager launches
     python benchmarks/profile_targets.py ns_big          # Newton-Schulz on 4 x (4096 x 4096): the 256 x 256-tile kernel
-    python benchmarks/profile_targets.py soap_small      # one plain SOAP step on 8 x 1024^2 (tf32 GEMMs with fused epilogues)
+    python benchmarks/profile_targets.py soap_small      # one plain SOAP step on 8 x 1024^2 (fp16-pair GEMMs with fused epilogues, split-tf32 statistics)
     python benchmarks/profile_targets.py psgd_small      # one plain PSGDKron step on 8 x 1024^2 (cached P = Q^T Q operands)
     python benchmarks/profile_targets.py psgd_fit        # one PSGDKron step with a preconditioner fit, 8 x (1024 x 4096)
     python benchmarks/profile_targets.py soap_refresh    # one SOAP step with an eigenbasis refresh, 8 x (2048 x 2048)

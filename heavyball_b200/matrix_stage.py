@@ -12,9 +12,10 @@ of them.  ``optimizer.state`` (and so ``state_dict()``) still shows tensors of t
 arithmetic is in place on the batched tensors, and nothing is copied per step.  If the entries are replaced from
 outside (``load_state_dict``), the next step notices the changed addresses and adopts again.
 
-Products.  Every product is written against a small operand interface with two backends: the split-tf32 tensor-core
+Products.  Every product is written against a small operand interface with two backends: the fp16-pair tensor-core
 GEMM of ``ops`` (fp32-level accuracy, element-wise stages fused into GEMM epilogues, rarely-changing matrices kept
-in split form between refreshes) and plain ``torch`` matmuls (CPU, small matrices, and the oracle in tests).
+as operands between refreshes; statistics on split tf32) and plain ``torch`` matmuls (CPU, small matrices, and the
+oracle in tests).
 
 Math restated from ``heavyball_b200.utils.soap`` / ``utils.psgd`` (parity targets ``heavyball/chainable.py:1257-1276,
 1531-1621`` and ``heavyball/utils.py:829-900, 1205-1259, 1391-1411, 3084-3122, 3557-3576``).

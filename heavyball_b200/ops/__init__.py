@@ -10,7 +10,8 @@ Entry points
 ``sumsq``            per-tensor sum of squares (segmented reduction)
 ``dot`` / ``absmax`` per-tensor dot products and absolute maxima (same chunk table)
 ``newton_schulz``    batched quintic Newton–Schulz / Polar-Express chain on tcgen05 tensor cores
-``matmul3``          fp32 matrix product on the tf32 tensor cores (3-term split), for SOAP / PSGD algebra
+``matmul3``          fp32 matrix product on the tf32 tensor cores (3-term split), for what eigenbases are made of
+``matmul16``         fp32 matrix product from pairs of fp16 numbers, for SOAP's projections and PSGD
 ``nn``               (sub-module) model-side ops: fused head + cross-entropy, LayerNorm (+ residual add), Linear with
                      column-sum bias gradients, bf16 cast cache
 ``noalloc``          (sub-module) ctypes access to the allocation-free AdamW entry point

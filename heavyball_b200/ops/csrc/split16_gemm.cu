@@ -3,14 +3,17 @@
 // The 3-term split product of tf32_gemm.cu with fp16 in the place of tf32: both carry 11 significant bits, so hi + lo keep 22 bits
 // of a value either way, but fp16 operands are half as wide and their products run at twice the rate.  What fp16 lacks is range,
 // hence one power of two per operand row that takes the row's largest value to the top of it and comes off again in the epilogue
-// (exact both ways).  Values down to 2^-29 of their row's largest keep all 22 bits; below that the error is 2^-51 of the largest,
-// far under the rounding of any sum in which both take part.
+// (exact both ways).  Values down to 2^-29 of their row's largest keep all 22 bits; below that the error is 2^-51 of the largest:
+// far under the rounding of any sum in which both take part, but everything to a result that the largest has no part in (because it meets a
+// zero, in triangular or block-diagonal factors).  The operand pass counts such values per row, the epilogue finds the results that may hang
+// on them and computes those from the matrices (settle_slowly in gemm_epilogue.cuh).  Subnormal values are scaled like others.
 //
 // Three walks over K share one fp32 accumulator: hi lo^T and lo hi^T first, with lo stored times 2^11 (so that small values keep it,
 // too), then hi hi^T on top, whose first instruction takes 2^-11 off the accumulator (the scale-input-d operand of tcgen05.mma).  The
 // large sum is rounded once per 16 of K that way; with the high parts first, as tf32 walks them, the two small sums would be rounded
 // at its magnitude as well.  Error against 64 bits, relative 2-norm, K = 1024 / 2048 / 8192: 1.2e-6 / 2.5e-6 / 9.7e-6 (tf32: 1.1e-5 /
-// 2.1e-5 / 8.4e-5), the same with rows over thirty decades and with entries over eight decades along K.
+// 2.1e-5 / 8.4e-5), the same with rows over thirty decades and with entries over eight decades along K.  Entry by entry, whatever the range:
+// 2^-20 + (K / 16 + 4) 2^-23 of |A| |B|^T, tested over thirty decades along K opposite zeros.
 //
 // Measured on one B200, of measured peak (1.64 PFLOP/s / 3): 2 of 5504 x 2048 x 2048 205 us = 451 TFLOP/s, 0.82 (split tf32 340 us);
 // 4 of 2048^3 159 us = 431, 0.79 (265); 8 of 1024^3 50 us = 346, 0.63, one wave (76).
@@ -49,7 +52,8 @@ struct HalfKind {
 //                            column maxima -> `trans`, turned through shared memory
 // What both saw first stays in registers (1024 columns of a row, 256 rows of a strip); only longer ones are read again, from L1 or L2.
 // Bound by memory: 4 of 2048^2 rows 24 us (5.6 TB/s; split tf32, twice the bytes out, 37), columns 38 us, both 50 (59); one block per
-// strip of 16 columns instead of a cluster 70 us for the columns.
+// strip of 16 columns instead of a cluster 70 us for the columns.  Watching the smallest value costs the columns 4 % (43 -> 45 us from a cold
+// L2), the rows nothing; counting every value as it is converted cost 9 %.
 constexpr int kSplitThreads = 256;
 constexpr int kRowChunk = 1024;
 constexpr int kStrip = 32, kStripRows = 256, kMaxSplitCluster = 8;

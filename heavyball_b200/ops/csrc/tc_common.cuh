@@ -31,9 +31,8 @@ __device__ inline bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 // True in one lane of a (converged) warp.  The roles that issue loads and products are guarded by this rather than by the lane's number:
-// the compiler knows then that one thread runs, and keeps descriptors and barrier addresses in uniform registers.  Behind `lane == 0`
-// it moves each of them over for every instruction, and the issuing thread, not the tensor core, set the pace of a main loop (720 cycles
-// per 256 x 256 x 64 block of bf16 on a pair of CTAs, with the loads or without; 562 this way, 512 at the full rate).
+// behind `lane == 0` the issuing thread, not the tensor core, set the pace of a main loop (720 cycles per 256 x 256 x 64 block of bf16 on a
+// pair of CTAs, with the loads or without; 562 this way, 512 at the full rate).
 __device__ inline bool elect_one() {
   uint32_t p;
   asm volatile("{\n\t.reg .pred P;\n\telect.sync _|P, 0xffffffff;\n\tselp.u32 %0, 1, 0, P;\n\t}" : "=r"(p));

@@ -13,14 +13,10 @@
 // rounding of the tensor core's accumulator.  One split buffer serves as either operand, so a symmetric product
 // X X^T needs one split of X, and matrices that change rarely (eigenbases, preconditioner factors) stay split.
 //
-// GEMM kernel (one 128x128 output tile per CTA, 192 threads, two CTAs per SM):
-//   warp 0     : TMA producer, cp.async.bulk.tensor 3-D loads (128-byte swizzle, 32 fp32 per row) into a 3-stage ring
-//   warp 1     : tcgen05.mma.cta_group::1.kind::tf32, 128x128x8 per instruction, accumulator in 128 TMEM columns
-//   warps 2..5 : tcgen05.ld, then the epilogue.  Plain stores go through the (now idle) ring and four bulk tensor
-//                stores.  Fused epilogues work in registers and store directly: scale; lerp into the statistics
-//                matrix (GG <- lerp(GG, G G^T)); Adam / LaProp in the eigenbasis (moments read and written in
-//                place, the preconditioned value goes on); and, for any of them, the result written in the split
-//                [hi | lo] layout - as it is or transposed - so the next product of the chain needs no split pass.
+// Kernels and epilogues: gemm_epilogue.cuh; which tile when: gemm_rules.h.  SOAP's statistics and refresh run on this product (lerp into the
+// statistics matrix; added to a view for Schur complements and solves), projections and PSGD on that of split16_gemm.cu.  Adam / LaProp on moment
+// buffers, a result written as a split operand - as it is or transposed - and products of upper-triangular matrices are here for callers of
+// ops.tf32_gemm and ops.matmul3.
 // Waits are bounded as in the bf16 kernels: on expiry the CTA flags `status`, drains, frees TMEM and returns.
 #include "tf32_gemm.h"
 

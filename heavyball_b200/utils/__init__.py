@@ -10,7 +10,7 @@ switches, which are read at call time:
 * ``fast_qr`` — on CUDA, orthogonalise eigenbasis refreshes with batched panel-wise Cholesky QR instead of Householder QR
 * ``graph_qr`` — replay that QR from a CUDA graph per shape (several hundred small launches otherwise)
 * ``tensor_core_matmul`` — on sm_100a, fp32 matrix products of SOAP / PSGD with all dimensions >= 128 use the
-  tensor-core kernels for products of fp16 pairs (error about 2^-20 of ``|a| @ |b|``) or, for what eigenbases are made of,
+  tensor-core kernels for products of fp16 pairs (error about 2^-20 of ``|a| @ |b|``, entry by entry and over any range) or, for what eigenbases are made of,
   split tf32 (2^-18) instead of fp32 SIMT library GEMMs
 * ``compile_mode`` / ``dynamic`` / ``compile_mode_recommended_to_none`` — accepted for source
   compatibility; there is no tracing compiler here, fused execution is done by the sm_100a kernels

@@ -11,7 +11,8 @@ The work models restate what each optimizer has to do at minimum:
 * Newton-Schulz on an ``m x n`` matrix (``m <= n``), ``steps`` iterations: ``steps * (4 m^2 n + 2 m^3)`` FLOPs as the
   reference computes it (``heavyball/utils.py:568-573``), ``steps * (3 m^2 n + m^3)`` when the symmetry of ``X X^T`` and
   of the polynomial is used;
-* fp32-accurate products on the tf32 tensor cores cost three tf32 passes.
+* fp32-accurate products on the tensor cores cost three passes over operands of 11 bits: at the bf16 rate as fp16 pairs, at half of it as
+  split tf32.
 """
 
 from __future__ import annotations
