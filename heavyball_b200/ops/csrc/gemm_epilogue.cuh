@@ -48,42 +48,61 @@ struct PairOperands {
   int K;
 };
 
-// kRows (32 or 16) rows of an operand's matrix, 16 of K at a time (zeros outside it), fetched in the order in which they lie in memory and put
-// down as rows of the stage.
+// kRows (32 or 16) rows of an operand's matrix, 16 of K at a time (zeros outside it), fetched in the order in which they lie in memory - four
+// neighbours at once where they are aligned - and put down as rows of the stage.
 template <int kRows>
 struct SourceWalk {
-  static constexpr int kValues = kRows / 2;  // a lane's
-  const float* p;         // of this lane's first value
-  int64_t step, advance;  // to its next value; to the next 16 of K
-  int rows, left;         // rows and values of K from here on, as seen from the first value
-  int at, at_step;        // where they go
-  bool along_k;           // a lane's values are two rows (or else one of K) apart
+  static constexpr int kPieces = kRows / 8;        // a lane's, of four values
+  static constexpr int kAcross = kRows / 4;        // not along_k: lanes side by side along the rows
+  static constexpr int kStep = 32 / kAcross;       // ... whose pieces are that many of K apart
+  const float* p;              // of this lane's first value
+  int64_t one, piece, advance;  // to the next value of a piece, to the next piece, to the next 16 of K
+  int rows, left;              // rows and values of K from the first value on
+  int at;                      // where it goes
+  bool along_k, wide;
   __device__ __forceinline__ SourceWalk(const PairOperand& op, int lane, int batch, int row0, int n_rows, int K) {
     along_k = op.src_k == 1;
-    const int r = along_k ? lane >> 4 : lane & (kRows - 1), k = along_k ? lane & 15 : lane / kRows * kValues;
+    const int r = along_k ? lane >> 2 : lane % kAcross * 4, k = along_k ? (lane & 3) * 4 : lane / kAcross;
     p = op.src + batch * op.src_batch + (row0 + r) * op.src_row + k * op.src_k;
-    step = along_k ? 2 * op.src_row : op.src_k;
+    one = along_k ? 1 : op.src_row;
+    piece = along_k ? 8 * op.src_row : kStep * op.src_k;
     advance = 16 * op.src_k;
     rows = n_rows - row0 - r;
     left = K - k;
     at = r * kStageLd + k;
-    at_step = along_k ? 2 * kStageLd : 1;
+    const int64_t between = along_k ? op.src_row : op.src_k;
+    wide = one == 1 && (between & 3) == 0 && (op.src_batch & 3) == 0 && ((uintptr_t)op.src & 15) == 0;
   }
-  __device__ __forceinline__ void fetch(float (&v)[kValues]) {
-    const int n = along_k ? (left > 0 ? (rows + 1) / 2 : 0) : (rows > 0 ? left : 0);  // values inside the matrix
-    if (__all_sync(0xFFFFFFFFu, n >= kValues)) {
+  __device__ __forceinline__ void fetch(float4 (&v)[kPieces]) {
+    const bool inside = along_k ? rows > 8 * (kPieces - 1) && left >= 4 : rows >= 4 && left > kStep * (kPieces - 1);
+    if (__all_sync(0xFFFFFFFFu, wide && inside)) {
 #pragma unroll
-      for (int i = 0; i < kValues; ++i) v[i] = p[i * step];
+      for (int i = 0; i < kPieces; ++i) v[i] = *(const float4*)(p + i * piece);
     } else {
 #pragma unroll
-      for (int i = 0; i < kValues; ++i) v[i] = i < n ? p[i * step] : 0.0f;
+      for (int i = 0; i < kPieces; ++i) {
+        const int n = along_k ? (rows > 8 * i ? left : 0) : (left > kStep * i ? rows : 0);  // values of the piece that are inside
+        const float* q = p + i * piece;
+        v[i] = make_float4(n > 0 ? q[0] : 0.0f, n > 1 ? q[one] : 0.0f, n > 2 ? q[2 * one] : 0.0f, n > 3 ? q[3 * one] : 0.0f);
+      }
     }
     p += advance;
     left -= 16;
   }
-  __device__ __forceinline__ void put(float* stage, const float (&v)[kValues]) const {
+  __device__ __forceinline__ void put(float* stage, const float4 (&v)[kPieces]) const {
+    float* s = stage + at;
+    if (along_k) {
 #pragma unroll
-    for (int i = 0; i < kValues; ++i) stage[at + i * at_step] = v[i];
+      for (int i = 0; i < kPieces; ++i) *(float4*)(s + 8 * i * kStageLd) = v[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < kPieces; ++i, s += kStep) {
+        s[0] = v[i].x;
+        s[kStageLd] = v[i].y;
+        s[2 * kStageLd] = v[i].z;
+        s[3 * kStageLd] = v[i].w;
+      }
+    }
   }
 };
 
@@ -131,13 +150,13 @@ __device__ __noinline__ void settle_slowly(uint32_t tmem, int lane, float* stage
     return;
   }
   // Half of the columns at a time: with all 32 the registers do not suffice, and what is spilled comes back from the L2 (shared memory leaves
-  // the L1 next to nothing).  A lane has rows y + 8 i and columns x + 4 j: eight loads from the stage for 64 products, no two of a quarter warp in
-  // one bank.
+  // the L1 next to nothing).  A lane has rows y + 8 i and columns x + 4 j, even and odd k in the halves of one register pair: eight loads from the
+  // stage for 64 products in 32 instructions, no two of a quarter warp in one bank.
   const int x = lane & 3, y = lane >> 2;
-  float kept[4][4];
 #pragma unroll 1
   for (int half = 0; half < 2; ++half) {
-    float out[4][4], next_a[16], next_b[8];
+    float out[4][4];
+    float4 next_a[4], next_b[2];
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -156,57 +175,50 @@ __device__ __noinline__ void settle_slowly(uint32_t tmem, int lane, float* stage
         walk_a.fetch(next_a);
         walk_b.fetch(next_b);
       }
-      float sum[4][4];
+      unsigned long long sum[4][4];  // two floats each
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) sum[i][j] = 0.0f;
+        for (int j = 0; j < 4; ++j) sum[i][j] = 0ull;
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
-        float a[4][4];
+        ulonglong2 a[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) *(float4*)a[i] = *(const float4*)(stage + (y + 8 * i) * kStageLd + q * 4);
+        for (int i = 0; i < 4; ++i) a[i] = *(const ulonglong2*)(stage + (y + 8 * i) * kStageLd + q * 4);
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          float b[4];
-          *(float4*)b = *(const float4*)(stage + (x + 4 * j) * kStageLd + 16 + q * 4);
+          const ulonglong2 b = *(const ulonglong2*)(stage + (x + 4 * j) * kStageLd + 16 + q * 4);
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
+          for (int i = 0; i < 4; ++i) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[i][j]) : "l"(a[i].x), "l"(b.x));
 #pragma unroll
-            for (int i = 0; i < 4; ++i) asm("fma.rn.f32 %0, %1, %2, %0;" : "+f"(sum[i][j]) : "f"(a[i][e]), "f"(b[e]));
+          for (int i = 0; i < 4; ++i) asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[i][j]) : "l"(a[i].y), "l"(b.y));
         }
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) asm("add.rn.f32 %0, %0, %1;" : "+f"(out[i][j]) : "f"(sum[i][j]));
+        for (int j = 0; j < 4; ++j) {
+          float both = __uint_as_float((uint32_t)sum[i][j]);
+          asm("add.rn.f32 %0, %0, %1;" : "+f"(both) : "f"(__uint_as_float((uint32_t)(sum[i][j] >> 32))));
+          asm("add.rn.f32 %0, %0, %1;" : "+f"(out[i][j]) : "f"(both));
+        }
     }
     __syncwarp();
-    if (half == 0) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) kept[i][j] = out[i][j];
-      continue;
-    }
 #pragma unroll
     for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        stage[(y + 8 * i) * kStageLd + x + 4 * j] = kept[i][j];
-        stage[(y + 8 * i) * kStageLd + 16 + x + 4 * j] = out[i][j];
-      }
-  }
-  __syncwarp();
-  uint32_t settled[32];
+      for (int j = 0; j < 4; ++j) stage[(y + 8 * i) * kStageLd + x + 4 * j] = out[i][j];
+    __syncwarp();
+    uint32_t settled[16];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const float4 t = *(const float4*)(stage + lane * kStageLd + q * 4);
-    settled[q * 4] = __float_as_uint(t.x); settled[q * 4 + 1] = __float_as_uint(t.y);
-    settled[q * 4 + 2] = __float_as_uint(t.z); settled[q * 4 + 3] = __float_as_uint(t.w);
+    for (int q = 0; q < 4; ++q) {
+      const float4 t = *(const float4*)(stage + lane * kStageLd + q * 4);
+      settled[q * 4] = __float_as_uint(t.x); settled[q * 4 + 1] = __float_as_uint(t.y);
+      settled[q * 4 + 2] = __float_as_uint(t.z); settled[q * 4 + 3] = __float_as_uint(t.w);
+    }
+    tmem_st16(tmem + 16u * (uint32_t)half, settled);
   }
   __syncwarp();
-  tmem_st32(tmem, settled);
 }
 
 // Units of a warp's 32 rows (lane = row) and four blocks of 32 columns (lane = column), fetched while the products are under way; `slow`: the blocks
