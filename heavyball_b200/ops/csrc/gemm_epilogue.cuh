@@ -122,8 +122,10 @@ constexpr uint32_t kManyShort = 1u << 19;  // counts of short values from here o
 // the block is computed from the matrices themselves, in fp32 arithmetic (subnormals kept), sums of 16 at a time, the next 16 of K on their
 // way meanwhile.  (One such value among ordinary ones, as in one of a hundred thousand rows of 1024 normally distributed values, does not
 // lead there: sums over ordinary values are around 2^25 and more.)
-// Measured, a warp by itself: 1.6 us per 16 of K.  A product half of which comes this way takes twenty times its tf32 time (4 of 2048^3 5.1 ms, 8
-// of 128^3 47 us instead of 14): rare by design, and bound by the latency of the loads.
+// Measured, a warp by itself: 1.3 us per 16 of K, most of it the latency of the loads (a second step of prefetch, in registers or by cp.async, was
+// slower: spills, and more instructions than it hides).  A product half of which comes this way takes sixteen times its tf32 time (4 of 2048^3
+// 4.3 ms, 8 of 128^3 43 us instead of 14); steps on 4 of 2048 x 1024 with half of the gradient's rows 1e-14 of the others, against split tf32:
+// PSGD with a fit 6.6 / 3.7 ms, SOAP without refresh 5.1 / 1.2 (ordinary gradients 2.8 / 3.6 and 0.9 / 1.1).
 // `tri`: entries below the diagonal are zeros whatever the values.
 __device__ __noinline__ void settle_slowly(uint32_t tmem, int lane, float* stage, const PairOperands& P, int batch, int row0, int col0, int M, int N,
                                            int tri) {
@@ -711,8 +713,8 @@ constexpr int kGPairEpiWarps = 8;
 constexpr int kGPairThreads = 64 + 32 * kGPairEpiWarps;
 constexpr int kGPairSmemBytes = kGPairStages * kGPairStageBytes + kGPairEpiWarps * kStageWarpBytes + 1024;
 
-// Epilogues of scaled operands may compute blocks from the matrices (16 ms for a tile's column of 2^17 of K), and everything in the pair waits for
-// them.
+// Epilogues of scaled operands may compute blocks from the matrices (65 ms for a tile all of whose blocks are, at K = 2^17), and everything in the
+// pair waits for them; 2^18 polls last around 10 ms.
 constexpr uint32_t kLongSpinLimit = kSpinLimit << 5;
 
 struct WalkTile {
