@@ -41,19 +41,24 @@ struct Philox {
   uint32_t k0, k1;
   __device__ Philox(uint64_t seed) : k0((uint32_t)seed), k1((uint32_t)(seed >> 32)) {}
   __device__ inline uint4 operator()(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) const {
+    uint4 r[1] = {make_uint4(c0, c1, c2, c3)};
+    rounds(r);
+    return r[0];
+  }
+  // Counters -> random bits.  A round waits for the one before; several draws of a thread side by side fill those waits.
+  template <int N>
+  __device__ __forceinline__ void rounds(uint4 (&c)[N]) const {
     uint32_t a = k0, b = k1;
 #pragma unroll
     for (int i = 0; i < 10; ++i) {
-      uint32_t hi0 = __umulhi(0xD2511F53u, c0), lo0 = 0xD2511F53u * c0;
-      uint32_t hi1 = __umulhi(0xCD9E8D57u, c2), lo1 = 0xCD9E8D57u * c2;
-      c0 = hi1 ^ c1 ^ a;
-      c1 = lo1;
-      c2 = hi0 ^ c3 ^ b;
-      c3 = lo0;
+#pragma unroll
+      for (int n = 0; n < N; ++n) {
+        const uint64_t p0 = (uint64_t)0xD2511F53u * c[n].x, p1 = (uint64_t)0xCD9E8D57u * c[n].z;
+        c[n] = make_uint4((uint32_t)(p1 >> 32) ^ c[n].y ^ a, (uint32_t)p1, (uint32_t)(p0 >> 32) ^ c[n].w ^ b, (uint32_t)p0);
+      }
       a += 0x9E3779B9u;
       b += 0xBB67AE85u;
     }
-    return make_uint4(c0, c1, c2, c3);
   }
 };
 

@@ -387,16 +387,24 @@ __device__ __forceinline__ F4 apply_rule(const ChainParams& P, const F4& u, F4& 
   return out;
 }
 
-template <int DTP, int DTG, int DTU, int DTS, int OUT, int UIN, bool COUNT>
+// RULE: one moment rule, with or without MARS, known at compile time (kAnyRule: whatever the launch asks for).
+constexpr int kAnyRule = -1;
+constexpr int rule_states(int rule) { return rule == kAdam ? 2 : 1; }
+
+template <int DTP, int DTG, int DTU, int DTS, int OUT, int UIN, bool COUNT, int RULE = kAnyRule, bool MARS = false>
 struct ChainKind {
   static constexpr int dt_p = DTP, dt_g = DTG, dt_u = DTU, dt_s = DTS, out_mode = OUT;
   static constexpr bool u_in = UIN != 0, count = COUNT, state = DTS != kNone;
   static constexpr bool reads_g = !u_in || count, reads_p = OUT == kOutParam;
   // Vectors per thread loaded together, and blocks per SM.  Two vectors through a rule need about 80 registers: three blocks.
-  // The codec and its random bits are 190 instructions per element and want warps rather than vectors in flight: with
-  // error-corrected state one vector is as many as fit (momentum of a Llama-3-8B layer by itself 1.76 -> 1.32 ms at one vector
-  // and four blocks, 1.65 at three; the three arrays of cautious Adam with MARS 295 us at two vectors and two blocks, 307 at one and four, 285 at one
-  // and three).
+  // The codec and its random bits are up to 190 instructions per element and want warps rather than vectors in flight: with
+  // error-corrected state one vector is as many as fit.  What such a launch then waits for is that vector's loads (a third of its stalls) and the
+  // ten dependent rounds of a random draw.  So the random bits are drawn side by side between the loads and their first use (cautious Adam with MARS
+  // on 8 x 2048^2: 287 -> 265 us), and where the rule is a constant - which also takes the spills of the ten-way switch away (255) - the next
+  // vector is fetched ahead of this one's arithmetic (232; three blocks, at two 248).  Without MARS 228 -> 169 us; Adam into fp32
+  // parameters 195 -> 174, into error-corrected ones 245 -> 232; exponential average of 25 M elements (one state: four blocks) 122 -> 75;
+  // momentum with MARS of a Llama-3-8B layer, at the clock that the products around it leave, 1.71 -> 1.45 ms.
+  // The rules that steps use most are compiled in; fp32 state is not worth it (momentum 250 -> 340 us: without spills, but with fewer loads in flight).
   static constexpr bool ecc = DTS == kBF16E8;
   // Otherwise a thread should have about 128 bytes on their way: two vectors of Adam's four arrays, four where a launch reads
   // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 288 us with two vectors,
@@ -404,12 +412,62 @@ struct ChainKind {
   // The momentum kinds spill at these counts (60 to 148 bytes per thread; the others at most 20): the times above are with
   // the spills, and the counts that spill 12 bytes or nothing are the slower ones.
   static constexpr int batch = ecc ? 1 : (state && (reads_p || count) ? 2 : 4);
-  static constexpr int min_blocks = state && !(ecc && !count) ? 3 : 4;
+  static constexpr int rule_n = rule_states(RULE);
+  static constexpr bool one_state = RULE != kAnyRule && rule_n == 1;
+  static constexpr bool ahead = ecc && RULE != kAnyRule;  // the next vector is fetched ahead
+  static constexpr int min_blocks = ahead ? (one_state ? 4 : 3) : state && !(ecc && !count) ? 3 : 4;
   static bool takes(const ChainParams& P, bool counting) {
     return counting == COUNT && P.out_mode == OUT && P.u_is_input == UIN && (!reads_p || P.dt_p == DTP) &&
-           (!reads_g || P.dt_g == DTG) && ((OUT == kOutParam && !u_in) || P.dt_u == DTU) && P.dt_s == DTS;
+           (!reads_g || P.dt_g == DTG) && ((OUT == kOutParam && !u_in) || P.dt_u == DTU) && P.dt_s == DTS &&
+           (RULE == kAnyRule || (P.algo == RULE && P.n_state == rule_states(RULE) && (P.mars != 0) == MARS));
+  }
+  static __device__ __forceinline__ bool mars(const ChainParams& P) { return RULE == kAnyRule ? P.mars != 0 : MARS; }
+  static __device__ __forceinline__ int n_state(const ChainParams& P) { return RULE == kAnyRule ? P.n_state : rule_n; }
+  static __device__ __forceinline__ F4 apply(const ChainParams& P, const F4& u, F4& s0, F4& s1) {
+    if constexpr (RULE == kAnyRule) {
+      return apply_rule(P, u, s0, s1);
+    } else {
+      F4 out;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) out.v[k] = rule_one<RULE>(P, u.v[k], s0.v[k], s1.v[k]);
+      return out;
+    }
   }
 };
+
+// Random bits of the states of four elements, drawn while their loads are on their way.
+struct StateDraws {
+  uint4 s0, s1, mars;
+};
+__device__ __forceinline__ void pin(uint4& r) { asm volatile("" : "+r"(r.x), "+r"(r.y), "+r"(r.z), "+r"(r.w)); }
+__device__ __forceinline__ StateDraws draw_states(bool mars, int n_state, const Philox& rng, int64_t i, uint32_t t) {
+  const uint32_t ctr = (uint32_t)(i >> 2), ctr_hi = (uint32_t)(i >> 34);
+  const uint4 c0 = make_uint4(ctr, ctr_hi, t, 0u), c1 = make_uint4(ctr, ctr_hi, t, 1u), cm = make_uint4(ctr, ctr_hi ^ 0x40000000u, t, 4u);
+  StateDraws r{};
+  if (mars && n_state >= 2) {
+    uint4 c[3] = {c0, c1, cm};
+    rng.rounds(c);
+    r = {c[0], c[1], c[2]};
+  } else if (mars) {
+    uint4 c[2] = {c0, cm};
+    rng.rounds(c);
+    r.s0 = c[0];
+    r.mars = c[1];
+  } else if (n_state >= 2) {
+    uint4 c[2] = {c0, c1};
+    rng.rounds(c);
+    r.s0 = c[0];
+    r.s1 = c[1];
+  } else {
+    uint4 c[1] = {c0};
+    rng.rounds(c);
+    r.s0 = c[0];
+  }
+  pin(r.s0);
+  pin(r.s1);
+  pin(r.mars);
+  return r;
+}
 
 template <class K, class Table>
 __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(const __grid_constant__ Table T, ChainParams P) {
@@ -441,21 +499,35 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
   int masked_local = 0;
   float sumsq_local = 0.f, nonzero_local = 0.f;
 
+  const int64_t first = base + threadIdx.x * 4;
+  const auto fetch = [&](int64_t i, Raw4& s0, Raw4& s1, Raw4& old, Raw4& g, Raw4& u, Raw4& p) {
+    const int nv = (int)max((int64_t)0, min((int64_t)4, end - i));
+    if (K::state) {
+      s0 = load_raw<K::dt_s>(m0, m0e, i, nv, vec_ok);
+      if (!K::one_state) s1 = load_raw<K::dt_s>(m1, m1e, i, nv, vec_ok);
+      if (K::mars(P)) old = load_raw<K::dt_s>(mm, mme, i, nv, vec_ok);
+    }
+    if (K::reads_g) g = load_raw<K::dt_g>(mg, nullptr, i, nv, vec_ok);
+    if (K::u_in) u = load_raw<K::dt_u>(mu, nullptr, i, nv, vec_ok);
+    if (K::reads_p) p = load_raw<K::dt_p>(mp, mpe, i, nv, vec_ok);
+  };
+  Raw4 s0_next{}, s1_next{}, old_next{}, g_next{}, u_next{}, p_next{};
+  if constexpr (K::ahead) fetch(first, s0_next, s1_next, old_next, g_next, u_next, p_next);
+
 #pragma unroll 1
-  for (int64_t i0 = base + threadIdx.x * 4; i0 < end; i0 += kBatch * kThreads * 4) {
+  for (int64_t i0 = first; i0 < end; i0 += kBatch * kThreads * 4) {
     Raw4 s0[kBatch], s1[kBatch], old[kBatch], g[kBatch], u[kBatch], p[kBatch];
+    StateDraws rnd[kBatch];
+    if constexpr (K::ahead) {  // (past the end: nothing is read)
+      s0[0] = s0_next; s1[0] = s1_next; old[0] = old_next; g[0] = g_next; u[0] = u_next; p[0] = p_next;
+      fetch(i0 + kThreads * 4, s0_next, s1_next, old_next, g_next, u_next, p_next);
+    } else {
 #pragma unroll
-    for (int v = 0; v < kBatch; ++v) {
-      const int64_t i = i0 + v * (kThreads * 4);
-      const int nv = (int)max((int64_t)0, min((int64_t)4, end - i));
-      if (K::state) {
-        s0[v] = load_raw<K::dt_s>(m0, m0e, i, nv, vec_ok);
-        s1[v] = load_raw<K::dt_s>(m1, m1e, i, nv, vec_ok);
-        if (P.mars) old[v] = load_raw<K::dt_s>(mm, mme, i, nv, vec_ok);
-      }
-      if (K::reads_g) g[v] = load_raw<K::dt_g>(mg, nullptr, i, nv, vec_ok);
-      if (K::u_in) u[v] = load_raw<K::dt_u>(mu, nullptr, i, nv, vec_ok);
-      if (K::reads_p) p[v] = load_raw<K::dt_p>(mp, mpe, i, nv, vec_ok);
+      for (int v = 0; v < kBatch; ++v) fetch(i0 + v * (kThreads * 4), s0[v], s1[v], old[v], g[v], u[v], p[v]);
+    }
+    if constexpr (K::ecc) {
+#pragma unroll
+      for (int v = 0; v < kBatch; ++v) rnd[v] = draw_states(K::mars(P), K::n_state(P), rng, i0 + v * (kThreads * 4), (uint32_t)t);
     }
 #pragma unroll
     for (int v = 0; v < kBatch; ++v) {
@@ -470,23 +542,23 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
 #pragma unroll
         for (int k = 0; k < 4; ++k) x.v[k] = trust_region(x.v[k]);
       }
-      if (K::state && P.mars) {  // g <- lerp(g, g_prev, a); g_prev <- raw g
+      if (K::state && K::mars(P)) {  // g <- lerp(g, g_prev, a); g_prev <- raw g
         const F4 raw = x, before = decode_raw<K::dt_s>(old[v]);
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
           x.v[k] = x.v[k] * (1.0f - P.mars_a) + before.v[k] * P.mars_a;
           grad.v[k] = x.v[k];
         }
-        store_values<K::dt_s>(mm, mme, i, nv, vec_ok, raw, draw(K::dt_s, rng, ctr, ctr_hi ^ 0x40000000u, (uint32_t)t, 4u));
+        store_values<K::dt_s>(mm, mme, i, nv, vec_ok, raw, rnd[v].mars);
       }
       F4 out = x;
       if (K::state) {
         F4 a{}, b{};
         if (m0 != nullptr) a = decode_raw<K::dt_s>(s0[v]);
-        if (m1 != nullptr) b = decode_raw<K::dt_s>(s1[v]);
-        out = apply_rule(P, x, a, b);
-        if (P.n_state >= 1) store_values<K::dt_s>(m0, m0e, i, nv, vec_ok, a, draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 0u));
-        if (P.n_state >= 2) store_values<K::dt_s>(m1, m1e, i, nv, vec_ok, b, draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 1u));
+        if (!K::one_state && m1 != nullptr) b = decode_raw<K::dt_s>(s1[v]);
+        out = K::apply(P, x, a, b);
+        if (K::n_state(P) >= 1) store_values<K::dt_s>(m0, m0e, i, nv, vec_ok, a, rnd[v].s0);
+        if (K::n_state(P) >= 2) store_values<K::dt_s>(m1, m1e, i, nv, vec_ok, b, rnd[v].s1);
       }
       if (K::count) {  // phase one of caution: mask, count, park the masked update
 #pragma unroll
@@ -606,6 +678,15 @@ template <class... Ks>
 struct KindList {};
 using Kinds = KindList<
     //        parameter gradient update state
+    // rules known at compile time
+    ChainKind<kF32, kF32, kNone, kBF16E8, kOutParam, 0, false, kAdam>,
+    ChainKind<kBF16E8, kBF16, kNone, kBF16E8, kOutParam, 0, false, kAdam>,
+    ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, false, kExpAvg>,
+    ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, false, kNesterovEma>,
+    ChainKind<kNone, kBF16, kF32, kBF16E8, kOutUpdate, 0, false, kNesterovEma, true>,
+    ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, true, kAdam, false>,
+    ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, true, kAdam, true>,
+    // any rule
     ChainKind<kF32, kF32, kNone, kF32, kOutParam, 0, false>,       // first-order rules on fp32 parameters
     ChainKind<kBF16, kBF16, kNone, kF32, kOutParam, 0, false>,     // ... on bf16 parameters
     ChainKind<kF32, kF32, kNone, kBF16E8, kOutParam, 0, false>,    // ... with error-corrected state

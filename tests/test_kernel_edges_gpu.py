@@ -37,6 +37,61 @@ def test_table_in_the_arguments_and_in_memory(ecc, extra):
         assert torch.equal(few, more)
 
 
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("sizes", [(1, 3, 4, 1023, 1024, 1025, 4097), (2_500_001, 8193, 7)], ids=len)
+@pytest.mark.parametrize("algo,mars,grad,param,count", [
+    (ops.ADAM, True, "f32", None, True), (ops.ADAM, False, "f32", None, True), (ops.ADAM, False, "f32", "f32", False),
+    (ops.ADAM, False, "bf16", "ecc", False), (ops.EXP_AVG, False, "f32", None, False), (ops.NESTEROV_EMA, False, "f32", None, False),
+    (ops.NESTEROV_EMA, True, "bf16", None, False)])  # fmt: skip
+def test_rules_known_at_compile_time_match_the_general_kernel(algo, mars, grad, param, count, sizes, shift):
+    """Error-corrected state through the instances with the rule compiled in (next vector fetched ahead, random bits drawn before the values
+    arrive) and through the general kernel, which a gradient given as the sum over one source selects, over aligned and misaligned starts,
+    remainders, zeros and values whose residuals take the slow codec.  The compiler may contract a product and a sum in one of the two:
+    2^-24 of a value, which is 2^-8 of a residual's unit (2^-16 of the value), so up to 2^-8 of the residuals may come out one unit apart
+    (255 apart where the rounded value goes the other way); fp32 results and their inputs differ by a few such roundings and units."""
+
+    def run(extra):
+        gen, dtypes = torch.Generator(DEV).manual_seed(3), {"f32": torch.float32, "bf16": torch.bfloat16, "ecc": torch.bfloat16}
+
+        def made(dtype, spread=0.0, positive=False):
+            out = []
+            for n in sizes:
+                x = torch.randn(n, device=DEV, generator=gen) * 10 ** (-spread * torch.rand(n, device=DEV, generator=gen))
+                x = torch.where(torch.rand(n, device=DEV, generator=gen) < 0.05, 0.0, x)
+                out.append(torch.zeros(n + shift, dtype=dtype, device=DEV)[shift:].copy_(x.abs() if positive else x))
+            return out
+
+        residuals = lambda: [t.zero_() for t in made(torch.int8)]  # noqa: E731
+        lists = {"g": made(dtypes[grad], 8.0), "s0": made(torch.bfloat16, 35.0), "s0e": residuals()}
+        cfg = dict(algo=algo, n_state=1, dt_g=ops.F32 if grad == "f32" else ops.BF16, dt_s=ops.BF16E8, dt_u=ops.F32, b1=0.9, b2=0.99, eps=1e-8)
+        if algo == ops.ADAM:
+            lists.update(s1=made(torch.bfloat16, 35.0, True), s1e=residuals())
+            cfg["n_state"] = 2
+        if mars:
+            lists.update(mars=made(torch.bfloat16, 35.0), marse=residuals())
+            cfg["mars_a"] = -0.0023
+        if param is None:
+            lists["u"] = made(torch.float32)
+            cfg["out_mode"] = ops.OUT_UPDATE
+        else:
+            lists.update(p=made(dtypes[param]), **({"pe": residuals()} if param == "ecc" else {}))
+            cfg.update(out_mode=ops.OUT_PARAM, dt_p=ops.F32 if param == "f32" else ops.BF16E8, lr=1e-2, wd=0.1)
+        masked = torch.zeros(len(sizes), dtype=torch.int32, device=DEV)
+        if count:
+            cfg.update(count_caution=1, masked=masked)
+        for seed in (5, 6):
+            ops.fused_chain(**lists, **cfg, **extra, seed=seed)
+        return {**lists, "masked": [masked]}
+
+    compiled, general = run({}), run({"g_delta": [0], "g_scale": 1.0})
+    for name, tensors in compiled.items():
+        for i, (a, b) in enumerate(zip(tensors, general[name])):
+            if a.dtype in (torch.int8, torch.bfloat16):
+                assert int((a != b).sum()) <= a.numel() >> 8, (name, i, int((a != b).sum()))
+            else:
+                torch.testing.assert_close(a, b, rtol=2**-14, atol=1e-30)
+
+
 @pytest.mark.parametrize("kw", [{}, {"ecc": "bf16+8", "mars": True, "caution": True}, {"ecc": "bf16+8"}, {"caution": True}], ids=str)
 @pytest.mark.parametrize("sizes", [(1,), (2047, 2048, 2049), (8191, 8193, 3, 16384), tuple(range(1, 41)), (10_000_000, 5),
                                    (4095, 4096, 4097, 2_500_001, 7), (8191, 8192, 8193, 1, 10_000_000, 5)], ids=len)  # fmt: skip
