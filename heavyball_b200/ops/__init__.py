@@ -33,7 +33,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 _SRC = os.path.join(_HERE, "csrc")
 _BUILD = os.path.join(_HERE, "_build")
 _NAME = "hb200_ops"
-_SOURCES = ["bindings.cpp", "colsum.cu", "cross_entropy.cu", "fused_chain.cu", "gelu.cu", "layer_norm.cu", "ns_gemm.cu", "noalloc_adamw.cu", "peer_sync.cu", "skinny.cu", "split16_gemm.cu", "tf32_gemm.cu"]
+_SOURCES = ["bindings.cpp", "chol_qr.cu", "colsum.cu", "cross_entropy.cu", "fused_chain.cu", "gelu.cu", "layer_norm.cu", "ns_gemm.cu", "noalloc_adamw.cu", "peer_sync.cu", "skinny.cu", "split16_gemm.cu", "tf32_gemm.cu"]
 _lock = threading.Lock()
 _ext = None
 _load_error: Optional[BaseException] = None
@@ -306,6 +306,15 @@ def tf32_gemm(a2: torch.Tensor, b2: torch.Tensor, K: int, *, mode: int = EPI_STO
     launch_counter.count += 1
     s = load().tf32_gemm(a2, b2, K, mode, alpha, w, b1, b2c, eps, out, split_out, m, v, _status(a2.device))
     return s if split_out else None
+
+
+def chol_qr_round(gram: torch.Tensor, a: torch.Tensor, info: torch.Tensor, want_trans: bool = True):
+    """One round of Cholesky QR: ``X = a R^-1`` with ``R^T R = gram`` (both overwritten) on the split-tf32 products.  Contiguous fp32
+    ``a``: ``[batch, n, k]``, ``n`` a multiple of 64 and ``k`` of 128; ``info``: int32 ``[batch]``, incremented per 128-wide leaf with a bad pivot.
+    Returns ``(X, operand)``; the latter is :func:`tf32_split` of ``X`` with its columns as rows (``None`` unless ``want_trans``)."""
+    x, trans, launches = load().chol_qr_round(gram, a, want_trans, info, _status(a.device))
+    launch_counter.count += launches
+    return x, trans
 
 
 class Split16:

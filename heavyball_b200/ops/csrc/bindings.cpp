@@ -13,6 +13,7 @@
 #include <unordered_map>
 #include <vector>
 
+#include "chol_qr.h"
 #include "colsum.h"
 #include "cross_entropy.h"
 #include "fused_chain.h"
@@ -746,6 +747,32 @@ void chol_inv_leaf(const at::Tensor& g, at::Tensor& r, at::Tensor& inv, int64_t 
                                  info.data_ptr<int>(), at::cuda::getCurrentCUDAStream()), "chol_inv_leaf launch");
 }
 
+// One round of Cholesky QR (chol_qr.h): X = A R^-1 with R^T R = gram; both are overwritten.  Contiguous fp32, a: [batch, n, k], n a multiple of
+// 64, k of 128; info: int32 [batch], incremented per leaf with a bad pivot.  Returns X, the split-tf32 operand of X^T (when asked) and the number
+// of launches.
+std::tuple<at::Tensor, OptT, int> chol_qr_round(const at::Tensor& gram, const at::Tensor& a, bool want_trans, const at::Tensor& info,
+                                                const at::Tensor& status) {
+  for (const at::Tensor* t : {&gram, &a})
+    TORCH_CHECK(t->is_cuda() && t->device() == a.device() && t->scalar_type() == at::kFloat && t->dim() == 3 && t->is_contiguous() && aligned16(t->data_ptr()),
+                "chol_qr_round: contiguous fp32 [batch, n, k] CUDA tensors");
+  const int64_t batch = a.size(0), n = a.size(1), k = a.size(2);
+  TORCH_CHECK(n >= 1 && k >= 1 && n % hb::kQrRows == 0 && k % hb::kQrBlock == 0 && batch <= 65535 && gram.size(0) == batch && gram.size(1) == k && gram.size(2) == k,
+              "chol_qr_round: a of n x k, n a multiple of 64 and k of 128, with its k x k Gram matrix");
+  TORCH_CHECK(at::get_overlap_status(gram, a) == at::MemOverlapStatus::No, "chol_qr_round: two tensors");
+  TORCH_CHECK(info.device() == a.device() && info.scalar_type() == at::kInt && info.is_contiguous() && info.numel() == batch, "chol_qr_round: info must be int32 [batch]");
+  c10::cuda::CUDAGuard guard(a.device());
+  const auto options = a.options().memory_format(at::MemoryFormat::Contiguous);
+  const at::Tensor x = at::empty({batch, n, k}, options), x_same = at::empty({batch, n, 2 * k}, options), l = at::empty({batch, k, 2 * k}, options);
+  const at::Tensor inv = at::empty({batch, k / hb::kQrBlock, hb::kQrBlock, hb::kQrBlock}, options);
+  OptT trans;
+  if (want_trans) trans = at::empty({batch, k, 2 * n}, options);
+  int launches = 0;
+  check(hb::launch_chol_qr_round({gram.data_ptr<float>(), a.data_ptr<float>(), x.data_ptr<float>(), want_trans ? trans->data_ptr<float>() : nullptr, l.data_ptr<float>(),
+                                  inv.data_ptr<float>(), x_same.data_ptr<float>(), (int)n, (int)k, (int)batch, info.data_ptr<int>(), status.data_ptr<int>()},
+                                 &launches, at::cuda::getCurrentCUDAStream()), "chol_qr_round");
+  return {x, trans, launches};
+}
+
 // Row-major upper triangles of contiguous [batch, n, n] matrices (2- or 4-byte elements) as [batch, n (n + 1) / 2].
 at::Tensor triu_pack(const at::Tensor& dense) {
   TORCH_CHECK(dense.is_cuda() && dense.dim() == 3 && dense.size(1) == dense.size(2) && dense.is_contiguous() &&
@@ -921,6 +948,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     return choice;
   });
   m.def("chol_inv_leaf", &chol_inv_leaf);
+  m.def("chol_qr_round", &chol_qr_round);
   m.def("triu_pack", &triu_pack);
   m.def("triu_unpack", &triu_unpack);
   m.def("chunk_elems", &hb::chain_chunk_elems);

@@ -560,12 +560,12 @@ __device__ __forceinline__ void epilogue_direct(uint32_t tmem_warp, int lane, fl
 // `Kind`: operand type.  kBlock elements of K fill a 128-byte row; kDesc is the instruction descriptor for a 128 x 128 tile; the product
 // is three walks over K, of which walk kTermLoA takes the low parts of A and walk kTermLoB those of B; kCrossFirst: these two come
 // first, and the sum they leave is scaled by 2^-11 when the walk over the high parts begins.  kPairDesc, mma_pair: the same for the pair
-// kernel.
+// kernel.  `lo_a`, `lo_b`: how far the low parts of an operand's rows lie behind the high parts.
 template <class Kind>
 __global__ void __launch_bounds__(kTThreads, 2)
 gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-               const __grid_constant__ CUtensorMap map_c, int M, int N, int kp, const Tf32Epilogue E, const __grid_constant__ PairOperands P,
-               int bulk_store, int* status) {
+               const __grid_constant__ CUtensorMap map_c, int M, int N, int kp, int lo_a, int lo_b, const Tf32Epilogue E,
+               const __grid_constant__ PairOperands P, int bulk_store, int* status) {
   constexpr int TBK = Kind::kBlock;
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kTStages];
@@ -622,8 +622,8 @@ gemm128_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         uint8_t* dst = tiles + s * kTStageBytes;
         const int seg = kb / seg_kb, k0 = (kb_lo + kb - seg * seg_kb) * TBK;
         mbar_expect_tx(&full_bar[s], kTStageBytes);
-        tma_load_3d(dst, &map_a, &full_bar[s], k0 + (seg == Kind::kTermLoA ? kp : 0), tm * TBM, batch);
-        tma_load_3d(dst + kTTileBytes, &map_b, &full_bar[s], k0 + (seg == Kind::kTermLoB ? kp : 0), tn * TBN, batch);
+        tma_load_3d(dst, &map_a, &full_bar[s], k0 + (seg == Kind::kTermLoA ? lo_a : 0), tm * TBM, batch);
+        tma_load_3d(dst + kTTileBytes, &map_b, &full_bar[s], k0 + (seg == Kind::kTermLoB ? lo_b : 0), tn * TBN, batch);
         issued = kb + 1;
       }
     }
@@ -731,8 +731,8 @@ __device__ __forceinline__ WalkTile walk_tile(const PairTile& t, int kp, int tri
 
 template <class Kind>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kGPairThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N, int kp, int tiles_m,
-                    int tiles_n, int per_batch, int total, const Tf32Epilogue E, const __grid_constant__ PairOperands P, int* status) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N, int kp, int lo_a, int lo_b,
+                    int tiles_m, int tiles_n, int per_batch, int total, const Tf32Epilogue E, const __grid_constant__ PairOperands P, int* status) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kGPairStages];   // used in the even CTA: both CTAs' loads of a stage have landed
   __shared__ __align__(8) uint64_t empty_bar[kGPairStages];  // in each CTA: the products that read the stage have finished
@@ -778,7 +778,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         const WalkTile h = walk_tile(t, kp, E.tri, Kind::kBlock);
         const int a_row = t.tm * kPairTile + (int)rank * 128, b_row = t.tn * kPairTile + (int)rank * 128;
         for (int term = 0; term < 3 && ok; ++term) {
-          const int ka = (term == Kind::kTermLoA ? kp : 0), kb_off = (term == Kind::kTermLoB ? kp : 0);
+          const int ka = (term == Kind::kTermLoA ? lo_a : 0), kb_off = (term == Kind::kTermLoB ? lo_b : 0);
           for (int kb = 0; kb < h.seg; ++kb, ++n) {
             const int s = n % kGPairStages, round = n / kGPairStages, k0 = (h.kb_lo + kb) * Kind::kBlock;
             ok = mbar_wait<Kind::kScaled ? kLongSpinLimit : kSpinLimit>(&empty_bar[s], (round & 1) ^ 1, &abort_flag);

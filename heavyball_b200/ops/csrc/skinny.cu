@@ -12,6 +12,7 @@
 #include "skinny.h"
 
 #include "per_device.h"
+#include "tc_common.cuh"
 
 #include <stdint.h>
 
@@ -262,6 +263,8 @@ __global__ void __launch_bounds__(kLeafThreads) chol_inv_leaf_kernel(const float
   __shared__ int failed;
   const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid == 0) failed = 0;
+  griddep_wait();
+  griddep_launch();
   load_upper(G + (long long)b * strideG, ldg, size, t, x);
   __syncthreads();
 
@@ -337,7 +340,7 @@ __global__ void __launch_bounds__(kLeafThreads) chol_inv_leaf_kernel(const float
   float* out = X + (long long)b * strideX;
   for (int idx = tid; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
     const int i = idx >> 7, j = idx & (kTriBlock - 1);
-    if (i < size && j < size) r[(long long)i * ldr + j] = j >= i ? t[i * kLeafLd + j] : 0.f;
+    if (R != nullptr && i < size && j < size) r[(long long)i * ldr + j] = j >= i ? t[i * kLeafLd + j] : 0.f;
     out[idx] = j >= i ? x[i * kLeafLd + j] : 0.f;
   }
   if (tid == 0 && failed && info != nullptr) atomicAdd(info + b, 1);
@@ -373,8 +376,7 @@ cudaError_t launch_chol_inv_leaf(const float* G, long long ldg, long long stride
   if (size > kTriBlock) return cudaErrorInvalidValue;
   cudaError_t e = configure_leaf_kernels();
   if (e != cudaSuccess) return e;
-  chol_inv_leaf_kernel<<<batch, kLeafThreads, kLeafBytes, stream>>>(G, ldg, strideG, R, ldr, strideR, X, strideX, size, info);
-  return cudaGetLastError();
+  return launch_chained(chol_inv_leaf_kernel, dim3(batch), kLeafThreads, kLeafBytes, stream, G, ldg, strideG, R, ldr, strideR, X, strideX, size, info);
 }
 
 // ------------------------------------------------------------------------------------------ packed upper triangles

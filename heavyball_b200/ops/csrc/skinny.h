@@ -19,7 +19,7 @@ cudaError_t launch_tri_inv_blocks(const float* Q, long long ld, long long stride
                                   cudaStream_t stream);
 
 // Upper Cholesky factor and its inverse of one diagonal leaf (size <= kTriBlock) of a batch of symmetric positive definite
-// matrices: G points at the leaf's first element (row stride ldg, batch stride strideG), likewise R; X: the leaf's
+// matrices: G points at the leaf's first element (row stride ldg, batch stride strideG), likewise R (null: not wanted); X: the leaf's
 // kTriBlock x kTriBlock inverse block per matrix (batch stride strideX), completed with an identity for short leaves.
 // info[b] is incremented when a pivot of matrix b was not positive.
 cudaError_t launch_chol_inv_leaf(const float* G, long long ldg, long long strideG, float* R, long long ldr, long long strideR,

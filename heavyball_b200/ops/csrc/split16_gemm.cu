@@ -366,7 +366,7 @@ cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N
   if (pair) {
     const int tm = (M + kPairTile - 1) / kPairTile, tn = (N + kPairTile - 1) / kPairTile;
     const int grid = 2 * (int)(big < max_pairs ? big : max_pairs);
-    return launch_chained(gemm_pair_kernel<HalfKind>, dim3(grid), kGPairThreads, kGPairSmemBytes, stream, ma, mb, M, N, (int)kp, tm, tn,
+    return launch_chained(gemm_pair_kernel<HalfKind>, dim3(grid), kGPairThreads, kGPairSmemBytes, stream, ma, mb, M, N, (int)kp, (int)kp, (int)kp, tm, tn,
                           tiles(kPairTile), (int)big, E, P, status);
   }
   // bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing past it
@@ -374,7 +374,7 @@ cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N
                     (((uintptr_t)E.C) & 15) == 0) ? 1 : 0;
   CUtensorMap mc = ma;  // placeholder when the bulk-store path is not taken (never dereferenced then)
   if (bulk && !make_store_map(&mc, E.C, M, N, E.ldc, E.strideC, batch)) return cudaErrorInvalidValue;
-  return launch_chained(gemm128_kernel<HalfKind>, dim3(tiles(TBM), batch), kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, P, bulk,
+  return launch_chained(gemm128_kernel<HalfKind>, dim3(tiles(TBM), batch), kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, (int)kp, (int)kp, E, P, bulk,
                         status);
 }
 

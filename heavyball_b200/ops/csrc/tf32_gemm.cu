@@ -165,6 +165,11 @@ cudaError_t tf32_gemm_tiles(int M, int N, int K, int batch, int symmetric, int* 
 
 cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int K, int batch, const Tf32Epilogue& E,
                              int* status, cudaStream_t stream) {
+  const int64_t kp = tf32_split_kp(K);
+  return launch_tf32_gemm(Tf32Operand{A2, 2 * kp, M * 2 * kp, kp}, Tf32Operand{B2, 2 * kp, N * 2 * kp, kp}, M, N, K, batch, E, status, stream);
+}
+
+cudaError_t launch_tf32_gemm(Tf32Operand A, Tf32Operand B, int M, int N, int K, int batch, const Tf32Epilogue& E, int* status, cudaStream_t stream) {
   int max_pairs = 0;
   const cudaError_t e = resident_pairs(&max_pairs);
   if (e != cudaSuccess) return e;
@@ -172,11 +177,12 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   if ((E.mode == kEpiAdam || E.mode == kEpiLaProp) && (E.m == nullptr || E.v == nullptr)) return cudaErrorInvalidValue;
   if ((E.mode == kEpiLerp || E.mode == kEpiAdd) && E.C == nullptr) return cudaErrorInvalidValue;
   if (E.tri && (M != N || M != K || E.symmetric)) return cudaErrorInvalidValue;
-  if (E.symmetric && (A2 != B2 || M != N || E.C == nullptr || E.S != nullptr || (E.mode != kEpiStore && E.mode != kEpiLerp && E.mode != kEpiAdd)))
+  if (E.symmetric && (A.p != B.p || M != N || E.C == nullptr || E.S != nullptr || (E.mode != kEpiStore && E.mode != kEpiLerp && E.mode != kEpiAdd)))
     return cudaErrorInvalidValue;
-  const int64_t kp = tf32_split_kp(K), ld = 2 * kp;
+  const int64_t kp = tf32_split_kp(K);
+  if (A.lo < kp || B.lo < kp || A.lo % 4 != 0 || B.lo % 4 != 0) return cudaErrorInvalidValue;
   CUtensorMap ma, mb, mc;
-  if (!make_f32_map(&ma, A2, M, ld, ld, (int64_t)M * ld, batch) || !make_f32_map(&mb, B2, N, ld, ld, (int64_t)N * ld, batch))
+  if (!make_f32_map(&ma, A.p, M, A.lo + kp, A.ld, A.stride, batch) || !make_f32_map(&mb, B.p, N, B.lo + kp, B.ld, B.stride, batch))
     return cudaErrorInvalidValue;
 
   TileChoice tiles = tf32_tiles(M, N, K, batch, E.symmetric != 0, max_pairs);
@@ -189,7 +195,7 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
     Tf32Epilogue E2 = E;
     if (tiles == kPairTilesSmallDiagonal) E2.symmetric = 2;
     return launch_chained(gemm_pair_kernel<Tf32Kind>, dim3(2 * (int)(total < max_pairs ? total : max_pairs)), kGPairThreads, kGPairSmemBytes, stream,
-                          ma, mb, M, N, (int)kp, big_m, big_n, per_batch, (int)total, E2, PairOperands{}, status);
+                          ma, mb, M, N, (int)kp, (int)A.lo, (int)B.lo, big_m, big_n, per_batch, (int)total, E2, PairOperands{}, status);
   }
 
   // plain products leave through the bulk-store path (bulk stores end on 16-byte boundaries: with N a multiple of 4 they write nothing
@@ -200,7 +206,8 @@ cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int
   if (bulk && !make_f32_map(&mc, E.C, M, N, E.ldc, E.strideC, batch)) return cudaErrorInvalidValue;
   const int tiles_m = (M + TBM - 1) / TBM, tiles_n = (N + TBN - 1) / TBN;
   dim3 grid(E.symmetric ? tiles_n * (tiles_n + 1) / 2 : tiles_m * tiles_n, batch);
-  return launch_chained(gemm128_kernel<Tf32Kind>, grid, kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, E, PairOperands{}, bulk, status);
+  return launch_chained(gemm128_kernel<Tf32Kind>, grid, kTThreads, kTSmemBytes, stream, ma, mb, mc, M, N, (int)kp, (int)A.lo, (int)B.lo, E, PairOperands{}, bulk,
+                        status);
 }
 
 }  // namespace hb

@@ -51,6 +51,14 @@ struct Tf32Epilogue {
 cudaError_t launch_tf32_gemm(const float* A2, const float* B2, int M, int N, int K, int batch, const Tf32Epilogue& E,
                              int* status, cudaStream_t stream);
 
+// The same over rows of a wider buffer: the high parts of row r of batch entry b begin at p + b * stride + r * ld (16-byte aligned, strides
+// multiples of 4), its low parts `lo` elements behind them.  What lies between K and its next multiple of 32 is read, too.
+struct Tf32Operand {
+  const float* p;
+  int64_t ld, stride, lo;
+};
+cudaError_t launch_tf32_gemm(Tf32Operand A, Tf32Operand B, int M, int N, int K, int batch, const Tf32Epilogue& E, int* status, cudaStream_t stream);
+
 // What launch_tf32_gemm takes on the current device for these sizes (TileChoice of gemm_rules.h).
 cudaError_t tf32_gemm_tiles(int M, int N, int K, int batch, int symmetric, int* choice);
 

@@ -271,6 +271,8 @@ def _cholesky_qr2(x: Tensor, shifted_rounds: int = 0):
     bad = torch.zeros(a.shape[0], dtype=torch.int32, device=a.device)
     rounds = shifted_rounds + 2
     info = torch.zeros_like(bad)  # failed leaves do not decide: what counts is the orthogonality reached at the end
+    if _whole_blocks(a):
+        return _cholesky_qr2_blocks(a, bad, info, shifted_rounds).reshape(*batch, n, k), bad
     for rnd in range(rounds):
         gram = _mm(a, a, True, False, pairs=False)
         if rnd < shifted_rounds:
@@ -290,6 +292,39 @@ def _cholesky_qr2(x: Tensor, shifted_rounds: int = 0):
         bad += (gram - torch.eye(k, device=a.device, dtype=a.dtype)).abs().amax(dim=(-2, -1)).gt(_CHOLQR_ACCEPT)
         bad += (~torch.isfinite(a)).flatten(1).any(dim=1)
     return a.reshape(*batch, n, k), bad
+
+
+def _whole_blocks(a: Tensor) -> bool:
+    """Whether a round of Cholesky QR on ``a`` consists of 128-wide blocks and tensor-core products only, so that the extension can run it
+    as one chain (``ops/csrc/chol_qr.cu``); other widths go block by block through library products, too."""
+    n, k = a.shape[-2:]
+    return (
+        _skinny_kernels(a) is not None and getattr(_settings(), "tensor_core_matmul", True)
+        and k >= _CHOLQR_MIN and k % _CHOL_LEAF == 0 and n >= k and n % 64 == 0 and 0 < a.shape[0] <= 65535
+    )  # fmt: skip
+
+
+def _cholesky_qr2_blocks(a: Tensor, bad: Tensor, info: Tensor, shifted_rounds: int) -> Tensor:
+    """The rounds of :func:`_cholesky_qr2` with the same products in the same order (same bits) by ``ops.chol_qr_round``.  ``a`` is
+    overwritten."""
+    from .. import ops
+
+    n, k = a.shape[-2:]
+    a = a.contiguous()
+    gram = torch.empty(a.shape[0], k, k, device=a.device, dtype=a.dtype)
+    operand = ops.tf32_split(a, False, True)[1]
+    for rnd in range(shifted_rounds + 2):
+        ops.tf32_gemm(operand, operand, n, out=gram)
+        shifted = rnd < shifted_rounds
+        if shifted:
+            gram.diagonal(dim1=-2, dim2=-1).add_(_CHOLQR_SHIFT * k)
+        a, operand = ops.chol_qr_round(gram, a, info, want_trans=not shifted)
+        if shifted:
+            a = a / a.norm(dim=-2, keepdim=True).clamp_(min=torch.finfo(a.dtype).tiny)
+            operand = ops.tf32_split(a, False, True)[1]
+    ops.tf32_gemm(operand, operand, n, out=gram)
+    ops.load().identity_defect(gram, _CHOLQR_ACCEPT, bad)
+    return a
 
 
 _cholqr_graphs = {}

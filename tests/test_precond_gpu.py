@@ -263,3 +263,37 @@ def test_a_step_does_not_depend_on_the_default_dtype(name, dtype):
 
     for got, want in zip(run(dtype), run(torch.float32)):
         assert torch.isfinite(want).all() and float((got - want).abs().max()) < 1e-5 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("shifted", [0, 1])
+@pytest.mark.parametrize("batch,n,k", [(3, 256, 256), (1, 320, 256), (2, 384, 384), (16, 512, 512), (2, 1024, 512), (3, 640, 640), (1, 896, 896), (16, 1024, 1024),
+                                       (2, 1152, 1152), (1, 1664, 1664), (2, 2048, 2048)])  # fmt: skip
+def test_cholesky_qr_of_whole_blocks_has_the_bits_of_the_block_by_block_form(batch, n, k, shifted, monkeypatch):
+    """The chain of ops.chol_qr_round against the same recursion through single products, splits, copies and the library's fp32 product with
+    the leaves' inverses: equal bits, and an orthonormal basis, for widths whose halves are even and odd numbers of blocks."""
+    from heavyball_b200.utils import orthogonal
+
+    gen = torch.Generator("cuda").manual_seed(k + batch)
+    x = torch.eye(n, k, device="cuda") + 0.3 / k**0.5 * torch.randn(batch, n, k, device="cuda", generator=gen)
+    x = x * torch.logspace(2, -2, k, device="cuda")
+    assert orthogonal._whole_blocks(x)
+    before = x.clone()
+    q, bad = orthogonal._cholesky_qr2(x, shifted)
+    monkeypatch.setattr(orthogonal, "_whole_blocks", lambda a: False)
+    want, want_bad = orthogonal._cholesky_qr2(x, shifted)
+    assert torch.equal(x, before) and torch.equal(bad, want_bad) and int(bad.sum()) == 0
+    assert torch.equal(q, want), float((q - want).abs().max())
+    defect = (q.double().mT @ q.double() - torch.eye(k, device="cuda", dtype=torch.float64)).abs().max()
+    assert defect < 1e-4
+
+
+def test_cholesky_qr_refuses_dependent_columns_either_way(monkeypatch):
+    from heavyball_b200.utils import orthogonal
+
+    x = torch.randn(2, 512, 512, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    x[1, :, 300] = x[1, :, 5]
+    assert orthogonal._cholesky_qr2(x)[1].gt(0).tolist() == [False, True]
+    x[0, 7, 9] = float("nan")
+    assert orthogonal._cholesky_qr2(x)[1].gt(0).tolist() == [True, True]
+    monkeypatch.setattr(orthogonal, "_whole_blocks", lambda a: False)
+    assert orthogonal._cholesky_qr2(x)[1].gt(0).tolist() == [True, True]
