@@ -143,98 +143,290 @@ cudaError_t launch_tall_t_mul(const float* X, long long ldx, long long strideX, 
 }
 
 // ------------------------------------------------------------------------------------------ 128 x 128 triangular leaves
-// Both leaf kernels work on one (up to) 128 x 128 block per CTA of 1024 threads, the block and its inverse in shared memory
+// Both leaf kernels work on one (up to) 128 x 128 block per CTA of 512 threads, the block and its inverse in shared memory
 // as 4 x 4 sub-blocks of 32.  A refresh of an eigenbasis factors 16 leaves per 2048-wide factor and round, one after the
 // other, so the latency of one CTA is all that counts; it is set by the length of the dependent chain, not by the 0.7 MFLOP.
-//   factor R^T R = G, panel of 32 rows by panel: the 32 x 32 diagonal block in one warp (lane = column, the column in
-//     registers, pivots and multipliers by shuffle), the rows of the panel to its right by substitution (thread = column,
-//     column in registers), the trailing blocks by a rank-32 update (4 x up to 3 elements per thread).  Every element
-//     receives the same products in the same order as in an element-wise right-looking factorisation; that form needed two
-//     barriers per pivot, 256 of them, and a leaf took 108 us (two SOAP steps on 8 x 1024^2, 32 leaves: 9.82 -> 8.19 ms).
-//   invert R: the four diagonal blocks (one warp each, lane = column in registers), then the blocks above the diagonal by
-//     distance d = 1, 2, 3:  X_IJ = -X_II (sum_{K = I+1 .. J} R_IK X_KJ), J = I + d, four rows per warp.
+//   factor R^T R = G, panel of 32 rows by panel: the 32 x 32 diagonal block in one warp (lane = column, the column in registers), four pivots at
+//     a time, whose 4 x 4 block every lane factors for itself; rows and reciprocal pivots go through shared memory, where three more warps
+//     pick them up four at a time and carry the columns to the right along (a barrier per step).  Then the trailing blocks by a rank-32
+//     update, 4 x 4 values per lane.  Every element receives the same products in the same order as in an element-wise right-looking
+//     factorisation.
+//   invert R, column of blocks by column while the next panel is factored:  X_JJ by one warp (lane = column in registers), then upwards
+//     X_IJ = -X_II (sum_{K = I+1 .. J} R_IK X_KJ) by eight warps, 2 x 2 values per lane.
+// 54 -> 25 us for 16 leaves (SM clocks of the former / this form: diagonal blocks 4 x 15.7k / 4.1k to 8k, with the inverse's columns under them;
+// rows to the right 3 x 2.7k / hidden; trailing 9.3k / 6k; inverse 20.7k / 9.9k behind the last panel; load 4k / 2k; store 5.4k / 2.1k).  The former
+// shuffled every multiplier: in a branch on the warp's number, which the compiler takes for divergent, shuffles go one at a time, 490 clocks
+// a pivot.  Hence the warp's number by a shuffle, too (uniform), and loads in groups before the arithmetic that uses them.
 // A non-positive or non-finite pivot is replaced by 1 and counted in info[b] (the result for that matrix is then
 // meaningless, the others are unaffected).
 namespace {
 
-constexpr int kLeafThreads = 1024;
+constexpr int kLeafThreads = 512;
 constexpr int kLeafLd = kTriBlock + 4;  // rows start on 16-byte boundaries: four values of a row per (broadcast) load
 constexpr int kLeafBytes = 2 * kTriBlock * kLeafLd * (int)sizeof(float);
 constexpr int kSub = 32, kSubs = kTriBlock / kSub;
+constexpr int kLoads = kTriBlock * kTriBlock / 4 / kLeafThreads;
 
-// Loads the upper part of a block of `size` rows; a short block is completed by an identity.  x <- 0.
-__device__ __forceinline__ void load_upper(const float* __restrict__ g, long long ld, int size, float* t, float* x) {
-  float v[kTriBlock * kTriBlock / kLeafThreads];
+// Named barriers of part of a block.
+enum LeafBarrier : int { kLowWarps = 1, kHighWarps = 2, kPanelStep = 4 };  // kPanelStep .. + 7: the eight steps of a panel
+template <int kThreads>
+__device__ __forceinline__ void part_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
+template <int kThreads>
+__device__ __forceinline__ void part_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kThreads) : "memory"); }
+
+
+// Loads the upper part of a block of `size` rows (what lies left of the diagonal is anything); a short block is completed by an identity.
+__device__ __forceinline__ void load_upper(const float* __restrict__ g, long long ld, int size, float* t) {
+  if (size == kTriBlock && (ld & 3) == 0 && ((uintptr_t)g & 15) == 0) {
+    float4 v[kLoads];
 #pragma unroll
-  for (int e = 0; e < kTriBlock * kTriBlock / kLeafThreads; ++e) {
-    const int idx = threadIdx.x + e * kLeafThreads, i = idx >> 7, j = idx & (kTriBlock - 1);
-    v[e] = (i == j) ? 1.f : 0.f;
-    if (i < size && j < size && j >= i) v[e] = g[(long long)i * ld + j];
-  }
+    for (int e = 0; e < kLoads; ++e) {
+      const int idx = threadIdx.x + e * kLeafThreads, i = idx >> 5, j = (idx & 31) * 4;
+      v[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (j + 3 >= i) v[e] = *(const float4*)(g + (long long)i * ld + j);
+    }
 #pragma unroll
-  for (int e = 0; e < kTriBlock * kTriBlock / kLeafThreads; ++e) {
-    const int idx = threadIdx.x + e * kLeafThreads, i = idx >> 7, j = idx & (kTriBlock - 1);
-    t[i * kLeafLd + j] = v[e];
-    x[i * kLeafLd + j] = 0.f;
+    for (int e = 0; e < kLoads; ++e) {
+      const int idx = threadIdx.x + e * kLeafThreads, i = idx >> 5, j = (idx & 31) * 4;
+      *(float4*)(t + i * kLeafLd + j) = v[e];
+    }
+  } else {
+    for (int idx = threadIdx.x; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
+      const int i = idx >> 7, j = idx & (kTriBlock - 1);
+      float v = i == j ? 1.f : 0.f;
+      if (i < size && j < size && j >= i) v = g[(long long)i * ld + j];
+      t[i * kLeafLd + j] = v;
+    }
   }
 }
 
-// x <- t^-1 for the upper-triangular block t; the part of x below the diagonal blocks is scratch.
-__device__ __forceinline__ void invert_upper(const float* t, float* x) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (warp < kSubs) {  // right-looking back substitution: row i of this lane's column is final when step i starts
-    const float* d = t + warp * kSub * (kLeafLd + 1);
-    float* xd = x + warp * kSub * (kLeafLd + 1);
-    float acc[kSub];
+struct Pivot {
+  float inv, root;
+  bool ok;
+};
+__device__ __forceinline__ Pivot pivot_of(float piv) {
+  Pivot p;
+  p.ok = piv > 0.f && piv < 3.0e38f;
+  const float r = rsqrtf(piv);
+  p.inv = p.ok ? r : 1.f;
+  p.root = p.ok ? piv * p.inv : 1.f;
+  return p;
+}
+
+// A panel on its way from the warp that factors to those that follow: reciprocal pivots and rows, four at a time.
+struct Panel {
+  float4 inv[kSub / 4];
+  float4 row[kSub / 4][kSub];
+};
+
+// 32 x 32 diagonal block by one warp
+__device__ __forceinline__ bool factor_diagonal(float* d, Panel& P) {
+  const int lane = threadIdx.x & 31;
+  float a[kSub], p[4][4];
+  bool bad = false;
 #pragma unroll
-    for (int i = 0; i < kSub; ++i) acc[i] = 0.f;
+  for (int i = 0; i < kSub; ++i) a[i] = d[i * kLeafLd + lane];
 #pragma unroll
-    for (int i = kSub - 1; i >= 0; --i) {
-      const float piv = d[i * kLeafLd + i];
-      const float xi = i == lane ? 1.0f / piv : (i < lane ? -acc[i] / piv : 0.f);
-      xd[i * kLeafLd + lane] = xi;
+  for (int r = 0; r < 4; ++r)
 #pragma unroll
-      for (int k = 0; k < i; ++k) acc[k] = fmaf(d[k * kLeafLd + i], xi, acc[k]);
+    for (int c = r; c < 4; ++c) p[r][c] = d[r * kLeafLd + c];
+#pragma unroll
+  for (int k = 0; k < kSub; k += 4) {
+    float m[4][4], inv[4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const Pivot v = pivot_of(p[r][r]);
+      bad |= !v.ok;
+      inv[r] = v.inv;
+#pragma unroll
+      for (int c = r + 1; c < 4; ++c) m[r][c] = p[r][c] * v.inv;
+#pragma unroll
+      for (int i = r + 1; i < 4; ++i)
+#pragma unroll
+        for (int c = i; c < 4; ++c) p[i][c] = fmaf(-m[r][i], m[r][c], p[i][c]);
+      a[k + r] = lane == k + r ? v.root : a[k + r] * v.inv;
+#pragma unroll
+      for (int i = r + 1; i < 4; ++i) a[k + i] = fmaf(-m[r][i], a[k + r], a[k + i]);
+    }
+    float4* row = P.row[k >> 2];
+    row[lane] = make_float4(a[k], a[k + 1], a[k + 2], a[k + 3]);
+    if (lane == 0) P.inv[k >> 2] = make_float4(inv[0], inv[1], inv[2], inv[3]);
+    __syncwarp();
+    part_arrive<128>(kPanelStep + (k >> 2));
+#pragma unroll
+    for (int i0 = k + 4; i0 < kSub; i0 += 4) {
+      float4 r[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) r[e] = row[i0 + e];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].x, a[k], a[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].y, a[k + 1], a[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].z, a[k + 2], a[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].w, a[k + 3], a[i0 + e]);
+      if (i0 == k + 4) {
+#pragma unroll
+        for (int r2 = 0; r2 < 4; ++r2)
+#pragma unroll
+          for (int c = r2; c < 4; ++c) p[r2][c] = __shfl_sync(0xffffffffu, a[i0 + r2], i0 + c);
+      }
     }
   }
-  __syncthreads();
-  const int I = warp >> 3, r0 = (warp & 7) * 4;  // four rows of the I-th block at the current distance
+#pragma unroll
+  for (int i = 0; i < kSub; ++i)
+    if (i <= lane) d[i * kLeafLd + lane] = a[i];
+  return bad;
+}
+
+// the rows of the panel right of its diagonal block, a column per lane, step by step behind the warp that factors
+__device__ __forceinline__ void follow_panel(float* col, const Panel& P, bool on) {
+  if (!on) {
+    for (int step = 0; step < kSub / 4; ++step) part_sync<128>(kPanelStep + step);
+    return;
+  }
+  float a[kSub];
+#pragma unroll
+  for (int i = 0; i < kSub; ++i) a[i] = col[i * kLeafLd];
+#pragma unroll
+  for (int k = 0; k < kSub; k += 4) {
+    part_sync<128>(kPanelStep + (k >> 2));
+    const float4* row = P.row[k >> 2];
+    const float4 inv4 = P.inv[k >> 2];
+    const float inv[4] = {inv4.x, inv4.y, inv4.z, inv4.w};
+    float4 m[4];
+#pragma unroll
+    for (int e = 1; e < 4; ++e) m[e] = row[k + e];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      a[k + r] *= inv[r];
+#pragma unroll
+      for (int i = r + 1; i < 4; ++i) a[k + i] = fmaf(-(r == 0 ? m[i].x : r == 1 ? m[i].y : m[i].z), a[k + r], a[k + i]);
+    }
+#pragma unroll
+    for (int i0 = k + 4; i0 < kSub; i0 += 4) {
+      float4 r[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) r[e] = row[i0 + e];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].x, a[k], a[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].y, a[k + 1], a[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].z, a[k + 2], a[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) a[i0 + e] = fmaf(-r[e].w, a[k + 3], a[i0 + e]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kSub; ++i)
+    col[i * kLeafLd] = a[i];
+}
+
+// xd <- d^-1 for an upper-triangular 32 x 32 block by one warp: right-looking back substitution, four rows at a time; zeros below the diagonal.
+__device__ __forceinline__ void invert_diagonal(const float* d, float* xd) {
+  const int lane = threadIdx.x & 31;
+  float x[kSub];
+#pragma unroll
+  for (int i = 0; i < kSub; ++i) x[i] = 0.f;
+#pragma unroll
+  for (int q = kSub - 4; q >= 0; q -= 4) {
+    float4 r4[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) r4[e] = *(const float4*)(d + (q + e) * kLeafLd + q);
+#pragma unroll
+    for (int i = q + 3; i >= q; --i) {
+      const float v[4] = {r4[i - q].x, r4[i - q].y, r4[i - q].z, r4[i - q].w};
+#pragma unroll
+      for (int c = 3; c > 0; --c)
+        if (q + c > i) x[i] = fmaf(v[c], x[q + c], x[i]);
+      const float piv = v[i - q], own = 1.0f / piv, other = -x[i] / piv;
+      x[i] = i == lane ? own : (i < lane ? other : 0.f);
+    }
+#pragma unroll
+    for (int i0 = q - 4; i0 >= 0; i0 -= 4) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) r4[e] = *(const float4*)(d + (i0 + e) * kLeafLd + q);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i0 + e] = fmaf(r4[e].w, x[q + 3], x[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i0 + e] = fmaf(r4[e].z, x[q + 2], x[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i0 + e] = fmaf(r4[e].y, x[q + 1], x[i0 + e]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) x[i0 + e] = fmaf(r4[e].x, x[q], x[i0 + e]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < kSub; ++i) xd[i * kLeafLd + lane] = x[i];
+}
+
+// s += a b for a lane's 2 x 2 values of a product of 32 x 32 blocks: `a` at its first row, `b` at its first column.
+__device__ __forceinline__ void tile_times(float (&s)[2][2], const float* a, const float* b) {
+#pragma unroll
+  for (int k = 0; k < kSub; k += 8) {
+    float4 m[2][2];
+    float2 v[8];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      m[0][e] = *(const float4*)(a + k + 4 * e);
+      m[1][e] = *(const float4*)(a + kLeafLd + k + 4 * e);
+    }
+#pragma unroll
+    for (int e = 0; e < 8; ++e) v[e] = *(const float2*)(b + (k + e) * kLeafLd);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float4 p4 = m[0][e >> 2], q4 = m[1][e >> 2];
+      const float p = (e & 3) == 0 ? p4.x : (e & 3) == 1 ? p4.y : (e & 3) == 2 ? p4.z : p4.w;
+      const float q = (e & 3) == 0 ? q4.x : (e & 3) == 1 ? q4.y : (e & 3) == 2 ? q4.z : q4.w;
+      s[0][0] = fmaf(p, v[e].x, s[0][0]); s[0][1] = fmaf(p, v[e].y, s[0][1]);
+      s[1][0] = fmaf(q, v[e].x, s[1][0]); s[1][1] = fmaf(q, v[e].y, s[1][1]);
+    }
+  }
+}
+// Column J of the inverse above its diagonal block, by eight warps that meet at barrier `kBar`.
+template <int kBar>
+__device__ __forceinline__ void invert_column(const float* t, float* x, int J, int warp) {
+  const int lane = threadIdx.x & 31, r0 = (warp >> 1) * 8 + (lane >> 3) * 2, c0 = (warp & 1) * 16 + (lane & 7) * 2;
 #pragma unroll 1
-  for (int dist = 1; dist < kSubs; ++dist) {
-    const int J = I + dist;
-    const bool on = J < kSubs;
-    if (on) {  // S = sum_K R_IK X_KJ, parked in the mirror position below the diagonal
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int k = kSub * (I + 1); k < kSub * (J + 1); k += 4) {
-        float xv[4];
+  for (int I = J - 1; I >= 0; --I) {
+    float s[2][2] = {};
+#pragma unroll 1
+    for (int K = I + 1; K <= J; ++K) tile_times(s, t + (kSub * I + r0) * kLeafLd + kSub * K, x + kSub * K * kLeafLd + kSub * J + c0);
+    float* park = x + kSub * J * kLeafLd + kSub * I;
+    *(float2*)(park + r0 * kLeafLd + c0) = make_float2(s[0][0], s[0][1]);
+    *(float2*)(park + (r0 + 1) * kLeafLd + c0) = make_float2(s[1][0], s[1][1]);
+    s[0][0] = s[0][1] = s[1][0] = s[1][1] = 0.f;
+    part_sync<256>(kBar);
+    tile_times(s, x + (kSub * I + r0) * kLeafLd + kSub * I, park + c0);
+    float* to = x + (kSub * I + r0) * kLeafLd + kSub * J + c0;
+    *(float2*)to = make_float2(-s[0][0], -s[0][1]);
+    *(float2*)(to + kLeafLd) = make_float2(-s[1][0], -s[1][1]);
+    part_sync<256>(kBar);
+  }
+}
+
+
+// x <- t^-1 for the upper-triangular block t; the part of x below the diagonal blocks is scratch.
+__device__ __forceinline__ void invert_upper(const float* t, float* x, int warp) {
+  if (warp < kSubs) invert_diagonal(t + warp * kSub * (kLeafLd + 1), x + warp * kSub * (kLeafLd + 1));
+  __syncthreads();
+  if (warp < 8) {
+    invert_column<kLowWarps>(t, x, 3, warp);
+  } else {
+    invert_column<kHighWarps>(t, x, 1, warp - 8);
+    invert_column<kHighWarps>(t, x, 2, warp - 8);
+  }
+  __syncthreads();
+}
+
+__device__ __forceinline__ void store_upper(const float* x, float* out) {
 #pragma unroll
-        for (int e = 0; e < 4; ++e) xv[e] = x[(k + e) * kLeafLd + kSub * J + lane];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const float4 a = *(const float4*)(t + (kSub * I + r0 + r) * kLeafLd + k);
-          s[r] = fmaf(a.x, xv[0], s[r]); s[r] = fmaf(a.y, xv[1], s[r]); s[r] = fmaf(a.z, xv[2], s[r]); s[r] = fmaf(a.w, xv[3], s[r]);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r) x[(kSub * J + r0 + r) * kLeafLd + kSub * I + lane] = s[r];
-    }
-    __syncthreads();
-    if (on) {
-      float s[4] = {0.f, 0.f, 0.f, 0.f};
-      for (int k = r0; k < kSub; k += 4) {  // X_II is upper triangular: columns left of the row are zero
-        float sv[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) sv[e] = x[(kSub * J + k + e) * kLeafLd + kSub * I + lane];
-#pragma unroll
-        for (int r = 0; r < 4; ++r) {
-          const float4 a = *(const float4*)(x + (kSub * I + r0 + r) * kLeafLd + kSub * I + k);
-          s[r] = fmaf(a.x, sv[0], s[r]); s[r] = fmaf(a.y, sv[1], s[r]); s[r] = fmaf(a.z, sv[2], s[r]); s[r] = fmaf(a.w, sv[3], s[r]);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 4; ++r) x[(kSub * I + r0 + r) * kLeafLd + kSub * J + lane] = -s[r];
-    }
-    __syncthreads();
+  for (int e = 0; e < kLoads; ++e) {
+    const int idx = threadIdx.x + e * kLeafThreads, i = idx >> 5, j = (idx & 31) * 4;
+    const float4 v = *(const float4*)(x + i * kLeafLd + j);
+    *(float4*)(out + i * kTriBlock + j) = make_float4(j >= i ? v.x : 0.f, j + 1 >= i ? v.y : 0.f, j + 2 >= i ? v.z : 0.f, j + 3 >= i ? v.w : 0.f);
   }
 }
 
@@ -243,14 +435,11 @@ __global__ void __launch_bounds__(kLeafThreads) tri_inv_blocks_kernel(const floa
   extern __shared__ __align__(16) float leaf_smem[];
   float *t = leaf_smem, *x = leaf_smem + kTriBlock * kLeafLd;
   const int blk = blockIdx.x, b = blockIdx.y, r0 = blk * kTriBlock;
-  load_upper(Q + (long long)b * strideQ + (long long)r0 * ld + r0, ld, min(kTriBlock, n - r0), t, x);
+  const int warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0);
+  load_upper(Q + (long long)b * strideQ + (long long)r0 * ld + r0, ld, min(kTriBlock, n - r0), t);
   __syncthreads();
-  invert_upper(t, x);
-  float* out = X + ((long long)b * gridDim.x + blk) * kTriBlock * kTriBlock;
-  for (int idx = threadIdx.x; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
-    const int i = idx >> 7, j = idx & (kTriBlock - 1);
-    out[idx] = j >= i ? x[i * kLeafLd + j] : 0.f;
-  }
+  invert_upper(t, x, warp);
+  store_upper(x, X + ((long long)b * gridDim.x + blk) * kTriBlock * kTriBlock);
 }
 
 __global__ void __launch_bounds__(kLeafThreads) chol_inv_leaf_kernel(const float* __restrict__ G, long long ldg, long long strideG,
@@ -259,89 +448,80 @@ __global__ void __launch_bounds__(kLeafThreads) chol_inv_leaf_kernel(const float
                                                                      int* __restrict__ info) {
   extern __shared__ __align__(16) float leaf_smem[];
   float *t = leaf_smem, *x = leaf_smem + kTriBlock * kLeafLd;
-  __shared__ float inv_piv[kSub];
+  __shared__ __align__(16) Panel P;
   __shared__ int failed;
-  const int b = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int b = blockIdx.x, tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, (int)threadIdx.x >> 5, 0), lane = tid & 31;
   if (tid == 0) failed = 0;
   griddep_wait();
   griddep_launch();
-  load_upper(G + (long long)b * strideG, ldg, size, t, x);
+  load_upper(G + (long long)b * strideG, ldg, size, t);
   __syncthreads();
-
-  for (int base = 0; base < size; base += kSub) {
-    float* d = t + base * (kLeafLd + 1);
+  const int panels = (size + kSub - 1) / kSub;
+#pragma unroll 1
+  for (int J = 0; J < kSubs; ++J) {
+    float* d = t + J * kSub * (kLeafLd + 1);
+    float* xd = x + J * kSub * (kLeafLd + 1);
+    const int nb = kSubs - 1 - J;  // blocks right of the diagonal
+    // warp 0: the diagonal block; 1 .. 3: the columns right of it; 8 .. 15: column J - 1 of the inverse
     if (warp == 0) {
-      float a[kSub];
-      bool bad = false;
-#pragma unroll
-      for (int i = 0; i < kSub; ++i) a[i] = d[i * kLeafLd + lane];
-#pragma unroll
-      for (int k = 0; k < kSub; ++k) {
-        const float piv = __shfl_sync(0xffffffffu, a[k], k);
-        const bool ok = piv > 0.f && piv < 3.0e38f;
-        const float inv = ok ? rsqrtf(piv) : 1.f;
-        bad = bad || !ok;
-        if (lane == k) {
-          a[k] = ok ? piv * inv : 1.f;  // sqrt of the pivot
-          inv_piv[k] = inv;
-        } else {
-          a[k] *= inv;
-        }
-#pragma unroll
-        for (int i = k + 1; i < kSub; ++i) a[i] = fmaf(-__shfl_sync(0xffffffffu, a[k], i), a[k], a[i]);
+      if (J < panels) {
+        const bool bad = factor_diagonal(d, P);
+        if (lane == 0 && bad) failed = 1;
       }
-#pragma unroll
-      for (int i = 0; i < kSub; ++i)
-        if (i <= lane) d[i * kLeafLd + lane] = a[i];
-      if (lane == 0 && bad) failed = 1;
+    } else if (warp < 4) {
+      if (J < panels) follow_panel(d + (warp <= nb ? warp * kSub : 0) + lane, P, warp <= nb);
+    } else if (warp >= 8 && J > 0) {
+      if (warp == 8) invert_diagonal(d - kSub * (kLeafLd + 1), xd - kSub * (kLeafLd + 1));
+      part_sync<256>(kLowWarps);
+      invert_column<kLowWarps>(t, x, J - 1, warp - 8);
     }
     __syncthreads();
-    const int rest = kTriBlock - base - kSub;  // columns right of the panel
-    if (tid < rest) {
-      float* col = d + kSub + tid;
-      float a[kSub];
+    // trailing blocks (I, K), I <= K, sixteen rows of a block per warp; a lane has 4 x 4 values
+    if (J < panels && warp < nb * (nb + 1)) {
+      const int I = warp < 2 * nb ? 0 : warp < 4 * nb - 2 ? 1 : 2, K = (warp >> 1) - (I == 0 ? 0 : I == 1 ? nb - 1 : 2 * nb - 3);
+      const int i0 = kSub * I + (warp & 1) * 16 + (lane >> 3) * 4, j0 = kSub * K + (lane & 7) * 4;
+      const float* panel = d + kSub;
+      float* trail = d + kSub * (kLeafLd + 1);
+      float v[4][4];
 #pragma unroll
-      for (int i = 0; i < kSub; ++i) a[i] = col[i * kLeafLd];
-#pragma unroll
-      for (int k = 0; k < kSub; ++k) {
-        a[k] *= inv_piv[k];
-#pragma unroll
-        for (int i = k + 1; i < kSub; ++i) a[i] = fmaf(-d[k * kLeafLd + i], a[k], a[i]);
-        col[k * kLeafLd] = a[k];
+      for (int r = 0; r < 4; ++r) {
+        const float4 q = *(const float4*)(trail + (i0 + r) * kLeafLd + j0);
+        v[r][0] = q.x; v[r][1] = q.y; v[r][2] = q.z; v[r][3] = q.w;
       }
-    }
-    __syncthreads();
-    if (warp * 4 < rest) {  // rows i0 .. i0+3 of the trailing block, columns from the 32-block of i0 on
-      const int i0 = warp * 4, first = i0 & ~(kSub - 1);
-      const float* panel = d + kSub;  // panel[k * ld + i] = r_ki of trailing row / column i
-      float* trail = t + (base + kSub) * (kLeafLd + 1);
-      for (int j = first + lane; j < rest; j += kSub) {
-        float acc[4];
+#pragma unroll 4
+      for (int k = 0; k < kSub; k += 4) {
+        float4 m[4], c[4];
 #pragma unroll
-        for (int r = 0; r < 4; ++r) acc[r] = trail[(i0 + r) * kLeafLd + j];
-#pragma unroll 8
-        for (int k = 0; k < kSub; ++k) {
-          const float4 m = *(const float4*)(panel + k * kLeafLd + i0);
-          const float rkj = panel[k * kLeafLd + j];
-          acc[0] = fmaf(-m.x, rkj, acc[0]); acc[1] = fmaf(-m.y, rkj, acc[1]);
-          acc[2] = fmaf(-m.z, rkj, acc[2]); acc[3] = fmaf(-m.w, rkj, acc[3]);
+        for (int e = 0; e < 4; ++e) {
+          m[e] = *(const float4*)(panel + (k + e) * kLeafLd + i0);
+          c[e] = *(const float4*)(panel + (k + e) * kLeafLd + j0);
         }
 #pragma unroll
-        for (int r = 0; r < 4; ++r)
-          if (j >= i0 + r) trail[(i0 + r) * kLeafLd + j] = acc[r];
+        for (int e = 0; e < 4; ++e) {
+          const float mv[4] = {m[e].x, m[e].y, m[e].z, m[e].w}, cv[4] = {c[e].x, c[e].y, c[e].z, c[e].w};
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = fmaf(-mv[i], cv[j], v[i][j]);
+        }
       }
+      // (left of the diagonal: nobody reads it)
+#pragma unroll
+      for (int r = 0; r < 4; ++r) *(float4*)(trail + (i0 + r) * kLeafLd + j0) = make_float4(v[r][0], v[r][1], v[r][2], v[r][3]);
     }
     __syncthreads();
   }
-
-  invert_upper(t, x);
-
-  float* r = R + (long long)b * strideR;
-  float* out = X + (long long)b * strideX;
-  for (int idx = tid; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
-    const int i = idx >> 7, j = idx & (kTriBlock - 1);
-    if (R != nullptr && i < size && j < size) r[(long long)i * ldr + j] = j >= i ? t[i * kLeafLd + j] : 0.f;
-    out[idx] = j >= i ? x[i * kLeafLd + j] : 0.f;
+  if (warp == 0) invert_diagonal(t + (kSubs - 1) * kSub * (kLeafLd + 1), x + (kSubs - 1) * kSub * (kLeafLd + 1));
+  __syncthreads();
+  if (warp < 8) invert_column<kLowWarps>(t, x, kSubs - 1, warp);
+  __syncthreads();
+  store_upper(x, X + (long long)b * strideX);
+  if (R != nullptr) {
+    float* r = R + (long long)b * strideR;
+    for (int idx = tid; idx < kTriBlock * kTriBlock; idx += kLeafThreads) {
+      const int i = idx >> 7, j = idx & (kTriBlock - 1);
+      if (i < size && j < size) r[(long long)i * ldr + j] = j >= i ? t[i * kLeafLd + j] : 0.f;
+    }
   }
   if (tid == 0 && failed && info != nullptr) atomicAdd(info + b, 1);
 }
