@@ -8,7 +8,9 @@
 // transpose of R[lo:mid, mid:hi], and every product that reads either - the Schur complement, the updates inside later solves, those of the
 // rows of A - wants its rows split into [hi | lo].  So the factor exists in that form alone (L, rows of R^T), written by the kernel that solves
 // against a leaf, and its blocks are operands by address; rows of A are split by the same kernel, in both orientations.  That leaves no
-// operand passes, no copies and no transposes between the products: 49 launches in the place of 95 for a 1024-wide round.
+// operand passes, no copies and no transposes between the products: 49 launches in the place of 95 for a 1024-wide round.  Two rounds and the
+// check, replayed, in that form / this: 16 of 1024^2 2.96 / 2.00 ms, 11 of 2048^2 8.33 / 6.09, 8 of 256^2 0.376 / 0.237 (half of it from the
+// leaf kernel, which bounds it now: 16 leaves of 25 us, 10 products over whole columns of 91 and 18, the others 8 to 25 us each).
 // The products, their tiles and their sums are those of the launch-by-launch form (utils/orthogonal.py), and so are the bits of the result.
 #include "chol_qr.h"
 
@@ -20,9 +22,9 @@
 namespace hb {
 namespace {
 
-constexpr int kLeafSolveThreads = 256;
+constexpr int kLeafSolveThreads = 512, kLeafSolveWarps = kLeafSolveThreads / 32;
 constexpr int kRowLd = kQrBlock + 4;  // floats per staged row: four values of K per lane and load, lanes on distinct banks
-constexpr int kLeafSolveBytes = (kQrBlock * kQrBlock + kQrRows * kRowLd) * (int)sizeof(float);
+constexpr int leaf_solve_bytes(int lane_rows) { return (kQrBlock * kQrBlock + 32 * lane_rows * kRowLd) * (int)sizeof(float); }
 
 __device__ __forceinline__ float qr_tf32(float x) {
   uint32_t bits;
@@ -35,76 +37,80 @@ __device__ __forceinline__ unsigned long long twice(float x) {
   return r;
 }
 
-// 64 rows x 128 columns of X per block, sums over K in its order in fp32.  A warp has 16 columns of all rows, a lane two rows: 16 paired
-// multiply-adds per four (broadcast) loads of the inverse and half a load of B.  Only k up to the warp's last column: the inverse is
-// upper triangular.  Column groups are dealt to warps so that the four schedulers get the same number of steps.
+// 32 kLaneRows rows x 128 columns of X per block, sums over K in its order in fp32.  A warp has 8 columns of all rows, a lane kLaneRows of the rows:
+// per k two (broadcast) loads of the inverse, half a load of B and four paired multiply-adds per row.  Only k up to the warp's last column: the
+// inverse is upper triangular.  Column groups are dealt to warps so that the four schedulers get the same number of steps.
+template <int kLaneRows>
 __global__ void __launch_bounds__(kLeafSolveThreads, 2) qr_leaf_solve_kernel(const QrLeafSolve S) {
+  constexpr int kRows = 32 * kLaneRows;
   extern __shared__ __align__(16) float qr_smem[];
   float *const t = qr_smem, *const b = qr_smem + kQrBlock * kQrBlock;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = blockIdx.x * kQrRows;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r0 = blockIdx.x * kRows;
   const int64_t batch = blockIdx.y;
   griddep_wait();
   griddep_launch();
   const float* inv = S.inv + batch * S.stride_inv;
-#pragma unroll 4
-  for (int i = threadIdx.x; i < kQrBlock * kQrBlock / 4; i += kLeafSolveThreads) ((float4*)t)[i] = ((const float4*)inv)[i];
+#pragma unroll
+  for (int i = 0; i < kQrBlock / kLeafSolveWarps; ++i) {  // (what lies left of the diagonal is needed as far as its group of eight columns)
+    const int r = warp + kLeafSolveWarps * i;
+    if (lane * 4 + 7 >= r) *(float4*)(t + r * kQrBlock + lane * 4) = *(const float4*)(inv + r * kQrBlock + lane * 4);
+  }
   const float* src = S.src + batch * S.stride;
   if (!S.from_rows) {
 #pragma unroll
-    for (int i = 0; i < kQrRows / 8; ++i) {
-      const int r = warp + 8 * i;
+    for (int i = 0; i < kRows / kLeafSolveWarps; ++i) {
+      const int r = warp + kLeafSolveWarps * i;
       *(float4*)(b + r * kRowLd + lane * 4) = *(const float4*)(src + (int64_t)(r0 + r) * S.ld + lane * 4);
     }
-  } else {  // 4 x 4 values per thread and step, turned in registers
+  } else if (threadIdx.x < 32 * kRows / 4) {  // 4 x 4 values per thread, turned in registers
+    const int r = threadIdx.x % (kRows / 4) * 4, k = threadIdx.x / (kRows / 4) * 4;
+    float4 v[4];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int r = (lane & 15) * 4, k = ((lane >> 4) + 2 * warp + 16 * i) * 4;
-      float4 v[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) v[e] = *(const float4*)(src + (int64_t)(k + e) * S.ld + r0 + r);
-      *(float4*)(b + (r + 0) * kRowLd + k) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
-      *(float4*)(b + (r + 1) * kRowLd + k) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
-      *(float4*)(b + (r + 2) * kRowLd + k) = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
-      *(float4*)(b + (r + 3) * kRowLd + k) = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
-    }
+    for (int e = 0; e < 4; ++e) v[e] = *(const float4*)(src + (int64_t)(k + e) * S.ld + r0 + r);
+    *(float4*)(b + (r + 0) * kRowLd + k) = make_float4(v[0].x, v[1].x, v[2].x, v[3].x);
+    *(float4*)(b + (r + 1) * kRowLd + k) = make_float4(v[0].y, v[1].y, v[2].y, v[3].y);
+    *(float4*)(b + (r + 2) * kRowLd + k) = make_float4(v[0].z, v[1].z, v[2].z, v[3].z);
+    *(float4*)(b + (r + 3) * kRowLd + k) = make_float4(v[0].w, v[1].w, v[2].w, v[3].w);
   }
   __syncthreads();
 
-  const int c0 = (warp < 4 ? warp : 11 - warp) * 16;
-  unsigned long long acc[2][8];  // two neighbouring columns each
+  // groups g, 7 - g, 8 + g and 15 - g on one scheduler
+  const int c0 = ((warp & 4) != 0 ? (warp ^ 3) : warp) * 8;
+  unsigned long long acc[kLaneRows][4];  // two neighbouring columns each
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
+  for (int r = 0; r < kLaneRows; ++r)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[r][j] = 0ull;
-#pragma unroll 1
-  for (int k = 0; k < c0 + 16; k += 4) {
-    const float4 b0 = *(const float4*)(b + lane * kRowLd + k), b1 = *(const float4*)(b + (lane + 32) * kRowLd + k);
-    const float x0[4] = {b0.x, b0.y, b0.z, b0.w}, x1[4] = {b1.x, b1.y, b1.z, b1.w};
+    for (int j = 0; j < 4; ++j) acc[r][j] = 0ull;
+#pragma unroll 2
+  for (int k = 0; k < c0 + 8; k += 4) {
+    float4 x[kLaneRows];
+#pragma unroll
+    for (int r = 0; r < kLaneRows; ++r) x[r] = *(const float4*)(b + (lane + 32 * r) * kRowLd + k);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
-      const unsigned long long p0 = twice(x0[e]), p1 = twice(x1[e]);
+      const ulonglong2 m0 = *(const ulonglong2*)(t + (k + e) * kQrBlock + c0), m1 = *(const ulonglong2*)(t + (k + e) * kQrBlock + c0 + 4);
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const ulonglong2 m = *(const ulonglong2*)(t + (k + e) * kQrBlock + c0 + q * 4);
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[0][2 * q]) : "l"(p0), "l"(m.x));
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[0][2 * q + 1]) : "l"(p0), "l"(m.y));
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[1][2 * q]) : "l"(p1), "l"(m.x));
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[1][2 * q + 1]) : "l"(p1), "l"(m.y));
+      for (int r = 0; r < kLaneRows; ++r) {
+        const unsigned long long p = twice(e == 0 ? x[r].x : e == 1 ? x[r].y : e == 2 ? x[r].z : x[r].w);
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[r][0]) : "l"(p), "l"(m0.x));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[r][1]) : "l"(p), "l"(m0.y));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[r][2]) : "l"(p), "l"(m1.x));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[r][3]) : "l"(p), "l"(m1.y));
       }
     }
   }
   __syncthreads();  // B has been read: its place takes X
 #pragma unroll
-  for (int r = 0; r < 2; ++r)
-#pragma unroll
-    for (int q = 0; q < 4; ++q)
-      *(ulonglong2*)(b + (lane + 32 * r) * kRowLd + c0 + q * 4) = make_ulonglong2(acc[r][2 * q], acc[r][2 * q + 1]);
+  for (int r = 0; r < kLaneRows; ++r) {
+    *(ulonglong2*)(b + (lane + 32 * r) * kRowLd + c0) = make_ulonglong2(acc[r][0], acc[r][1]);
+    *(ulonglong2*)(b + (lane + 32 * r) * kRowLd + c0 + 4) = make_ulonglong2(acc[r][2], acc[r][3]);
+  }
   __syncthreads();
 
   if (S.out != nullptr || S.same != nullptr) {
 #pragma unroll
-    for (int i = 0; i < kQrRows / 8; ++i) {
-      const int r = warp + 8 * i;
+    for (int i = 0; i < kRows / kLeafSolveWarps; ++i) {
+      const int r = warp + kLeafSolveWarps * i;
       const float4 x = *(const float4*)(b + r * kRowLd + lane * 4);
       if (S.out != nullptr) *(float4*)(S.out + batch * S.stride_out + (int64_t)(r0 + r) * S.ld_out + lane * 4) = x;
       if (S.same != nullptr) {
@@ -115,10 +121,10 @@ __global__ void __launch_bounds__(kLeafSolveThreads, 2) qr_leaf_solve_kernel(con
       }
     }
   }
-  if (S.trans != nullptr) {  // consecutive lanes on consecutive rows: half a column is a line
+  if (S.trans != nullptr) {  // consecutive lanes on consecutive rows: 32 of a column are a line
 #pragma unroll 4
-    for (int i = warp; i < 2 * kQrBlock; i += kLeafSolveThreads / 32) {
-      const int c = i >> 1, r = (i & 1) * 32 + lane;
+    for (int i = warp; i < kLaneRows * kQrBlock; i += kLeafSolveWarps) {
+      const int c = i / kLaneRows, r = i % kLaneRows * 32 + lane;
       const float x = b[r * kRowLd + c], hi = qr_tf32(x);
       float* to = S.trans + batch * S.stride_trans + (int64_t)c * S.ld_trans + r0 + r;
       to[0] = hi;
@@ -254,18 +260,26 @@ struct Round {
 }  // namespace
 
 cudaError_t launch_qr_leaf_solve(const QrLeafSolve& S, int rows, int batch, cudaStream_t stream) {
-  static PerDevice<bool> configured;
-  int device = 0;
+  static PerDevice<int> resident;  // blocks of 32 rows
+  int device = 0, slots = 0;
   cudaError_t e = cudaGetDevice(&device);
-  bool done = false;
   if (e == cudaSuccess)
-    e = configured.get(device, cudaSuccess, &done, [](bool&) {
-      return cudaFuncSetAttribute(qr_leaf_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kLeafSolveBytes);
+    e = resident.get(device, cudaSuccess, &slots, [device](int& found) {
+      int sms = 0;
+      cudaError_t s = cudaFuncSetAttribute(qr_leaf_solve_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, leaf_solve_bytes(1));
+      if (s == cudaSuccess) s = cudaFuncSetAttribute(qr_leaf_solve_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, leaf_solve_bytes(2));
+      if (s == cudaSuccess) s = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+      found = 2 * sms;
+      return s;
     });
   if (e != cudaSuccess) return e;
   if (rows % kQrRows != 0 || batch > 65535) return cudaErrorInvalidValue;
   if (rows == 0 || batch == 0) return cudaSuccess;
-  return launch_chained(qr_leaf_solve_kernel, dim3(rows / kQrRows, batch), kLeafSolveThreads, kLeafSolveBytes, stream, S);
+  // few rows: the chain waits for one block, and one of 32 rows is done sooner (rows of 16 matrices, 64 / 32 per block: 128 rows 11.8 / 8.2 us, 512
+  // rows 12.0 / 11.7); more than fit at once: 64, the inverse is read half as often
+  if ((int64_t)(rows / 32) * batch <= slots)
+    return launch_chained(qr_leaf_solve_kernel<1>, dim3(rows / 32, batch), kLeafSolveThreads, leaf_solve_bytes(1), stream, S);
+  return launch_chained(qr_leaf_solve_kernel<2>, dim3(rows / 64, batch), kLeafSolveThreads, leaf_solve_bytes(2), stream, S);
 }
 
 cudaError_t launch_chol_qr_round(const QrRound& Q, int* launches, cudaStream_t stream) {
