@@ -431,6 +431,15 @@ at::Tensor cross_entropy_(at::Tensor& logits, const at::Tensor& targets, const a
   return loss;
 }
 
+// x *= s[0] in place for a contiguous fp32 or bf16 tensor; s: one fp32 value on the same device.
+void scale_(const at::Tensor& x, const at::Tensor& s) {
+  TORCH_CHECK(x.is_cuda() && x.is_contiguous() && (x.scalar_type() == at::kFloat || x.scalar_type() == at::kBFloat16) && aligned16(x.data_ptr()),
+              "scale_: contiguous fp32 or bf16 CUDA tensor");
+  TORCH_CHECK(s.device() == x.device() && s.scalar_type() == at::kFloat && s.numel() == 1, "scale_: fp32 device scalar");
+  c10::cuda::CUDAGuard guard(x.device());
+  check(hb::launch_scale(x.data_ptr(), x.scalar_type() == at::kBFloat16, x.numel(), s.data_ptr<float>(), at::cuda::getCurrentCUDAStream()), "scale launch");
+}
+
 // Split-tf32 operands of a contiguous fp32 [batch, R, C] tensor: rows of [hi | lo] (see tf32_gemm.h).  Returns
 // (same, trans): same = [batch, R, 2 kp(C)] (operand rows = rows of x), trans = [batch, C, 2 kp(R)] (operand rows =
 // columns of x); an orientation that was not asked for comes back undefined.
@@ -932,6 +941,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("layer_norm_bwd", &layer_norm_bwd);
   m.def("layer_norm_supported", &hb::layer_norm_supported);
   m.def("cross_entropy_", &cross_entropy_);
+  m.def("scale_", &scale_);
   m.def("peer_signal", &peer_signal);
   m.def("peer_wait", &peer_wait);
   m.attr("MAX_WORLD") = hb::kMaxWorld;

@@ -40,6 +40,15 @@ def _mm_f32(a: torch.Tensor, b: torch.Tensor) -> torch.Tensor:
         return torch.mm(a, b).float()
 
 
+def _times(x: torch.Tensor, grad_out: torch.Tensor) -> torch.Tensor:
+    """``x *= grad_out`` for a fresh gradient and the (0-dim, fp32) gradient of the loss."""
+    if grad_out.dtype != torch.float32 or grad_out.requires_grad:
+        return x.mul_(grad_out)
+    launch_counter.count += 1
+    load().scale_(x, grad_out)
+    return x
+
+
 class _LinearCrossEntropy(torch.autograd.Function):
     @staticmethod
     def forward(ctx, h, weight, targets, vocab, ignore_index):
@@ -61,9 +70,9 @@ class _LinearCrossEntropy(torch.autograd.Function):
         (h_shape, h_dtype), w_dtype = ctx.h_meta, ctx.w_dtype
         dh = dw = None
         if ctx.needs_input_grad[0]:
-            dh = (dlogits @ w16).mul_(grad_out).reshape(h_shape).to(h_dtype)
+            dh = _times(dlogits @ w16, grad_out).reshape(h_shape).to(h_dtype)
         if ctx.needs_input_grad[1]:
-            dw = _mm_f32(dlogits.mT, h16).mul_(grad_out).to(w_dtype)
+            dw = _times(_mm_f32(dlogits.mT, h16), grad_out).to(w_dtype)
         return dh, dw, None, None, None
 
 

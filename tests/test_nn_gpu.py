@@ -52,6 +52,28 @@ def test_linear_cross_entropy_gradients_match_autograd_of_plain_ops():
     assert (w.grad[vocab:] == 0).all()
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [1, 7, 8, 2047, 2048, 2049, 5_000_003])
+def test_scaling_by_the_gradient_of_the_loss_has_the_bits_of_the_library(dtype, n):
+    x = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(n)).to(dtype)
+    for by in (1.0, 0.3, -2.0, float("inf"), float("nan")):
+        s = torch.tensor(by, device="cuda")
+        got, want = x.clone(), x.clone().mul_(s)
+        ops.load().scale_(got, s)
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0))
+
+
+@pytest.mark.parametrize("by", [1.0, 0.25])
+def test_head_gradients_are_scaled_by_the_gradient_of_the_loss(by):
+    torch.manual_seed(1)
+    h, w = torch.randn(64, 128, device="cuda", requires_grad=True), (torch.randn(512, 128, device="cuda") * 0.05).requires_grad_()
+    loss = linear_cross_entropy(h, w, torch.randint(0, 500, (64,), device="cuda"), 500)
+    unit = torch.autograd.grad(loss, (h, w), retain_graph=True)
+    scaled = torch.autograd.grad(loss * by, (h, w))
+    for a, b in zip(unit, scaled):  # powers of two are exact in either type
+        assert torch.equal(a * by, b)
+
+
 def test_gpt_pads_its_vocabulary_and_trains():
     from heavyball_b200.models import GPT, GPTConfig
 
