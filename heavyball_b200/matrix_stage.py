@@ -29,7 +29,7 @@ import torch
 from torch import Tensor
 
 from . import ops, utils
-from .utils.core import _mm
+from .utils.core import _captured_into, _mm
 
 MIN_TC_DIM = 128  # below this a 128 x 128 tensor-core tile is mostly padding: use the library product
 
@@ -155,7 +155,7 @@ class Captured:
         if self.graph is None:
             try:
                 graph = torch.cuda.CUDAGraph()
-                with torch.cuda.graph(graph):  # own memory pool: it lives exactly as long as this graph
+                with _captured_into(graph):  # own memory pool: it lives exactly as long as this graph
                     fn()
                 self.graph = graph
             except Exception as err:  # noqa: BLE001 - whatever stops capture, the eager sequence is still correct

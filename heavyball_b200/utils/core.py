@@ -13,7 +13,9 @@ semantics those kernels are tested against, and the fallback for chains that are
 
 from __future__ import annotations
 
+import contextlib
 import enum
+import gc
 import sys
 import warnings
 from typing import Iterable, List, Optional, Sequence, Union
@@ -483,6 +485,20 @@ def _mm_upper(a: Tensor, b: Tensor) -> Tensor:
     walks only the K range where both are non-zero."""
     out = _tc_matmul(a, b, upper_upper=True) if a.ndim == 3 and a.shape == b.shape and a.shape[-1] == a.shape[-2] else None
     return out if out is not None else a @ b
+
+
+@contextlib.contextmanager
+def _captured_into(graph):
+    """``torch.cuda.graph(graph)`` with the automatic collection of reference cycles held meanwhile: a cycle that keeps another graph alive
+    (an optimizer that went out of use) would take that graph down with it, and destroying a graph invalidates any capture."""
+    collecting = gc.isenabled()
+    gc.disable()
+    try:
+        with torch.cuda.graph(graph):
+            yield
+    finally:
+        if collecting:
+            gc.enable()
 
 
 # ---------------------------------------------------------------------------------------- blocked triangular solve

@@ -23,7 +23,7 @@ import torch
 from torch import Tensor
 
 from .core import copy_stochastic_, list_guard, promote, stochastic_divide_, stochastic_divide_with_eps_, stochastic_round_
-from .core import _mm, _solve_right_upper, _tc_sub_product
+from .core import _captured_into, _mm, _solve_right_upper, _tc_sub_product
 
 
 def _settings():
@@ -349,7 +349,7 @@ def _cholesky_qr2_replayed(x: Tensor, shifted_rounds: int = 0):
         try:
             static_in = x.clone()
             graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
+            with _captured_into(graph):
                 static_out, static_bad = _cholesky_qr2(static_in, shifted_rounds)
             slot[1] = (graph, static_in, static_out, static_bad)
         except Exception as err:  # noqa: BLE001 - any capture failure means "do not graph this shape"
@@ -395,7 +395,7 @@ def _panel_qr_replayed(x: Tensor, fallback: Tensor = None):
         try:
             static_in = x.clone()
             graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
+            with _captured_into(graph):
                 static_out, static_bad = _panel_cholesky_qr(static_in, defer_check=True)
             slot[1] = (graph, static_in, static_out, static_bad)
         except Exception as err:  # noqa: BLE001 - any capture failure means "do not graph this shape"
