@@ -33,7 +33,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 _SRC = os.path.join(_HERE, "csrc")
 _BUILD = os.path.join(_HERE, "_build")
 _NAME = "hb200_ops"
-_SOURCES = ["bindings.cpp", "chol_qr.cu", "colsum.cu", "cross_entropy.cu", "fused_chain.cu", "gelu.cu", "layer_norm.cu", "ns_gemm.cu", "noalloc_adamw.cu", "peer_sync.cu", "skinny.cu", "split16_gemm.cu", "tf32_gemm.cu"]
+_SOURCES = ["bindings.cpp", "chol_qr.cu", "colsum.cu", "cross_entropy.cu", "fused_chain.cu", "gelu.cu", "layer_norm.cu", "matrix_passes.cu", "ns_gemm.cu", "noalloc_adamw.cu", "peer_sync.cu", "skinny.cu", "split16_gemm.cu", "tf32_gemm.cu"]
 _lock = threading.Lock()
 _ext = None
 _load_error: Optional[BaseException] = None
@@ -378,13 +378,21 @@ def split16_accumulate(c: torch.Tensor, a: torch.Tensor, b: torch.Tensor, trans_
     launch_counter.count += 3
 
 
+def _dense(x: torch.Tensor, trans: bool):
+    """Contiguous ``x`` and whether it is meant transposed: operands are split in either orientation, so the transpose of a contiguous
+    matrix is used where it lies (a strided copy of 8 x 1024^2 takes 39 us)."""
+    if not x.is_contiguous() and x.mT.is_contiguous():
+        return x.mT, not trans
+    return x.contiguous(), trans
+
+
 def _matmul(kernel, a, b, trans_a, trans_b, alpha, upper_upper):
     lead = a.shape[:-2]
     if b.shape[:-2] != lead:
         lead = torch.broadcast_shapes(a.shape[:-2], b.shape[:-2])
         a, b = a.expand(*lead, *a.shape[-2:]), b.expand(*lead, *b.shape[-2:])
-    a3 = a.reshape(-1, *a.shape[-2:]).contiguous()
-    b3 = b.reshape(-1, *b.shape[-2:]).contiguous()
+    a3, trans_a = _dense(a.reshape(-1, *a.shape[-2:]), trans_a)
+    b3, trans_b = _dense(b.reshape(-1, *b.shape[-2:]), trans_b)
     out = kernel(a3, b3, trans_a, trans_b, alpha, _status(a.device), upper_upper)
     launch_counter.count += 3
     return out.reshape(*lead, *out.shape[-2:])

@@ -19,6 +19,7 @@
 #include "fused_chain.h"
 #include "gelu.h"
 #include "layer_norm.h"
+#include "matrix_passes.h"
 #include "ns_gemm.h"
 #include "peer_sync.h"
 #include "skinny.h"
@@ -782,6 +783,71 @@ std::tuple<at::Tensor, OptT, int> chol_qr_round(const at::Tensor& gram, const at
   return {x, trans, launches};
 }
 
+// (x / norm, split-tf32 operand of its transpose) for contiguous fp32 x: [batch, n, k] and norm: [batch, 1, k]; n a multiple of 64, k of 128.
+std::tuple<at::Tensor, at::Tensor> qr_unit_columns(const at::Tensor& x, const at::Tensor& norm) {
+  for (const at::Tensor* t : {&x, &norm})
+    TORCH_CHECK(t->is_cuda() && t->device() == x.device() && t->scalar_type() == at::kFloat && t->dim() == 3 && t->is_contiguous() && aligned16(t->data_ptr()),
+                "qr_unit_columns: contiguous fp32 CUDA tensors");
+  const int64_t batch = x.size(0), n = x.size(1), k = x.size(2);
+  TORCH_CHECK(n >= 1 && k >= 1 && n % 64 == 0 && k % hb::kQrBlock == 0 && batch <= 65535 && norm.size(0) == batch && norm.size(1) == 1 && norm.size(2) == k,
+              "qr_unit_columns: x of n x k, n a multiple of 64 and k of 128, and one norm per column");
+  c10::cuda::CUDAGuard guard(x.device());
+  const auto options = x.options().memory_format(at::MemoryFormat::Contiguous);
+  const at::Tensor a = at::empty({batch, n, k}, options), trans = at::empty({batch, k, 2 * n}, options);
+  check(hb::launch_qr_unit_columns(x.data_ptr<float>(), norm.data_ptr<float>(), a.data_ptr<float>(), trans.data_ptr<float>(), (int)batch, (int)n, (int)k,
+                                   at::cuda::getCurrentCUDAStream()), "qr_unit_columns launch");
+  return {a, trans};
+}
+
+void check_matrices(const at::Tensor& x, const char* name) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() == 3 && x.is_contiguous() && x.size(0) <= 65535 && x.size(1) < (1 << 22) && x.size(2) < (1 << 22),
+              name, ": contiguous fp32 [batch <= 65535, rows, cols] CUDA tensors");
+}
+
+// Contiguous [batch, C, R] copy of the transposes of x: [batch, R, C].
+at::Tensor transposed(const at::Tensor& x) {
+  check_matrices(x, "transposed");
+  c10::cuda::CUDAGuard guard(x.device());
+  at::Tensor out = at::empty({x.size(0), x.size(2), x.size(1)}, x.options().memory_format(at::MemoryFormat::Contiguous));
+  check(hb::launch_transpose(x.data_ptr<float>(), out.data_ptr<float>(), (int)x.size(0), (int)x.size(1), (int)x.size(2), at::cuda::getCurrentCUDAStream()),
+        "transpose launch");
+  return out;
+}
+
+// a <- a + b, b <- triu(a - b), in place.
+void sum_triu_diff_(const at::Tensor& a, const at::Tensor& b) {
+  check_matrices(a, "sum_triu_diff_");
+  check_matrices(b, "sum_triu_diff_");
+  TORCH_CHECK(a.sizes() == b.sizes() && a.size(1) == a.size(2) && a.device() == b.device() && at::get_overlap_status(a, b) == at::MemOverlapStatus::No,
+              "sum_triu_diff_: two batches of square matrices of one size");
+  c10::cuda::CUDAGuard guard(a.device());
+  check(hb::launch_sum_triu_diff(a.data_ptr<float>(), b.data_ptr<float>(), (int)a.size(0), (int)a.size(1), at::cuda::getCurrentCUDAStream()), "sum_triu_diff launch");
+}
+
+// g + (damp + eps |g|) v for contiguous fp32 tensors of one shape.
+at::Tensor dampen(const at::Tensor& g, const at::Tensor& v, double damp, double eps) {
+  for (const at::Tensor* t : {&g, &v})
+    TORCH_CHECK(t->is_cuda() && t->scalar_type() == at::kFloat && t->is_contiguous() && t->sizes() == g.sizes() && t->device() == g.device(),
+                "dampen: contiguous fp32 CUDA tensors of one shape");
+  c10::cuda::CUDAGuard guard(g.device());
+  at::Tensor out = at::empty_like(g);
+  check(hb::launch_dampen(g.data_ptr<float>(), v.data_ptr<float>(), out.data_ptr<float>(), g.numel(), (float)damp, (float)eps, at::cuda::getCurrentCUDAStream()),
+        "dampen launch");
+  return out;
+}
+
+// line -= packed upper triangle of step / ell * lr, in place.  line: contiguous fp32 [batch, n (n + 1) / 2], ell: contiguous fp32 [batch].
+void triu_step_(const at::Tensor& line, const at::Tensor& step, const at::Tensor& ell, double lr) {
+  check_matrices(step, "triu_step_");
+  const int64_t batch = step.size(0), n = step.size(1);
+  TORCH_CHECK(step.size(2) == n && line.device() == step.device() && line.scalar_type() == at::kFloat && line.is_contiguous() && line.dim() == 2 &&
+                  line.size(0) == batch && line.size(1) == n * (n + 1) / 2, "triu_step_: packed triangles of the matrices' size");
+  TORCH_CHECK(ell.device() == step.device() && ell.scalar_type() == at::kFloat && ell.is_contiguous() && ell.numel() == batch, "triu_step_: one fp32 divisor per matrix");
+  c10::cuda::CUDAGuard guard(step.device());
+  check(hb::launch_triu_step(step.data_ptr<float>(), ell.data_ptr<float>(), line.data_ptr<float>(), (int)batch, (int)n, (float)lr, at::cuda::getCurrentCUDAStream()),
+        "triu_step launch");
+}
+
 // Row-major upper triangles of contiguous [batch, n, n] matrices (2- or 4-byte elements) as [batch, n (n + 1) / 2].
 at::Tensor triu_pack(const at::Tensor& dense) {
   TORCH_CHECK(dense.is_cuda() && dense.dim() == 3 && dense.size(1) == dense.size(2) && dense.is_contiguous() &&
@@ -959,6 +1025,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("chol_inv_leaf", &chol_inv_leaf);
   m.def("chol_qr_round", &chol_qr_round);
+  m.def("qr_unit_columns", &qr_unit_columns);
+  m.def("transposed", &transposed);
+  m.def("sum_triu_diff_", &sum_triu_diff_);
+  m.def("dampen", &dampen);
+  m.def("triu_step_", &triu_step_);
   m.def("triu_pack", &triu_pack);
   m.def("triu_unpack", &triu_unpack);
   m.def("chunk_elems", &hb::chain_chunk_elems);

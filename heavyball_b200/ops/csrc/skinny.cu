@@ -584,6 +584,24 @@ __global__ void __launch_bounds__(256) triu_unpack_kernel(const T* __restrict__ 
   for (int j = threadIdx.x; j < n; j += blockDim.x) dst[j] = j >= (int)i ? src[j] : T(0);
 }
 
+// Four rows and a column of 16-byte stores per step (8 of 1024^2: 9 us, with one row per block and 4-byte stores 14).
+__global__ void __launch_bounds__(256) triu_unpack_wide_kernel(const uint32_t* __restrict__ line, uint32_t* __restrict__ dense, int n) {
+  const long long b = blockIdx.y, len = (long long)n * (n + 1) / 2;
+  const int i0 = blockIdx.x * 4;  // n is a multiple of 4
+  for (int j = threadIdx.x * 4; j < n; j += blockDim.x * 4) {
+    uint32_t v[4][4];
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const long long i = i0 + r;
+      const uint32_t* src = line + b * len + i * n - i * (i - 1) / 2 - i + j;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) v[r][e] = j + e >= i ? src[e] : 0u;
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) *(uint4*)(dense + (b * n + i0 + r) * n + j) = make_uint4(v[r][0], v[r][1], v[r][2], v[r][3]);
+  }
+}
+
 }  // namespace
 
 cudaError_t launch_triu_pack(const void* dense, void* line, int elem_bytes, int batch, int n, cudaStream_t stream) {
@@ -598,7 +616,9 @@ cudaError_t launch_triu_pack(const void* dense, void* line, int elem_bytes, int 
 cudaError_t launch_triu_unpack(const void* line, void* dense, int elem_bytes, int batch, int n, cudaStream_t stream) {
   if (batch == 0 || n == 0) return cudaSuccess;
   dim3 grid(n, batch);
-  if (elem_bytes == 4) triu_unpack_kernel<uint32_t><<<grid, 256, 0, stream>>>((const uint32_t*)line, (uint32_t*)dense, n);
+  if (elem_bytes == 4 && (n & 3) == 0 && ((uintptr_t)dense & 15) == 0)
+    triu_unpack_wide_kernel<<<dim3(n / 4, batch), 256, 0, stream>>>((const uint32_t*)line, (uint32_t*)dense, n);
+  else if (elem_bytes == 4) triu_unpack_kernel<uint32_t><<<grid, 256, 0, stream>>>((const uint32_t*)line, (uint32_t*)dense, n);
   else if (elem_bytes == 2) triu_unpack_kernel<uint16_t><<<grid, 256, 0, stream>>>((const uint16_t*)line, (uint16_t*)dense, n);
   else return cudaErrorInvalidValue;
   return cudaGetLastError();
@@ -606,25 +626,52 @@ cudaError_t launch_triu_unpack(const void* line, void* dense, int elem_bytes, in
 
 // ------------------------------------------------------------------------------------------ around the eigenbasis refresh
 // Passes over n x k matrices that only memory bounds: a block turns a few rows in shared memory, so that both sides are read and written
-// in whole lines (16 of 1024^2: 33 us, back 34; the library's gather and scatter, element by element through 64-bit indices, 54 and 78).
+// in whole lines, 16 bytes per access where rows start on such boundaries (16 of 1024^2, the library's gather and scatter, element by element
+// through 64-bit indices, 54 and 78 us; this with 4 bytes per access 27 each, 11 of 2048^2 195).
+template <typename V>  // float4 or float
 __global__ void __launch_bounds__(256) permute_columns_kernel(const float* __restrict__ x, const long long* __restrict__ order, float* __restrict__ out,
                                                              int n, int k, int rows, int inverse) {
-  extern __shared__ float turned[];  // rows x k
-  const int r0 = blockIdx.x * rows, count = min(rows, n - r0);
+  constexpr int kWide = sizeof(V) / sizeof(float);
+  extern __shared__ __align__(16) float turned[];  // rows x k
+  const int r0 = blockIdx.x * rows, count = min(rows, n - r0), vectors = k / kWide;
   const long long base = ((long long)blockIdx.y * n + r0) * k;
   const long long* o = order + (long long)blockIdx.y * k;
-  for (int j = threadIdx.x; j < k; j += blockDim.x) {
-    const long long to = inverse ? o[j] : j;
-    if (to < 0 || to >= k) continue;
-#pragma unroll 8
-    for (int r = 0; r < count; ++r) turned[r * k + to] = x[base + (long long)r * k + j];
+  const V* from = (const V*)(x + base);
+  V* to = (V*)(out + base);
+  if (!inverse) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < count * vectors; i += blockDim.x) ((V*)turned)[i] = from[i];
+    __syncthreads();
   }
-  __syncthreads();
-  for (int j = threadIdx.x; j < k; j += blockDim.x) {
-    const long long from = inverse ? j : o[j];
-    if (from < 0 || from >= k) continue;
+  for (int j = threadIdx.x; j < vectors; j += blockDim.x) {
+    int at[kWide];
+#pragma unroll
+    for (int e = 0; e < kWide; ++e) {
+      const long long v = o[j * kWide + e];
+      at[e] = v < 0 || v >= k ? -1 : (int)v;
+    }
+    if (inverse) {
 #pragma unroll 8
-    for (int r = 0; r < count; ++r) out[base + (long long)r * k + j] = turned[r * k + from];
+      for (int r = 0; r < count; ++r) {
+        const V v = from[r * vectors + j];
+#pragma unroll
+        for (int e = 0; e < kWide; ++e)
+          if (at[e] >= 0) turned[r * k + at[e]] = ((const float*)&v)[e];
+      }
+    } else {
+#pragma unroll 8
+      for (int r = 0; r < count; ++r) {
+        V v;
+#pragma unroll
+        for (int e = 0; e < kWide; ++e) ((float*)&v)[e] = at[e] >= 0 ? turned[r * k + at[e]] : 0.0f;
+        to[r * vectors + j] = v;
+      }
+    }
+  }
+  if (inverse) {
+    __syncthreads();
+#pragma unroll 4
+    for (int i = threadIdx.x; i < count * vectors; i += blockDim.x) to[i] = ((const V*)turned)[i];
   }
 }
 
@@ -632,7 +679,9 @@ cudaError_t launch_permute_columns(const float* x, const long long* order, float
   if (batch == 0 || n == 0 || k == 0) return cudaSuccess;
   if (k > kMaxPermuted || batch > 65535) return cudaErrorInvalidValue;
   const int rows = kMaxPermuted / k < 8 ? kMaxPermuted / k : 8;  // 48 KB of shared memory at most
-  permute_columns_kernel<<<dim3((n + rows - 1) / rows, batch), 256, (size_t)rows * k * sizeof(float), stream>>>(x, order, out, n, k, rows, inverse);
+  const bool vec = (k & 3) == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0;
+  const auto kernel = vec ? permute_columns_kernel<float4> : permute_columns_kernel<float>;
+  kernel<<<dim3((n + rows - 1) / rows, batch), 256, (size_t)rows * k * sizeof(float), stream>>>(x, order, out, n, k, rows, inverse);
   return cudaGetLastError();
 }
 

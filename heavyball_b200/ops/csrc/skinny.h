@@ -31,7 +31,7 @@ cudaError_t launch_triu_pack(const void* dense, void* line, int elem_bytes, int 
 cudaError_t launch_triu_unpack(const void* line, void* dense, int elem_bytes, int batch, int n, cudaStream_t stream);
 
 // out[b][i][j] = x[b][i][order[b][j]] or, `inverse`, out[b][i][order[b][j]] = x[b][i][j]; x, out: [batch, n, k] fp32, order: [batch, k]
-// permutations (entries outside [0, k) are skipped), k <= kMaxPermuted.
+// permutations (entries outside [0, k) read as zero, `inverse`: are dropped), k <= kMaxPermuted.
 constexpr int kMaxPermuted = 12288;
 cudaError_t launch_permute_columns(const float* x, const long long* order, float* out, int batch, int n, int k, int inverse, cudaStream_t stream);
 

@@ -267,12 +267,12 @@ def _cholesky_qr2(x: Tensor, shifted_rounds: int = 0):
     batch, (n, k) = x.shape[:-2], x.shape[-2:]
     a = x.reshape(-1, n, k)
     tiny = torch.finfo(a.dtype).tiny
-    a = a / a.norm(dim=-2, keepdim=True).clamp_(min=tiny)
     bad = torch.zeros(a.shape[0], dtype=torch.int32, device=a.device)
     rounds = shifted_rounds + 2
     info = torch.zeros_like(bad)  # failed leaves do not decide: what counts is the orthogonality reached at the end
     if _whole_blocks(a):
-        return _cholesky_qr2_blocks(a, bad, info, shifted_rounds).reshape(*batch, n, k), bad
+        return _cholesky_qr2_blocks(a.contiguous(), bad, info, shifted_rounds).reshape(*batch, n, k), bad
+    a = a / a.norm(dim=-2, keepdim=True).clamp_(min=tiny)
     for rnd in range(rounds):
         gram = _mm(a, a, True, False, pairs=False)
         if rnd < shifted_rounds:
@@ -305,14 +305,17 @@ def _whole_blocks(a: Tensor) -> bool:
 
 
 def _cholesky_qr2_blocks(a: Tensor, bad: Tensor, info: Tensor, shifted_rounds: int) -> Tensor:
-    """The rounds of :func:`_cholesky_qr2` with the same products in the same order (same bits) by ``ops.chol_qr_round``.  ``a`` is
-    overwritten."""
+    """The rounds of :func:`_cholesky_qr2` with the same products in the same order (same bits) by ``ops.chol_qr_round``."""
     from .. import ops
 
     n, k = a.shape[-2:]
-    a = a.contiguous()
+
+    def unit_columns(x):  # and the operand of the transpose
+        ops.launch_counter.count += 1
+        return ops.load().qr_unit_columns(x, x.norm(dim=-2, keepdim=True).clamp_(min=torch.finfo(x.dtype).tiny))
+
     gram = torch.empty(a.shape[0], k, k, device=a.device, dtype=a.dtype)
-    operand = ops.tf32_split(a, False, True)[1]
+    a, operand = unit_columns(a)
     for rnd in range(shifted_rounds + 2):
         ops.tf32_gemm(operand, operand, n, out=gram)
         shifted = rnd < shifted_rounds
@@ -320,8 +323,7 @@ def _cholesky_qr2_blocks(a: Tensor, bad: Tensor, info: Tensor, shifted_rounds: i
             gram.diagonal(dim1=-2, dim2=-1).add_(_CHOLQR_SHIFT * k)
         a, operand = ops.chol_qr_round(gram, a, info, want_trans=not shifted)
         if shifted:
-            a = a / a.norm(dim=-2, keepdim=True).clamp_(min=torch.finfo(a.dtype).tiny)
-            operand = ops.tf32_split(a, False, True)[1]
+            a, operand = unit_columns(a)
     ops.tf32_gemm(operand, operand, n, out=gram)
     ops.load().identity_defect(gram, _CHOLQR_ACCEPT, bad)
     return a
