@@ -384,3 +384,27 @@ def test_cycles_are_not_collected_while_a_graph_is_captured():
     assert gc.isenabled() and len(objects) == 2000
     fresh.replay()
     assert x.tolist() == [3.0] * 8
+
+
+@pytest.mark.parametrize("turn", [0.0, 1e-6, 0.03])
+def test_rotated_moments_are_as_close_to_64_bits_as_before(turn):
+    """A state moved from one basis to another, the bases equal up to rounding or a few percent apart: no further from 64 bits than the split-tf32
+    products, and within three products' bound of 2^-20 + (K / 16 + 4) 2^-23 = 5.2e-6 of |A| |B| each."""
+    from heavyball_b200.utils import soap
+
+    gen = torch.Generator("cuda").manual_seed(3)
+    draw = lambda *s: torch.randn(*s, device="cuda", dtype=torch.float64, generator=gen)  # noqa: E731
+    n, m = 512, 384
+    old = [torch.linalg.qr(draw(2, k, k)).Q for k in (n, m)]
+    new = [torch.linalg.qr(q + turn * draw(2, *q.shape[1:]) / q.shape[1] ** 0.5).Q for q in old]
+    new = [q * torch.sign(torch.einsum("bij,bij->bj", q, o)).unsqueeze(1) for q, o in zip(new, old)]
+    old, new = [q.float() for q in old], [q.float() for q in new]
+    state = torch.randn(2, n, m, device="cuda", generator=gen) * 10.0 ** -torch.randint(0, 4, (2, n, 1), device="cuda", generator=gen)
+    rots = [a.double().mT @ b.double() for a, b in zip(new, old)]
+    want = rots[0] @ state.double() @ rots[1].mT
+    got = state.clone()
+    soap._rotate_states(old, new, [got])
+    tf32 = [utils.core._mm(a, b, True, False, pairs=False) for a, b in zip(new, old)]
+    before = utils.core._mm(utils.core._mm(tf32[0], state, pairs=False), tf32[1], False, True, pairs=False)
+    error = lambda x: float((x.double() - want).norm() / want.norm())  # noqa: E731
+    assert error(got) <= error(before) and error(got) < 3 * 5.2e-6
