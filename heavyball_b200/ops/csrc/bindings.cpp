@@ -824,6 +824,39 @@ void sum_triu_diff_(const at::Tensor& a, const at::Tensor& b) {
   check(hb::launch_sum_triu_diff(a.data_ptr<float>(), b.data_ptr<float>(), (int)a.size(0), (int)a.size(1), at::cuda::getCurrentCUDAStream()), "sum_triu_diff launch");
 }
 
+// x[b] / by[b] (divide) or x[b] * by[b]; x: contiguous fp32, first dimension the batch; out: like x, may be x.
+void scale_matrices(const at::Tensor& x, const at::Tensor& by, bool divide, const at::Tensor& out) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() >= 1 && x.is_contiguous() && x.size(0) >= 1 && x.size(0) <= 65535 && out.device() == x.device() &&
+                  out.scalar_type() == at::kFloat && out.is_contiguous() && out.sizes() == x.sizes(), "scale_matrices: contiguous fp32 CUDA tensors of one shape");
+  const at::MemOverlapStatus overlap = at::get_overlap_status(x, out);
+  TORCH_CHECK(overlap != at::MemOverlapStatus::Partial, "scale_matrices: in place or elsewhere");
+  TORCH_CHECK(by.device() == x.device() && by.scalar_type() == at::kFloat && by.is_contiguous() && by.numel() == x.size(0), "scale_matrices: one fp32 value per matrix");
+  c10::cuda::CUDAGuard guard(x.device());
+  check(hb::launch_scale_matrices(x.data_ptr<float>(), by.data_ptr<float>(), out.data_ptr<float>(), (int)x.size(0), x.numel() / x.size(0), divide,
+                                  at::cuda::getCurrentCUDAStream()), "scale_matrices launch");
+}
+
+// X = B T^-1 for 128 columns: b, x: fp32 [batch, rows, 128] with unit inner stride and rows on 16-byte boundaries, rows a multiple of 64; inv:
+// [batch, blocks, 128, 128] contiguous, inverses of upper-triangular blocks, of which `block` is used.  x may not overlap b.
+void leaf_solve(const at::Tensor& b, const at::Tensor& inv, int64_t block, const at::Tensor& x) {
+  const int64_t batch = b.size(0), rows = b.dim() == 3 ? b.size(1) : 0;
+  for (const at::Tensor* t : {&b, &x})
+    TORCH_CHECK(t->is_cuda() && t->device() == b.device() && t->scalar_type() == at::kFloat && t->dim() == 3 && t->size(0) == batch && t->size(1) == rows &&
+                    t->size(2) == hb::kQrBlock && t->stride(2) == 1 && t->stride(1) % 4 == 0 && t->stride(0) % 4 == 0 && aligned16(t->data_ptr()),
+                "leaf_solve: fp32 [batch, rows, 128] CUDA tensors with rows on 16-byte boundaries");
+  TORCH_CHECK(rows >= 1 && rows % hb::kQrRows == 0 && batch <= 65535, "leaf_solve: a multiple of 64 rows");
+  TORCH_CHECK(inv.device() == b.device() && inv.scalar_type() == at::kFloat && inv.is_contiguous() && inv.dim() == 4 && inv.size(0) == batch && block >= 0 &&
+                  block < inv.size(1) && inv.size(2) == hb::kQrBlock && inv.size(3) == hb::kQrBlock, "leaf_solve: contiguous fp32 inverses [batch, blocks, 128, 128]");
+  const at::MemOverlapStatus overlap = at::get_overlap_status(b, x);
+  TORCH_CHECK(overlap != at::MemOverlapStatus::Full && overlap != at::MemOverlapStatus::Partial, "leaf_solve: not in place");
+  c10::cuda::CUDAGuard guard(b.device());
+  hb::QrLeafSolve S{};
+  S.src = b.data_ptr<float>(); S.ld = b.stride(1); S.stride = b.stride(0);
+  S.inv = inv.data_ptr<float>() + block * hb::kQrBlock * hb::kQrBlock; S.stride_inv = inv.stride(0);
+  S.out = x.data_ptr<float>(); S.ld_out = x.stride(1); S.stride_out = x.stride(0);
+  check(hb::launch_qr_leaf_solve(S, (int)rows, (int)batch, at::cuda::getCurrentCUDAStream()), "leaf_solve launch");
+}
+
 // g + (damp + eps |g|) v for contiguous fp32 tensors of one shape.
 at::Tensor dampen(const at::Tensor& g, const at::Tensor& v, double damp, double eps) {
   for (const at::Tensor* t : {&g, &v})
@@ -1029,6 +1062,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("transposed", &transposed);
   m.def("sum_triu_diff_", &sum_triu_diff_);
   m.def("dampen", &dampen);
+  m.def("scale_matrices", &scale_matrices);
+  m.def("leaf_solve", &leaf_solve);
   m.def("triu_step_", &triu_step_);
   m.def("triu_pack", &triu_pack);
   m.def("triu_unpack", &triu_unpack);

@@ -118,6 +118,21 @@ __global__ void __launch_bounds__(256) triu_step_kernel(const float* __restrict_
   for (int j = threadIdx.x; j < n - (int)i; j += blockDim.x) t[j] = sub(t[j], mul(div(s[j], by), lr));
 }
 
+template <typename V>
+__global__ void __launch_bounds__(256) scale_matrices_kernel(const V* x, const float* __restrict__ by, V* out, int64_t count, bool divide) {
+  constexpr int kWide = sizeof(V) / sizeof(float);
+  const int64_t base = blockIdx.y * count, step = (int64_t)gridDim.x * blockDim.x;
+  const float s = by[blockIdx.y];
+#pragma unroll 2
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += step) {
+    V v = x[base + i];
+    float* p = (float*)&v;
+#pragma unroll
+    for (int e = 0; e < kWide; ++e) p[e] = divide ? div(p[e], s) : mul(p[e], s);
+    out[base + i] = v;
+  }
+}
+
 unsigned blocks_for(int64_t items) {
   const int64_t blocks = (items + 511) / 512;  // two steps a thread until the device is full several times over
   return (unsigned)(blocks < 1 ? 1 : blocks > 4736 ? 4736 : blocks);
@@ -156,6 +171,16 @@ cudaError_t launch_triu_step(const float* step, const float* ell, float* line, i
   if (batch == 0 || n == 0) return cudaSuccess;
   if (batch > 65535) return cudaErrorInvalidValue;
   triu_step_kernel<<<dim3(n, batch), 256, 0, stream>>>(step, ell, line, n, lr);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_scale_matrices(const float* x, const float* by, float* out, int batch, int64_t count, bool divide, cudaStream_t stream) {
+  if (batch == 0 || count == 0) return cudaSuccess;
+  if (batch > 65535) return cudaErrorInvalidValue;
+  if ((count & 3) == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0)
+    scale_matrices_kernel<<<dim3(blocks_for(count / 4), batch), 256, 0, stream>>>((const float4*)x, by, (float4*)out, count / 4, divide);
+  else
+    scale_matrices_kernel<<<dim3(blocks_for(count), batch), 256, 0, stream>>>(x, by, out, count, divide);
   return cudaGetLastError();
 }
 

@@ -562,13 +562,42 @@ def _tc_sub_product(c: Tensor, a: Tensor, b: Tensor, b_transposed: bool = False,
     return True
 
 
+def _solve_leaf(b: Tensor, inv: Tensor, block: int, x: Tensor):
+    """``x <- b inv[:, block]`` for an upper-triangular inverse, sums over its rows in order in fp32: a kernel of its own for whole 128-wide leaves
+    (which leaves out the half that is zero), the library's product with the same bits otherwise."""
+    d, rows = b.shape[-1], b.shape[-2]
+    if d == _TRSM_LEAF and rows % 64 == 0 and 0 < b.shape[0] <= 65535 and all(
+        t.is_cuda and t.data_ptr() % 16 == 0 and t.stride(-1) == 1 and t.stride(-2) % 4 == 0 and t.stride(0) % 4 == 0 for t in (b, x)
+    ):
+        from .. import ops
+
+        if ops.available():
+            ops.launch_counter.count += 1
+            ops.load().leaf_solve(b, inv, block, x)
+            return
+    torch.bmm(b, inv[:, block, :d, :d], out=x)
+
+
+def _scaled_matrices(x: Tensor, by: Tensor, divide: bool = False, in_place: bool = False) -> Tensor:
+    """``x / by`` or ``x * by`` with one factor per leading index of ``x``."""
+    ext = _own_pass(x, by) if x.ndim >= 2 and by.numel() == x.shape[0] and 0 < x.shape[0] <= 65535 and x.numel() > 0 else None
+    if ext is not None:
+        out = x if in_place else torch.empty_like(x)
+        ext.scale_matrices(x, by, divide, out)
+        return out
+    wide = by.view(-1, *([1] * (x.ndim - 1)))
+    if in_place:
+        return x.div_(wide) if divide else x.mul_(wide)
+    return x / wide if divide else x * wide
+
+
 def _solve_right_upper_into(q: Tensor, b: Tensor, x: Tensor, inv: Tensor, first_block: int, pairs: bool):
     """``x <- b q^-1`` for upper-triangular ``q`` through the leaf inverses ``inv``; ``b`` is consumed (its columns to the
     right receive the updates in place).  All three are views with unit inner stride; nothing is allocated besides the
     split operands, nothing is concatenated."""
     d = q.shape[-1]
     if d <= _TRSM_LEAF:
-        torch.bmm(b, inv[:, first_block, :d, :d], out=x)
+        _solve_leaf(b, inv, first_block, x)
         return
     h = max(_TRSM_LEAF, (d // 2) // _TRSM_LEAF * _TRSM_LEAF)
     _solve_right_upper_into(q[..., :h, :h], b[..., :h], x[..., :h], inv, first_block, pairs)

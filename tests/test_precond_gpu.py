@@ -386,6 +386,34 @@ def test_cycles_are_not_collected_while_a_graph_is_captured():
     assert x.tolist() == [3.0] * 8
 
 
+@pytest.mark.parametrize("shape", [(1, 1), (3, 7), (2, 128, 128), (8, 1000, 33), (2, 524800)], ids=str)
+@pytest.mark.parametrize("divide", [False, True])
+def test_scaled_matrices_have_the_bits_of_the_broadcast(shape, divide):
+    from heavyball_b200.utils import core
+
+    gen = torch.Generator("cuda").manual_seed(len(shape))
+    x = torch.randn(*shape, device="cuda", generator=gen) * 10.0 ** torch.randint(-38, 3, shape, device="cuda", generator=gen)
+    by = torch.randn(shape[0], device="cuda", generator=gen)
+    wide = by.view(-1, *[1] * (len(shape) - 1))
+    want = x / wide if divide else x * wide
+    assert torch.equal(core._scaled_matrices(x, by, divide), want)
+    core._scaled_matrices(x, by, divide, in_place=True)
+    assert torch.equal(x, want)
+
+
+@pytest.mark.parametrize("batch,rows", [(1, 64), (8, 1024), (3, 4096), (2, 192)])
+def test_leaf_solve_has_the_bits_of_the_library_product(batch, rows):
+    """Sums over the 128 rows of the inverse in their order, each product fused into its sum, in either kernel."""
+    from heavyball_b200 import ops
+
+    gen = torch.Generator("cuda").manual_seed(rows)
+    wide = torch.randn(batch, rows, 384, device="cuda", generator=gen)
+    inv = torch.randn(batch, 3, 128, 128, device="cuda", generator=gen).triu()
+    x = torch.full((batch, rows, 256), 7.0, device="cuda")
+    ops.load().leaf_solve(wide[..., 128:256], inv, 1, x[..., 128:])
+    assert torch.equal(x[..., 128:], torch.bmm(wide[..., 128:256], inv[:, 1])) and bool((x[..., :128] == 7).all())
+
+
 @pytest.mark.parametrize("turn", [0.0, 1e-6, 0.03])
 def test_rotated_moments_are_as_close_to_64_bits_as_before(turn):
     """A state moved from one basis to another, the bases equal up to rounding or a few percent apart: no further from 64 bits than the split-tf32
