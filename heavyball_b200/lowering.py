@@ -30,6 +30,7 @@ and writes the same state keys, so checkpoints do not depend on which path ran.
 from __future__ import annotations
 
 import functools
+import math
 import os
 from typing import List, Optional
 
@@ -263,12 +264,14 @@ def _mark_all(prog, states: List[dict]):
 def _state_ready(tr: C.FunctionTransform, states: List[dict], ecc: bool) -> bool:
     keys = [k for layer in tr.layers if not isinstance(layer, C.AccumSlots) for k in layer.keys.values()]
     warm = [(layer.counter, len(layer.warmup_fns)) for layer in tr.layers if isinstance(layer, C.Warmup)]
+    if ecc:
+        keys += [k + "::ecc" for k in keys]
+    need = frozenset(keys)
     for st in states:
-        for k in keys:
-            if k not in st or (ecc and k + "::ecc" not in st):
-                return False
-        for counter, need in warm:
-            if st.get(counter, 0) < need:
+        if not need <= st.keys():
+            return False
+        for counter, count in warm:
+            if st.get(counter, 0) < count:
                 return False
     return True
 
@@ -644,17 +647,15 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
     # iteration writes its result over its own input: no second buffer of the group's size
     layout, scratch, _ = _bucket_layout(prog, params_v)
     dev = params[0].device
-    sq = torch.zeros(len(scratch), dtype=torch.float32, device=dev)  # squared norms, accumulated by the momentum kernel
+    sq = _norms(prog, len(scratch), dev)  # squared norms, accumulated by the momentum kernel
     with _stage("momentum"):
         launch(g=grads_v, u=scratch, s0=s0, s0e=s0e, s1=s1, s1e=s1e, s2=s2, s2e=s2e, out_mode=ops.OUT_UPDATE, dt_u=ops.F32,
                scale=sq, accum_sumsq=1, seed=_seed(opt, group, 0), **base, **mars_kw, **peer_in)  # fmt: skip
     scale_mode = "scale"
     final = list(scratch)
-    buckets = [(shape, idx, U) for shape, idx, U, _ in layout if len(shape) >= 2]
     pending = []  # (bytes of work copies, group); groups go through the iteration together, as many as the workspace holds
-    for shape, idx, U in buckets:
-        R, Cc = shape[0], U[0].numel() // shape[0]
-        U3 = U.view(len(idx), R, Cc)
+    for idx, U3, single in _bucket_matrices(prog, layout):
+        R, Cc = U3.shape[1:]
         if not ops.ns_supported(R, Cc):
             for b in range(len(idx)):
                 utils.inplace_orthogonal_(U3[b], out=U3[b], scale_mode=scale_mode)
@@ -663,8 +664,9 @@ def _run(opt, prog, states, group, grads, params, on_gpu, check_only) -> bool:
         chunk = max(1, _NS_WORKSPACE_BYTES // per_matrix)
         for c0 in range(0, len(idx), chunk):
             part = idx[c0 : c0 + chunk]
-            pending.append((per_matrix * len(part), (U3[c0 : c0 + len(part)].unbind(0), part, U3[c0 : c0 + len(part)],
-                                                     max(1, R / Cc) ** 0.5, _seed(opt, group, 2 + len(final) + R + c0))))  # fmt: skip
+            mats = U3 if len(part) == len(idx) else U3[c0 : c0 + len(part)]
+            pending.append((per_matrix * len(part), (single[c0 : c0 + len(part)], part, mats, max(1, R / Cc) ** 0.5,
+                                                     _seed(opt, group, 2 + len(final) + R + c0))))  # fmt: skip
     with _stage("newton_schulz"):
         while pending:
             room, wave = _NS_WORKSPACE_BYTES, []
@@ -691,6 +693,15 @@ def _orthogonal_update(opt, group, caution, params_v, grads_v, final, pe, base, 
         ops.fused_chain(p=params_v, pe=pe, u=final, algo=ops.IDENTITY, u_is_input=1, out_mode=ops.OUT_PARAM, dt_u=ops.F32,
                         dt_p=base["dt_p"], dt_g=ops.NONE, dt_s=ops.NONE, seed=_seed(opt, group, 3), **epilogue,
                         **peer_out)  # fmt: skip
+
+
+def _norms(prog: _Program, n: int, device) -> torch.Tensor:
+    """Zeroed fp32 sums, one per parameter, in a buffer kept on the program (like its updates)."""
+    key = ("norms", n, device)
+    hit = prog.workspace.get(key)
+    if hit is None:
+        hit = prog.workspace[key] = torch.empty(n, dtype=torch.float32, device=device)
+    return hit.zero_()
 
 
 def _scratch(prog: _Program, params) -> List[torch.Tensor]:
@@ -733,6 +744,20 @@ def _bucket_layout(prog: _Program, params):
     prog.workspace = {k: v for k, v in prog.workspace.items() if k[0] != "layout"}
     hit = prog.workspace[key] = (buckets, u_views, out_views)
     return hit
+
+
+def _bucket_matrices(prog: _Program, layout):
+    """Per bucket of a :func:`_bucket_layout` whose members are matrices (higher orders flattened): ``(positions, U as (B, R, C), its
+    matrices)``, views of the layout's buffers that are made once and kept with them."""
+    held = prog.workspace.get(("layout matrices",))
+    if held is None or held[0] is not layout:
+        views = []
+        for shape, idx, U, _ in layout:
+            if len(shape) >= 2:
+                U3 = U.view(len(idx), shape[0], math.prod(shape[1:]))
+                views.append((idx, U3, U3.unbind(0)))
+        held = prog.workspace[("layout matrices",)] = (layout, views)
+    return held[1]
 
 
 def _stage_bucket(prog: _Program, group, shape, n: int, make):

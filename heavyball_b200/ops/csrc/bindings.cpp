@@ -357,41 +357,48 @@ int64_t ns_orthogonalize(const std::vector<std::vector<at::Tensor>>& mats, int s
                               (int)src.size(), first.back(), src_dt, (float)eps, stream), "ns_prepare launch");
   int launches = 1;
   std::vector<hb::NsProduct> stage(n);
+  // the products of one kind for every bucket, reading iterate `cur`; the last apply writes the results
+  const auto plan = [&](int mode, int cur, bool last) {
+    for (size_t g = 0; g < n; ++g) {
+      const Bucket& b = buckets[g];
+      hb::NsProduct& X = stage[g];
+      hb::GemmParams P{};
+      P.mode = mode; P.batch = (int)b.batch; P.status = status.data_ptr<int>(); P.M = (int)b.m; P.f_scale = 1.f;
+      if (mode == hb::kModeApply) {  // X' = Y X
+        X = {b.y, b.lds, b.m * b.lds, b.x[cur], b.ldx, b.m * b.ldx, {}};
+        P.N = (int)b.n; P.K = (int)b.m; P.b_mn = 1;
+        if (!last) {
+          P.C = b.x[1 - cur]; P.ldc = b.ldx; P.strideC = b.m * b.ldx;
+        } else {
+          P.F = outs[g].data_ptr<float>(); P.ldf = b.C; P.strideF = b.R * b.C; P.f_transposed = b.R > b.C ? 1 : 0;
+          P.f_scale = (float)out_scales[g];
+        }
+      } else {  // S = X X^T,  Y = c S S + b S + a I
+        const bool poly = mode == hb::kModePoly;
+        if (poly)
+          X = {b.s, b.lds, b.m * b.lds, b.s, b.lds, b.m * b.lds, {}};
+        else
+          X = {b.x[cur], b.ldx, b.m * b.ldx, b.x[cur], b.ldx, b.m * b.ldx, {}};
+        P.N = (int)b.m; P.K = (int)(poly ? b.m : b.n); P.symmetric = 1;
+        P.C = P.CT = poly ? b.y : b.s; P.ldc = P.ldct = b.lds; P.strideC = P.strideCT = b.m * b.lds;
+        if (poly) { P.S = b.s; P.lds = b.lds; P.strideS = b.m * b.lds; }
+      }
+      X.P = P;
+    }
+    hb::NsPlan made;
+    check(hb::prepare_ns_products(stage.data(), (int)n, &made), "ns_orthogonalize products");
+    return made;
+  };
+  hb::NsPlan gram[2], poly, apply[2];
   int cur = 0;
   for (size_t step = 0; step < coeffs.size(); ++step, cur = 1 - cur) {
     TORCH_CHECK(coeffs[step].size() == 3, "ns_orthogonalize: (a, b, c) per step");
-    for (int mode : {(int)hb::kModeGram, (int)hb::kModePoly, (int)hb::kModeApply}) {
-      for (size_t g = 0; g < n; ++g) {
-        const Bucket& b = buckets[g];
-        hb::NsProduct& X = stage[g];
-        hb::GemmParams P{};
-        P.mode = mode; P.batch = (int)b.batch; P.status = status.data_ptr<int>(); P.M = (int)b.m; P.f_scale = 1.f;
-        if (mode == hb::kModeApply) {  // X' = Y X
-          X = {b.y, b.lds, b.m * b.lds, b.x[cur], b.ldx, b.m * b.ldx, {}};
-          P.N = (int)b.n; P.K = (int)b.m; P.b_mn = 1;
-          if (step + 1 < coeffs.size()) {
-            P.C = b.x[1 - cur]; P.ldc = b.ldx; P.strideC = b.m * b.ldx;
-          } else {
-            P.F = outs[g].data_ptr<float>(); P.ldf = b.C; P.strideF = b.R * b.C; P.f_transposed = b.R > b.C ? 1 : 0;
-            P.f_scale = (float)out_scales[g];
-          }
-        } else {  // S = X X^T,  Y = c S S + b S + a I
-          const bool poly = mode == hb::kModePoly;
-          if (poly)
-            X = {b.s, b.lds, b.m * b.lds, b.s, b.lds, b.m * b.lds, {}};
-          else
-            X = {b.x[cur], b.ldx, b.m * b.ldx, b.x[cur], b.ldx, b.m * b.ldx, {}};
-          P.N = (int)b.m; P.K = (int)(poly ? b.m : b.n); P.symmetric = 1;
-          P.C = P.CT = poly ? b.y : b.s; P.ldc = P.ldct = b.lds; P.strideC = P.strideCT = b.m * b.lds;
-          if (poly) {
-            P.S = b.s; P.lds = b.lds; P.strideS = b.m * b.lds;
-            P.ca = (float)coeffs[step][0]; P.cb = (float)coeffs[step][1]; P.cc = (float)coeffs[step][2];
-          }
-        }
-        X.P = P;
-      }
-      check(hb::launch_ns_products(stage.data(), (int)n, &launches, stream), "ns_orthogonalize launch");
-    }
+    const bool last = step + 1 == coeffs.size();
+    if (!gram[cur].launches) gram[cur] = plan(hb::kModeGram, cur, false);
+    if (!poly.launches) poly = plan(hb::kModePoly, cur, false);
+    if (last || !apply[cur].launches) apply[cur] = plan(hb::kModeApply, cur, last);
+    hb::set_ns_coefficients(poly, (float)coeffs[step][0], (float)coeffs[step][1], (float)coeffs[step][2]);
+    for (const hb::NsPlan* p : {&gram[cur], &poly, &apply[cur]}) check(hb::launch_ns_plan(*p, &launches, stream), "ns_orthogonalize launch");
   }
   return launches;
 }

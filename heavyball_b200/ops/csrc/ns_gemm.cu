@@ -69,21 +69,26 @@ struct GemmGroup {
   int tiles_m, tiles_n, per_batch;
   int f_bulk;                  // F leaves through bulk stores, described by `c` (pair kernel)
 };
+// kRoom groups at most.  A launch's arguments are copied by the host, and 7 KB take longer than 3.5: up to kFewGroups groups go in a
+// smaller struct (five small odd matrices in four shapes, a step's 15 launches: 80 -> 65 us of host time).
+constexpr int kFewGroups = 4;
+template <int kRoom>
 struct GemmGroups {
   int n, total;
-  int first[kMaxGroups];       // index of each group's first tile within the launch
+  int first[kRoom];            // index of each group's first tile within the launch
   int* status;
-  GemmGroup g[kMaxGroups];
+  GemmGroup g[kRoom];
 };
 
 struct TileAt : PairTile {
   int group;
 };
-__device__ __forceinline__ TileAt tile_at(const GemmGroups& L, int idx) {
+template <int kRoom>
+__device__ __forceinline__ TileAt tile_at(const GemmGroups<kRoom>& L, int idx) {
   TileAt t;
   t.group = 0;
 #pragma unroll
-  for (int i = 1; i < kMaxGroups; ++i)
+  for (int i = 1; i < kRoom; ++i)
     if (i < L.n && idx >= L.first[i]) t.group = i;
   const GemmGroup& G = L.g[t.group];
   static_cast<PairTile&>(t) = pair_tile(idx - L.first[t.group], G.tiles_m, G.tiles_n, G.per_batch, G.P.symmetric);
@@ -91,7 +96,8 @@ __device__ __forceinline__ TileAt tile_at(const GemmGroups& L, int idx) {
 }
 
 // ------------------------------------------------------------------------------------------ kernel
-__global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_constant__ GemmGroups L) {
+template <int kRoom>
+__global__ void __launch_bounds__(kGemmThreads, 2) ns_gemm_kernel(const __grid_constant__ GemmGroups<kRoom> L) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kStages];
   __shared__ __align__(8) uint64_t empty_bar[kStages];
@@ -315,7 +321,8 @@ constexpr int kPairEpiWarps = 8;
 constexpr int kPairThreads = 64 + 32 * kPairEpiWarps;
 constexpr int kPairSmemBytes = kPairStages * kPairStageBytes + kPairEpiWarps * 2 * kWarpStage + 1024;  // C and C^T of a warp
 constexpr uint32_t kInstrDescPair = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPairTile >> 3) << 17) | ((uint32_t)(kPairTile >> 4) << 24);
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_gemm_pair_kernel(const __grid_constant__ GemmGroups L) {
+template <int kRoom>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1) ns_gemm_pair_kernel(const __grid_constant__ GemmGroups<kRoom> L) {
   extern __shared__ uint8_t smem_raw[];
   __shared__ __align__(8) uint64_t full_bar[kPairStages];   // used in the even CTA: both CTAs' loads of a stage have landed
   __shared__ __align__(8) uint64_t empty_bar[kPairStages];  // in each CTA: the products that read the stage have finished
@@ -729,15 +736,28 @@ static cudaError_t resident_pairs(int* out) {
   const cudaError_t e = cudaGetDevice(&device);
   if (e != cudaSuccess) return e;
   return pairs.get(device, cudaSuccess, out, [](int& found) {
-    cudaError_t s = cudaFuncSetAttribute(ns_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
-    if (s == cudaSuccess) s = cudaFuncSetAttribute(ns_gemm_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
-    return s != cudaSuccess ? s : max_resident_pairs(ns_gemm_pair_kernel, kPairThreads, kPairSmemBytes, &found);
+    cudaError_t s = cudaSuccess;
+    for (const void* kernel : {(const void*)ns_gemm_kernel<kFewGroups>, (const void*)ns_gemm_kernel<kMaxGroups>})
+      if (s == cudaSuccess) s = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+    for (const void* kernel : {(const void*)ns_gemm_pair_kernel<kFewGroups>, (const void*)ns_gemm_pair_kernel<kMaxGroups>})
+      if (s == cudaSuccess) s = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes);
+    return s != cudaSuccess ? s : max_resident_pairs(ns_gemm_pair_kernel<kMaxGroups>, kPairThreads, kPairSmemBytes, &found);
   });
 }
 
 // One launch of the pair kernel (`pair`) or of the 128 x 128 kernel over up to kMaxGroups products.
-static cudaError_t launch_group(const NsProduct* const* products, int n, bool pair, int max_pairs, cudaStream_t stream) {
-  GemmGroups L;
+struct NsLaunch {
+  GemmGroups<kMaxGroups> L;
+  bool pair;
+  int blocks;
+};
+struct NsLaunches {
+  std::vector<NsLaunch> all;
+};
+
+static cudaError_t prepare_group(const NsProduct* const* products, int n, bool pair, int max_pairs, NsLaunch& out) {
+  GemmGroups<kMaxGroups>& L = out.L;
+  out.pair = pair;
   L.n = n;
   L.total = 0;
   L.status = products[0]->P.status;
@@ -766,15 +786,11 @@ static cudaError_t launch_group(const NsProduct* const* products, int n, bool pa
     if (pair && P.mode == kModePoly) ok = ok && make_map(&G.s, P.S, P.M, P.N, P.lds, P.strideS, P.batch, 64, 32);
     if (!ok) return cudaErrorInvalidValue;
   }
-  if (L.total == 0) return cudaSuccess;
-  if (pair) {
-    const int pairs = L.total < max_pairs ? L.total : max_pairs;
-    return launch_chained(ns_gemm_pair_kernel, dim3(2 * pairs), kPairThreads, kPairSmemBytes, stream, L);
-  }
-  return launch_chained(ns_gemm_kernel, dim3(L.total), kGemmThreads, kSmemBytes, stream, L);
+  out.blocks = pair ? 2 * std::min(L.total, max_pairs) : L.total;
+  return cudaSuccess;
 }
 
-cudaError_t launch_ns_products(const NsProduct* products, int n, int* launches, cudaStream_t stream) {
+cudaError_t prepare_ns_products(const NsProduct* products, int n, NsPlan* plan) {
   int max_pairs = 0;
   const cudaError_t found = resident_pairs(&max_pairs);
   if (found != cudaSuccess) return found;
@@ -786,17 +802,64 @@ cudaError_t launch_ns_products(const NsProduct* products, int n, int* launches, 
   const bool pairs = force == 0 && ns_take_pairs(extents.data(), n, max_pairs);
   std::vector<const NsProduct*> side[2];
   for (int i = 0; i < n; ++i) side[force == 256 || (pairs && ns_pair_sized(extents[i])) ? 1 : 0].push_back(&products[i]);
+  plan->launches = std::make_shared<NsLaunches>();
+  plan->launches->all.reserve(side[0].size() / kMaxGroups + side[1].size() / kMaxGroups + 2);
   for (int pair = 1; pair >= 0; --pair) {
     auto& list = side[pair];
     // tiles are dealt out in order: the ones with the longest main loop first
     std::stable_sort(list.begin(), list.end(), [](const NsProduct* a, const NsProduct* b) { return a->P.K > b->P.K; });
     for (size_t i = 0; i < list.size(); i += kMaxGroups) {
-      const cudaError_t e = launch_group(list.data() + i, (int)std::min<size_t>(kMaxGroups, list.size() - i), pair != 0, max_pairs, stream);
+      plan->launches->all.emplace_back();
+      const cudaError_t e =
+          prepare_group(list.data() + i, (int)std::min<size_t>(kMaxGroups, list.size() - i), pair != 0, max_pairs, plan->launches->all.back());
       if (e != cudaSuccess) return e;
-      if (launches != nullptr) ++*launches;
     }
   }
   return cudaSuccess;
+}
+
+void set_ns_coefficients(const NsPlan& plan, float ca, float cb, float cc) {
+  for (NsLaunch& launch : plan.launches->all)
+    for (int i = 0; i < launch.L.n; ++i) {
+      launch.L.g[i].P.ca = ca;
+      launch.L.g[i].P.cb = cb;
+      launch.L.g[i].P.cc = cc;
+    }
+}
+
+template <int kRoom>
+static cudaError_t launch_groups(const NsLaunch& launch, const GemmGroups<kRoom>& L, cudaStream_t stream) {
+  void* args[] = {const_cast<GemmGroups<kRoom>*>(&L)};
+  return launch.pair ? launch_chained_with((const void*)ns_gemm_pair_kernel<kRoom>, dim3(launch.blocks), kPairThreads, kPairSmemBytes, stream, args)
+                     : launch_chained_with((const void*)ns_gemm_kernel<kRoom>, dim3(launch.blocks), kGemmThreads, kSmemBytes, stream, args);
+}
+
+cudaError_t launch_ns_plan(const NsPlan& plan, int* launches, cudaStream_t stream) {
+  for (const NsLaunch& launch : plan.launches->all) {
+    if (launch.L.total > 0) {
+      cudaError_t e;
+      if (launch.L.n <= kFewGroups) {
+        GemmGroups<kFewGroups> few;
+        few.n = launch.L.n;
+        few.total = launch.L.total;
+        few.status = launch.L.status;
+        std::copy_n(launch.L.first, launch.L.n, few.first);
+        std::copy_n(launch.L.g, launch.L.n, few.g);
+        e = launch_groups(launch, few, stream);
+      } else {
+        e = launch_groups(launch, launch.L, stream);
+      }
+      if (e != cudaSuccess) return e;
+    }
+    if (launches != nullptr) ++*launches;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t launch_ns_products(const NsProduct* products, int n, int* launches, cudaStream_t stream) {
+  NsPlan plan;
+  const cudaError_t e = prepare_ns_products(products, n, &plan);
+  return e != cudaSuccess ? e : launch_ns_plan(plan, launches, stream);
 }
 
 cudaError_t launch_ns_prepare(const NsSource* mats, const int* first, int n_mats, int total_tiles, int src_dt, float eps,

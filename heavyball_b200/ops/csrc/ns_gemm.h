@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <memory>
+
 namespace hb {
 
 enum GemmMode : int { kModeGram = 0, kModePoly = 1, kModeApply = 2 };
@@ -41,7 +43,17 @@ struct NsProduct {
   int64_t ldb, strideB;
   GemmParams P;
 };
-// Independent products, in as few launches as their tile sizes allow; `launches` (may be null) is advanced by their number.
+// Independent products, in as few launches as their tile sizes allow, ready to be issued any number of times while their buffers live on the
+// current device: an iteration alternates between two buffers, so its five steps are made of as many different launches as two.
+struct NsLaunches;
+struct NsPlan {
+  std::shared_ptr<NsLaunches> launches;
+};
+cudaError_t prepare_ns_products(const NsProduct* products, int n, NsPlan* plan);
+void set_ns_coefficients(const NsPlan& plan, float ca, float cb, float cc);
+// `launches` (may be null) is advanced by their number.
+cudaError_t launch_ns_plan(const NsPlan& plan, int* launches, cudaStream_t stream);
+// Both at once.
 cudaError_t launch_ns_products(const NsProduct* products, int n, int* launches, cudaStream_t stream);
 
 // One matrix to be normalised and rounded into the bf16 iterate (as it is, or transposed).

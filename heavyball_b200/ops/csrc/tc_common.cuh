@@ -291,6 +291,21 @@ __device__ __forceinline__ PairTile pair_tile(int idx, int tiles_m, int tiles_n,
 __device__ inline void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ inline void griddep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The same for kernels whose argument is a large struct: `args` points at each argument, nothing is copied on the way.
+inline cudaError_t launch_chained_with(const void* kernel, dim3 grid, int threads, int smem_bytes, cudaStream_t stream, void** args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem_bytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelExC(&cfg, kernel, args);
+}
+
 template <class... KArgs, class... Args>
 inline cudaError_t launch_chained(void (*kernel)(KArgs...), dim3 grid, int threads, int smem_bytes, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg{};
