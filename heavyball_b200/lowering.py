@@ -264,14 +264,12 @@ def _mark_all(prog, states: List[dict]):
 def _state_ready(tr: C.FunctionTransform, states: List[dict], ecc: bool) -> bool:
     keys = [k for layer in tr.layers if not isinstance(layer, C.AccumSlots) for k in layer.keys.values()]
     warm = [(layer.counter, len(layer.warmup_fns)) for layer in tr.layers if isinstance(layer, C.Warmup)]
-    if ecc:
-        keys += [k + "::ecc" for k in keys]
-    need = frozenset(keys)
     for st in states:
-        if not need <= st.keys():
-            return False
-        for counter, count in warm:
-            if st.get(counter, 0) < count:
+        for k in keys:
+            if k not in st or (ecc and k + "::ecc" not in st):
+                return False
+        for counter, need in warm:
+            if st.get(counter, 0) < need:
                 return False
     return True
 

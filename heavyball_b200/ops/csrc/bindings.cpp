@@ -22,6 +22,7 @@
 #include "matrix_passes.h"
 #include "ns_gemm.h"
 #include "peer_sync.h"
+#include "power_iteration.h"
 #include "skinny.h"
 #include "split16_gemm.h"
 #include "tf32_gemm.h"
@@ -831,6 +832,18 @@ void sum_triu_diff_(const at::Tensor& a, const at::Tensor& b) {
   check(hb::launch_sum_triu_diff(a.data_ptr<float>(), b.data_ptr<float>(), (int)a.size(0), (int)a.size(1), at::cuda::getCurrentCUDAStream()), "sum_triu_diff launch");
 }
 
+// Estimates of the largest eigenvalues of contiguous fp32 symmetric positive semi-definite matrices [batch, n, n] (power_iteration.h).
+at::Tensor power_iteration(const at::Tensor& a, int64_t iterations) {
+  check_matrices(a, "power_iteration");
+  TORCH_CHECK(a.size(1) == a.size(2) && a.size(1) >= 1 && a.size(1) <= hb::kMaxPowerSize && iterations >= 0 && iterations < (1 << 20),
+              "power_iteration: square matrices of at most 2048 rows");
+  c10::cuda::CUDAGuard guard(a.device());
+  at::Tensor out = at::empty({a.size(0)}, a.options().memory_format(at::MemoryFormat::Contiguous));
+  check(hb::launch_power_iteration(a.data_ptr<float>(), (int)a.size(0), (int)a.size(1), (int)iterations, out.data_ptr<float>(),
+                                   at::cuda::getCurrentCUDAStream()), "power_iteration launch");
+  return out;
+}
+
 // x[b] / by[b] (divide) or x[b] * by[b]; x: contiguous fp32, first dimension the batch; out: like x, may be x.
 void scale_matrices(const at::Tensor& x, const at::Tensor& by, bool divide, const at::Tensor& out) {
   TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() >= 1 && x.is_contiguous() && x.size(0) >= 1 && x.size(0) <= 65535 && out.device() == x.device() &&
@@ -1069,6 +1082,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("transposed", &transposed);
   m.def("sum_triu_diff_", &sum_triu_diff_);
   m.def("dampen", &dampen);
+  m.def("power_iteration", &power_iteration);
   m.def("scale_matrices", &scale_matrices);
   m.def("leaf_solve", &leaf_solve);
   m.def("triu_step_", &triu_step_);

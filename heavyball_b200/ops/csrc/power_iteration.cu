@@ -1,0 +1,217 @@
+// Power iteration on A^2 for the step length of a PSGD fit: heavyball/utils.py's estimate of the largest eigenvalue, started from A's largest row.
+//
+// As single operations that is thirty dependent launches per factor: row norms, their maximum, a gather, A over the largest norm, and for every
+// product a matrix-vector kernel, a norm, a clamp and a division.  Here a cluster of CTAs takes a matrix from beginning to end.  A CTA owns a
+// share of the rows, which it reads once for the norms and twice a step (from the L2: 4 MB at 1024), a warp four rows at a time; every CTA keeps
+// the whole vectors in shared memory, and each product's entries are stored into all of them.  What is left of each step is the reading and one
+// cluster barrier per product.  A is divided by its largest row norm on the way, entry by entry, so that no scale of A over- or underflows.
+// Two factors of 8 of 1024^2, two iterations each, in the graph of a fit: 245 us of the library's kernels, 2 x 54 here.
+#include "power_iteration.h"
+
+#include "per_device.h"
+#include "tc_common.cuh"
+
+namespace hb {
+namespace {
+
+constexpr int kPowerThreads = 512, kPowerWarps = kPowerThreads / 32;
+constexpr int kPowerRows = 4;  // of a warp at a time
+
+// Subnormal values are kept (squares of a small A's entries), against the flags of this library.
+__device__ __forceinline__ float fma_full(float a, float b, float c) {
+  float r;
+  asm("fma.rn.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float mul_full(float a, float b) {
+  float r;
+  asm("mul.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float add_full(float a, float b) {
+  float r;
+  asm("add.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float sqrt_full(float a) {
+  float r;
+  asm("sqrt.rn.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float inverse_full(float a) {
+  float r;
+  asm("rcp.rn.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = add_full(v, __shfl_xor_sync(0xFFFFFFFFu, v, o));
+  return v;
+}
+__device__ __forceinline__ float block_sum(float v, float* scratch) {
+  v = warp_sum(v);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  return warp_sum((threadIdx.x & 31) < kPowerWarps ? scratch[threadIdx.x & 31] : 0.0f);
+}
+// One value per row, from the lanes that hold it to the same place of every CTA.
+__device__ __forceinline__ void store_everywhere(float* to, float v, int lane, int ctas) {
+  if (lane < ctas) cluster_store(cluster_addr(to, (uint32_t)lane), __float_as_int(v));
+}
+
+// For each row r of [first, last): done(r, s, lane) with s from zero through s <- term(s, a_rk, k).
+template <bool kWide, class Term, class Done>
+__device__ __forceinline__ void over_rows(const float* __restrict__ A, int n, int first, int last, const Term& term, const Done& done) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r0 = first + warp * kPowerRows; r0 < last; r0 += kPowerWarps * kPowerRows) {
+    float s[kPowerRows] = {};
+    const float* row[kPowerRows];
+#pragma unroll
+    for (int i = 0; i < kPowerRows; ++i) row[i] = A + (int64_t)min(r0 + i, last - 1) * n;
+    if (kWide) {
+#pragma unroll 2
+      for (int k = lane * 4; k < n; k += 128) {
+        float4 a[kPowerRows];
+#pragma unroll
+        for (int i = 0; i < kPowerRows; ++i) a[i] = *(const float4*)(row[i] + k);
+#pragma unroll
+        for (int i = 0; i < kPowerRows; ++i) {
+          s[i] = term(s[i], a[i].x, k);
+          s[i] = term(s[i], a[i].y, k + 1);
+          s[i] = term(s[i], a[i].z, k + 2);
+          s[i] = term(s[i], a[i].w, k + 3);
+        }
+      }
+    } else {
+      for (int k = lane; k < n; k += 32) {
+#pragma unroll
+        for (int i = 0; i < kPowerRows; ++i) s[i] = term(s[i], row[i][k], k);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < kPowerRows; ++i) {
+      const float total = warp_sum(s[i]);
+      if (r0 + i < last) done(r0 + i, total, lane);
+    }
+  }
+}
+
+template <bool kWide>
+__global__ void __launch_bounds__(kPowerThreads) power_iteration_kernel(const float* __restrict__ matrices, int n, int iterations, int ctas,
+                                                                       float* __restrict__ out) {
+  extern __shared__ __align__(16) float vectors[];  // three of n, padded to 16 bytes
+  __shared__ float scratch[kPowerWarps], best_norm[kPowerWarps];
+  __shared__ int best_row[kPowerWarps];
+  const int pad = (n + 3) & ~3;
+  float *const x = vectors, *const ax = vectors + pad, *const aax = vectors + 2 * pad;
+  const int rank = (int)cluster_rank(), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const float* A = matrices + (int64_t)(blockIdx.x / ctas) * n * n;
+  const int per = (n + ctas - 1) / ctas, first = min(n, rank * per), last = min(n, first + per);
+  cluster_sync();  // every CTA's shared memory is there to be written
+
+  over_rows<kWide>(A, n, first, last, [](float s, float a, int) { return fma_full(a, a, s); },
+                   [&](int r, float s, int l) { store_everywhere(aax + r, sqrt_full(s), l, ctas); });
+  cluster_sync();
+  float norm = -1.0f;
+  int at = 0;
+  for (int i = threadIdx.x; i < n; i += kPowerThreads)
+    if (!(aax[i] <= norm)) {  // (a row with a NaN is the largest)
+      norm = aax[i];
+      at = i;
+    }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const float other = __shfl_xor_sync(0xFFFFFFFFu, norm, o);
+    const int other_at = __shfl_xor_sync(0xFFFFFFFFu, at, o);
+    if (!(other <= norm) && (other != norm || other_at < at)) {
+      norm = other;
+      at = other_at;
+    }
+  }
+  if (lane == 0) {
+    best_norm[warp] = norm;
+    best_row[warp] = at;
+  }
+  __syncthreads();
+  norm = best_norm[0];
+  at = best_row[0];
+  for (int w = 1; w < kPowerWarps; ++w)
+    if (!(best_norm[w] <= norm)) {
+      norm = best_norm[w];
+      at = best_row[w];
+    }
+  const float top = norm < 1.17549435e-38f ? 1.17549435e-38f : norm, by = inverse_full(top);
+  for (int k = threadIdx.x; k < n; k += kPowerThreads) x[k] = mul_full(A[(int64_t)at * n + k], by);
+  cluster_sync();  // x is complete, and nobody reads the norms any more
+
+  const auto times = [&](const float* v, float* to) {
+    over_rows<kWide>(A, n, first, last, [&](float s, float a, int k) { return fma_full(mul_full(a, by), v[k], s); }, [&](int r, float s, int l) { store_everywhere(to + r, s, l, ctas); });
+    cluster_sync();
+  };
+  for (int it = 0; it < iterations; ++it) {
+    times(x, ax);
+    times(ax, aax);
+    float s = 0.0f;
+    for (int k = threadIdx.x; k < n; k += kPowerThreads) s = fma_full(aax[k], aax[k], s);
+    const float length = sqrt_full(block_sum(s, scratch)), inv = inverse_full(length < 1e-12f ? 1e-12f : length);
+    for (int k = threadIdx.x; k < n; k += kPowerThreads) x[k] = mul_full(aax[k], inv);
+    __syncthreads();
+  }
+  times(x, ax);
+  times(ax, aax);
+  float s = 0.0f;
+  for (int k = threadIdx.x; k < n; k += kPowerThreads) s = fma_full(x[k], aax[k], s);
+  s = block_sum(s, scratch);
+  if (rank == 0 && threadIdx.x == 0) out[blockIdx.x / ctas] = mul_full(sqrt_full(s), top);
+}
+
+}  // namespace
+
+cudaError_t launch_power_iteration(const float* A, int batch, int n, int iterations, float* out, cudaStream_t stream) {
+  const bool wide = (n & 3) == 0 && ((uintptr_t)A & 15) == 0;
+  const auto kernel = wide ? power_iteration_kernel<true> : power_iteration_kernel<false>;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.blockDim = dim3(kPowerThreads);
+  cfg.dynamicSmemBytes = 3 * ((n + 3) & ~3) * sizeof(float);
+  cfg.stream = stream;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  const auto shape = [&](int ctas) {
+    attr[0].val.clusterDim.x = ctas;
+    cfg.gridDim = dim3(batch * ctas);
+  };
+  static PerDevice<int> wide_clusters;  // clusters of sixteen that the device holds at once
+  int device = 0, held = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e == cudaSuccess)
+    e = wide_clusters.get(device, cudaSuccess, &held, [](int& found) {
+      for (const auto k : {power_iteration_kernel<true>, power_iteration_kernel<false>})
+        if (const cudaError_t s = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); s != cudaSuccess) return s;
+      cudaLaunchConfig_t c{};
+      cudaLaunchAttribute a[1];
+      a[0].id = cudaLaunchAttributeClusterDimension;
+      a[0].val.clusterDim.x = 16;
+      a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
+      c.gridDim = dim3(16);
+      c.blockDim = dim3(kPowerThreads);
+      c.dynamicSmemBytes = 3 * kMaxPowerSize * sizeof(float);
+      c.attrs = a;
+      c.numAttrs = 1;
+      return cudaOccupancyMaxActiveClusters(&found, power_iteration_kernel<true>, &c);
+    });
+  if (e != cudaSuccess) return e;
+  if (n > kMaxPowerSize || iterations < 0) return cudaErrorInvalidValue;
+  if (batch == 0 || n == 0) return cudaSuccess;
+  // sixteen where every matrix still gets its cluster at once and has rows for them (8 / 16 CTAs: one of 512^2 23 / 23 us, four of 1024^2 49 / 37, of
+  // 2048^2 146 / 89)
+  const int ctas = batch <= held && n >= 512 ? 16 : 8;
+  shape(ctas);
+  return cudaLaunchKernelEx(&cfg, kernel, A, n, iterations, ctas, out);
+}
+
+}  // namespace hb

@@ -436,3 +436,41 @@ def test_rotated_moments_are_as_close_to_64_bits_as_before(turn):
     before = utils.core._mm(utils.core._mm(tf32[0], state, pairs=False), tf32[1], False, True, pairs=False)
     error = lambda x: float((x.double() - want).norm() / want.norm())  # noqa: E731
     assert error(got) <= error(before) and error(got) < 3 * 5.2e-6
+
+
+@pytest.mark.parametrize("batch,n", [(1, 1), (3, 2), (2, 31), (1, 130), (8, 1024), (2, 1001), (3, 2048), (1, 4097)])
+@pytest.mark.parametrize("iterations", [0, 2, 4])
+@pytest.mark.parametrize("scale", [1.0, 1e-30, 1e15])
+def test_power_iteration_in_one_launch_matches_its_operations_in_64_bits(batch, n, iterations, scale, monkeypatch):
+    """Sums of n terms in fp32, in another order than the library's: the estimate is a quotient of such sums, good to n 2^-24 at worst and about
+    the square root of that in fact; 1e-5 covers the former up to a few hundred and the latter with room.  Scales whose squares leave fp32 are none
+    of the iteration's business (row norms overflow there, as they did): 1e15 and 1e-30 stay inside once divided by the largest norm."""
+    from heavyball_b200.utils import psgd
+
+    gen = torch.Generator("cuda").manual_seed(n)
+    b = torch.randn(batch, n, n, device="cuda", generator=gen) / n**0.5
+    a = (b @ b.mT + torch.eye(n, device="cuda")) * scale
+    if scale < 1e-20:
+        a = a * 1e12  # squares of 1e-18 are normal numbers
+    got = psgd.max_eigenvalue_spd(a, power_iter=iterations)
+    assert got.shape == (batch,)
+    wide = a.double()
+    norms = wide.norm(dim=-1)
+    top = norms.amax(-1)
+    x = wide[torch.arange(batch), norms.argmax(-1)] / top[:, None]
+    m = wide / top[:, None, None]
+    for _ in range(iterations):
+        x = torch.einsum("bij,bj->bi", m, torch.einsum("bij,bj->bi", m, x))
+        x = x / x.norm(dim=-1, keepdim=True)
+    want = (x * torch.einsum("bij,bj->bi", m, torch.einsum("bij,bj->bi", m, x))).sum(-1).sqrt() * top
+    torch.testing.assert_close(got.double(), want, rtol=1e-5, atol=0)
+
+
+def test_power_iteration_of_zeros_and_of_what_is_not_finite():
+    from heavyball_b200.utils import psgd
+
+    a = torch.zeros(3, 64, 64, device="cuda")
+    a[1] = torch.eye(64, device="cuda")
+    a[2, 3, 5] = float("nan")
+    got = psgd.max_eigenvalue_spd(a, power_iter=2)
+    assert got[0] == 0 and abs(float(got[1]) - 1) < 1e-6 and bool(got[2].isnan())
