@@ -403,19 +403,20 @@ struct ChainKind {
   // on 8 x 2048^2: 287 -> 265 us), and where the rule is a constant - which also takes the spills of the ten-way switch away (255) - the next
   // vector is fetched ahead of this one's arithmetic (232; three blocks, at two 248).  Without MARS 228 -> 169 us; Adam into fp32
   // parameters 195 -> 174, into error-corrected ones 245 -> 232; exponential average of 25 M elements (one state: four blocks) 122 -> 75;
-  // momentum with MARS of a Llama-3-8B layer, at the clock that the products around it leave, 1.71 -> 1.45 ms.
-  // The rules that steps use most are compiled in; fp32 state is not worth it (momentum 250 -> 340 us: without spills, but with fewer loads in flight).
+  // momentum with MARS of a Llama-3-8B layer, at the clock that the products around it leave, 1.71 -> 1.42 ms.
+  // The rules that steps use most are compiled in; of fp32 state only Nesterov's momentum, which spills without that (85 M elements: 228 -> 202 us;
+  // Adam 165.6 -> 165.4, not worth a kernel).
   static constexpr bool ecc = DTS == kBF16E8;
   // Otherwise a thread should have about 128 bytes on their way: two vectors of Adam's four arrays, four where a launch reads
-  // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 288 us with two vectors,
-  // 250 with four, of which the bytes take 207 at 6.54 TB/s).
-  // The momentum kinds spill at these counts (60 to 148 bytes per thread; the others at most 20): the times above are with
-  // the spills, and the counts that spill 12 bytes or nothing are the slower ones.
+  // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 202 us, of which the
+  // bytes take 207 at 6.54 TB/s).
   static constexpr int batch = ecc ? 1 : (state && (reads_p || count) ? 2 : 4);
   static constexpr int rule_n = rule_states(RULE);
   static constexpr bool one_state = RULE != kAnyRule && rule_n == 1;
   static constexpr bool ahead = ecc && RULE != kAnyRule;  // the next vector is fetched ahead
   static constexpr int min_blocks = ahead ? (one_state ? 4 : 3) : state && !(ecc && !count) ? 3 : 4;
+  // Adam's four fp32 arrays at two vectors are in flight either way (166 us with the test per load on 39.5 M elements, 169 with one for all)
+  static constexpr bool either = state && reads_p && DTS == kF32 && DTG == kF32;
   static bool takes(const ChainParams& P, bool counting) {
     return counting == COUNT && P.out_mode == OUT && P.u_is_input == UIN && (!reads_p || P.dt_p == DTP) &&
            (!reads_g || P.dt_g == DTG) && ((OUT == kOutParam && !u_in) || P.dt_u == DTU) && P.dt_s == DTS &&
@@ -469,6 +470,9 @@ __device__ __forceinline__ StateDraws draw_states(bool mars, int n_state, const 
   return r;
 }
 
+template <int kCase>
+using LoadAs = std::integral_constant<int, kCase>;
+
 template <class K, class Table>
 __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(const __grid_constant__ Table T, ChainParams P) {
   // a launch that applies a parked update walks backwards: what the launch before it wrote last is still in the L2
@@ -500,19 +504,24 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
   float sumsq_local = 0.f, nonzero_local = 0.f;
 
   const int64_t first = base + threadIdx.x * 4;
-  const auto fetch = [&](int64_t i, Raw4& s0, Raw4& s1, Raw4& old, Raw4& g, Raw4& u, Raw4& p) {
+  const auto fetch_as = [&](auto load_case, int64_t i, Raw4& s0, Raw4& s1, Raw4& old, Raw4& g, Raw4& u, Raw4& p) {
+    constexpr int kCase = decltype(load_case)::value;
     const int nv = (int)max((int64_t)0, min((int64_t)4, end - i));
     if (K::state) {
-      s0 = load_raw<K::dt_s>(m0, m0e, i, nv, vec_ok);
-      if (!K::one_state) s1 = load_raw<K::dt_s>(m1, m1e, i, nv, vec_ok);
-      if (K::mars(P)) old = load_raw<K::dt_s>(mm, mme, i, nv, vec_ok);
+      s0 = load_raw<K::dt_s, kCase>(m0, m0e, i, nv, vec_ok);
+      if (!K::one_state) s1 = load_raw<K::dt_s, kCase>(m1, m1e, i, nv, vec_ok);
+      if (K::mars(P)) old = load_raw<K::dt_s, kCase>(mm, mme, i, nv, vec_ok);
     }
-    if (K::reads_g) g = load_raw<K::dt_g>(mg, nullptr, i, nv, vec_ok);
-    if (K::u_in) u = load_raw<K::dt_u>(mu, nullptr, i, nv, vec_ok);
-    if (K::reads_p) p = load_raw<K::dt_p>(mp, mpe, i, nv, vec_ok);
+    if (K::reads_g) g = load_raw<K::dt_g, kCase>(mg, nullptr, i, nv, vec_ok);
+    if (K::u_in) u = load_raw<K::dt_u, kCase>(mu, nullptr, i, nv, vec_ok);
+    if (K::reads_p) p = load_raw<K::dt_p, kCase>(mp, mpe, i, nv, vec_ok);
   };
   Raw4 s0_next{}, s1_next{}, old_next{}, g_next{}, u_next{}, p_next{};
-  if constexpr (K::ahead) fetch(first, s0_next, s1_next, old_next, g_next, u_next, p_next);
+  const auto fetch_next = [&](int64_t i) {
+    if (vec_ok && i + 4 <= end) fetch_as(LoadAs<kWhole>{}, i, s0_next, s1_next, old_next, g_next, u_next, p_next);
+    else fetch_as(LoadAs<kElements>{}, i, s0_next, s1_next, old_next, g_next, u_next, p_next);
+  };
+  if constexpr (K::ahead) fetch_next(first);
 
 #pragma unroll 1
   for (int64_t i0 = first; i0 < end; i0 += kBatch * kThreads * 4) {
@@ -520,10 +529,16 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
     StateDraws rnd[kBatch];
     if constexpr (K::ahead) {  // (past the end: nothing is read)
       s0[0] = s0_next; s1[0] = s1_next; old[0] = old_next; g[0] = g_next; u[0] = u_next; p[0] = p_next;
-      fetch(i0 + kThreads * 4, s0_next, s1_next, old_next, g_next, u_next, p_next);
+      fetch_next(i0 + kThreads * 4);
+    } else if constexpr (K::either) {
+#pragma unroll
+      for (int v = 0; v < kBatch; ++v) fetch_as(LoadAs<kEither>{}, i0 + v * (kThreads * 4), s0[v], s1[v], old[v], g[v], u[v], p[v]);
+    } else if (vec_ok && i0 + (kBatch - 1) * (kThreads * 4) + 4 <= end) {  // only a part's last batch is not whole
+#pragma unroll
+      for (int v = 0; v < kBatch; ++v) fetch_as(LoadAs<kWhole>{}, i0 + v * (kThreads * 4), s0[v], s1[v], old[v], g[v], u[v], p[v]);
     } else {
 #pragma unroll
-      for (int v = 0; v < kBatch; ++v) fetch(i0 + v * (kThreads * 4), s0[v], s1[v], old[v], g[v], u[v], p[v]);
+      for (int v = 0; v < kBatch; ++v) fetch_as(LoadAs<kElements>{}, i0 + v * (kThreads * 4), s0[v], s1[v], old[v], g[v], u[v], p[v]);
     }
     if constexpr (K::ecc) {
 #pragma unroll
@@ -684,6 +699,7 @@ using Kinds = KindList<
     ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, false, kExpAvg>,
     ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, false, kNesterovEma>,
     ChainKind<kNone, kBF16, kF32, kBF16E8, kOutUpdate, 0, false, kNesterovEma, true>,
+    ChainKind<kNone, kF32, kF32, kF32, kOutUpdate, 0, false, kNesterovEma>,
     ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, true, kAdam, false>,
     ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, true, kAdam, true>,
     // any rule

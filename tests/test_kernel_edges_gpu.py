@@ -92,6 +92,48 @@ def test_rules_known_at_compile_time_match_the_general_kernel(algo, mars, grad, 
                 torch.testing.assert_close(a, b, rtol=2**-14, atol=1e-30)
 
 
+@pytest.mark.parametrize("kind", ["momentum", "momentum-ecc", "caution", "update-ecc", "adam", "adam-bf16"])
+@pytest.mark.parametrize("sizes", [(1, 3, 4, 5), (1023, 1024, 1025, 4092, 4095), (4096, 4097, 4100, 8188, 8192), (2_000_003, 2_500_000)], ids=str)
+def test_whole_and_element_loads_read_the_same_values(sizes, kind):
+    """A batch of vectors is loaded whole where all its elements are there and the buffers start on a 16-byte boundary, else
+    element by element.  The arithmetic and the random bits of an element don't depend on that: off the boundary the same bits come out."""
+
+    def run(shift):
+        gen = torch.Generator(DEV).manual_seed(7)
+
+        def made(dtype, positive=False):
+            values = [torch.randn(n, device=DEV, generator=gen) for n in sizes]
+            return [torch.zeros(v.numel() + shift, dtype=dtype, device=DEV)[shift:].copy_(v.abs() if positive else v) for v in values]
+
+        masked = torch.zeros(len(sizes), dtype=torch.int32, device=DEV)
+        if kind.startswith("momentum"):
+            ecc = kind == "momentum-ecc"
+            lists = {"g": made(torch.bfloat16 if ecc else torch.float32), "s0": made(torch.bfloat16 if ecc else torch.float32), "u": made(torch.float32)}
+            if ecc:
+                lists["s0e"] = made(torch.int8)
+            cfg = dict(algo=ops.NESTEROV_EMA, n_state=1, b1=0.9, out_mode=ops.OUT_UPDATE, dt_u=ops.F32, dt_p=ops.NONE,
+                       dt_g=ops.BF16 if ecc else ops.F32, dt_s=ops.BF16E8 if ecc else ops.F32)  # fmt: skip
+        elif kind == "caution":
+            lists = {"g": made(torch.bfloat16), "u": made(torch.float32)}
+            cfg = dict(algo=ops.IDENTITY, u_is_input=1, count_caution=1, masked=masked, out_mode=ops.OUT_UPDATE,
+                       dt_u=ops.F32, dt_g=ops.BF16, dt_s=ops.NONE, dt_p=ops.NONE)  # fmt: skip
+        elif kind == "update-ecc":
+            lists = {"p": made(torch.bfloat16), "pe": made(torch.int8), "u": made(torch.float32)}
+            cfg = dict(algo=ops.IDENTITY, u_is_input=1, out_mode=ops.OUT_PARAM, dt_u=ops.F32, dt_p=ops.BF16E8,
+                       dt_g=ops.NONE, dt_s=ops.NONE, lr=1e-2, wd=0.1)  # fmt: skip
+        else:
+            dtype, dt = (torch.float32, ops.F32) if kind == "adam" else (torch.bfloat16, ops.BF16)
+            lists = {"p": made(dtype), "g": made(dtype), "s0": made(torch.float32), "s1": made(torch.float32, True)}
+            cfg = dict(algo=ops.ADAM, n_state=2, b1=0.9, b2=0.99, eps=1e-8, out_mode=ops.OUT_PARAM, dt_p=dt, dt_g=dt, dt_s=ops.F32, lr=1e-2, wd=0.1)
+        ops.fused_chain(**lists, **cfg, seed=3)
+        return {**lists, "masked": [masked]}
+
+    whole, elements = run(0), run(1)
+    for name, tensors in whole.items():
+        for a, b in zip(tensors, elements[name]):
+            assert torch.equal(a, b), (name, a.numel(), int((a != b).sum()))
+
+
 @pytest.mark.parametrize("kw", [{}, {"ecc": "bf16+8", "mars": True, "caution": True}, {"ecc": "bf16+8"}, {"caution": True}], ids=str)
 @pytest.mark.parametrize("sizes", [(1,), (2047, 2048, 2049), (8191, 8193, 3, 16384), tuple(range(1, 41)), (10_000_000, 5),
                                    (4095, 4096, 4097, 2_500_001, 7), (8191, 8192, 8193, 1, 10_000_000, 5)], ids=len)  # fmt: skip
