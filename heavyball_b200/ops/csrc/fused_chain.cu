@@ -401,16 +401,19 @@ struct ChainKind {
   // error-corrected state one vector is as many as fit.  What such a launch then waits for is that vector's loads (a third of its stalls) and the
   // ten dependent rounds of a random draw.  So the random bits are drawn side by side between the loads and their first use (cautious Adam with MARS
   // on 8 x 2048^2: 287 -> 265 us), and where the rule is a constant - which also takes the spills of the ten-way switch away (255) - the next
-  // vector is fetched ahead of this one's arithmetic (232; three blocks, at two 248).  Without MARS 228 -> 169 us; Adam into fp32
-  // parameters 195 -> 174, into error-corrected ones 245 -> 232; exponential average of 25 M elements (one state: four blocks) 122 -> 75;
+  // vector is fetched ahead of this one's arithmetic (231; three blocks, at two 248).  Without MARS 228 -> 162 us; Adam into fp32
+  // parameters 195 -> 169, into error-corrected ones 245 -> 222; exponential average of 25 M elements (one state: four blocks) 122 -> 75;
   // momentum with MARS of a Llama-3-8B layer, at the clock that the products around it leave, 1.71 -> 1.42 ms.
   // The rules that steps use most are compiled in; of fp32 state only Nesterov's momentum, which spills without that (85 M elements: 228 -> 202 us;
   // Adam 165.6 -> 165.4, not worth a kernel).
+  // Launches without codec state draw the bits of 16-bit parameters early too (64 M elements, Adam into bf16: 254 -> 235 us; a parked update
+  // into bf16, four vectors: 111 -> 91; into error-corrected parameters, where four vectors no longer fit: 159 -> 166, with two vectors 167 -> 145).
   static constexpr bool ecc = DTS == kBF16E8;
+  static constexpr bool p_draws = (DTP == kBF16E8 || DTP == kBF16) && !ecc && OUT == kOutParam;
   // Otherwise a thread should have about 128 bytes on their way: two vectors of Adam's four arrays, four where a launch reads
   // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 202 us, of which the
   // bytes take 207 at 6.54 TB/s).
-  static constexpr int batch = ecc ? 1 : (state && (reads_p || count) ? 2 : 4);
+  static constexpr int batch = ecc ? 1 : (DTP == kBF16E8 && !state) ? 2 : (state && (reads_p || count) ? 2 : 4);
   static constexpr int rule_n = rule_states(RULE);
   static constexpr bool one_state = RULE != kAnyRule && rule_n == 1;
   static constexpr bool ahead = ecc && RULE != kAnyRule;  // the next vector is fetched ahead
@@ -540,6 +543,17 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
 #pragma unroll
       for (int v = 0; v < kBatch; ++v) fetch_as(LoadAs<kElements>{}, i0 + v * (kThreads * 4), s0[v], s1[v], old[v], g[v], u[v], p[v]);
     }
+    uint4 p_rnd[kBatch];
+    if constexpr (K::p_draws) {
+#pragma unroll
+      for (int v = 0; v < kBatch; ++v) {
+        const int64_t i = i0 + v * (kThreads * 4);
+        p_rnd[v] = make_uint4((uint32_t)(i >> 2), (uint32_t)(i >> 34), (uint32_t)t, 3u);
+      }
+      rng.rounds(p_rnd);
+#pragma unroll
+      for (int v = 0; v < kBatch; ++v) pin(p_rnd[v]);
+    }
     if constexpr (K::ecc) {
 #pragma unroll
       for (int v = 0; v < kBatch; ++v) rnd[v] = draw_states(K::mars(P), K::n_state(P), rng, i0 + v * (kThreads * 4), (uint32_t)t);
@@ -603,7 +617,7 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
         if (P.cautious_wd && ((__float_as_uint(np.v[k]) ^ __float_as_uint(uu)) >> 31)) d = 0.f;
         np.v[k] = np.v[k] * (1.0f - d * P.lr) + uu * -P.lr;
       }
-      store_values<K::dt_p>(mp, mpe, i, nv, vec_ok, np, draw(K::dt_p, rng, ctr, ctr_hi, (uint32_t)t, 3u));
+      store_values<K::dt_p>(mp, mpe, i, nv, vec_ok, np, K::p_draws ? p_rnd[v] : draw(K::dt_p, rng, ctr, ctr_hi, (uint32_t)t, 3u));
     }
   }
   finish_block<K::count>(P, M, sumsq_local, nonzero_local, masked_local);
