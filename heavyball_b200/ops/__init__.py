@@ -360,6 +360,7 @@ def matmul3(a: torch.Tensor, b: torch.Tensor, trans_a: bool = False, trans_b: bo
     cores with the 3-term split (measured error about 2^-18 of ``|a| @ |b|``; one tf32 pass gives 2^-11, fp32 SIMT 2^-21).
     ``upper_upper``: ``op(a)`` and ``op(b)`` are upper triangular matrices of one size (entries below their diagonals
     ARE zero): a sixth of the tile products, and exact zeros below the diagonal of the result."""
+    launch_counter.count += 1  # a pass per operand
     return _matmul(load().tf32x3_matmul, a, b, trans_a, trans_b, alpha, upper_upper)
 
 
@@ -375,7 +376,7 @@ def split16_accumulate(c: torch.Tensor, a: torch.Tensor, b: torch.Tensor, trans_
     """``c += alpha * a @ op(b)`` from fp16 pairs, in place on the fp32 view ``c``; all three ``[batch, rows, cols]`` with unit inner
     stride, ``c`` apart from the others."""
     load().split16_accumulate(c, a, b, trans_b, alpha, _status(a.device))
-    launch_counter.count += 3
+    launch_counter.count += 2
 
 
 def _dense(x: torch.Tensor, trans: bool):
@@ -394,5 +395,5 @@ def _matmul(kernel, a, b, trans_a, trans_b, alpha, upper_upper):
     a3, trans_a = _dense(a.reshape(-1, *a.shape[-2:]), trans_a)
     b3, trans_b = _dense(b.reshape(-1, *b.shape[-2:]), trans_b)
     out = kernel(a3, b3, trans_a, trans_b, alpha, _status(a.device), upper_upper)
-    launch_counter.count += 3
+    launch_counter.count += 2
     return out.reshape(*lead, *out.shape[-2:])

@@ -535,8 +535,8 @@ std::vector<at::Tensor> split16(const at::Tensor& x, bool want_same, bool want_t
     out[2 * i + 1] = at::empty({batch, hb::split16_units(rows)}, x.options().memory_format(at::MemoryFormat::Contiguous));
     op[i] = {out[2 * i].data_ptr(), out[2 * i + 1].data_ptr<float>(), source_of(x, i == 1)};
   }
-  check(hb::launch_split16(x.data_ptr<float>(), x.stride(1), x.stride(0), (int)R, (int)C, (int)batch, op[0], op[1],
-                           at::cuda::getCurrentCUDAStream()), "split16");
+  const hb::Split16Pass pass{x.data_ptr<float>(), x.stride(1), x.stride(0), (int)R, (int)C, op[0], op[1]};
+  check(hb::launch_split16(&pass, 1, (int)batch, at::cuda::getCurrentCUDAStream()), "split16");
   return out;
 }
 
@@ -610,11 +610,11 @@ void split16_product(const at::Tensor& a, const at::Tensor& b, bool ta, bool tb,
   const hb::Split16Operand A{p, (float*)(p + a_bytes + b_bytes), source_of(a, ta)};
   // B as the K-major [N, K] operand: b given as [K, N] must be transposed, b given as [N, K] is used as it is
   const hb::Split16Operand B = one ? A : hb::Split16Operand{p + a_bytes, (float*)(p + a_bytes + b_bytes + a_units), source_of(b, !tb)};
-  check(hb::launch_split16(a.data_ptr<float>(), a.stride(1), a.stride(0), (int)a.size(1), (int)a.size(2), (int)batch, ta ? none : A, ta ? A : none, stream),
-        "split16 of the left operand");
-  if (!one)
-    check(hb::launch_split16(b.data_ptr<float>(), b.stride(1), b.stride(0), (int)b.size(1), (int)b.size(2), (int)batch, tb ? B : none, tb ? none : B, stream),
-          "split16 of the right operand");
+  const auto pass_of = [&](const at::Tensor& t, bool as_rows, const hb::Split16Operand& to) {
+    return hb::Split16Pass{t.data_ptr<float>(), t.stride(1), t.stride(0), (int)t.size(1), (int)t.size(2), as_rows ? to : none, as_rows ? none : to};
+  };
+  const hb::Split16Pass passes[2] = {pass_of(a, !ta, A), pass_of(b, tb, B)};
+  check(hb::launch_split16(passes, one ? 1 : 2, (int)batch, stream), "split16 of a product's operands");
   hb::Tf32Epilogue E{};
   E.mode = mode; E.alpha = (float)alpha;
   E.C = c.data_ptr<float>(); E.ldc = c.stride(1); E.strideC = c.stride(0);

@@ -106,19 +106,39 @@ __device__ __forceinline__ float4 load4(const float* p, int left, bool vec) {
 // position of row r of column c in the turned tile: four columns of a thread and four rows of a warp fall into distinct banks
 __device__ __forceinline__ int turned(int c, int r) { return c * kStripRows + (r ^ (c & ~3)); }
 
-__global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* __restrict__ src, int64_t ld_src, int64_t stride_src, int R, int C,
-                                                                 int row_blocks, int cluster, uint16_t* __restrict__ same,
-                                                                 float* __restrict__ same_unit, uint16_t* __restrict__ trans,
-                                                                 float* __restrict__ trans_unit) {
+// One or two source matrices per batch entry: the two operands of a product come from one launch, side by side (the blocks of the first
+// come first), with the cluster of the one that needs the larger.  Such passes are short - 8 of 1024 x 128 rows 7.5 us, 8 of 128 x 128 columns 8.6 - and a pass of its own for the second operand was
+// one more step of a chain of dependent launches: a PSGD fit of 8 of 1024^2 takes 1645 us with a launch each, 1621 with one.
+struct SplitJob {
+  const float* src;
+  int64_t ld, stride;
+  uint16_t *same, *trans;
+  float *same_unit, *trans_unit;
+  int R, C, row_blocks, blocks;  // of `blocks`, the first `row_blocks` write rows (both multiples of the cluster)
+};
+struct SplitJobs {
+  SplitJob job[2];
+};
+
+__global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const __grid_constant__ SplitJobs jobs, int cluster) {
   griddep_wait();
   griddep_launch();
+  const bool second = (int)blockIdx.x >= jobs.job[0].blocks;  // the same for the blocks of a cluster
+  const SplitJob& J = jobs.job[second];
+  const int block = (int)blockIdx.x - (second ? jobs.job[0].blocks : 0), row_blocks = J.row_blocks, R = J.R, C = J.C;
+  const float* __restrict__ const src = J.src;
+  const int64_t ld_src = J.ld, stride_src = J.stride;
+  uint16_t* __restrict__ const same = J.same;
+  uint16_t* __restrict__ const trans = J.trans;
+  float* __restrict__ const same_unit = J.same_unit;
+  float* __restrict__ const trans_unit = J.trans_unit;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t batch = blockIdx.y;
   const float* s = src + batch * stride_src;
   const bool vec = (ld_src & 3) == 0 && (stride_src & 3) == 0 && (((uintptr_t)src) & 15) == 0;
 
-  if ((int)blockIdx.x < row_blocks) {  // whole clusters take this branch (row_blocks is a multiple of `cluster`)
-    const int r = blockIdx.x * (kSplitThreads / 32) + warp;
+  if (block < row_blocks) {  // whole clusters take this branch (row_blocks is a multiple of `cluster`)
+    const int r = block * (kSplitThreads / 32) + warp;
     if (r >= R) return;
     const int kp = (C + 63) / 64 * 64;
     const float* row = s + (int64_t)r * ld_src;
@@ -171,7 +191,7 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* 
   __shared__ uint32_t tops[kStrip];  // of this block's rows; the blocks of the cluster read each other's
   __shared__ uint32_t short_below[kStrip], shorts[kStrip];
   __shared__ float muls[kStrip];
-  const int at = blockIdx.x - row_blocks, rank = at % cluster, c0 = at / cluster * kStrip;
+  const int at = block - row_blocks, rank = at % cluster, c0 = at / cluster * kStrip;
   const int q = threadIdx.x & 7, line = threadIdx.x >> 3, c = c0 + q * 4, kp = (R + 63) / 64 * 64;
   const int first = rank * kStripRows, step = cluster * kStripRows;
   float4 v[kStripRows / 32];
@@ -306,16 +326,26 @@ int g_split16_tile = 0;
 
 void set_split16_gemm_tile_override(int tile) { g_split16_tile = (tile == 128 || tile == 256) ? tile : 0; }
 
-cudaError_t launch_split16(const float* src, int64_t ld_src, int64_t stride_src, int R, int C, int batch, Split16Operand same,
-                           Split16Operand trans, cudaStream_t stream) {
-  if (R == 0 || C == 0 || batch == 0 || (same.data == nullptr && trans.data == nullptr)) return cudaSuccess;
-  const int strips = trans.data != nullptr ? (C + kStrip - 1) / kStrip : 0;
+cudaError_t launch_split16(const Split16Pass* passes, int n, int batch, cudaStream_t stream) {
+  SplitJobs jobs{};
+  if (n < 1 || n > 2 || batch == 0) return n < 1 || n > 2 ? cudaErrorInvalidValue : cudaSuccess;
   int cluster = 1;  // strips longer than one block's rows are shared
-  while (strips > 0 && cluster < kMaxSplitCluster && cluster * kStripRows < R) cluster *= 2;
-  int row_blocks = same.data != nullptr ? (R + kSplitThreads / 32 - 1) / (kSplitThreads / 32) : 0;
-  row_blocks = (row_blocks + cluster - 1) / cluster * cluster;
+  for (int i = 0; i < n; ++i)
+    while (passes[i].trans.data != nullptr && cluster < kMaxSplitCluster && cluster * kStripRows < passes[i].R) cluster *= 2;
+  int used = 0, blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    const Split16Pass& p = passes[i];
+    if (p.R == 0 || p.C == 0 || (p.same.data == nullptr && p.trans.data == nullptr)) continue;
+    const int strips = p.trans.data != nullptr ? (p.C + kStrip - 1) / kStrip : 0;
+    int row_blocks = p.same.data != nullptr ? (p.R + kSplitThreads / 32 - 1) / (kSplitThreads / 32) : 0;
+    row_blocks = (row_blocks + cluster - 1) / cluster * cluster;
+    jobs.job[used] = {p.src, p.ld, p.stride, (uint16_t*)p.same.data, (uint16_t*)p.trans.data, p.same.unit, p.trans.unit,
+                      p.R, p.C, row_blocks, row_blocks + strips * cluster};
+    blocks += jobs.job[used++].blocks;
+  }
+  if (used == 0) return cudaSuccess;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3(row_blocks + strips * cluster, batch);
+  cfg.gridDim = dim3(blocks, batch);
   cfg.blockDim = dim3(kSplitThreads);
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
@@ -326,8 +356,7 @@ cudaError_t launch_split16(const float* src, int64_t ld_src, int64_t stride_src,
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, split16_kernel, src, ld_src, stride_src, R, C, row_blocks, cluster, (uint16_t*)same.data, same.unit,
-                            (uint16_t*)trans.data, trans.unit);
+  return cudaLaunchKernelEx(&cfg, split16_kernel, jobs, cluster);
 }
 
 cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N, int K, int batch, const Tf32Epilogue& E, int* status,

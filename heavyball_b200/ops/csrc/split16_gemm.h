@@ -28,10 +28,16 @@ struct Split16Operand {
   Split16Source src;
 };
 
-// src: [batch, R, C] fp32 (row stride ld_src, batch stride stride_src).  Writes either or both operands (data null = not wanted):
+// src: [batch, R, C] fp32 (row stride ld, batch stride `stride`).  Writes either or both operands (data null = not wanted):
 //   same : rows = src rows, K = C;   trans: rows = src columns, K = R
-cudaError_t launch_split16(const float* src, int64_t ld_src, int64_t stride_src, int R, int C, int batch, Split16Operand same,
-                           Split16Operand trans, cudaStream_t stream);
+struct Split16Pass {
+  const float* src;
+  int64_t ld, stride;
+  int R, C;
+  Split16Operand same, trans;
+};
+// One or two passes over matrices of one batch in a launch.
+cudaError_t launch_split16(const Split16Pass* passes, int n, int batch, cudaStream_t stream);
 
 // out[b] = epilogue(A[b] * B[b]^T); epilogue and flags as for launch_tf32_gemm, without split outputs (E.S null).
 cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N, int K, int batch, const Tf32Epilogue& E, int* status,

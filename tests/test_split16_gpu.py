@@ -339,3 +339,18 @@ def test_accumulation_into_a_view_with_one_allocation(M, N, K, tb, tile):
     with pytest.raises(RuntimeError):
         ops.split16_accumulate(ac, ac, bc, bool(tb))
     ops.check_status()
+
+
+@pytest.mark.parametrize("ta,tb", [(False, False), (True, False), (False, True), (True, True)])
+@pytest.mark.parametrize("B,M,K,N", [(1, 1, 1, 1), (2, 33, 64, 31), (3, 128, 300, 129), (1, 257, 2100, 40), (2, 1030, 128, 1100)])
+def test_operands_of_a_product_from_one_launch(ta, tb, B, M, K, N):
+    """The launch that makes both operands of a product gives each what a launch of its own gives (the same bits), whatever cluster the other
+    one needs; rows with values too small for 22 bits among them."""
+    a, b = _rand(B, *((K, M) if ta else (M, K)), seed=41), _rand(B, *((N, K) if tb else (K, N)), seed=42)
+    a[:, ::3] *= 2.0**-20
+    b[..., ::5] *= 2.0**-31
+    pa = ops.split16(a, not ta, ta)[1 if ta else 0]
+    pb = ops.split16(b, tb, not tb)[0 if tb else 1]
+    want = torch.empty(B, M, (N + 3) // 4 * 4, device="cuda")[..., :N]
+    ops.split16_gemm(pa, pb, out=want)
+    assert torch.equal(ops.matmul16(a, b, ta, tb), want)
