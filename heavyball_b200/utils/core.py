@@ -458,7 +458,7 @@ def apply_flat_add(params: List[Tensor], update: Tensor, alpha):
 
 # Two tensor-core products of fp32 matrices exist: of fp16 pairs (the faster and more exact one; results that hang on values which a pair does
 # not hold are computed in fp32, many times slower) and split-tf32.  Everything that an
-# eigenbasis is made from - statistics, power iteration, orthogonalisation, the rotation of the moments that follows - asks for the
+# eigenbasis is made from - statistics, power iteration, orthogonalisation - asks for the
 # second (``pairs=False``): eigenvectors with nearly equal Rayleigh quotients trade places when the last bits of any of these change,
 # so moving them would move every trajectory (two refreshes of eleven 2048-wide bases: one to three such pairs).
 
