@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(kThreads, 4) fused_chain_kernel(const TensorMe
 // constants, and a kind's batch of vectors per thread is loaded before anything is computed or stored (stores may alias later loads,
 // so the compiler cannot move those up by itself: a vector at a time is a memory round trip each).  Against the general kernel:
 // AdamW on the 39.5 M fp32 parameters of GPT-2-small's embeddings 242 -> 170 us (6.5 TB/s), cautious AdamW with error-corrected
-// state on 8 x 2048^2 965 -> 562 us, and 353 us with the loads separated from the codec.
+// state on 8 x 2048^2 965 -> 562 us, 353 us with the loads separated from the codec, and 290 us with
+// the rule compiled in (ChainKind).
 // Storage kinds outside the list below (fp16, 16-bit residuals, plain bf16 state, bf16 gradients into an update with fp32 state or
 // without state), peers, clips and the other launches named here run the general kernel at its speed.
 // ---------------------------------------------------------------------------------------------
