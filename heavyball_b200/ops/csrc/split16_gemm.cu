@@ -120,18 +120,9 @@ struct SplitJobs {
   SplitJob job[2];
 };
 
-__global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const __grid_constant__ SplitJobs jobs, int cluster) {
-  griddep_wait();
-  griddep_launch();
-  const bool second = (int)blockIdx.x >= jobs.job[0].blocks;  // the same for the blocks of a cluster
-  const SplitJob& J = jobs.job[second];
-  const int block = (int)blockIdx.x - (second ? jobs.job[0].blocks : 0), row_blocks = J.row_blocks, R = J.R, C = J.C;
-  const float* __restrict__ const src = J.src;
-  const int64_t ld_src = J.ld, stride_src = J.stride;
-  uint16_t* __restrict__ const same = J.same;
-  uint16_t* __restrict__ const trans = J.trans;
-  float* __restrict__ const same_unit = J.same_unit;
-  float* __restrict__ const trans_unit = J.trans_unit;
+__device__ __forceinline__ void split16_block(const float* __restrict__ src, int64_t ld_src, int64_t stride_src, int R, int C, int block, int row_blocks,
+                                              int cluster, uint16_t* __restrict__ same, float* __restrict__ same_unit,
+                                              uint16_t* __restrict__ trans, float* __restrict__ trans_unit) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t batch = blockIdx.y;
   const float* s = src + batch * stride_src;
@@ -281,6 +272,24 @@ __global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const __grid_
     atomicAdd((uint32_t*)&trans_unit[batch * ((C + 255) / 256 * 256) + c0 + threadIdx.x], min(shorts[threadIdx.x], kManyShort));
 }
 
+// A kernel of its own for a single matrix: with the arguments behind a choice the column passes are 3 % slower (2 of 4096^2 71.7 -> 73.9 us).
+__global__ void __launch_bounds__(kSplitThreads, 4) split16_kernel(const float* __restrict__ src, int64_t ld_src, int64_t stride_src, int R, int C,
+                                                                 int row_blocks, int cluster, uint16_t* __restrict__ same,
+                                                                 float* __restrict__ same_unit, uint16_t* __restrict__ trans,
+                                                                 float* __restrict__ trans_unit) {
+  griddep_wait();
+  griddep_launch();
+  split16_block(src, ld_src, stride_src, R, C, blockIdx.x, row_blocks, cluster, same, same_unit, trans, trans_unit);
+}
+__global__ void __launch_bounds__(kSplitThreads, 4) split16_two_kernel(const __grid_constant__ SplitJobs jobs, int cluster) {
+  griddep_wait();
+  griddep_launch();
+  const bool second = (int)blockIdx.x >= jobs.job[0].blocks;  // the same for the blocks of a cluster
+  const SplitJob& J = jobs.job[second];
+  split16_block(J.src, J.ld, J.stride, J.R, J.C, (int)blockIdx.x - (second ? jobs.job[0].blocks : 0), J.row_blocks, cluster, J.same, J.same_unit,
+                J.trans, J.trans_unit);
+}
+
 // fp16 operand [batch, rows, cols]; box = 64 columns x 128 rows, 128-byte swizzle
 bool make_half_map(CUtensorMap* map, const void* base, int rows, int64_t cols, int batch) {
   EncodeTiledFn fn = tensor_map_encoder();
@@ -356,7 +365,9 @@ cudaError_t launch_split16(const Split16Pass* passes, int n, int batch, cudaStre
   attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  return cudaLaunchKernelEx(&cfg, split16_kernel, jobs, cluster);
+  if (used == 2) return cudaLaunchKernelEx(&cfg, split16_two_kernel, jobs, cluster);
+  const SplitJob& J = jobs.job[0];
+  return cudaLaunchKernelEx(&cfg, split16_kernel, J.src, J.ld, J.stride, J.R, J.C, J.row_blocks, cluster, J.same, J.same_unit, J.trans, J.trans_unit);
 }
 
 cudaError_t launch_split16_gemm(Split16Operand A, Split16Operand B, int M, int N, int K, int batch, const Tf32Epilogue& E, int* status,
