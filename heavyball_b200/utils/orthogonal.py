@@ -315,7 +315,8 @@ def _cholesky_qr2_blocks(a: Tensor, bad: Tensor, info: Tensor, shifted_rounds: i
         return ops.load().qr_unit_columns(x, x.norm(dim=-2, keepdim=True).clamp_(min=torch.finfo(x.dtype).tiny))
 
     gram = torch.empty(a.shape[0], k, k, device=a.device, dtype=a.dtype)
-    a, operand = unit_columns(a)
+    # rows are read 16 bytes at a time: a view that begins elsewhere in its buffer is copied
+    a, operand = unit_columns(a if a.data_ptr() % 16 == 0 else a.clone())
     for rnd in range(shifted_rounds + 2):
         ops.tf32_gemm(operand, operand, n, out=gram)
         shifted = rnd < shifted_rounds
