@@ -487,3 +487,20 @@ def test_power_iteration_of_zeros_and_of_what_is_not_finite():
     a[2, 3, 5] = float("nan")
     got = psgd.max_eigenvalue_spd(a, power_iter=2)
     assert got[0] == 0 and abs(float(got[1]) - 1) < 1e-6 and bool(got[2].isnan())
+
+
+@pytest.mark.parametrize("count", [-1, -7])
+@pytest.mark.parametrize("name", ["PSGDKron", "PSGDPRO"])
+def test_a_negative_number_of_power_iterations_is_none(name, count):
+    """``range`` of it is empty; the spectral norms next to it take it as a request for the sketch."""
+    from heavyball_b200.utils import psgd
+
+    b = torch.randn(3, 96, 96, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    a = b @ b.mT
+    torch.testing.assert_close(psgd.max_eigenvalue_spd(a, count), psgd.max_eigenvalue_spd(a, 0), rtol=1e-5, atol=0)
+    p = torch.nn.Parameter(torch.randn(128, 128, device="cuda"))
+    opt = getattr(hb, name)([p], lr=1e-3, precond_update_power_iterations=count)
+    for _ in range(2):
+        p.grad = torch.randn_like(p)
+        opt.step()
+    assert torch.isfinite(p).all()
