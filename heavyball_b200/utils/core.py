@@ -22,6 +22,7 @@ from typing import Iterable, List, Optional, Sequence, Union
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
 from torch.utils._pytree import tree_map
 
 Number = Union[int, float, Tensor]
@@ -501,10 +502,23 @@ def _captured_into(graph):
             gc.enable()
 
 
+def _values_only(*ts: Tensor) -> bool:
+    """Whether nothing but the values of these tensors is asked for, so that a kernel may stand in for PyTorch's operations: no gradient or
+    tangent is recorded, none of them is a subclass or a wrapper of a transform, and nothing traces or intercepts the operations."""
+    if torch.compiler.is_compiling() or torch.jit.is_tracing() or torch._C._len_torch_dispatch_stack() > 0:
+        return False
+    recording, dual = torch.is_grad_enabled(), forward_ad._current_level >= 0
+    return not any(
+        type(t) not in (Tensor, torch.nn.Parameter) or (recording and t.requires_grad) or torch._C._functorch.is_functorch_wrapped_tensor(t)
+        or (dual and forward_ad.unpack_dual(t).tangent is not None)
+        for t in ts
+    )  # fmt: skip
+
+
 def _own_pass(*ts: Tensor):
-    """The extension, for one launch over these tensors, when its element-wise passes apply (contiguous fp32 CUDA tensors on sm_100a), else
-    ``None``."""
-    if not all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() for t in ts):
+    """The extension, for one launch over these tensors, when its element-wise passes apply (values of contiguous fp32 CUDA tensors on sm_100a),
+    else ``None``."""
+    if not all(t.is_cuda and t.dtype == torch.float32 and t.is_contiguous() for t in ts) or not _values_only(*ts):
         return None
     from .. import ops
 
@@ -566,7 +580,7 @@ def _solve_leaf(b: Tensor, inv: Tensor, block: int, x: Tensor):
     """``x <- b inv[:, block]`` for an upper-triangular inverse, sums over its rows in order in fp32: a kernel of its own for whole 128-wide leaves
     (which leaves out the half that is zero), the library's product with the same bits otherwise."""
     d, rows = b.shape[-1], b.shape[-2]
-    if d == _TRSM_LEAF and rows % 64 == 0 and 0 < b.shape[0] <= 65535 and all(
+    if d == _TRSM_LEAF and rows % 64 == 0 and 0 < b.shape[0] <= 65535 and _values_only(b, inv) and all(
         t.is_cuda and t.data_ptr() % 16 == 0 and t.stride(-1) == 1 and t.stride(-2) % 4 == 0 and t.stride(0) % 4 == 0 for t in (b, x)
     ):
         from .. import ops
@@ -584,6 +598,8 @@ def _scaled_matrices(x: Tensor, by: Tensor, divide: bool = False, in_place: bool
     if ext is not None:
         out = x if in_place else torch.empty_like(x)
         ext.scale_matrices(x, by, divide, out)
+        if in_place:
+            torch.autograd.graph.increment_version(x)
         return out
     wide = by.view(-1, *([1] * (x.ndim - 1)))
     if in_place:

@@ -23,7 +23,7 @@ import torch
 from torch import Tensor
 
 from .core import copy_stochastic_, list_guard, promote, stochastic_divide_, stochastic_divide_with_eps_, stochastic_round_
-from .core import _captured_into, _mm, _solve_right_upper, _tc_sub_product
+from .core import _captured_into, _mm, _solve_right_upper, _tc_sub_product, _values_only
 
 
 def _settings():
@@ -300,7 +300,7 @@ def _whole_blocks(a: Tensor) -> bool:
     n, k = a.shape[-2:]
     return (
         _skinny_kernels(a) is not None and getattr(_settings(), "tensor_core_matmul", True)
-        and k >= _CHOLQR_MIN and k % _CHOL_LEAF == 0 and n >= k and n % 64 == 0 and 0 < a.shape[0] <= 65535
+        and k >= _CHOLQR_MIN and k % _CHOL_LEAF == 0 and n >= k and n % 64 == 0 and 0 < a.shape[0] <= 65535 and _values_only(a)
     )  # fmt: skip
 
 

@@ -504,3 +504,62 @@ def test_a_negative_number_of_power_iterations_is_none(name, count):
         p.grad = torch.randn_like(p)
         opt.step()
     assert torch.isfinite(p).all()
+
+
+def _spd(*shape, seed=5):
+    b = torch.randn(*shape, device="cuda", generator=torch.Generator("cuda").manual_seed(seed))
+    return b @ b.mT
+
+
+def test_power_iteration_and_noise_under_gradients_and_transforms():
+    """Kernels in the place of these expressions read values only: where a gradient or a tangent is wanted, or a transform or a trace looks on, the
+    expressions run.  Both are sums and products of a few hundred fp32 values: 1e-4 relative."""
+    from torch.autograd import forward_ad
+    from torch.fx.experimental.proxy_tensor import make_fx
+
+    from heavyball_b200.utils import psgd
+
+    a = _spd(3, 64, 64)
+    eig = lambda m: psgd.max_eigenvalue_spd(m, 2)  # noqa: E731
+    close = lambda x, y: torch.testing.assert_close(x, y, rtol=1e-4, atol=1e-4 * float(y.abs().max()))  # noqa: E731
+    want = eig(a)
+    x = a.clone().requires_grad_()
+    (slope,) = torch.autograd.grad(eig(x).sum(), x)
+    along = torch.randn_like(a)
+    change = (slope * along).sum((-2, -1))
+    close(torch.func.jvp(eig, (a,), (along,))[1], change)
+    with forward_ad.dual_level():
+        close(forward_ad.unpack_dual(eig(forward_ad.make_dual(a, along))).tangent, change)
+    close(torch.func.vmap(eig)(torch.stack([a, 2 * a])), torch.stack([want, 2 * want]))
+    close(make_fx(eig)(a)(4 * a), 4 * want)
+    with torch.no_grad():
+        assert torch.equal(eig(x), want)
+    g = torch.randn(3, 64, 64, device="cuda").requires_grad_()
+    v, damped = psgd.dampen_grad(g, 0.5)
+    (slope,) = torch.autograd.grad(damped.sum(), g)
+    close(slope, 1 + 2.0**-23 * g.sign() * v)
+    noisy = torch.func.vmap(lambda m: psgd.dampen_grad(m, 0.5)[1], randomness="different")(g.detach())
+    assert noisy.shape == g.shape
+
+
+def test_factors_written_in_place_are_seen_by_autograd():
+    """A balanced or updated factor counts as written to (by a kernel, too), and what would lose a gradient is refused."""
+    from heavyball_b200.utils import psgd
+
+    factors = lambda: [torch.eye(128, device="cuda").repeat(2, 1, 1) * s for s in (1.0, 3.0)]  # noqa: E731
+    qs = factors()
+    psgd.psgd_balance_Q(qs)
+    assert all(q._version > 0 for q in qs)
+    qs = factors()
+    qs[0].requires_grad_()
+    with pytest.raises(RuntimeError):
+        psgd.psgd_balance_Q(qs)
+    with pytest.raises(RuntimeError):  # no gradient is recorded through the solve: refused, not dropped
+        utils.core._solve_right_upper(qs[1], torch.randn(2, 128, 128, device="cuda").requires_grad_())
+    with pytest.raises(RuntimeError):
+        utils.inplace_orthogonal_(torch.eye(256, device="cuda").requires_grad_(), "qr")
+    packed = [(tuple(q.shape), psgd.triu_to_line([q])[0][1]) for q in factors()]
+    before = [line._version for _, line in packed]
+    g = torch.randn(2, 128, 128, device="cuda")
+    psgd.psgd_update_precond(g, 0.1, packed, True, 0.9, torch.randn_like(g), [torch.zeros(2, device="cuda") for _ in packed], 0.9, 2)
+    assert all(line._version >= b + 2 for (_, line), b in zip(packed, before))
