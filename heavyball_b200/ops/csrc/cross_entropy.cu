@@ -134,6 +134,13 @@ __global__ void __launch_bounds__(kThreads) ce_fwd_bwd_kernel(__nv_bfloat16* __r
   if (threadIdx.x == 0) x[target] = __float2bfloat16_rn(exp2f(fmaf(x_target, kLog2e, bias)) * coef - g);
 }
 
+// Subnormal values are kept, as the library's multiplication keeps them, against the flags of this library.
+__device__ __forceinline__ float times(float a, float b) {
+  float r;
+  asm("mul.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+  return r;
+}
+
 // Gradients of the head times the gradient of the loss.  That is one unless the caller scales or averages losses, and the host does not know:
 // a block looks first and leaves when there is nothing to do (x * 1 is x), else it is a pass that memory bounds.  50304 x 768 fp32 / 16384 x 768
 // bf16 by itself: the library's multiplication by a device scalar 97 / 41 us, this one 54 / 8, by one what an empty launch takes.
@@ -141,7 +148,7 @@ __global__ void __launch_bounds__(kThreads) scale_kernel(uint4* __restrict__ x, 
   const float by = *s;
   if (by == 1.0f) return;
   const long long step = (long long)gridDim.x * kThreads, full = n / (bf16 ? 8 : 4);
-  const __nv_bfloat16 by16 = __float2bfloat16_rn(by);
+  const float by16 = __bfloat162float(__float2bfloat16_rn(by));
   for (long long i = (long long)blockIdx.x * kThreads + threadIdx.x; i < full; i += step) {
     uint4 v = x[i];
     if (bf16) {
@@ -149,10 +156,10 @@ __global__ void __launch_bounds__(kThreads) scale_kernel(uint4* __restrict__ x, 
       unpack8(v, f);
       __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
 #pragma unroll
-      for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(f[2 * e] * __bfloat162float(by16), f[2 * e + 1] * __bfloat162float(by16));
+      for (int e = 0; e < 4; ++e) h[e] = __floats2bfloat162_rn(times(f[2 * e], by16), times(f[2 * e + 1], by16));
     } else {
-      v = make_uint4(__float_as_uint(__uint_as_float(v.x) * by), __float_as_uint(__uint_as_float(v.y) * by), __float_as_uint(__uint_as_float(v.z) * by),
-                     __float_as_uint(__uint_as_float(v.w) * by));
+      v = make_uint4(__float_as_uint(times(__uint_as_float(v.x), by)), __float_as_uint(times(__uint_as_float(v.y), by)),
+                     __float_as_uint(times(__uint_as_float(v.z), by)), __float_as_uint(times(__uint_as_float(v.w), by)));
     }
     x[i] = v;
   }
@@ -160,9 +167,10 @@ __global__ void __launch_bounds__(kThreads) scale_kernel(uint4* __restrict__ x, 
   if (blockIdx.x == 0 && (int)threadIdx.x < left) {
     if (bf16) {
       __nv_bfloat16* t = reinterpret_cast<__nv_bfloat16*>(x) + full * 8 + threadIdx.x;
-      *t = __float2bfloat16_rn(__bfloat162float(*t) * __bfloat162float(by16));
+      *t = __float2bfloat16_rn(times(__bfloat162float(*t), by16));
     } else {
-      reinterpret_cast<float*>(x)[full * 4 + threadIdx.x] *= by;
+      float* t = reinterpret_cast<float*>(x) + full * 4 + threadIdx.x;
+      *t = times(*t, by);
     }
   }
 }

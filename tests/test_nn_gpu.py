@@ -63,6 +63,20 @@ def test_scaling_by_the_gradient_of_the_loss_has_the_bits_of_the_library(dtype, 
         assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.nan_to_num(7.0), want.nan_to_num(7.0))
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("n", [3, 8, 2051])
+@pytest.mark.parametrize("by", [0.25, 1e-3, 2.0**20, 1e-39])
+def test_scaling_keeps_subnormal_values(dtype, n, by):
+    """Values, products and factors below the smallest normal number, in the vectors and in the remainder."""
+    gen = torch.Generator("cuda").manual_seed(n)
+    x = torch.randn(n, device="cuda", generator=gen) * 10.0 ** torch.randint(-44, -36, (n,), device="cuda", generator=gen)
+    x[-1] = 1e-39
+    got = x.to(dtype)
+    want = got.clone().mul_(torch.tensor(by, device="cuda"))
+    ops.load().scale_(got, torch.tensor(by, device="cuda"))
+    assert torch.equal(got, want) and (by < 1e-30 or bool((want[-1] != 0).all()))
+
+
 @pytest.mark.parametrize("by", [1.0, 0.25])
 def test_head_gradients_are_scaled_by_the_gradient_of_the_loss(by):
     torch.manual_seed(1)
