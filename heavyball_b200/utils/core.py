@@ -17,6 +17,7 @@ import contextlib
 import enum
 import gc
 import sys
+import threading
 import warnings
 from typing import Iterable, List, Optional, Sequence, Union
 
@@ -488,18 +489,28 @@ def _mm_upper(a: Tensor, b: Tensor) -> Tensor:
     return out if out is not None else a @ b
 
 
+_captures = {"under way": 0, "collecting": False}  # of the process, like the collector
+_captures_lock = threading.Lock()
+
+
 @contextlib.contextmanager
 def _captured_into(graph):
     """``torch.cuda.graph(graph)`` with the automatic collection of reference cycles held meanwhile: a cycle that keeps another graph alive
-    (an optimizer that went out of use) would take that graph down with it, and destroying a graph invalidates any capture."""
-    collecting = gc.isenabled()
-    gc.disable()
+    (an optimizer that went out of use) would take that graph down with it, and destroying a graph invalidates any capture.  Threads may
+    capture at once: the collector resumes, if it was on, when the last of them is done."""
+    with _captures_lock:
+        if _captures["under way"] == 0:
+            _captures["collecting"] = gc.isenabled()
+            gc.disable()
+        _captures["under way"] += 1
     try:
         with torch.cuda.graph(graph):
             yield
     finally:
-        if collecting:
-            gc.enable()
+        with _captures_lock:
+            _captures["under way"] -= 1
+            if _captures["under way"] == 0 and _captures["collecting"]:
+                gc.enable()
 
 
 def _values_only(*ts: Tensor) -> bool:

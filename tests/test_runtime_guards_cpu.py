@@ -1,6 +1,10 @@
 """Host-side guards: slab-membership checks of the peer kernels' inputs, rank-invariant kernel seeds, and the
 checkpoint round trip of user-defined preconditioner schedules."""
 
+import contextlib
+import gc
+import threading
+
 import pytest
 import torch
 
@@ -72,3 +76,33 @@ def test_user_schedule_round_trips_only_when_allowed():
         assert fresh.precond_schedule is custom_schedule
     finally:
         pickle_compat.allowed_globals.clear()
+
+
+@pytest.mark.parametrize("collecting", [True, False])
+def test_collector_stays_off_until_the_last_capture_is_done(collecting, monkeypatch):
+    """Two threads capture at once; the one that ends first, by an error, leaves the collector as the other needs it."""
+    from heavyball_b200.utils import core
+
+    monkeypatch.setattr(torch.cuda, "graph", lambda graph: contextlib.nullcontext())
+    inside, first_done = threading.Event(), threading.Event()
+    seen = []
+
+    def second():
+        with core._captured_into(None):
+            inside.set()
+            assert first_done.wait(30)
+            seen.append(gc.isenabled())
+
+    before = gc.isenabled()
+    (gc.enable if collecting else gc.disable)()
+    try:
+        thread = threading.Thread(target=second)
+        with pytest.raises(RuntimeError), core._captured_into(None):
+            thread.start()
+            assert inside.wait(30)
+            raise RuntimeError
+        first_done.set()
+        thread.join()
+        assert seen == [False] and gc.isenabled() == collecting
+    finally:
+        (gc.enable if before else gc.disable)()
