@@ -541,7 +541,8 @@ def _own_pass(*ts: Tensor):
 
 def _transposed(x: Tensor) -> Tensor:
     """``x.mT.contiguous()``."""
-    ext = _own_pass(x) if x.ndim == 3 and 0 < x.shape[0] <= 65535 and max(x.shape[1:]) < 1 << 22 else None
+    # (the kernel counts matrices, and 64 rows at a time, in dimensions of the grid that end at 65535)
+    ext = _own_pass(x) if x.ndim == 3 and 0 < x.shape[0] <= 65535 and x.shape[1] <= 64 * 65535 and x.shape[2] < 1 << 22 else None
     return x.mT.contiguous() if ext is None else ext.transposed(x)
 
 

@@ -337,6 +337,14 @@ def test_passes_over_matrices_have_the_bits_of_the_chains_they_replace(shape):
     assert torch.equal(dense[:, rows, cols], line) and torch.equal(dense, dense.triu())
 
 
+@pytest.mark.parametrize("shape", [(1, 64 * 65535, 32), (1, 64 * 65535 + 1, 32), (1, (1 << 22) - 1, 33), (1, 32, (1 << 22) - 1)], ids=str)
+def test_transposes_of_the_longest_matrices(shape):
+    from heavyball_b200.utils import core
+
+    x = torch.arange(shape[1] * shape[2], dtype=torch.int32, device="cuda").view(torch.float32).view(shape)  # (bits that all differ)
+    assert torch.equal(core._transposed(x).view(torch.int32), x.view(torch.int32).mT)
+
+
 @pytest.mark.parametrize("n,k", [(1, 3), (7, 130), (64, 1024), (100, 2048), (5, 5000), (9, 12288)])
 def test_columns_permuted_and_put_back(n, k):
     x = torch.randn(3, n, k, device="cuda", generator=torch.Generator("cuda").manual_seed(k))
