@@ -565,7 +565,7 @@ def test_factors_written_in_place_are_seen_by_autograd():
     with pytest.raises(RuntimeError):  # no gradient is recorded through the solve: refused, not dropped
         utils.core._solve_right_upper(qs[1], torch.randn(2, 128, 128, device="cuda").requires_grad_())
     with pytest.raises(RuntimeError):
-        utils.inplace_orthogonal_(torch.eye(256, device="cuda").requires_grad_(), "qr")
+        utils.orthogonal._cholesky_qr2(torch.eye(256, device="cuda").requires_grad_())
     packed = [(tuple(q.shape), psgd.triu_to_line([q])[0][1]) for q in factors()]
     before = [line._version for _, line in packed]
     g = torch.randn(2, 128, 128, device="cuda")
