@@ -4,7 +4,8 @@
 // product a matrix-vector kernel, a norm, a clamp and a division.  Here a cluster of CTAs takes a matrix from beginning to end.  A CTA owns a
 // share of the rows, which it reads once for the norms and twice a step (from the L2: 4 MB at 1024), a warp four rows at a time; every CTA keeps
 // the whole vectors in shared memory, and each product's entries are stored into all of them.  What is left of each step is the reading and one
-// cluster barrier per product.  A is divided by its largest row norm on the way, entry by entry, so that no scale of A over- or underflows.
+// cluster barrier per product.  A is divided by its largest row norm on the way, entry by entry: what may not leave fp32 are the squares of its
+// entries and their sums along a row.
 // Two factors of 8 of 1024^2, two iterations each, in the graph of a fit: 245 us of the library's kernels, 2 x 54 here.
 #include "power_iteration.h"
 
@@ -59,6 +60,13 @@ __device__ __forceinline__ float block_sum(float v, float* scratch) {
 // One value per row, from the lanes that hold it to the same place of every CTA.
 __device__ __forceinline__ void store_everywhere(float* to, float v, int lane, int ctas) {
   if (lane < ctas) cluster_store(cluster_addr(to, (uint32_t)lane), __float_as_int(v));
+}
+
+// The row to start from: a NaN before any number, then the largest norm, of equal ones the first row.  Which of them it is decides what a
+// block-diagonal matrix converges to.
+__device__ __forceinline__ bool ranks_before(float norm, int row, float than, int than_row) {
+  if (isnan(norm) || isnan(than)) return isnan(norm) && (!isnan(than) || row < than_row);
+  return norm > than || (norm == than && row < than_row);
 }
 
 // For each row r of [first, last): done(r, s, lane) with s from zero through s <- term(s, a_rk, k).
@@ -117,7 +125,7 @@ __global__ void __launch_bounds__(kPowerThreads) power_iteration_kernel(const fl
   float norm = -1.0f;
   int at = 0;
   for (int i = threadIdx.x; i < n; i += kPowerThreads)
-    if (!(aax[i] <= norm)) {  // (a row with a NaN is the largest)
+    if (ranks_before(aax[i], i, norm, at)) {
       norm = aax[i];
       at = i;
     }
@@ -125,7 +133,7 @@ __global__ void __launch_bounds__(kPowerThreads) power_iteration_kernel(const fl
   for (int o = 16; o > 0; o >>= 1) {
     const float other = __shfl_xor_sync(0xFFFFFFFFu, norm, o);
     const int other_at = __shfl_xor_sync(0xFFFFFFFFu, at, o);
-    if (!(other <= norm) && (other != norm || other_at < at)) {
+    if (ranks_before(other, other_at, norm, at)) {
       norm = other;
       at = other_at;
     }
@@ -138,7 +146,7 @@ __global__ void __launch_bounds__(kPowerThreads) power_iteration_kernel(const fl
   norm = best_norm[0];
   at = best_row[0];
   for (int w = 1; w < kPowerWarps; ++w)
-    if (!(best_norm[w] <= norm)) {
+    if (ranks_before(best_norm[w], best_row[w], norm, at)) {
       norm = best_norm[w];
       at = best_row[w];
     }

@@ -487,6 +487,18 @@ def test_power_iteration_in_one_launch_matches_its_operations_in_64_bits(batch, 
     torch.testing.assert_close(got.double(), want, rtol=1e-5, atol=0)
 
 
+@pytest.mark.parametrize("block,single", [(1, 512), (512, 1), (3, 40), (40, 3), (30, 32), (600, 88), (88, 600), (0, 639), (638, 0)])
+def test_power_iteration_starts_from_the_first_of_equal_rows(block, single):
+    """Rows (3, 4), (4, 3) and (5): norms of 5 that are exact, in blocks of eigenvalues 7 and 5 that the iteration does not leave."""
+    from heavyball_b200.utils import psgd
+
+    a = torch.zeros(1, 640, 640, device="cuda")
+    a[0, block, block] = a[0, block + 1, block + 1] = 3
+    a[0, block, block + 1] = a[0, block + 1, block] = 4
+    a[0, single, single] = 5
+    assert abs(float(psgd.max_eigenvalue_spd(a, power_iter=2)) - (7 if block < single else 5)) < 1e-5
+
+
 def test_power_iteration_of_zeros_and_of_what_is_not_finite():
     from heavyball_b200.utils import psgd
 
