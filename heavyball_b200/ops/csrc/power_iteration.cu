@@ -193,11 +193,14 @@ cudaError_t launch_power_iteration(const float* A, int batch, int n, int iterati
     attr[0].val.clusterDim.x = ctas;
     cfg.gridDim = dim3(batch * ctas);
   };
-  static PerDevice<int> wide_clusters;  // clusters of sixteen that the device holds at once
-  int device = 0, held = 0;
+  struct Device {
+    int clusters, sms;  // of sixteen that it holds at once
+  } on{};
+  static PerDevice<Device> devices;
+  int device = 0;
   cudaError_t e = cudaGetDevice(&device);
   if (e == cudaSuccess)
-    e = wide_clusters.get(device, cudaSuccess, &held, [](int& found) {
+    e = devices.get(device, cudaSuccess, &on, [device](Device& found) {
       for (const auto k : {power_iteration_kernel<true>, power_iteration_kernel<false>})
         if (const cudaError_t s = cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1); s != cudaSuccess) return s;
       cudaLaunchConfig_t c{};
@@ -210,14 +213,19 @@ cudaError_t launch_power_iteration(const float* A, int batch, int n, int iterati
       c.dynamicSmemBytes = 3 * kMaxPowerSize * sizeof(float);
       c.attrs = a;
       c.numAttrs = 1;
-      return cudaOccupancyMaxActiveClusters(&found, power_iteration_kernel<true>, &c);
+      if (const cudaError_t s = cudaOccupancyMaxActiveClusters(&found.clusters, power_iteration_kernel<true>, &c); s != cudaSuccess) return s;
+      return cudaDeviceGetAttribute(&found.sms, cudaDevAttrMultiProcessorCount, device);
     });
   if (e != cudaSuccess) return e;
   if (n > kMaxPowerSize || iterations < 0) return cudaErrorInvalidValue;
   if (batch == 0 || n == 0) return cudaSuccess;
-  // sixteen where every matrix still gets its cluster at once and has rows for them (8 / 16 CTAs: one of 512^2 23 / 23 us, four of 1024^2 49 / 37, of
-  // 2048^2 146 / 89)
-  const int ctas = batch <= held && n >= 512 ? 16 : 8;
+  // Sixteen where every matrix still gets its cluster at once and has rows for them, else eight (two iterations, 8 / 16 CTAs: four of 512^2
+  // 21 / 23 us, of 1024^2 48 / 37, of 2048^2 146 / 138, three of them 146 / 88).  Many small matrices fill the device by themselves, and waves of short
+  // CTAs with barriers between them are all that larger clusters add: while there are more than two CTAs per SM, half as many, as long as each has
+  // no more than 128 rows (8 / 4 / 2 / 1 CTAs: 64 of 64^2 26 / 13 / 12 / 14 us, 1024 of them 382 / 167 / 81 / 57, 256 of 128^2 106 / 51 / 31 / 24, 64 of 256^2
+  // 40 / 22 / 24 / 35, 300 of 512^2 305 / 230 / 366 / 400).
+  int ctas = batch <= on.clusters && n >= 512 ? 16 : 8;
+  while (ctas > 1 && ctas <= 8 && (int64_t)batch * ctas > 2 * on.sms && ctas / 2 * 128 >= n) ctas /= 2;
   shape(ctas);
   return cudaLaunchKernelEx(&cfg, kernel, A, n, iterations, ctas, out);
 }

@@ -487,6 +487,13 @@ def test_power_iteration_in_one_launch_matches_its_operations_in_64_bits(batch, 
     torch.testing.assert_close(got.double(), want, rtol=1e-5, atol=0)
 
 
+@pytest.mark.parametrize("batch,n", [(37, 20), (38, 300), (75, 200), (150, 128), (149, 129), (300, 64), (75, 512), (1024, 5), (1025, 5), (1100, 64), (1, 1280),
+                                     (1, 1284), (2, 1284), (2, 1024), (2, 1025)])  # fmt: skip
+def test_power_iteration_of_many_and_of_few_matrices(batch, n, monkeypatch):
+    """Clusters of one to sixteen CTAs, and sizes on either side of where the library's operations are the faster."""
+    test_power_iteration_in_one_launch_matches_its_operations_in_64_bits(batch, n, 2, 1.0, monkeypatch)
+
+
 @pytest.mark.parametrize("block,single", [(1, 512), (512, 1), (3, 40), (40, 3), (30, 32), (600, 88), (88, 600), (0, 639), (638, 0)])
 def test_power_iteration_starts_from_the_first_of_equal_rows(block, single):
     """Rows (3, 4), (4, 3) and (5): norms of 5 that are exact, in blocks of eigenvalues 7 and 5 that the iteration does not leave."""
