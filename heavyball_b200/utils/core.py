@@ -539,10 +539,19 @@ def _own_pass(*ts: Tensor):
     return ops.load()
 
 
+def _turned_faster(x: Tensor) -> bool:
+    """Whether the kernel's blocks of 64 x 64 are filled well enough to beat the library's copy, us of the library / the kernel: 16 M elements as 32 x 32
+    66 / 32, as 24 x 24 41 / 49, as 16 x 4096 47 / 37, as 8 x 4096 44 / 61, as 4 x 4 (1 M) 4 / 68; with sides or a start that are no multiples of four,
+    read by element, 1 M as 130 x 130 6.3 / 6.3, 0.25 M 3.2 / 3.7, 4 M as 65 x 65 11 / 14.  The grid holds 65535 matrices of 65535 blocks' rows."""
+    if x.ndim != 3 or not 0 < x.shape[0] <= 65535 or x.shape[1] > 64 * 65535 or x.shape[2] >= 1 << 22:
+        return False
+    whole = x.shape[1] % 4 == 0 and x.shape[2] % 4 == 0 and x.storage_offset() % 4 == 0
+    return min(x.shape[1:]) >= (32 if whole else 128) and (whole or x.numel() >= 1 << 20)
+
+
 def _transposed(x: Tensor) -> Tensor:
     """``x.mT.contiguous()``."""
-    # (the kernel counts matrices, and 64 rows at a time, in dimensions of the grid that end at 65535)
-    ext = _own_pass(x) if x.ndim == 3 and 0 < x.shape[0] <= 65535 and x.shape[1] <= 64 * 65535 and x.shape[2] < 1 << 22 else None
+    ext = _own_pass(x) if _turned_faster(x) else None
     return x.mT.contiguous() if ext is None else ext.transposed(x)
 
 

@@ -337,6 +337,15 @@ def test_passes_over_matrices_have_the_bits_of_the_chains_they_replace(shape):
     assert torch.equal(dense[:, rows, cols], line) and torch.equal(dense, dense.triu())
 
 
+def test_transposes_on_either_side_of_the_rule():
+    from heavyball_b200.utils import core
+
+    for shape in [(65535, 4, 4), (3, 31, 4096), (3, 32, 4096), (2, 28, 28), (7, 32, 32), (2, 1000, 127), (16, 600, 129), (1, 129, 130), (64, 129, 130)]:
+        flat = torch.randn(shape[0] * shape[1] * shape[2] + 1, device="cuda")
+        for x in (flat[:-1].view(shape), flat[1:].view(shape)):
+            assert torch.equal(core._transposed(x), x.mT) and core._transposed(x).is_contiguous()
+
+
 @pytest.mark.parametrize("shape", [(1, 64 * 65535, 32), (1, 64 * 65535 + 1, 32), (1, (1 << 22) - 1, 33), (1, 32, (1 << 22) - 1)], ids=str)
 def test_transposes_of_the_longest_matrices(shape):
     from heavyball_b200.utils import core
