@@ -615,7 +615,9 @@ def _solve_leaf(b: Tensor, inv: Tensor, block: int, x: Tensor):
 
 def _scaled_matrices(x: Tensor, by: Tensor, divide: bool = False, in_place: bool = False) -> Tensor:
     """``x / by`` or ``x * by`` with one factor per leading index of ``x``."""
-    ext = _own_pass(x, by) if x.ndim >= 2 and by.numel() == x.shape[0] and 0 < x.shape[0] <= 65535 and x.numel() > 0 else None
+    # a block per matrix: from 256 elements on (65535 of them 37 us either way; of 10 the library's broadcast 4, blocks 36)
+    whole = x.ndim >= 2 and by.numel() == x.shape[0] and 0 < x.shape[0] <= 65535 and x.numel() >= 256 * x.shape[0]
+    ext = _own_pass(x, by) if whole else None
     if ext is not None:
         out = x if in_place else torch.empty_like(x)
         ext.scale_matrices(x, by, divide, out)
