@@ -844,16 +844,15 @@ at::Tensor power_iteration(const at::Tensor& a, int64_t iterations) {
   return out;
 }
 
-// x[b] / by[b] (divide) or x[b] * by[b]; x: contiguous fp32, first dimension the batch; out: like x, may be x.
-void scale_matrices(const at::Tensor& x, const at::Tensor& by, bool divide, const at::Tensor& out) {
-  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() >= 1 && x.is_contiguous() && x.size(0) >= 1 && x.size(0) <= 65535 && out.device() == x.device() &&
-                  out.scalar_type() == at::kFloat && out.is_contiguous() && out.sizes() == x.sizes(), "scale_matrices: contiguous fp32 CUDA tensors of one shape");
-  const at::MemOverlapStatus overlap = at::get_overlap_status(x, out);
-  TORCH_CHECK(overlap != at::MemOverlapStatus::Partial, "scale_matrices: in place or elsewhere");
-  TORCH_CHECK(by.device() == x.device() && by.scalar_type() == at::kFloat && by.is_contiguous() && by.numel() == x.size(0), "scale_matrices: one fp32 value per matrix");
+// x[b] *= by[b] in place; x: contiguous fp32, first dimension the batch.
+void scale_matrices_(const at::Tensor& x, const at::Tensor& by) {
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kFloat && x.dim() >= 1 && x.is_contiguous() && x.size(0) >= 1 && x.size(0) <= 65535,
+              "scale_matrices_: contiguous fp32 CUDA tensor");
+  TORCH_CHECK(by.device() == x.device() && by.scalar_type() == at::kFloat && by.is_contiguous() && by.numel() == x.size(0) &&
+                  at::get_overlap_status(x, by) == at::MemOverlapStatus::No, "scale_matrices_: one fp32 value per matrix");
   c10::cuda::CUDAGuard guard(x.device());
-  check(hb::launch_scale_matrices(x.data_ptr<float>(), by.data_ptr<float>(), out.data_ptr<float>(), (int)x.size(0), x.numel() / x.size(0), divide,
-                                  at::cuda::getCurrentCUDAStream()), "scale_matrices launch");
+  check(hb::launch_scale_matrices(x.data_ptr<float>(), by.data_ptr<float>(), (int)x.size(0), x.numel() / x.size(0), at::cuda::getCurrentCUDAStream()),
+        "scale_matrices launch");
 }
 
 // X = B T^-1 for 128 columns: b, x: fp32 [batch, rows, 128] with unit inner stride and rows on 16-byte boundaries, rows a multiple of 64; inv:
@@ -1083,7 +1082,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("sum_triu_diff_", &sum_triu_diff_);
   m.def("dampen", &dampen);
   m.def("power_iteration", &power_iteration);
-  m.def("scale_matrices", &scale_matrices);
+  m.def("scale_matrices_", &scale_matrices_);
   m.def("leaf_solve", &leaf_solve);
   m.def("triu_step_", &triu_step_);
   m.def("triu_pack", &triu_pack);

@@ -119,7 +119,7 @@ __global__ void __launch_bounds__(256) triu_step_kernel(const float* __restrict_
 }
 
 template <typename V>
-__global__ void __launch_bounds__(256) scale_matrices_kernel(const V* x, const float* __restrict__ by, V* out, int64_t count, bool divide) {
+__global__ void __launch_bounds__(256) scale_matrices_kernel(V* __restrict__ x, const float* __restrict__ by, int64_t count) {
   constexpr int kWide = sizeof(V) / sizeof(float);
   const int64_t base = blockIdx.y * count, step = (int64_t)gridDim.x * blockDim.x;
   const float s = by[blockIdx.y];
@@ -128,8 +128,8 @@ __global__ void __launch_bounds__(256) scale_matrices_kernel(const V* x, const f
     V v = x[base + i];
     float* p = (float*)&v;
 #pragma unroll
-    for (int e = 0; e < kWide; ++e) p[e] = divide ? div(p[e], s) : mul(p[e], s);
-    out[base + i] = v;
+    for (int e = 0; e < kWide; ++e) p[e] = mul(p[e], s);
+    x[base + i] = v;
   }
 }
 
@@ -174,13 +174,13 @@ cudaError_t launch_triu_step(const float* step, const float* ell, float* line, i
   return cudaGetLastError();
 }
 
-cudaError_t launch_scale_matrices(const float* x, const float* by, float* out, int batch, int64_t count, bool divide, cudaStream_t stream) {
+cudaError_t launch_scale_matrices(float* x, const float* by, int batch, int64_t count, cudaStream_t stream) {
   if (batch == 0 || count == 0) return cudaSuccess;
   if (batch > 65535) return cudaErrorInvalidValue;
-  if ((count & 3) == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0)
-    scale_matrices_kernel<<<dim3(blocks_for(count / 4), batch), 256, 0, stream>>>((const float4*)x, by, (float4*)out, count / 4, divide);
+  if ((count & 3) == 0 && ((uintptr_t)x & 15) == 0)
+    scale_matrices_kernel<<<dim3(blocks_for(count / 4), batch), 256, 0, stream>>>((float4*)x, by, count / 4);
   else
-    scale_matrices_kernel<<<dim3(blocks_for(count), batch), 256, 0, stream>>>(x, by, out, count, divide);
+    scale_matrices_kernel<<<dim3(blocks_for(count), batch), 256, 0, stream>>>(x, by, count);
   return cudaGetLastError();
 }
 

@@ -17,7 +17,7 @@ cudaError_t launch_dampen(const float* g, const float* v, float* out, int64_t co
 // line[b] -= triu(step[b]) / ell[b] * lr; step: [batch, n, n], line: row-major upper triangles [batch, n (n + 1) / 2]; batch <= 65535.
 cudaError_t launch_triu_step(const float* step, const float* ell, float* line, int batch, int n, float lr, cudaStream_t stream);
 
-// out[b][i] = x[b][i] / by[b] (divide) or x[b][i] * by[b] for i < count; out may be x; batch <= 65535.
-cudaError_t launch_scale_matrices(const float* x, const float* by, float* out, int batch, int64_t count, bool divide, cudaStream_t stream);
+// x[b][i] *= by[b] for i < count; batch <= 65535.
+cudaError_t launch_scale_matrices(float* x, const float* by, int batch, int64_t count, cudaStream_t stream);
 
 }  // namespace hb

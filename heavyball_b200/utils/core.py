@@ -613,21 +613,16 @@ def _solve_leaf(b: Tensor, inv: Tensor, block: int, x: Tensor):
     torch.bmm(b, inv[:, block, :d, :d], out=x)
 
 
-def _scaled_matrices(x: Tensor, by: Tensor, divide: bool = False, in_place: bool = False) -> Tensor:
-    """``x / by`` or ``x * by`` with one factor per leading index of ``x``."""
+def _scale_matrices_(x: Tensor, by: Tensor) -> None:
+    """``x *= by`` with one factor per leading index of ``x``."""
     # a block per matrix: from 256 elements on (65535 of them 37 us either way; of 10 the library's broadcast 4, blocks 36)
     whole = x.ndim >= 2 and by.numel() == x.shape[0] and 0 < x.shape[0] <= 65535 and x.numel() >= 256 * x.shape[0]
     ext = _own_pass(x, by) if whole else None
-    if ext is not None:
-        out = x if in_place else torch.empty_like(x)
-        ext.scale_matrices(x, by, divide, out)
-        if in_place:
-            torch.autograd.graph.increment_version(x)
-        return out
-    wide = by.view(-1, *([1] * (x.ndim - 1)))
-    if in_place:
-        return x.div_(wide) if divide else x.mul_(wide)
-    return x / wide if divide else x * wide
+    if ext is None:
+        x *= by.view(-1, *([1] * (x.ndim - 1)))
+        return
+    ext.scale_matrices_(x, by)
+    torch.autograd.graph.increment_version(x)
 
 
 def _solve_right_upper_into(q: Tensor, b: Tensor, x: Tensor, inv: Tensor, first_block: int, pairs: bool):
