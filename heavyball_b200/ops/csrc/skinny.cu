@@ -626,8 +626,10 @@ cudaError_t launch_triu_unpack(const void* line, void* dense, int elem_bytes, in
 
 // ------------------------------------------------------------------------------------------ around the eigenbasis refresh
 // Passes over n x k matrices that only memory bounds: a block turns a few rows in shared memory, so that both sides are read and written
-// in whole lines, 16 bytes per access where rows start on such boundaries (16 of 1024^2, the library's gather and scatter, element by element
-// through 64-bit indices, 54 and 78 us; this with 4 bytes per access 27 each, 11 of 2048^2 195).
+// in whole lines (16 of 1024^2, the library's gather and scatter, element by element through 64-bit indices, 54 and 78 us).  16 bytes per access
+// where rows start on such boundaries and are long enough to give the threads of a block a vector each, us there and back with 16 / 4 bytes:
+// 3000 of 16^2 14, 11 / 8, 9; 64 of 256^2 7.6, 7.8 / 6.5, 7.3; 64 of 512^2 30, 27 / 28, 31; 16 of 768^2 12, 13 / 13, 15; 16 of 1024^2 28, 26 / 32, 39;
+// 11 of 2048^2 94, 85 / 206, 202.  A thread's eight loads are of eight rows (through a flat index 16 of 1024^2 33 in the place of 28).
 template <typename V>  // float4 or float
 __global__ void __launch_bounds__(256) permute_columns_kernel(const float* __restrict__ x, const long long* __restrict__ order, float* __restrict__ out,
                                                              int n, int k, int rows, int inverse) {
@@ -639,8 +641,10 @@ __global__ void __launch_bounds__(256) permute_columns_kernel(const float* __res
   const V* from = (const V*)(x + base);
   V* to = (V*)(out + base);
   if (!inverse) {
-#pragma unroll 4
-    for (int i = threadIdx.x; i < count * vectors; i += blockDim.x) ((V*)turned)[i] = from[i];
+    for (int j = threadIdx.x; j < vectors; j += blockDim.x) {
+#pragma unroll 8
+      for (int r = 0; r < count; ++r) ((V*)turned)[r * vectors + j] = from[r * vectors + j];
+    }
     __syncthreads();
   }
   for (int j = threadIdx.x; j < vectors; j += blockDim.x) {
@@ -679,7 +683,7 @@ cudaError_t launch_permute_columns(const float* x, const long long* order, float
   if (batch == 0 || n == 0 || k == 0) return cudaSuccess;
   if (k > kMaxPermuted || batch > 65535) return cudaErrorInvalidValue;
   const int rows = kMaxPermuted / k < 8 ? kMaxPermuted / k : 8;  // 48 KB of shared memory at most
-  const bool vec = (k & 3) == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0;
+  const bool vec = k >= 768 && (k & 3) == 0 && (((uintptr_t)x | (uintptr_t)out) & 15) == 0;
   const auto kernel = vec ? permute_columns_kernel<float4> : permute_columns_kernel<float>;
   kernel<<<dim3((n + rows - 1) / rows, batch), 256, (size_t)rows * k * sizeof(float), stream>>>(x, order, out, n, k, rows, inverse);
   return cudaGetLastError();

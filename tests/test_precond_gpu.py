@@ -354,7 +354,7 @@ def test_transposes_of_the_longest_matrices(shape):
     assert torch.equal(core._transposed(x).view(torch.int32), x.view(torch.int32).mT)
 
 
-@pytest.mark.parametrize("n,k", [(1, 3), (7, 130), (64, 1024), (100, 2048), (5, 5000), (9, 12288)])
+@pytest.mark.parametrize("n,k", [(1, 3), (7, 130), (64, 1024), (100, 2048), (5, 5000), (9, 12288), (17, 764), (17, 768), (3, 769), (1, 772)])
 def test_columns_permuted_and_put_back(n, k):
     x = torch.randn(3, n, k, device="cuda", generator=torch.Generator("cuda").manual_seed(k))
     order = torch.stack([torch.randperm(k, device="cuda") for _ in range(3)])
