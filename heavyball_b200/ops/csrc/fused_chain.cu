@@ -410,6 +410,9 @@ struct ChainKind {
   // Launches without codec state draw the bits of 16-bit parameters early too (64 M elements, Adam into bf16: 254 -> 235 us; a parked update
   // into bf16, four vectors: 111 -> 91; into error-corrected parameters, where four vectors no longer fit: 159 -> 166, with two vectors 167 -> 145).
   static constexpr bool ecc = DTS == kBF16E8;
+  // With the rule left open and an error-corrected parameter beside the states, bits that wait for their use cost more than the waits they fill (one
+  // state, 33.5 M elements: drawn at use 181 us, early 190; two 243 to 247, early 239 to 249).
+  static constexpr bool s_draws = ecc && (RULE != kAnyRule || DTP != kBF16E8);
   static constexpr bool p_draws = (DTP == kBF16E8 || DTP == kBF16) && !ecc && OUT == kOutParam;
   // Otherwise a thread should have about 128 bytes on their way: two vectors of Adam's four arrays, four where a launch reads
   // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 202 us, of which the
@@ -555,7 +558,7 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
 #pragma unroll
       for (int v = 0; v < kBatch; ++v) pin(p_rnd[v]);
     }
-    if constexpr (K::ecc) {
+    if constexpr (K::s_draws) {
 #pragma unroll
       for (int v = 0; v < kBatch; ++v) rnd[v] = draw_states(K::mars(P), K::n_state(P), rng, i0 + v * (kThreads * 4), (uint32_t)t);
     }
@@ -579,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
           x.v[k] = x.v[k] * (1.0f - P.mars_a) + before.v[k] * P.mars_a;
           grad.v[k] = x.v[k];
         }
-        store_values<K::dt_s>(mm, mme, i, nv, vec_ok, raw, rnd[v].mars);
+        store_values<K::dt_s>(mm, mme, i, nv, vec_ok, raw, K::s_draws ? rnd[v].mars : draw(K::dt_s, rng, ctr, ctr_hi ^ 0x40000000u, (uint32_t)t, 4u));
       }
       F4 out = x;
       if (K::state) {
@@ -587,8 +590,8 @@ __global__ void __launch_bounds__(kThreads, K::min_blocks) plain_chain_kernel(co
         if (m0 != nullptr) a = decode_raw<K::dt_s>(s0[v]);
         if (!K::one_state && m1 != nullptr) b = decode_raw<K::dt_s>(s1[v]);
         out = K::apply(P, x, a, b);
-        if (K::n_state(P) >= 1) store_values<K::dt_s>(m0, m0e, i, nv, vec_ok, a, rnd[v].s0);
-        if (K::n_state(P) >= 2) store_values<K::dt_s>(m1, m1e, i, nv, vec_ok, b, rnd[v].s1);
+        if (K::n_state(P) >= 1) store_values<K::dt_s>(m0, m0e, i, nv, vec_ok, a, K::s_draws ? rnd[v].s0 : draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 0u));
+        if (K::n_state(P) >= 2) store_values<K::dt_s>(m1, m1e, i, nv, vec_ok, b, K::s_draws ? rnd[v].s1 : draw(K::dt_s, rng, ctr, ctr_hi, (uint32_t)t, 1u));
       }
       if (K::count) {  // phase one of caution: mask, count, park the masked update
 #pragma unroll
