@@ -388,9 +388,9 @@ __device__ __forceinline__ F4 apply_rule(const ChainParams& P, const F4& u, F4& 
   return out;
 }
 
-// RULE: one moment rule, with or without MARS, known at compile time (kAnyRule: whatever the launch asks for).
-constexpr int kAnyRule = -1;
-constexpr int rule_states(int rule) { return rule == kAdam ? 2 : 1; }
+// RULE: one moment rule, with or without MARS, known at compile time (kAnyRule: whatever the launch asks for; kAnyOfTwo: any rule with two states).
+constexpr int kAnyRule = -1, kAnyOfTwo = -2;
+constexpr int rule_states(int rule) { return rule == kAdam || rule == kAnyOfTwo ? 2 : 1; }
 
 template <int DTP, int DTG, int DTU, int DTS, int OUT, int UIN, bool COUNT, int RULE = kAnyRule, bool MARS = false>
 struct ChainKind {
@@ -422,17 +422,18 @@ struct ChainKind {
   static constexpr bool one_state = RULE != kAnyRule && rule_n == 1;
   static constexpr bool ahead = ecc && RULE != kAnyRule;  // the next vector is fetched ahead
   static constexpr int min_blocks = ahead ? (one_state ? 4 : 3) : state && !(ecc && !count) ? 3 : 4;
-  // Adam's four fp32 arrays at two vectors are in flight either way (166 us with the test per load on 39.5 M elements, 169 with one for all)
-  static constexpr bool either = state && reads_p && DTS == kF32 && DTG == kF32;
+  // Adam's four fp32 arrays at two vectors are in flight either way (166 us with the test per load on 39.5 M elements, 169 with one for all; into an
+  // update, two states, 33.5 M elements: 126.5 / 129.7), one state's are not (87 us with one test for all, 93 per load)
+  static constexpr bool either = state && (reads_p || RULE == kAnyOfTwo) && DTS == kF32 && DTG == kF32;
   static bool takes(const ChainParams& P, bool counting) {
     return counting == COUNT && P.out_mode == OUT && P.u_is_input == UIN && (!reads_p || P.dt_p == DTP) &&
            (!reads_g || P.dt_g == DTG) && ((OUT == kOutParam && !u_in) || P.dt_u == DTU) && P.dt_s == DTS &&
-           (RULE == kAnyRule || (P.algo == RULE && P.n_state == rule_states(RULE) && (P.mars != 0) == MARS));
+           (RULE == kAnyRule || ((P.algo == RULE || RULE == kAnyOfTwo) && P.n_state == rule_states(RULE) && (P.mars != 0) == MARS));
   }
   static __device__ __forceinline__ bool mars(const ChainParams& P) { return RULE == kAnyRule ? P.mars != 0 : MARS; }
   static __device__ __forceinline__ int n_state(const ChainParams& P) { return RULE == kAnyRule ? P.n_state : rule_n; }
   static __device__ __forceinline__ F4 apply(const ChainParams& P, const F4& u, F4& s0, F4& s1) {
-    if constexpr (RULE == kAnyRule) {
+    if constexpr (RULE == kAnyRule || RULE == kAnyOfTwo) {
       return apply_rule(P, u, s0, s1);
     } else {
       F4 out;
@@ -720,6 +721,8 @@ using Kinds = KindList<
     ChainKind<kNone, kF32, kF32, kF32, kOutUpdate, 0, false, kNesterovEma>,
     ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, true, kAdam, false>,
     ChainKind<kNone, kF32, kF32, kBF16E8, kOutUpdate, 0, true, kAdam, true>,
+    // any rule with two states
+    ChainKind<kNone, kF32, kF32, kF32, kOutUpdate, 0, false, kAnyOfTwo>,
     // any rule
     ChainKind<kF32, kF32, kNone, kF32, kOutParam, 0, false>,       // first-order rules on fp32 parameters
     ChainKind<kBF16, kBF16, kNone, kF32, kOutParam, 0, false>,     // ... on bf16 parameters

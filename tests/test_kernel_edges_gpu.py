@@ -92,7 +92,7 @@ def test_rules_known_at_compile_time_match_the_general_kernel(algo, mars, grad, 
                 torch.testing.assert_close(a, b, rtol=2**-14, atol=1e-30)
 
 
-@pytest.mark.parametrize("kind", ["momentum", "momentum-ecc", "caution", "update-ecc", "adam", "adam-bf16"])
+@pytest.mark.parametrize("kind", ["momentum", "momentum-ecc", "caution", "update-ecc", "adam", "adam-bf16", "adam-update"])
 @pytest.mark.parametrize("sizes", [(1, 3, 4, 5), (1023, 1024, 1025, 4092, 4095), (4096, 4097, 4100, 8188, 8192), (2_000_003, 2_500_000)], ids=str)
 def test_whole_and_element_loads_read_the_same_values(sizes, kind):
     """A batch of vectors is loaded whole where all its elements are there and the buffers start on a 16-byte boundary, else
@@ -121,6 +121,9 @@ def test_whole_and_element_loads_read_the_same_values(sizes, kind):
             lists = {"p": made(torch.bfloat16), "pe": made(torch.int8), "u": made(torch.float32)}
             cfg = dict(algo=ops.IDENTITY, u_is_input=1, out_mode=ops.OUT_PARAM, dt_u=ops.F32, dt_p=ops.BF16E8,
                        dt_g=ops.NONE, dt_s=ops.NONE, lr=1e-2, wd=0.1)  # fmt: skip
+        elif kind == "adam-update":
+            lists = {"g": made(torch.float32), "s0": made(torch.float32), "s1": made(torch.float32, True), "u": made(torch.float32)}
+            cfg = dict(algo=ops.ADAM, n_state=2, b1=0.9, b2=0.99, eps=1e-8, out_mode=ops.OUT_UPDATE, dt_u=ops.F32, dt_p=ops.NONE, dt_g=ops.F32, dt_s=ops.F32)
         else:
             dtype, dt = (torch.float32, ops.F32) if kind == "adam" else (torch.bfloat16, ops.BF16)
             lists = {"p": made(dtype), "g": made(dtype), "s0": made(torch.float32), "s1": made(torch.float32, True)}
