@@ -47,8 +47,10 @@ def test_rules_known_at_compile_time_match_the_general_kernel(algo, mars, grad, 
     """Error-corrected state through the instances with the rule compiled in (next vector fetched ahead, random bits drawn before the values
     arrive) and through the general kernel, which a gradient given as the sum over one source selects, over aligned and misaligned starts,
     remainders, zeros and values whose residuals take the slow codec.  The compiler may contract a product and a sum in one of the two:
-    2^-24 of a value, which is 2^-8 of a residual's unit (2^-16 of the value), so up to 2^-8 of the residuals may come out one unit apart
-    (255 apart where the rounded value goes the other way); fp32 results and their inputs differ by a few such roundings and units."""
+    2^-24 of a value, which is 2^-8 of a residual's unit (half a unit in the last place of bf16 over 127: 2^-15 of the value), so up to 2^-8 of the
+    residuals may come out one unit apart (255 apart where the rounded value goes the other way).  After one launch, whose inputs are the same, no
+    pair may stand for a value further off than two units and a few roundings of the terms it was summed from; fp32 results of the second
+    differ by a few such roundings and units."""
 
     def run(extra):
         gen, dtypes = torch.Generator(DEV).manual_seed(3), {"f32": torch.float32, "bf16": torch.bfloat16, "ecc": torch.bfloat16}
@@ -79,20 +81,39 @@ def test_rules_known_at_compile_time_match_the_general_kernel(algo, mars, grad, 
         masked = torch.zeros(len(sizes), dtype=torch.int32, device=DEV)
         if count:
             cfg.update(count_caution=1, masked=masked)
+        seen = [{k: [t.clone() for t in v] for k, v in lists.items()}]
         for seed in (5, 6):
             ops.fused_chain(**lists, **cfg, **extra, seed=seed)
-        return {**lists, "masked": [masked]}
+            seen.append({k: [t.clone() for t in v] for k, v in {**lists, "masked": [masked]}.items()})
+        return seen
 
-    compiled, general = run({}), run({"g_delta": [0], "g_scale": 1.0})
-    for name, tensors in compiled.items():
-        for i, (a, b) in enumerate(zip(tensors, general[name])):
+    def value(of, name, i):
+        x = of[name][i]
+        return (utils._ULPState(of[name + "e"][i], 127).decode(x) if name + "e" in of else x).double()
+
+    (before, first, last), (_, first_general, last_general) = run({}), run({"g_delta": [0], "g_scale": 1.0})
+    for i in range(len(sizes)):
+        g = value(before, "g", i).abs() + (value(before, "mars", i).abs() if mars else 0)
+        terms = {"mars": 0 * g, "s0": value(before, "s0", i).abs() + g}
+        if algo == ops.ADAM:
+            terms["s1"] = value(before, "s1", i) + g * g
+            if param is not None:
+                terms["p"] = value(before, "p", i).abs() + 1e-2 * terms["s0"] / value(first, "s1", i).sqrt().clamp(min=1e-8)
+        for name, scale in terms.items():
+            if name in first:
+                a, b = value(first, name, i), value(first_general, name, i)
+                off = (a - b).abs() - (2.0**-14 * torch.maximum(a.abs(), b.abs()) + 2.0**-21 * scale + 2.0**-133)
+                assert bool((off <= 0).all()), (name, i, int(off.argmax()), float(off.max()))
+    for name, tensors in last.items():
+        for i, (a, b) in enumerate(zip(tensors, last_general[name])):
             if a.dtype in (torch.int8, torch.bfloat16):
                 assert int((a != b).sum()) <= a.numel() >> 8, (name, i, int((a != b).sum()))
             else:
                 torch.testing.assert_close(a, b, rtol=2**-14, atol=1e-30)
 
 
-@pytest.mark.parametrize("kind", ["momentum", "momentum-ecc", "caution", "update-ecc", "adam", "adam-bf16", "adam-update"])
+@pytest.mark.parametrize("kind", ["momentum", "momentum-ecc", "caution", "update-ecc", "adam", "adam-bf16", "adam-update",
+                                  "adam-ecc", "adam-ecc-param", "adam-ecc-count", "adam-ecc-count-mars"])  # fmt: skip
 @pytest.mark.parametrize("sizes", [(1, 3, 4, 5), (1023, 1024, 1025, 4092, 4095), (4096, 4097, 4100, 8188, 8192), (2_000_003, 2_500_000)], ids=str)
 def test_whole_and_element_loads_read_the_same_values(sizes, kind):
     """A batch of vectors is loaded whole where all its elements are there and the buffers start on a 16-byte boundary, else
@@ -124,6 +145,16 @@ def test_whole_and_element_loads_read_the_same_values(sizes, kind):
         elif kind == "adam-update":
             lists = {"g": made(torch.float32), "s0": made(torch.float32), "s1": made(torch.float32, True), "u": made(torch.float32)}
             cfg = dict(algo=ops.ADAM, n_state=2, b1=0.9, b2=0.99, eps=1e-8, out_mode=ops.OUT_UPDATE, dt_u=ops.F32, dt_p=ops.NONE, dt_g=ops.F32, dt_s=ops.F32)
+        elif kind.startswith("adam-ecc"):
+            pe, count = kind.endswith("param"), "count" in kind
+            g, made8 = made(torch.bfloat16 if pe else torch.float32), lambda: made(torch.int8)
+            lists = {"g": g, "s0": made(torch.bfloat16), "s0e": made8(), "s1": made(torch.bfloat16, True), "s1e": made8()}
+            if kind.endswith("mars"):
+                lists.update(mars=made(torch.bfloat16), marse=made8())
+            lists.update({"u": made(torch.float32)} if count else {"p": made(g[0].dtype), **({"pe": made8()} if pe else {})})
+            cfg = dict(algo=ops.ADAM, n_state=2, b1=0.9, b2=0.99, eps=1e-8, mars_a=-0.0023, dt_g=ops.BF16 if pe else ops.F32, dt_s=ops.BF16E8)
+            cfg.update(dict(out_mode=ops.OUT_UPDATE, dt_u=ops.F32, dt_p=ops.NONE, count_caution=1, masked=masked) if count else
+                       dict(out_mode=ops.OUT_PARAM, dt_p=ops.BF16E8 if pe else ops.F32, lr=1e-2, wd=0.1))  # fmt: skip
         else:
             dtype, dt = (torch.float32, ops.F32) if kind == "adam" else (torch.bfloat16, ops.BF16)
             lists = {"p": made(dtype), "g": made(dtype), "s0": made(torch.float32), "s1": made(torch.float32, True)}
