@@ -4,8 +4,8 @@
 // product a matrix-vector kernel, a norm, a clamp and a division.  Here a cluster of CTAs takes a matrix from beginning to end.  A CTA owns a
 // share of the rows, which it reads once for the norms and twice a step (from the L2: 4 MB at 1024), a warp four rows at a time; every CTA keeps
 // the whole vectors in shared memory, and each product's entries are stored into all of them.  What is left of each step is the reading and one
-// cluster barrier per product.  A is divided by its largest row norm on the way, entry by entry: what may not leave fp32 are the squares of its
-// entries and their sums along a row.
+// cluster barrier per product.  A is scaled by a power of two near its largest row norm on the way, entry by entry: what may not leave fp32 are the
+// squares of its entries and their sums along a row.
 // Two factors of 8 of 1024^2, two iterations each, in the graph of a fit: 245 us of the library's kernels, 2 x 54 here.
 #include "power_iteration.h"
 
@@ -39,11 +39,16 @@ __device__ __forceinline__ float sqrt_full(float a) {
   asm("sqrt.rn.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
 }
-__device__ __forceinline__ float inverse_full(float a) {
+__device__ __forceinline__ float div_full(float a, float b) {
   float r;
-  asm("rcp.rn.f32 %0, %1;" : "=f"(r) : "f"(a));
+  asm("div.rn.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
   return r;
 }
+
+// A and the vectors are scaled by powers of two, which rounds nothing; what is left of the vector's length is divided out at the end.  Of a value
+// that is not finite: NaN.
+__device__ __forceinline__ float power_of_two(float v) { return v < 1.7e38f ? __uint_as_float(__float_as_uint(v) & 0x7F800000u) : v - v; }
+__device__ __forceinline__ float inverse_power(float p) { return p > 0.0f ? __uint_as_float((254u << 23) - __float_as_uint(p)) : p; }
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
@@ -150,7 +155,8 @@ __global__ void __launch_bounds__(kPowerThreads) power_iteration_kernel(const fl
       norm = best_norm[w];
       at = best_row[w];
     }
-  const float top = norm < 1.17549435e-38f ? 1.17549435e-38f : norm, by = inverse_full(top);
+  const float top = norm < 1.17549435e-38f ? 1.17549435e-38f : norm;
+  const float unit = power_of_two(top), by = inverse_power(unit);
   for (int k = threadIdx.x; k < n; k += kPowerThreads) x[k] = mul_full(A[(int64_t)at * n + k], by);
   cluster_sync();  // x is complete, and nobody reads the norms any more
 
@@ -158,21 +164,27 @@ __global__ void __launch_bounds__(kPowerThreads) power_iteration_kernel(const fl
     over_rows<kWide>(A, n, first, last, [&](float s, float a, int k) { return fma_full(mul_full(a, by), v[k], s); }, [&](int r, float s, int l) { store_everywhere(to + r, s, l, ctas); });
     cluster_sync();
   };
+  const auto times_itself = [&](const float* v) {
+    float s = 0.0f;
+    for (int k = threadIdx.x; k < n; k += kPowerThreads) s = fma_full(x[k], v[k], s);
+    return block_sum(s, scratch);
+  };
+  bool vanished = false;  // a vector shorter than 1e-12 counts as one of that length
   for (int it = 0; it < iterations; ++it) {
     times(x, ax);
     times(ax, aax);
     float s = 0.0f;
     for (int k = threadIdx.x; k < n; k += kPowerThreads) s = fma_full(aax[k], aax[k], s);
-    const float length = sqrt_full(block_sum(s, scratch)), inv = inverse_full(length < 1e-12f ? 1e-12f : length);
+    const float length = sqrt_full(block_sum(s, scratch));
+    vanished = length < 1e-12f;
+    const float inv = vanished ? 1e12f : inverse_power(power_of_two(length));
     for (int k = threadIdx.x; k < n; k += kPowerThreads) x[k] = mul_full(aax[k], inv);
     __syncthreads();
   }
   times(x, ax);
   times(ax, aax);
-  float s = 0.0f;
-  for (int k = threadIdx.x; k < n; k += kPowerThreads) s = fma_full(x[k], aax[k], s);
-  s = block_sum(s, scratch);
-  if (rank == 0 && threadIdx.x == 0) out[blockIdx.x / ctas] = mul_full(sqrt_full(s), top);
+  const float product = times_itself(aax), square = times_itself(x);
+  if (rank == 0 && threadIdx.x == 0) out[blockIdx.x / ctas] = mul_full(sqrt_full(vanished || square == 0.0f ? product : div_full(product, square)), unit);
 }
 
 }  // namespace
