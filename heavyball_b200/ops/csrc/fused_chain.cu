@@ -405,8 +405,12 @@ struct ChainKind {
   // vector is fetched ahead of this one's arithmetic (231; three blocks, at two 248).  Without MARS 228 -> 162 us; Adam into fp32
   // parameters 195 -> 169, into error-corrected ones 245 -> 222; exponential average of 25 M elements (one state: four blocks) 122 -> 75;
   // momentum with MARS of a Llama-3-8B layer, at the clock that the products around it leave, 1.71 -> 1.42 ms.
-  // The rules that steps use most are compiled in; of fp32 state only Nesterov's momentum, which spills without that (85 M elements: 228 -> 202 us;
-  // Adam 165.6 -> 165.4, not worth a kernel).
+  // Compiled in are the rules whose steps have been measured as workloads: Adam with codec state into fp32 and error-corrected parameters and under
+  // caution, PSGD's exponential average, Muon's Nesterov average from fp32 gradients and, with MARS, from bf16 ones; of fp32 state only that
+  // average, which spills without (85 M elements: 228 -> 202 us; Adam 165.6 -> 165.4, not worth a kernel).  An instance is two kernels of the same
+  // length again, so others come in by measurement.  What the rest pays, 33.5 M elements, before these changes / with the rule left open: heavy-ball
+  // momentum of fp32 gradients 156 / 154 us, of bf16 ones 129 / 128, with MARS 229 / 207; into fp32 parameters 136 / 135; LaProp 197 / 183, under
+  // caution 233 / 214.
   // Launches without codec state draw the bits of 16-bit parameters early too (64 M elements, Adam into bf16: 254 -> 235 us; a parked update
   // into bf16, four vectors: 111 -> 91; into error-corrected parameters, where four vectors no longer fit: 159 -> 166, with two vectors 167 -> 145).
   static constexpr bool ecc = DTS == kBF16E8;
@@ -415,8 +419,8 @@ struct ChainKind {
   static constexpr bool s_draws = ecc && (RULE != kAnyRule || DTP != kBF16E8);
   static constexpr bool p_draws = (DTP == kBF16E8 || DTP == kBF16) && !ecc && OUT == kOutParam;
   // Otherwise a thread should have about 128 bytes on their way: two vectors of Adam's four arrays, four where a launch reads
-  // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written: 202 us, of which the
-  // bytes take 207 at 6.54 TB/s).
+  // two arrays (momentum of GPT-2-small's fp32 matrices, 85M elements, two arrays read and two written, 1.36 GB:
+  // 202 us, the rate of a copy).
   static constexpr int batch = ecc ? 1 : (DTP == kBF16E8 && !state) ? 2 : (state && (reads_p || count) ? 2 : 4);
   static constexpr int rule_n = rule_states(RULE);
   static constexpr bool one_state = RULE != kAnyRule && rule_n == 1;

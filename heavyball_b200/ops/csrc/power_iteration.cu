@@ -6,7 +6,7 @@
 // the whole vectors in shared memory, and each product's entries are stored into all of them.  What is left of each step is the reading and one
 // cluster barrier per product.  A is scaled by a power of two near its largest row norm on the way, entry by entry: what may not leave fp32 are the
 // squares of its entries and their sums along a row.
-// Two factors of 8 of 1024^2, two iterations each, in the graph of a fit: 245 us of the library's kernels, 2 x 54 here.
+// Two factors of 8 of 1024^2, two iterations each, in the graph of a fit: 245 us of the library's kernels, 2 x 51 here.
 #include "power_iteration.h"
 
 #include "per_device.h"
