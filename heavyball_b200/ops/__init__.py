@@ -309,12 +309,12 @@ def tf32_gemm(a2: torch.Tensor, b2: torch.Tensor, K: int, *, mode: int = EPI_STO
 
 
 def chol_qr_round(gram: torch.Tensor, a: torch.Tensor, info: torch.Tensor, want_trans: bool = True):
-    """One round of Cholesky QR: ``X = a R^-1`` with ``R^T R = gram`` (both overwritten) on the split-tf32 products.  Contiguous fp32
+    """One round of Cholesky QR: ``a <- a R^-1`` with ``R^T R = gram`` (overwritten, too) on the split-tf32 products.  Contiguous fp32
     ``a``: ``[batch, n, k]``, ``n`` a multiple of 64 and ``k`` of 128; ``info``: int32 ``[batch]``, incremented per 128-wide leaf with a bad pivot.
-    Returns ``(X, operand)``; the latter is :func:`tf32_split` of ``X`` with its columns as rows (``None`` unless ``want_trans``)."""
-    x, trans, launches = load().chol_qr_round(gram, a, want_trans, info, _status(a.device))
+    Returns :func:`tf32_split` of the new ``a`` with its columns as rows (``None`` unless ``want_trans``)."""
+    trans, launches = load().chol_qr_round(gram, a, want_trans, info, _status(a.device))
     launch_counter.count += launches
-    return x, trans
+    return trans
 
 
 class Split16:

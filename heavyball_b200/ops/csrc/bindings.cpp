@@ -765,10 +765,10 @@ void chol_inv_leaf(const at::Tensor& g, at::Tensor& r, at::Tensor& inv, int64_t 
                                  info.data_ptr<int>(), at::cuda::getCurrentCUDAStream()), "chol_inv_leaf launch");
 }
 
-// One round of Cholesky QR (chol_qr.h): X = A R^-1 with R^T R = gram; both are overwritten.  Contiguous fp32, a: [batch, n, k], n a multiple of
-// 64, k of 128; info: int32 [batch], incremented per leaf with a bad pivot.  Returns X, the split-tf32 operand of X^T (when asked) and the number
-// of launches.
-std::tuple<at::Tensor, OptT, int> chol_qr_round(const at::Tensor& gram, const at::Tensor& a, bool want_trans, const at::Tensor& info,
+// One round of Cholesky QR (chol_qr.h): a <- a R^-1 with R^T R = gram, which is overwritten.  Contiguous fp32, a: [batch, n, k], n a multiple of
+// 64, k of 128; info: int32 [batch], incremented per leaf with a bad pivot.  Returns the split-tf32 operand of the new a^T (when asked) and the
+// number of launches.
+std::tuple<OptT, int> chol_qr_round(const at::Tensor& gram, const at::Tensor& a, bool want_trans, const at::Tensor& info,
                                                 const at::Tensor& status) {
   for (const at::Tensor* t : {&gram, &a})
     TORCH_CHECK(t->is_cuda() && t->device() == a.device() && t->scalar_type() == at::kFloat && t->dim() == 3 && t->is_contiguous() && aligned16(t->data_ptr()),
@@ -780,19 +780,20 @@ std::tuple<at::Tensor, OptT, int> chol_qr_round(const at::Tensor& gram, const at
   TORCH_CHECK(info.device() == a.device() && info.scalar_type() == at::kInt && info.is_contiguous() && info.numel() == batch, "chol_qr_round: info must be int32 [batch]");
   c10::cuda::CUDAGuard guard(a.device());
   const auto options = a.options().memory_format(at::MemoryFormat::Contiguous);
-  const at::Tensor x = at::empty({batch, n, k}, options), x_same = at::empty({batch, n, 2 * k}, options), l = at::empty({batch, k, 2 * k}, options);
+  const at::Tensor x_same = at::empty({batch, n, 2 * k}, options), l = at::empty({batch, k, 2 * k}, options);
   const at::Tensor inv = at::empty({batch, k / hb::kQrBlock, hb::kQrBlock, hb::kQrBlock}, options);
   OptT trans;
   if (want_trans) trans = at::empty({batch, k, 2 * n}, options);
   int launches = 0;
-  check(hb::launch_chol_qr_round({gram.data_ptr<float>(), a.data_ptr<float>(), x.data_ptr<float>(), want_trans ? trans->data_ptr<float>() : nullptr, l.data_ptr<float>(),
-                                  inv.data_ptr<float>(), x_same.data_ptr<float>(), (int)n, (int)k, (int)batch, info.data_ptr<int>(), status.data_ptr<int>()},
-                                 &launches, at::cuda::getCurrentCUDAStream()), "chol_qr_round");
-  return {x, trans, launches};
+  const hb::QrRound round{gram.data_ptr<float>(), a.data_ptr<float>(), want_trans ? trans->data_ptr<float>() : nullptr, l.data_ptr<float>(),
+                          inv.data_ptr<float>(), x_same.data_ptr<float>(), (int)n, (int)k, (int)batch, info.data_ptr<int>(), status.data_ptr<int>()};
+  check(hb::launch_chol_qr_round(round, &launches, at::cuda::getCurrentCUDAStream()), "chol_qr_round");
+  return {trans, launches};
 }
 
 // (x / norm, split-tf32 operand of its transpose) for contiguous fp32 x: [batch, n, k] and norm: [batch, 1, k]; n a multiple of 64, k of 128.
-std::tuple<at::Tensor, at::Tensor> qr_unit_columns(const at::Tensor& x, const at::Tensor& norm) {
+// `in_place`: x itself is divided.
+std::tuple<at::Tensor, at::Tensor> qr_unit_columns(const at::Tensor& x, const at::Tensor& norm, bool in_place) {
   for (const at::Tensor* t : {&x, &norm})
     TORCH_CHECK(t->is_cuda() && t->device() == x.device() && t->scalar_type() == at::kFloat && t->dim() == 3 && t->is_contiguous() && aligned16(t->data_ptr()),
                 "qr_unit_columns: contiguous fp32 CUDA tensors");
@@ -801,7 +802,7 @@ std::tuple<at::Tensor, at::Tensor> qr_unit_columns(const at::Tensor& x, const at
               "qr_unit_columns: x of n x k, n a multiple of 64 and k of 128, and one norm per column");
   c10::cuda::CUDAGuard guard(x.device());
   const auto options = x.options().memory_format(at::MemoryFormat::Contiguous);
-  const at::Tensor a = at::empty({batch, n, k}, options), trans = at::empty({batch, k, 2 * n}, options);
+  const at::Tensor a = in_place ? x : at::empty({batch, n, k}, options), trans = at::empty({batch, k, 2 * n}, options);
   check(hb::launch_qr_unit_columns(x.data_ptr<float>(), norm.data_ptr<float>(), a.data_ptr<float>(), trans.data_ptr<float>(), (int)batch, (int)n, (int)k,
                                    at::cuda::getCurrentCUDAStream()), "qr_unit_columns launch");
   return {a, trans};

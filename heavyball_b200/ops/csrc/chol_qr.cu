@@ -135,8 +135,8 @@ __global__ void __launch_bounds__(kLeafSolveThreads, 2) qr_leaf_solve_kernel(con
 
 // 64 x 64 values per block: divided by their column's norm (in full, subnormal values kept), stored, and turned through shared memory into rows of
 // the operand.  One pass in the place of a division (138 us for 11 of 2048^2, the library's broadcast along rows) and an operand pass (86).
-__global__ void __launch_bounds__(256) qr_unit_columns_kernel(const float* __restrict__ X, const float* __restrict__ norm, float* __restrict__ A,
-                                                             float* __restrict__ trans, int n, int k) {
+__global__ void __launch_bounds__(256) qr_unit_columns_kernel(const float* X, const float* __restrict__ norm, float* A, float* __restrict__ trans, int n,
+                                                             int k) {
   __shared__ float tile[64][65];
   const int64_t b = blockIdx.z;
   const int c0 = blockIdx.x * 64, r0 = blockIdx.y * 64, q = (threadIdx.x & 15) * 4, line = threadIdx.x >> 4;
@@ -232,7 +232,7 @@ struct Round {
       } else {
         S.src = Q.A + lo;
         S.stride = (int64_t)Q.n * Q.k;
-        S.out = Q.X + lo;
+        S.out = Q.A + lo;  // in the place of B, whose rows a block of threads has read when it writes them
         S.ld_out = Q.k;
         S.stride_out = (int64_t)Q.n * Q.k;
         if (hi < Q.k) {  // (nothing to the right of the last block: never an operand)

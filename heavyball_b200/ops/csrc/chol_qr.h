@@ -29,17 +29,17 @@ struct QrLeafSolve {
 };
 cudaError_t launch_qr_leaf_solve(const QrLeafSolve& S, int rows, int batch, cudaStream_t stream);
 
-// A[b][i][j] = X[b][i][j] / norm[b][j]; A_trans: [batch, k, 2 n], the split-tf32 operand of A^T.  X, A: contiguous [batch, n, k], n a multiple of
-// 64, k of 128.
+// A[b][i][j] = X[b][i][j] / norm[b][j]; A_trans: [batch, k, 2 n], the split-tf32 operand of A^T.  X, A (may be X): contiguous [batch, n, k], n a
+// multiple of 64, k of 128.
 cudaError_t launch_qr_unit_columns(const float* X, const float* norm, float* A, float* A_trans, int batch, int n, int k, cudaStream_t stream);
 
-// G: [batch, k, k] symmetric positive definite, overwritten; A: [batch, n, k], overwritten; contiguous, n % 64 == 0, k % 128 == 0.
-//   X       : [batch, n, k]  <- A R^-1
+// G: [batch, k, k] symmetric positive definite, overwritten; A: [batch, n, k]; contiguous, n % 64 == 0, k % 128 == 0.
+//   A       : <- X = A R^-1
 //   X_trans : [batch, k, 2 n] <- the split-tf32 operand of X^T (null: not wanted)
 // Workspaces: L [batch, k, 2 k] (the split rows of R^T below its diagonal blocks), inv [batch, k / 128, 128, 128], X_same [batch, n, 2 k].
 // info[b] is incremented per leaf with a bad pivot.  *launches += kernels issued.
 struct QrRound {
-  float *G, *A, *X, *X_trans, *L, *inv, *X_same;
+  float *G, *A, *X_trans, *L, *inv, *X_same;
   int n, k, batch;
   int* info;
   int* status;

@@ -305,26 +305,29 @@ def _whole_blocks(a: Tensor) -> bool:
 
 
 def _cholesky_qr2_blocks(a: Tensor, bad: Tensor, info: Tensor, shifted_rounds: int) -> Tensor:
-    """The rounds of :func:`_cholesky_qr2` with the same products in the same order (same bits) by ``ops.chol_qr_round``."""
+    """The rounds of :func:`_cholesky_qr2` with the same products in the same order (same bits) by ``ops.chol_qr_round``.  At its height a round
+    holds the matrix, its Gram matrix and three split operands: 32 bytes per element of a square one (block by block: 24)."""
     from .. import ops
 
     n, k = a.shape[-2:]
 
-    def unit_columns(x):  # and the operand of the transpose
+    def unit_columns(x, in_place):  # and the operand of the transpose
         ops.launch_counter.count += 1
-        return ops.load().qr_unit_columns(x, x.norm(dim=-2, keepdim=True).clamp_(min=torch.finfo(x.dtype).tiny))
+        return ops.load().qr_unit_columns(x, x.norm(dim=-2, keepdim=True).clamp_(min=torch.finfo(x.dtype).tiny), in_place)
 
     gram = torch.empty(a.shape[0], k, k, device=a.device, dtype=a.dtype)
     # rows are read 16 bytes at a time: a view that begins elsewhere in its buffer is copied
-    a, operand = unit_columns(a if a.data_ptr() % 16 == 0 else a.clone())
+    aligned = a.data_ptr() % 16 == 0
+    a, operand = unit_columns(a if aligned else a.clone(), not aligned)
     for rnd in range(shifted_rounds + 2):
         ops.tf32_gemm(operand, operand, n, out=gram)
         shifted = rnd < shifted_rounds
         if shifted:
             gram.diagonal(dim1=-2, dim2=-1).add_(_CHOLQR_SHIFT * k)
-        a, operand = ops.chol_qr_round(gram, a, info, want_trans=not shifted)
+        operand = None  # (its memory serves the round)
+        operand = ops.chol_qr_round(gram, a, info, want_trans=not shifted)
         if shifted:
-            a, operand = unit_columns(a)
+            a, operand = unit_columns(a, True)
     ops.tf32_gemm(operand, operand, n, out=gram)
     ops.load().identity_defect(gram, _CHOLQR_ACCEPT, bad)
     return a

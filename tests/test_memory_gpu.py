@@ -40,6 +40,21 @@ def test_adamw_peak_memory_envelope():
     assert peak - rest < 1.3 * model_bytes, ((peak - rest) / model_bytes, rest / model_bytes)
 
 
+@pytest.mark.parametrize("shifted", [0, 1, 3])
+def test_refresh_of_a_basis_works_in_place(shifted):
+    """The matrix, its Gram matrix (4 bytes per element each) and three operands (8 each), the leaves' inverses beside them."""
+    from heavyball_b200.utils import orthogonal
+
+    x = torch.eye(1024, device="cuda") + 0.01 * torch.randn(4, 1024, 1024, device="cuda")
+    orthogonal._cholesky_qr2(x, shifted)
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    torch.cuda.reset_peak_memory_stats()
+    orthogonal._cholesky_qr2(x, shifted)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before < 34 * x.numel()
+
+
 def test_long_psgd_run_does_not_grow():
     model = _model(width=256, depth=3)
     opt = hb.PSGDKron(model.parameters(), lr=1e-3, preconditioner_update_probability=0.5)
