@@ -14,7 +14,7 @@
 // X X^T needs one split of X, and matrices that change rarely (eigenbases, preconditioner factors) stay split.
 //
 // Kernels and epilogues: gemm_epilogue.cuh; which tile when: gemm_rules.h.  SOAP's statistics and refresh run on this product (lerp into the
-// statistics matrix; added to a view for Schur complements and solves), projections, the rotation of the first moment and PSGD on that of
+// statistics matrix; added to a view for Schur complements and solves) and so does the rotation of its moments, projections and PSGD on that of
 // split16_gemm.cu.  Adam / LaProp on moment
 // buffers, a result written as a split operand - as it is or transposed - and products of upper-triangular matrices are here for callers of
 // ops.tf32_gemm and ops.matmul3.

@@ -462,7 +462,8 @@ def apply_flat_add(params: List[Tensor], update: Tensor, alpha):
 # not hold are computed in fp32, many times slower) and split-tf32.  Everything that an
 # eigenbasis is made from - statistics, power iteration, orthogonalisation - asks for the
 # second (``pairs=False``): eigenvectors with nearly equal Rayleigh quotients trade places when the last bits of any of these change,
-# so moving them would move every trajectory (two refreshes of eleven 2048-wide bases: one to three such pairs).
+# so moving them would move every trajectory (two refreshes of eleven 2048-wide bases: one to three such pairs).  So does the rotation of the
+# moments that follows, whose results are mostly near zero.
 
 
 def _tc_matmul(a: Tensor, b: Tensor, ta: bool = False, tb: bool = False, upper_upper: bool = False, pairs: bool = True):
